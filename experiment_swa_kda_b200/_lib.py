@@ -36,6 +36,7 @@ _SIGNATURES = {
     "kda_chunk_status": (C.c_int, [C.POINTER(ChunkShape), _P, _P]),
     "kda_chunk_status_async": (C.c_int, [C.POINTER(ChunkShape), _P, _P, _P]),
     "kda_status_word_code": (C.c_int, [C.c_int32]),
+    "kda_set_status_mirror": (C.c_int, [C.c_int32, _P]),
     "kda_selftest_bounded_wait": (C.c_int, [_P, C.c_uint32, _P]),
     "kda_gate_fwd": (C.c_int, [C.c_int32] * 4 + [_P] * 4 + [C.c_float] + [_P] * 3),
     "kda_gate_bwd_scratch_bytes": (C.c_size_t, [C.c_int32] * 3),

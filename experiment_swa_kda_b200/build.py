@@ -90,10 +90,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 # ----------------------------------------------------------------------------------------------
-# the operator library: TORCH_LIBRARY(nanochat_kda) over the C ABI, compiled by the host compiler against the
-# installed PyTorch (the role of torch.utils.cpp_extension.load(is_python_module=False) in the reference loader)
+# the operator library: TORCH_LIBRARY(nanochat_kda) over the C ABI and the native host path of the Python surface,
+# compiled by the host compiler against the installed PyTorch (the role of
+# torch.utils.cpp_extension.load(is_python_module=False) in the reference loader)
 # ----------------------------------------------------------------------------------------------
-SHIM_SRC = os.path.join(PKG, "torch_shim", "nanochat_kda_ops.cpp")
+SHIM_DIR = os.path.join(PKG, "torch_shim")
+SHIM_SRCS = [os.path.join(SHIM_DIR, "nanochat_kda_ops.cpp"), os.path.join(SHIM_DIR, "kda_host.cpp")]
 SHIM_LIB = os.path.join(LIBDIR, "libkda_b200_torch.so")
 
 
@@ -102,7 +104,8 @@ def torch_ops_stale() -> bool:
         return True
     t = os.path.getmtime(SHIM_LIB)
     inc = os.path.join(os.path.dirname(PKG), "include", "kda_b200.h")
-    return os.path.getmtime(SHIM_SRC) > t or os.path.getmtime(inc) > t or os.path.getmtime(LIB) > t
+    deps = SHIM_SRCS + [os.path.join(SHIM_DIR, "host_common.h"), inc, LIB]
+    return any(os.path.getmtime(p) > t for p in deps)
 
 
 def build_torch_ops(force: bool = False) -> str:
@@ -110,6 +113,7 @@ def build_torch_ops(force: bool = False) -> str:
     if not force and not torch_ops_stale():
         return SHIM_LIB
     import torch
+    import sysconfig
     from torch.utils import cpp_extension as ce
     cxx = shutil.which("g++") or shutil.which("c++")
     if not cxx:
@@ -118,8 +122,8 @@ def build_torch_ops(force: bool = False) -> str:
     cuda_inc = os.path.join(os.path.dirname(os.path.dirname(nvcc_path())), "include")
     cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            "-I" + os.path.join(os.path.dirname(PKG), "include"), "-I" + cuda_inc, *["-I" + i for i in ce.include_paths()],
-           SHIM_SRC, "-o", SHIM_LIB, "-L" + tlib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
-           "-L" + LIBDIR, "-lkda_b200", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib]
+           "-I" + sysconfig.get_paths()["include"], *SHIM_SRCS, "-o", SHIM_LIB, "-L" + tlib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
+           "-lc10_cuda", "-ltorch_python", "-L" + LIBDIR, "-lkda_b200", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib]
     with _BuildLock():
         if not force and not torch_ops_stale():
             return SHIM_LIB

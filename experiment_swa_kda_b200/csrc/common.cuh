@@ -7,6 +7,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "../../include/kda_b200.h"
 
 namespace kda {
@@ -31,6 +33,19 @@ __device__ __forceinline__ float warp_sum(float x) {
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
+// Device status of a workspace: int 0 is the status word, ints 2 and 3 hold the address of a page-locked host word that
+// mirrors it (null: none), left there by the forward's first kernel.  Only a failure writes either, so a call that goes
+// well pays nothing for being watched: the host reads its own memory at the next call.
+__device__ __forceinline__ void raise_status(int* status, int code) {
+    atomicCAS(status, 0, code);
+    volatile int* mirror = *reinterpret_cast<int* const*>(status + 2);
+    if (mirror != nullptr) {
+        *mirror = code;
+        __threadfence_system();
+    }
+}
+int* status_mirror();      // host: the mirror word registered for the current device, or null (kda_api.cu)
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -38,15 +53,46 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // KDA_LAUNCH, which counts it and, when profiling is enabled, brackets it with CUDA events on the
 // launching stream so a caller can read per-kernel device time.
 namespace prof {
+extern std::atomic<unsigned long long> launches;
+extern std::atomic<bool> enabled;
 void begin(const char* name, cudaStream_t st);
 void end(cudaStream_t st);
 }  // namespace prof
-#define KDA_LAUNCH(name, st, ...)      \
-    do {                               \
-        ::kda::prof::begin(name, st);  \
-        __VA_ARGS__;                   \
-        ::kda::prof::end(st);          \
+#define KDA_LAUNCH(name, st, ...)                                                        \
+    do {                                                                                 \
+        ::kda::prof::launches.fetch_add(1, std::memory_order_relaxed);                   \
+        const bool timed_ = ::kda::prof::enabled.load(std::memory_order_relaxed);        \
+        if (timed_) ::kda::prof::begin(name, st);                                        \
+        __VA_ARGS__;                                                                     \
+        if (timed_) ::kda::prof::end(st);                                                \
     } while (0)
+
+// Dynamic shared memory limit of a kernel: the attribute is a driver call, so it is set once per kernel and device.
+template <class Kern>
+inline int set_smem_limit(Kern kern, size_t bytes) {
+    constexpr int kDevices = 64, kKernels = 8;      // kernels that share a signature share this function's statics
+    static std::atomic<const void*> done[kDevices][kKernels];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return KDA_ERR_CUDA;
+    const void* key = reinterpret_cast<const void*>(kern);
+    if (dev < kDevices)
+        for (int i = 0; i < kKernels; ++i)
+            if (done[dev][i].load(std::memory_order_acquire) == key) return KDA_OK;
+    int most = 0;
+    if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return KDA_ERR_CUDA;
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, key) != cudaSuccess) return KDA_ERR_CUDA;
+    // the most the kernel may ask for, so that one call covers every size it is launched with
+    const int limit = most - (int)at.sharedSizeBytes;
+    if ((size_t)limit < bytes || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess)
+        return KDA_ERR_CUDA;
+    if (dev < kDevices)
+        for (int i = 0; i < kKernels; ++i) {
+            const void* none = nullptr;
+            if (done[dev][i].compare_exchange_strong(none, key, std::memory_order_release)) break;
+        }
+    return KDA_OK;
+}
 
 // Host-side launch check: returns a KDA_ERR_* code instead of throwing.
 inline int launch_status() {

@@ -155,15 +155,14 @@ struct Rec {
     cudaEvent_t a, b;
 };
 std::mutex mu;
-bool enabled = false;
-unsigned long long launches = 0;
 std::vector<Rec> recs;
 }  // namespace
 
+std::atomic<unsigned long long> launches{0};
+std::atomic<bool> enabled{false};
+
 void begin(const char* name, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(mu);
-    ++launches;
-    if (!enabled) return;
     Rec r{name, nullptr, nullptr};
     if (cudaEventCreate(&r.a) != cudaSuccess || cudaEventCreate(&r.b) != cudaSuccess) return;
     cudaEventRecord(r.a, st);
@@ -172,7 +171,7 @@ void begin(const char* name, cudaStream_t st) {
 
 void end(cudaStream_t st) {
     std::lock_guard<std::mutex> lk(mu);
-    if (!enabled || recs.empty()) return;
+    if (recs.empty()) return;
     cudaEventRecord(recs.back().b, st);
 }
 }  // namespace prof
@@ -188,16 +187,33 @@ extern "C" int kda_chunk_status_async(const KdaChunkShape* shape, const void* wo
     return chunk_status_async(shape, workspace, host_word, (cudaStream_t)stream);
 }
 
+namespace kda {
+namespace {
+constexpr int kMirrorDevices = 64;
+std::atomic<int32_t*> g_mirror[kMirrorDevices];
+}  // namespace
+
+int* status_mirror() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMirrorDevices) return nullptr;
+    return g_mirror[dev].load(std::memory_order_acquire);
+}
+}  // namespace kda
+
+extern "C" int kda_set_status_mirror(int32_t device, int32_t* host_word) {
+    if (device < 0 || device >= kMirrorDevices) return KDA_ERR_BAD_SHAPE;
+    g_mirror[device].store(host_word, std::memory_order_release);
+    return KDA_OK;
+}
+
 extern "C" int kda_status_word_code(int32_t word) { return status_word_to_code(word); }
 
 extern "C" unsigned long long kda_launch_count(void) {
-    std::lock_guard<std::mutex> lk(kda::prof::mu);
-    return kda::prof::launches;
+    return kda::prof::launches.load(std::memory_order_relaxed);
 }
 
 extern "C" void kda_profile_enable(int on) {
-    std::lock_guard<std::mutex> lk(kda::prof::mu);
-    kda::prof::enabled = on != 0;
+    kda::prof::enabled.store(on != 0);
 }
 
 extern "C" int kda_profile_report(char* out, size_t cap) {

@@ -1669,8 +1669,7 @@ int conv_bwd_fast(int n, int B, int T, int C, int bf16, int wf32, int silu, cons
         const int run = warps64 >= 148LL * 48 ? 64 : 32;
         grid = dim3(C / 128, ceil_div(T, 8 * run), B * n);                  // never more partial rows than the tile kernel's
         const size_t ring_bytes = (size_t)pw::kConvRingDepth * 2 * 256 * 8;
-        if (cudaFuncSetAttribute(pw::conv_bwd_ring_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes) != cudaSuccess)
-            return KDA_ERR_CUDA;
+        if (set_smem_limit(pw::conv_bwd_ring_kernel<W>, ring_bytes)) return KDA_ERR_CUDA;
         KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_ring_kernel<W><<<grid, 256, ring_bytes, st>>>(B, T, C, run, silu, wf32, it, part));
     } else if (bf16) KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_tile_kernel<W, true><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it, part));
     else KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_tile_kernel<W, false><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it, part));

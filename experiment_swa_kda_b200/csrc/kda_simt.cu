@@ -113,7 +113,7 @@ __device__ __forceinline__ void st_acc_g(float* dst, size_t ld, const float (&ac
 constexpr int kStatusBadCuSeqlens = 10;
 constexpr int kScanOrderMax = 512;      // batches up to this many sequences get a longest-first scan order
 
-__global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_seq, int seq_len, int tokens, int* status) {
+__global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_seq, int seq_len, int tokens, int* status, int* mirror) {
     __shared__ int total;
     if (threadIdx.x == 0) {
         int flag = 0;
@@ -134,7 +134,9 @@ __global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_s
         if (cu && (cu[0] != 0 || prev_end != tokens)) flag = 1;
         w.seq_chunk0[n_seq] = acc;
         total = acc;
-        *status = flag ? kStatusBadCuSeqlens : 0;      // every forward starts with a clean status word
+        *status = 0;                                   // every forward starts with a clean status word
+        *reinterpret_cast<int**>(status + 2) = mirror;
+        if (flag) raise_status(status, kStatusBadCuSeqlens);
     }
     __syncthreads();
     for (int s = threadIdx.x; s < n_seq; s += blockDim.x) {
@@ -946,11 +948,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
 
 template <class Kern>
 static int set_smem(Kern kern, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-            return KDA_ERR_CUDA;
-    }
-    return KDA_OK;
+    return bytes > 48 * 1024 ? set_smem_limit(kern, bytes) : KDA_OK;
 }
 
 int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const void* v, const void* g, const void* beta,
@@ -967,7 +965,7 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         simt::carve_ws(*sh, nullptr, &ws_bytes);
         tc::TcWs t = tc::carve_tc(*sh, static_cast<char*>(workspace) + ws_bytes);
         t.status = w.status;      // one status word per workspace, shared by both lanes
-        KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status));
+        KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status, status_mirror()));
         if (w.nslots > 0) {
             int rc = tc_intra_forward(w, t, q, k, v, g, beta, gbf16, sh->l2norm, sh->scale, sh->tokens, conv, st);
             if (rc) return rc;
@@ -977,7 +975,7 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         }
         return launch_status();
     }
-    KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status));
+    KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status, status_mirror()));
     if (w.nslots > 0) {
         dim3 gch(w.nslots, w.H);
         KDA_LAUNCH("prep_kernel", st, simt::prep_kernel<<<gch, 256, 0, st>>>(w, q, k, g, beta, bf16, gbf16, sh->l2norm, sh->scale));

@@ -725,7 +725,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     a.qinv = w.qinv; a.kinv = w.kinv; a.beta = w.beta; a.Mt = t.Mt;
     a.dq = static_cast<__nv_bfloat16*>(dq); a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
     a.dg = dg; a.dbeta = dbeta; a.gbf16 = gbf16; a.l2norm = l2norm; a.H = w.H; a.scale = scale; a.status = t.status;
-    if (cudaFuncSetAttribute(tc_intra_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kIntraBwdSmem) != cudaSuccess)
+    if (set_smem_limit(tc_intra_bwd_kernel, kIntraBwdSmem))
         return launch_status();
     KDA_LAUNCH("tc_intra_bwd_kernel", st,
                tc_intra_bwd_kernel<<<dim3(w.nslots, w.H), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, a));

@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(256, 3)
 static int scan_fixup(const simt::Ws& w, const tc::TcWs& t, int n_seq, __nv_bfloat16* panels, float* s_out, int bwd,
                       const CUtensorMap& mPp, const CUtensorMap& mF, cudaStream_t st) {
     using namespace tc;
-    if (cudaFuncSetAttribute(tc_scan_fixup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFixSmem) != cudaSuccess)
+    if (set_smem_limit(tc_scan_fixup_kernel, kFixSmem))
         return KDA_ERR_CUDA;
     ScanFixArgs f;
     f.seq_chunk0 = w.seq_chunk0; f.chunk_seq = w.chunk_seq; f.chunk_len = w.chunk_len; f.seg_fin = t.seg_fin;
@@ -874,8 +874,8 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
     else mG = mAT;
     if (rc) return KDA_ERR_CUDA;
     const int out_smem = fused_norm ? kChunkOutNormSmem : kChunkOutSmem;
-    if (cudaFuncSetAttribute(tc_affine_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAffineScanSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(tc_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkOutNormSmem) != cudaSuccess)
+    if (set_smem_limit(tc_affine_scan_kernel<false>, kAffineScanSmem) ||
+        set_smem_limit(tc_chunk_out_kernel, kChunkOutNormSmem))
         return KDA_ERR_CUDA;
     AffineScanArgs a;
     a.seq_chunk0 = w.seq_chunk0; a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len; a.decay_end = t.decay_end; a.s_in = h0; a.s_out = final_state;
@@ -920,8 +920,8 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
     rc |= make_map_bf16(&mRm, t.RmT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mdZT, t.dZT, nch * 128, 64, 64, 128);
     if (rc) return KDA_ERR_CUDA;
-    if (cudaFuncSetAttribute(tc_affine_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAffineScanSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(tc_chunk_dz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkDzSmem) != cudaSuccess)
+    if (set_smem_limit(tc_affine_scan_kernel<true>, kAffineScanSmem) ||
+        set_smem_limit(tc_chunk_dz_kernel, kChunkDzSmem))
         return KDA_ERR_CUDA;
     AffineScanArgs a;
     a.seq_chunk0 = w.seq_chunk0; a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len; a.decay_end = t.decay_end; a.s_in = d_final; a.s_out = dh0;

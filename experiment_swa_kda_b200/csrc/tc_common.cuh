@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace kda {
 namespace tc {
 
@@ -38,12 +40,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait.  On expiry writes `code` to *status (if not yet set) and returns false.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t limit = kSpinLimit) {
+// The bare bounded wait: false when the limit expires.
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity, uint32_t limit) {
     for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
     }
-    if (status) atomicCAS(status, 0, code);
+    return false;
+}
+// Bounded wait.  On expiry writes `code` to the workspace's status word (if not yet set) and to its host mirror, and
+// returns false.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code, uint32_t limit = kSpinLimit) {
+    if (mbar_poll(bar, parity, limit)) return true;
+    if (status) raise_status(status, code);
     return false;
 }
 

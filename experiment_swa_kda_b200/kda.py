@@ -20,7 +20,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import _lib, ops
+from . import _lib, _native, ops
 
 Tensor = torch.Tensor
 
@@ -173,35 +173,36 @@ def chunk_kda(q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor, *, initi
     When gradients are disabled, or no input requires one, the call is a prefill: the kernels skip every panel that
     only a backward would read and no workspace outlives the call.
     """
-    n_states = None
-    if cu_seqlens is not None:
-        if q.shape[0] != 1:
-            raise ValueError("packed inputs (cu_seqlens) require batch size 1")
-        if cu_seqlens.dtype != torch.int32 or cu_seqlens.ndim != 1 or cu_seqlens.numel() < 2:
-            raise ValueError("cu_seqlens must be int32 [N+1]")
-        n_states = cu_seqlens.numel() - 1
+    lane_id = _LANES.get(lane)
+    if lane_id is not None and q.is_cuda:
+        out = _native.load().chunk_kda(q, k, v, g, beta, initial_state, bool(output_final_state), cu_seqlens, scale, bool(use_qk_l2norm), lane_id)
+        if out is not None:
+            return out
+    # not the plain valid case: say why
+    n_states = _packed_states(q, cu_seqlens)
     _validate_operator_inputs(q, k, v, g, beta, initial_state, n_states)
     reason = _backend_reason(q, k, v, g, beta, None, None, initial_state, lower_bound=-1.0, allow_fp32=True)
     if reason is None and g.dtype != beta.dtype:
         reason = "g and beta must share a dtype"
-    if reason is not None:
-        raise RuntimeError(f"project CUDA KDA backend unavailable: {reason}")
-    sc = float(q.shape[-1] ** -0.5 if scale is None else scale)
-    lane_id = _select_lane(lane, q, v)
-    cu = None if cu_seqlens is None else cu_seqlens.contiguous()
-    return _chunk_dispatch(q, k, v, g, beta, initial_state, bool(output_final_state), cu, sc, bool(use_qk_l2norm), lane_id)
+    if reason is None:
+        _select_lane(lane, q, v)
+    raise RuntimeError(f"project CUDA KDA backend unavailable: {reason or _OTHER_REASON}")
 
 
-def _chunk_dispatch(q, k, v, g, beta, initial_state, output_final_state, cu, scale, l2norm, lane_id):
-    """Training calls go through the autograd Function (workspace kept for the backward); calls that cannot need a
-    backward take the forward-only kernels' path (the reference sends those to its token loop, chunk.cu:1694-1698)."""
-    tracked = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, g, beta, initial_state))
-    if tracked:
-        return ops.ChunkKDAFunction.apply(q, k, v, g, beta, initial_state, output_final_state, cu, scale, l2norm, lane_id)
-    q, k, v, g, beta = (t.detach().contiguous() for t in (q, k, v, g, beta))
-    h0 = None if initial_state is None else initial_state.detach().contiguous()
-    o, fs, _ = ops.chunk_kda_fwd(q, k, v, g, beta, h0, cu, scale, l2norm, output_final_state, lane_id, forward_only=True)
-    return o, fs
+# lane argument -> KDA_LANE_* (-1: the tensor-core lane whenever the shape allows it)
+_LANES = {"auto": -1, "fp32": _lib.LANE_FP32, "tc": _lib.LANE_TC}
+_OTHER_REASON = "g and beta must be float32 or bfloat16, and every tensor on the device of q"
+
+
+def _packed_states(q, cu_seqlens):
+    """Number of packed segments, or None for a fixed-length batch."""
+    if cu_seqlens is None:
+        return None
+    if q.shape[0] != 1:
+        raise ValueError("packed inputs (cu_seqlens) require batch size 1")
+    if cu_seqlens.dtype != torch.int32 or cu_seqlens.ndim != 1 or cu_seqlens.numel() < 2:
+        raise ValueError("cu_seqlens must be int32 [N+1]")
+    return cu_seqlens.numel() - 1
 
 
 def chunk_kda_norm(q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor, gate: Tensor, norm_weight: Tensor, *,
@@ -213,13 +214,12 @@ def chunk_kda_norm(q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor, gat
     Same results as the two operators in sequence (bit for bit in the forward), one launch and one read of the output
     less.  Needs the tensor-core lane: bfloat16 activations and K = V = 128; anything else raises.  gate [B,T,H,V];
     norm_weight [V]."""
-    n_states = None
-    if cu_seqlens is not None:
-        if q.shape[0] != 1:
-            raise ValueError("packed inputs (cu_seqlens) require batch size 1")
-        if cu_seqlens.dtype != torch.int32 or cu_seqlens.ndim != 1 or cu_seqlens.numel() < 2:
-            raise ValueError("cu_seqlens must be int32 [N+1]")
-        n_states = cu_seqlens.numel() - 1
+    if q.is_cuda:
+        out = _native.load().chunk_kda_norm(q, k, v, g, beta, gate, norm_weight, eps, initial_state, bool(output_final_state), cu_seqlens,
+                                            scale, bool(use_qk_l2norm))
+        if out is not None:
+            return out
+    n_states = _packed_states(q, cu_seqlens)
     _validate_operator_inputs(q, k, v, g, beta, initial_state, n_states)
     if gate.shape != v.shape:
         raise ValueError("gate must have the shape of v")
@@ -232,12 +232,7 @@ def chunk_kda_norm(q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor, gat
         reason = "the fused output norm needs the tensor-core lane (bfloat16, K = V = 128)"
     if reason is None and (gate.device != q.device or norm_weight.device != q.device):
         reason = "all KDA tensors must be on the same CUDA device"
-    if reason is not None:
-        raise RuntimeError(f"project CUDA KDA backend unavailable: {reason}")
-    sc = float(q.shape[-1] ** -0.5 if scale is None else scale)
-    cu = None if cu_seqlens is None else cu_seqlens.contiguous()
-    return ops.ChunkKDANormFunction.apply(q, k, v, g, beta, gate, norm_weight, initial_state, bool(output_final_state), cu, sc,
-                                          bool(use_qk_l2norm), float(eps))
+    raise RuntimeError(f"project CUDA KDA backend unavailable: {reason or _OTHER_REASON}")
 
 
 def _select_lane(lane: str, q: Tensor, v: Tensor) -> int:
@@ -257,8 +252,7 @@ def _select_lane(lane: str, q: Tensor, v: Tensor) -> int:
 
 def recurrent_kda_step(q, k, v, g, beta, state, *, scale=None, use_qk_l2norm=True):
     """One decode token on activated inputs; returns (o, new_state); `state` is not modified."""
-    sc = float(q.shape[-1] ** -0.5 if scale is None else scale)
-    return ops.decode_step(q, k, v, g, beta, state, sc, use_qk_l2norm)
+    return ops.decode_step(q, k, v, g, beta, state, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
 
 
 def kda(q: Tensor, k: Tensor, v: Tensor, raw_gate: Tensor, beta_logits: Tensor, A_log: Tensor, dt_bias: Tensor, *,
@@ -270,6 +264,12 @@ def kda(q: Tensor, k: Tensor, v: Tensor, raw_gate: Tensor, beta_logits: Tensor, 
     Only the project modes exist here; anything else raises (fail closed)."""
     if mode not in MODES:
         raise ValueError(f"unknown KDA mode: {mode}")
+    lane_id = _LANES.get(lane)
+    if mode == "project_chunk" and lane_id is not None and q.is_cuda:
+        out = _native.load().kda_raw(q, k, v, raw_gate, beta_logits, A_log, dt_bias, initial_state, bool(output_final_state), lower_bound,
+                                     scale, cu_seqlens, lane_id)
+        if out is not None:
+            return out
     n_states = None if cu_seqlens is None else cu_seqlens.numel() - 1
     _validate_operator_inputs(q, k, v, raw_gate, beta_logits, initial_state, n_states)
     _gate_shapes(raw_gate, A_log, dt_bias)
@@ -289,8 +289,9 @@ def kda(q: Tensor, k: Tensor, v: Tensor, raw_gate: Tensor, beta_logits: Tensor, 
             state = torch.zeros(q.shape[0], q.shape[2], v.shape[3], q.shape[3], dtype=torch.float32, device=q.device)
         o, new_state = ops.decode_step(q, k, v, g, beta, state.contiguous(), sc, True)
         return o, (new_state if output_final_state else None)
-    cu = None if cu_seqlens is None else cu_seqlens.contiguous()
-    return _chunk_dispatch(q, k, v, g, beta, initial_state, bool(output_final_state), cu, sc, True, _select_lane(lane, q, v))
+    _packed_states(q, cu_seqlens)
+    _select_lane(lane, q, v)
+    raise RuntimeError(f"project CUDA KDA backend unavailable: {_OTHER_REASON}")
 
 
 # ------------------------------------------------------------------------------------------
@@ -314,7 +315,7 @@ class RMSNormGated(nn.Module):
     def forward(self, x: Tensor, gate: Tensor) -> Tensor:
         if not x.is_cuda:
             raise RuntimeError("project CUDA gated RMSNorm cannot fall back on CPU")
-        return ops.RMSNormGateFunction.apply(x, gate, self.weight, self.eps)
+        return ops.rmsnorm_gated(x, gate, self.weight, self.eps)
 
 
 class ShortConvolution(nn.Conv1d):
@@ -340,7 +341,7 @@ class ShortConvolution(nn.Conv1d):
         if length == 0:
             cur = x.new_zeros(batch, channels, width) if state is None else state.to(x.dtype).clone()
             return x.new_empty(batch, 0, channels), (cur if output_final_state else None)
-        return ops.ConvFunction.apply(x, self.weight.squeeze(1), state, output_final_state, True)
+        return ops.conv(x, self.weight, state, output_final_state)
 
 
 def short_convolutions(convs, xs):
@@ -358,7 +359,7 @@ def short_convolutions(convs, xs):
             raise RuntimeError("project CUDA causal convolution cannot fall back on CPU")
     if len(convs) > 4 or xs[0].shape[1] == 0:
         return [conv(x)[0] for conv, x in zip(convs, xs)]
-    return list(ops.ConvMultiFunction.apply(True, len(convs), *xs, *[c.weight.squeeze(1) for c in convs]))
+    return list(ops.ConvMultiFunction.apply(True, len(convs), *xs, *[c.weight for c in convs]))
 
 
 class KimiDeltaAttention(nn.Module):

@@ -2,6 +2,8 @@
 
 PyTorch is used for device memory, the current CUDA stream and autograd bookkeeping;
 every arithmetic step runs in libkda_b200.so.  Nothing here falls back to PyTorch math.
+The differentiable operators are C++ (_native); the functions that call the C ABI through
+ctypes are its thin binding for callers that manage workspaces themselves.
 """
 
 from __future__ import annotations
@@ -10,7 +12,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 
 Tensor = torch.Tensor
 
@@ -60,53 +62,10 @@ def _shape(q, v, g, n_seq, seq_len, scale, l2norm, lane, forward_only=False) -> 
                            1 if l2norm else 0, float(scale), 1 if forward_only else 0)
 
 
-# ---- device status word without a hot-path synchronisation ------------------------------------
-# Every chunk forward / backward queues a 4-byte copy of its workspace's status word into a page-locked ring with an
-# event behind it.  The next call on that device reads the words whose events have completed (host memory, no wait) and
-# raises if one is non-zero, so an expired bounded wait or an inconsistent cu_seqlens cannot pass silently.  Nothing is
-# queued or polled while the stream is being captured into a CUDA graph.
-_STATUS_SLOTS = 64
-_status = {}      # device index -> [pinned int32 words, deque of (event, slot), next slot]
-
-
-def _capturing() -> bool:
-    return torch.cuda.is_current_stream_capturing()
-
-
 def poll_status(dev) -> None:
-    ring = _status.get(dev.index)
-    if ring is None or _capturing():
-        return
-    words, pending, _ = ring
-    bad = 0
-    while pending and pending[0][0].query():
-        _, slot = pending.popleft()
-        w = int(words[slot])
-        words[slot] = 0
-        bad = bad or w
-    if bad:
-        code = _lib.load().kda_status_word_code(bad)
-        msg = _lib.load().kda_error_string(code).decode()
-        raise RuntimeError(f"an earlier KDA call on {dev} reported device status {bad}: {msg} ({code}); its results are undefined")
-
-
-def _queue_status(sh, ws, dev) -> None:
-    if _capturing():
-        return
-    ring = _status.get(dev.index)
-    if ring is None:
-        import collections
-        ring = _status[dev.index] = [torch.zeros(_STATUS_SLOTS, dtype=torch.int32).pin_memory(), collections.deque(), 0]
-    words, pending, nxt = ring
-    if len(pending) >= _STATUS_SLOTS:      # the host is far ahead of the device: skip this sample
-        return
-    slot = nxt % _STATUS_SLOTS
-    ring[2] = nxt + 1
-    rc = _lib.load().kda_chunk_status_async(sh, _ptr(ws), words.data_ptr() + 4 * slot, _stream(dev))
-    if rc == _lib.OK:
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(dev))
-        pending.append((ev, slot))
+    """Raise if an earlier chunk call on `dev` left a device status (an expired bounded wait, an inconsistent cu_seqlens).
+    The kernels write a page-locked host word when something fails, so this is one read of host memory."""
+    _native.load().watch_status(torch.device(dev).index or 0)
 
 
 def chunk_kda_fwd(q, k, v, g, beta, h0, cu_seqlens, scale, l2norm, want_final, lane=_lib.LANE_FP32, forward_only=False, norm=None):
@@ -141,7 +100,6 @@ def chunk_kda_fwd(q, k, v, g, beta, h0, cu_seqlens, scale, l2norm, want_final, l
                                         _ptr(fs), _ptr(ws), ws.numel(), _ptr(gate), _ptr(nw), float(eps), _ptr(y), _ptr(inv),
                                         _stream(dev))
             _lib.check(rc, "kda_chunk_fwd_norm")
-        _queue_status(sh, ws, dev)
     if norm is not None:
         return o, fs, (sh, ws), y, inv
     return o, fs, (sh, ws)
@@ -172,7 +130,6 @@ def chunk_kda_conv_fwd(xq, xk, xv, wq, wk, wv, g, beta, h0, cu_seqlens, scale, l
                                     _lib.DTYPE_F32 if ws_[0].dtype == torch.float32 else _lib.DTYPE_BF16, _ptr(g), _ptr(beta),
                                     _ptr(h0), _ptr(cu_seqlens), _ptr(o), _ptr(fs), _ptr(ws), ws.numel(), _stream(dev))
         _lib.check(rc, "kda_chunk_fwd_conv")
-        _queue_status(sh, ws, dev)
     return o, fs
 
 
@@ -191,7 +148,6 @@ def chunk_kda_bwd(q, k, v, g, beta, cu_seqlens, do, dfs, saved, want_dh0):
                                _ptr(ws), ws.numel(), _ptr(scr), scr.numel(), _ptr(dq), _ptr(dk), _ptr(dv), _ptr(dg),
                                _ptr(db), _ptr(dh0), _stream(dev))
         _lib.check(rc, "kda_chunk_bwd")
-        _queue_status(sh, ws, dev)
     return dq, dk, dv, dg, db, dh0
 
 
@@ -203,115 +159,22 @@ def chunk_status(saved, dev) -> None:
     _lib.check(rc, "kda_chunk_status")
 
 
-class ChunkKDAFunction(torch.autograd.Function):
-    """Autograd boundary of the chunked operator on activated inputs.
-
-    Argument list of the operator surface: (q, k, v, g, beta, initial_state,
-    output_final_state, cu_seqlens) plus scale / l2norm / lane.  Mirrors the role of
-    the reference's _ProjectKDAAutograd (nanochat/mixers/kda.py:383-415).
-    """
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, beta, initial_state, output_final_state, cu_seqlens, scale, l2norm, lane):
-        q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g, beta))
-        h0 = None if initial_state is None else initial_state.contiguous()
-        o, fs, (sh, ws) = chunk_kda_fwd(q, k, v, g, beta, h0, cu_seqlens, scale, l2norm, output_final_state, lane)
-        ctx.shape = sh
-        ctx.cu = cu_seqlens
-        ctx.has_h0 = initial_state is not None
-        # The workspace rides with the saved tensors: it lives exactly as long as the graph does, and a second backward
-        # through a retained graph finds it intact (the backward kernels only read it).
-        ctx.save_for_backward(q, k, v, g, beta, ws)
-        ctx.set_materialize_grads(False)
-        return o, fs
-
-    @staticmethod
-    def backward(ctx, do, dfs):
-        q, k, v, g, beta, ws = ctx.saved_tensors
-        do = torch.zeros_like(v) if do is None else do.contiguous()
-        if dfs is not None:
-            dfs = dfs.contiguous().float()
-        dq, dk, dv, dg, db, dh0 = chunk_kda_bwd(q, k, v, g, beta, ctx.cu, do, dfs, (ctx.shape, ws), ctx.has_h0)
-        return dq, dk, dv, dg, db, dh0, None, None, None, None, None
-
-
-class ChunkKDANormFunction(torch.autograd.Function):
-    """Chunked KDA followed by the layer's gated RMSNorm, the norm applied in the output kernel's epilogue (one launch and
-    one pass over the output less than the two operators in sequence; the reference layer crosses an operator boundary
-    here, nanochat/mixers/kda.py:768-795).  Tensor-core lane only.  The backward is the two existing backwards in sequence."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, beta, gate, norm_weight, initial_state, output_final_state, cu_seqlens, scale, l2norm, eps):
-        q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g, beta))
-        gate = gate.contiguous().to(v.dtype)
-        w32 = norm_weight.contiguous().float()
-        h0 = None if initial_state is None else initial_state.contiguous()
-        o, fs, (sh, ws), y, inv = chunk_kda_fwd(q, k, v, g, beta, h0, cu_seqlens, scale, l2norm, output_final_state,
-                                                _lib.LANE_TC, norm=(gate, w32, eps))
-        ctx.shape, ctx.cu, ctx.has_h0, ctx.wdtype = sh, cu_seqlens, initial_state is not None, norm_weight.dtype
-        ctx.save_for_backward(q, k, v, g, beta, ws, o, gate, w32, inv)
-        ctx.set_materialize_grads(False)
-        return y, fs
-
-    @staticmethod
-    def backward(ctx, dy, dfs):
-        q, k, v, g, beta, ws, o, gate, w32, inv = ctx.saved_tensors
-        dy = torch.zeros_like(o) if dy is None else dy.contiguous().to(o.dtype)
-        do, dgate, dw = rmsnorm_gate_bwd(o, gate, w32, inv, dy)
-        if dfs is not None:
-            dfs = dfs.contiguous().float()
-        dq, dk, dv, dg, db, dh0 = chunk_kda_bwd(q, k, v, g, beta, ctx.cu, do, dfs, (ctx.shape, ws), ctx.has_h0)
-        return dq, dk, dv, dg, db, dgate, dw.to(ctx.wdtype), dh0, None, None, None, None, None
-
-
 # --------------------------------------------------------------------------------------------
 # gate activations
 # --------------------------------------------------------------------------------------------
 
-class GateFunction(torch.autograd.Function):
-    """(raw_gate, beta_logits, A_log, dt_bias) -> (g, beta) in float32, with the parameter
-    gradients reduced deterministically (reference chunk_wy_backward.cu:3881-3987)."""
+class GateFunction:
+    """(raw_gate, beta_logits, A_log, dt_bias) -> (g, beta) in float32, differentiable, with the parameter gradients
+    reduced deterministically (reference chunk_wy_backward.cu:3881-3987)."""
 
     @staticmethod
-    def forward(ctx, raw_gate, beta_logits, A_log, dt_bias, lower_bound):
-        lib = _lib.load()
-        dev = _need_cuda(raw_gate, beta_logits, A_log, dt_bias)
-        raw_gate, beta_logits = raw_gate.contiguous(), beta_logits.contiguous()
-        A32, b32 = A_log.contiguous().float(), dt_bias.contiguous().float().reshape(-1)
-        B, T, H, K = raw_gate.shape
-        if beta_logits.dtype != raw_gate.dtype:
-            beta_logits = beta_logits.to(raw_gate.dtype)
-        g = torch.empty(B, T, H, K, dtype=torch.float32, device=dev)
-        beta = torch.empty(B, T, H, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            rc = lib.kda_gate_fwd(B * T, H, K, _dt(raw_gate), _ptr(raw_gate), _ptr(beta_logits), _ptr(A32), _ptr(b32),
-                                  float(lower_bound), _ptr(g), _ptr(beta), _stream(dev))
-        _lib.check(rc, "kda_gate_fwd")
-        ctx.save_for_backward(raw_gate, beta_logits, A32, b32)
-        ctx.lb = float(lower_bound)
-        ctx.bias_shape = dt_bias.shape
-        ctx.out_dtypes = (A_log.dtype, dt_bias.dtype)
-        return g, beta
-
-    @staticmethod
-    def backward(ctx, dg, dbeta):
-        lib = _lib.load()
-        raw_gate, beta_logits, A32, b32 = ctx.saved_tensors
-        dev = raw_gate.device
-        B, T, H, K = raw_gate.shape
-        dg = dg.contiguous().float()
-        dbeta = dbeta.contiguous().float()
-        d_raw = torch.empty_like(raw_gate)
-        d_bl = torch.empty_like(beta_logits)
-        dA = torch.empty(H, dtype=torch.float32, device=dev)
-        dbias = torch.empty(H * K, dtype=torch.float32, device=dev)
-        scr = _bytes(lib.kda_gate_bwd_scratch_bytes(B * T, H, K), dev)
-        with torch.cuda.device(dev):
-            rc = lib.kda_gate_bwd(B * T, H, K, _dt(raw_gate), _ptr(raw_gate), _ptr(beta_logits), _ptr(A32), _ptr(b32),
-                                  ctx.lb, _ptr(dg), _ptr(dbeta), _ptr(d_raw), _ptr(d_bl), _ptr(dA), _ptr(dbias),
-                                  _ptr(scr), scr.numel(), _stream(dev))
-        _lib.check(rc, "kda_gate_bwd")
-        return d_raw, d_bl, dA.to(ctx.out_dtypes[0]), dbias.reshape(ctx.bias_shape).to(ctx.out_dtypes[1]), None
+    def apply(raw_gate, beta_logits, A_log, dt_bias, lower_bound):
+        out = _native.load().gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound)
+        if out is None:
+            _need_cuda(raw_gate, beta_logits, A_log, dt_bias)
+            _dt(raw_gate)
+            raise RuntimeError("kda_gate_fwd takes raw_gate [B,T,H,K], beta_logits [B,T,H], A_log [H] and dt_bias with H*K values")
+        return out
 
 
 # --------------------------------------------------------------------------------------------
@@ -322,6 +185,10 @@ def decode_step(q, k, v, g, beta, state, scale, l2norm=True, out_state: Optional
     """One token per sequence.  q,k,g [B,1,H,K] (or [B,H,K]); state [B,H,V,K] float32.
     Returns (o shaped like v, new state).  The input state is left untouched unless
     out_state aliases it."""
+    if q.is_cuda:
+        out = _native.load().decode_step(q, k, v, g, beta, state, scale, bool(l2norm), out_state)
+        if out is not None:
+            return out
     lib = _lib.load()
     dev = _need_cuda(q, k, v, g, beta, state)
     q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g, beta))
@@ -450,100 +317,32 @@ def conv_bwd(x, weight, initial_state, dy, dfin, silu=True):
     return dx, dw, dinit
 
 
-class ConvFunction(torch.autograd.Function):
-    """Causal depthwise convolution + SiLU with an explicit cache
-    (role of the reference's _ProjectConvolutionAutograd, nanochat/mixers/kda.py:439-466)."""
-
-    @staticmethod
-    def forward(ctx, x, weight, initial_state, output_final_state, silu):
-        x = x.contiguous()
-        w = weight.contiguous()
-        if w.dtype != torch.float32:
-            w = w.to(x.dtype)
-        s0 = None if initial_state is None else initial_state.contiguous().to(x.dtype)
-        y, fin = conv_fwd(x, w, s0, output_final_state, silu)
-        ctx.save_for_backward(x, w, s0)
-        ctx.silu = silu
-        ctx.wdtype = weight.dtype
-        return y, fin
-
-    @staticmethod
-    def backward(ctx, dy, dfin):
-        x, w, s0 = ctx.saved_tensors
-        dy = dy.contiguous().to(x.dtype)
-        if dfin is not None:
-            dfin = dfin.contiguous().to(x.dtype)
-        dx, dw, dinit = conv_bwd(x, w, s0, dy, dfin, ctx.silu)
-        return dx, dw.to(ctx.wdtype), dinit, None, None
-
-
 def _ptr_array(ts):
     import ctypes as C
     arr = (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
     return arr
 
 
-class ConvMultiFunction(torch.autograd.Function):
-    """n same-shaped causal convolutions + SiLU (the q, k and v branches of a layer) in one launch each way.
-    Training path only (no cache, no final state); falls back to the per-tensor operator when the library declines."""
+class ConvMultiFunction:
+    """n same-shaped causal convolutions + SiLU (the q, k and v branches of a layer) in one launch each way, differentiable.
+    Training path only (no cache, no final state); runs the tensors one by one when the library declines."""
 
     @staticmethod
-    def forward(ctx, silu, n, *tensors):
-        import ctypes as C
-        xs = [t.contiguous() for t in tensors[:n]]
-        ws = []
-        for w in tensors[n:]:
-            w = w.contiguous()
-            ws.append(w if w.dtype == torch.float32 else w.to(xs[0].dtype))
-        lib = _lib.load()
-        dev = _need_cuda(*xs, *ws)
-        B, T, Cc = xs[0].shape
-        W = ws[0].shape[-1]
-        same = all(x.shape == xs[0].shape and x.dtype == xs[0].dtype for x in xs) and \
-            all(w.shape == ws[0].shape and w.dtype == ws[0].dtype for w in ws)
-        ys = [torch.empty_like(x) for x in xs]
-        rc = _lib.ERR_UNSUPPORTED
-        if same:
-            with torch.cuda.device(dev):
-                rc = lib.kda_conv_fwd_multi(n, B, T, Cc, W, _dt(xs[0]) | _wflag(xs[0], ws[0]), 1 if silu else 0,
-                                            C.cast(_ptr_array(xs), C.c_void_p), C.cast(_ptr_array(ws), C.c_void_p),
-                                            C.cast(_ptr_array(ys), C.c_void_p), _stream(dev))
-        if rc == _lib.ERR_UNSUPPORTED:
-            ys = [conv_fwd(x, w, None, False, silu)[0] for x, w in zip(xs, ws)]
-        else:
-            _lib.check(rc, "kda_conv_fwd_multi")
-        ctx.save_for_backward(*xs, *ws)
-        ctx.n, ctx.silu, ctx.same = n, silu, same
-        ctx.wdtypes = [w.dtype for w in tensors[n:]]
-        return tuple(ys)
+    def apply(silu, n, *tensors):
+        xs, ws = list(tensors[:n]), list(tensors[n:])
+        ys = _native.load().conv_multi(xs, ws, bool(silu))
+        return tuple(ys) if ys is not None else tuple(conv(x, w, None, False, silu)[0] for x, w in zip(xs, ws))
 
-    @staticmethod
-    def backward(ctx, *dys):
-        import ctypes as C
-        n = ctx.n
-        saved = ctx.saved_tensors
-        xs, ws = list(saved[:n]), list(saved[n:])
-        dys = [(torch.zeros_like(x) if d is None else d.contiguous().to(x.dtype)) for d, x in zip(dys, xs)]
-        lib = _lib.load()
-        dev = xs[0].device
-        B, T, Cc = xs[0].shape
-        W = ws[0].shape[-1]
-        dxs = [torch.empty_like(x) for x in xs]
-        dws = [torch.empty(Cc, W, dtype=torch.float32, device=dev) for _ in xs]
-        rc = _lib.ERR_UNSUPPORTED
-        if ctx.same:
-            scr = _bytes(lib.kda_conv_bwd_multi_scratch_bytes(n, B, T, Cc, W), dev)
-            with torch.cuda.device(dev):
-                rc = lib.kda_conv_bwd_multi(n, B, T, Cc, W, _dt(xs[0]) | _wflag(xs[0], ws[0]), 1 if ctx.silu else 0,
-                                            C.cast(_ptr_array(xs), C.c_void_p), C.cast(_ptr_array(ws), C.c_void_p),
-                                            C.cast(_ptr_array(dys), C.c_void_p), C.cast(_ptr_array(dxs), C.c_void_p),
-                                            C.cast(_ptr_array(dws), C.c_void_p), _ptr(scr), scr.numel(), _stream(dev))
-        if rc == _lib.ERR_UNSUPPORTED:
-            res = [conv_bwd(x, w, None, d, None, ctx.silu) for x, w, d in zip(xs, ws, dys)]
-            dxs, dws = [r[0] for r in res], [r[1] for r in res]
-        else:
-            _lib.check(rc, "kda_conv_bwd_multi")
-        return (None, None, *dxs, *[dw.to(dt) for dw, dt in zip(dws, ctx.wdtypes)])
+
+def conv(x, weight, initial_state, output_final_state, silu=True):
+    """Causal depthwise convolution (+ SiLU) with an explicit cache, differentiable (role of the reference's
+    _ProjectConvolutionAutograd, nanochat/mixers/kda.py:439-466).  weight [C,W] or [C,1,W]."""
+    out = _native.load().conv(x, weight, initial_state, bool(output_final_state), bool(silu))
+    if out is None:
+        _need_cuda(x, weight, initial_state)
+        _dt(x)
+        raise RuntimeError("the convolution takes x [B,T,C], weight [C,W] and a state [B,C,W], none of them empty")
+    return out
 
 
 # --------------------------------------------------------------------------------------------
@@ -579,22 +378,14 @@ def rmsnorm_gate_bwd(x, gate, weight, inv, dy):
     return dx, dgate, dw
 
 
-class RMSNormGateFunction(torch.autograd.Function):
-    """y = rms_norm(x; w, eps) * sigmoid(gate)
+def rmsnorm_gated(x, gate, weight, eps):
+    """y = rms_norm(x; w, eps) * sigmoid(gate), differentiable
     (role of the reference's _ProjectRMSNormGateAutograd, nanochat/mixers/kda.py:418-436)."""
-
-    @staticmethod
-    def forward(ctx, x, gate, weight, eps):
-        x = x.contiguous()
-        gate = gate.contiguous().to(x.dtype)
-        w32 = weight.contiguous().float()
-        y, inv = rmsnorm_gate_fwd(x, gate, w32, eps)
-        ctx.save_for_backward(x, gate, w32, inv)
-        ctx.wdtype = weight.dtype
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, gate, w32, inv = ctx.saved_tensors
-        dx, dgate, dw = rmsnorm_gate_bwd(x, gate, w32, inv, dy.contiguous().to(x.dtype))
-        return dx, dgate, dw.to(ctx.wdtype), None
+    y = _native.load().rmsnorm(x, gate, weight, eps)
+    if y is None:
+        _need_cuda(x, gate, weight)
+        _dt(x)
+        if x.numel() == 0 and gate.shape == x.shape:
+            return x * gate * weight.to(x.dtype)      # nothing to normalise; keeps the graph
+        raise RuntimeError("the gated RMSNorm takes x and gate of one shape and a weight of their last dimension")
+    return y

@@ -19,40 +19,21 @@
 // backward kernels.  An `output` that is not such a head (a copy, or a forward that ran without gradients) makes the
 // backward run the forward again into a fresh workspace first.
 
-#include <ATen/ATen.h>
-#include <ATen/cuda/CUDAContext.h>
-#include <ATen/cuda/CUDAEvent.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
-#include <c10/cuda/CUDAGuard.h>
-#include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
 
-#include <deque>
 #include <mutex>
 #include <tuple>
 #include <unordered_map>
 
-#include "kda_b200.h"
+#include "host_common.h"
 
 namespace {
 
-using at::Tensor;
-using OptTensor = c10::optional<Tensor>;
+using namespace kda_host;
 
 void check(int rc, const char* what) {
     TORCH_CHECK(rc == 0, "libkda_b200: ", what, " failed: ", kda_error_string(rc), " (", rc, ")");
 }
-
-void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
-
-bool has(const OptTensor& t) { return t.has_value() && t->defined(); }
-const void* ptr(const OptTensor& t) { return has(t) ? t->data_ptr() : nullptr; }
-
-Tensor bytes(size_t n, const Tensor& like) {
-    return at::empty({(int64_t)(n < 256 ? 256 : n)}, like.options().dtype(at::kByte));
-}
-
-size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 
 // ------------------------------------------------------------------------------------------------ validation
 struct Dims {
@@ -111,61 +92,6 @@ Dims validate_chunk_inputs(const Tensor& q, const Tensor& k, const Tensor& v, co
 void validate_only(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& raw_gate, const Tensor& beta_logits, const Tensor& A_log,
                    const Tensor& dt_bias, const OptTensor& initial_state, double lower_bound, const OptTensor& cu_seqlens) {
     validate_chunk_inputs(q, k, v, raw_gate, beta_logits, A_log, dt_bias, initial_state, lower_bound, cu_seqlens);
-}
-
-// ------------------------------------------------------------------------------------------------ device status
-// Every chunk forward / backward queues a 4-byte copy of its workspace's status word into a page-locked ring and an
-// event behind it; the next call on that device reads the words whose events have completed (a host memory read, no
-// synchronisation) and raises if one is non-zero - an expired bounded wait or an inconsistent cu_seqlens therefore
-// cannot pass silently, and the hot path never waits.  Skipped while a stream capture is in progress.
-struct StatusRing {
-    Tensor words;      // pinned int32 [kSlots]
-    struct Pending {
-        at::cuda::CUDAEvent ev;
-        int slot;
-    };
-    std::deque<Pending> pending;
-    int next = 0;
-};
-constexpr int kSlots = 64;
-std::mutex status_mu;
-std::unordered_map<int, StatusRing> rings;
-
-bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
-
-void poll_status(int device) {
-    if (capturing()) return;
-    std::lock_guard<std::mutex> lk(status_mu);
-    auto it = rings.find(device);
-    if (it == rings.end()) return;
-    StatusRing& r = it->second;
-    int bad = 0;
-    while (!r.pending.empty() && r.pending.front().ev.query()) {
-        int32_t* w = r.words.data_ptr<int32_t>() + r.pending.front().slot;
-        if (*w != 0 && bad == 0) bad = *w;
-        *w = 0;
-        r.pending.pop_front();
-    }
-    if (bad != 0) {
-        const int rc = kda_status_word_code(bad);
-        TORCH_CHECK(false, "libkda_b200: an earlier KDA call on cuda:", device, " reported device status ", bad, ": ", kda_error_string(rc),
-                    " (", rc, "); its results are undefined");
-    }
-}
-
-void queue_status(const KdaChunkShape& sh, const void* workspace, const Tensor& like) {
-    if (capturing()) return;
-    const int device = like.device().index();
-    std::lock_guard<std::mutex> lk(status_mu);
-    StatusRing& r = rings[device];
-    if (!r.words.defined()) r.words = at::zeros({kSlots}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-    if ((int)r.pending.size() >= kSlots) return;      // the host is far ahead of the device: skip this sample
-    const int slot = r.next++ % kSlots;
-    auto stream = c10::cuda::getCurrentCUDAStream(device);
-    if (kda_chunk_status_async(&sh, workspace, r.words.data_ptr<int32_t>() + slot, stream.stream()) != KDA_OK) return;
-    r.pending.emplace_back();
-    r.pending.back().slot = slot;
-    r.pending.back().ev.record(stream);
 }
 
 // ------------------------------------------------------------------------------------------------ chunked operator
@@ -227,7 +153,7 @@ std::tuple<Tensor, OptTensor> chunk_forward(const Tensor& q_, const Tensor& k_, 
                                             const OptTensor& cu_seqlens) {
     const Dims d = validate_chunk_inputs(q_, k_, v_, raw_gate_, beta_logits_, A_log, dt_bias, initial_state, lower_bound, cu_seqlens);
     c10::cuda::CUDAGuard guard(q_.device());
-    poll_status(q_.device().index());
+    watch_status(q_.device().index());
     const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), raw_gate = raw_gate_.contiguous(),
                  beta_logits = beta_logits_.contiguous();
     // A call none of whose inputs takes part in a graph is inference / prefill: nothing is kept for a backward.
@@ -249,7 +175,6 @@ std::tuple<Tensor, OptTensor> chunk_forward(const Tensor& q_, const Tensor& k_, 
                             static_cast<const int32_t*>(ptr(cu_seqlens)), output.data_ptr(),
                             output_final_state ? final_state->data_ptr<float>() : nullptr, base + l.ws_off, l.ws_bytes, stream_of(q)),
               "kda_chunk_fwd");
-        queue_status(sh, base + l.ws_off, q);
     } else if (output_final_state) {
         if (has(initial_state)) final_state->copy_(*initial_state);
         else final_state->zero_();
@@ -278,7 +203,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
         TORCH_CHECK(grad_final_state->is_cuda() && grad_final_state->device() == q_.device(), "grad_final_state must be on the same device as q");
     }
     c10::cuda::CUDAGuard guard(q_.device());
-    poll_status(q_.device().index());
+    watch_status(q_.device().index());
     const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), raw_gate = raw_gate_.contiguous(),
                  beta_logits = beta_logits_.contiguous();
     const bool packed = has(cu_seqlens);
@@ -331,7 +256,6 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
                         l.ws_bytes, scratch.data_ptr(), (size_t)scratch.numel(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(),
                         db.data_ptr(), dh0.has_value() ? dh0->data_ptr<float>() : nullptr, stream_of(q)),
           "kda_chunk_bwd");
-    queue_status(sh, base + l.ws_off, q);
     Tensor gscr = bytes(kda_gate_bwd_scratch_bytes((int32_t)(d.B * d.T), (int32_t)d.H, (int32_t)d.K), q);
     check(kda_gate_bwd((int32_t)(d.B * d.T), (int32_t)d.H, (int32_t)d.K, KDA_DTYPE_BF16, raw_gate.data_ptr(), beta_logits.data_ptr(),
                        A_log.data_ptr<float>(), dt_bias.data_ptr<float>(), (float)lower_bound, dg.data_ptr<float>(), db.data_ptr<float>(),

@@ -133,6 +133,11 @@ int kda_chunk_bwd(const KdaChunkShape* shape, const void* q, const void* k, cons
 int kda_chunk_status(const KdaChunkShape* shape, const void* workspace, void* stream);
 int kda_chunk_status_async(const KdaChunkShape* shape, const void* workspace, int32_t* host_word, void* stream);
 int kda_status_word_code(int32_t word);
+/* Registers a page-locked (device-accessible) host word for `device`: a forward / backward whose status word is raised
+ * also stores the code there, so the host can watch for failures by reading its own memory - no copy, event or
+ * synchronisation per call, and it works for kernels replayed from a CUDA graph too.  The word must stay valid while
+ * calls are in flight; null unregisters.  No reference counterpart. */
+int kda_set_status_mirror(int32_t device, int32_t* host_word);
 /* Self-test of the bounded wait: a one-warp kernel waits poll_limit (<= 1,000,000) polls on a barrier nothing arrives
  * at, then returns.  device_words[0] receives the status word (non-zero after the wait ran out), device_words[1] is 2
  * when the kernel carried on past the expired wait.  Never traps and never spins without bound.  No reference
