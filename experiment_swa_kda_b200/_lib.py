@@ -31,6 +31,7 @@ _SIGNATURES = {
     "kda_chunk_bwd_scratch_bytes": (C.c_size_t, [C.POINTER(ChunkShape)]),
     "kda_chunk_fwd": (C.c_int, [C.POINTER(ChunkShape)] + [_P] * 10 + [C.c_size_t, _P]),
     "kda_chunk_fwd_conv": (C.c_int, [C.POINTER(ChunkShape)] + [_P] * 6 + [C.c_int32, C.c_int32] + [_P] * 7 + [C.c_size_t, _P]),
+    "kda_chunk_fwd_ex": (C.c_int, [C.POINTER(ChunkShape)] + [_P] * 11 + [C.c_size_t, _P]),
     "kda_chunk_fwd_norm": (C.c_int, [C.POINTER(ChunkShape)] + [_P] * 10 + [C.c_size_t, _P, _P, C.c_float, _P, _P, _P]),
     "kda_chunk_bwd": (C.c_int, [C.POINTER(ChunkShape)] + [_P] * 9 + [C.c_size_t, _P, C.c_size_t] + [_P] * 7),
     "kda_chunk_status": (C.c_int, [C.POINTER(ChunkShape), _P, _P]),
@@ -41,6 +42,9 @@ _SIGNATURES = {
     "kda_gate_fwd": (C.c_int, [C.c_int32] * 4 + [_P] * 4 + [C.c_float] + [_P] * 3),
     "kda_gate_bwd_scratch_bytes": (C.c_size_t, [C.c_int32] * 3),
     "kda_gate_bwd": (C.c_int, [C.c_int32] * 4 + [_P] * 4 + [C.c_float] + [_P] * 7 + [C.c_size_t, _P]),
+    "kda_gate_fwd_rows": (C.c_int, [C.c_int32] * 4 + [_P] * 2 + [C.c_int32] + [_P] * 2 + [C.c_float] + [_P] * 3),
+    "kda_gate_bwd_rows": (C.c_int, [C.c_int32] * 4 + [_P] * 2 + [C.c_int32] * 2 + [_P] * 2 + [C.c_float] + [_P] * 7 + [C.c_size_t, _P]),
+    "kda_pack_bf16": (C.c_int, [C.c_int32] * 2 + [_P] * 4),
     "kda_decode_step": (C.c_int, [C.c_int32] * 7 + [C.c_float] + [_P] * 9),
     "kda_decode_step_raw": (C.c_int, [C.c_int32] * 5 + [C.c_float] + [_P] * 7 + [C.c_float] + [_P] * 4),
     "kda_conv_step_multi": (C.c_int, [C.c_int32] * 6 + [_P] * 5),
@@ -51,6 +55,9 @@ _SIGNATURES = {
     "kda_conv_fwd_multi": (C.c_int, [C.c_int32] * 7 + [_P] * 4),
     "kda_conv_bwd_multi_scratch_bytes": (C.c_size_t, [C.c_int32] * 5),
     "kda_conv_bwd_multi": (C.c_int, [C.c_int32] * 7 + [_P] * 6 + [C.c_size_t, _P]),
+    "kda_conv_fwd_rows": (C.c_int, [C.c_int32] * 7 + [_P, C.c_int32] + [_P] * 5),
+    "kda_conv_bwd_rows": (C.c_int, [C.c_int32] * 7 + [_P, C.c_int32] + [_P] * 5 + [C.c_size_t, _P]),
+    "kda_rmsnorm_gate_bwd_rows": (C.c_int, [C.c_int64] + [C.c_int32] * 3 + [_P] * 9 + [C.c_size_t, _P]),
     "kda_rmsnorm_gate_fwd": (C.c_int, [C.c_int64, C.c_int32, C.c_int32, C.c_float] + [_P] * 6),
     "kda_rmsnorm_gate_bwd_scratch_bytes": (C.c_size_t, [C.c_int64, C.c_int32]),
     "kda_rmsnorm_gate_bwd": (C.c_int, [C.c_int64, C.c_int32, C.c_int32] + [_P] * 9 + [C.c_size_t, _P]),

@@ -95,7 +95,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 # torch.utils.cpp_extension.load(is_python_module=False) in the reference loader)
 # ----------------------------------------------------------------------------------------------
 SHIM_DIR = os.path.join(PKG, "torch_shim")
-SHIM_SRCS = [os.path.join(SHIM_DIR, "nanochat_kda_ops.cpp"), os.path.join(SHIM_DIR, "kda_host.cpp")]
+SHIM_SRCS = [os.path.join(SHIM_DIR, f) for f in ("nanochat_kda_ops.cpp", "kda_host.cpp", "kda_layer.cpp")]
 SHIM_LIB = os.path.join(LIBDIR, "libkda_b200_torch.so")
 
 
@@ -104,7 +104,7 @@ def torch_ops_stale() -> bool:
         return True
     t = os.path.getmtime(SHIM_LIB)
     inc = os.path.join(os.path.dirname(PKG), "include", "kda_b200.h")
-    deps = SHIM_SRCS + [os.path.join(SHIM_DIR, "host_common.h"), inc, LIB]
+    deps = SHIM_SRCS + [os.path.join(SHIM_DIR, f) for f in ("host_common.h", "host_node.h")] + [inc, LIB]
     return any(os.path.getmtime(p) > t for p in deps)
 
 

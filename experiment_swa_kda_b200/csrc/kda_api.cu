@@ -90,39 +90,59 @@ extern "C" int kda_chunk_fwd(const KdaChunkShape* shape, const void* q, const vo
     return simt_chunk_fwd(shape, q, k, v, g, beta, h0, cu_seqlens, o, final_state, workspace, (cudaStream_t)stream, nullptr);
 }
 
+extern "C" int kda_chunk_fwd_ex(const KdaChunkShape* shape, const KdaChunkExtras* ex, const void* q, const void* k, const void* v, const void* g,
+                                const void* beta, const float* h0, const int32_t* cu_seqlens, void* o, float* final_state,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+    int rc = check_shape(shape, cu_seqlens);
+    if (rc) return rc;
+    if (!ex) return KDA_ERR_NULL;
+    // the extras live in the tensor-core lane's kernels
+    if (shape->lane != KDA_LANE_TC) return KDA_ERR_UNSUPPORTED;
+    const bool norm = ex->gate != nullptr, conv = ex->conv_weight[0] != nullptr;
+    // the convolutions (width 4 with SiLU) run inside the forward kernel only where nothing is kept for a backward, which
+    // would need the activations in memory
+    if (conv && (!shape->forward_only || ex->conv_width != 4)) return KDA_ERR_UNSUPPORTED;
+    if (shape->tokens > 0) {
+        if (!q || !k || !v || !g || !beta || (!o && !(norm && shape->forward_only))) return KDA_ERR_NULL;
+        if (norm && (!ex->norm_weight || !ex->y || (!ex->inv_rms && !shape->forward_only))) return KDA_ERR_NULL;
+        if (conv && (!ex->conv_weight[1] || !ex->conv_weight[2])) return KDA_ERR_NULL;
+    }
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0 || workspace_bytes < kda_chunk_workspace_bytes(shape))
+        return KDA_ERR_WORKSPACE;
+    const int64_t hk = (int64_t)shape->heads * shape->key_dim, gate_ld = ex->gate_ld ? ex->gate_ld : hk, x_ld = ex->x_ld ? ex->x_ld : hk;
+    if (norm && (gate_ld < hk || gate_ld % 8 != 0 ||
+                 (reinterpret_cast<uintptr_t>(ex->gate) | reinterpret_cast<uintptr_t>(ex->y) | reinterpret_cast<uintptr_t>(ex->norm_weight)) % 16 != 0))
+        return KDA_ERR_UNSUPPORTED;
+    if (conv && (x_ld < hk || x_ld % 8 != 0 ||
+                 (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                  reinterpret_cast<uintptr_t>(ex->conv_weight[0]) | reinterpret_cast<uintptr_t>(ex->conv_weight[1]) |
+                  reinterpret_cast<uintptr_t>(ex->conv_weight[2])) % 16 != 0))
+        return KDA_ERR_UNSUPPORTED;
+    tc::ConvPrep cp{{ex->conv_weight[0], ex->conv_weight[1], ex->conv_weight[2]}, ex->conv_weight_dtype == KDA_DTYPE_F32 ? 1 : 0, x_ld};
+    tc::NormEpilogue ep{static_cast<const __nv_bfloat16*>(ex->gate), ex->norm_weight, ex->eps, static_cast<__nv_bfloat16*>(ex->y), ex->inv_rms, gate_ld};
+    return simt_chunk_fwd(shape, q, k, v, g, beta, h0, cu_seqlens, o, final_state, workspace, (cudaStream_t)stream, norm ? &ep : nullptr,
+                          conv ? &cp : nullptr);
+}
+
 extern "C" int kda_chunk_fwd_conv(const KdaChunkShape* shape, const void* xq, const void* xk, const void* xv, const void* wq,
                                   const void* wk, const void* wv, int32_t conv_width, int32_t weight_dtype, const void* g,
                                   const void* beta, const float* h0, const int32_t* cu_seqlens, void* o, float* final_state,
                                   void* workspace, size_t workspace_bytes, void* stream) {
-    int rc = check_shape(shape, cu_seqlens);
-    if (rc) return rc;
-    // the convolution lives in the tensor-core lane's forward kernel, width 4 with SiLU, and only where nothing is kept for
-    // a backward (which would need the activations in memory)
-    if (shape->lane != KDA_LANE_TC || !shape->forward_only || conv_width != 4) return KDA_ERR_UNSUPPORTED;
-    if (shape->tokens > 0 && (!xq || !xk || !xv || !wq || !wk || !wv || !g || !beta || !o)) return KDA_ERR_NULL;
-    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0 || workspace_bytes < kda_chunk_workspace_bytes(shape))
-        return KDA_ERR_WORKSPACE;
-    if ((reinterpret_cast<uintptr_t>(xq) | reinterpret_cast<uintptr_t>(xk) | reinterpret_cast<uintptr_t>(xv) | reinterpret_cast<uintptr_t>(wq) |
-         reinterpret_cast<uintptr_t>(wk) | reinterpret_cast<uintptr_t>(wv)) % 16 != 0)
-        return KDA_ERR_UNSUPPORTED;
-    tc::ConvPrep cp{{wq, wk, wv}, weight_dtype == KDA_DTYPE_F32 ? 1 : 0};
-    return simt_chunk_fwd(shape, xq, xk, xv, g, beta, h0, cu_seqlens, o, final_state, workspace, (cudaStream_t)stream, nullptr, &cp);
+    if (shape && shape->tokens > 0 && !wq) return KDA_ERR_NULL;
+    KdaChunkExtras ex = {};
+    ex.conv_weight[0] = wq; ex.conv_weight[1] = wk; ex.conv_weight[2] = wv;
+    ex.conv_width = conv_width; ex.conv_weight_dtype = weight_dtype;
+    return kda_chunk_fwd_ex(shape, &ex, xq, xk, xv, g, beta, h0, cu_seqlens, o, final_state, workspace, workspace_bytes, stream);
 }
 
 extern "C" int kda_chunk_fwd_norm(const KdaChunkShape* shape, const void* q, const void* k, const void* v, const void* g,
                                   const void* beta, const float* h0, const int32_t* cu_seqlens, void* o, float* final_state,
                                   void* workspace, size_t workspace_bytes, const void* gate, const float* norm_weight, float eps,
                                   void* y, float* inv_rms, void* stream) {
-    int rc = check_shape(shape, cu_seqlens);
-    if (rc) return rc;
-    if (shape->lane != KDA_LANE_TC) return KDA_ERR_UNSUPPORTED;      // the epilogue lives in the tensor-core lane's output kernel
-    if (shape->tokens > 0 && (!q || !k || !v || !g || !beta || !o || !gate || !norm_weight || !y || !inv_rms)) return KDA_ERR_NULL;
-    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0 || workspace_bytes < kda_chunk_workspace_bytes(shape))
-        return KDA_ERR_WORKSPACE;
-    if ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(norm_weight)) % 16 != 0)
-        return KDA_ERR_UNSUPPORTED;
-    tc::NormEpilogue ep{static_cast<const __nv_bfloat16*>(gate), norm_weight, eps, static_cast<__nv_bfloat16*>(y), inv_rms};
-    return simt_chunk_fwd(shape, q, k, v, g, beta, h0, cu_seqlens, o, final_state, workspace, (cudaStream_t)stream, &ep);
+    if (shape && shape->tokens > 0 && (!gate || !o || !inv_rms)) return KDA_ERR_NULL;
+    KdaChunkExtras ex = {};
+    ex.gate = gate; ex.norm_weight = norm_weight; ex.eps = eps; ex.y = y; ex.inv_rms = inv_rms;
+    return kda_chunk_fwd_ex(shape, &ex, q, k, v, g, beta, h0, cu_seqlens, o, final_state, workspace, workspace_bytes, stream);
 }
 
 extern "C" int kda_chunk_bwd(const KdaChunkShape* shape, const void* q, const void* k, const void* v, const void* g,

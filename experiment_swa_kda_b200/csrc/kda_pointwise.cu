@@ -466,9 +466,8 @@ __global__ void __launch_bounds__(256) conv_step_kernel(int B, int C, int silu, 
     for (int j = 0; j < W; ++j) st_io(cache, idx * W + j, BF16, xx[j]);
 }
 
-// Forward without a carried-in window and without a final-state output (the training path).  Lane = channel pair, so
-// every global access of a warp is one contiguous 128-byte (bf16) row segment; each thread slides the window over 8
-// consecutive tokens with all of its loads issued up front.
+// Lane = channel pair or quad, so every global access of a warp is one contiguous row segment; each thread slides the
+// window over 8 consecutive tokens with all of its loads issued up front.
 template <bool BF16>
 __device__ __forceinline__ float2 ld_pair(const void* p, size_t i) {
     // read-only path: the inputs are never written by the kernel that reads them
@@ -549,7 +548,7 @@ __device__ __forceinline__ void st_cvec(void* p, size_t i, const float (&s)[VEC]
 // move as 8- / 16-byte accesses and the head's exp(A_log) is computed once per 4 elements.
 template <bool BF16>
 __global__ void __launch_bounds__(256) gate_fwd4_kernel(unsigned n4, unsigned n_beta, int H, int K, const void* __restrict__ raw,
-                                                        const void* __restrict__ bl, const float* __restrict__ A_log,
+                                                        const void* __restrict__ bl, int bl_ld, const float* __restrict__ A_log,
                                                         const float* __restrict__ dt_bias, float lb, float* __restrict__ g,
                                                         float* __restrict__ beta) {
     const unsigned hk4 = (unsigned)(H * K) >> 2;
@@ -567,13 +566,14 @@ __global__ void __launch_bounds__(256) gate_fwd4_kernel(unsigned n4, unsigned n_
         o.w = lb * sigmoidf_(ea * (r[3] + bias.w));
         *reinterpret_cast<float4*>(g + (size_t)i4 * 4) = o;
     }
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n_beta; i += stride) beta[i] = sigmoidf_(ld_io(bl, i, BF16));
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n_beta; i += stride)
+        beta[i] = sigmoidf_(ld_io(bl, (size_t)(i / (unsigned)H) * bl_ld + i % (unsigned)H, BF16));
 }
 
 // grid: x = blocks of 128 columns (lane = 4 channels), y = blocks of kGateRows tokens; warp w takes rows w, w + 8, ...
 template <bool BF16>
 __global__ void __launch_bounds__(256) gate_bwd4_kernel(int tokens, int H, int K, const void* __restrict__ raw,
-                                                        const void* __restrict__ bl, const float* __restrict__ A_log,
+                                                        const void* __restrict__ bl, int bl_ld, int bl_pad, const float* __restrict__ A_log,
                                                         const float* __restrict__ dt_bias, float lb, const float* __restrict__ dg,
                                                         const float* __restrict__ dbeta, void* __restrict__ d_raw,
                                                         void* __restrict__ d_bl, float* __restrict__ part_b,
@@ -633,11 +633,17 @@ __global__ void __launch_bounds__(256) gate_bwd4_kernel(int tokens, int H, int K
         part_a[o] = ta;
     }
     if (blockIdx.x == 0) {                  // beta logits of this block's rows
-        const int nb = min(kGateRows, tokens - t0) * H;
+        // rows bl_ld apart; columns H .. H + bl_pad - 1 of d_bl pad a wider matrix and are zeroed
+        const int wide = H + bl_pad, nb = min(kGateRows, tokens - t0) * wide;
         for (int i = threadIdx.x; i < nb; i += 256) {
-            const size_t o = (size_t)t0 * H + i;
-            const float b = sigmoidf_(ld_io(bl, o, BF16));
-            st_io(d_bl, o, BF16, dbeta[o] * b * (1.f - b));
+            const int t = t0 + i / wide, h = i % wide;
+            const size_t o = (size_t)t * bl_ld + h;
+            float d = 0.f;
+            if (h < H) {
+                const float b = sigmoidf_(ld_io(bl, o, BF16));
+                d = dbeta[(size_t)t * H + h] * b * (1.f - b);
+            }
+            st_io(d_bl, o, BF16, d);
         }
     }
 }
@@ -649,6 +655,8 @@ struct ConvFwdItems {
     const void* x[kConvItems];
     const void* w[kConvItems];
     void* y[kConvItems];
+    const void* cache[kConvItems];     // carried-in windows [B][C][W], or null: zeros before the first token
+    void* fin[kConvItems];             // carried-out windows [B][C][W], or null
 };
 struct ConvBwdItems {
     const void* x[kConvItems];
@@ -670,9 +678,13 @@ __device__ __forceinline__ T pick_item(T const (&a)[kConvItems], int i) {
     return r;
 }
 
-// grid: x = channel blocks of 32*VEC, y = blocks of 8 time groups x kConvPairT tokens, z = item * B + batch
-template <int W, int VEC, bool BF16>
-__global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C, int silu, int wf32, ConvFwdItems items) {
+// grid: x = channel blocks of 32*VEC, y = blocks of 8 time groups x kConvPairT tokens, z = item * B + batch.  x rows are
+// ldx elements apart (a slice of a wider projection), y rows are dense.  WIN: a window is carried in or out; only the
+// threads at either end of a sequence touch it.  The kernel moves 2 x B x T x C elements and is bound by instruction issue
+// at 0.62 of the copy rate (131 us at 65,536 x 2,048 bf16); the windows used to go through a 4-token, 8-channel kernel
+// whose lanes read 16-byte pieces of strided rows: 78 us at 8,191 x 2,048, now 17.
+template <int W, int VEC, bool BF16, bool WIN>
+__global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C, int ldx, int silu, int wf32, ConvFwdItems items) {
     const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int c = (blockIdx.x * 32 + p) * VEC;
     const int item = blockIdx.z / B;
@@ -696,18 +708,31 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
     float xin[kConvPairT + W - 1][VEC];
     if (t0 >= W - 1 && t0 + kConvPairT <= T) {
         // interior: plain address arithmetic, every load independent
-        const size_t base = (rowbase + t0 - (W - 1)) * C + cl;
+        const size_t base = (rowbase + t0 - (W - 1)) * ldx + cl;
 #pragma unroll
-        for (int j = 0; j < kConvPairT + W - 1; ++j) ld_cvec<VEC, BF16>(xin[j], x, base + (size_t)j * C);
+        for (int j = 0; j < kConvPairT + W - 1; ++j) ld_cvec<VEC, BF16>(xin[j], x, base + (size_t)j * ldx);
     } else {
 #pragma unroll
         for (int j = 0; j < kConvPairT + W - 1; ++j) {
             const int t = t0 - (W - 1) + j;
             const int tc = min(max(t, 0), T - 1);
-            ld_cvec<VEC, BF16>(xin[j], x, (rowbase + tc) * C + cl);
+            ld_cvec<VEC, BF16>(xin[j], x, (rowbase + tc) * ldx + cl);
             if (t < 0 || t >= T) {
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) xin[j][e] = 0.f;
+            }
+        }
+        if (WIN && t0 < W - 1) {
+            const void* cache = pick_item(items.cache, item);      // slot s holds the input at time s - W
+            if (cache != nullptr) {
+#pragma unroll
+                for (int j = 0; j < W - 1; ++j) {
+                    const int t = t0 - (W - 1) + j;
+                    if (t < 0) {
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) xin[j][e] = ld_io(cache, ((size_t)b * C + cl + e) * W + W + t, BF16);
+                    }
+                }
             }
         }
     }
@@ -722,6 +747,28 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
             out[e] = silu ? z * sigmoid_t<BF16>(z) : z;
         }
         if (t0 + tt < T && cok) st_cvec<VEC, BF16>(y, (rowbase + t0 + tt) * C + c, out);
+    }
+    if (WIN && cok && (t0 + kConvPairT > T - W || t0 == 0)) {
+        void* fin = pick_item(items.fin, item);                    // slot s holds the input at time T - W + s
+        if (fin != nullptr) {
+#pragma unroll
+            for (int tt = 0; tt < kConvPairT; ++tt) {
+                const int t = t0 + tt, s = t - (T - W);
+                if (t < T && s >= 0) {
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) st_io(fin, ((size_t)b * C + c + e) * W + s, BF16, xin[tt + W - 1][e]);
+                }
+            }
+            if (t0 == 0 && T < W) {                                // a sequence shorter than the window keeps what was carried in
+                const void* cache = pick_item(items.cache, item);
+                for (int s = 0; s < W - T; ++s)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) {
+                        const size_t row = ((size_t)b * C + c + e) * W;
+                        st_io(fin, row + s, BF16, cache != nullptr ? ld_io(cache, row + T + s, BF16) : 0.f);
+                    }
+            }
+        }
     }
 }
 
@@ -922,7 +969,7 @@ __global__ void __launch_bounds__(256) conv_bwd_kernel(int B, int T, int C, int 
 constexpr int kConvTileT = 64, kConvTileC = 64;
 
 template <int W, bool BF16>
-__global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C, int silu, int wf32, ConvBwdItems items,
+__global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C, int ldx, int silu, int wf32, ConvBwdItems items,
                                                             float* __restrict__ dw_part) {
     constexpr int XR = kConvTileT + 2 * (W - 1);   // x rows  t0-(W-1) .. t0+63+(W-1)
     constexpr int GR = kConvTileT + W - 1;         // dy rows t0 .. t0+63+(W-1)
@@ -956,31 +1003,31 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
     const size_t rowbase = (size_t)b * T;
     auto xload = [&](int tc) -> xpair_t {
         if constexpr (BF16) {
-            const unsigned u = __ldg(reinterpret_cast<const unsigned*>(reinterpret_cast<const __nv_bfloat16*>(x) + (rowbase + tc) * C + cl));
+            const unsigned u = __ldg(reinterpret_cast<const unsigned*>(reinterpret_cast<const __nv_bfloat16*>(x) + (rowbase + tc) * ldx + cl));
             return *reinterpret_cast<const __nv_bfloat162*>(&u);
         } else {
-            return __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(x) + (rowbase + tc) * C + cl));
+            return __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(x) + (rowbase + tc) * ldx + cl));
         }
     };
     auto xwide = [](const xpair_t& v) -> float2 {
         if constexpr (BF16) return __bfloat1622float2(v);
         else return v;
     };
-    if (t0 >= W - 1 && t0 + GR <= T && cb + kConvTileC <= C && (C & 3) == 0) {
+    if (t0 >= W - 1 && t0 + GR <= T && cb + kConvTileC <= C && (C & 3) == 0 && (ldx & 3) == 0) {
         // interior tile: no clamping, four channels per thread (sixteen threads cover a 64-channel row, a warp two rows),
         // addresses advance by a constant stride
         const int q = threadIdx.x & 15, rg = threadIdx.x >> 4;
-        const size_t e0 = (rowbase + t0 - (W - 1) + rg) * C + cb + 4 * q;       // x row rg of the tile, this thread's channels
-        const size_t step = (size_t)16 * C;
+        const size_t e0 = (rowbase + t0 - (W - 1) + rg) * ldx + cb + 4 * q;       // x row rg of the tile, this thread's channels
+        const size_t xstep = (size_t)16 * ldx, step = (size_t)16 * C;
 #pragma unroll
         for (int it = 0; it < (XR + 15) / 16; ++it) {
             const int r = rg + 16 * it;
             if (r < XR) {
                 if constexpr (BF16) {
-                    const uint2 u = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(x) + e0 + it * step));
+                    const uint2 u = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(x) + e0 + it * xstep));
                     *reinterpret_cast<uint2*>(&xs[r][2 * q]) = u;
                 } else {
-                    const float4 f = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + e0 + it * step));
+                    const float4 f = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + e0 + it * xstep));
                     *reinterpret_cast<float4*>(&xs[r][2 * q]) = f;
                 }
             }
@@ -1081,7 +1128,7 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
                 a0 += w0[m] * dw_[W - 1 - m].x;
                 a1 += w1[m] * dw_[W - 1 - m].y;
             }
-            if (t < T && cok) st_pair<BF16>(dx, (rowbase + t) * C + c, a0, a1);
+            if (t < T && cok) st_pair<BF16>(dx, (rowbase + t) * ldx + c, a0, a1);
 #pragma unroll
             for (int m = 0; m < W - 1; ++m) dw_[m] = dw_[m + 1];
         }
@@ -1107,7 +1154,7 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
 constexpr int kConvRingDepth = 16;
 
 template <int W>
-__global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int C, int run, int silu, int wf32, ConvBwdItems items,
+__global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int C, int ldx, int run, int silu, int wf32, ConvBwdItems items,
                                                                float* __restrict__ dw_part) {
     constexpr int D = kConvRingDepth;
     extern __shared__ __align__(16) uint8_t ring_raw[];
@@ -1149,10 +1196,10 @@ __global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int
         auto issue = [&](int j) {
             if (j < nr) {
                 const int tx = min(max(t0 - (W - 1) + j, 0), T - 1);
-                const size_t off = (rowbase + tx) * C + c;
+                const size_t row = rowbase + tx;
                 const uint32_t dst = slot0 + (uint32_t)((j % D) * 2) * 256u * 8u;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(x + off) : "memory");
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 256u * 8u), "l"(dy + off) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(x + row * ldx + c) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 256u * 8u), "l"(dy + row * C + c) : "memory");
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -1208,7 +1255,7 @@ __global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int
 #pragma unroll
                         for (int m = 0; m < W; ++m) a[e] += wv[m][e] * dzc[(u - m + W) % W][e];  // dz[tx - m]
                     }
-                    st_cvec<4, true>(dx, (rowbase + td) * C + c, a);
+                    st_cvec<4, true>(dx, (rowbase + td) * ldx + c, a);
                 }
             }
         }
@@ -1421,8 +1468,10 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd128_kernel(long long rows, flo
     }
 }
 
-template <bool BF16>
-__global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, const void* __restrict__ x,
+// ROWS: gate and dgate are the [token][head][128] part of wider rows gate_ld elements apart (a slice of the layer's
+// projection), heads rows to a token.
+template <bool BF16, bool ROWS>
+__global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, int heads, int gate_ld, const void* __restrict__ x,
                                                              const void* __restrict__ gate, const float* __restrict__ w,
                                                              const float* __restrict__ inv_rms, const void* __restrict__ dy,
                                                              void* __restrict__ dx, void* __restrict__ dgate,
@@ -1434,6 +1483,10 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, con
     const float4 ww = *reinterpret_cast<const float4*>(w + 4 * lane);
     const float wa[4] = {ww.x, ww.y, ww.z, ww.w};
     float dwa[4] = {0.f, 0.f, 0.f, 0.f};
+    auto gate_at = [&](long long row) {
+        const unsigned r = (unsigned)row, tok = r / (unsigned)heads;
+        return (size_t)tok * gate_ld + (r - tok * (unsigned)heads) * 128 + 4 * lane;
+    };
     for (long long row0 = warp0 * kRmsRows; row0 < rows; row0 += nwarp * kRmsRows) {
         float a[kRmsRows][4], gt[kRmsRows][4], gy[kRmsRows][4], inv[kRmsRows], dot[kRmsRows];
 #pragma unroll
@@ -1441,7 +1494,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, con
             const long long rr = min(row0 + r, rows - 1);
             const size_t base = (size_t)rr * 128 + 4 * lane;
             ld4<BF16>(a[r], x, base);
-            ld4<BF16>(gt[r], gate, base);
+            ld4<BF16>(gt[r], gate, ROWS ? gate_at(rr) : base);
             ld4<BF16>(gy[r], dy, base);
             inv[r] = inv_rms[rr];
         }
@@ -1474,7 +1527,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, con
                 }
                 const size_t base = (size_t)(row0 + r) * 128 + 4 * lane;
                 st4<BF16>(dx, base, ox);
-                st4<BF16>(dgate, base, og);
+                st4<BF16>(dgate, ROWS ? gate_at(row0 + r) : base, og);
             }
         }
     }
@@ -1511,6 +1564,42 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(int nblk, int N, const
 }
 
 
+// Casts to bf16 of several dense float32 (or bf16) arrays laid end to end: the projection weights of a layer gathered
+// into one matrix, so that the products on one input become one GEMM.  A null source writes zeros (padding rows).
+// Bound by the weights' bytes; one launch instead of one cast per weight (8 x 2.3 us at width 768).
+constexpr int kPackItems = 10;
+struct PackItems {
+    const void* src[kPackItems];
+    unsigned long long end8[kPackItems];      // running ends, in groups of 8 elements
+};
+template <bool F32>
+__global__ void __launch_bounds__(256) pack_bf16_kernel(unsigned long long total8, int n, PackItems items, __nv_bfloat16* __restrict__ dst) {
+    const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += step) {
+        unsigned long long begin = 0;
+        const void* src = items.src[0];
+#pragma unroll
+        for (int k = 1; k < kPackItems; ++k)
+            if (k < n && i >= items.end8[k - 1]) {
+                begin = items.end8[k - 1];
+                src = items.src[k];
+            }
+        uint4 u = make_uint4(0, 0, 0, 0);
+        if (src != nullptr) {
+            if (F32) {
+                const float4* p = reinterpret_cast<const float4*>(src) + 2 * (i - begin);
+                const float4 a = __ldg(p), b = __ldg(p + 1);
+                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+                h[0] = __floats2bfloat162_rn(a.x, a.y); h[1] = __floats2bfloat162_rn(a.z, a.w);
+                h[2] = __floats2bfloat162_rn(b.x, b.y); h[3] = __floats2bfloat162_rn(b.z, b.w);
+            } else {
+                u = __ldg(reinterpret_cast<const uint4*>(src) + (i - begin));
+            }
+        }
+        *reinterpret_cast<uint4*>(dst + 8 * i) = u;
+    }
+}
+
 }  // namespace pw
 }  // namespace kda
 
@@ -1519,10 +1608,32 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(int nblk, int N, const
 // =============================================================================================
 using namespace kda;
 
-extern "C" int kda_gate_fwd(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
-                            const void* beta_logits, const float* A_log, const float* dt_bias, float lower_bound,
+extern "C" int kda_pack_bf16(int32_t n_items, int32_t src_dtype, const void* const* src, const int64_t* elems, void* dst, void* stream) {
+    if (n_items < 1 || n_items > pw::kPackItems) return KDA_ERR_BAD_SHAPE;
+    if (!src || !elems || !dst) return KDA_ERR_NULL;
+    pw::PackItems it = {};
+    unsigned long long end = 0;
+    uintptr_t al = reinterpret_cast<uintptr_t>(dst);
+    for (int i = 0; i < n_items; ++i) {
+        if (elems[i] < 0 || elems[i] % 8 != 0) return KDA_ERR_UNSUPPORTED;
+        end += (unsigned long long)elems[i] / 8;
+        it.src[i] = src[i];
+        it.end8[i] = end;
+        al |= reinterpret_cast<uintptr_t>(src[i]);
+    }
+    if (al % 16 != 0) return KDA_ERR_UNSUPPORTED;
+    if (end == 0) return KDA_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int blocks = (int)std::min<unsigned long long>((end + 255) / 256, 148ULL * 8);
+    if (src_dtype == KDA_DTYPE_F32) KDA_LAUNCH("pack_bf16_kernel", st, pw::pack_bf16_kernel<true><<<blocks, 256, 0, st>>>(end, n_items, it, static_cast<__nv_bfloat16*>(dst)));
+    else KDA_LAUNCH("pack_bf16_kernel", st, pw::pack_bf16_kernel<false><<<blocks, 256, 0, st>>>(end, n_items, it, static_cast<__nv_bfloat16*>(dst)));
+    return launch_status();
+}
+
+extern "C" int kda_gate_fwd_rows(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
+                                 const void* beta_logits, int32_t bl_ld, const float* A_log, const float* dt_bias, float lower_bound,
                             float* g_out, float* beta_out, void* stream) {
-    if (tokens < 0 || heads <= 0 || key_dim <= 0) return KDA_ERR_BAD_SHAPE;
+    if (tokens < 0 || heads <= 0 || key_dim <= 0 || bl_ld < heads) return KDA_ERR_BAD_SHAPE;
     if (tokens == 0) return KDA_OK;
     if (!raw_gate || !beta_logits || !A_log || !dt_bias || !g_out || !beta_out) return KDA_ERR_NULL;
     const size_t n = (size_t)tokens * heads * key_dim;
@@ -1532,11 +1643,12 @@ extern "C" int kda_gate_fwd(int32_t tokens, int32_t heads, int32_t key_dim, int3
         const unsigned n4 = (unsigned)(n / 4), nb = (unsigned)((size_t)tokens * heads);
         const int blocks4 = (int)std::min<size_t>(((size_t)n4 + 255) / 256, 148 * 16);
         if (io_dtype == KDA_DTYPE_BF16)
-            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<true><<<blocks4, 256, 0, fst>>>(n4, nb, heads, key_dim, raw_gate, beta_logits, A_log, dt_bias, lower_bound, g_out, beta_out));
+            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<true><<<blocks4, 256, 0, fst>>>(n4, nb, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
         else
-            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<false><<<blocks4, 256, 0, fst>>>(n4, nb, heads, key_dim, raw_gate, beta_logits, A_log, dt_bias, lower_bound, g_out, beta_out));
+            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<false><<<blocks4, 256, 0, fst>>>(n4, nb, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
         return launch_status();
     }
+    if (bl_ld != heads) return KDA_ERR_UNSUPPORTED;      // strided beta logits: the vector path only
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
     KDA_LAUNCH("gate_fwd_kernel", (cudaStream_t)stream, pw::gate_fwd_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(n, (size_t)tokens * heads, heads, key_dim,
                                                                    io_dtype == KDA_DTYPE_BF16, raw_gate, beta_logits,
@@ -1544,16 +1656,22 @@ extern "C" int kda_gate_fwd(int32_t tokens, int32_t heads, int32_t key_dim, int3
     return launch_status();
 }
 
+extern "C" int kda_gate_fwd(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
+                            const void* beta_logits, const float* A_log, const float* dt_bias, float lower_bound,
+                            float* g_out, float* beta_out, void* stream) {
+    return kda_gate_fwd_rows(tokens, heads, key_dim, io_dtype, raw_gate, beta_logits, heads, A_log, dt_bias, lower_bound, g_out, beta_out, stream);
+}
+
 extern "C" size_t kda_gate_bwd_scratch_bytes(int32_t tokens, int32_t heads, int32_t key_dim) {
     const size_t nblk = (size_t)ceil_div(tokens > 0 ? tokens : 1, pw::kGateRows);
     return align_up(2 * nblk * heads * key_dim * sizeof(float), 256);
 }
 
-extern "C" int kda_gate_bwd(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
-                            const void* beta_logits, const float* A_log, const float* dt_bias, float lower_bound,
-                            const float* dg, const float* dbeta, void* d_raw_gate, void* d_beta_logits, float* dA_log,
-                            float* ddt_bias, void* scratch, size_t scratch_bytes, void* stream) {
-    if (tokens < 0 || heads <= 0 || key_dim <= 0) return KDA_ERR_BAD_SHAPE;
+extern "C" int kda_gate_bwd_rows(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
+                                 const void* beta_logits, int32_t bl_ld, int32_t bl_pad, const float* A_log, const float* dt_bias,
+                                 float lower_bound, const float* dg, const float* dbeta, void* d_raw_gate, void* d_beta_logits,
+                                 float* dA_log, float* ddt_bias, void* scratch, size_t scratch_bytes, void* stream) {
+    if (tokens < 0 || heads <= 0 || key_dim <= 0 || bl_pad < 0 || bl_ld < heads + bl_pad) return KDA_ERR_BAD_SHAPE;
     if (!A_log || !dt_bias || !dA_log || !ddt_bias) return KDA_ERR_NULL;
     if (tokens > 0 && (!raw_gate || !beta_logits || !dg || !dbeta || !d_raw_gate || !d_beta_logits)) return KDA_ERR_NULL;
     if (!scratch || scratch_bytes < kda_gate_bwd_scratch_bytes(tokens, heads, key_dim)) return KDA_ERR_WORKSPACE;
@@ -1566,15 +1684,25 @@ extern "C" int kda_gate_bwd(int32_t tokens, int32_t heads, int32_t key_dim, int3
     if (nblk > 0 && key_dim % 4 == 0 && al) {
         const dim3 grid(ceil_div(heads * key_dim, 128), nblk);
         if (io_dtype == KDA_DTYPE_BF16)
-            KDA_LAUNCH("gate_bwd_kernel", st, pw::gate_bwd4_kernel<true><<<grid, 256, 0, st>>>(tokens, heads, key_dim, raw_gate, beta_logits, A_log, dt_bias, lower_bound, dg, dbeta, d_raw_gate, d_beta_logits, part_b, part_a));
+            KDA_LAUNCH("gate_bwd_kernel", st, pw::gate_bwd4_kernel<true><<<grid, 256, 0, st>>>(tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, bl_pad, A_log, dt_bias, lower_bound, dg, dbeta, d_raw_gate, d_beta_logits, part_b, part_a));
         else
-            KDA_LAUNCH("gate_bwd_kernel", st, pw::gate_bwd4_kernel<false><<<grid, 256, 0, st>>>(tokens, heads, key_dim, raw_gate, beta_logits, A_log, dt_bias, lower_bound, dg, dbeta, d_raw_gate, d_beta_logits, part_b, part_a));
+            KDA_LAUNCH("gate_bwd_kernel", st, pw::gate_bwd4_kernel<false><<<grid, 256, 0, st>>>(tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, bl_pad, A_log, dt_bias, lower_bound, dg, dbeta, d_raw_gate, d_beta_logits, part_b, part_a));
+    } else if (nblk > 0 && bl_ld != heads) {
+        return KDA_ERR_UNSUPPORTED;      // strided beta logits: the vector path only
     } else if (nblk > 0)
         KDA_LAUNCH("gate_bwd_kernel", st, pw::gate_bwd_kernel<<<nblk, 256, 0, st>>>(tokens, heads, key_dim, io_dtype == KDA_DTYPE_BF16, raw_gate,
                                                   beta_logits, A_log, dt_bias, lower_bound, dg, dbeta, d_raw_gate,
                                                   d_beta_logits, part_b, part_a));
     KDA_LAUNCH("gate_bwd_reduce_kernel", st, pw::gate_bwd_reduce_kernel<<<heads, 1024, 0, st>>>(nblk, heads, key_dim, part_b, part_a, ddt_bias, dA_log));
     return launch_status();
+}
+
+extern "C" int kda_gate_bwd(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
+                            const void* beta_logits, const float* A_log, const float* dt_bias, float lower_bound,
+                            const float* dg, const float* dbeta, void* d_raw_gate, void* d_beta_logits, float* dA_log,
+                            float* ddt_bias, void* scratch, size_t scratch_bytes, void* stream) {
+    return kda_gate_bwd_rows(tokens, heads, key_dim, io_dtype, raw_gate, beta_logits, heads, 0, A_log, dt_bias, lower_bound, dg, dbeta,
+                             d_raw_gate, d_beta_logits, dA_log, ddt_bias, scratch, scratch_bytes, stream);
 }
 
 static int decode_launch(int n_seq, int heads, int key_dim, int value_dim, int bf16, int gbf16, int l2norm, float scale, const void* q,
@@ -1643,36 +1771,40 @@ extern "C" int kda_decode_steps(int32_t n_steps, int32_t n_seq, int32_t heads, i
 
 namespace {
 
-// training path (no carried-in window, no final state) for n same-shaped convolutions in one launch
+inline bool conv_grid_ok(int n, int B, int T) { return ceil_div(T, 8 * pw::kConvPairT) <= 65535 && (long long)B * n <= 65535; }
+
+// n same-shaped convolutions in one launch; x rows ldx elements apart
 template <int W>
-int conv_fwd_fast(int n, int B, int T, int C, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st) {
-    const int vec = C % 128 == 0 ? 4 : 2;         // channels per thread
-    const dim3 grid(ceil_div(C, 32 * vec), ceil_div(T, 8 * pw::kConvPairT), B * n);
-    if (vec == 4) {
-        if (bf16) KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, 4, true><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it));
-        else KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, 4, false><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it));
-    } else {
-        if (bf16) KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, 2, true><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it));
-        else KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, 2, false><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it));
-    }
+int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st) {
+    const bool vec4 = C % 128 == 0 && ldx % 4 == 0;         // channels per thread: 4 when a warp's 128 channels fill a row segment
+    const dim3 grid(ceil_div(C, vec4 ? 128 : 64), ceil_div(T, 8 * pw::kConvPairT), B * n);
+    bool win = false;
+    for (int i = 0; i < n; ++i) win = win || it.cache[i] != nullptr || it.fin[i] != nullptr;
+#define KDA_CONV_FWD(VEC, BF, WIN) \
+    KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, VEC, BF, WIN><<<grid, 256, 0, st>>>(B, T, C, ldx, silu, wf32, it))
+    if (vec4 && bf16) { if (win) KDA_CONV_FWD(4, true, true); else KDA_CONV_FWD(4, true, false); }
+    else if (vec4) { if (win) KDA_CONV_FWD(4, false, true); else KDA_CONV_FWD(4, false, false); }
+    else if (bf16) { if (win) KDA_CONV_FWD(2, true, true); else KDA_CONV_FWD(2, true, false); }
+    else { if (win) KDA_CONV_FWD(2, false, true); else KDA_CONV_FWD(2, false, false); }
+#undef KDA_CONV_FWD
     return launch_status();
 }
 
 template <int W>
-int conv_bwd_fast(int n, int B, int T, int C, int bf16, int wf32, int silu, const pw::ConvBwdItems& it, float* const* dwgt,
+int conv_bwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvBwdItems& it, float* const* dwgt,
                   float* part, cudaStream_t st) {
     dim3 grid(ceil_div(C, pw::kConvTileC), ceil_div(T, pw::kConvTileT), B * n);
     // tokens per thread run of the streaming kernel: long runs amortise the W-1 halo rows; below ~12 warps per SM at
     // 32-token runs the tile kernel (64 tokens x 64 channels per block, more and smaller blocks) is the faster one
     const long long warps64 = (long long)(C / 128) * ceil_div(T, 64) * B * n;
-    if (bf16 && C % 128 == 0 && warps64 >= 148LL * 12) {
+    if (bf16 && C % 128 == 0 && ldx % 4 == 0 && warps64 >= 148LL * 12) {
         const int run = warps64 >= 148LL * 48 ? 64 : 32;
         grid = dim3(C / 128, ceil_div(T, 8 * run), B * n);                  // never more partial rows than the tile kernel's
         const size_t ring_bytes = (size_t)pw::kConvRingDepth * 2 * 256 * 8;
         if (set_smem_limit(pw::conv_bwd_ring_kernel<W>, ring_bytes)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_ring_kernel<W><<<grid, 256, ring_bytes, st>>>(B, T, C, run, silu, wf32, it, part));
-    } else if (bf16) KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_tile_kernel<W, true><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it, part));
-    else KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_tile_kernel<W, false><<<grid, 256, 0, st>>>(B, T, C, silu, wf32, it, part));
+        KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_ring_kernel<W><<<grid, 256, ring_bytes, st>>>(B, T, C, ldx, run, silu, wf32, it, part));
+    } else if (bf16) KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_tile_kernel<W, true><<<grid, 256, 0, st>>>(B, T, C, ldx, silu, wf32, it, part));
+    else KDA_LAUNCH("conv_bwd_kernel", st, pw::conv_bwd_tile_kernel<W, false><<<grid, 256, 0, st>>>(B, T, C, ldx, silu, wf32, it, part));
     const int nblk = grid.y * B;                  // partial rows per item
     pw::ColumnSumItems outs = {};
     for (int i = 0; i < n; ++i) outs.out[i] = dwgt[i];
@@ -1683,21 +1815,16 @@ int conv_bwd_fast(int n, int B, int T, int C, int bf16, int wf32, int silu, cons
 template <int W>
 int conv_fwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x, const void* w, const void* cache, void* y,
                void* fin, cudaStream_t st) {
-    const int ntile = ceil_div(T, pw::kConvTT);
-    auto blocks = [&](int vec) { return (unsigned)(((size_t)B * ntile * (C / vec) + 255) / 256); };
     const bool al16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16) == 0;
-    if (!cache && !fin && C % 2 == 0 && al16) {
+    if (C % 2 == 0 && al16 && conv_grid_ok(1, B, T)) {
         pw::ConvFwdItems it = {};
-        it.x[0] = x; it.w[0] = w; it.y[0] = y;
-        return conv_fwd_fast<W>(1, B, T, C, bf16, wf32, silu, it, st);
+        it.x[0] = x; it.w[0] = w; it.y[0] = y; it.cache[0] = cache; it.fin[0] = fin;
+        return conv_fwd_fast<W>(1, B, T, C, C, bf16, wf32, silu, it, st);
     }
-    if (bf16) {
-        if (C % 8 == 0 && al16) KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_kernel<W, 8, true><<<blocks(8), 256, 0, st>>>(B, T, C, silu, wf32, x, w, cache, y, fin));
-        else KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_kernel<W, 1, true><<<blocks(1), 256, 0, st>>>(B, T, C, silu, wf32, x, w, cache, y, fin));
-    } else {
-        if (C % 4 == 0 && al16) KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_kernel<W, 4, false><<<blocks(4), 256, 0, st>>>(B, T, C, silu, wf32, x, w, cache, y, fin));
-        else KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_kernel<W, 1, false><<<blocks(1), 256, 0, st>>>(B, T, C, silu, wf32, x, w, cache, y, fin));
-    }
+    // odd channel counts, unaligned tensors, batches past a grid's y / z extent: one channel per thread
+    const unsigned blocks = (unsigned)(((size_t)B * ceil_div(T, pw::kConvTT) * C + 255) / 256);
+    if (bf16) KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_kernel<W, 1, true><<<blocks, 256, 0, st>>>(B, T, C, silu, wf32, x, w, cache, y, fin));
+    else KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_kernel<W, 1, false><<<blocks, 256, 0, st>>>(B, T, C, silu, wf32, x, w, cache, y, fin));
     return launch_status();
 }
 
@@ -1716,7 +1843,7 @@ int conv_bwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x,
         if (!cache && !dfin && !dcache && C % 2 == 0 && al16) {
             pw::ConvBwdItems it = {};
             it.x[0] = x; it.w[0] = w; it.dy[0] = dy; it.dx[0] = dx;
-            return conv_bwd_fast<W>(1, B, T, C, bf16, wf32, silu, it, &dwgt, part, st);
+            return conv_bwd_fast<W>(1, B, T, C, C, bf16, wf32, silu, it, &dwgt, part, st);
         }
     }
     // the vector path keeps W*VEC partials per thread in shared memory; wide windows use the scalar path
@@ -1801,9 +1928,9 @@ extern "C" int kda_conv_bwd(int32_t batch, int32_t seq_len, int32_t channels, in
 #undef CALL
 }
 
-// n same-shaped convolutions (the q, k and v branches of a layer) in one launch each way: training path only (no
-// carried-in window, no final state), width <= 4, even channel count, 16-byte aligned tensors; anything else returns
-// KDA_ERR_UNSUPPORTED and the caller issues the per-tensor calls.
+// n same-shaped convolutions (the q, k and v branches of a layer) in one launch each way: width <= 4, even channel count
+// and row stride, 16-byte aligned tensors; anything else returns KDA_ERR_UNSUPPORTED and the caller issues the per-tensor
+// calls.
 namespace {
 bool conv_multi_ok(int n, int channels, int width, const void* const* a, const void* const* b, const void* const* c) {
     if (n < 1 || n > pw::kConvItems || width > 4 || channels % 2 != 0) return false;
@@ -1815,26 +1942,36 @@ bool conv_multi_ok(int n, int channels, int width, const void* const* a, const v
 }
 }  // namespace
 
-extern "C" int kda_conv_fwd_multi(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width,
-                                  int32_t io_dtype, int32_t silu, const void* const* x, const void* const* weight,
-                                  void* const* y, void* stream) {
-    if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0) return KDA_ERR_BAD_SHAPE;
+extern "C" int kda_conv_fwd_rows(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width, int32_t io_dtype,
+                                 int32_t silu, const void* const* x, int32_t x_ld, const void* const* weight, const void* const* cache,
+                                 void* const* y, void* const* final_state, void* stream) {
+    if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0 || x_ld < channels) return KDA_ERR_BAD_SHAPE;
     if (!x || !weight || !y) return KDA_ERR_NULL;
-    if (!conv_multi_ok(n_items, channels, width, x, const_cast<const void* const*>(y), nullptr)) return KDA_ERR_UNSUPPORTED;
+    if (x_ld % 2 != 0 || !conv_grid_ok(n_items, batch, seq_len) ||
+        !conv_multi_ok(n_items, channels, width, x, const_cast<const void* const*>(y), nullptr))
+        return KDA_ERR_UNSUPPORTED;
     const int wf32 = (io_dtype & KDA_WEIGHT_F32) != 0;
     const int bf16 = (io_dtype & 0xff) == KDA_DTYPE_BF16;
     pw::ConvFwdItems it = {};
     for (int i = 0; i < n_items; ++i) {
         if (!weight[i]) return KDA_ERR_NULL;
         it.x[i] = x[i]; it.w[i] = weight[i]; it.y[i] = y[i];
+        it.cache[i] = cache ? cache[i] : nullptr;
+        it.fin[i] = final_state ? final_state[i] : nullptr;
     }
     cudaStream_t st = (cudaStream_t)stream;
     switch (width) {
-        case 1: return conv_fwd_fast<1>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, st);
-        case 2: return conv_fwd_fast<2>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, st);
-        case 3: return conv_fwd_fast<3>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, st);
-        default: return conv_fwd_fast<4>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, st);
+        case 1: return conv_fwd_fast<1>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
+        case 2: return conv_fwd_fast<2>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
+        case 3: return conv_fwd_fast<3>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
+        default: return conv_fwd_fast<4>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
     }
+}
+
+extern "C" int kda_conv_fwd_multi(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width,
+                                  int32_t io_dtype, int32_t silu, const void* const* x, const void* const* weight,
+                                  void* const* y, void* stream) {
+    return kda_conv_fwd_rows(n_items, batch, seq_len, channels, width, io_dtype, silu, x, channels, weight, nullptr, y, nullptr, stream);
 }
 
 extern "C" int kda_conv_step_multi(int32_t n_items, int32_t batch, int32_t channels, int32_t width, int32_t io_dtype, int32_t silu,
@@ -1870,13 +2007,13 @@ extern "C" size_t kda_conv_bwd_multi_scratch_bytes(int32_t n_items, int32_t batc
     return (size_t)(n_items > 0 ? n_items : 1) * kda_conv_bwd_scratch_bytes(batch, seq_len, channels, width);
 }
 
-extern "C" int kda_conv_bwd_multi(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width,
-                                  int32_t io_dtype, int32_t silu, const void* const* x, const void* const* weight,
-                                  const void* const* d_y, void* const* dx, float* const* dweight, void* scratch,
-                                  size_t scratch_bytes, void* stream) {
-    if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0) return KDA_ERR_BAD_SHAPE;
+extern "C" int kda_conv_bwd_rows(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width,
+                                 int32_t io_dtype, int32_t silu, const void* const* x, int32_t x_ld, const void* const* weight,
+                                 const void* const* d_y, void* const* dx, float* const* dweight, void* scratch,
+                                 size_t scratch_bytes, void* stream) {
+    if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0 || x_ld < channels) return KDA_ERR_BAD_SHAPE;
     if (!x || !weight || !d_y || !dx || !dweight) return KDA_ERR_NULL;
-    if (!conv_multi_ok(n_items, channels, width, x, d_y, const_cast<const void* const*>(dx))) return KDA_ERR_UNSUPPORTED;
+    if (x_ld % 2 != 0 || !conv_grid_ok(n_items, batch, seq_len) || !conv_multi_ok(n_items, channels, width, x, d_y, const_cast<const void* const*>(dx))) return KDA_ERR_UNSUPPORTED;
     if (!scratch || scratch_bytes < kda_conv_bwd_multi_scratch_bytes(n_items, batch, seq_len, channels, width)) return KDA_ERR_WORKSPACE;
     const int wf32 = (io_dtype & KDA_WEIGHT_F32) != 0;
     const int bf16 = (io_dtype & 0xff) == KDA_DTYPE_BF16;
@@ -1888,11 +2025,19 @@ extern "C" int kda_conv_bwd_multi(int32_t n_items, int32_t batch, int32_t seq_le
     cudaStream_t st = (cudaStream_t)stream;
     float* part = static_cast<float*>(scratch);
     switch (width) {
-        case 1: return conv_bwd_fast<1>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, dweight, part, st);
-        case 2: return conv_bwd_fast<2>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, dweight, part, st);
-        case 3: return conv_bwd_fast<3>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, dweight, part, st);
-        default: return conv_bwd_fast<4>(n_items, batch, seq_len, channels, bf16, wf32, silu, it, dweight, part, st);
+        case 1: return conv_bwd_fast<1>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, dweight, part, st);
+        case 2: return conv_bwd_fast<2>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, dweight, part, st);
+        case 3: return conv_bwd_fast<3>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, dweight, part, st);
+        default: return conv_bwd_fast<4>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, dweight, part, st);
     }
+}
+
+extern "C" int kda_conv_bwd_multi(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width,
+                                  int32_t io_dtype, int32_t silu, const void* const* x, const void* const* weight,
+                                  const void* const* d_y, void* const* dx, float* const* dweight, void* scratch,
+                                  size_t scratch_bytes, void* stream) {
+    return kda_conv_bwd_rows(n_items, batch, seq_len, channels, width, io_dtype, silu, x, channels, weight, d_y, dx, dweight, scratch,
+                             scratch_bytes, stream);
 }
 
 namespace {
@@ -1944,8 +2089,8 @@ extern "C" int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype,
                      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(d_y) |
                        reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate) | reinterpret_cast<uintptr_t>(weight)) % 16) == 0;
     if (nb > 0 && vec && dim == 128) {
-        if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<true><<<nb, 256, 0, st>>>(rows, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-        else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false><<<nb, 256, 0, st>>>(rows, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+        if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<true, false><<<nb, 256, 0, st>>>(rows, 1, 128, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+        else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false, false><<<nb, 256, 0, st>>>(rows, 1, 128, x, gate, weight, inv_rms, d_y, dx, dgate, part));
     } else if (nb > 0) {
         if (io_dtype == KDA_DTYPE_BF16) {
             if (vec) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<true, true><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
@@ -1958,6 +2103,26 @@ extern "C" int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype,
     pw::ColumnSumItems outs = {};
     outs.out[0] = dweight;
     KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(dim, 32), 1024, 0, st>>>(nb, dim, part, outs));
+    return launch_status();
+}
+
+extern "C" int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t heads, int32_t gate_ld, const void* x, const void* gate,
+                                         const float* weight, const float* inv_rms, const void* d_y, void* dx, void* dgate,
+                                         float* dweight, void* scratch, size_t scratch_bytes, void* stream) {
+    if (rows <= 0 || rows >= (1LL << 31) || heads <= 0 || rows % heads != 0 || gate_ld < heads * 128) return KDA_ERR_BAD_SHAPE;
+    if (!x || !gate || !weight || !inv_rms || !d_y || !dx || !dgate || !dweight) return KDA_ERR_NULL;
+    if (!scratch || scratch_bytes < kda_rmsnorm_gate_bwd_scratch_bytes(rows, 128)) return KDA_ERR_WORKSPACE;
+    if (gate_ld % 8 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(d_y) |
+                              reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate) | reinterpret_cast<uintptr_t>(weight)) % 16) != 0)
+        return KDA_ERR_UNSUPPORTED;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int nb = rms_blocks(rows);
+    float* part = static_cast<float*>(scratch);
+    if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<true, true><<<nb, 256, 0, st>>>(rows, heads, gate_ld, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+    else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false, true><<<nb, 256, 0, st>>>(rows, heads, gate_ld, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+    pw::ColumnSumItems outs = {};
+    outs.out[0] = dweight;
+    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<4, 1024, 0, st>>>(nb, 128, part, outs));
     return launch_status();
 }
 

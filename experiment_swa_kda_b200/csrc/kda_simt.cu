@@ -970,7 +970,7 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
             int rc = tc_intra_forward(w, t, q, k, v, g, beta, gbf16, sh->l2norm, sh->scale, sh->tokens, conv, st);
             if (rc) return rc;
             rc = tc_scan_forward(w, t, sh->n_seq, sh->tokens, h0, final_state, o,
-                                 norm != nullptr ? *norm : tc::NormEpilogue{nullptr, nullptr, 0.f, nullptr, nullptr}, st);
+                                 norm != nullptr ? *norm : tc::NormEpilogue{nullptr, nullptr, 0.f, nullptr, nullptr, 0}, st);
             if (rc) return rc;
         }
         return launch_status();

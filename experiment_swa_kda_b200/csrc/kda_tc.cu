@@ -30,11 +30,12 @@ static EncodeFn encode_fn() {
 }
 
 // 2-D bf16 row-major tensor [rows][cols]; box = box_cols x box_rows; 128-byte swizzle (box_cols must be 64).
-int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows) {
+// Rows are `ld` elements apart (a multiple of 8).
+int make_map_bf16_ld(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_cols, uint32_t box_rows) {
     EncodeFn enc = encode_fn();
     if (!enc) return KDA_ERR_CUDA;
     cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * 2};
+    cuuint64_t strides[1] = {ld * 2};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t es[2] = {1, 1};
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
@@ -53,6 +54,10 @@ int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
         fprintf(stderr, "libkda_b200: cuTensorMapEncodeTiled failed (%d): ptr %p rows %llu cols %llu box %u x %u\n", (int)r, ptr,
                 (unsigned long long)rows, (unsigned long long)cols, box_cols, box_rows);
     return r == CUDA_SUCCESS ? KDA_OK : KDA_ERR_CUDA;
+}
+
+int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows) {
+    return make_map_bf16_ld(m, ptr, rows, cols, cols, box_cols, box_rows);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kNT, 2)
             for (int jj = 0; jj < 7; ++jj) {
                 const int i = 4 * rq - 3 + jj;
                 const long long ic = min(i, len - 1);      // rows past the tail feed masked outputs only
-                xr[jj] = (i >= 0 || !first) ? __ldg(reinterpret_cast<const uint4*>(x + (long long)base + ic * (long long)rstride))
+                xr[jj] = (i >= 0 || !first) ? __ldg(reinterpret_cast<const uint4*>(x + ((long long)tok0 + ic) * p.conv.x_ld + h * 128 + 8 * cg))
                                             : make_uint4(0, 0, 0, 0);
             }
         };
@@ -792,7 +792,7 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
     a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
     a.g = g; a.beta = beta; a.gbf16 = gbf16; a.l2norm = l2norm; a.H = w.H; a.scale = scale; a.t = t; a.w = w;
     a.xv = static_cast<const __nv_bfloat16*>(v);
-    a.conv = conv != nullptr ? *conv : tc::ConvPrep{{nullptr, nullptr, nullptr}, 0};
+    a.conv = conv != nullptr ? *conv : tc::ConvPrep{{nullptr, nullptr, nullptr}, 0, 0};
     if (conv != nullptr && !t.fwd_only) return KDA_ERR_UNSUPPORTED;      // a backward would need q, k, v in memory
     const uint64_t nch = (uint64_t)w.nslots * w.H;
     CUtensorMap mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp;

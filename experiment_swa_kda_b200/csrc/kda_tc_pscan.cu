@@ -22,6 +22,7 @@
 namespace kda {
 namespace tc {
 
+int make_map_bf16_ld(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_cols, uint32_t box_rows);
 int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
 
 // ---------------------------------------------------------------------------------------------
@@ -561,7 +562,7 @@ struct ChunkOutArgs {
     const int* chunk_tok0;
     const int* chunk_len;
     __nv_bfloat16* ZT;
-    __nv_bfloat16* o;          // [tokens][H][128]
+    __nv_bfloat16* o;          // [tokens][H][128]; nullptr with the norm's epilogue when only y is wanted
     int H;
     int* status;
     NormEpilogue norm;
@@ -707,7 +708,7 @@ __global__ void __launch_bounds__(256, 2)
             for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
             if (i < len) {
                 const float inv = rsqrtf(ss * (1.0f / 128.0f) + p.norm.eps);
-                if (lane == 0) p.norm.inv_rms[row] = inv;
+                if (lane == 0 && p.norm.inv_rms != nullptr) p.norm.inv_rms[row] = inv;
                 float out[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -715,7 +716,7 @@ __global__ void __launch_bounds__(256, 2)
                     asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(0.5f * gt[e]));
                     out[e] = a[e] * inv * wa[e] * fmaf(0.5f, th, 0.5f);
                 }
-                *reinterpret_cast<uint2*>(p.o + row * 128 + 4 * lane) = ou;
+                if (p.o != nullptr) *reinterpret_cast<uint2*>(p.o + row * 128 + 4 * lane) = ou;
                 *reinterpret_cast<uint2*>(p.norm.y + row * 128 + 4 * lane) =
                     make_uint2(pack_bf16(out[0], out[1]), pack_bf16(out[2], out[3]));
             }
@@ -870,7 +871,7 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
     rc |= make_map_bf16(&mP, t.Pn, nch * 128, 128, 64, 128);
     rc |= make_map_bf16(&mZT, t.fwd_only ? t.UT : t.ZT, nch * 128, 64, 64, 128);      // not stored in a forward-only call
     const bool fused_norm = norm.gate != nullptr;
-    if (fused_norm) rc |= make_map_bf16(&mG, norm.gate, (uint64_t)tokens, (uint64_t)w.H * 128, 64, 64);
+    if (fused_norm) rc |= make_map_bf16_ld(&mG, norm.gate, (uint64_t)tokens, (uint64_t)w.H * 128, (uint64_t)norm.gate_ld, 64, 64);
     else mG = mAT;
     if (rc) return KDA_ERR_CUDA;
     const int out_smem = fused_norm ? kChunkOutNormSmem : kChunkOutSmem;

@@ -13,6 +13,7 @@ namespace tc {
 struct ConvPrep {
     const void* w[3];       // weights of the q, k, v convolutions, [H*128][4]
     int wf32;               // 1: float32 weights (rounded to bf16 as loaded, like the stand-alone kernel), 0: bf16
+    long long x_ld;         // elements between consecutive tokens of the convolutions' inputs
 };
 
 struct TcWs {
@@ -39,13 +40,14 @@ struct TcWs {
 
 // Optional epilogue of the chunk-output kernel: the gated RMSNorm that follows the operator in the layer
 // (y = o * rsqrt(mean(o^2) + eps) * weight * sigmoid(gate) over the 128 values of a token and head), applied to the
-// output tile while it is still on chip.  o is written as well: the norm's backward needs it.
+// output tile while it is still on chip.  o is written as well when the caller passes it: the norm's backward needs it.
 struct NormEpilogue {
-    const __nv_bfloat16* gate;   // [tokens][H][128], or nullptr: no epilogue
+    const __nv_bfloat16* gate;   // [tokens][H][128] in rows gate_ld elements apart, or nullptr: no epilogue
     const float* weight;         // [128]
     float eps;
     __nv_bfloat16* y;            // [tokens][H][128]
-    float* inv_rms;              // [tokens][H]
+    float* inv_rms;              // [tokens][H], or nullptr: not wanted (no backward follows)
+    long long gate_ld;
 };
 
 // Scans are split when a batch has so few (sequence, head) recurrences that most SMs would idle behind them, and the

@@ -375,7 +375,9 @@ class KimiDeltaAttention(nn.Module):
             raise ValueError("conv_size must be positive")
         self.hidden_size, self.num_heads, self.head_dim = hidden_size, num_heads, head_dim
         self.conv_size, self.layer_idx, self.mode = conv_size, layer_idx, mode
-        self.fuse_prefill_conv = False      # see forward(): convolutions inside the intra-chunk kernel for no-grad prefill
+        # opt-in no-grad prefill with the three convolutions inside the intra-chunk kernel, so that q, k, v are never written
+        # to memory; identical results, slower (that kernel is bound by instruction issue, the convolution by bandwidth)
+        self.fuse_prefill_conv = False
         self.lower_bound, self.allow_fallback = lower_bound, allow_fallback
         self.q_proj = Linear(hidden_size, hidden_size, bias=False)
         self.k_proj = Linear(hidden_size, hidden_size, bias=False)
@@ -398,19 +400,19 @@ class KimiDeltaAttention(nn.Module):
             raise ValueError(f"hidden_states must have shape [B,T,{self.hidden_size}]")
         batch, length, _ = hidden_states.shape
         requested_mode = self.mode if mode is None else mode
-        want_state = output_final_state
+        want_state = bool(output_final_state)
+        if requested_mode == "project_chunk" and hidden_states.is_cuda and self.head_dim == 128 and type(hidden_states) is Tensor:
+            weights = self._plain_weights()
+            if weights is not None:
+                incoming = () if state is None else (state.memory, state.q_conv, state.k_conv, state.v_conv)
+                out = _native.load().layer(hidden_states, weights, self.num_heads, self.o_norm.eps, self.lower_bound, incoming, want_state,
+                                           self.fuse_prefill_conv)
+                if out is not None:
+                    return out[0], (KDAState(*out[1:]) if want_state else None)
         q_state = None if state is None else state.q_conv
         k_state = None if state is None else state.k_conv
         v_state = None if state is None else state.v_conv
         memory = None if state is None else state.memory
-        if (self.fuse_prefill_conv and state is None and length > 0 and requested_mode == "project_chunk"
-                and not torch.is_grad_enabled() and hidden_states.is_cuda and hidden_states.dtype == torch.bfloat16
-                and self.head_dim == 128 and self.conv_size == 4):
-            # opt-in no-grad prefill at the tensor-core lane's shape: the three convolutions run inside the intra-chunk
-            # kernel, so q, k, v are never written to memory (3 x T x hidden_size x 2 bytes less per layer); identical
-            # results.  Measured 3 % slower than the separate convolution launch (the intra-chunk kernel is bound by
-            # instruction issue, the convolution by bandwidth), hence off by default.
-            return self._prefill_fused(hidden_states, want_state)
         if state is None and not want_state and length > 0:
             # training path: the three branches share one launch each way
             q, k, v = short_convolutions((self.q_conv1d, self.k_conv1d, self.v_conv1d),
@@ -442,28 +444,24 @@ class KimiDeltaAttention(nn.Module):
         final_state = KDAState(final_memory, q_final, k_final, v_final) if want_state else None
         return output, final_state
 
-    def _prefill_fused(self, hidden_states: Tensor, want_state: bool):
-        batch, length, _ = hidden_states.shape
-        shape4 = (batch, length, self.num_heads, self.head_dim)
-        xq, xk, xv = self.q_proj(hidden_states), self.k_proj(hidden_states), self.v_proj(hidden_states)
-        raw_gate = self.f_b_proj(self.f_a_proj(hidden_states)).reshape(shape4)
-        beta_logits = self.b_proj(hidden_states)
-        g, beta = ops.GateFunction.apply(raw_gate, beta_logits, self.A_log, self.dt_bias, float(self.lower_bound))
-        conv_w = [c.weight.squeeze(1) for c in (self.q_conv1d, self.k_conv1d, self.v_conv1d)]
-        mixed, memory = ops.chunk_kda_conv_fwd(xq.reshape(shape4), xk.reshape(shape4), xv.reshape(shape4), *conv_w, g, beta, None, None,
-                                               self.head_dim ** -0.5, True, want_state)
-        mixed = self.o_norm(mixed, self.g_proj(hidden_states).reshape(shape4))
-        output = self.o_proj(mixed.reshape(batch, length, self.hidden_size))
-        if not want_state:
-            return output, None
+    _PLAIN = (tuple((n, Linear) for n in ("q_proj", "k_proj", "v_proj", "g_proj", "f_a_proj", "b_proj", "f_b_proj", "o_proj"))
+              + tuple((n, ShortConvolution) for n in ("q_conv1d", "k_conv1d", "v_conv1d")) + (("o_norm", RMSNormGated),))
 
-        def cache(x):      # [B, C, W]: the last W inputs, the current token included, zero-padded on the left
-            tail = x[:, max(0, length - self.conv_size):, :]
-            if length < self.conv_size:
-                tail = torch.nn.functional.pad(tail, (0, 0, self.conv_size - length, 0))
-            return tail.transpose(1, 2).contiguous()
-
-        return output, KDAState(memory, cache(xq), cache(xk), cache(xv))
+    def _plain_weights(self):
+        """The layer's parameters in the native path's order, or None when a submodule is not the plain one this class built
+        (replaced, hooked, parametrised, given a bias): such a layer runs its modules one by one."""
+        mods, weights = self._modules, []
+        if torch.nn.modules.module._has_any_global_hook():
+            return None
+        for name, cls in self._PLAIN:
+            m = mods[name]
+            if (type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                    or "forward" in m.__dict__ or m._parameters.get("bias") is not None):
+                return None
+            weights.append(m._parameters.get("weight"))
+        own = self._parameters
+        weights[-1:] = (own.get("A_log"), own.get("dt_bias"), weights[-1])
+        return weights if all(type(w) in (nn.Parameter, Tensor) for w in weights) else None
 
     @torch.no_grad()
     def decode_token(self, hidden_states: Tensor, state: KDAState) -> Tensor:

@@ -10,25 +10,14 @@
 // Every entry checks that its inputs are the plain valid case and otherwise returns None without having done anything;
 // kda.py then runs its Python checks, which name the mistake.  Results, error texts and defaults are kda.py's.
 
-#include <torch/csrc/autograd/function.h>
-#include <torch/csrc/autograd/functions/utils.h>
-#include <torch/csrc/autograd/saved_variable.h>
-#include <torch/csrc/autograd/variable.h>
 #include <torch/extension.h>
 
 #include <atomic>
-#include <mutex>
 #include <tuple>
-#include <vector>
 
-#include "host_common.h"
+#include "host_node.h"
 
 namespace kda_host {
-
-namespace py = pybind11;
-using torch::autograd::Node;
-using torch::autograd::SavedVariable;
-using torch::autograd::variable_list;
 
 // ------------------------------------------------------------------------------------------------ device status
 namespace {
@@ -61,32 +50,6 @@ void watch_status(int device) {
 }
 
 namespace {
-
-// ------------------------------------------------------------------------------------------------ helpers
-bool is_io(const Tensor& t) { return t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kFloat; }
-int dt(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? KDA_DTYPE_BF16 : KDA_DTYPE_F32; }
-int wflag(const Tensor& x, const Tensor& w) {
-    return (w.scalar_type() == at::kFloat && x.scalar_type() != at::kFloat) ? KDA_WEIGHT_F32 : 0;
-}
-bool on(const Tensor& t, const Tensor& like) { return t.is_cuda() && t.device() == like.device(); }
-Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
-Tensor dense_as(const Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? dense(t) : t.to(type).contiguous(); }
-
-// A backward node: saved inputs, released with the graph.  Derived classes hold their sizes as plain fields.
-struct HostNode : public Node {
-    std::vector<SavedVariable> saved;
-    void keep(const Tensor& t) { saved.emplace_back(t, false); }
-    Tensor get(size_t i) { return saved[i].unpack(); }
-    void release_variables() override {
-        std::lock_guard<std::mutex> lk(mutex_);
-        for (auto& s : saved) s.reset_data();
-    }
-};
-
-template <class N>
-std::shared_ptr<N> make_node() {
-    return std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
-}
 
 // ------------------------------------------------------------------------------------------------ chunked operator
 struct Dims {
@@ -659,6 +622,10 @@ OptTensor rmsnorm(const Tensor& x_, const Tensor& gate_, const Tensor& w_, doubl
 }  // namespace
 }  // namespace kda_host
 
+namespace kda_host {
+void bind_layer(pybind11::module_& m);      // kda_layer.cpp
+}
+
 PYBIND11_MODULE(libkda_b200_torch, m) {
     namespace py = pybind11;
     using namespace kda_host;
@@ -672,4 +639,5 @@ PYBIND11_MODULE(libkda_b200_torch, m) {
     m.def("conv", &conv, nogil());
     m.def("conv_multi", &conv_multi, nogil());
     m.def("rmsnorm", &rmsnorm, nogil());
+    bind_layer(m);
 }

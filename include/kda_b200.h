@@ -108,6 +108,26 @@ int kda_chunk_fwd_norm(const KdaChunkShape* shape, const void* q, const void* k,
                        void* workspace, size_t workspace_bytes, const void* gate, const float* norm_weight, float eps,
                        void* y, float* inv_rms, void* stream);
 
+/* The forward with either or both of the fusions above and strided neighbours, for a caller whose layer keeps its
+ * projections side by side in one matrix: gate rows gate_ld elements apart, the convolutions' inputs (q, k, v of the call)
+ * x_ld elements apart; 0 means dense.  A forward_only call with the norm may leave out `o` and `inv_rms`.  Unused parts
+ * are zero / NULL.  Tensor-core lane only. */
+typedef struct KdaChunkExtras {
+    const void* gate;           /* norm epilogue: gate [tokens,H,V], or NULL */
+    int64_t gate_ld;
+    const float* norm_weight;
+    float eps;
+    void* y;
+    float* inv_rms;
+    const void* conv_weight[3]; /* convolution prologue: weights [H*128,4] of q, k, v, or NULL */
+    int32_t conv_width;
+    int32_t conv_weight_dtype;
+    int64_t x_ld;
+} KdaChunkExtras;
+int kda_chunk_fwd_ex(const KdaChunkShape* shape, const KdaChunkExtras* extras, const void* q, const void* k, const void* v, const void* g,
+                     const void* beta, const float* h0, const int32_t* cu_seqlens, void* o, float* final_state,
+                     void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- chunked KDA, backward ------------------------------------------------
  * Stands in for nanochat_kda::chunk_backward (reference chunk.cu:1758-2113,
  * chunk_wy_backward.cu:3991-4323).  `workspace` is the buffer the matching
@@ -159,6 +179,22 @@ int kda_gate_bwd(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtyp
                  const void* beta_logits, const float* A_log, const float* dt_bias, float lower_bound, const float* dg,
                  const float* dbeta, void* d_raw_gate, void* d_beta_logits, float* dA_log, float* ddt_bias,
                  void* scratch, size_t scratch_bytes, void* stream);
+
+/* The same with beta logits (and their gradient) in rows bl_ld elements apart; columns H .. H + bl_pad - 1 of a gradient
+ * row are written as zeros.  bl_ld != H needs key_dim % 4 == 0 and 16-byte aligned tensors, else KDA_ERR_UNSUPPORTED. */
+int kda_gate_fwd_rows(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
+                      const void* beta_logits, int32_t bl_ld, const float* A_log, const float* dt_bias, float lower_bound,
+                      float* g_out, float* beta_out, void* stream);
+int kda_gate_bwd_rows(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
+                      const void* beta_logits, int32_t bl_ld, int32_t bl_pad, const float* A_log, const float* dt_bias,
+                      float lower_bound, const float* dg, const float* dbeta, void* d_raw_gate, void* d_beta_logits,
+                      float* dA_log, float* ddt_bias, void* scratch, size_t scratch_bytes, void* stream);
+
+/* ---- weights of one input gathered into one bf16 matrix -------------------------
+ * dst = the n_items (1..10) dense arrays src[i] of elems[i] elements (float32 or bf16; multiples of 8, 16-byte aligned)
+ * rounded to bf16 and laid end to end; a NULL source writes zeros.  src, elems: HOST arrays.  No reference counterpart
+ * (the reference casts every Linear weight by itself). */
+int kda_pack_bf16(int32_t n_items, int32_t src_dtype, const void* const* src, const int64_t* elems, void* dst, void* stream);
 
 /* ---- recurrent decode step --------------------------------------------------
  * One token per sequence on activated inputs: reads state_in, writes state_out
@@ -225,6 +261,16 @@ int kda_conv_bwd_multi(int32_t n_items, int32_t batch, int32_t seq_len, int32_t 
                        int32_t silu, const void* const* x, const void* const* weight, const void* const* d_y,
                        void* const* dx, float* const* dweight, void* scratch, size_t scratch_bytes, void* stream);
 
+/* The batched convolutions with x (and dx) in rows x_ld elements apart (even; y and d_y are dense) and, forward only,
+ * carried-in / carried-out windows (HOST arrays with NULL entries, or NULL). */
+int kda_conv_fwd_rows(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width, int32_t io_dtype,
+                      int32_t silu, const void* const* x, int32_t x_ld, const void* const* weight, const void* const* cache,
+                      void* const* y, void* const* final_state, void* stream);
+int kda_conv_bwd_rows(int32_t n_items, int32_t batch, int32_t seq_len, int32_t channels, int32_t width,
+                      int32_t io_dtype, int32_t silu, const void* const* x, int32_t x_ld, const void* const* weight,
+                      const void* const* d_y, void* const* dx, float* const* dweight, void* scratch,
+                      size_t scratch_bytes, void* stream);
+
 /* ---- gated RMSNorm --------------------------------------------------------------
  * y = x * rsqrt(mean(x^2) + eps) * weight * sigmoid(gate) over the last dimension.
  * x, gate, y [rows, dim] in io_dtype; weight float32 [dim]; inv_rms float32 [rows].
@@ -236,6 +282,11 @@ size_t kda_rmsnorm_gate_bwd_scratch_bytes(int64_t rows, int32_t dim);
 int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype, const void* x, const void* gate,
                          const float* weight, const float* inv_rms, const void* d_y, void* dx, void* dgate,
                          float* dweight, void* scratch, size_t scratch_bytes, void* stream);
+
+/* dim = 128 with gate and dgate in rows of `heads` norms, gate_ld elements (a multiple of 8) apart. */
+int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t heads, int32_t gate_ld, const void* x, const void* gate,
+                              const float* weight, const float* inv_rms, const void* d_y, void* dx, void* dgate,
+                              float* dweight, void* scratch, size_t scratch_bytes, void* stream);
 
 /* ---- gated RMSNorm backward without a scratch argument (no counterpart in the reference) ----
  * Same result as kda_rmsnorm_gate_bwd, for callers that cannot supply scratch memory: a serving
