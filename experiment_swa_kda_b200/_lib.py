@@ -47,6 +47,10 @@ _SIGNATURES = {
     "kda_pack_bf16": (C.c_int, [C.c_int32] * 2 + [_P] * 4),
     "kda_decode_step": (C.c_int, [C.c_int32] * 7 + [C.c_float] + [_P] * 9),
     "kda_decode_step_raw": (C.c_int, [C.c_int32] * 5 + [C.c_float] + [_P] * 7 + [C.c_float] + [_P] * 4),
+    "kda_decode_step_raw_rows": (C.c_int, [C.c_int32] * 5 + [C.c_float] + [_P] * 5 + [C.c_int64] + [_P] * 2 + [C.c_float] + [_P] * 4),
+    "kda_rows_linear": (C.c_int, [C.c_int32] * 4 + [_P, C.c_int64] + [_P] * 3 + [C.c_int64] + [_P] * 2),
+    "kda_narrow_linear": (C.c_int, [C.c_int32] * 3 + [_P, C.c_int64] + [_P] * 3),
+    "kda_token_mix": (C.c_int, [C.c_int32] * 2 + [C.c_float] + [_P] * 6 + [C.c_int64, _P, C.c_int32, _P, _P, C.c_float, _P, C.c_float] + [_P] * 4),
     "kda_conv_step_multi": (C.c_int, [C.c_int32] * 6 + [_P] * 5),
     "kda_decode_steps": (C.c_int, [C.c_int32] * 8 + [C.c_float] + [_P] * 8),
     "kda_conv_fwd": (C.c_int, [C.c_int32] * 6 + [_P] * 6),
@@ -57,6 +61,7 @@ _SIGNATURES = {
     "kda_conv_bwd_multi": (C.c_int, [C.c_int32] * 7 + [_P] * 6 + [C.c_size_t, _P]),
     "kda_conv_fwd_rows": (C.c_int, [C.c_int32] * 7 + [_P, C.c_int32] + [_P] * 5),
     "kda_conv_bwd_rows": (C.c_int, [C.c_int32] * 7 + [_P, C.c_int32] + [_P] * 5 + [C.c_size_t, _P]),
+    "kda_rmsnorm_gate_fwd_rows": (C.c_int, [C.c_int64] + [C.c_int32] * 3 + [C.c_float] + [_P] * 6),
     "kda_rmsnorm_gate_bwd_rows": (C.c_int, [C.c_int64] + [C.c_int32] * 3 + [_P] * 9 + [C.c_size_t, _P]),
     "kda_rmsnorm_gate_fwd": (C.c_int, [C.c_int64, C.c_int32, C.c_int32, C.c_float] + [_P] * 6),
     "kda_rmsnorm_gate_bwd_scratch_bytes": (C.c_size_t, [C.c_int64, C.c_int32]),

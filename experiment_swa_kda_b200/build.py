@@ -123,7 +123,7 @@ def build_torch_ops(force: bool = False) -> str:
     cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            "-I" + os.path.join(os.path.dirname(PKG), "include"), "-I" + cuda_inc, *["-I" + i for i in ce.include_paths()],
            "-I" + sysconfig.get_paths()["include"], *SHIM_SRCS, "-o", SHIM_LIB, "-L" + tlib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
-           "-lc10_cuda", "-ltorch_python", "-L" + LIBDIR, "-lkda_b200", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib]
+           "-lc10_cuda", "-ltorch_python", "-L" + os.path.join(os.path.dirname(cuda_inc), "lib64"), "-lcublas", "-lcudart", "-L" + LIBDIR, "-lkda_b200", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib]
     with _BuildLock():
         if not force and not torch_ops_stale():
             return SHIM_LIB

@@ -31,6 +31,35 @@ __device__ __forceinline__ float warp_sum(float x) {
     return x;
 }
 
+// One output of a 128-wide product: lane holds x[4 lane .. 4 lane + 3] in xv; weights (float32 masters are rounded to
+// bf16, as a cast of the matrix would) start at w[base].  Every lane gets the sum.
+__device__ __forceinline__ void narrow_x(const __nv_bfloat16* x, int lane, float (&xv)[4]) {
+    const uint2 u = *reinterpret_cast<const uint2*>(x + 4 * lane);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    xv[0] = a.x; xv[1] = a.y; xv[2] = b.x; xv[3] = b.y;
+}
+template <bool F32W>
+__device__ __forceinline__ void narrow_w(const void* w, size_t base, int lane, float (&wv)[4]) {
+    if (F32W) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(w) + base) + lane);
+        wv[0] = __bfloat162float(__float2bfloat16(f.x)); wv[1] = __bfloat162float(__float2bfloat16(f.y));
+        wv[2] = __bfloat162float(__float2bfloat16(f.z)); wv[3] = __bfloat162float(__float2bfloat16(f.w));
+    } else {
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(w) + base) + lane);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        wv[0] = a.x; wv[1] = a.y; wv[2] = b.x; wv[3] = b.y;
+    }
+}
+__device__ __forceinline__ float narrow_sum(const float (&xv)[4], const float (&wv)[4]) {
+    float y = xv[0] * wv[0];
+    y = fmaf(xv[1], wv[1], y);
+    y = fmaf(xv[2], wv[2], y);
+    y = fmaf(xv[3], wv[3], y);
+    return warp_sum(y);
+}
+
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // Device status of a workspace: int 0 is the status word, ints 2 and 3 hold the address of a page-locked host word that

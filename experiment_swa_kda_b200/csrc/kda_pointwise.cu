@@ -25,6 +25,31 @@ __device__ __forceinline__ float sigmoid_t(float x) {
     return 1.0f / (1.0f + expf(-x));
 }
 
+template <bool BF16>
+__device__ __forceinline__ void ld4(float (&d)[4], const void* p, size_t i) {
+    if (BF16) {
+        uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p) + i);
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+        float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
+        d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
+    } else {
+        float4 f = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
+        d[0] = f.x; d[1] = f.y; d[2] = f.z; d[3] = f.w;
+    }
+}
+template <bool BF16>
+__device__ __forceinline__ void st4(void* p, size_t i, const float (&s)[4]) {
+    if (BF16) {
+        uint2 u;
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+        h[0] = __floats2bfloat162_rn(s[0], s[1]);
+        h[1] = __floats2bfloat162_rn(s[2], s[3]);
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p) + i) = u;
+    } else {
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p) + i) = make_float4(s[0], s[1], s[2], s[3]);
+    }
+}
+
 // =============================================================================================
 // gate / beta activations
 // =============================================================================================
@@ -135,14 +160,32 @@ struct RawGate {
     const float* A_log;      // [H], or nullptr: g and beta are already activated
     const float* dt_bias;    // [H*K]
     float lb;
+    long long bl_ld;         // elements between the beta logits of consecutive sequences (heads when dense)
 };
 
-template <int NV4, int R>
-__global__ void __launch_bounds__(256) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
+// FUSED: the layer's decode step around the recurrence (K = V = 128, bf16, raw gate).  The kernel forms its head's raw
+// gate from the low-rank projection, steps the state, and applies the gated RMSNorm to the head's output: three launches
+// of a token become one.  Each part repeats the stand-alone kernel's arithmetic, so both forms give the same bits.  The
+// block then owns all 128 rows of a state: 32 warps hold the whole 64 KB in flight when there are fewer blocks than SMs
+// (4.5 -> 3.4 us at one sequence and 3 heads), eight warps otherwise.
+struct TokenMix {
+    const __nv_bfloat16* fa;       // [n_seq][128], rows ld apart
+    const void* fb_w;              // [heads*128][128]
+    const __nv_bfloat16* gate;     // [n_seq][heads][128], rows ld apart
+    const float* norm_w;           // [128]
+    long long ld;
+    float eps;
+    int fb_f32;
+};
+
+template <int NV4, int R, int NW, bool FUSED>
+__global__ void __launch_bounds__(NW * 32) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
                                                      const void* __restrict__ q, const void* __restrict__ k,
                                                      const void* __restrict__ v, const void* __restrict__ g,
                                                      const void* __restrict__ beta, const float* s_in, float* s_out,
-                                                     void* __restrict__ o, int rows_per_cta, RawGate raw) {
+                                                     void* __restrict__ o, int rows_per_cta, RawGate raw, TokenMix mix) {
+    __shared__ __align__(16) float raw_s[FUSED ? 128 : 4];
+    __shared__ __align__(16) __nv_bfloat16 o_s[FUSED ? 128 : 8];
     constexpr int NE = NV4 > 0 ? 4 * NV4 : 8;     // state elements per lane per row
     const int bh = blockIdx.x;                    // sequence * H + head
     const int v_base = blockIdx.y * rows_per_cta;
@@ -172,6 +215,29 @@ __global__ void __launch_bounds__(256) decode_kernel(int H, int K, int V, int bf
     float s[R][NE], vv[R];
     int r0 = v_base + warp * R;
     if (r0 < v_end) load_rows(r0, s, vv);
+    if (FUSED) {
+        const int hh = bh % H;
+        float xv[4];
+        narrow_x(mix.fa + (size_t)(bh / H) * mix.ld, lane, xv);
+        constexpr int PER = 128 / NW, G = PER < 8 ? PER : 8;       // gate rows per warp, G weight rows in flight
+#pragma unroll 1
+        for (int i0 = 0; i0 < PER; i0 += G) {
+            float wv[G][4], y[G];
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                const size_t base = ((size_t)hh * 128 + (i0 + i) * NW + warp) * 128;
+                if (mix.fb_f32) narrow_w<true>(mix.fb_w, base, lane, wv[i]);
+                else narrow_w<false>(mix.fb_w, base, lane, wv[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < G; ++i) y[i] = narrow_sum(xv, wv[i]);
+            if (lane == 0) {
+#pragma unroll
+                for (int i = 0; i < G; ++i) raw_s[(i0 + i) * NW + warp] = __bfloat162float(__float2bfloat16(y[i]));
+            }
+        }
+        __syncthreads();
+    }
 
     float qe[NE], ke[NE], dec[NE];
 #pragma unroll
@@ -179,9 +245,9 @@ __global__ void __launch_bounds__(256) decode_kernel(int H, int K, int V, int bf
         const size_t i = (size_t)bh * K + min(key_of(e), K - 1);
         qe[e] = ld_io(q, i, bf16);
         ke[e] = ld_io(k, i, bf16);
-        dec[e] = ld_io(g, i, gbf16);
+        dec[e] = FUSED ? raw_s[key_of(e)] : ld_io(g, i, gbf16);
     }
-    float bt = ld_io(beta, bh, gbf16);
+    float bt = ld_io(beta, raw.A_log != nullptr ? (size_t)(bh / H) * raw.bl_ld + bh % H : (size_t)bh, gbf16);
     if (raw.A_log != nullptr) {
         const int hh = bh % H;
         const float ea = expf(raw.A_log[hh]);
@@ -213,7 +279,7 @@ __global__ void __launch_bounds__(256) decode_kernel(int H, int K, int V, int bf
     }
     qk = warp_sum(qk);
 
-    for (; r0 < v_end; r0 += 8 * R) {
+    for (; r0 < v_end; r0 += NW * R) {
         float a[R], b[R];
 #pragma unroll
         for (int j = 0; j < R; ++j) {
@@ -257,10 +323,30 @@ __global__ void __launch_bounds__(256) decode_kernel(int H, int K, int V, int bf
                         if (kk < K) dst[kk] = s[j][e] + br * ke[e];
                     }
                 }
-                if (lane == 0) st_io(o, (size_t)bh * V + row, bf16, b[j] + br * qk);
+                if (lane == 0) {
+                    if (FUSED) o_s[row] = __float2bfloat16(b[j] + br * qk);
+                    else st_io(o, (size_t)bh * V + row, bf16, b[j] + br * qk);
+                }
             }
         }
-        if (r0 + 8 * R < v_end) load_rows(r0 + 8 * R, s, vv);
+        if (r0 + NW * R < v_end) load_rows(r0 + NW * R, s, vv);
+    }
+    if (FUSED) {
+        __syncthreads();
+        if (warp == 0) {      // the head's 128 outputs: lane = 4 adjacent values, as in the stand-alone norm
+            float a[4], gt[4], out[4];
+            ld4<true>(a, o_s, 4 * lane);
+            ld4<true>(gt, mix.gate, (size_t)(bh / H) * mix.ld + (bh % H) * 128 + 4 * lane);
+            const float4 ww = *reinterpret_cast<const float4*>(mix.norm_w + 4 * lane);
+            const float wa[4] = {ww.x, ww.y, ww.z, ww.w};
+            float ss = a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            const float inv = rsqrtf(ss * (1.0f / 128.0f) + mix.eps);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) out[e] = a[e] * inv * wa[e] * sigmoid_t<true>(gt[e]);
+            st4<true>(o, (size_t)bh * 128 + 4 * lane, out);
+        }
     }
 }
 
@@ -1282,31 +1368,6 @@ __global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int
 // =============================================================================================
 // gated RMSNorm:  y = x * inv * w * sigmoid(gate),  inv = rsqrt(mean(x^2) + eps).  One warp per row.
 // =============================================================================================
-template <bool BF16>
-__device__ __forceinline__ void ld4(float (&d)[4], const void* p, size_t i) {
-    if (BF16) {
-        uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p) + i);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-        float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-        d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
-    } else {
-        float4 f = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
-        d[0] = f.x; d[1] = f.y; d[2] = f.z; d[3] = f.w;
-    }
-}
-template <bool BF16>
-__device__ __forceinline__ void st4(void* p, size_t i, const float (&s)[4]) {
-    if (BF16) {
-        uint2 u;
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
-        h[0] = __floats2bfloat162_rn(s[0], s[1]);
-        h[1] = __floats2bfloat162_rn(s[2], s[3]);
-        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p) + i) = u;
-    } else {
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p) + i) = make_float4(s[0], s[1], s[2], s[3]);
-    }
-}
-
 // VEC4: dim % 128 == 0, lane owns 4 contiguous elements per 128-wide segment; else scalar stride-32.
 template <bool BF16, bool VEC4>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(long long rows, int D, float eps, const void* __restrict__ x,
@@ -1431,8 +1492,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(long long rows, int D,
 // 8-byte (bf16) loads in flight instead of one row's worth.
 constexpr int kRmsRows = 4;
 
-template <bool BF16>
-__global__ void __launch_bounds__(256) rmsnorm_fwd128_kernel(long long rows, float eps, const void* __restrict__ x,
+template <bool BF16, bool ROWS>
+__global__ void __launch_bounds__(256) rmsnorm_fwd128_kernel(long long rows, int heads, int gate_ld, float eps, const void* __restrict__ x,
                                                              const void* __restrict__ gate, const float* __restrict__ w,
                                                              void* __restrict__ y, float* __restrict__ inv_rms) {
     const int lane = threadIdx.x & 31;
@@ -1440,13 +1501,17 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd128_kernel(long long rows, flo
     const long long nwarp = (long long)gridDim.x * 8;
     const float4 ww = *reinterpret_cast<const float4*>(w + 4 * lane);
     const float wa[4] = {ww.x, ww.y, ww.z, ww.w};
+    auto gate_at = [&](long long row) {      // as in the backward below
+        const unsigned r = (unsigned)row, tok = r / (unsigned)heads;
+        return (size_t)tok * gate_ld + (r - tok * (unsigned)heads) * 128 + 4 * lane;
+    };
     for (long long row0 = warp0 * kRmsRows; row0 < rows; row0 += nwarp * kRmsRows) {
         float a[kRmsRows][4], gt[kRmsRows][4], ss[kRmsRows];
 #pragma unroll
         for (int r = 0; r < kRmsRows; ++r) {
             const size_t base = (size_t)min(row0 + r, rows - 1) * 128 + 4 * lane;
             ld4<BF16>(a[r], x, base);
-            ld4<BF16>(gt[r], gate, base);
+            ld4<BF16>(gt[r], gate, ROWS ? gate_at(min(row0 + r, rows - 1)) : base);
         }
 #pragma unroll
         for (int r = 0; r < kRmsRows; ++r) ss[r] = a[r][0] * a[r][0] + a[r][1] * a[r][1] + a[r][2] * a[r][2] + a[r][3] * a[r][3];
@@ -1707,7 +1772,7 @@ extern "C" int kda_gate_bwd(int32_t tokens, int32_t heads, int32_t key_dim, int3
 
 static int decode_launch(int n_seq, int heads, int key_dim, int value_dim, int bf16, int gbf16, int l2norm, float scale, const void* q,
                          const void* k, const void* v, const void* g, const void* beta, const float* state_in, float* state_out,
-                         void* o, cudaStream_t st, pw::RawGate raw = pw::RawGate{nullptr, nullptr, 0.f}) {
+                         void* o, cudaStream_t st, pw::RawGate raw = pw::RawGate{nullptr, nullptr, 0.f, 0}) {
     // four rows in flight per warp: at ~70 registers three to four CTAs share an SM, so one CTA's prologue (norms, decay) hides
     // under the others' streaming; eight rows per warp measured 20 % slower
     // one CTA per (sequence, head) once there are enough of them to fill the GPU; otherwise split the value rows
@@ -1715,26 +1780,59 @@ static int decode_launch(int n_seq, int heads, int key_dim, int value_dim, int b
     dim3 grid(n_seq * heads, ceil_div(value_dim, rows_per_cta));
     const bool vec = (key_dim % 4 == 0) &&
                      ((reinterpret_cast<uintptr_t>(state_in) | reinterpret_cast<uintptr_t>(state_out)) % 16 == 0);
-    if (vec && key_dim <= 128)
-        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<1, 4><<<grid, 256, 0, st>>>(heads, key_dim, value_dim, bf16, gbf16, l2norm, scale, q, k, v, g, beta, state_in, state_out, o, rows_per_cta, raw));
-    else if (vec)
-        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<2, 4><<<grid, 256, 0, st>>>(heads, key_dim, value_dim, bf16, gbf16, l2norm, scale, q, k, v, g, beta, state_in, state_out, o, rows_per_cta, raw));
-    else
-        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<0, 4><<<grid, 256, 0, st>>>(heads, key_dim, value_dim, bf16, gbf16, l2norm, scale, q, k, v, g, beta, state_in, state_out, o, rows_per_cta, raw));
+    const pw::TokenMix none = {};
+#define KDA_DECODE(NV4) \
+    KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<NV4, 4, 8, false><<<grid, 256, 0, st>>>(heads, key_dim, value_dim, bf16, gbf16, l2norm, scale, q, k, v, g, beta, state_in, state_out, o, rows_per_cta, raw, none))
+    if (vec && key_dim <= 128) KDA_DECODE(1);
+    else if (vec) KDA_DECODE(2);
+    else KDA_DECODE(0);
+#undef KDA_DECODE
     return launch_status();
+}
+
+extern "C" int kda_decode_step_raw_rows(int32_t n_seq, int32_t heads, int32_t key_dim, int32_t value_dim, int32_t io_dtype, float scale,
+                                        const void* q, const void* k, const void* v, const void* raw_gate, const void* beta_logits, int64_t bl_ld,
+                                        const float* A_log, const float* dt_bias, float lower_bound, const float* state_in,
+                                        float* state_out, void* o, void* stream) {
+    if (n_seq < 0 || heads <= 0 || key_dim <= 0 || value_dim <= 0 || key_dim > KDA_MAX_DIM || value_dim > KDA_MAX_DIM || bl_ld < heads)
+        return KDA_ERR_BAD_SHAPE;
+    if (n_seq == 0) return KDA_OK;
+    if (!q || !k || !v || !raw_gate || !beta_logits || !A_log || !dt_bias || !state_in || !state_out || !o) return KDA_ERR_NULL;
+    const int bf16 = io_dtype == KDA_DTYPE_BF16;
+    return decode_launch(n_seq, heads, key_dim, value_dim, bf16, bf16, 1, scale, q, k, v, raw_gate, beta_logits, state_in, state_out, o,
+                         (cudaStream_t)stream, pw::RawGate{A_log, dt_bias, lower_bound, bl_ld});
 }
 
 extern "C" int kda_decode_step_raw(int32_t n_seq, int32_t heads, int32_t key_dim, int32_t value_dim, int32_t io_dtype, float scale,
                                    const void* q, const void* k, const void* v, const void* raw_gate, const void* beta_logits,
                                    const float* A_log, const float* dt_bias, float lower_bound, const float* state_in,
                                    float* state_out, void* o, void* stream) {
-    if (n_seq < 0 || heads <= 0 || key_dim <= 0 || value_dim <= 0 || key_dim > KDA_MAX_DIM || value_dim > KDA_MAX_DIM)
-        return KDA_ERR_BAD_SHAPE;
+    return kda_decode_step_raw_rows(n_seq, heads, key_dim, value_dim, io_dtype, scale, q, k, v, raw_gate, beta_logits, heads, A_log, dt_bias,
+                                    lower_bound, state_in, state_out, o, stream);
+}
+
+extern "C" int kda_token_mix(int32_t n_seq, int32_t heads, float scale, const void* q, const void* k, const void* v, const void* fa,
+                             const void* beta_logits, const void* gate, int64_t ld, const void* fb_weight, int32_t fb_dtype, const float* A_log,
+                             const float* dt_bias, float lower_bound, const float* norm_weight, float eps, const float* state_in,
+                             float* state_out, void* mixed, void* stream) {
+    if (n_seq < 0 || heads <= 0 || ld < heads) return KDA_ERR_BAD_SHAPE;
     if (n_seq == 0) return KDA_OK;
-    if (!q || !k || !v || !raw_gate || !beta_logits || !A_log || !dt_bias || !state_in || !state_out || !o) return KDA_ERR_NULL;
-    const int bf16 = io_dtype == KDA_DTYPE_BF16;
-    return decode_launch(n_seq, heads, key_dim, value_dim, bf16, bf16, 1, scale, q, k, v, raw_gate, beta_logits, state_in, state_out, o,
-                         (cudaStream_t)stream, pw::RawGate{A_log, dt_bias, lower_bound});
+    if (!q || !k || !v || !fa || !beta_logits || !gate || !fb_weight || !A_log || !dt_bias || !norm_weight || !state_in || !state_out || !mixed)
+        return KDA_ERR_NULL;
+    if (ld % 4 != 0 || (reinterpret_cast<uintptr_t>(state_in) | reinterpret_cast<uintptr_t>(state_out) | reinterpret_cast<uintptr_t>(fb_weight) |
+                        reinterpret_cast<uintptr_t>(norm_weight)) % 16 != 0 ||
+        (reinterpret_cast<uintptr_t>(fa) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(mixed)) % 8 != 0)
+        return KDA_ERR_UNSUPPORTED;
+    const pw::TokenMix mix{static_cast<const __nv_bfloat16*>(fa), fb_weight, static_cast<const __nv_bfloat16*>(gate), norm_weight, ld, eps,
+                           fb_dtype == KDA_DTYPE_F32 ? 1 : 0};
+    const pw::RawGate raw{A_log, dt_bias, lower_bound, ld};
+    cudaStream_t st = (cudaStream_t)stream;
+    const int blocks = n_seq * heads;
+    if (blocks <= 148)
+        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<1, 4, 32, true><<<blocks, 1024, 0, st>>>(heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits, state_in, state_out, mixed, 128, raw, mix));
+    else
+        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<1, 4, 8, true><<<blocks, 256, 0, st>>>(heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits, state_in, state_out, mixed, 128, raw, mix));
+    return launch_status();
 }
 
 extern "C" int kda_decode_step(int32_t n_seq, int32_t heads, int32_t key_dim, int32_t value_dim, int32_t io_dtype,
@@ -2056,8 +2154,8 @@ extern "C" int kda_rmsnorm_gate_fwd(int64_t rows, int32_t dim, int32_t io_dtype,
                        reinterpret_cast<uintptr_t>(weight)) % 16) == 0;
     if (vec && dim == 128) {
         const int nb4 = (int)std::min<long long>((rows + 8 * pw::kRmsRows - 1) / (8 * pw::kRmsRows), 148LL * 8);
-        if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd128_kernel<true><<<nb4, 256, 0, st>>>(rows, eps, x, gate, weight, y, inv_rms));
-        else KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd128_kernel<false><<<nb4, 256, 0, st>>>(rows, eps, x, gate, weight, y, inv_rms));
+        if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd128_kernel<true, false><<<nb4, 256, 0, st>>>(rows, 1, 128, eps, x, gate, weight, y, inv_rms));
+        else KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd128_kernel<false, false><<<nb4, 256, 0, st>>>(rows, 1, 128, eps, x, gate, weight, y, inv_rms));
         return launch_status();
     }
     if (io_dtype == KDA_DTYPE_BF16) {
@@ -2067,6 +2165,20 @@ extern "C" int kda_rmsnorm_gate_fwd(int64_t rows, int32_t dim, int32_t io_dtype,
         if (vec) KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd_kernel<false, true><<<nb, 256, 0, st>>>(rows, dim, eps, x, gate, weight, y, inv_rms));
         else KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd_kernel<false, false><<<nb, 256, 0, st>>>(rows, dim, eps, x, gate, weight, y, inv_rms));
     }
+    return launch_status();
+}
+
+extern "C" int kda_rmsnorm_gate_fwd_rows(int64_t rows, int32_t io_dtype, int32_t heads, int32_t gate_ld, float eps, const void* x,
+                                         const void* gate, const float* weight, void* y, float* inv_rms, void* stream) {
+    if (rows <= 0 || rows >= (1LL << 31) || heads <= 0 || rows % heads != 0 || gate_ld < heads * 128) return KDA_ERR_BAD_SHAPE;
+    if (!x || !gate || !weight || !y || !inv_rms) return KDA_ERR_NULL;
+    if (gate_ld % 8 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(y) |
+                              reinterpret_cast<uintptr_t>(weight)) % 16) != 0)
+        return KDA_ERR_UNSUPPORTED;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int nb4 = (int)std::min<long long>((rows + 8 * pw::kRmsRows - 1) / (8 * pw::kRmsRows), 148LL * 8);
+    if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd128_kernel<true, true><<<nb4, 256, 0, st>>>(rows, heads, gate_ld, eps, x, gate, weight, y, inv_rms));
+    else KDA_LAUNCH("rmsnorm_fwd_kernel", st, pw::rmsnorm_fwd128_kernel<false, true><<<nb4, 256, 0, st>>>(rows, heads, gate_ld, eps, x, gate, weight, y, inv_rms));
     return launch_status();
 }
 

@@ -401,12 +401,17 @@ class KimiDeltaAttention(nn.Module):
         batch, length, _ = hidden_states.shape
         requested_mode = self.mode if mode is None else mode
         want_state = bool(output_final_state)
-        if requested_mode == "project_chunk" and hidden_states.is_cuda and self.head_dim == 128 and type(hidden_states) is Tensor:
+        if hidden_states.is_cuda and self.head_dim == 128 and type(hidden_states) is Tensor:
             weights = self._plain_weights()
             if weights is not None:
-                incoming = () if state is None else (state.memory, state.q_conv, state.k_conv, state.v_conv)
-                out = _native.load().layer(hidden_states, weights, self.num_heads, self.o_norm.eps, self.lower_bound, incoming, want_state,
-                                           self.fuse_prefill_conv)
+                out = None
+                if requested_mode == "project_chunk":
+                    incoming = () if state is None else (state.memory, state.q_conv, state.k_conv, state.v_conv)
+                    out = _native.load().layer(hidden_states, weights, self.num_heads, self._modules["o_norm"].eps, self.lower_bound, incoming, want_state,
+                                               self.fuse_prefill_conv)
+                elif requested_mode == "project_recurrent" and length == 1 and state is not None and want_state and not torch.is_grad_enabled():
+                    out = _native.load().token(hidden_states, weights, self.num_heads, self._modules["o_norm"].eps, self.lower_bound,
+                                               (state.memory, state.q_conv, state.k_conv, state.v_conv), False)
                 if out is not None:
                     return out[0], (KDAState(*out[1:]) if want_state else None)
         q_state = None if state is None else state.q_conv
@@ -463,22 +468,33 @@ class KimiDeltaAttention(nn.Module):
         weights[-1:] = (own.get("A_log"), own.get("dt_bias"), weights[-1])
         return weights if all(type(w) in (nn.Parameter, Tensor) for w in weights) else None
 
-    @torch.no_grad()
     def decode_token(self, hidden_states: Tensor, state: KDAState) -> Tensor:
         """One decode token with the state updated IN PLACE (inference only).
 
         The non-mutating contract of `forward(..., state, output_final_state=True, mode="project_recurrent")` costs a
         serving loop six library launches and four freshly allocated state tensors per layer and token (the reference's
         cache plumbing: nanochat/engine.py:83-226, get/set_kda_state :160-170).  Here the caller owns one `KDAState`
-        (see `KDAState.zeros`); the three convolution caches are advanced by one fused launch, the gate and beta
-        activations run inside the decode kernel, and the memory is rewritten where it lies: three library launches, no
-        state allocation.  Same arithmetic, same results as the non-mutating path."""
+        (see `KDAState.zeros`) and a token is three launches: the six projections of the input with the convolution step in
+        their epilogue, the decode step with the gate projection before and the gated norm behind it, and the output
+        projection.  The projections read the parameters as they are, no cast or copy is kept.  Same arithmetic, same
+        results as the non-mutating path.  Batches above 64 run the modules one by one."""
         if hidden_states.ndim != 3 or hidden_states.shape[1] != 1 or hidden_states.shape[-1] != self.hidden_size:
             raise ValueError(f"hidden_states must have shape [B,1,{self.hidden_size}]")
         if not hidden_states.is_cuda:
             raise RuntimeError("project CUDA KDA backend unavailable: project KDA requires CUDA")
-        batch = hidden_states.shape[0]
         x = hidden_states
+        if self.head_dim == 128 and type(x) is Tensor:
+            weights = self._plain_weights()
+            if weights is not None:
+                out = _native.load().token(x, weights, self.num_heads, self._modules["o_norm"].eps, self.lower_bound,
+                                           (state.memory, state.q_conv, state.k_conv, state.v_conv), True)
+                if out is not None:
+                    return out[0]
+        return self._decode_modules(x, state)
+
+    @torch.no_grad()
+    def _decode_modules(self, x: Tensor, state: KDAState) -> Tensor:
+        batch = x.shape[0]
         conv_w = [c.weight.squeeze(1) for c in (self.q_conv1d, self.k_conv1d, self.v_conv1d)]
         q, k, v = ops.conv_step_multi((self.q_proj(x), self.k_proj(x), self.v_proj(x)), conv_w,
                                       (state.q_conv, state.k_conv, state.v_conv))

@@ -30,6 +30,27 @@ inline Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& li
 inline Tensor empty_as(const Tensor& t) { return empty(t.sizes(), t.scalar_type(), t); }
 inline Tensor bytes(size_t n, const Tensor& like) { return empty({(int64_t)(n < 256 ? 256 : n)}, at::kByte, like); }
 
+// One allocation cut into 256-byte aligned tensors: a call's temporaries cost one trip to the allocator.
+class Slab {
+public:
+    size_t take(size_t n_bytes) {
+        const size_t at = size_;
+        size_ += (n_bytes + 255) / 256 * 256;
+        return at;
+    }
+    Tensor make(const Tensor& like) {
+        all_ = bytes(size_, like);
+        return all_;
+    }
+    const Tensor& tensor() const { return all_; }
+    char* at(size_t offset) const { return static_cast<char*>(all_.data_ptr()) + offset; }
+    float* f32(size_t offset) const { return reinterpret_cast<float*>(at(offset)); }
+
+private:
+    size_t size_ = 0;
+    Tensor all_;
+};
+
 inline size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 
 // Device status without a hot-path cost: every device has one page-locked word that the kernels write to only when

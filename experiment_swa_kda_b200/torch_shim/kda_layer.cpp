@@ -6,7 +6,7 @@
 // projection in place, and the backward forms the gradient of the input as one GEMM over all six and the six weight
 // gradients as another, both accumulated in float32.  Columns of the projection P [tokens][n]:
 //     q | k | v | output gate (hidden each) | f_a (128) | b (heads) | zero padding to a multiple of 8
-// B2 T2045 width 768, forward and backward: 1,141 -> see DESIGN; 65 -> 27 launches.
+// B2 T2045 width 768, forward and backward: 1,141 us and 65 launches -> 420 us and 27.
 
 #include <torch/extension.h>
 
@@ -14,6 +14,8 @@
 #include <tuple>
 
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <cublas_v2.h>
 
 #include "host_node.h"
 
@@ -31,26 +33,45 @@ struct Sizes {
     int64_t b() const { return 4 * hid + kHead; }
 };
 
-// all weights of the layer's products in bf16: rows of P's matrix, then f_b, then the output projection
-struct Packed {
-    Tensor all, p, fb, o;
-};
+char* at_col(char* p, int64_t col) { return p + 2 * col; }
 
-Packed pack_weights(const std::vector<Tensor>& w, const Sizes& z) {
+// all weights of the layer's products in bf16: rows of P's matrix, then f_b, then the output projection
+size_t packed_bytes(const Sizes& z) { return 2 * (size_t)((z.n + kHead + z.hid) * z.hid); }
+char* packed_fb(char* pack, const Sizes& z) { return pack + 2 * z.n * z.hid; }
+char* packed_o(char* pack, const Sizes& z) { return pack + 2 * (z.n + kHead) * z.hid; }
+
+void pack_weights(const std::vector<Tensor>& w, const Sizes& z, char* pack, void* st) {
     const int64_t h = z.hid;
-    Packed r;
-    r.all = empty({(z.n + kHead + h) * h}, at::kBFloat16, w[kQ]);
     const void* src[9] = {w[kQ].data_ptr(), w[kK].data_ptr(), w[kV].data_ptr(), w[kG].data_ptr(), w[kFa].data_ptr(),
                           w[kB].data_ptr(), nullptr, w[kFb].data_ptr(), w[kO].data_ptr()};
     const int64_t elems[9] = {h * h, h * h, h * h, h * h, kHead * h, z.H * h, z.pad * h, h * kHead, h * h};
-    must(kda_pack_bf16(9, dt(w[kQ]), src, elems, r.all.data_ptr(), stream_of(w[kQ])), "kda_pack_bf16");
-    r.p = r.all.narrow(0, 0, z.n * h).view({z.n, h});
-    r.fb = r.all.narrow(0, z.n * h, h * kHead).view({h, kHead});
-    r.o = r.all.narrow(0, (z.n + kHead) * h, h * h).view({h, h});
-    return r;
+    must(kda_pack_bf16(9, dt(w[kQ]), src, elems, pack, st), "kda_pack_bf16");
 }
 
-char* at_col(const Tensor& p, int64_t col) { return static_cast<char*>(p.data_ptr()) + 2 * col; }
+// Row-major products with row strides, bf16 operands and float32 accumulation.  cuBLAS directly: at::mm spends as long in
+// dispatch and views as the call itself takes, and these operands are slices.
+void gemm(cublasOperation_t ta, cublasOperation_t tb, int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, const void* b, int64_t ldb,
+          void* c, int64_t ldc, at::ScalarType ctype) {
+    const float one = 1.f, zero = 0.f;
+    const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), ta, tb, (int)m, (int)n, (int)k, &one, a, CUDA_R_16BF, (int)lda, b,
+                                           CUDA_R_16BF, (int)ldb, &zero, c, ctype == at::kFloat ? CUDA_R_32F : CUDA_R_16BF, (int)ldc,
+                                           CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+    TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed (", (int)rc, ")");
+}
+// y [m][n] = x [m][k] w^T, w [n][k]
+void linear(const void* x, int64_t ldx, const void* w, int64_t ldw, void* y, int64_t ldy, int64_t m, int64_t n, int64_t k) {
+    gemm(CUBLAS_OP_T, CUBLAS_OP_N, n, m, k, w, ldw, x, ldx, y, ldy, at::kBFloat16);
+}
+// dx [m][k] = dy [m][n] w
+void linear_dx(const void* dy, int64_t ldy, const void* w, int64_t ldw, void* dx, int64_t ldx, int64_t m, int64_t n, int64_t k) {
+    gemm(CUBLAS_OP_N, CUBLAS_OP_N, k, m, n, w, ldw, dy, ldy, dx, ldx, at::kBFloat16);
+}
+// dw [n][k] = dy^T x, in float32 straight from the accumulators when the parameter is float32
+Tensor linear_dw(const void* dy, int64_t ldy, const void* x, int64_t ldx, int64_t m, int64_t n, int64_t k, at::ScalarType type, const Tensor& like) {
+    Tensor dw = empty({n, k}, type, like);
+    gemm(CUBLAS_OP_N, CUBLAS_OP_T, k, n, m, x, ldx, dy, ldy, dw.data_ptr(), k, type);
+    return dw;
+}
 
 KdaChunkShape layer_shape(const Sizes& z, bool forward_only) {
     KdaChunkShape sh;
@@ -68,10 +89,27 @@ KdaChunkShape layer_shape(const Sizes& z, bool forward_only) {
     return sh;
 }
 
-// weight gradient dY^T X: float32 straight from the accumulators when the parameter is float32
-Tensor weight_grad(const Tensor& dy, const Tensor& x, at::ScalarType type) {
-    return type == at::kFloat ? at::mm(dy.t(), x, at::kFloat) : at::mm(dy.t(), x);
-}
+// What a forward keeps for its backward, one allocation
+struct Kept {
+    Slab slab;
+    size_t pack, P, raw, g, beta, q, k, v, ws, o, inv, mixed, ws_bytes;
+    Kept(const Sizes& z, const KdaChunkShape& sh, bool tracked, bool with_pack, bool with_qkv) {
+        const size_t act = 2 * (size_t)(z.M * z.hid);
+        pack = slab.take(with_pack ? packed_bytes(z) : 0);
+        P = slab.take(2 * (size_t)(z.M * z.n));
+        raw = slab.take(act);
+        g = slab.take(2 * act);
+        beta = slab.take(4 * (size_t)(z.M * z.H));
+        q = slab.take(with_qkv ? act : 0);
+        k = slab.take(with_qkv ? act : 0);
+        v = slab.take(with_qkv ? act : 0);
+        mixed = slab.take(act);
+        o = slab.take(tracked ? act : 0);
+        inv = slab.take(tracked ? 4 * (size_t)(z.M * z.H) : 0);
+        ws_bytes = kda_chunk_workspace_bytes(&sh);
+        ws = slab.take(ws_bytes);
+    }
+};
 
 struct LayerNode : public HostNode {
     Sizes z;
@@ -81,8 +119,8 @@ struct LayerNode : public HostNode {
     std::vector<int64_t> cshape[3], dt_shape;
     bool has_state = false;
     std::string name() const override { return "KimiDeltaAttentionBackward"; }
-    // saved: x, conv weights, A_log, dt_bias, norm weight | pack, P, raw, g, beta, q, k, v, ws, o, inv, mixed | windows
-    enum { sX, sCq, sCk, sCv, sA, sDt, sN, sPack, sP, sRaw, sG, sBeta, sQ, sK, sV, sWs, sO, sInv, sMixed, sWq, sWk, sWv };
+    // saved: x, conv weights, A_log, dt_bias, norm weight, the forward's slab | windows
+    enum { sX, sCq, sCk, sCv, sA, sDt, sN, sKept, sWq, sWk, sWv };
 
     variable_list apply(variable_list&& grads) override {
         std::vector<Tensor> t;
@@ -95,56 +133,59 @@ struct LayerNode : public HostNode {
         c10::cuda::CUDAGuard guard(x.device());
         watch_status(x.device().index());
         void* st = stream_of(x);
-        const int64_t h = z.hid, M = z.M, H = z.H;
+        const int64_t h = z.hid, M = z.M, H = z.H, n = z.n;
+        const size_t act = 2 * (size_t)(M * h);
         variable_list out(15 + (has_state ? 4 : 0));
         auto want = [&](size_t i) { return task_should_compute_output(i); };
-        const Tensor P = t[sP], x2 = x.view({M, h});
-        const Tensor wp = t[sPack].narrow(0, 0, z.n * h).view({z.n, h}), wfb = t[sPack].narrow(0, z.n * h, h * kHead).view({h, kHead}),
-                     wo = t[sPack].narrow(0, (z.n + kHead) * h, h * h).view({h, h});
+        const KdaChunkShape sh = layer_shape(z, false);
+        const Kept kept(z, sh, true, true, true);
+        char* base = static_cast<char*>(t[sKept].data_ptr());
+        char *pack = base + kept.pack, *P = base + kept.P;
 
-        const Tensor dy = grads[0].defined() ? dense_as(grads[0], at::kBFloat16).view({M, h}) : at::zeros({M, h}, x.options());
-        if (want(1 + kO)) out[1 + kO] = weight_grad(dy, t[sMixed].view({M, h}), wtype);
-        const Tensor d_mixed = at::mm(dy, wo);
+        Slab tmp;      // the backward's temporaries
+        const size_t t_dmix = tmp.take(act), t_dP = tmp.take(2 * (size_t)(M * n)), t_do = tmp.take(act), t_dq = tmp.take(3 * act),
+                     t_dg = tmp.take(2 * act), t_db = tmp.take(4 * (size_t)(M * H)), t_draw = tmp.take(act);
+        const size_t nb_norm = kda_rmsnorm_gate_bwd_scratch_bytes(M * H, (int32_t)kHead), nb_chunk = std::max<size_t>(kda_chunk_bwd_scratch_bytes(&sh), 256),
+                     nb_gate = kda_gate_bwd_scratch_bytes((int32_t)M, (int32_t)H, (int32_t)kHead),
+                     nb_conv = kda_conv_bwd_multi_scratch_bytes(3, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W);
+        const size_t t_scr = tmp.take(std::max(std::max(nb_norm, nb_chunk), std::max(nb_gate, nb_conv)));      // one after the other on one stream
+        tmp.make(x);
+        char *dmix = tmp.at(t_dmix), *dP = tmp.at(t_dP), *dq = tmp.at(t_dq), *draw = tmp.at(t_draw), *scr = tmp.at(t_scr);
+        Tensor small = empty({kHead + H + h + 3 * h * z.W}, at::kFloat, x);      // gradients of the vectors and the taps
+        float *dnw = small.data_ptr<float>(), *dA = dnw + kHead, *dbias = dA + H, *dcw = dbias + h;
+
+        const Tensor dy = grads[0].defined() ? dense_as(grads[0], at::kBFloat16) : at::zeros({M, h}, x.options());
+        if (want(1 + kO)) out[1 + kO] = linear_dw(dy.data_ptr(), h, base + kept.mixed, h, M, h, h, wtype, x);
+        linear_dx(dy.data_ptr(), h, packed_o(pack, z), h, dmix, h, M, h, h);
 
         // gated norm: its gate and the gate's gradient are slices of P and dP
-        Tensor dP = empty({M, z.n}, at::kBFloat16, x);
-        Tensor d_o = empty_as(t[sO]), dnw = empty({kHead}, at::kFloat, x);
-        Tensor nscr = bytes(kda_rmsnorm_gate_bwd_scratch_bytes(M * H, (int32_t)kHead), x);
-        must(kda_rmsnorm_gate_bwd_rows(M * H, KDA_DTYPE_BF16, (int32_t)H, (int32_t)z.n, t[sO].data_ptr(), at_col(P, 3 * h),
-                                       t[sN].data_ptr<float>(), t[sInv].data_ptr<float>(), d_mixed.data_ptr(), d_o.data_ptr(), at_col(dP, 3 * h),
-                                       dnw.data_ptr<float>(), nscr.data_ptr(), (size_t)nscr.numel(), st),
+        must(kda_rmsnorm_gate_bwd_rows(M * H, KDA_DTYPE_BF16, (int32_t)H, (int32_t)n, base + kept.o, at_col(P, 3 * h), t[sN].data_ptr<float>(),
+                                       reinterpret_cast<float*>(base + kept.inv), dmix, tmp.at(t_do), at_col(dP, 3 * h), dnw, scr, nb_norm, st),
              "kda_rmsnorm_gate_bwd_rows");
-        out[1 + kNorm] = ntype == at::kFloat ? dnw : dnw.to(ntype);
+        const Tensor g_nw = small.narrow(0, 0, kHead);
+        out[1 + kNorm] = ntype == at::kFloat ? g_nw : g_nw.to(ntype);
 
         // chunked operator
-        const KdaChunkShape sh = layer_shape(z, false);
         const Tensor dmem = grads[1].defined() ? dense_as(grads[1], at::kFloat) : Tensor();
-        Tensor dqkv = empty({3, M, h}, at::kBFloat16, x), dg = empty_as(t[sG]), db = empty_as(t[sBeta]), dh0;
+        Tensor dh0;
         if (has_state) dh0 = empty({z.B, H, kHead, kHead}, at::kFloat, x);
-        char* d3 = static_cast<char*>(dqkv.data_ptr());
-        Tensor scr = bytes(kda_chunk_bwd_scratch_bytes(&sh), x);
-        must(kda_chunk_bwd(&sh, t[sQ].data_ptr(), t[sK].data_ptr(), t[sV].data_ptr(), t[sG].data_ptr(), t[sBeta].data_ptr(), nullptr, d_o.data_ptr(),
-                           dmem.defined() ? dmem.data_ptr<float>() : nullptr, t[sWs].data_ptr(), (size_t)t[sWs].numel(), scr.data_ptr(),
-                           (size_t)scr.numel(), d3, d3 + 2 * M * h, d3 + 4 * M * h, dg.data_ptr(), db.data_ptr(),
-                           has_state ? dh0.data_ptr<float>() : nullptr, st),
+        must(kda_chunk_bwd(&sh, base + kept.q, base + kept.k, base + kept.v, base + kept.g, base + kept.beta, nullptr, tmp.at(t_do),
+                           dmem.defined() ? dmem.data_ptr<float>() : nullptr, base + kept.ws, kept.ws_bytes, scr, nb_chunk, dq, dq + act, dq + 2 * act,
+                           tmp.at(t_dg), tmp.at(t_db), has_state ? dh0.data_ptr<float>() : nullptr, st),
              "kda_chunk_bwd");
 
         // gate activations, then the low-rank gate projection
-        Tensor d_raw = empty_as(t[sRaw]), dA = empty({H}, at::kFloat, x), dbias = empty({h}, at::kFloat, x);
-        Tensor gscr = bytes(kda_gate_bwd_scratch_bytes((int32_t)M, (int32_t)H, (int32_t)kHead), x);
-        must(kda_gate_bwd_rows((int32_t)M, (int32_t)H, (int32_t)kHead, KDA_DTYPE_BF16, t[sRaw].data_ptr(), at_col(P, z.b()), (int32_t)z.n,
-                               (int32_t)z.pad, t[sA].data_ptr<float>(), t[sDt].data_ptr<float>(), (float)lb, dg.data_ptr<float>(),
-                               db.data_ptr<float>(), d_raw.data_ptr(), at_col(dP, z.b()), dA.data_ptr<float>(), dbias.data_ptr<float>(),
-                               gscr.data_ptr(), (size_t)gscr.numel(), st),
+        must(kda_gate_bwd_rows((int32_t)M, (int32_t)H, (int32_t)kHead, KDA_DTYPE_BF16, base + kept.raw, at_col(P, z.b()), (int32_t)n, (int32_t)z.pad,
+                               t[sA].data_ptr<float>(), t[sDt].data_ptr<float>(), (float)lb, tmp.f32(t_dg), tmp.f32(t_db), draw, at_col(dP, z.b()), dA,
+                               dbias, scr, nb_gate, st),
              "kda_gate_bwd_rows");
-        out[1 + kAlog] = dA;
-        out[1 + kDt] = dbias.view(dt_shape);
-        if (want(1 + kFb)) out[1 + kFb] = weight_grad(d_raw, P.narrow(1, z.fa(), kHead), wtype);
-        Tensor dfa = dP.narrow(1, z.fa(), kHead);
-        at::mm_out(dfa, d_raw, wfb);
+        out[1 + kAlog] = small.narrow(0, kHead, H);
+        out[1 + kDt] = small.narrow(0, kHead + H, h).view(dt_shape);
+        if (want(1 + kFb)) out[1 + kFb] = linear_dw(draw, h, at_col(P, z.fa()), n, M, h, kHead, wtype, x);
+        linear_dx(draw, h, packed_fb(pack, z), kHead, at_col(dP, z.fa()), n, M, h, kHead);
 
         // convolutions
-        Tensor dcw = empty({3, h, z.W}, at::kFloat, x);
+        const int io = KDA_DTYPE_BF16 | wflag(x, t[sCq]);
         const bool windows = has_state || grads[2].defined() || grads[3].defined() || grads[4].defined();
         if (!windows) {
             const void *xp[3], *wpt[3], *gp[3];
@@ -153,42 +194,47 @@ struct LayerNode : public HostNode {
             for (int i = 0; i < 3; ++i) {
                 xp[i] = at_col(P, i * h);
                 wpt[i] = t[sCq + i].data_ptr();
-                gp[i] = d3 + 2 * i * M * h;
+                gp[i] = dq + i * act;
                 dp[i] = at_col(dP, i * h);
-                wg[i] = dcw.data_ptr<float>() + i * h * z.W;
+                wg[i] = dcw + i * h * z.W;
             }
-            Tensor cscr = bytes(kda_conv_bwd_multi_scratch_bytes(3, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W), x);
-            must(kda_conv_bwd_rows(3, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, KDA_DTYPE_BF16 | wflag(x, t[sCq]), 1, xp, (int32_t)z.n,
-                                   wpt, gp, dp, wg, cscr.data_ptr(), (size_t)cscr.numel(), st),
+            must(kda_conv_bwd_rows(3, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xp, (int32_t)n, wpt, gp, dp, wg, scr, nb_conv, st),
                  "kda_conv_bwd_rows");
         } else {      // windows carried in or out: the general kernel, on dense copies
+            const size_t row = 2 * h;
+            Tensor xc = empty({M, h}, at::kBFloat16, x), dx = empty({M, h}, at::kBFloat16, x);
+            auto copy_rows = [&](void* dst, size_t dld, const void* src, size_t sld) {
+                TORCH_CHECK(cudaMemcpy2DAsync(dst, dld, src, sld, row, (size_t)M, cudaMemcpyDeviceToDevice, (cudaStream_t)st) == cudaSuccess,
+                            "copying a slice of the projection failed");
+            };
             for (int i = 0; i < 3; ++i) {
-                const Tensor xc = P.narrow(1, i * h, h).contiguous();
+                copy_rows(xc.data_ptr(), row, at_col(P, i * h), 2 * n);
                 const Tensor dfin = grads[2 + i].defined() ? dense_as(grads[2 + i], at::kBFloat16) : Tensor();
-                Tensor dx = empty({M, h}, at::kBFloat16, x), dinit;
+                Tensor dinit;
                 if (has_state) dinit = empty({z.B, h, z.W}, at::kBFloat16, x);
-                Tensor cscr = bytes(kda_conv_bwd_scratch_bytes((int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W), x);
-                must(kda_conv_bwd((int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, KDA_DTYPE_BF16 | wflag(x, t[sCq]), 1, xc.data_ptr(),
-                                  t[sCq + i].data_ptr(), has_state ? t[sWq + i].data_ptr() : nullptr, d3 + 2 * i * M * h,
-                                  dfin.defined() ? dfin.data_ptr() : nullptr, dx.data_ptr(), dcw.data_ptr<float>() + i * h * z.W,
-                                  has_state ? dinit.data_ptr() : nullptr, cscr.data_ptr(), (size_t)cscr.numel(), st),
+                must(kda_conv_bwd((int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xc.data_ptr(), t[sCq + i].data_ptr(),
+                                  has_state ? t[sWq + i].data_ptr() : nullptr, dq + i * act, dfin.defined() ? dfin.data_ptr() : nullptr,
+                                  dx.data_ptr(), dcw + i * h * z.W, has_state ? dinit.data_ptr() : nullptr, scr, nb_conv, st),
                      "kda_conv_bwd");
-                dP.narrow(1, i * h, h).copy_(dx);
+                copy_rows(at_col(dP, i * h), 2 * n, dx.data_ptr(), row);
                 if (has_state) out[16 + i] = stype[i] == at::kBFloat16 ? dinit : dinit.to(stype[i]);
             }
             if (has_state) out[15] = dh0;
         }
         for (int i = 0; i < 3; ++i) {
-            const Tensor d = dcw.select(0, i);
+            const Tensor d = small.narrow(0, kHead + H + h + i * h * z.W, h * z.W);
             out[1 + kCq + i] = (ctype == at::kFloat ? d : d.to(ctype)).view(cshape[i]);
         }
 
         // the input and the six weights of P
-        if (want(0)) out[0] = at::mm(dP, wp).view(x.sizes());
+        if (want(0)) {
+            out[0] = empty_as(x);
+            linear_dx(dP, n, pack, h, out[0].data_ptr(), h, M, n, h);
+        }
         bool any = false;
         for (int i = kQ; i <= kB; ++i) any = any || want(1 + i);
         if (any) {
-            const Tensor dW = weight_grad(dP, x2, wtype);
+            const Tensor dW = linear_dw(dP, n, x.data_ptr(), h, M, n, h, wtype, x);
             for (int i = kQ; i <= kG; ++i) out[1 + i] = dW.narrow(0, i * h, h);
             out[1 + kFa] = dW.narrow(0, z.fa(), kHead);
             out[1 + kB] = dW.narrow(0, z.b(), H);
@@ -233,6 +279,20 @@ bool layer_sizes(const Tensor& x, const std::vector<Tensor>& w, int64_t heads, c
     return !at::autocast::is_autocast_enabled(at::kCUDA);
 }
 
+constexpr int64_t kFewRows = 64;
+
+// products of at most kFewRows rows with `count` consecutive weights of the list, straight from the parameters
+void few_rows(const std::vector<Tensor>& w, int first, int count, const Sizes& z, const void* x, int64_t ldx, int64_t k, char* out, int64_t ldo,
+              const KdaTokenConv* conv, void* st) {
+    const void* wp[6];
+    int32_t rows[6];
+    for (int i = 0; i < count; ++i) {
+        wp[i] = w[first + i].data_ptr();
+        rows[i] = (int32_t)w[first + i].size(0);
+    }
+    must(kda_rows_linear((int32_t)z.M, (int32_t)k, count, dt(w[first]), x, ldx, wp, rows, out, ldo, conv, st), "kda_rows_linear");
+}
+
 using LayerResult = c10::optional<std::vector<c10::optional<Tensor>>>;
 
 // x [B,T,hidden], the parameters in the order above, state {memory, q, k, v windows} or empty
@@ -245,27 +305,21 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     for (const auto& t : w) tracked = tracked || torch::autograd::compute_requires_grad(t);
     for (const auto& t : state) tracked = tracked || torch::autograd::compute_requires_grad(t);
     fuse_conv = fuse_conv && !tracked && state.empty() && z.W == 4;
+    // without a backward, up to 64 rows go straight to the float32 masters (kda_rows_linear): nothing to pack
+    const bool few = !tracked && z.M <= kFewRows;
     c10::cuda::CUDAGuard guard(x_.device());
     watch_status(x_.device().index());
     void* st = stream_of(x_);
-    const int64_t h = z.hid, M = z.M;
-    Tensor x, P, raw, g, beta, qkv, o, mixed, inv, nw, y, ws, mem, win[3], cache[3], h0;
-    Packed pk;
+    const int64_t h = z.hid, M = z.M, n = z.n;
+    const KdaChunkShape sh = layer_shape(z, !tracked);
+    Kept kept(z, sh, tracked, !few, !fuse_conv);
+    Tensor x, nw, y, mem, win[3], cache[3], h0;
     {
         at::AutoDispatchBelowADInplaceOrView below;
         x = dense(x_);
-        pk = pack_weights(w, z);
         nw = dense_as(w[kNorm], at::kFloat);
-        P = at::mm(x.view({M, h}), pk.p.t());
-        raw = at::mm(P.narrow(1, z.fa(), kHead), pk.fb.t());
-        if (!fuse_conv) qkv = empty({3, M, h}, at::kBFloat16, x);
-        g = empty({M, h}, at::kFloat, x);
-        beta = empty({M, heads}, at::kFloat, x);
-        mixed = empty({M, h}, at::kBFloat16, x);
-        if (tracked) {
-            o = empty({z.B, z.T, heads, kHead}, at::kBFloat16, x);
-            inv = empty({M * heads}, at::kFloat, x);
-        }
+        kept.slab.make(x);
+        y = empty({z.B, z.T, h}, at::kBFloat16, x);
         if (want_state) {
             mem = empty({z.B, heads, kHead, kHead}, at::kFloat, x);
             for (auto& t : win) t = empty({z.B, h, z.W}, at::kBFloat16, x);
@@ -275,56 +329,64 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
             for (int i = 0; i < 3; ++i) cache[i] = dense_as(state[1 + i], at::kBFloat16);
         }
     }
+    const Slab& sl = kept.slab;
+    char *P = sl.at(kept.P), *raw = sl.at(kept.raw), *pack = sl.at(kept.pack);
+    if (few) {
+        few_rows(w, kQ, 6, z, x.data_ptr(), h, h, P, n, nullptr, st);
+        few_rows(w, kFb, 1, z, at_col(P, z.fa()), n, kHead, raw, h, nullptr, st);
+    } else {
+        pack_weights(w, z, pack, st);
+        linear(x.data_ptr(), h, pack, h, P, n, M, n, h);
+        linear(at_col(P, z.fa()), n, packed_fb(pack, z), kHead, raw, h, M, h, kHead);
+    }
     // convolutions on their slices of P: one launch; a call that carries windows issues them one by one
-    char* q3 = fuse_conv ? nullptr : static_cast<char*>(qkv.data_ptr());
+    const char* qkv[3] = {sl.at(kept.q), sl.at(kept.k), sl.at(kept.v)};
     if (!fuse_conv) {
         const void *xp[3], *wp[3], *cp[3];
         void *yp[3], *fp[3];
         for (int i = 0; i < 3; ++i) {
             xp[i] = at_col(P, i * h);
             wp[i] = w[kCq + i].data_ptr();
-            yp[i] = q3 + 2 * i * M * h;
+            yp[i] = const_cast<char*>(qkv[i]);
             cp[i] = cache[i].defined() ? cache[i].data_ptr() : nullptr;
             fp[i] = want_state ? win[i].data_ptr() : nullptr;
         }
         const int io = KDA_DTYPE_BF16 | wflag(x, w[kCq]), step = (want_state || !state.empty()) ? 1 : 3;
         for (int i = 0; i < 3; i += step)
-            must(kda_conv_fwd_rows(step, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xp + i, (int32_t)z.n, wp + i, cp + i, yp + i, fp + i, st),
+            must(kda_conv_fwd_rows(step, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xp + i, (int32_t)n, wp + i, cp + i, yp + i, fp + i, st),
                  "kda_conv_fwd_rows");
     }
-    must(kda_gate_fwd_rows((int32_t)M, (int32_t)heads, (int32_t)kHead, KDA_DTYPE_BF16, raw.data_ptr(), at_col(P, z.b()), (int32_t)z.n,
-                           w[kAlog].data_ptr<float>(), w[kDt].data_ptr<float>(), (float)lb, g.data_ptr<float>(), beta.data_ptr<float>(), st),
+    must(kda_gate_fwd_rows((int32_t)M, (int32_t)heads, (int32_t)kHead, KDA_DTYPE_BF16, raw, at_col(P, z.b()), (int32_t)n, w[kAlog].data_ptr<float>(),
+                           w[kDt].data_ptr<float>(), (float)lb, sl.f32(kept.g), sl.f32(kept.beta), st),
          "kda_gate_fwd_rows");
-    const KdaChunkShape sh = layer_shape(z, !tracked);
-    ws = bytes(kda_chunk_workspace_bytes(&sh), x);
     KdaChunkExtras ex = {};
     ex.gate = at_col(P, 3 * h);
-    ex.gate_ld = z.n;
+    ex.gate_ld = n;
     ex.norm_weight = nw.data_ptr<float>();
     ex.eps = (float)eps;
-    ex.y = mixed.data_ptr();
-    ex.inv_rms = tracked ? inv.data_ptr<float>() : nullptr;
-    const void *qp = q3, *kp = q3 ? q3 + 2 * M * h : nullptr, *vp = q3 ? q3 + 4 * M * h : nullptr;
+    ex.y = sl.at(kept.mixed);
+    ex.inv_rms = tracked ? sl.f32(kept.inv) : nullptr;
     if (fuse_conv) {
-        qp = at_col(P, 0), kp = at_col(P, h), vp = at_col(P, 2 * h);
-        for (int i = 0; i < 3; ++i) ex.conv_weight[i] = w[kCq + i].data_ptr();
+        for (int i = 0; i < 3; ++i) {
+            qkv[i] = at_col(P, i * h);
+            ex.conv_weight[i] = w[kCq + i].data_ptr();
+        }
         ex.conv_width = 4;
         ex.conv_weight_dtype = dt(w[kCq]);
-        ex.x_ld = z.n;
+        ex.x_ld = n;
     }
-    must(kda_chunk_fwd_ex(&sh, &ex, qp, kp, vp, g.data_ptr(), beta.data_ptr(), h0.defined() ? h0.data_ptr<float>() : nullptr, nullptr,
-                          tracked ? o.data_ptr() : nullptr, want_state ? mem.data_ptr<float>() : nullptr, ws.data_ptr(), (size_t)ws.numel(), st),
+    must(kda_chunk_fwd_ex(&sh, &ex, qkv[0], qkv[1], qkv[2], sl.at(kept.g), sl.at(kept.beta), h0.defined() ? h0.data_ptr<float>() : nullptr, nullptr,
+                          tracked ? sl.at(kept.o) : nullptr, want_state ? mem.data_ptr<float>() : nullptr, sl.at(kept.ws), kept.ws_bytes, st),
          "kda_chunk_fwd_ex");
-    {
+    if (few) few_rows(w, kO, 1, z, sl.at(kept.mixed), h, h, static_cast<char*>(y.data_ptr()), h, nullptr, st);
+    else linear(sl.at(kept.mixed), h, packed_o(pack, z), h, y.data_ptr(), h, M, h, h);
+    if (fuse_conv && want_state) {      // windows of the convolutions' inputs: the last W rows, zeros before the first
         at::AutoDispatchBelowADInplaceOrView below;
-        y = at::mm(mixed, pk.o.t()).view({z.B, z.T, h});
-        if (fuse_conv && want_state) {      // windows of the convolutions' inputs: the last W rows, zeros before the first
-            const int64_t keep = std::min<int64_t>(z.T, z.W);
-            for (int i = 0; i < 3; ++i) {
-                const Tensor tail = P.view({z.B, z.T, z.n}).narrow(1, z.T - keep, keep).narrow(2, i * h, h).transpose(1, 2);
-                if (keep < z.W) win[i].zero_();
-                win[i].narrow(2, z.W - keep, keep).copy_(tail);
-            }
+        const Tensor Pt = at::from_blob(P, {z.B, z.T, n}, x.options());
+        const int64_t keep = std::min<int64_t>(z.T, z.W);
+        for (int i = 0; i < 3; ++i) {
+            if (keep < z.W) win[i].zero_();
+            win[i].narrow(2, z.W - keep, keep).copy_(Pt.narrow(1, z.T - keep, keep).narrow(2, i * h, h).transpose(1, 2));
         }
     }
     if (tracked) {
@@ -345,10 +407,8 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         }
         node->dt_shape = w[kDt].sizes().vec();
         node->has_state = !state.empty();
-        const Tensor q = qkv.select(0, 0), k = qkv.select(0, 1), v = qkv.select(0, 2);
-        for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &w[kCq], &w[kCk], &w[kCv], &w[kAlog], &w[kDt], &nw, &pk.all, &P, &raw, &g, &beta, &q, &k,
-                                                                    &v, &ws, &o, &inv, &mixed})
-            node->keep(*t);
+        const Tensor all = kept.slab.tensor();
+        for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &w[kCq], &w[kCk], &w[kCv], &w[kAlog], &w[kDt], &nw, &all}) node->keep(*t);
         if (!state.empty())
             for (auto& t : cache) node->keep(t);
         torch::autograd::set_history(y, node);
@@ -359,12 +419,82 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     return std::vector<c10::optional<Tensor>>{y, mem, win[0], win[1], win[2]};
 }
 
+// ------------------------------------------------------------------------------------------------ one token
+// x [B,1,hidden] with B <= 64, no gradients.  in_place: three launches, the state tensors (windows bf16, dense) are
+// rewritten -> {y}; otherwise six, into new tensors -> {y, memory, q, k, v windows}.  Both give the same bits.
+LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads, double eps, double lb, const std::vector<Tensor>& state, bool in_place) {
+    Sizes z;
+    if (state.size() != 4 || !layer_sizes(x_, w, heads, state, z) || z.T != 1 || z.M > kFewRows || !(lb >= -5.0 && lb < 0.0)) return c10::nullopt;
+    if (in_place)
+        for (int i = 0; i < 4; ++i)
+            if (!state[i].is_contiguous() || (i > 0 && state[i].scalar_type() != at::kBFloat16)) return c10::nullopt;
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = dense(x_), nw = dense_as(w[kNorm], at::kFloat);
+    void* st = stream_of(x);
+    const int64_t h = z.hid, M = z.M, n = z.n;
+    const size_t act = 2 * (size_t)(M * h);
+    Slab tmp;
+    const size_t oP = tmp.take(2 * (size_t)(M * n)), oq = tmp.take(3 * act), omix = tmp.take(act), oraw = tmp.take(in_place ? 0 : act),
+                 oo = tmp.take(in_place ? 0 : act), oinv = tmp.take(in_place ? 0 : 4 * (size_t)(M * heads));
+    tmp.make(x);
+    Tensor y = empty({z.B, 1, h}, at::kBFloat16, x);
+    char *P = tmp.at(oP), *q = tmp.at(oq), *mixed = tmp.at(omix);
+    const float scale = (float)(1.0 / std::sqrt((double)kHead));
+    std::vector<c10::optional<Tensor>> out{y};
+    if (in_place) {
+        KdaTokenConv cv = {};
+        for (int i = 0; i < 3; ++i) {
+            cv.weight[i] = w[kCq + i].data_ptr();
+            cv.cache[i] = state[1 + i].data_ptr();
+        }
+        cv.act = q;
+        cv.width = (int32_t)z.W;
+        cv.weight_dtype = dt(w[kCq]);
+        few_rows(w, kQ, 6, z, x.data_ptr(), h, h, P, n, &cv, st);
+        must(kda_token_mix((int32_t)M, (int32_t)heads, scale, q, q + act, q + 2 * act, at_col(P, z.fa()), at_col(P, z.b()), at_col(P, 3 * h), n,
+                           w[kFb].data_ptr(), dt(w[kFb]), w[kAlog].data_ptr<float>(), w[kDt].data_ptr<float>(), (float)lb, nw.data_ptr<float>(),
+                           (float)eps, state[0].data_ptr<float>(), state[0].data_ptr<float>(), mixed, st),
+             "kda_token_mix");
+    } else {
+        const Tensor mem_in = dense(state[0]), mem = empty_as(mem_in);
+        out.push_back(mem);
+        const void *xp[3], *wp[3], *cp[3];
+        void *yp[3], *fp[3];
+        Tensor cache[3];
+        for (int i = 0; i < 3; ++i) {
+            cache[i] = dense_as(state[1 + i], at::kBFloat16);
+            const Tensor win = empty_as(cache[i]);
+            out.push_back(win);
+            xp[i] = at_col(P, i * h);
+            wp[i] = w[kCq + i].data_ptr();
+            yp[i] = q + i * act;
+            cp[i] = cache[i].data_ptr();
+            fp[i] = win.data_ptr();
+        }
+        few_rows(w, kQ, 6, z, x.data_ptr(), h, h, P, n, nullptr, st);
+        must(kda_conv_fwd_rows(3, (int32_t)z.B, 1, (int32_t)h, (int32_t)z.W, KDA_DTYPE_BF16 | wflag(x, w[kCq]), 1, xp, (int32_t)n, wp, cp, yp, fp, st),
+             "kda_conv_fwd_rows");
+        must(kda_narrow_linear((int32_t)M, (int32_t)h, dt(w[kFb]), at_col(P, z.fa()), n, w[kFb].data_ptr(), tmp.at(oraw), st), "kda_narrow_linear");
+        must(kda_decode_step_raw_rows((int32_t)M, (int32_t)heads, (int32_t)kHead, (int32_t)kHead, KDA_DTYPE_BF16, scale, q, q + act, q + 2 * act,
+                                      tmp.at(oraw), at_col(P, z.b()), n, w[kAlog].data_ptr<float>(), w[kDt].data_ptr<float>(), (float)lb,
+                                      mem_in.data_ptr<float>(), mem.data_ptr<float>(), tmp.at(oo), st),
+             "kda_decode_step_raw_rows");
+        must(kda_rmsnorm_gate_fwd_rows(M * heads, KDA_DTYPE_BF16, (int32_t)heads, (int32_t)n, (float)eps, tmp.at(oo), at_col(P, 3 * h),
+                                       nw.data_ptr<float>(), mixed, tmp.f32(oinv), st),
+             "kda_rmsnorm_gate_fwd_rows");
+    }
+    few_rows(w, kO, 1, z, mixed, h, h, static_cast<char*>(y.data_ptr()), h, nullptr, st);
+    return out;
+}
+
 }  // namespace
 
 void bind_layer(pybind11::module_& m) {
     namespace py = pybind11;
     using nogil = py::call_guard<py::gil_scoped_release>;
     m.def("layer", &layer, nogil());
+    m.def("token", &token, nogil());
 }
 
 }  // namespace kda_host

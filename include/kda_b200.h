@@ -215,6 +215,41 @@ int kda_decode_step_raw(int32_t n_seq, int32_t heads, int32_t key_dim, int32_t v
                         const float* A_log, const float* dt_bias, float lower_bound, const float* state_in, float* state_out,
                         void* o, void* stream);
 
+/* The same with the beta logits of consecutive sequences bl_ld elements apart. */
+int kda_decode_step_raw_rows(int32_t n_seq, int32_t heads, int32_t key_dim, int32_t value_dim, int32_t io_dtype, float scale,
+                             const void* q, const void* k, const void* v, const void* raw_gate, const void* beta_logits, int64_t bl_ld,
+                             const float* A_log, const float* dt_bias, float lower_bound, const float* state_in, float* state_out,
+                             void* o, void* stream);
+
+/* ---- a decode step of the whole layer --------------------------------------------
+ * Three calls make one token of a 128-wide-head layer (bf16 activations): kda_rows_linear on the input with the q, k, v
+ * (stepping the convolutions), output-gate, f_a and b projections; kda_token_mix; kda_rows_linear with the output
+ * projection.  The reference makes 8 Linear calls, 3 convolution calls, 1 decode and 1 norm call per token and layer
+ * (nanochat/mixers/kda.py:722-798).
+ *
+ * kda_rows_linear: out[m][row] = sum_k x[m][k] W[row][k] for m <= 64 rows of x and the rows of n_items (<= 6) dense bf16
+ * or float32 matrices (float32 is rounded to bf16 as it is read; float32 accumulation; one rounding to bf16), every matrix
+ * but the last a multiple of 16 rows, k a multiple of 32.  With conv the first three matrices are the q, k, v projections:
+ * their results go through one step of the short convolution + SiLU into conv->act [3][m][rows] instead, and the windows
+ * conv->cache [m][rows][width] are advanced in place.  weight, rows: HOST arrays.
+ * kda_narrow_linear: the same product for k = 128 with the arithmetic of kda_token_mix's prologue.
+ * kda_token_mix: raw gate = fa fb^T for the head, one decode step (as kda_decode_step_raw), gated RMSNorm of the head's
+ * output -> mixed [n_seq, heads*128].  fa, beta_logits and gate rows are ld elements apart. */
+typedef struct KdaTokenConv {
+    const void* weight[3];
+    void* cache[3];
+    void* act;
+    int32_t width;
+    int32_t weight_dtype;
+} KdaTokenConv;
+int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t weight_dtype, const void* x, int64_t x_ld, const void* const* weight,
+                    const int32_t* rows, void* out, int64_t out_ld, const KdaTokenConv* conv, void* stream);
+int kda_narrow_linear(int32_t m, int32_t n, int32_t weight_dtype, const void* x, int64_t x_ld, const void* weight, void* out, void* stream);
+int kda_token_mix(int32_t n_seq, int32_t heads, float scale, const void* q, const void* k, const void* v, const void* fa,
+                  const void* beta_logits, const void* gate, int64_t ld, const void* fb_weight, int32_t fb_dtype, const float* A_log,
+                  const float* dt_bias, float lower_bound, const float* norm_weight, float eps, const float* state_in,
+                  float* state_out, void* mixed, void* stream);
+
 /* n_steps consecutive decode steps in one call: step i reads q,k,g [n_steps,n_seq,H,K], v [n_steps,n_seq,H,V],
  * beta [n_steps,n_seq,H] at index i, updates `state` in place and writes o[i].  One kernel launch per step (the state
  * crosses HBM once each way per step, exactly as n_steps calls of kda_decode_step would), without a host round trip
@@ -284,6 +319,8 @@ int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype, const void
                          float* dweight, void* scratch, size_t scratch_bytes, void* stream);
 
 /* dim = 128 with gate and dgate in rows of `heads` norms, gate_ld elements (a multiple of 8) apart. */
+int kda_rmsnorm_gate_fwd_rows(int64_t rows, int32_t io_dtype, int32_t heads, int32_t gate_ld, float eps, const void* x,
+                              const void* gate, const float* weight, void* y, float* inv_rms, void* stream);
 int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t heads, int32_t gate_ld, const void* x, const void* gate,
                               const float* weight, const float* inv_rms, const void* d_y, void* dx, void* dgate,
                               float* dweight, void* scratch, size_t scratch_bytes, void* stream);
