@@ -179,7 +179,7 @@ struct TokenMix {
 };
 
 template <int NV4, int R, int NW, bool FUSED>
-__global__ void __launch_bounds__(NW * 32) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
+__global__ void __launch_bounds__(NW * 32, FUSED && NW == 8 ? 4 : 1) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
                                                      const void* __restrict__ q, const void* __restrict__ k,
                                                      const void* __restrict__ v, const void* __restrict__ g,
                                                      const void* __restrict__ beta, const float* s_in, float* s_out,
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(NW * 32) decode_kernel(int H, int K, int V, in
         const int hh = bh % H;
         float xv[4];
         narrow_x(mix.fa + (size_t)(bh / H) * mix.ld, lane, xv);
-        constexpr int PER = 128 / NW, G = PER < 8 ? PER : 8;       // gate rows per warp, G weight rows in flight
+        constexpr int PER = 128 / NW, G = 4;                        // gate rows per warp, G weight rows in flight
 #pragma unroll 1
         for (int i0 = 0; i0 < PER; i0 += G) {
             float wv[G][4], y[G];

@@ -5,8 +5,9 @@
 // copy, and several weight matrices with a common input share the launch.  A CTA owns 16 weight rows; its eight warps split
 // k in interleaved 32-wide steps, so a row is read as contiguous kilobytes and about 100 KB per SM are in flight.  The
 // contraction runs on mma.sync m16n8k16 with the weights as the 16-row operand (a tcgen05 tile would need the weights
-// staged in shared memory as bf16 first, which is the copy this kernel avoids); k is permuted inside a step so that each
-// lane's operands are 32 (weights) and 16 (x) contiguous bytes.  Partial sums meet in shared memory in a fixed order: a
+// staged in shared memory as bf16 first, which is the copy this kernel avoids); k is permuted inside a step so that
+// every 16-byte piece of a lane lies next to its neighbours' (a quad covers 64 contiguous bytes of a row; two 16-byte
+// halves of a 32-byte sector in different copies would fetch it twice).  Partial sums meet in shared memory in a fixed order: a
 // result depends on its row of x and of w alone, not on how many rows the call has.
 
 #include "common.cuh"
@@ -41,109 +42,138 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// NT: 8-row tiles of x.  U: steps whose loads are issued together.
-template <int NT, bool F32W, bool CONV, int U>
+// NT: 8-row tiles of x.  RT: 16-row tiles of weights per CTA; two halve the reads of x (every CTA reads all of it) where
+// there are enough rows to give every SM a CTA all the same.
+// Weights arrive through a thread-private ring in shared memory filled by 16-byte asynchronous copies, 96 KB per CTA in
+// flight and no registers held for it (register-staged loads reached 2.3 TB/s at 2,048 x 8,336 and 32 rows, 68 MB of
+// masters); x, which L2 serves, is loaded one step ahead.
+template <int RT>
+constexpr int kDepth = RT == 1 ? 6 : 3;
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+template <int NT, bool F32W, bool CONV, int RT>
 __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
-    __shared__ float red[kWarps][kRows][NT * 8 + 1];
+    constexpr int D = kDepth<RT>, PIECES = F32W ? 4 : 2, NTH = kWarps * 32, ROWS = kRows * RT, LD = NT * 8 + 1;
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint4* ring = reinterpret_cast<uint4*>(smem);                    // [D][RT][PIECES][threads]
+    float* red = reinterpret_cast<float*>(smem);                     // [warps][ROWS][LD], once the ring is drained
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int row0 = blockIdx.x * kRows;
-    int item = 0, begin = 0;
+    const int row0 = blockIdx.x * ROWS;
+    const uint8_t* src[RT][2];                                       // rows g and g + 8 of each tile; past the end: the last row
+    constexpr int ES = F32W ? 4 : 2;
 #pragma unroll
-    for (int i = 1; i < kItems; ++i)
-        if (i < p.n_items && row0 >= p.end[i - 1]) {
-            item = i;
-            begin = p.end[i - 1];
-        }
-    int end = p.end[0];
-    const void* w = p.w[0];
+    for (int r = 0; r < RT; ++r)
 #pragma unroll
-    for (int i = 1; i < kItems; ++i)
-        if (i == item) {
-            end = p.end[i];
-            w = p.w[i];
-        }
-    const int lo = min(row0 + g, end - 1) - begin, hi = min(row0 + g + 8, end - 1) - begin;      // rows past the end repeat the last one
-    const size_t olo = (size_t)lo * p.k + 8 * tig, ohi = (size_t)hi * p.k + 8 * tig;
-    float acc[NT][4];
+        for (int hf = 0; hf < 2; ++hf) {
+            int row = min(row0 + 16 * r + 8 * hf + g, p.end[p.n_items - 1] - 1), begin = 0;
+            const void* w = p.w[0];
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
-    const int steps = p.k / kStep;
-    for (int s0 = warp; s0 < steps; s0 += kWarps * U) {
-        uint4 a[U][2];                             // bf16 weights: 8 of each row
-        uint4 xb[U][NT];
-        if (F32W) {
-            float4 f[U][4];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int s = s0 + kWarps * u;
-                if (s < steps) {
-                    const float4* pl = reinterpret_cast<const float4*>(static_cast<const float*>(w) + olo + (size_t)s * kStep);
-                    const float4* ph = reinterpret_cast<const float4*>(static_cast<const float*>(w) + ohi + (size_t)s * kStep);
-                    f[u][0] = __ldg(pl); f[u][1] = __ldg(pl + 1);
-                    f[u][2] = __ldg(ph); f[u][3] = __ldg(ph + 1);
+            for (int i = 1; i < kItems; ++i)
+                if (i < p.n_items && row >= p.end[i - 1]) {
+                    begin = p.end[i - 1];
+                    w = p.w[i];
                 }
-            }
+            src[r][hf] = static_cast<const uint8_t*>(w) + (size_t)(row - begin) * p.k * ES + 16 * tig;
+        }
+    const int steps = p.k / kStep, mine = steps > warp ? (steps - warp + kWarps - 1) / kWarps : 0;      // steps warp, warp + 8, ...
+    const uint32_t slot = (uint32_t)__cvta_generic_to_shared(ring + threadIdx.x);
+    auto issue = [&](int i) {
+        if (i < mine) {
+            const size_t off = (size_t)(warp + kWarps * i) * kStep * ES;
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int r = 0; r < RT; ++r)
 #pragma unroll
-                for (int r = 0; r < 2; ++r)
-                    a[u][r] = make_uint4(pk(f[u][2 * r].x, f[u][2 * r].y), pk(f[u][2 * r].z, f[u][2 * r].w),
-                                         pk(f[u][2 * r + 1].x, f[u][2 * r + 1].y), pk(f[u][2 * r + 1].z, f[u][2 * r + 1].w));
-        } else {
+                for (int q = 0; q < PIECES; ++q)
+                    cp16(slot + (uint32_t)((((i % D) * RT + r) * PIECES + q) * NTH) * 16u, src[r][q / (PIECES / 2)] + off + (q % (PIECES / 2)) * 64);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint4 xb[NT];
+    auto load_x = [&](int i) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int s = s0 + kWarps * u;
-                if (s < steps) {
-                    a[u][0] = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(w) + olo + (size_t)s * kStep));
-                    a[u][1] = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(w) + ohi + (size_t)s * kStep));
+        for (int t = 0; t < NT; ++t) {
+            xb[t] = make_uint4(0, 0, 0, 0);
+            if (i < mine && t * 8 + g < p.m) {
+                const __nv_bfloat16* xr = p.x + (size_t)(t * 8 + g) * p.ldx + (size_t)(warp + kWarps * i) * kStep;
+                if (F32W) {
+                    const uint2 u = __ldg(reinterpret_cast<const uint2*>(xr + 4 * tig)), v = __ldg(reinterpret_cast<const uint2*>(xr + 16 + 4 * tig));
+                    xb[t] = make_uint4(u.x, u.y, v.x, v.y);
+                } else {
+                    xb[t] = __ldg(reinterpret_cast<const uint4*>(xr + 8 * tig));
                 }
             }
         }
+    };
+    float acc[RT][NT][4];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int s = s0 + kWarps * u;
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[r][t][e] = 0.f;
+#pragma unroll
+    for (int i = 0; i < D - 1; ++i) issue(i);
+    load_x(0);
+#pragma unroll 1
+    for (int i = 0; i < mine; ++i) {
+        issue(i + D - 1);
+        uint4 xc[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) xc[t] = xb[t];
+        load_x(i + 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+            uint4 a[2];                             // 8 bf16 of rows g and g + 8
+            const uint4* mem = ring + (((i % D) * RT + r) * PIECES) * NTH + threadIdx.x;
+            if (F32W) {
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const float4 u = *reinterpret_cast<const float4*>(mem + (2 * hf) * NTH), v = *reinterpret_cast<const float4*>(mem + (2 * hf + 1) * NTH);
+                    a[hf] = make_uint4(pk(u.x, u.y), pk(u.z, u.w), pk(v.x, v.y), pk(v.z, v.w));
+                }
+            } else {
+                a[0] = mem[0];
+                a[1] = mem[NTH];
+            }
+            const uint32_t a0[4] = {a[0].x, a[1].x, a[0].y, a[1].y}, a1[4] = {a[0].z, a[1].z, a[0].w, a[1].w};
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-                xb[u][t] = make_uint4(0, 0, 0, 0);
-                if (s < steps && t * 8 + g < p.m)
-                    xb[u][t] = __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)(t * 8 + g) * p.ldx + (size_t)s * kStep + 8 * tig));
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (s0 + kWarps * u < steps) {
-                const uint32_t a0[4] = {a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y}, a1[4] = {a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w};
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    mma_bf16(acc[t], a0, xb[u][t].x, xb[u][t].y);
-                    mma_bf16(acc[t], a1, xb[u][t].z, xb[u][t].w);
-                }
+                mma_bf16(acc[r][t], a0, xc[t].x, xc[t].y);
+                mma_bf16(acc[r][t], a1, xc[t].z, xc[t].w);
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                                 // every warp has drained its ring: the memory becomes the partials
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        red[warp][g][t * 8 + 2 * tig] = acc[t][0];
-        red[warp][g][t * 8 + 2 * tig + 1] = acc[t][1];
-        red[warp][g + 8][t * 8 + 2 * tig] = acc[t][2];
-        red[warp][g + 8][t * 8 + 2 * tig + 1] = acc[t][3];
-    }
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            float* d = red + (size_t)(warp * ROWS + 16 * r + g) * LD + t * 8 + 2 * tig;
+            d[0] = acc[r][t][0];
+            d[1] = acc[r][t][1];
+            d[8 * LD] = acc[r][t][2];
+            d[8 * LD + 1] = acc[r][t][3];
+        }
     __syncthreads();
-    for (int i = threadIdx.x; i < kRows * p.m; i += kWarps * 32) {
-        const int r = i & (kRows - 1), m = i / kRows;
-        if (row0 + r >= end) continue;
+    for (int i = threadIdx.x; i < ROWS * p.m; i += NTH) {
+        const int r = i % ROWS, m = i / ROWS, row = row0 + r;
+        if (row >= p.end[p.n_items - 1]) continue;
         float y = 0.f;
 #pragma unroll
-        for (int k = 0; k < kWarps; ++k) y += red[k][r][m];
+        for (int k = 0; k < kWarps; ++k) y += red[(size_t)(k * ROWS + r) * LD + m];
         const __nv_bfloat16 yb = __float2bfloat16(y);
-        if (CONV && item < 3) {
+        if (CONV && row < p.end[2]) {
             // one token of the short convolution + SiLU, the arithmetic of the stand-alone step: the window drops its oldest
             // value and takes y; the cache is rewritten in place
+            const int item = row < p.end[0] ? 0 : (row < p.end[1] ? 1 : 2);
             void* cache = item == 0 ? p.cache[0] : (item == 1 ? p.cache[1] : p.cache[2]);
             const void* cw = item == 0 ? p.conv_w[0] : (item == 1 ? p.conv_w[1] : p.conv_w[2]);
-            const int C = end - begin, c = row0 + r - begin;
+            const int C = p.end[0], c = row - item * C;      // the three have the same channels
             const size_t base = ((size_t)m * C + c) * p.width;
             float z = 0.f;
             for (int j = 0; j < p.width; ++j) {
@@ -158,19 +188,27 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
             asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(0.5f * z));
             p.act[((size_t)item * p.m + m) * C + c] = __float2bfloat16(z * fmaf(0.5f, th, 0.5f));
         } else {
-            p.out[(size_t)m * p.ldo + row0 + r] = yb;
+            p.out[(size_t)m * p.ldo + row] = yb;
         }
     }
 }
 
+template <int NT, bool F32W, bool CONV, int RT>
+int launch_tile(const RowsArgs& p, cudaStream_t st) {
+    constexpr size_t ring = (size_t)kDepth<RT> * RT * (F32W ? 4 : 2) * kWarps * 32 * 16, red = (size_t)kWarps * kRows * RT * (NT * 8 + 1) * 4;
+    constexpr size_t bytes = ring > red ? ring : red;
+    if (set_smem_limit(rows_kernel<NT, F32W, CONV, RT>, bytes)) return KDA_ERR_CUDA;
+    KDA_LAUNCH("rows_kernel", st, rows_kernel<NT, F32W, CONV, RT><<<ceil_div(p.end[p.n_items - 1], kRows * RT), kWarps * 32, bytes, st>>>(p));
+    return launch_status();
+}
+
 template <bool F32W, bool CONV>
 int launch_rows(const RowsArgs& p, cudaStream_t st) {
-    const int blocks = ceil_div(p.end[p.n_items - 1], kRows);
-    if (p.m <= 8) KDA_LAUNCH("rows_kernel", st, rows_kernel<1, F32W, CONV, 4><<<blocks, kWarps * 32, 0, st>>>(p));
-    else if (p.m <= 16) KDA_LAUNCH("rows_kernel", st, rows_kernel<2, F32W, CONV, 4><<<blocks, kWarps * 32, 0, st>>>(p));
-    else if (p.m <= 32) KDA_LAUNCH("rows_kernel", st, rows_kernel<4, F32W, CONV, 2><<<blocks, kWarps * 32, 0, st>>>(p));
-    else KDA_LAUNCH("rows_kernel", st, rows_kernel<8, F32W, CONV, 2><<<blocks, kWarps * 32, 0, st>>>(p));
-    return launch_status();
+    const bool wide = p.end[p.n_items - 1] >= 148 * kRows * 2;       // at least one CTA of two tiles for every SM
+    if (p.m <= 8) return wide ? launch_tile<1, F32W, CONV, 2>(p, st) : launch_tile<1, F32W, CONV, 1>(p, st);
+    if (p.m <= 16) return wide ? launch_tile<2, F32W, CONV, 2>(p, st) : launch_tile<2, F32W, CONV, 1>(p, st);
+    if (p.m <= 32) return wide ? launch_tile<4, F32W, CONV, 2>(p, st) : launch_tile<4, F32W, CONV, 1>(p, st);
+    return wide ? launch_tile<8, F32W, CONV, 2>(p, st) : launch_tile<8, F32W, CONV, 1>(p, st);
 }
 
 // y[m][n] for one 128-wide product (the low-rank gate projection), a warp per (row of x, weight row): the form the decode
@@ -208,8 +246,7 @@ extern "C" int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t we
     int end = 0;
     for (int i = 0; i < n_items; ++i) {
         if (!weight[i]) return KDA_ERR_NULL;
-        // a 16-row group belongs to one matrix: every matrix but the last fills its groups
-        if (rows[i] < 1 || (i + 1 < n_items && rows[i] % tok::kRows != 0)) return KDA_ERR_UNSUPPORTED;
+        if (rows[i] < 1) return KDA_ERR_BAD_SHAPE;
         end += rows[i];
         p.w[i] = weight[i];
         p.end[i] = end;
@@ -219,7 +256,7 @@ extern "C" int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t we
     cudaStream_t st = (cudaStream_t)stream;
     const bool f32 = weight_dtype == KDA_DTYPE_F32;
     if (!conv) return f32 ? tok::launch_rows<true, false>(p, st) : tok::launch_rows<false, false>(p, st);
-    if (n_items < 3 || conv->width < 1 || conv->width > 4 || !conv->act) return KDA_ERR_BAD_SHAPE;
+    if (n_items < 3 || rows[1] != rows[0] || rows[2] != rows[0] || conv->width < 1 || conv->width > 4 || !conv->act) return KDA_ERR_BAD_SHAPE;
     for (int i = 0; i < 3; ++i) {
         if (!conv->weight[i] || !conv->cache[i]) return KDA_ERR_NULL;
         p.conv_w[i] = conv->weight[i];

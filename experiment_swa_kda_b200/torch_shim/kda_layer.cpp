@@ -48,6 +48,14 @@ void pack_weights(const std::vector<Tensor>& w, const Sizes& z, char* pack, void
     must(kda_pack_bf16(9, dt(w[kQ]), src, elems, pack, st), "kda_pack_bf16");
 }
 
+// cuBLAS wants a context on the calling thread; an engine thread that has made no runtime call yet has none
+void bind_context(int device) {
+    thread_local int bound = -1;
+    if (bound == device) return;
+    TORCH_CHECK(cudaSetDevice(device) == cudaSuccess, "cudaSetDevice failed");
+    bound = device;
+}
+
 // Row-major products with row strides, bf16 operands and float32 accumulation.  cuBLAS directly: at::mm spends as long in
 // dispatch and views as the call itself takes, and these operands are slices.
 void gemm(cublasOperation_t ta, cublasOperation_t tb, int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, const void* b, int64_t ldb,
@@ -131,6 +139,7 @@ struct LayerNode : public HostNode {
         at::AutoDispatchBelowADInplaceOrView below;
         const Tensor& x = t[sX];
         c10::cuda::CUDAGuard guard(x.device());
+        bind_context(x.device().index());
         watch_status(x.device().index());
         void* st = stream_of(x);
         const int64_t h = z.hid, M = z.M, H = z.H, n = z.n;

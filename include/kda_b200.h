@@ -228,8 +228,8 @@ int kda_decode_step_raw_rows(int32_t n_seq, int32_t heads, int32_t key_dim, int3
  * (nanochat/mixers/kda.py:722-798).
  *
  * kda_rows_linear: out[m][row] = sum_k x[m][k] W[row][k] for m <= 64 rows of x and the rows of n_items (<= 6) dense bf16
- * or float32 matrices (float32 is rounded to bf16 as it is read; float32 accumulation; one rounding to bf16), every matrix
- * but the last a multiple of 16 rows, k a multiple of 32.  With conv the first three matrices are the q, k, v projections:
+ * or float32 matrices (float32 is rounded to bf16 as it is read; float32 accumulation; one rounding to bf16), k a
+ * multiple of 32.  With conv the first three matrices are the q, k, v projections:
  * their results go through one step of the short convolution + SiLU into conv->act [3][m][rows] instead, and the windows
  * conv->cache [m][rows][width] are advanced in place.  weight, rows: HOST arrays.
  * kda_narrow_linear: the same product for k = 128 with the arithmetic of kda_token_mix's prologue.
