@@ -1,18 +1,23 @@
 // Chunked KDA forward and backward in float32 on the CUDA cores ("fp32 lane").
 //
-// General shapes: any K, V <= 256, any sequence length, packed sequences,
-// initial / final state.  Every matrix of the chunked WY algebra is handled as
-// 64x64 float32 tiles staged in shared memory; rows beyond a ragged chunk tail
-// and columns beyond K / V are zero, which makes them inert in every product
-// (zero q, k, v, beta and log-decay rows leave A, M, T, U, W, Z and all adjoints
-// unchanged for the valid rows).
+// General shapes: any K, V <= 256, any sequence length, packed sequences, initial / final state.  Every matrix of the
+// chunked WY algebra is handled as 64x64 float32 tiles staged in shared memory; rows beyond a ragged chunk tail and
+// columns beyond K / V are zero, which makes them inert in every product.
 //
 // Per chunk (64 tokens of one sequence and head), H = incoming state [K,V]:
 //   G = cumsum(g);  A = tril(sum_d qn kn rho);  M = beta * stril(sum_d kn kn rho), rho = exp(G_i - G_s)
 //   T = (I + M)^-1;  U = T (beta v);  W = T (beta exp(G) kn);  Z = U - W H
-//   O = (qn exp(G)) H + A Z;  H' = exp(G_end) H + (kn exp(G_end - G))^T Z
+//   O = R H + A Z, R = qn exp(G);  H' = exp(G_end) H + E^T Z, E = kn exp(G_end - G)
+// Substituting Z, the recurrence is affine in H with coefficients that do not depend on it:
+//   H' = exp(G_end) . H - (E^T W) H + E^T U        dH = exp(G_end) . dH' - (E^T W)^T dH' + (R - A W)^T dO
+// so everything but one K x K product per step is formed for all chunks side by side, and the scans carry a quarter of
+// the work they would with Z inside: at K = V = 64 and 32 chunks 303 + 533 us became 17 + 17.
 // The equations restate reference chunk_wy_forward.cu:125-405, 761-858, 940-1275, 1498-1588
 // and, for the adjoints, chunk_wy_backward.cu:2445-2562, 2818-3331, 3337-3552, 3787-3894.
+//
+// Products are 64^3 tiles on 256 threads, 4 x 4 outputs each: two 16-byte shared loads per 16 multiply-adds, both of them
+// broadcast or conflict-free, so a tile is bound by the float32 pipe.  The left operand is stored with the contraction
+// index leading ("At"), the right one naturally.
 
 #include <cstdlib>
 
@@ -23,36 +28,69 @@
 namespace kda {
 namespace simt {
 
+constexpr int kTile = 64 * kLD;      // floats of one shared tile
+
 // ---------------------------------------------------------------------------------------------
 // tile helpers (256 threads)
 // ---------------------------------------------------------------------------------------------
-
-// 64x64 tile from a padded float32 array (row stride ld_src floats, 16-byte aligned).
-template <bool TR>
-__device__ __forceinline__ void ld_tile(float* dst, const float* __restrict__ src, size_t ld_src) {
-    for (int idx = threadIdx.x; idx < 1024; idx += 256) {
-        int r = idx >> 4, c4 = (idx & 15) << 2;
-        float4 x = *reinterpret_cast<const float4*>(src + (size_t)r * ld_src + c4);
-        if (!TR) {
-            *reinterpret_cast<float4*>(dst + r * kLD + c4) = x;
-        } else {
-            dst[(c4 + 0) * kLD + r] = x.x;
-            dst[(c4 + 1) * kLD + r] = x.y;
-            dst[(c4 + 2) * kLD + r] = x.z;
-            dst[(c4 + 3) * kLD + r] = x.w;
-        }
+__device__ __forceinline__ void ld_nat(float* dst, const float* __restrict__ src, size_t ld) {
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = threadIdx.x + 256 * it, r = idx >> 4, c4 = (idx & 15) << 2;
+        *reinterpret_cast<float4*>(dst + r * kLD + c4) = *reinterpret_cast<const float4*>(src + (size_t)r * ld + c4);
     }
 }
-
-// 64x64 tile from a caller tensor in its I/O dtype; element (r,c) at base[r*stride + c]; zero outside nr x nc.
+// transposed: lanes run down the rows, so the four scalar stores of a lane are conflict-free (the 64-byte pieces of a row
+// that a warp leaves behind are served by L1 in the next iterations)
+__device__ __forceinline__ void ld_tr(float* dst, const float* __restrict__ src, size_t ld) {
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = threadIdx.x + 256 * it, r = idx & 63, c4 = (idx >> 6) << 2;
+        const float4 x = *reinterpret_cast<const float4*>(src + (size_t)r * ld + c4);
+        dst[(c4 + 0) * kLD + r] = x.x;
+        dst[(c4 + 1) * kLD + r] = x.y;
+        dst[(c4 + 2) * kLD + r] = x.z;
+        dst[(c4 + 3) * kLD + r] = x.w;
+    }
+}
+// four adjacent elements of a caller tensor, zero outside nr x nc; vec: the tensor allows 4-element accesses
+__device__ __forceinline__ void ld4_io(float (&x)[4], const void* base, int bf16, size_t off, size_t stride, int r, int c4, int nr, int nc, int vec) {
+    const size_t i = off + (size_t)r * stride + c4;
+    if (r >= nr || c4 >= nc) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = 0.f;
+    } else if (vec && c4 + 4 <= nc) {
+        if (bf16) {
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(base) + i));
+            const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+            const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+            x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+        } else {
+            const float4 f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + i));
+            x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = c4 + e < nc ? ld_io(base, i + e, bf16) : 0.f;
+    }
+}
+// 64x64 tile of a caller tensor, each element times scale[row] when scale is given
 template <bool TR>
-__device__ __forceinline__ void ld_tile_io(float* dst, const void* base, int bf16, size_t off, size_t stride, int nr,
-                                           int nc) {
-    for (int idx = threadIdx.x; idx < 4096; idx += 256) {
-        int r = idx >> 6, c = idx & 63;
-        float x = (r < nr && c < nc) ? ld_io(base, off + (size_t)r * stride + c, bf16) : 0.0f;
-        if (!TR) dst[r * kLD + c] = x;
-        else dst[c * kLD + r] = x;
+__device__ __forceinline__ void ld_tile_io(float* dst, const void* base, int bf16, size_t off, size_t stride, int nr, int nc, int vec,
+                                           const float* scale = nullptr) {
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = threadIdx.x + 256 * it;
+        const int r = TR ? idx & 63 : idx >> 4, c4 = (TR ? idx >> 6 : idx & 15) << 2;
+        float x[4];
+        ld4_io(x, base, bf16, off, stride, r, c4, nr, nc, vec);
+        const float s = scale ? scale[r] : 1.f;
+        if (TR) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dst[(c4 + e) * kLD + r] = x[e] * s;
+        } else {
+            *reinterpret_cast<float4*>(dst + r * kLD + c4) = make_float4(x[0] * s, x[1] * s, x[2] * s, x[3] * s);
+        }
     }
 }
 
@@ -62,44 +100,48 @@ __device__ __forceinline__ void zero_acc(float (&acc)[4][4]) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[r][c] = 0.0f;
 }
+__device__ __forceinline__ void fma16(float (&acc)[4][4], const float4& a, const float4& b) {
+    acc[0][0] += a.x * b.x; acc[0][1] += a.x * b.y; acc[0][2] += a.x * b.z; acc[0][3] += a.x * b.w;
+    acc[1][0] += a.y * b.x; acc[1][1] += a.y * b.y; acc[1][2] += a.y * b.z; acc[1][3] += a.y * b.w;
+    acc[2][0] += a.z * b.x; acc[2][1] += a.z * b.y; acc[2][2] += a.z * b.z; acc[2][3] += a.z * b.w;
+    acc[3][0] += a.w * b.x; acc[3][1] += a.w * b.y; acc[3][2] += a.w * b.z; acc[3][3] += a.w * b.w;
+}
+// acc[r][c] += sum_{kk < n} ap[kk * lda + r] * bp[kk * ldb + c]: ap, bp already at the thread's rows / columns
+__device__ __forceinline__ void mm_at(float (&acc)[4][4], const float* ap, int lda, const float* bp, int ldb, int n) {
+#pragma unroll 8
+    for (int kk = 0; kk < n; ++kk)
+        fma16(acc, *reinterpret_cast<const float4*>(ap + kk * lda), *reinterpret_cast<const float4*>(bp + kk * ldb));
+}
+__device__ __forceinline__ void mm64(float (&acc)[4][4], const float* At, const float* Bs) {
+    mm_at(acc, At + 4 * (threadIdx.x >> 4), kLD, Bs + 4 * (threadIdx.x & 15), kLD, 64);
+}
 
-// acc[r][c] += sum_kk At[kk][4*ty + r] * Bs[kk][4*tx + c]   (At holds the left operand transposed)
-__device__ __forceinline__ void mm64(float (&acc)[4][4], const float* __restrict__ At, const float* __restrict__ Bs,
-                                     int kk0 = 0, int kk1 = 64) {
+// the thread's 4x4 patch -> shared or global rows, naturally or transposed (16-byte stores either way)
+__device__ __forceinline__ void st_nat(float* dst, size_t ld, const float (&acc)[4][4]) {
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const float* ap = At + 4 * ty;
-    const float* bp = Bs + 4 * tx;
-#pragma unroll 4
-    for (int kk = kk0; kk < kk1; ++kk) {
-        float4 a = *reinterpret_cast<const float4*>(ap + kk * kLD);
-        float4 b = *reinterpret_cast<const float4*>(bp + kk * kLD);
-        acc[0][0] += a.x * b.x; acc[0][1] += a.x * b.y; acc[0][2] += a.x * b.z; acc[0][3] += a.x * b.w;
-        acc[1][0] += a.y * b.x; acc[1][1] += a.y * b.y; acc[1][2] += a.y * b.z; acc[1][3] += a.y * b.w;
-        acc[2][0] += a.z * b.x; acc[2][1] += a.z * b.y; acc[2][2] += a.z * b.z; acc[2][3] += a.z * b.w;
-        acc[3][0] += a.w * b.x; acc[3][1] += a.w * b.y; acc[3][2] += a.w * b.z; acc[3][3] += a.w * b.w;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        *reinterpret_cast<float4*>(dst + (size_t)(4 * ty + r) * ld + 4 * tx) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+}
+__device__ __forceinline__ void st_tr(float* dst, size_t ld, const float (&acc)[4][4]) {
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<float4*>(dst + (size_t)(4 * tx + c) * ld + 4 * ty) = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
+}
+__device__ __forceinline__ void ld_patch(float (&x)[4][4], const float* src, size_t ld) {
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const float4 f = *reinterpret_cast<const float4*>(src + (size_t)(4 * ty + r) * ld + 4 * tx);
+        x[r][0] = f.x; x[r][1] = f.y; x[r][2] = f.z; x[r][3] = f.w;
     }
 }
-
-// registers -> shared tile, row-major or transposed
-template <bool TR>
-__device__ __forceinline__ void st_acc(float* dst, const float (&acc)[4][4], float alpha = 1.0f) {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+// sum over the 16 lanes that share a patch row
+__device__ __forceinline__ float row_sum16(float x) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (!TR) dst[(4 * ty + r) * kLD + 4 * tx + c] = alpha * acc[r][c];
-            else dst[(4 * tx + c) * kLD + 4 * ty + r] = alpha * acc[r][c];
-        }
-}
-
-// registers -> padded float32 global tile
-__device__ __forceinline__ void st_acc_g(float* dst, size_t ld, const float (&acc)[4][4]) {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-        *reinterpret_cast<float4*>(dst + (size_t)(4 * ty + r) * ld + 4 * tx) =
-            make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -172,336 +214,532 @@ __global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_s
 }
 
 // ---------------------------------------------------------------------------------------------
-// K1  prep: normalise q, k; cumulative log-decay; padded float32 copies
+// T = (I + M)^-1
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) prep_kernel(Ws w, const void* __restrict__ q, const void* __restrict__ k,
-                                                   const void* __restrict__ g, const void* __restrict__ beta, int bf16,
-                                                   int gbf16, int l2norm, float scale) {
-    const int slot = blockIdx.x, h = blockIdx.y;
-    const int len = w.chunk_len[slot];
-    if (len == 0) return;
-    const int tok0 = w.chunk_tok0[slot];
-    const int K = w.K, Kp = w.Kp, H = w.H;
-    const size_t ch = (size_t)slot * H + h;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    for (int i = warp; i < kChunk; i += 8) {
-        float* qo = w.qn + (ch * kChunk + i) * Kp;
-        float* ko = w.kn + (ch * kChunk + i) * Kp;
-        if (i < len) {
-            size_t off = ((size_t)(tok0 + i) * H + h) * K;
-            float sq = 0.f, sk = 0.f;
-            for (int d = lane; d < K; d += 32) {
-                float a = ld_io(q, off + d, bf16), b = ld_io(k, off + d, bf16);
-                sq += a * a;
-                sk += b * b;
-            }
-            sq = warp_sum(sq);
-            sk = warp_sum(sk);
-            float qi = l2norm ? 1.0f / fmaxf(sqrtf(sq), 1e-12f) : 1.0f;
-            float ki = l2norm ? 1.0f / fmaxf(sqrtf(sk), 1e-12f) : 1.0f;
-            for (int d = lane; d < Kp; d += 32) {
-                qo[d] = d < K ? ld_io(q, off + d, bf16) * qi * scale : 0.f;
-                ko[d] = d < K ? ld_io(k, off + d, bf16) * ki : 0.f;
-            }
-            if (lane == 0) {
-                w.qinv[ch * kChunk + i] = qi;
-                w.kinv[ch * kChunk + i] = ki;
-                w.beta[ch * kChunk + i] = ld_io(beta, (size_t)(tok0 + i) * H + h, gbf16);
-            }
-        } else {
-            for (int d = lane; d < Kp; d += 32) { qo[d] = 0.f; ko[d] = 0.f; }
-            if (lane == 0) {
-                w.qinv[ch * kChunk + i] = 0.f;
-                w.kinv[ch * kChunk + i] = 0.f;
-                w.beta[ch * kChunk + i] = 0.f;
-            }
-        }
+// dst = alpha * A * B for NP independent S x S problems (row-major, leading dimension kLD): a thread owns CW adjacent
+// columns of one row
+template <int S, int NP, class PA, class PB, class PD>
+__device__ __forceinline__ void merge_mm(PA pa, PB pb, PD pd, float alpha) {
+    constexpr int CW = S * S * NP / 256, TPR = S / CW;      // 1 (8x8x4), 2 (16x16x2), 4 (32x32x1)
+    const int prob = threadIdx.x / (S * TPR), rem = threadIdx.x % (S * TPR);
+    const int i = rem / TPR, j0 = (rem % TPR) * CW;
+    const float* A = pa(prob) + i * kLD;
+    const float* B = pb(prob) + j0;
+    float acc[CW];
+#pragma unroll
+    for (int c = 0; c < CW; ++c) acc[c] = 0.f;
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+        const float a = A[t];
+#pragma unroll
+        for (int c = 0; c < CW; ++c) acc[c] += a * B[t * kLD + c];
     }
-    for (int d = threadIdx.x; d < Kp; d += 256) {
-        float run = 0.f;
-        float* Go = w.G + ch * kChunk * Kp + d;
-        for (int i = 0; i < kChunk; ++i) {
-            if (i < len && d < K) run += ld_io(g, ((size_t)(tok0 + i) * H + h) * K + d, gbf16);
-            Go[(size_t)i * Kp] = run;
-        }
-    }
+    float* D = pd(prob) + i * kLD + j0;
+#pragma unroll
+    for (int c = 0; c < CW; ++c) D[c] = alpha * acc[c];
 }
 
-// ---------------------------------------------------------------------------------------------
-// K2  A, M under the decay mask and T = (I + M)^-1
-// ---------------------------------------------------------------------------------------------
-
-// dst[m x n] (+)= alpha * A[m x kd] * B[kd x n]; all row-major with leading dimension kLD
-__device__ __forceinline__ void small_mm(float* dst, const float* A, const float* B, int m, int n, int kd, float alpha) {
-    for (int idx = threadIdx.x; idx < m * n; idx += 256) {
-        int i = idx / n, j = idx - i * n;
-        float s = 0.f;
-        for (int t = 0; t < kd; ++t) s += A[i * kLD + t] * B[t * kLD + j];
-        dst[i * kLD + j] = alpha * s;
-    }
-}
-
-// In-place inverse of the unit lower-triangular L = I + Ms (Ms strictly lower, 64x64) -> Ts.
-// Block forward substitution: 16x16 diagonal blocks, then 32x32 and 64x64 merges
-//   inv([[A,0],[C,B]]) = [[Ai,0],[-Bi C Ai, Bi]].
+// Ts = (I + Ms)^-1 for strictly lower-triangular Ms: 8x8 diagonal solves, then merges to 16, 32 and 64 with
+//   inv([[A,0],[C,B]]) = [[Ai,0],[-Bi C Ai, Bi]];  tmp: 32 rows
 __device__ void unit_lower_inverse(const float* Ms, float* Ts, float* tmp) {
     const int tid = threadIdx.x;
-    for (int idx = tid; idx < 64 * kLD; idx += 256) Ts[idx] = 0.f;
+    for (int idx = tid; idx < kTile / 4; idx += 256) reinterpret_cast<float4*>(Ts)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     if (tid < 64) {
-        const int b = tid >> 4, j = tid & 15;
-        const float* Lb = Ms + (16 * b) * kLD + 16 * b;
-        float x[16];
+        const int b = tid >> 3, j = tid & 7;
+        const float* Lb = Ms + (8 * b) * kLD + 8 * b;
+        float x[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = (i == j) ? 1.f : 0.f;
+        for (int i = 0; i < 8; ++i) x[i] = (i == j) ? 1.f : 0.f;
 #pragma unroll
-        for (int i = 1; i < 16; ++i) {
+        for (int i = 1; i < 8; ++i) {
             float s = 0.f;
 #pragma unroll
             for (int t = 0; t < i; ++t) s += Lb[i * kLD + t] * x[t];
             x[i] = (i > j) ? -s : x[i];
         }
-        float* Tb = Ts + (16 * b) * kLD + 16 * b;
+        float* Tb = Ts + (8 * b) * kLD + 8 * b;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) Tb[i * kLD + j] = x[i];
+        for (int i = 0; i < 8; ++i) Tb[i * kLD + j] = x[i];
     }
     __syncthreads();
-    // 32x32 merges (two independent pairs)
-    for (int p = 0; p < 2; ++p) {
-        const int o = 32 * p;
-        small_mm(tmp + p * 16 * kLD, Ms + (o + 16) * kLD + o, Ts + o * kLD + o, 16, 16, 16, 1.f);  // C * Ai
-    }
+    merge_mm<8, 4>([&](int p) { return Ms + (16 * p + 8) * kLD + 16 * p; }, [&](int p) { return Ts + (16 * p) * kLD + 16 * p; },
+                   [&](int p) { return tmp + p * 8 * kLD; }, 1.f);
     __syncthreads();
-    for (int p = 0; p < 2; ++p) {
-        const int o = 32 * p;
-        small_mm(Ts + (o + 16) * kLD + o, Ts + (o + 16) * kLD + o + 16, tmp + p * 16 * kLD, 16, 16, 16, -1.f);
-    }
+    merge_mm<8, 4>([&](int p) { return Ts + (16 * p + 8) * kLD + 16 * p + 8; }, [&](int p) { return tmp + p * 8 * kLD; },
+                   [&](int p) { return Ts + (16 * p + 8) * kLD + 16 * p; }, -1.f);
     __syncthreads();
-    // 64x64 merge
-    small_mm(tmp, Ms + 32 * kLD, Ts, 32, 32, 32, 1.f);
+    merge_mm<16, 2>([&](int p) { return Ms + (32 * p + 16) * kLD + 32 * p; }, [&](int p) { return Ts + (32 * p) * kLD + 32 * p; },
+                    [&](int p) { return tmp + p * 16 * kLD; }, 1.f);
     __syncthreads();
-    small_mm(Ts + 32 * kLD, Ts + 32 * kLD + 32, tmp, 32, 32, 32, -1.f);
+    merge_mm<16, 2>([&](int p) { return Ts + (32 * p + 16) * kLD + 32 * p + 16; }, [&](int p) { return tmp + p * 16 * kLD; },
+                    [&](int p) { return Ts + (32 * p + 16) * kLD + 32 * p; }, -1.f);
+    __syncthreads();
+    merge_mm<32, 1>([&](int) { return Ms + 32 * kLD; }, [&](int) { return Ts; }, [&](int) { return tmp; }, 1.f);
+    __syncthreads();
+    merge_mm<32, 1>([&](int) { return Ts + 32 * kLD + 32; }, [&](int) { return tmp; }, [&](int) { return Ts + 32 * kLD; }, -1.f);
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) build_am_kernel(Ws w) {
+// ---------------------------------------------------------------------------------------------
+// decay factors of the masked products
+// ---------------------------------------------------------------------------------------------
+// rho(i, s) = exp(G_i - G_s) is taken apart per 16-row target block I around the reference c_I = G at the block's row 8:
+//   targets  x~_i = x_i exp(G_i - c_I)        sources for block I  k_s exp(c_I - G_s), s < 16 (I + 1)
+// so that the masked products are plain tile products.  Within the block both exponents are at most eight tokens' decay
+// (40 at the gate's lowest), for earlier sources the factor only shrinks.  The blocks' sums are kept apart from the prefix
+// (L, counted from the block's first row), so a factor's exponent is rounded at its own size, not at G's.  A chunk whose
+// decay exceeds kMaxExponent inside a block takes the pairwise exponentials instead (log-decays below -10 per token).
+constexpr float kMaxExponent = 80.f;
+constexpr int kSrcCols = 16 + 32 + 48 + 64;
+// source array of block I: [64 d][16 (I + 1)] with 4 floats of padding, after the two target tiles
+__device__ __forceinline__ int src_ld(int I) { return 16 * (I + 1) + 4; }
+__device__ __forceinline__ int src_off(int I) { return 64 * (8 * I * (I + 1) + 4 * I); }
+constexpr int kSrcFloats = 64 * (kSrcCols + 16);
+
+// ---------------------------------------------------------------------------------------------
+// K1  chunk-parallel part of the forward, one CTA per (chunk, head): norms, decay, A, T, W, U and the scan's coefficients
+// ---------------------------------------------------------------------------------------------
+struct IntraArgs {
+    const void *q, *k, *v, *g, *beta;
+    int bf16, gbf16, l2norm, vec_v, backward;
+    float scale;
+};
+constexpr int kIntraFloats = 2 * kTile + kSrcFloats;      // target stacks and sources, later five tiles
+static_assert(kIntraFloats >= 4 * kTile + 32 * kLD, "the second half's tiles overlap");
+constexpr size_t kIntraSmem = (kIntraFloats + 64 * 3 + 4 * 64 * 2) * sizeof(float);
+
+__global__ void __launch_bounds__(256, 2) intra_fwd_kernel(Ws w, IntraArgs p) {
     extern __shared__ __align__(16) float sm[];
-    float* qT = sm;                  // [d][i]
-    float* kT = qT + 64 * kLD;
-    float* GT = kT + 64 * kLD;
-    float* Ms = GT + 64 * kLD;
-    float* Ts = Ms + 64 * kLD;
-    float* tmp = Ts + 64 * kLD;      // 32 rows
+    float* tq = sm;                      // [d][i] q~
+    float* tk = tq + kTile;              // [d][i] k~
+    float* src = tk + kTile;             // four source arrays
+    float* qi_s = sm + kIntraFloats;     // [64] inverse norms, beta
+    float* ki_s = qi_s + 64;
+    float* bet = ki_s + 64;
+    float* bsum = bet + 64;              // [4][64] block sums of g
+    float* cref = bsum + 256;            // [4][64] G at row 8 of each block
     const int slot = blockIdx.x, h = blockIdx.y;
-    if (w.chunk_len[slot] == 0) return;
-    const size_t ch = (size_t)slot * w.H + h;
-    const int Kp = w.Kp;
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    float accA[4][4], accM[4][4];
-    zero_acc(accA);
-    zero_acc(accM);
-    for (int kt = 0; kt < Kp / 64; ++kt) {
-        __syncthreads();
-        ld_tile<true>(qT, w.qn + ch * kChunk * Kp + kt * 64, Kp);
-        ld_tile<true>(kT, w.kn + ch * kChunk * Kp + kt * 64, Kp);
-        ld_tile<true>(GT, w.G + ch * kChunk * Kp + kt * 64, Kp);
-        __syncthreads();
-        if (tx <= ty) {
-            for (int d = 0; d < 64; ++d) {
-                float4 qi = *reinterpret_cast<const float4*>(qT + d * kLD + 4 * ty);
-                float4 ki = *reinterpret_cast<const float4*>(kT + d * kLD + 4 * ty);
-                float4 gi = *reinterpret_cast<const float4*>(GT + d * kLD + 4 * ty);
-                float4 ks = *reinterpret_cast<const float4*>(kT + d * kLD + 4 * tx);
-                float4 gs = *reinterpret_cast<const float4*>(GT + d * kLD + 4 * tx);
-                const float qa[4] = {qi.x, qi.y, qi.z, qi.w}, ka[4] = {ki.x, ki.y, ki.z, ki.w};
-                const float ga[4] = {gi.x, gi.y, gi.z, gi.w}, kb[4] = {ks.x, ks.y, ks.z, ks.w};
-                const float gb[4] = {gs.x, gs.y, gs.z, gs.w};
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (4 * ty + r >= 4 * tx + c) {
-                            float t = kb[c] * expf(ga[r] - gb[c]);
-                            accA[r][c] += qa[r] * t;
-                            accM[r][c] += ka[r] * t;
-                        }
-                    }
+    const int len = w.chunk_len[slot];
+    if (len == 0) return;
+    const int tok0 = w.chunk_tok0[slot], K = w.K, Kp = w.Kp, V = w.V, Vp = w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
+    const size_t ch = (size_t)slot * H + h;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    for (int i = warp; i < 64; i += 8) {
+        float qi = 0.f, ki = 0.f, b = 0.f;
+        if (i < len) {
+            const size_t off = ((size_t)(tok0 + i) * H + h) * K;
+            float sq = 0.f, sk = 0.f;
+            for (int d = lane; d < K; d += 32) {
+                const float x = ld_io(p.q, off + d, p.bf16), y = ld_io(p.k, off + d, p.bf16);
+                sq += x * x;
+                sk += y * y;
             }
+            sq = warp_sum(sq);
+            sk = warp_sum(sk);
+            qi = p.l2norm ? 1.0f / fmaxf(sqrtf(sq), 1e-12f) : 1.0f;
+            ki = p.l2norm ? 1.0f / fmaxf(sqrtf(sk), 1e-12f) : 1.0f;
+            b = ld_io(p.beta, (size_t)(tok0 + i) * H + h, p.gbf16);
+        }
+        if (lane == 0) {
+            qi_s[i] = qi;
+            ki_s[i] = ki;
+            bet[i] = b;
+            w.qinv[ch * 64 + i] = qi;
+            w.kinv[ch * 64 + i] = ki;
+            w.beta[ch * 64 + i] = b;
+        }
+    }
+    float* kn_g = w.kn + ch * 64 * Kp;
+    float* G_g = w.G + ch * 64 * Kp;
+
+    // ---- A and M: 320 4x4 tiles of [q~; k~] (32 rows per target block) x sources over 256 threads
+    const int t1 = tid < 32 ? 0 : (tid < 96 ? 1 : (tid < 192 ? 2 : 3));
+    const int b1 = t1 == 0 ? 0 : (t1 == 1 ? 32 : (t1 == 2 ? 96 : 192));
+    const int r1 = (tid - b1) / (4 * (t1 + 1)), c1 = (tid - b1) % (4 * (t1 + 1));      // row tile (0-3 q, 4-7 k), source tile
+    const int r2 = (tid + 64) / 16, c2 = (tid + 64) % 16;                              // second tile of threads 0..63: block 3
+    float acc1[4][4], acc2[4][4];
+    zero_acc(acc1);
+    zero_acc(acc2);
+    const int d = tid & 63, I = tid >> 6;      // element-wise: column d, rows 16 I .. 16 I + 15
+    for (int kt = 0; kt < KT; ++kt) {
+        const int dd = kt * 64 + d;
+        const bool in = dd < K;
+        const size_t col = ((size_t)tok0 * H + h) * K + (in ? dd : 0), rstep = (size_t)H * K;
+        float L[16], qn[16], kn[16];
+        {
+            float run = 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) L[r] = (16 * I + r < len && in) ? ld_io(p.g, col + (size_t)(16 * I + r) * rstep, p.gbf16) : 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) L[r] = run += L[r];
+        }
+        __syncthreads();                       // norms on the first round; the previous round's tiles are free
+        bsum[I * 64 + d] = L[15];
+        __syncthreads();
+        float pre = 0.f;
+        for (int J = 0; J < I; ++J) pre += bsum[J * 64 + d];
+        const float c = L[8];
+        cref[I * 64 + d] = pre + c;
+        bool far = false;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) far = far || !(fabsf(L[r] - c) <= kMaxExponent);
+        const bool pairwise = __syncthreads_or(far);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const int i = 16 * I + r;
+            const bool ok = i < len && in;
+            qn[r] = ok ? ld_io(p.q, col + (size_t)i * rstep, p.bf16) * qi_s[i] * p.scale : 0.f;
+            kn[r] = ok ? ld_io(p.k, col + (size_t)i * rstep, p.bf16) * ki_s[i] : 0.f;
+            kn_g[(size_t)i * Kp + dd] = kn[r];
+            G_g[(size_t)i * Kp + dd] = pre + L[r];
+            if (p.backward) w.qn[(ch * 64 + i) * Kp + dd] = qn[r];
+        }
+        {
+            float* rt = w.RT + (ch * Kp + dd) * 64 + 16 * I;      // R^T: 16 rows of column d
+#pragma unroll
+            for (int r4 = 0; r4 < 4; ++r4)
+                *reinterpret_cast<float4*>(rt + 4 * r4) =
+                    make_float4(qn[4 * r4] * expf(pre + L[4 * r4]), qn[4 * r4 + 1] * expf(pre + L[4 * r4 + 1]),
+                                qn[4 * r4 + 2] * expf(pre + L[4 * r4 + 2]), qn[4 * r4 + 3] * expf(pre + L[4 * r4 + 3]));
+        }
+        if (!pairwise) {
+            float e[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) e[r] = expf(L[r] - c);
+#pragma unroll
+            for (int r4 = 0; r4 < 4; ++r4) {
+                *reinterpret_cast<float4*>(tq + d * kLD + 16 * I + 4 * r4) =
+                    make_float4(qn[4 * r4] * e[4 * r4], qn[4 * r4 + 1] * e[4 * r4 + 1], qn[4 * r4 + 2] * e[4 * r4 + 2], qn[4 * r4 + 3] * e[4 * r4 + 3]);
+                *reinterpret_cast<float4*>(tk + d * kLD + 16 * I + 4 * r4) =
+                    make_float4(kn[4 * r4] * e[4 * r4], kn[4 * r4 + 1] * e[4 * r4 + 1], kn[4 * r4 + 2] * e[4 * r4 + 2], kn[4 * r4 + 3] * e[4 * r4 + 3]);
+            }
+#pragma unroll
+            for (int r = 0; r < 16; ++r) e[r] = kn[r] * expf(c - L[r]);
+            for (int T = I; T < 4; ++T) {
+                const float f = T == I ? 1.f : expf(cref[T * 64 + d] - cref[I * 64 + d]);
+                float* s = src + src_off(T) + d * src_ld(T) + 16 * I;
+#pragma unroll
+                for (int r4 = 0; r4 < 4; ++r4)
+                    *reinterpret_cast<float4*>(s + 4 * r4) = make_float4(e[4 * r4] * f, e[4 * r4 + 1] * f, e[4 * r4 + 2] * f, e[4 * r4 + 3] * f);
+            }
+            __syncthreads();
+            mm_at(acc1, (r1 < 4 ? tq : tk) + 16 * t1 + 4 * (r1 & 3), kLD, src + src_off(t1) + 4 * c1, src_ld(t1), 64);
+            if (tid < 64) mm_at(acc2, (r2 < 4 ? tq : tk) + 48 + 4 * (r2 & 3), kLD, src + src_off(3) + 4 * c2, src_ld(3), 64);
+        } else {
+            float* Gs = src;                   // plain q, k, G columns
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                tq[d * kLD + 16 * I + r] = qn[r];
+                tk[d * kLD + 16 * I + r] = kn[r];
+                Gs[d * kLD + 16 * I + r] = pre + L[r];
+            }
+            __syncthreads();
+            auto pairs = [&](float (&acc)[4][4], int T, int rt, int ct) {
+                const float* x = (rt < 4 ? tq : tk);
+                for (int r = 0; r < 4; ++r)
+                    for (int s4 = 0; s4 < 4; ++s4) {
+                        const int i = 16 * T + 4 * (rt & 3) + r, s = 4 * ct + s4;
+                        if (s > i) continue;
+                        float a = 0.f;
+                        for (int e = 0; e < 64; ++e) a += x[e * kLD + i] * tk[e * kLD + s] * expf(Gs[e * kLD + i] - Gs[e * kLD + s]);
+#pragma unroll
+                        for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+                            for (int ss = 0; ss < 4; ++ss)
+                                if (rr == r && ss == s4) acc[rr][ss] += a;
+                    }
+            };
+            pairs(acc1, t1, r1, c1);
+            if (tid < 64) pairs(acc2, 3, r2, c2);
         }
     }
     __syncthreads();
-    const float* bet = w.beta + ch * kChunk;
-    float* Ao = w.A + ch * 4096;
+    // ---- A out (both orientations), M and its inverse
+    float* Ms = sm;
+    float* Ts = Ms + kTile;
+    float* tmp = Ts + kTile;             // 32 rows
+    float* TT = tmp + 32 * kLD;          // [s][i] = T[i][s]
+    float* op = TT + kTile;              // operand tile
+    for (int idx = tid; idx < 2 * kTile / 4; idx += 256) reinterpret_cast<float4*>(sm)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    auto place = [&](const float (&acc)[4][4], int T, int rt, int ct) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int i = 4 * ty + r;
-        const float bi = bet[i];
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int s = 4 * tx + c;
-            Ao[i * 64 + s] = (s <= i) ? accA[r][c] : 0.f;
-            Ms[i * kLD + s] = (s < i) ? bi * accM[r][c] : 0.f;
-        }
+            for (int c4 = 0; c4 < 4; ++c4) {
+                const int i = 16 * T + 4 * (rt & 3) + r, s = 4 * ct + c4;
+                if (rt < 4) Ts[i * kLD + s] = s <= i ? acc[r][c4] : 0.f;      // A, until the inverse overwrites it
+                else Ms[i * kLD + s] = s < i ? bet[i] * acc[r][c4] : 0.f;
+            }
+    };
+    place(acc1, t1, r1, c1);
+    if (tid < 64) place(acc2, 3, r2, c2);
+    __syncthreads();
+    for (int idx = tid; idx < 4096; idx += 256) {
+        w.AT[ch * 4096 + idx] = Ts[(idx & 63) * kLD + (idx >> 6)];
+        if (p.backward) w.A[ch * 4096 + idx] = Ts[(idx >> 6) * kLD + (idx & 63)];
     }
     __syncthreads();
     unit_lower_inverse(Ms, Ts, tmp);
-    float* To = w.T + ch * 4096;
-    for (int idx = threadIdx.x; idx < 4096; idx += 256) To[idx] = Ts[(idx >> 6) * kLD + (idx & 63)];
-}
-
-// ---------------------------------------------------------------------------------------------
-// K3  U = T (beta v),  W = T (beta exp(G) kn); one 64-column tile per CTA
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) uw_kernel(Ws w, const void* __restrict__ v, int bf16) {
-    extern __shared__ __align__(16) float sm[];
-    float* Tt = sm;               // [s][i] = T[i][s]
-    float* Bs = Tt + 64 * kLD;    // [s][col]
-    const int slot = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
-    const int len = w.chunk_len[slot];
-    if (len == 0) return;
-    const size_t ch = (size_t)slot * w.H + h;
-    const int Kp = w.Kp, Vp = w.Vp, KT = Kp / 64;
-    const float* bet = w.beta + ch * kChunk;
-    ld_tile<true>(Tt, w.T + ch * 4096, 64);
-    if (z < KT) {
-        const float* kn = w.kn + ch * kChunk * Kp + z * 64;
-        const float* G = w.G + ch * kChunk * Kp + z * 64;
-        for (int idx = threadIdx.x; idx < 4096; idx += 256) {
-            int s = idx >> 6, d = idx & 63;
-            Bs[s * kLD + d] = bet[s] * expf(G[(size_t)s * Kp + d]) * kn[(size_t)s * Kp + d];
-        }
-    } else {
-        const int vt = z - KT;
-        const int tok0 = w.chunk_tok0[slot];
-        const int nc = min(64, w.V - vt * 64);
-        ld_tile_io<false>(Bs, v, bf16, ((size_t)tok0 * w.H + h) * w.V + vt * 64, (size_t)w.H * w.V, len, nc);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < 4096; idx += 256) Bs[(idx >> 6) * kLD + (idx & 63)] *= bet[idx >> 6];
+    for (int idx = tid; idx < 4096; idx += 256) {
+        const int r = idx >> 6, c = idx & 63;
+        TT[r * kLD + c] = Ts[c * kLD + r];
+        if (p.backward) w.T[ch * 4096 + idx] = Ts[r * kLD + c];
     }
-    __syncthreads();
+    // ---- W = T (beta e^G k), U = T (beta v)
     float acc[4][4];
-    zero_acc(acc);
-    mm64(acc, Tt, Bs);
-    if (z < KT) st_acc_g(w.W + ch * kChunk * Kp + z * 64, Kp, acc);
-    else st_acc_g(w.Z + ch * kChunk * Vp + (z - KT) * 64, Vp, acc);
+    float* W_g = w.W + ch * 64 * Kp;
+    float* Z_g = w.Z + ch * 64 * Vp;
+    for (int kt = 0; kt < KT; ++kt) {
+        __syncthreads();
+        for (int idx = tid; idx < 1024; idx += 256) {
+            const int r = idx >> 4, c4 = (idx & 15) << 2;
+            const float4 k4 = *reinterpret_cast<const float4*>(kn_g + (size_t)r * Kp + kt * 64 + c4);
+            const float4 g4 = *reinterpret_cast<const float4*>(G_g + (size_t)r * Kp + kt * 64 + c4);
+            const float b = bet[r];
+            *reinterpret_cast<float4*>(op + r * kLD + c4) =
+                make_float4(b * expf(g4.x) * k4.x, b * expf(g4.y) * k4.y, b * expf(g4.z) * k4.z, b * expf(g4.w) * k4.w);
+        }
+        __syncthreads();
+        zero_acc(acc);
+        mm64(acc, TT, op);
+        st_nat(W_g + kt * 64, Kp, acc);
+        st_tr(w.WT + (ch * Kp + kt * 64) * 64, 64, acc);
+    }
+    for (int vt = 0; vt < VT; ++vt) {
+        __syncthreads();
+        ld_tile_io<false>(op, p.v, p.bf16, ((size_t)tok0 * H + h) * V + vt * 64, (size_t)H * V, len, V - vt * 64, p.vec_v, bet);
+        __syncthreads();
+        zero_acc(acc);
+        mm64(acc, TT, op);
+        st_nat(Z_g + vt * 64, Vp, acc);
+    }
+    // ---- the scan's coefficients: E^T W, E^T U, exp(G_end);  Rm = R - A W for the adjoint scan
+    float* Es = sm;                      // [s][k]
+    float* Xs = sm + kTile;
+    const float* ge = G_g + (size_t)63 * Kp;
+    for (int kt = 0; kt < KT; ++kt) {
+        __syncthreads();
+        for (int idx = tid; idx < 1024; idx += 256) {
+            const int r = idx >> 4, c4 = (idx & 15) << 2;
+            const float4 k4 = *reinterpret_cast<const float4*>(kn_g + (size_t)r * Kp + kt * 64 + c4);
+            const float4 g4 = *reinterpret_cast<const float4*>(G_g + (size_t)r * Kp + kt * 64 + c4);
+            const float4 e4 = *reinterpret_cast<const float4*>(ge + kt * 64 + c4);
+            *reinterpret_cast<float4*>(Es + r * kLD + c4) =
+                make_float4(k4.x * expf(e4.x - g4.x), k4.y * expf(e4.y - g4.y), k4.z * expf(e4.z - g4.z), k4.w * expf(e4.w - g4.w));
+        }
+        if (tid < 64) w.dec[ch * Kp + kt * 64 + tid] = expf(ge[kt * 64 + tid]);
+        for (int k2 = 0; k2 < KT; ++k2) {
+            __syncthreads();
+            ld_nat(Xs, W_g + k2 * 64, Kp);
+            __syncthreads();
+            zero_acc(acc);
+            mm64(acc, Xs, Es);           // [k'][k] = sum_s W[s][k'] E[s][k]
+            st_nat(w.PT + (ch * Kp + k2 * 64) * Kp + kt * 64, Kp, acc);
+            if (p.backward) st_tr(w.P + (ch * Kp + kt * 64) * Kp + k2 * 64, Kp, acc);
+        }
+        for (int vt = 0; vt < VT; ++vt) {
+            __syncthreads();
+            ld_nat(Xs, Z_g + vt * 64, Vp);
+            __syncthreads();
+            zero_acc(acc);
+            mm64(acc, Es, Xs);
+            st_nat(w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp, acc);
+        }
+    }
+    if (p.backward) {
+        __syncthreads();
+        ld_nat(Es, w.AT + ch * 4096, 64);
+        for (int kt = 0; kt < KT; ++kt) {
+            __syncthreads();
+            ld_nat(Xs, W_g + kt * 64, Kp);
+            __syncthreads();
+            zero_acc(acc);
+            mm64(acc, Es, Xs);           // A W
+            float qv[4][4], gv[4][4];
+            ld_patch(qv, w.qn + ch * 64 * Kp + kt * 64, Kp);
+            ld_patch(gv, G_g + kt * 64, Kp);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c4 = 0; c4 < 4; ++c4) acc[r][c4] = qv[r][c4] * expf(gv[r][c4]) - acc[r][c4];
+            st_nat(w.Rm + ch * 64 * Kp + kt * 64, Kp, acc);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
-// K4  forward state scan over the chunks of one (sequence, head, 16-column value strip)
+// K2  state scan over the chunks of one (sequence, head, 16-column value strip), in either direction:
+//     forward  S = H:   S' = dec . S + B - P S       B = E^T U, leaves the chunk-start states in its place
+//     backward S = dH': S' = dec . S + B - P^T S     B = Rm^T dO, leaves the adjoints of the outgoing states
+// A step is one Kp x Kp product against a 16-column strip.  Its matrix comes through a ring of 64x64 tiles filled by
+// asynchronous copies ahead of the step, four groups of two warps share the contraction, and the strip lives in registers
+// (one float4 per thread and 64-row block) and, for the products, in shared memory.
 // ---------------------------------------------------------------------------------------------
-constexpr int kVS = 16;
+constexpr int kVS = 16, kScanStages = 4;
 
-__global__ void __launch_bounds__(256) scan_fwd_kernel(Ws w, const float* __restrict__ h0, float* __restrict__ final_state) {
+struct ScanArgs {
+    const float* M;       // [ch][Kp][Kp], contraction index leading: P^T forward, P backward
+    float* B;             // [ch][Kp][Vp]
+    const float* s_in;    // [n_seq][H][V][K] or null
+    float* s_out;
+    int backward;
+};
+
+__global__ void __launch_bounds__(256) scan_kernel(Ws w, ScanArgs p) {
     extern __shared__ __align__(16) float sm[];
-    const int Kp = w.Kp, Vp = w.Vp, K = w.K, V = w.V, H = w.H;
-    const int ldw = Kp + 1;
-    float* Ws_ = sm;                       // [64][Kp+1]
-    float* Es = Ws_ + 64 * ldw;            // [64][Kp+1]
-    float* Hs = Es + 64 * ldw;             // [Kp][16]
-    float* Zs = Hs + Kp * kVS;             // [64][16]
-    float* eGe = Zs + 64 * kVS;            // [Kp]
-    const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kVS;
-    const int tid = threadIdx.x;
-
-    for (int idx = tid; idx < Kp * kVS; idx += 256) {
-        int kk = idx / kVS, vv = idx % kVS;
-        float x = 0.f;
-        if (h0 && kk < K && v0 + vv < V) x = h0[(((size_t)seq * H + h) * V + v0 + vv) * K + kk];
-        Hs[idx] = x;
-    }
-    const int c_begin = w.seq_chunk0[seq], c_end = w.seq_chunk0[seq + 1];
-    for (int slot = c_begin; slot < c_end; ++slot) {
-        const size_t ch = (size_t)slot * H + h;
-        __syncthreads();
-        const float* Wg = w.W + ch * kChunk * Kp;
-        const float* kng = w.kn + ch * kChunk * Kp;
-        const float* Gg = w.G + ch * kChunk * Kp;
-        for (int idx = tid; idx < Kp; idx += 256) eGe[idx] = Gg[(size_t)63 * Kp + idx];
-        __syncthreads();
-        for (int idx = tid; idx < 64 * Kp; idx += 256) {
-            int i = idx / Kp, d = idx - i * Kp;
-            Ws_[i * ldw + d] = Wg[idx];
-            Es[i * ldw + d] = kng[idx] * expf(eGe[d] - Gg[idx]);
-        }
-        // publish the chunk-start state for the output kernel and the backward
-        float* Hg = w.Hc + ch * Kp * Vp;
-        for (int idx = tid; idx < Kp * kVS; idx += 256) Hg[(size_t)(idx / kVS) * Vp + v0 + (idx % kVS)] = Hs[idx];
-        __syncthreads();
-        // Z = U - W H   (thread: row i, 4 value columns)
-        {
-            const int i = tid >> 2, vq = (tid & 3) << 2;
-            float* Zg = w.Z + (ch * kChunk + i) * Vp + v0 + vq;
-            float4 u = *reinterpret_cast<const float4*>(Zg);
-            float a0 = u.x, a1 = u.y, a2 = u.z, a3 = u.w;
-            const float* wr = Ws_ + i * ldw;
-            for (int kk = 0; kk < Kp; ++kk) {
-                float wv = wr[kk];
-                float4 hv = *reinterpret_cast<const float4*>(Hs + kk * kVS + vq);
-                a0 -= wv * hv.x; a1 -= wv * hv.y; a2 -= wv * hv.z; a3 -= wv * hv.w;
+    float* ring = sm;                                  // [stages][64][64]
+    float* part = ring + kScanStages * 4096;           // [4][64][16]
+    float* S = part + 4 * 64 * kVS;                    // [Kp][16]
+    const int Kp = w.Kp, Vp = w.Vp, K = w.K, V = w.V, H = w.H, KT = Kp / 64;
+    const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kVS, tid = threadIdx.x;
+    const int c0 = w.seq_chunk0[seq], c1 = w.seq_chunk0[seq + 1], n = c1 - c0;
+    const int row = tid >> 2, c4 = (tid & 3) << 2;      // this thread's float4 of a 64-row block
+    const int kg = tid >> 6, pr = (tid & 15) << 2, pc = ((tid >> 4) & 3) << 2;      // product: contraction group, rows, columns
+    auto chunk = [&](int step) { return (size_t)(p.backward ? c1 - 1 - step : c0 + step) * H + h; };
+    const int tiles = n * KT * KT;
+    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+    auto issue = [&](int t) {      // tile t: step, then output block, then contraction block
+        if (t < tiles) {
+            const int step = t / (KT * KT), rt = (t / KT) % KT, kt = t % KT;
+            const float* src = p.M + (chunk(step) * Kp + kt * 64) * Kp + rt * 64;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int idx = tid + 256 * i, r = idx >> 4, c = (idx & 15) << 2;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_s + ((t % kScanStages) * 4096 + r * 64 + c) * 4), "l"(src + (size_t)r * Kp + c)
+                             : "memory");
             }
-            *reinterpret_cast<float4*>(Zg) = make_float4(a0, a1, a2, a3);
-            *reinterpret_cast<float4*>(Zs + i * kVS + vq) = make_float4(a0, a1, a2, a3);
         }
-        __syncthreads();
-        for (int idx = tid; idx < Kp; idx += 256) eGe[idx] = expf(eGe[idx]);
-        __syncthreads();
-        // H <- exp(G_end) H + E^T Z   (thread: key row kk, 4 value columns)
-        for (int o = tid; o < Kp * 4; o += 256) {
-            const int kk = o >> 2, vq = (o & 3) << 2;
-            float4 hv = *reinterpret_cast<const float4*>(Hs + kk * kVS + vq);
-            const float dec = eGe[kk];
-            float a0 = dec * hv.x, a1 = dec * hv.y, a2 = dec * hv.z, a3 = dec * hv.w;
-            for (int i = 0; i < 64; ++i) {
-                float e = Es[i * ldw + kk];
-                float4 zv = *reinterpret_cast<const float4*>(Zs + i * kVS + vq);
-                a0 += e * zv.x; a1 += e * zv.y; a2 += e * zv.z; a3 += e * zv.w;
-            }
-            *reinterpret_cast<float4*>(Hs + kk * kVS + vq) = make_float4(a0, a1, a2, a3);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float4 s[4], b[4];
+    float dec[4];
+    auto load_step = [&](int step) {
+        if (step < n) {
+            const size_t ch = chunk(step);
+#pragma unroll
+            for (int rt = 0; rt < 4; ++rt)
+                if (rt < KT) {
+                    b[rt] = *reinterpret_cast<const float4*>(p.B + (ch * Kp + rt * 64 + row) * Vp + v0 + c4);
+                    dec[rt] = w.dec[ch * Kp + rt * 64 + row];
+                }
         }
+    };
+#pragma unroll
+    for (int rt = 0; rt < 4; ++rt) {
+        s[rt] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int kk = rt * 64 + row;
+        if (rt < KT && p.s_in && kk < K) {
+            const float* src = p.s_in + (((size_t)seq * H + h) * V + v0 + c4) * K + kk;
+            if (v0 + c4 + 0 < V) s[rt].x = src[0];
+            if (v0 + c4 + 1 < V) s[rt].y = src[K];
+            if (v0 + c4 + 2 < V) s[rt].z = src[2 * (size_t)K];
+            if (v0 + c4 + 3 < V) s[rt].w = src[3 * (size_t)K];
+        }
+        if (rt < KT) *reinterpret_cast<float4*>(S + kk * kVS + c4) = s[rt];
     }
-    __syncthreads();
-    if (final_state) {
-        for (int idx = tid; idx < Kp * kVS; idx += 256) {
-            int vv = idx / Kp, kk = idx - vv * Kp;
-            if (kk < K && v0 + vv < V) final_state[(((size_t)seq * H + h) * V + v0 + vv) * K + kk] = Hs[kk * kVS + vv];
+    for (int t = 0; t < kScanStages - 1; ++t) issue(t);
+    load_step(0);
+    int t = 0;
+    for (int step = 0; step < n; ++step) {
+        const size_t ch = chunk(step);
+        float4 bc[4];
+        float dc[4];
+#pragma unroll
+        for (int rt = 0; rt < 4; ++rt) {
+            bc[rt] = b[rt];
+            dc[rt] = dec[rt];
+            if (rt < KT) *reinterpret_cast<float4*>(p.B + (ch * Kp + rt * 64 + row) * Vp + v0 + c4) = s[rt];      // the state the chunk sees
+        }
+        load_step(step + 1);
+        for (int rt = 0; rt < KT; ++rt) {
+            float acc[4][4];
+            zero_acc(acc);
+            for (int kt = 0; kt < KT; ++kt, ++t) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kScanStages - 2) : "memory");
+                __syncthreads();                       // tile t has landed for everyone; tile t - 1 and (rt = 0) the old strip are read out
+                issue(t + kScanStages - 1);
+                mm_at(acc, ring + (t % kScanStages) * 4096 + 16 * kg * 64 + pr, 64, S + (kt * 64 + 16 * kg) * kVS + pc, kVS, 16);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                *reinterpret_cast<float4*>(part + (kg * 64 + pr + r) * kVS + pc) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            __syncthreads();
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const float4 y = *reinterpret_cast<const float4*>(part + (g * 64 + row) * kVS + c4);
+                x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q == rt) {
+                    s[q].x = dc[q] * s[q].x + bc[q].x - x.x;
+                    s[q].y = dc[q] * s[q].y + bc[q].y - x.y;
+                    s[q].z = dc[q] * s[q].z + bc[q].z - x.z;
+                    s[q].w = dc[q] * s[q].w + bc[q].w - x.w;
+                }
+        }
+        __syncthreads();                               // every product has read the strip
+#pragma unroll
+        for (int rt = 0; rt < 4; ++rt)
+            if (rt < KT) *reinterpret_cast<float4*>(S + (rt * 64 + row) * kVS + c4) = s[rt];
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (p.s_out) {
+#pragma unroll
+        for (int rt = 0; rt < 4; ++rt) {
+            const int kk = rt * 64 + row;
+            if (rt < KT && kk < K) {
+                float* dst = p.s_out + (((size_t)seq * H + h) * V + v0 + c4) * K + kk;
+                if (v0 + c4 + 0 < V) dst[0] = s[rt].x;
+                if (v0 + c4 + 1 < V) dst[K] = s[rt].y;
+                if (v0 + c4 + 2 < V) dst[2 * (size_t)K] = s[rt].z;
+                if (v0 + c4 + 3 < V) dst[3 * (size_t)K] = s[rt].w;
+            }
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// K5  output  O = (qn exp(G)) H + A Z; one 64-column value tile per CTA
+// K3  Z = U - W H, O = R H + A Z; one 64-column value tile per CTA
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, int bf16) {
     extern __shared__ __align__(16) float sm[];
-    float* At = sm;
-    float* Bs = At + 64 * kLD;
+    float *Wt = sm, *Rt = sm + kTile, *Bs = sm + 2 * kTile;
     const int slot = blockIdx.x, h = blockIdx.y, vt = blockIdx.z;
     const int len = w.chunk_len[slot];
     if (len == 0) return;
     const size_t ch = (size_t)slot * w.H + h;
     const int Kp = w.Kp, Vp = w.Vp;
-    float acc[4][4];
-    zero_acc(acc);
+    float az[4][4], ao[4][4];
+    zero_acc(az);
+    zero_acc(ao);
     for (int kt = 0; kt < Kp / 64; ++kt) {
         __syncthreads();
-        const float* qn = w.qn + ch * kChunk * Kp + kt * 64;
-        const float* G = w.G + ch * kChunk * Kp + kt * 64;
-        for (int idx = threadIdx.x; idx < 4096; idx += 256) {
-            int i = idx >> 6, d = idx & 63;
-            At[d * kLD + i] = qn[(size_t)i * Kp + d] * expf(G[(size_t)i * Kp + d]);
-        }
-        ld_tile<false>(Bs, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+        ld_nat(Wt, w.WT + (ch * Kp + kt * 64) * 64, 64);
+        ld_nat(Rt, w.RT + (ch * Kp + kt * 64) * 64, 64);
+        ld_nat(Bs, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
         __syncthreads();
-        mm64(acc, At, Bs);
+        mm64(az, Wt, Bs);
+        mm64(ao, Rt, Bs);
     }
     __syncthreads();
-    ld_tile<true>(At, w.A + ch * 4096, 64);
-    ld_tile<false>(Bs, w.Z + ch * kChunk * Vp + vt * 64, Vp);
+    ld_nat(Wt, w.AT + ch * 4096, 64);
+    float* Zg = w.Z + ch * 64 * Vp + vt * 64;
+    float u[4][4];
+    ld_patch(u, Zg, Vp);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) u[r][c] -= az[r][c];
+    st_nat(Zg, Vp, u);
+    st_nat(Bs, kLD, u);
     __syncthreads();
-    mm64(acc, At, Bs);
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const int tok0 = w.chunk_tok0[slot];
+    mm64(ao, Wt, Bs);
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15, tok0 = w.chunk_tok0[slot];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int i = 4 * ty + r;
@@ -509,421 +747,480 @@ __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, in
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int vv = vt * 64 + 4 * tx + c;
-            if (vv < w.V) st_io(o, ((size_t)(tok0 + i) * w.H + h) * w.V + vv, bf16, acc[r][c]);
+            if (vv < w.V) st_io(o, ((size_t)(tok0 + i) * w.H + h) * w.V + vv, bf16, ao[r][c]);
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// K6  reverse scan of the state adjoint
-//   dZ = A^T dO + E dH' ;  dH = R^T dO + exp(G_end) dH' - W^T dZ
+// K4  Rm^T dO, the adjoint scan's state-independent term; one (key tile, value tile) per CTA
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) scan_bwd_kernel(Ws w, Scr s, const void* __restrict__ d_o, int bf16,
-                                                       const float* __restrict__ d_final, float* __restrict__ dh0) {
+__global__ void __launch_bounds__(256) adjoint_term_kernel(Ws w, Scr s, const void* __restrict__ d_o, int bf16, int vec_v) {
     extern __shared__ __align__(16) float sm[];
-    const int Kp = w.Kp, Vp = w.Vp, K = w.K, V = w.V, H = w.H;
-    const int ldw = Kp + 1;
-    float* B1 = sm;                      // [64][Kp+1]  E, then R
-    float* B2 = B1 + 64 * ldw;           // [64][Kp+1]  W
-    float* As = B2 + 64 * ldw;           // [64][kLD]   A row-major
-    float* dHs = As + 64 * kLD;          // [Kp][16]
-    float* dHn = dHs + Kp * kVS;         // [Kp][16]   new value
-    float* dOs = dHn + Kp * kVS;         // [64][16]
-    float* dZs = dOs + 64 * kVS;         // [64][16]
-    float* eGe = dZs + 64 * kVS;         // [Kp]
-    const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kVS;
-    const int tid = threadIdx.x;
-
-    for (int idx = tid; idx < Kp * kVS; idx += 256) {
-        int kk = idx / kVS, vv = idx % kVS;
-        float x = 0.f;
-        if (d_final && kk < K && v0 + vv < V) x = d_final[(((size_t)seq * H + h) * V + v0 + vv) * K + kk];
-        dHs[idx] = x;
-    }
-    const int c_begin = w.seq_chunk0[seq], c_end = w.seq_chunk0[seq + 1];
-    for (int slot = c_end - 1; slot >= c_begin; --slot) {
-        const size_t ch = (size_t)slot * H + h;
-        const int len = w.chunk_len[slot], tok0 = w.chunk_tok0[slot];
-        __syncthreads();
-        const float* kng = w.kn + ch * kChunk * Kp;
-        const float* qng = w.qn + ch * kChunk * Kp;
-        const float* Gg = w.G + ch * kChunk * Kp;
-        const float* Wg = w.W + ch * kChunk * Kp;
-        for (int idx = tid; idx < Kp; idx += 256) eGe[idx] = Gg[(size_t)63 * Kp + idx];
-        ld_tile<false>(As, w.A + ch * 4096, 64);
-        for (int idx = tid; idx < 64 * kVS; idx += 256) {
-            int i = idx / kVS, vv = idx % kVS;
-            dOs[idx] = (i < len && v0 + vv < V) ? ld_io(d_o, ((size_t)(tok0 + i) * H + h) * V + v0 + vv, bf16) : 0.f;
-        }
-        __syncthreads();
-        for (int idx = tid; idx < 64 * Kp; idx += 256) {
-            int i = idx / Kp, d = idx - i * Kp;
-            B1[i * ldw + d] = kng[idx] * expf(eGe[d] - Gg[idx]);
-            B2[i * ldw + d] = Wg[idx];
-        }
-        // publish dH' (adjoint of this chunk's outgoing state)
-        float* dHg = s.dHn + ch * Kp * Vp;
-        for (int idx = tid; idx < Kp * kVS; idx += 256) dHg[(size_t)(idx / kVS) * Vp + v0 + (idx % kVS)] = dHs[idx];
-        __syncthreads();
-        // dZ[i] = sum_{s>=i} A[s][i] dO[s] + sum_k E[i][k] dH'[k]
-        {
-            const int i = tid >> 2, vq = (tid & 3) << 2;
-            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-            for (int ss = i; ss < 64; ++ss) {
-                float av = As[ss * kLD + i];
-                float4 dv = *reinterpret_cast<const float4*>(dOs + ss * kVS + vq);
-                a0 += av * dv.x; a1 += av * dv.y; a2 += av * dv.z; a3 += av * dv.w;
-            }
-            const float* er = B1 + i * ldw;
-            for (int kk = 0; kk < Kp; ++kk) {
-                float ev = er[kk];
-                float4 hv = *reinterpret_cast<const float4*>(dHs + kk * kVS + vq);
-                a0 += ev * hv.x; a1 += ev * hv.y; a2 += ev * hv.z; a3 += ev * hv.w;
-            }
-            *reinterpret_cast<float4*>(dZs + i * kVS + vq) = make_float4(a0, a1, a2, a3);
-            *reinterpret_cast<float4*>(s.dZ + (ch * kChunk + i) * Vp + v0 + vq) = make_float4(a0, a1, a2, a3);
-        }
-        __syncthreads();
-        // B1 <- R = qn exp(G)
-        for (int idx = tid; idx < 64 * Kp; idx += 256) {
-            int i = idx / Kp, d = idx - i * Kp;
-            B1[i * ldw + d] = qng[idx] * expf(Gg[idx]);
-        }
-        for (int idx = tid; idx < Kp; idx += 256) eGe[idx] = expf(eGe[idx]);
-        __syncthreads();
-        for (int o = tid; o < Kp * 4; o += 256) {
-            const int kk = o >> 2, vq = (o & 3) << 2;
-            float4 hv = *reinterpret_cast<const float4*>(dHs + kk * kVS + vq);
-            const float dec = eGe[kk];
-            float a0 = dec * hv.x, a1 = dec * hv.y, a2 = dec * hv.z, a3 = dec * hv.w;
-            for (int i = 0; i < 64; ++i) {
-                float rv = B1[i * ldw + kk], wv = B2[i * ldw + kk];
-                float4 ov = *reinterpret_cast<const float4*>(dOs + i * kVS + vq);
-                float4 zv = *reinterpret_cast<const float4*>(dZs + i * kVS + vq);
-                a0 += rv * ov.x - wv * zv.x; a1 += rv * ov.y - wv * zv.y;
-                a2 += rv * ov.z - wv * zv.z; a3 += rv * ov.w - wv * zv.w;
-            }
-            *reinterpret_cast<float4*>(dHn + kk * kVS + vq) = make_float4(a0, a1, a2, a3);
-        }
-        __syncthreads();
-        for (int idx = tid; idx < Kp * kVS; idx += 256) dHs[idx] = dHn[idx];
-    }
+    const int slot = blockIdx.x, h = blockIdx.y, VT = w.Vp / 64, kt = blockIdx.z / VT, vt = blockIdx.z % VT;
+    const int len = w.chunk_len[slot];
+    if (len == 0) return;
+    const size_t ch = (size_t)slot * w.H + h;
+    ld_nat(sm, w.Rm + ch * 64 * w.Kp + kt * 64, w.Kp);
+    ld_tile_io<false>(sm + kTile, d_o, bf16, ((size_t)w.chunk_tok0[slot] * w.H + h) * w.V + vt * 64, (size_t)w.H * w.V, len, w.V - vt * 64, vec_v);
     __syncthreads();
-    if (dh0) {
-        for (int idx = tid; idx < Kp * kVS; idx += 256) {
-            int vv = idx / Kp, kk = idx - vv * Kp;
-            if (kk < K && v0 + vv < V) dh0[(((size_t)seq * H + h) * V + v0 + vv) * K + kk] = dHs[kk * kVS + vv];
-        }
-    }
+    float acc[4][4];
+    zero_acc(acc);
+    mm64(acc, sm, sm + kTile);
+    st_nat(s.dHn + (ch * w.Kp + kt * 64) * w.Vp + vt * 64, w.Vp, acc);
 }
 
 // ---------------------------------------------------------------------------------------------
-// K7  chunk-local adjoints: dv, dA, dM and the direct parts of dqn, dkn, dG, dbeta
+// K5  chunk-local adjoints, one CTA per (chunk, head): dZ, the products with the states, the adjoint of the inverse, the
+//     pull-back through the decay-masked products and the L2-normalisation VJP, in one launch.  16 tile products at
+//     K = V = 64; six tiles of shared memory, so that two CTAs share an SM.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) bwd_local_kernel(Ws w, Scr s, const void* __restrict__ v,
-                                                        const void* __restrict__ d_o, void* __restrict__ dv, int bf16) {
+struct LocalArgs {
+    const void *q, *k, *v, *g, *d_o;
+    void *dq, *dk, *dv, *dg, *dbeta;
+    int bf16, gbf16, l2norm, vec_k, vec_v;
+    float scale;
+};
+constexpr size_t kLocalSmem = (6 * kTile + 64 * 3 + 4 * 64 * 3 + KDA_MAX_DIM) * sizeof(float);
+
+__global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArgs p) {
     extern __shared__ __align__(16) float sm[];
-    float* Tr = sm;                 // T row-major  [s][i] view gives T^T products
-    float* Tt = Tr + 64 * kLD;      // T transposed
-    float* P0 = Tt + 64 * kLD;      // operand tiles
-    float* P1 = P0 + 64 * kLD;
-    float* P2 = P1 + 64 * kLD;
-    float* P3 = P2 + 64 * kLD;
-    float* P4 = P3 + 64 * kLD;
-    float* red = P4 + 64 * kLD;     // [64][17] row partials / [16][64] column partials
-    float* dbv = red + 64 * 17;     // [64]
+    float *t0 = sm, *t1 = sm + kTile, *t2 = sm + 2 * kTile, *t3 = sm + 3 * kTile, *t4 = sm + 4 * kTile, *t5 = sm + 5 * kTile;
+    float* bet = sm + 6 * kTile;         // [64] beta, inverse norms
+    float* qi_s = bet + 64;
+    float* ki_s = qi_s + 64;
+    float* bsum = ki_s + 64;             // [4][64] scratch
+    float* cref = bsum + 256;            // [4][64] G at row 8 of each block
+    float* tot = cref + 256;             // [4][64] scratch
+    float* gend = tot + 256;             // [Kp]    d G_end
     const int slot = blockIdx.x, h = blockIdx.y;
     const int len = w.chunk_len[slot];
     if (len == 0) return;
-    const int tok0 = w.chunk_tok0[slot];
-    const size_t ch = (size_t)slot * w.H + h;
-    const int Kp = w.Kp, Vp = w.Vp, KT = Kp / 64, VT = Vp / 64, H = w.H, V = w.V;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const float* bet = w.beta + ch * kChunk;
-
-    ld_tile<false>(Tr, w.T + ch * 4096, 64);
-    ld_tile<true>(Tt, w.T + ch * 4096, 64);
-    if (tid < 64) dbv[tid] = 0.f;
-    float accX[4][4], accA[4][4], acc[4][4];
-    zero_acc(accX);
-    zero_acc(accA);
-
-    // ---- value tiles: dA += dO Z^T ; X += dZ P^T ; dP = T^T dZ
-    for (int vt = 0; vt < VT; ++vt) {
-        const int nc = min(64, V - vt * 64);
-        const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
-        __syncthreads();
-        ld_tile_io<true>(P0, d_o, bf16, voff, (size_t)H * V, len, nc);          // [v][i] = dO[i][v]
-        ld_tile<true>(P1, w.Z + ch * kChunk * Vp + vt * 64, Vp);                 // [v][s] = Z[s][v]
-        ld_tile<true>(P2, s.dZ + ch * kChunk * Vp + vt * 64, Vp);                // [v][i] = dZ[i][v]
-        ld_tile_io<true>(P3, v, bf16, voff, (size_t)H * V, len, nc);             // [v][s] = v[s][v]
-        ld_tile<false>(P4, s.dZ + ch * kChunk * Vp + vt * 64, Vp);               // [s][v] = dZ[s][v]
-        __syncthreads();
-        for (int idx = tid; idx < 4096; idx += 256) P3[(idx >> 6) * kLD + (idx & 63)] *= bet[idx & 63];  // P^T
-        mm64(accA, P0, P1);
-        __syncthreads();
-        mm64(accX, P2, P3);
-        zero_acc(acc);
-        mm64(acc, Tr, P4);   // dP[i][v] = sum_s T[s][i] dZ[s][v]
-        // dv = beta dP ; dbeta += sum_v dP * v   (v[i][vv] = P3[vv][i] / beta_i, so reload v directly)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int i = 4 * ty + r;
-            float part = 0.f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int vv = vt * 64 + 4 * tx + c;
-                if (i < len && vv < V) {
-                    const size_t o = ((size_t)(tok0 + i) * H + h) * V + vv;
-                    part += acc[r][c] * ld_io(v, o, bf16);
-                    st_io(dv, o, bf16, bet[i] * acc[r][c]);
-                }
-            }
-            red[i * 17 + tx] = part;
-        }
-        __syncthreads();
-        if (tid < 64) {
-            float t = 0.f;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) t += red[tid * 17 + j];
-            dbv[tid] += t;
-        }
+    const int tok0 = w.chunk_tok0[slot], K = w.K, Kp = w.Kp, V = w.V, Vp = w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
+    const size_t ch = (size_t)slot * H + h;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, d = tid & 63, I = tid >> 6;
+    const float* kn_g = w.kn + ch * 64 * Kp;
+    const float* G_g = w.G + ch * 64 * Kp;
+    const float* qn_g = w.qn + ch * 64 * Kp;
+    const size_t vrow = (size_t)H * V, krow = (size_t)H * K;
+    if (tid < 64) {
+        bet[tid] = w.beta[ch * 64 + tid];
+        qi_s[tid] = w.qinv[ch * 64 + tid];
+        ki_s[tid] = w.kinv[ch * 64 + tid];
     }
-
-    // ---- key tiles
+    // column d, rows 16 I ..: x(row) -> four 16-byte stores along row d of a transposed tile
+    auto st_col = [&](float* t, const float (&x)[16]) {
+#pragma unroll
+        for (int r4 = 0; r4 < 4; ++r4)
+            *reinterpret_cast<float4*>(t + d * kLD + 16 * I + 4 * r4) = make_float4(x[4 * r4], x[4 * r4 + 1], x[4 * r4 + 2], x[4 * r4 + 3]);
+    };
+    float acc[4][4], accX[4][4];
+    float db[4] = {0.f, 0.f, 0.f, 0.f};      // dbeta of this thread's rows (equal in the 16 lanes of a row)
+    zero_acc(accX);
+    {
+        float accA[4][4];
+        zero_acc(accA);
+        for (int vt = 0; vt < VT; ++vt) {
+            const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
+            const int nc = V - vt * 64;
+            // ---- dZ = A^T dO + E dH'
+            __syncthreads();
+            ld_nat(t4, w.A + ch * 4096, 64);
+            ld_tile_io<false>(t5, p.d_o, p.bf16, voff, vrow, len, nc, p.vec_v);
+            __syncthreads();
+            zero_acc(acc);
+            mm64(acc, t4, t5);
+            for (int kt = 0; kt < KT; ++kt) {
+                __syncthreads();
+                {
+                    float e[16];
+                    const float ge = G_g[(size_t)63 * Kp + kt * 64 + d];
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const size_t o = (size_t)(16 * I + r) * Kp + kt * 64 + d;
+                        e[r] = kn_g[o] * expf(ge - G_g[o]);
+                    }
+                    st_col(t4, e);
+                }
+                ld_nat(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+                __syncthreads();
+                mm64(acc, t4, t5);
+            }
+            // ---- dA += dO Z^T, X += dZ (beta v)^T, dv = beta T^T dZ
+            __syncthreads();
+            st_tr(t2, kLD, acc);
+            st_nat(t4, kLD, acc);
+            if (VT > 1) st_nat(s.dZ + ch * 64 * Vp + vt * 64, Vp, acc);
+            if (vt == 0) ld_nat(t3, w.T + ch * 4096, 64);
+            ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, nc, p.vec_v);
+            ld_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
+            ld_tile_io<true>(t5, p.v, p.bf16, voff, vrow, len, nc, p.vec_v, bet);
+            __syncthreads();
+            mm64(accA, t0, t1);
+            mm64(accX, t2, t5);
+            zero_acc(acc);
+            mm64(acc, t3, t4);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int i = 4 * ty + r;
+                float x[4], part = 0.f;
+                ld4_io(x, p.v, p.bf16, voff, vrow, i, 4 * tx, len, nc, p.vec_v);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    part += acc[r][c] * x[c];
+                    if (i < len && 4 * tx + c < nc) st_io(p.dv, voff + (size_t)i * vrow + 4 * tx + c, p.bf16, bet[i] * acc[r][c]);
+                }
+                db[r] += row_sum16(part);
+            }
+        }
+        st_nat(s.dA + ch * 4096, 64, accA);      // waits in L2 while the registers serve the key tiles
+    }
     for (int kt = 0; kt < KT; ++kt) {
-        float aR[4][4], aE[4][4], aW[4][4];
+        float aR[4][4], aE[4][4], aW[4][4], dd = 0.f;
         zero_acc(aR);
         zero_acc(aE);
         zero_acc(aW);
-        float dd = 0.f;   // threads < 64: sum_v dH'[k][v] H[k][v]
         for (int vt = 0; vt < VT; ++vt) {
-            const int nc = min(64, V - vt * 64);
-            const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
             __syncthreads();
-            ld_tile_io<true>(P0, d_o, bf16, voff, (size_t)H * V, len, nc);                   // dO^T
-            ld_tile<true>(P1, w.Z + ch * kChunk * Vp + vt * 64, Vp);                          // Z^T
-            ld_tile<true>(P2, s.dZ + ch * kChunk * Vp + vt * 64, Vp);                         // dZ^T
-            ld_tile<true>(P3, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);                 // [v][k] = H[k][v]
-            ld_tile<true>(P4, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);                // [v][k] = dH'[k][v]
-            __syncthreads();
-            mm64(aR, P0, P3);
-            mm64(aE, P1, P4);
-            mm64(aW, P2, P3);
-            if (tid < 64) {
-                for (int vv = 0; vv < 64; ++vv) dd += P3[vv * kLD + tid] * P4[vv * kLD + tid];
+            if (VT > 1) {
+                const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
+                ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, V - vt * 64, p.vec_v);
+                ld_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
+                ld_tr(t2, s.dZ + ch * 64 * Vp + vt * 64, Vp);
             }
+            ld_tr(t4, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+            ld_tr(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+            __syncthreads();
+            mm64(aR, t0, t4);
+            mm64(aE, t1, t5);
+            mm64(aW, t2, t4);
+            for (int vv = 16 * I; vv < 16 * I + 16; ++vv) dd += t4[vv * kLD + d] * t5[vv * kLD + d];
         }
+        // ---- X -= dW Q^T, T^T dW
         __syncthreads();
-        // dW to shared in both orientations; Q^T tile for X -= dW Q^T
-        st_acc<true>(P0, aW);    // [k][i]
-        st_acc<false>(P1, aW);   // [s][k]
+        st_tr(t4, kLD, aW);
         {
-            const float* kn = w.kn + ch * kChunk * Kp + kt * 64;
-            const float* G = w.G + ch * kChunk * Kp + kt * 64;
-            for (int idx = tid; idx < 4096; idx += 256) {
-                int ss = idx >> 6, d = idx & 63;
-                P2[d * kLD + ss] = bet[ss] * expf(G[(size_t)ss * Kp + d]) * kn[(size_t)ss * Kp + d];   // [k][s] = Q[s][k]
+            float x[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const size_t o = (size_t)(16 * I + r) * Kp + kt * 64 + d;
+                x[r] = bet[16 * I + r] * expf(G_g[o]) * kn_g[o];
             }
+            st_col(t5, x);
         }
+        bsum[I * 64 + d] = dd;
         __syncthreads();
         zero_acc(acc);
-        mm64(acc, P0, P2);
+        mm64(acc, t4, t5);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
             for (int c = 0; c < 4; ++c) accX[r][c] -= acc[r][c];
+        __syncthreads();
+        st_nat(t4, kLD, aW);
+        __syncthreads();
         zero_acc(acc);
-        mm64(acc, Tr, P1);     // (T^T dW)[i][k];  dQ = -that
-        // element-wise part on this thread's 4x4 patch
-        const float* Gp = w.G + ch * kChunk * Kp + kt * 64;
-        const float* qp = w.qn + ch * kChunk * Kp + kt * 64;
-        const float* kp = w.kn + ch * kChunk * Kp + kt * 64;
-        float colE[4] = {0.f, 0.f, 0.f, 0.f};
+        mm64(acc, t3, t4);
+        // ---- the direct parts of dq, dk, dG, dbeta and dG_end
+        float ga[4][4], qa[4][4], ka[4][4], colE[4] = {0.f, 0.f, 0.f, 0.f};
+        ld_patch(ga, G_g + kt * 64, Kp);
+        ld_patch(qa, qn_g + kt * 64, Kp);
+        ld_patch(ka, kn_g + kt * 64, Kp);
+        const float4 e4 = *reinterpret_cast<const float4*>(G_g + (size_t)63 * Kp + kt * 64 + 4 * tx);
+        const float ea[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int i = 4 * ty + r;
-            const float bi = bet[i];
-            float4 g4 = *reinterpret_cast<const float4*>(Gp + (size_t)i * Kp + 4 * tx);
-            float4 q4 = *reinterpret_cast<const float4*>(qp + (size_t)i * Kp + 4 * tx);
-            float4 k4 = *reinterpret_cast<const float4*>(kp + (size_t)i * Kp + 4 * tx);
-            float4 e4 = *reinterpret_cast<const float4*>(Gp + (size_t)63 * Kp + 4 * tx);
-            const float ga[4] = {g4.x, g4.y, g4.z, g4.w}, qa[4] = {q4.x, q4.y, q4.z, q4.w};
-            const float ka[4] = {k4.x, k4.y, k4.z, k4.w}, ea[4] = {e4.x, e4.y, e4.z, e4.w};
-            float oq[4], ok[4], og[4];
+            const float bi = bet[4 * ty + r];
             float brow = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const float eg = expf(ga[c]);
-                const float ee = expf(ea[c] - ga[c]);
-                const float R = qa[c] * eg, E = ka[c] * ee;
-                const float dQ = -acc[r][c];
-                oq[c] = aR[r][c] * eg;
-                ok[c] = aE[r][c] * ee + dQ * bi * eg;
-                og[c] = aR[r][c] * R - aE[r][c] * E + dQ * bi * eg * ka[c];
-                brow += dQ * eg * ka[c];
+                const float eg = expf(ga[r][c]), ee = expf(ea[c] - ga[r][c]);
+                const float R = qa[r][c] * eg, E = ka[r][c] * ee, dQ = -acc[r][c] * eg;
+                brow += dQ * ka[r][c];
                 colE[c] += aE[r][c] * E;
+                ga[r][c] = aR[r][c] * R - aE[r][c] * E + dQ * bi * ka[r][c];      // dG
+                qa[r][c] = aR[r][c] * eg;                                          // dq
+                ka[r][c] = aE[r][c] * ee + dQ * bi;                                // dk
             }
-            *reinterpret_cast<float4*>(s.dqn + (ch * kChunk + i) * Kp + kt * 64 + 4 * tx) = make_float4(oq[0], oq[1], oq[2], oq[3]);
-            *reinterpret_cast<float4*>(s.dkn + (ch * kChunk + i) * Kp + kt * 64 + 4 * tx) = make_float4(ok[0], ok[1], ok[2], ok[3]);
-            *reinterpret_cast<float4*>(s.dG + (ch * kChunk + i) * Kp + kt * 64 + 4 * tx) = make_float4(og[0], og[1], og[2], og[3]);
-            red[i * 17 + tx] = brow;
+            db[r] += row_sum16(brow);
         }
+        const size_t so = ch * 64 * Kp + kt * 64;
+        st_nat(s.dqn + so, Kp, qa);
+        st_nat(s.dkn + so, Kp, ka);
+        st_nat(s.dG + so, Kp, ga);
+        *reinterpret_cast<float4*>(t5 + ty * 64 + 4 * tx) = make_float4(colE[0], colE[1], colE[2], colE[3]);      // Q^T is read out
         __syncthreads();
         if (tid < 64) {
             float t = 0.f;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) t += red[tid * 17 + j];
-            dbv[tid] += t;
-        }
-        __syncthreads();
-        // column sums of dE*E over the 64 rows -> dG_end
-#pragma unroll
-        for (int c = 0; c < 4; ++c) red[ty * 64 + 4 * tx + c] = colE[c];
-        __syncthreads();
-        if (tid < 64) {
-            float t = 0.f;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) t += red[j * 64 + tid];
-            const float ge = Gp[(size_t)63 * Kp + tid];
-            s.dGend[ch * Kp + kt * 64 + tid] = t + expf(ge) * dd;
+            for (int j = 0; j < 16; ++j) t += t5[j * 64 + tid];
+            gend[kt * 64 + tid] = t + expf(G_g[(size_t)63 * Kp + kt * 64 + tid]) * (bsum[tid] + bsum[64 + tid] + bsum[128 + tid] + bsum[192 + tid]);
         }
     }
-
-    // ---- dM = -stril(T^T X T^T),  dA = tril(dO Z^T)
+    // ---- dM = -stril(T^T X T^T), dA = tril(dO Z^T)
+    float accA[4][4], accM[4][4];
     __syncthreads();
-    st_acc<false>(P0, accX);         // X row-major: [s][j]
-    __syncthreads();
-    zero_acc(acc);
-    mm64(acc, Tr, P0);               // Y[i][j] = sum_s T[s][i] X[s][j]
-    __syncthreads();
-    st_acc<true>(P1, acc);           // [s][i] = Y[i][s]
+    st_nat(t4, kLD, accX);
+    ld_tr(t2, w.T + ch * 4096, 64);
     __syncthreads();
     zero_acc(acc);
-    mm64(acc, P1, Tt);               // sum_s Y[i][s] T[j][s]   (Tt[s][j] = T[j][s])
-    float* dAo = s.dA + ch * 4096;
-    float* dMo = s.dM + ch * 4096;
+    mm64(acc, t3, t4);
+    st_tr(t5, kLD, acc);
+    __syncthreads();
+    zero_acc(accM);
+    mm64(accM, t5, t2);
+    ld_patch(accA, s.dA + ch * 4096, 64);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int i = 4 * ty + r;
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int j = 4 * tx + c;
-            dAo[i * 64 + j] = (j <= i) ? accA[r][c] : 0.f;
-            dMo[i * 64 + j] = (j < i) ? -acc[r][c] : 0.f;
+            const int i = 4 * ty + r, j = 4 * tx + c;
+            accA[r][c] = j <= i ? accA[r][c] : 0.f;
+            accM[r][c] = j < i ? -accM[r][c] : 0.f;
         }
-    }
-    __syncthreads();
-    if (tid < 64) s.dbl[ch * kChunk + tid] = dbv[tid];
-}
-
-// ---------------------------------------------------------------------------------------------
-// K8  pull dA, dM back through the decay-masked products; finish dG and emit dg
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) pullback_kernel(Ws w, Scr s, void* __restrict__ dg, int bf16) {
-    extern __shared__ __align__(16) float sm[];
-    float* dAs = sm;                // [i][s]
-    float* dMs = dAs + 64 * kLD;    // [i][s]
-    float* qs = dMs + 64 * kLD;     // [i][d]
-    float* ks = qs + 64 * kLD;
-    float* Gs = ks + 64 * kLD;
-    float* dGs = Gs + 64 * kLD;     // [i][d] accumulated dG
-    float* red = dGs + 64 * kLD;    // [64][2]
-    const int slot = blockIdx.x, h = blockIdx.y, kt = blockIdx.z;
-    const int len = w.chunk_len[slot];
-    if (len == 0) return;
-    const size_t ch = (size_t)slot * w.H + h;
-    const int Kp = w.Kp, KT = Kp / 64, K = w.K;
-    const int tid = threadIdx.x;
-    const float* bet = w.beta + ch * kChunk;
-    ld_tile<false>(dAs, s.dA + ch * 4096, 64);
-    ld_tile<false>(dMs, s.dM + ch * 4096, 64);
-    ld_tile<false>(qs, w.qn + ch * kChunk * Kp + kt * 64, Kp);
-    ld_tile<false>(ks, w.kn + ch * kChunk * Kp + kt * 64, Kp);
-    ld_tile<false>(Gs, w.G + ch * kChunk * Kp + kt * 64, Kp);
-    ld_tile<false>(dGs, s.dG + ch * kChunk * Kp + kt * 64, Kp);
-    __syncthreads();
-    const int d = tid & 63, rg = tid >> 6;
-    float* dqn = s.dqn + ch * kChunk * Kp + kt * 64;
-    float* dkn = s.dkn + ch * kChunk * Kp + kt * 64;
-    for (int j = 0; j < 16; ++j) {
-        const int i = rg + 4 * j;
-        const float gi = Gs[i * kLD + d], qi = qs[i * kLD + d], ki = ks[i * kLD + d], bi = bet[i];
-        // row part: sources s <= i
-        float aq = 0.f, am = 0.f;
-        for (int ss = 0; ss <= i; ++ss) {
-            const float t = expf(gi - Gs[ss * kLD + d]) * ks[ss * kLD + d];
-            aq += dAs[i * kLD + ss] * t;
-            am += dMs[i * kLD + ss] * t;   // dM[i][i] == 0
+    // ---- pull-back, one key tile at a time
+    const int T0 = ty >> 2;              // 16-row block of this thread's patch rows
+    for (int kt = 0; kt < KT; ++kt) {
+        const int dd = kt * 64 + d;
+        const bool in = dd < K;
+        float L[16];
+        {
+            const size_t col = ((size_t)tok0 * H + h) * K + (in ? dd : 0);
+            float run = 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) L[r] = (16 * I + r < len && in) ? ld_io(p.g, col + (size_t)(16 * I + r) * krow, p.gbf16) : 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) L[r] = run += L[r];
         }
-        // column part: targets i2 >= i for source row i
-        float a2 = 0.f;
-        for (int i2 = i; i2 < 64; ++i2) {
-            const float rho = expf(Gs[i2 * kLD + d] - gi);
-            a2 += rho * (dAs[i2 * kLD + i] * qs[i2 * kLD + d] + bet[i2] * dMs[i2 * kLD + i] * ks[i2 * kLD + d]);
-        }
-        dqn[(size_t)i * Kp + d] += aq;
-        dkn[(size_t)i * Kp + d] += bi * am + a2;
-        dGs[i * kLD + d] += qi * aq + bi * ki * am - ki * a2;
-        // dbeta_i += sum_d kn[i][d] * am
-        float pb = warp_sum(ki * am);
-        if ((tid & 31) == 0) red[i * 2 + ((tid >> 5) & 1)] = pb;
-    }
-    __syncthreads();
-    if (tid < 64) s.dbp[(ch * KT + kt) * kChunk + tid] = red[tid * 2] + red[tid * 2 + 1];
-    // reverse cumulative sum over the rows; the chunk-end term enters at the last row
-    if (tid < 64) {
-        float run = s.dGend[ch * Kp + kt * 64 + tid];
-        const int tok0 = w.chunk_tok0[slot];
-        const int kk = kt * 64 + tid;
-        for (int i = 63; i >= 0; --i) {
-            run += dGs[i * kLD + tid];
-            if (i < len && kk < K) st_io(dg, ((size_t)(tok0 + i) * w.H + h) * K + kk, bf16, run);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
-// K9  finalize: L2-normalisation VJP for dq, dk; collect dbeta
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) finalize_kernel(Ws w, Scr s, const void* __restrict__ q, const void* __restrict__ k,
-                                                       void* __restrict__ dq, void* __restrict__ dk,
-                                                       void* __restrict__ dbeta, int bf16, int gbf16, int l2norm, float scale) {
-    const int slot = blockIdx.x, h = blockIdx.y;
-    const int len = w.chunk_len[slot];
-    if (len == 0) return;
-    const int tok0 = w.chunk_tok0[slot];
-    const size_t ch = (size_t)slot * w.H + h;
-    const int K = w.K, Kp = w.Kp, KT = Kp / 64, H = w.H;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = warp; i < len; i += 8) {
-        const size_t off = ((size_t)(tok0 + i) * H + h) * K;
-        const float* dqn = s.dqn + (ch * kChunk + i) * Kp;
-        const float* dkn = s.dkn + (ch * kChunk + i) * Kp;
-        const float qi = w.qinv[ch * kChunk + i], ki = w.kinv[ch * kChunk + i];
-        if (l2norm) {
-            float pq = 0.f, pk = 0.f;
-            for (int d = lane; d < K; d += 32) {
-                pq += ld_io(q, off + d, bf16) * qi * dqn[d] * scale;
-                pk += ld_io(k, off + d, bf16) * ki * dkn[d];
+        __syncthreads();
+        bsum[I * 64 + d] = L[15];
+        __syncthreads();
+        float pre = 0.f;
+        for (int J = 0; J < I; ++J) pre += bsum[J * 64 + d];
+        const float c = L[8];
+        cref[I * 64 + d] = pre + c;
+        bool far = false;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) far = far || !(fabsf(L[r] - c) <= kMaxExponent);
+        const bool pairwise = __syncthreads_or(far);
+        float aq[4][4], am[4][4], a2[4][4];      // with the decay factors applied, below
+        zero_acc(aq);
+        zero_acc(am);
+        zero_acc(a2);
+        if (!pairwise) {
+            // row part: (dA | dM)[i][s] k_s exp(c_I - G_s); sources of block I: rows 8 I (I + 1) .. of the array at t2
+            st_tr(t0, kLD, accA);
+            st_tr(t1, kLD, accM);
+            float kc[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) kc[r] = kn_g[(size_t)(16 * I + r) * Kp + dd] * expf(c - L[r]);
+            for (int T = I; T < 4; ++T) {
+                const float f = T == I ? 1.f : expf(cref[T * 64 + d] - cref[I * 64 + d]);
+                float* o = t2 + (8 * T * (T + 1) + 16 * I) * kLD + d;
+#pragma unroll
+                for (int r = 0; r < 16; ++r) o[r * kLD] = kc[r] * f;
             }
-            pq = warp_sum(pq);
-            pk = warp_sum(pk);
-            for (int d = lane; d < K; d += 32) {
-                const float qh = ld_io(q, off + d, bf16) * qi, kh = ld_io(k, off + d, bf16) * ki;
-                st_io(dq, off + d, bf16, qi * (dqn[d] * scale - qh * pq));
-                st_io(dk, off + d, bf16, ki * (dkn[d] - kh * pk));
+#pragma unroll
+            for (int r = 0; r < 16; ++r) t5[(16 * I + r) * kLD + d] = L[r] - c;
+            __syncthreads();
+            {
+                const float *x = t0 + 4 * ty, *y = t1 + 4 * ty, *b = t2 + 8 * T0 * (T0 + 1) * kLD + 4 * tx;
+                const int n = 16 * (T0 + 1);
+#pragma unroll 4
+                for (int kk = 0; kk < n; ++kk) {
+                    const float4 bb = *reinterpret_cast<const float4*>(b + kk * kLD);
+                    fma16(aq, *reinterpret_cast<const float4*>(x + kk * kLD), bb);
+                    fma16(am, *reinterpret_cast<const float4*>(y + kk * kLD), bb);
+                }
+            }
+            __syncthreads();
+            // column part: sum over target blocks of exp(c_T - G_s) sum_{i in T} dA[i][s] q~_i + beta_i dM[i][s] k~_i
+            st_nat(t0, kLD, accA);
+            {
+                float bm[4][4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int cc = 0; cc < 4; ++cc) bm[r][cc] = bet[4 * ty + r] * accM[r][cc];
+                st_nat(t1, kLD, bm);
+            }
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const float e = expf(L[r] - c);
+                const size_t o = (size_t)(16 * I + r) * Kp + dd;
+                t2[(16 * I + r) * kLD + d] = qn_g[o] * e;
+                t3[(16 * I + r) * kLD + d] = kn_g[o] * e;
+            }
+            __syncthreads();
+            for (int T = 3; T >= T0; --T) {
+                if (T < 3) {
+                    float f[4];
+#pragma unroll
+                    for (int cc = 0; cc < 4; ++cc) f[cc] = expf(cref[(T + 1) * 64 + 4 * tx + cc] - cref[T * 64 + 4 * tx + cc]);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc) a2[r][cc] *= f[cc];
+                }
+                mm_at(a2, t0 + 16 * T * kLD + 4 * ty, kLD, t2 + 16 * T * kLD + 4 * tx, kLD, 16);
+                mm_at(a2, t1 + 16 * T * kLD + 4 * ty, kLD, t3 + 16 * T * kLD + 4 * tx, kLD, 16);
+            }
+            float x[4][4];
+            ld_patch(x, t5, kLD);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) {
+                    const float e = expf(x[r][cc]), f = expf(-x[r][cc]);
+                    aq[r][cc] *= e;
+                    am[r][cc] *= e;
+                    a2[r][cc] *= f;
+                }
+        } else {
+            st_nat(t0, kLD, accA);
+            st_nat(t1, kLD, accM);
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const size_t o = (size_t)(16 * I + r) * Kp + dd;
+                t2[(16 * I + r) * kLD + d] = qn_g[o];
+                t3[(16 * I + r) * kLD + d] = kn_g[o];
+                t5[(16 * I + r) * kLD + d] = pre + L[r];
+            }
+            __syncthreads();
+            for (int r = 0; r < 4; ++r)
+                for (int cc = 0; cc < 4; ++cc) {
+                    const int i = 4 * ty + r, col = 4 * tx + cc;
+                    const float gi = t5[i * kLD + col];
+                    float vq = 0.f, vm = 0.f, v2 = 0.f;
+                    for (int ss = 0; ss <= i; ++ss) {
+                        const float e = expf(gi - t5[ss * kLD + col]) * t3[ss * kLD + col];
+                        vq += t0[i * kLD + ss] * e;
+                        vm += t1[i * kLD + ss] * e;
+                    }
+                    for (int ii = i; ii < 64; ++ii)
+                        v2 += expf(t5[ii * kLD + col] - gi) * (t0[ii * kLD + i] * t2[ii * kLD + col] + bet[ii] * t1[ii * kLD + i] * t3[ii * kLD + col]);
+#pragma unroll
+                    for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+                        for (int ss = 0; ss < 4; ++ss)
+                            if (rr == r && ss == cc) {
+                                aq[rr][ss] = vq;
+                                am[rr][ss] = vm;
+                                a2[rr][ss] = v2;
+                            }
+                }
+        }
+        // ---- assemble
+        const size_t so = ch * 64 * Kp + kt * 64;
+        {
+            float q[4][4], k[4][4], x[4][4];
+            ld_patch(q, qn_g + kt * 64, Kp);
+            ld_patch(k, kn_g + kt * 64, Kp);
+            ld_patch(x, s.dG + so, Kp);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float bi = bet[4 * ty + r];
+                float part = 0.f;
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) {
+                    part += k[r][cc] * am[r][cc];
+                    x[r][cc] += q[r][cc] * aq[r][cc] + bi * k[r][cc] * am[r][cc] - k[r][cc] * a2[r][cc];
+                    am[r][cc] = bi * am[r][cc] + a2[r][cc];
+                }
+                db[r] += row_sum16(part);
+            }
+            st_nat(t4, kLD, x);
+            ld_patch(q, s.dqn + so, Kp);
+            ld_patch(k, s.dkn + so, Kp);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) {
+                    aq[r][cc] += q[r][cc];
+                    am[r][cc] += k[r][cc];
+                }
+        }
+        if (KT == 1) {      // a row lies in 16 lanes: normalise here
+            const size_t koff = ((size_t)tok0 * H + h) * K;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int i = 4 * ty + r;
+                float x[4], y[4], pq = 0.f, pk = 0.f;
+                ld4_io(x, p.q, p.bf16, koff, krow, i, 4 * tx, len, K, p.vec_k);
+                ld4_io(y, p.k, p.bf16, koff, krow, i, 4 * tx, len, K, p.vec_k);
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) {
+                    x[cc] *= qi_s[i];
+                    y[cc] *= ki_s[i];
+                    aq[r][cc] *= p.scale;
+                    pq += x[cc] * aq[r][cc];
+                    pk += y[cc] * am[r][cc];
+                }
+                if (p.l2norm) {
+                    pq = row_sum16(pq);
+                    pk = row_sum16(pk);
+                }
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc)
+                    if (i < len && 4 * tx + cc < K) {
+                        const size_t o = koff + (size_t)i * krow + 4 * tx + cc;
+                        st_io(p.dq, o, p.bf16, p.l2norm ? qi_s[i] * (aq[r][cc] - x[cc] * pq) : aq[r][cc]);
+                        st_io(p.dk, o, p.bf16, p.l2norm ? ki_s[i] * (am[r][cc] - y[cc] * pk) : am[r][cc]);
+                    }
             }
         } else {
-            for (int d = lane; d < K; d += 32) {
-                st_io(dq, off + d, bf16, dqn[d] * scale);
-                st_io(dk, off + d, bf16, dkn[d]);
+            st_nat(s.dqn + so, Kp, aq);
+            st_nat(s.dkn + so, Kp, am);
+        }
+        // reverse cumulative sum of dG down the rows; the chunk-end term enters at the last one
+        __syncthreads();
+        {
+            float x[16], sum = 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) sum += x[r] = t4[(16 * I + r) * kLD + d];
+            tot[I * 64 + d] = sum;
+            __syncthreads();
+            float run = gend[dd];
+            for (int J = 3; J > I; --J) run += tot[J * 64 + d];
+#pragma unroll
+            for (int r = 15; r >= 0; --r) {
+                run += x[r];
+                const int i = 16 * I + r;
+                if (i < len && in) st_io(p.dg, ((size_t)tok0 * H + h) * K + (size_t)i * krow + dd, p.gbf16, run);
             }
         }
-        if (lane == 0) {
-            float b = s.dbl[ch * kChunk + i];
-            for (int kt = 0; kt < KT; ++kt) b += s.dbp[(ch * KT + kt) * kChunk + i];
-            st_io(dbeta, (size_t)(tok0 + i) * H + h, gbf16, b);
+    }
+    if (tx == 0) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (4 * ty + r < len) st_io(p.dbeta, (size_t)(tok0 + 4 * ty + r) * H + h, p.gbf16, db[r]);
+    }
+    if (KT > 1) {
+        __syncthreads();
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int i = warp; i < len; i += 8) {
+            const size_t off = ((size_t)(tok0 + i) * H + h) * K;
+            const float* dqn = s.dqn + (ch * 64 + i) * Kp;
+            const float* dkn = s.dkn + (ch * 64 + i) * Kp;
+            const float qi = qi_s[i], ki = ki_s[i];
+            float pq = 0.f, pk = 0.f;
+            if (p.l2norm) {
+                for (int e = lane; e < K; e += 32) {
+                    pq += ld_io(p.q, off + e, p.bf16) * qi * dqn[e] * p.scale;
+                    pk += ld_io(p.k, off + e, p.bf16) * ki * dkn[e];
+                }
+                pq = warp_sum(pq);
+                pk = warp_sum(pk);
+            }
+            for (int e = lane; e < K; e += 32) {
+                if (p.l2norm) {
+                    st_io(p.dq, off + e, p.bf16, qi * (dqn[e] * p.scale - ld_io(p.q, off + e, p.bf16) * qi * pq));
+                    st_io(p.dk, off + e, p.bf16, ki * (dkn[e] - ld_io(p.k, off + e, p.bf16) * ki * pk));
+                } else {
+                    st_io(p.dq, off + e, p.bf16, dqn[e] * p.scale);
+                    st_io(p.dk, off + e, p.bf16, dkn[e]);
+                }
+            }
         }
     }
 }
@@ -951,6 +1248,17 @@ static int set_smem(Kern kern, size_t bytes) {
     return bytes > 48 * 1024 ? set_smem_limit(kern, bytes) : KDA_OK;
 }
 
+// four-element accesses along a tensor's last dimension are aligned
+static int vec4(const void* p, int dim) { return dim % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+static int launch_scan(const Ws& w, int n_seq, const simt::ScanArgs& a, const char* name, cudaStream_t st) {
+    const size_t bytes = (size_t)(simt::kScanStages * 4096 + 4 * 64 * simt::kVS + w.Kp * simt::kVS) * sizeof(float);
+    if (set_smem(simt::scan_kernel, bytes)) return KDA_ERR_CUDA;
+    // padding strips hold zeros already: E^T U and Rm^T dO of zero columns
+    KDA_LAUNCH(name, st, simt::scan_kernel<<<dim3(n_seq, w.H, ceil_div(w.V, simt::kVS)), 256, bytes, st>>>(w, a));
+    return launch_status();
+}
+
 int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const void* v, const void* g, const void* beta,
                    const float* h0, const int32_t* cu, void* o, float* final_state, void* workspace, cudaStream_t st,
                    const tc::NormEpilogue* norm, const tc::ConvPrep* conv) {
@@ -976,22 +1284,16 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         return launch_status();
     }
     KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status, status_mirror()));
+    const dim3 gch(w.nslots, w.H);
     if (w.nslots > 0) {
-        dim3 gch(w.nslots, w.H);
-        KDA_LAUNCH("prep_kernel", st, simt::prep_kernel<<<gch, 256, 0, st>>>(w, q, k, g, beta, bf16, gbf16, sh->l2norm, sh->scale));
-        size_t sm_am = (size_t)(5 * 64 + 32) * kLD * sizeof(float);
-        if (set_smem(simt::build_am_kernel, sm_am)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("build_am_kernel", st, simt::build_am_kernel<<<gch, 256, sm_am, st>>>(w));
-        size_t sm_uw = (size_t)2 * 64 * kLD * sizeof(float);
-        KDA_LAUNCH("uw_kernel", st, simt::uw_kernel<<<dim3(w.nslots, w.H, KT + VT), 256, sm_uw, st>>>(w, v, bf16));
+        const simt::IntraArgs a{q, k, v, g, beta, bf16, gbf16, sh->l2norm, vec4(v, sh->value_dim), sh->forward_only ? 0 : 1, sh->scale};
+        if (set_smem(simt::intra_fwd_kernel, simt::kIntraSmem)) return KDA_ERR_CUDA;
+        KDA_LAUNCH("intra_fwd_kernel", st, simt::intra_fwd_kernel<<<gch, 256, simt::kIntraSmem, st>>>(w, a));
     }
-    {
-        size_t sm_scan = ((size_t)2 * 64 * (w.Kp + 1) + (size_t)w.Kp * simt::kVS + 64 * simt::kVS + w.Kp) * sizeof(float);
-        if (set_smem(simt::scan_fwd_kernel, sm_scan)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("scan_fwd_kernel", st, simt::scan_fwd_kernel<<<dim3(sh->n_seq, w.H, w.Vp / simt::kVS), 256, sm_scan, st>>>(w, h0, final_state));
-    }
+    if (int rc = launch_scan(w, sh->n_seq, simt::ScanArgs{w.PT, w.Hc, h0, final_state, 0}, "scan_fwd_kernel", st)) return rc;
     if (w.nslots > 0) {
-        size_t sm_out = (size_t)2 * 64 * kLD * sizeof(float);
+        const size_t sm_out = (size_t)3 * simt::kTile * sizeof(float);
+        if (set_smem(simt::out_kernel, sm_out)) return KDA_ERR_CUDA;
         KDA_LAUNCH("out_kernel", st, simt::out_kernel<<<dim3(w.nslots, w.H, VT), 256, sm_out, st>>>(w, o, bf16));
     }
     return launch_status();
@@ -1042,21 +1344,19 @@ int simt_chunk_bwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         } else if (dh0) {
             return KDA_ERR_UNSUPPORTED;
         }
-    } else {
-        size_t sm_scan = ((size_t)2 * 64 * (w.Kp + 1) + 64 * kLD + (size_t)2 * w.Kp * simt::kVS + 2 * 64 * simt::kVS + w.Kp) *
-                         sizeof(float);
-        if (set_smem(simt::scan_bwd_kernel, sm_scan)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("scan_bwd_kernel", st, simt::scan_bwd_kernel<<<dim3(sh->n_seq, w.H, w.Vp / simt::kVS), 256, sm_scan, st>>>(w, s, d_o, bf16, d_final, dh0));
+        return launch_status();
     }
+    const int vec_v = vec4(v, sh->value_dim) && vec4(d_o, sh->value_dim);
     if (w.nslots > 0) {
-        dim3 gch(w.nslots, w.H);
-        size_t sm_loc = ((size_t)7 * 64 * kLD + 64 * 17 + 128) * sizeof(float);
-        if (set_smem(simt::bwd_local_kernel, sm_loc)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("bwd_local_kernel", st, simt::bwd_local_kernel<<<gch, 256, sm_loc, st>>>(w, s, v, d_o, dv, bf16));
-        size_t sm_pb = ((size_t)6 * 64 * kLD + 128) * sizeof(float);
-        if (set_smem(simt::pullback_kernel, sm_pb)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("pullback_kernel", st, simt::pullback_kernel<<<dim3(w.nslots, w.H, KT), 256, sm_pb, st>>>(w, s, dg, gbf16));
-        KDA_LAUNCH("finalize_kernel", st, simt::finalize_kernel<<<gch, 256, 0, st>>>(w, s, q, k, dq, dk, dbeta, bf16, gbf16, sh->l2norm, sh->scale));
+        const size_t sm_term = (size_t)2 * simt::kTile * sizeof(float);
+        KDA_LAUNCH("adjoint_term_kernel", st, simt::adjoint_term_kernel<<<dim3(w.nslots, w.H, KT * (w.Vp / 64)), 256, sm_term, st>>>(w, s, d_o, bf16, vec_v));
+    }
+    if (int rc = launch_scan(w, sh->n_seq, simt::ScanArgs{w.P, s.dHn, d_final, dh0, 1}, "scan_bwd_kernel", st)) return rc;
+    if (w.nslots > 0) {
+        const simt::LocalArgs a{q, k, v, g, d_o, dq, dk, dv, dg, dbeta, bf16, gbf16, sh->l2norm,
+                                vec4(q, sh->key_dim) && vec4(k, sh->key_dim), vec_v, sh->scale};
+        if (set_smem(simt::local_bwd_kernel, simt::kLocalSmem)) return KDA_ERR_CUDA;
+        KDA_LAUNCH("local_bwd_kernel", st, simt::local_bwd_kernel<<<dim3(w.nslots, w.H), 256, simt::kLocalSmem, st>>>(w, s, a));
     }
     return launch_status();
 }

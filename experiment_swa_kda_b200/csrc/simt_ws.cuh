@@ -11,23 +11,25 @@ namespace simt {
 struct Ws {
     int *chunk_seq, *chunk_tok0, *chunk_len, *seq_chunk0;
     int* seq_order;             // [n_seq] sequences by falling chunk count: the order the state scans start them in
-    float *qn, *kn, *G, *W;     // [nch][64][Kp]   scaled unit q, unit k, cumulative log-decay, W
-    float* Z;                   // [nch][64][Vp]   U after the intra-chunk step, Z after the scan
-    float *A, *T;               // [nch][64][64]
-    float* Hc;                  // [nch][Kp][Vp]   state at the start of each chunk
+    // float32 lane, per chunk-head.  R = qn e^G, E = kn e^{G_end - G}; ...T arrays are transposed
+    float *kn, *G;              // [64][Kp]   unit k, cumulative log-decay
+    float *qn, *Rm;             // [64][Kp]   scaled unit q; R - A W (backward only)
+    float *W, *WT, *RT;         // [64][Kp], [Kp][64], [Kp][64]
+    float* Z;                   // [64][Vp]   U after the intra-chunk step, Z after the output kernel
+    float *AT, *A, *T;          // [64][64]   A and T: backward only
+    float *PT, *P;              // [Kp][Kp]   (E^T W)^T, and E^T W for the adjoint scan (backward only)
+    float* Hc;                  // [Kp][Vp]   E^T U, replaced by the chunk-start state in the scan
+    float* dec;                 // [Kp]       exp(G_end)
     float *qinv, *kinv, *beta;  // [nch][64]
     int* status;                // device status word of the forward / backward pair that owns this workspace (0 = ok)
     int nslots, H, K, V, Kp, Vp;
 };
 
 struct Scr {
-    float* dZ;              // [nch][64][Vp]
-    float* dHn;             // [nch][Kp][Vp]   adjoint of each chunk's outgoing state
+    float* dHn;             // [nch][Kp][Vp]   Rm^T dO, replaced by the adjoint of each chunk's outgoing state in the scan
     float *dqn, *dkn, *dG;  // [nch][64][Kp]
-    float *dA, *dM;         // [nch][64][64]
-    float* dGend;           // [nch][Kp]
-    float* dbl;             // [nch][64]
-    float* dbp;             // [nch][KT][64]
+    float* dA;              // [nch][64][64]
+    float* dZ;              // [nch][64][Vp]   only when V > 64 (one value tile stays on chip)
 };
 
 inline int slots_for(const KdaChunkShape& sh, bool varlen_hint) {
@@ -69,14 +71,22 @@ inline Ws carve_ws(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr) 
     w.chunk_len = c.take<int>(w.nslots + 1);
     w.seq_chunk0 = c.take<int>(sh.n_seq + 1);
     w.seq_order = c.take<int>(sh.n_seq);
-    w.qn = c.take<float>(big * nch * 64 * w.Kp);
+    const size_t bw = sh.forward_only ? 0 : big;      // arrays only a backward reads
     w.kn = c.take<float>(big * nch * 64 * w.Kp);
     w.G = c.take<float>(big * nch * 64 * w.Kp);
+    w.qn = c.take<float>(bw * nch * 64 * w.Kp);
+    w.Rm = c.take<float>(bw * nch * 64 * w.Kp);
     w.W = c.take<float>(big * nch * 64 * w.Kp);
+    w.WT = c.take<float>(big * nch * 64 * w.Kp);
+    w.RT = c.take<float>(big * nch * 64 * w.Kp);
     w.Z = c.take<float>(big * nch * 64 * w.Vp);
-    w.A = c.take<float>(big * nch * 4096);
-    w.T = c.take<float>(big * nch * 4096);
+    w.AT = c.take<float>(big * nch * 4096);
+    w.A = c.take<float>(bw * nch * 4096);
+    w.T = c.take<float>(bw * nch * 4096);
+    w.PT = c.take<float>(big * nch * w.Kp * w.Kp);
+    w.P = c.take<float>(bw * nch * w.Kp * w.Kp);
     w.Hc = c.take<float>(big * nch * w.Kp * w.Vp);
+    w.dec = c.take<float>(big * nch * w.Kp);
     w.qinv = c.take<float>(nch * 64);
     w.kinv = c.take<float>(nch * 64);
     w.beta = c.take<float>(nch * 64);
@@ -90,16 +100,12 @@ inline Scr carve_scr(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr
     const int Kp = ceil_div(sh.key_dim, 64) * 64, Vp = ceil_div(sh.value_dim, 64) * 64;
     const size_t nch = sh.lane == KDA_LANE_TC ? 0 : (size_t)slots_for(sh, false) * sh.heads;   // float32 lane only
     Carver c(mem);
-    s.dZ = c.take<float>(nch * 64 * Vp);
     s.dHn = c.take<float>(nch * Kp * Vp);
     s.dqn = c.take<float>(nch * 64 * Kp);
     s.dkn = c.take<float>(nch * 64 * Kp);
     s.dG = c.take<float>(nch * 64 * Kp);
     s.dA = c.take<float>(nch * 4096);
-    s.dM = c.take<float>(nch * 4096);
-    s.dGend = c.take<float>(nch * Kp);
-    s.dbl = c.take<float>(nch * 64);
-    s.dbp = c.take<float>(nch * (Kp / 64) * 64);
+    s.dZ = c.take<float>(Vp > 64 ? nch * 64 * Vp : 0);
     if (bytes) *bytes = align_up(c.off, 256);
     return s;
 }
