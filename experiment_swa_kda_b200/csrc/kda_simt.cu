@@ -53,6 +53,27 @@ __device__ __forceinline__ void ld_tr(float* dst, const float* __restrict__ src,
         dst[(c4 + 3) * kLD + r] = x.w;
     }
 }
+// the same two as asynchronous copies: commit with cpa_commit, then cpa_wait and a barrier
+__device__ __forceinline__ void cpa_nat(float* dst, const float* __restrict__ src, size_t ld) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = threadIdx.x + 256 * it, r = idx >> 4, c4 = (idx & 15) << 2;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + (r * kLD + c4) * 4), "l"(src + (size_t)r * ld + c4) : "memory");
+    }
+}
+// transposed, element by element: a warp takes 4 rows x 8 columns, whole 32-byte sectors and 32 different banks
+__device__ __forceinline__ void cpa_tr(float* dst, const float* __restrict__ src, size_t ld) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int warp = threadIdx.x >> 5, r0 = threadIdx.x & 3, q0 = (threadIdx.x & 31) >> 2;
+#pragma unroll
+    for (int it = 0; it < 16; ++it) {
+        const int r = 4 * it + r0, c = 8 * warp + q0;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + (c * kLD + r) * 4), "l"(src + (size_t)r * ld + c) : "memory");
+    }
+}
+__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 // four adjacent elements of a caller tensor, zero outside nr x nc; vec: the tensor allows 4-element accesses
 __device__ __forceinline__ void ld4_io(float (&x)[4], const void* base, int bf16, size_t off, size_t stride, int r, int c4, int nr, int nc, int vec) {
     const size_t i = off + (size_t)r * stride + c4;
@@ -574,11 +595,16 @@ __global__ void __launch_bounds__(256, 2) intra_fwd_kernel(Ws w, IntraArgs p) {
 // K2  state scan over the chunks of one (sequence, head, 16-column value strip), in either direction:
 //     forward  S = H:   S' = dec . S + B - P S       B = E^T U, leaves the chunk-start states in its place
 //     backward S = dH': S' = dec . S + B - P^T S     B = Rm^T dO, leaves the adjoints of the outgoing states
-// A step is one Kp x Kp product against a 16-column strip.  Its matrix comes through a ring of 64x64 tiles filled by
-// asynchronous copies ahead of the step, four groups of two warps share the contraction, and the strip lives in registers
-// (one float4 per thread and 64-row block) and, for the products, in shared memory.
+// A step is one Kp x Kp product against a 16-column strip.  What a step reads (its matrix as 64x64 tiles, its strip of B,
+// its decay) comes through a ring filled by asynchronous copies three tiles ahead; four groups of two warps share the
+// contraction and meet in shared memory, laid out so that no access of the step has a bank conflict.  The strip lives in
+// registers (thread = row x 4 columns) and, for the products, in shared memory.  1.9 us a step at K = 64 while B was loaded
+// one step ahead into registers and the partial sums conflicted; 0.7 now, a chain of four barriers and 16 x 18 instructions.
 // ---------------------------------------------------------------------------------------------
 constexpr int kVS = 16, kScanStages = 4;
+constexpr int kStageFloats = 4096 + 64 * kVS + 64;      // tile, strip of B, decay of one 64-row block
+constexpr int kSLD = 20;                                // row stride of the shared strip
+constexpr int kPartBlock = 72;                          // float4s per (group, column quad): row 4 l + r at r * 18 + l
 
 struct ScanArgs {
     const float* M;       // [ch][Kp][Kp], contraction index leading: P^T forward, P backward
@@ -587,117 +613,107 @@ struct ScanArgs {
     float* s_out;
     int backward;
 };
+inline size_t scan_smem(int Kp) { return (size_t)(kScanStages * kStageFloats + 16 * kPartBlock * 4 + Kp * kSLD) * sizeof(float); }
 
+template <int KT>
 __global__ void __launch_bounds__(256) scan_kernel(Ws w, ScanArgs p) {
     extern __shared__ __align__(16) float sm[];
-    float* ring = sm;                                  // [stages][64][64]
-    float* part = ring + kScanStages * 4096;           // [4][64][16]
-    float* S = part + 4 * 64 * kVS;                    // [Kp][16]
-    const int Kp = w.Kp, Vp = w.Vp, K = w.K, V = w.V, H = w.H, KT = Kp / 64;
+    float* ring = sm;
+    float4* part = reinterpret_cast<float4*>(ring + kScanStages * kStageFloats);
+    float* S = reinterpret_cast<float*>(part + 16 * kPartBlock);      // [Kp][kSLD]
+    const int Kp = 64 * KT, Vp = w.Vp, K = w.K, V = w.V, H = w.H;
     const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kVS, tid = threadIdx.x;
     const int c0 = w.seq_chunk0[seq], c1 = w.seq_chunk0[seq + 1], n = c1 - c0;
-    const int row = tid >> 2, c4 = (tid & 3) << 2;      // this thread's float4 of a 64-row block
-    const int kg = tid >> 6, pr = (tid & 15) << 2, pc = ((tid >> 4) & 3) << 2;      // product: contraction group, rows, columns
+    const int row = tid & 63, cq = tid >> 6;                          // the state element group this thread owns in every 64-row block
+    const int l = tid & 15, pq = (tid >> 4) & 3, kg = tid >> 6;       // product: rows 4 l .., column quad, contraction group
+    const int grow = tid >> 2, gc = (tid & 3) << 2;                   // global rows of 64 bytes
     auto chunk = [&](int step) { return (size_t)(p.backward ? c1 - 1 - step : c0 + step) * H + h; };
     const int tiles = n * KT * KT;
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+    auto cp16 = [](uint32_t dst, const float* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); };
     auto issue = [&](int t) {      // tile t: step, then output block, then contraction block
         if (t < tiles) {
             const int step = t / (KT * KT), rt = (t / KT) % KT, kt = t % KT;
-            const float* src = p.M + (chunk(step) * Kp + kt * 64) * Kp + rt * 64;
+            const size_t ch = chunk(step);
+            const float* src = p.M + (ch * Kp + kt * 64) * Kp + rt * 64;
+            const uint32_t dst = ring_s + (t % kScanStages) * kStageFloats * 4;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int idx = tid + 256 * i, r = idx >> 4, c = (idx & 15) << 2;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_s + ((t % kScanStages) * 4096 + r * 64 + c) * 4), "l"(src + (size_t)r * Kp + c)
-                             : "memory");
+                cp16(dst + (r * 64 + c) * 4, src + (size_t)r * Kp + c);
+            }
+            if (kt == 0) {
+                cp16(dst + (4096 + tid * 4) * 4, p.B + (ch * Kp + rt * 64 + grow) * Vp + v0 + gc);
+                if (tid < 16) cp16(dst + (4096 + 64 * kVS + tid * 4) * 4, w.dec + ch * Kp + rt * 64 + tid * 4);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float4 s[4], b[4];
-    float dec[4];
-    auto load_step = [&](int step) {
-        if (step < n) {
-            const size_t ch = chunk(step);
+    float4 s[KT];
 #pragma unroll
-            for (int rt = 0; rt < 4; ++rt)
-                if (rt < KT) {
-                    b[rt] = *reinterpret_cast<const float4*>(p.B + (ch * Kp + rt * 64 + row) * Vp + v0 + c4);
-                    dec[rt] = w.dec[ch * Kp + rt * 64 + row];
-                }
-        }
-    };
-#pragma unroll
-    for (int rt = 0; rt < 4; ++rt) {
+    for (int rt = 0; rt < KT; ++rt) {
         s[rt] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int kk = rt * 64 + row;
-        if (rt < KT && p.s_in && kk < K) {
-            const float* src = p.s_in + (((size_t)seq * H + h) * V + v0 + c4) * K + kk;
-            if (v0 + c4 + 0 < V) s[rt].x = src[0];
-            if (v0 + c4 + 1 < V) s[rt].y = src[K];
-            if (v0 + c4 + 2 < V) s[rt].z = src[2 * (size_t)K];
-            if (v0 + c4 + 3 < V) s[rt].w = src[3 * (size_t)K];
+        const int kk = rt * 64 + row, vv = v0 + 4 * cq;
+        if (p.s_in && kk < K) {
+            const float* src = p.s_in + (((size_t)seq * H + h) * V + vv) * K + kk;
+            if (vv + 0 < V) s[rt].x = src[0];
+            if (vv + 1 < V) s[rt].y = src[K];
+            if (vv + 2 < V) s[rt].z = src[2 * (size_t)K];
+            if (vv + 3 < V) s[rt].w = src[3 * (size_t)K];
         }
-        if (rt < KT) *reinterpret_cast<float4*>(S + kk * kVS + c4) = s[rt];
+        *reinterpret_cast<float4*>(S + kk * kSLD + 4 * cq) = s[rt];
     }
     for (int t = 0; t < kScanStages - 1; ++t) issue(t);
-    load_step(0);
     int t = 0;
     for (int step = 0; step < n; ++step) {
         const size_t ch = chunk(step);
-        float4 bc[4];
-        float dc[4];
 #pragma unroll
-        for (int rt = 0; rt < 4; ++rt) {
-            bc[rt] = b[rt];
-            dc[rt] = dec[rt];
-            if (rt < KT) *reinterpret_cast<float4*>(p.B + (ch * Kp + rt * 64 + row) * Vp + v0 + c4) = s[rt];      // the state the chunk sees
-        }
-        load_step(step + 1);
         for (int rt = 0; rt < KT; ++rt) {
             float acc[4][4];
             zero_acc(acc);
+#pragma unroll
             for (int kt = 0; kt < KT; ++kt, ++t) {
                 asm volatile("cp.async.wait_group %0;" ::"n"(kScanStages - 2) : "memory");
-                __syncthreads();                       // tile t has landed for everyone; tile t - 1 and (rt = 0) the old strip are read out
+                __syncthreads();                       // tile t has landed for everyone; tile t - 1 and (rt = 0) the old partials are read out
                 issue(t + kScanStages - 1);
-                mm_at(acc, ring + (t % kScanStages) * 4096 + 16 * kg * 64 + pr, 64, S + (kt * 64 + 16 * kg) * kVS + pc, kVS, 16);
+                const float* stage = ring + (t % kScanStages) * kStageFloats;
+                mm_at(acc, stage + 16 * kg * 64 + 4 * l, 64, S + (kt * 64 + 16 * kg) * kSLD + 4 * pq, kSLD, 16);
+                if (kt == 0) {
+                    const float* bd = stage + 4096;    // this block's strip of B and decay
+                    const float4 b = *reinterpret_cast<const float4*>(bd + row * kVS + 4 * cq);
+                    const float dc = bd[64 * kVS + row];
+                    // the state the chunk sees takes B's place in memory (B of this block has landed), then the row's own terms
+                    *reinterpret_cast<float4*>(p.B + (ch * Kp + rt * 64 + grow) * Vp + v0 + gc) = *reinterpret_cast<const float4*>(S + (rt * 64 + grow) * kSLD + gc);
+                    s[rt].x = dc * s[rt].x + b.x;
+                    s[rt].y = dc * s[rt].y + b.y;
+                    s[rt].z = dc * s[rt].z + b.z;
+                    s[rt].w = dc * s[rt].w + b.w;
+                }
             }
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-                *reinterpret_cast<float4*>(part + (kg * 64 + pr + r) * kVS + pc) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            for (int r = 0; r < 4; ++r) part[(kg * 4 + pq) * kPartBlock + r * 18 + l] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
             __syncthreads();
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                const float4 y = *reinterpret_cast<const float4*>(part + (g * 64 + row) * kVS + c4);
-                x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+                const float4 y = part[(g * 4 + cq) * kPartBlock + (row & 3) * 18 + (row >> 2)];
+                s[rt].x -= y.x; s[rt].y -= y.y; s[rt].z -= y.z; s[rt].w -= y.w;
             }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (q == rt) {
-                    s[q].x = dc[q] * s[q].x + bc[q].x - x.x;
-                    s[q].y = dc[q] * s[q].y + bc[q].y - x.y;
-                    s[q].z = dc[q] * s[q].z + bc[q].z - x.z;
-                    s[q].w = dc[q] * s[q].w + bc[q].w - x.w;
-                }
         }
-        __syncthreads();                               // every product has read the strip
+        if (KT > 1) __syncthreads();                   // every block's products have read the strip (one block: the barrier above)
 #pragma unroll
-        for (int rt = 0; rt < 4; ++rt)
-            if (rt < KT) *reinterpret_cast<float4*>(S + (rt * 64 + row) * kVS + c4) = s[rt];
+        for (int rt = 0; rt < KT; ++rt) *reinterpret_cast<float4*>(S + (rt * 64 + row) * kSLD + 4 * cq) = s[rt];
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (p.s_out) {
 #pragma unroll
-        for (int rt = 0; rt < 4; ++rt) {
-            const int kk = rt * 64 + row;
-            if (rt < KT && kk < K) {
-                float* dst = p.s_out + (((size_t)seq * H + h) * V + v0 + c4) * K + kk;
-                if (v0 + c4 + 0 < V) dst[0] = s[rt].x;
-                if (v0 + c4 + 1 < V) dst[K] = s[rt].y;
-                if (v0 + c4 + 2 < V) dst[2 * (size_t)K] = s[rt].z;
-                if (v0 + c4 + 3 < V) dst[3 * (size_t)K] = s[rt].w;
+        for (int rt = 0; rt < KT; ++rt) {
+            const int kk = rt * 64 + row, vv = v0 + 4 * cq;
+            if (kk < K) {
+                float* dst = p.s_out + (((size_t)seq * H + h) * V + vv) * K + kk;
+                if (vv + 0 < V) dst[0] = s[rt].x;
+                if (vv + 1 < V) dst[K] = s[rt].y;
+                if (vv + 2 < V) dst[2 * (size_t)K] = s[rt].z;
+                if (vv + 3 < V) dst[3 * (size_t)K] = s[rt].w;
             }
         }
     }
@@ -823,43 +839,56 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
         for (int vt = 0; vt < VT; ++vt) {
             const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
             const int nc = V - vt * 64;
-            // ---- dZ = A^T dO + E dH'
+            // ---- dZ = A^T dO + E dH'; every tile of the step is on its way before the first product
             __syncthreads();
-            ld_nat(t4, w.A + ch * 4096, 64);
+            cpa_nat(t4, w.A + ch * 4096, 64);
+            cpa_nat(t2, s.dHn + ch * Kp * Vp + vt * 64, Vp);
+            cpa_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
+            if (vt == 0) cpa_nat(t3, w.T + ch * 4096, 64);
+            cpa_commit();
             ld_tile_io<false>(t5, p.d_o, p.bf16, voff, vrow, len, nc, p.vec_v);
+            ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, nc, p.vec_v);
+            float e[16];
+            auto source_col = [&](int kt) {      // column of E^T
+                const float ge = G_g[(size_t)63 * Kp + kt * 64 + d];
+#pragma unroll
+                for (int r = 0; r < 16; ++r) {
+                    const size_t o = (size_t)(16 * I + r) * Kp + kt * 64 + d;
+                    e[r] = kn_g[o] * expf(ge - G_g[o]);
+                }
+            };
+            source_col(0);
+            cpa_wait();
             __syncthreads();
             zero_acc(acc);
             mm64(acc, t4, t5);
             for (int kt = 0; kt < KT; ++kt) {
                 __syncthreads();
-                {
-                    float e[16];
-                    const float ge = G_g[(size_t)63 * Kp + kt * 64 + d];
-#pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        const size_t o = (size_t)(16 * I + r) * Kp + kt * 64 + d;
-                        e[r] = kn_g[o] * expf(ge - G_g[o]);
-                    }
-                    st_col(t4, e);
+                if (kt > 0) {
+                    source_col(kt);
+                    ld_nat(t2, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
                 }
-                ld_nat(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+                st_col(t5, e);
                 __syncthreads();
-                mm64(acc, t4, t5);
+                mm64(acc, t5, t2);
             }
-            // ---- dA += dO Z^T, X += dZ (beta v)^T, dv = beta T^T dZ
+            // ---- X += dZ (beta v)^T, dv = beta T^T dZ, dA += dO Z^T
             __syncthreads();
             st_tr(t2, kLD, acc);
             st_nat(t4, kLD, acc);
             if (VT > 1) st_nat(s.dZ + ch * 64 * Vp + vt * 64, Vp, acc);
-            if (vt == 0) ld_nat(t3, w.T + ch * 4096, 64);
-            ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, nc, p.vec_v);
-            ld_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
             ld_tile_io<true>(t5, p.v, p.bf16, voff, vrow, len, nc, p.vec_v, bet);
             __syncthreads();
-            mm64(accA, t0, t1);
             mm64(accX, t2, t5);
             zero_acc(acc);
             mm64(acc, t3, t4);
+            __syncthreads();
+            if (VT == 1) {      // the first key tile's states, behind the last product
+                cpa_tr(t4, w.Hc + ch * Kp * Vp, Vp);
+                cpa_tr(t5, s.dHn + ch * Kp * Vp, Vp);
+                cpa_commit();
+            }
+            mm64(accA, t0, t1);
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int i = 4 * ty + r;
@@ -888,8 +917,12 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
                 ld_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
                 ld_tr(t2, s.dZ + ch * 64 * Vp + vt * 64, Vp);
             }
-            ld_tr(t4, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
-            ld_tr(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+            if (VT > 1 || kt > 0) {
+                cpa_tr(t4, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+                cpa_tr(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+                cpa_commit();
+            }
+            cpa_wait();
             __syncthreads();
             mm64(aR, t0, t4);
             mm64(aE, t1, t5);
@@ -898,6 +931,10 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
         }
         // ---- X -= dW Q^T, T^T dW
         __syncthreads();
+        if (kt == KT - 1) {      // dZ^T is read out: T^T for the adjoint of the inverse
+            cpa_tr(t2, w.T + ch * 4096, 64);
+            cpa_commit();
+        }
         st_tr(t4, kLD, aW);
         {
             float x[16];
@@ -961,7 +998,7 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
     float accA[4][4], accM[4][4];
     __syncthreads();
     st_nat(t4, kLD, accX);
-    ld_tr(t2, w.T + ch * 4096, 64);
+    cpa_wait();
     __syncthreads();
     zero_acc(acc);
     mm64(acc, t3, t4);
@@ -1252,10 +1289,22 @@ static int set_smem(Kern kern, size_t bytes) {
 static int vec4(const void* p, int dim) { return dim % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 static int launch_scan(const Ws& w, int n_seq, const simt::ScanArgs& a, const char* name, cudaStream_t st) {
-    const size_t bytes = (size_t)(simt::kScanStages * 4096 + 4 * 64 * simt::kVS + w.Kp * simt::kVS) * sizeof(float);
-    if (set_smem(simt::scan_kernel, bytes)) return KDA_ERR_CUDA;
+    const size_t bytes = simt::scan_smem(w.Kp);
     // padding strips hold zeros already: E^T U and Rm^T dO of zero columns
-    KDA_LAUNCH(name, st, simt::scan_kernel<<<dim3(n_seq, w.H, ceil_div(w.V, simt::kVS)), 256, bytes, st>>>(w, a));
+    const dim3 grid(n_seq, w.H, ceil_div(w.V, simt::kVS));
+#define KDA_SCAN(KT)                                                                                              \
+    case KT:                                                                                                      \
+        if (set_smem(simt::scan_kernel<KT>, bytes)) return KDA_ERR_CUDA;                                          \
+        KDA_LAUNCH(name, st, simt::scan_kernel<KT><<<grid, 256, bytes, st>>>(w, a));                               \
+        break
+    switch (w.Kp / 64) {
+        KDA_SCAN(1);
+        KDA_SCAN(2);
+        KDA_SCAN(3);
+        KDA_SCAN(4);
+        default: return KDA_ERR_BAD_SHAPE;
+    }
+#undef KDA_SCAN
     return launch_status();
 }
 
