@@ -799,6 +799,8 @@ struct LocalArgs {
 };
 constexpr size_t kLocalSmem = (6 * kTile + 64 * 3 + 4 * 64 * 3 + KDA_MAX_DIM) * sizeof(float);
 
+// ONE: K, V <= 64, the loops over tiles are gone (and the loop-invariant addresses the compiler would keep for them)
+template <bool ONE>
 __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArgs p) {
     extern __shared__ __align__(16) float sm[];
     float *t0 = sm, *t1 = sm + kTile, *t2 = sm + 2 * kTile, *t3 = sm + 3 * kTile, *t4 = sm + 4 * kTile, *t5 = sm + 5 * kTile;
@@ -812,7 +814,7 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
     const int slot = blockIdx.x, h = blockIdx.y;
     const int len = w.chunk_len[slot];
     if (len == 0) return;
-    const int tok0 = w.chunk_tok0[slot], K = w.K, Kp = w.Kp, V = w.V, Vp = w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
+    const int tok0 = w.chunk_tok0[slot], K = w.K, Kp = ONE ? 64 : w.Kp, V = w.V, Vp = ONE ? 64 : w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
     const size_t ch = (size_t)slot * H + h;
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, d = tid & 63, I = tid >> 6;
     const float* kn_g = w.kn + ch * 64 * Kp;
@@ -905,29 +907,65 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
         st_nat(s.dA + ch * 4096, 64, accA);      // waits in L2 while the registers serve the key tiles
     }
     for (int kt = 0; kt < KT; ++kt) {
-        float aR[4][4], aE[4][4], aW[4][4], dd = 0.f;
-        zero_acc(aR);
-        zero_acc(aE);
+        // Products with the states, one at a time where one value tile is all there is: dR, dE and dW then never live
+        // together (with them the kernel spills, and a spill reload costs an L2 round trip next to 218 KB of shared memory).
+        float dG[4][4], dk[4][4], aW[4][4], colE[4] = {0.f, 0.f, 0.f, 0.f}, dd = 0.f;
+        zero_acc(dG);
+        zero_acc(dk);
         zero_acc(aW);
-        for (int vt = 0; vt < VT; ++vt) {
+        const size_t so = ch * 64 * Kp + kt * 64;
+        if (VT == 1) {
             __syncthreads();
-            if (VT > 1) {
-                const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
-                ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, V - vt * 64, p.vec_v);
-                ld_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
-                ld_tr(t2, s.dZ + ch * 64 * Vp + vt * 64, Vp);
-            }
-            if (VT > 1 || kt > 0) {
-                cpa_tr(t4, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
-                cpa_tr(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+            if (kt > 0) {
+                cpa_tr(t4, w.Hc + (ch * Kp + kt * 64) * Vp, Vp);
+                cpa_tr(t5, s.dHn + (ch * Kp + kt * 64) * Vp, Vp);
                 cpa_commit();
             }
             cpa_wait();
             __syncthreads();
-            mm64(aR, t0, t4);
-            mm64(aE, t1, t5);
             mm64(aW, t2, t4);
+            zero_acc(acc);
+            mm64(acc, t0, t4);                   // dR
+            mm64(dk, t1, t5);                    // dE
             for (int vv = 16 * I; vv < 16 * I + 16; ++vv) dd += t4[vv * kLD + d] * t5[vv * kLD + d];
+        } else {
+            zero_acc(acc);
+            for (int vt = 0; vt < VT; ++vt) {
+                const size_t voff = ((size_t)tok0 * H + h) * V + vt * 64;
+                __syncthreads();
+                cpa_tr(t4, w.Hc + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+                cpa_tr(t5, s.dHn + (ch * Kp + kt * 64) * Vp + vt * 64, Vp);
+                cpa_tr(t1, w.Z + ch * 64 * Vp + vt * 64, Vp);
+                cpa_tr(t2, s.dZ + ch * 64 * Vp + vt * 64, Vp);
+                cpa_commit();
+                ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, V - vt * 64, p.vec_v);
+                cpa_wait();
+                __syncthreads();
+                mm64(aW, t2, t4);
+                mm64(acc, t0, t4);
+                mm64(dk, t1, t5);
+                for (int vv = 16 * I; vv < 16 * I + 16; ++vv) dd += t4[vv * kLD + d] * t5[vv * kLD + d];
+            }
+        }
+        {
+            const float4 e4 = *reinterpret_cast<const float4*>(G_g + (size_t)63 * Kp + kt * 64 + 4 * tx);
+            const float ea[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const size_t o = (size_t)(4 * ty + r) * Kp + kt * 64 + 4 * tx;
+                const float4 g4 = *reinterpret_cast<const float4*>(G_g + o), q4 = *reinterpret_cast<const float4*>(qn_g + o),
+                             k4 = *reinterpret_cast<const float4*>(kn_g + o);
+                const float ga[4] = {g4.x, g4.y, g4.z, g4.w}, qa[4] = {q4.x, q4.y, q4.z, q4.w}, ka[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    acc[r][c] *= expf(ga[c]);                  // dq = dR e^G
+                    dk[r][c] *= expf(ea[c] - ga[c]);           // dE e^{G_end - G}
+                    const float eE = dk[r][c] * ka[c];
+                    dG[r][c] = acc[r][c] * qa[c] - eE;
+                    colE[c] += eE;
+                }
+            }
+            st_nat(s.dqn + so, Kp, acc);
         }
         // ---- X -= dW Q^T, T^T dW
         __syncthreads();
@@ -941,50 +979,37 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
                 const size_t o = (size_t)(16 * I + r) * Kp + kt * 64 + d;
-                x[r] = bet[16 * I + r] * expf(G_g[o]) * kn_g[o];
+                x[r] = -bet[16 * I + r] * expf(G_g[o]) * kn_g[o];
             }
             st_col(t5, x);
         }
         bsum[I * 64 + d] = dd;
         __syncthreads();
-        zero_acc(acc);
-        mm64(acc, t4, t5);
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) accX[r][c] -= acc[r][c];
+        mm64(accX, t4, t5);
         __syncthreads();
         st_nat(t4, kLD, aW);
         __syncthreads();
         zero_acc(acc);
         mm64(acc, t3, t4);
-        // ---- the direct parts of dq, dk, dG, dbeta and dG_end
-        float ga[4][4], qa[4][4], ka[4][4], colE[4] = {0.f, 0.f, 0.f, 0.f};
-        ld_patch(ga, G_g + kt * 64, Kp);
-        ld_patch(qa, qn_g + kt * 64, Kp);
-        ld_patch(ka, kn_g + kt * 64, Kp);
-        const float4 e4 = *reinterpret_cast<const float4*>(G_g + (size_t)63 * Kp + kt * 64 + 4 * tx);
-        const float ea[4] = {e4.x, e4.y, e4.z, e4.w};
+        // ---- the part through Q: dQ = -(T^T dW)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
+            const size_t o = (size_t)(4 * ty + r) * Kp + kt * 64 + 4 * tx;
+            const float4 g4 = *reinterpret_cast<const float4*>(G_g + o), k4 = *reinterpret_cast<const float4*>(kn_g + o);
+            const float ga[4] = {g4.x, g4.y, g4.z, g4.w}, ka[4] = {k4.x, k4.y, k4.z, k4.w};
             const float bi = bet[4 * ty + r];
             float brow = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const float eg = expf(ga[r][c]), ee = expf(ea[c] - ga[r][c]);
-                const float R = qa[r][c] * eg, E = ka[r][c] * ee, dQ = -acc[r][c] * eg;
-                brow += dQ * ka[r][c];
-                colE[c] += aE[r][c] * E;
-                ga[r][c] = aR[r][c] * R - aE[r][c] * E + dQ * bi * ka[r][c];      // dG
-                qa[r][c] = aR[r][c] * eg;                                          // dq
-                ka[r][c] = aE[r][c] * ee + dQ * bi;                                // dk
+                const float dQ = -acc[r][c] * expf(ga[c]);
+                brow += dQ * ka[c];
+                dG[r][c] += dQ * bi * ka[c];
+                dk[r][c] += dQ * bi;
             }
             db[r] += row_sum16(brow);
         }
-        const size_t so = ch * 64 * Kp + kt * 64;
-        st_nat(s.dqn + so, Kp, qa);
-        st_nat(s.dkn + so, Kp, ka);
-        st_nat(s.dG + so, Kp, ga);
+        st_nat(s.dkn + so, Kp, dk);
+        st_nat(s.dG + so, Kp, dG);
         *reinterpret_cast<float4*>(t5 + ty * 64 + 4 * tx) = make_float4(colE[0], colE[1], colE[2], colE[3]);      // Q^T is read out
         __syncthreads();
         if (tid < 64) {
@@ -1063,7 +1088,7 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
             {
                 const float *x = t0 + 4 * ty, *y = t1 + 4 * ty, *b = t2 + 8 * T0 * (T0 + 1) * kLD + 4 * tx;
                 const int n = 16 * (T0 + 1);
-#pragma unroll 4
+#pragma unroll 2
                 for (int kk = 0; kk < n; ++kk) {
                     const float4 bb = *reinterpret_cast<const float4*>(b + kk * kLD);
                     fma16(aq, *reinterpret_cast<const float4*>(x + kk * kLD), bb);
@@ -1083,7 +1108,7 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
             }
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
-                const float e = expf(L[r] - c);
+                const float e = expf(t5[(16 * I + r) * kLD + d]);      // L - c, back from this thread's own store
                 const size_t o = (size_t)(16 * I + r) * Kp + dd;
                 t2[(16 * I + r) * kLD + d] = qn_g[o] * e;
                 t3[(16 * I + r) * kLD + d] = kn_g[o] * e;
@@ -1404,8 +1429,9 @@ int simt_chunk_bwd(const KdaChunkShape* sh, const void* q, const void* k, const 
     if (w.nslots > 0) {
         const simt::LocalArgs a{q, k, v, g, d_o, dq, dk, dv, dg, dbeta, bf16, gbf16, sh->l2norm,
                                 vec4(q, sh->key_dim) && vec4(k, sh->key_dim), vec_v, sh->scale};
-        if (set_smem(simt::local_bwd_kernel, simt::kLocalSmem)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("local_bwd_kernel", st, simt::local_bwd_kernel<<<dim3(w.nslots, w.H), 256, simt::kLocalSmem, st>>>(w, s, a));
+        const auto kern = KT == 1 && w.Vp == 64 ? simt::local_bwd_kernel<true> : simt::local_bwd_kernel<false>;
+        if (set_smem(kern, simt::kLocalSmem)) return KDA_ERR_CUDA;
+        KDA_LAUNCH("local_bwd_kernel", st, kern<<<dim3(w.nslots, w.H), 256, simt::kLocalSmem, st>>>(w, s, a));
     }
     return launch_status();
 }
