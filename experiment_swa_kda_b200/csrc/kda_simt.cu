@@ -313,10 +313,11 @@ __device__ void unit_lower_inverse(const float* Ms, float* Ts, float* tmp) {
 // decay exceeds kMaxExponent inside a block takes the pairwise exponentials instead (log-decays below -10 per token).
 constexpr float kMaxExponent = 80.f;
 constexpr int kSrcCols = 16 + 32 + 48 + 64;
-// source array of block I: [64 d][16 (I + 1)] with 4 floats of padding, after the two target tiles
+// source array of block I in the forward: [32 d][16 (I + 1)] with 4 floats of padding, after the two target stacks
+constexpr int kHalf = 32;
 __device__ __forceinline__ int src_ld(int I) { return 16 * (I + 1) + 4; }
-__device__ __forceinline__ int src_off(int I) { return 64 * (8 * I * (I + 1) + 4 * I); }
-constexpr int kSrcFloats = 64 * (kSrcCols + 16);
+__device__ __forceinline__ int src_off(int I) { return kHalf * (8 * I * (I + 1) + 4 * I); }
+constexpr int kSrcFloats = kHalf * (kSrcCols + 16);
 
 // ---------------------------------------------------------------------------------------------
 // K1  chunk-parallel part of the forward, one CTA per (chunk, head): norms, decay, A, T, W, U and the scan's coefficients
@@ -326,20 +327,22 @@ struct IntraArgs {
     int bf16, gbf16, l2norm, vec_v, backward;
     float scale;
 };
-constexpr int kIntraFloats = 2 * kTile + kSrcFloats;      // target stacks and sources, later five tiles
-static_assert(kIntraFloats >= 4 * kTile + 32 * kLD, "the second half's tiles overlap");
-constexpr size_t kIntraSmem = (kIntraFloats + 64 * 3 + 4 * 64 * 2) * sizeof(float);
+// 46 KB and at most 80 registers, so that three CTAs share an SM: the kernel alternates between loads, short products and
+// barriers, and two CTAs (64-wide factor tiles, 83 KB) left the issue slots 60 % idle.
+constexpr int kIntraFloats = 160 * kLD;                   // factor stacks of 32 channels, later M, T and 32 rows of scratch
+static_assert(kIntraFloats >= 2 * kHalf * kLD + kSrcFloats, "factor stacks do not fit");
+constexpr size_t kIntraSmem = (kIntraFloats + 64 * 3 + 8 * kHalf + 4 * kHalf) * sizeof(float);
 
-__global__ void __launch_bounds__(256, 2) intra_fwd_kernel(Ws w, IntraArgs p) {
+__global__ void __launch_bounds__(256, 3) intra_fwd_kernel(Ws w, IntraArgs p) {
     extern __shared__ __align__(16) float sm[];
     float* tq = sm;                      // [d][i] q~
-    float* tk = tq + kTile;              // [d][i] k~
-    float* src = tk + kTile;             // four source arrays
+    float* tk = tq + kHalf * kLD;        // [d][i] k~
+    float* src = tk + kHalf * kLD;       // four source arrays
     float* qi_s = sm + kIntraFloats;     // [64] inverse norms, beta
     float* ki_s = qi_s + 64;
     float* bet = ki_s + 64;
-    float* bsum = bet + 64;              // [4][64] block sums of g
-    float* cref = bsum + 256;            // [4][64] G at row 8 of each block
+    float* bsum = bet + 64;              // [8][32] sums of g over 8 rows
+    float* cref = bsum + 8 * kHalf;      // [4][32] G at row 8 of each block
     const int slot = blockIdx.x, h = blockIdx.y;
     const int len = w.chunk_len[slot];
     if (len == 0) return;
@@ -383,88 +386,91 @@ __global__ void __launch_bounds__(256, 2) intra_fwd_kernel(Ws w, IntraArgs p) {
     float acc1[4][4], acc2[4][4];
     zero_acc(acc1);
     zero_acc(acc2);
-    const int d = tid & 63, I = tid >> 6;      // element-wise: column d, rows 16 I .. 16 I + 15
-    for (int kt = 0; kt < KT; ++kt) {
-        const int dd = kt * 64 + d;
+    const int I = warp >> 1, i0 = 8 * warp;    // element-wise: channel `lane` of 32, rows i0 .. i0 + 7 of block I
+    for (int dt = 0; dt < 2 * KT; ++dt) {
+        const int dd = dt * kHalf + lane;
         const bool in = dd < K;
         const size_t col = ((size_t)tok0 * H + h) * K + (in ? dd : 0), rstep = (size_t)H * K;
-        float L[16], qn[16], kn[16];
+        float L[8];
         {
             float run = 0.f;
 #pragma unroll
-            for (int r = 0; r < 16; ++r) L[r] = (16 * I + r < len && in) ? ld_io(p.g, col + (size_t)(16 * I + r) * rstep, p.gbf16) : 0.f;
+            for (int r = 0; r < 8; ++r) L[r] = (i0 + r < len && in) ? ld_io(p.g, col + (size_t)(i0 + r) * rstep, p.gbf16) : 0.f;
+            const float first = L[0];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) L[r] = run += L[r];
+            for (int r = 0; r < 8; ++r) L[r] = run += L[r];
+            __syncthreads();                   // norms on the first round; the previous round's stacks are free
+            bsum[warp * kHalf + lane] = run;
+            if (warp & 1) cref[I * kHalf + lane] = first;      // g of row 8, completed below
         }
-        __syncthreads();                       // norms on the first round; the previous round's tiles are free
-        bsum[I * 64 + d] = L[15];
         __syncthreads();
         float pre = 0.f;
-        for (int J = 0; J < I; ++J) pre += bsum[J * 64 + d];
-        const float c = L[8];
-        cref[I * 64 + d] = pre + c;
+        for (int J = 0; J < 2 * I; ++J) pre += bsum[J * kHalf + lane];
+        const float half = bsum[2 * I * kHalf + lane], c = half + cref[I * kHalf + lane];      // L of the block's row 8
+        if (warp & 1) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) L[r] += half;
+        }
         bool far = false;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) far = far || !(fabsf(L[r] - c) <= kMaxExponent);
-        const bool pairwise = __syncthreads_or(far);
+        for (int r = 0; r < 8; ++r) far = far || !(fabsf(L[r] - c) <= kMaxExponent);
+        const bool pairwise = __syncthreads_or(far);           // every warp has read the block sums and the rows' g
+        if (!(warp & 1)) cref[I * kHalf + lane] = pre + c;
+        __syncthreads();
+        float kn[8];
+        float* rt = w.RT + (ch * Kp + dd) * 64 + i0;           // R^T: 8 rows of this channel
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const int i = 16 * I + r;
-            const bool ok = i < len && in;
-            qn[r] = ok ? ld_io(p.q, col + (size_t)i * rstep, p.bf16) * qi_s[i] * p.scale : 0.f;
-            kn[r] = ok ? ld_io(p.k, col + (size_t)i * rstep, p.bf16) * ki_s[i] : 0.f;
-            kn_g[(size_t)i * Kp + dd] = kn[r];
-            G_g[(size_t)i * Kp + dd] = pre + L[r];
-            if (p.backward) w.qn[(ch * 64 + i) * Kp + dd] = qn[r];
-        }
-        {
-            float* rt = w.RT + (ch * Kp + dd) * 64 + 16 * I;      // R^T: 16 rows of column d
+        for (int r4 = 0; r4 < 2; ++r4) {
+            float R[4], q[4];
 #pragma unroll
-            for (int r4 = 0; r4 < 4; ++r4)
-                *reinterpret_cast<float4*>(rt + 4 * r4) =
-                    make_float4(qn[4 * r4] * expf(pre + L[4 * r4]), qn[4 * r4 + 1] * expf(pre + L[4 * r4 + 1]),
-                                qn[4 * r4 + 2] * expf(pre + L[4 * r4 + 2]), qn[4 * r4 + 3] * expf(pre + L[4 * r4 + 3]));
+            for (int e = 0; e < 4; ++e) {
+                const int r = 4 * r4 + e, i = i0 + r;
+                const bool ok = i < len && in;
+                const float qn = ok ? ld_io(p.q, col + (size_t)i * rstep, p.bf16) * qi_s[i] * p.scale : 0.f;
+                kn[r] = ok ? ld_io(p.k, col + (size_t)i * rstep, p.bf16) * ki_s[i] : 0.f;
+                const float G = pre + L[r];
+                kn_g[(size_t)i * Kp + dd] = kn[r];
+                G_g[(size_t)i * Kp + dd] = G;
+                if (p.backward) w.qn[(ch * 64 + i) * Kp + dd] = qn;
+                R[e] = qn * expf(G);
+                q[e] = pairwise ? qn : qn * expf(L[r] - c);
+            }
+            *reinterpret_cast<float4*>(rt + 4 * r4) = make_float4(R[0], R[1], R[2], R[3]);
+            *reinterpret_cast<float4*>(tq + lane * kLD + i0 + 4 * r4) = make_float4(q[0], q[1], q[2], q[3]);
         }
         if (!pairwise) {
-            float e[16];
+            float e[8];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) e[r] = expf(L[r] - c);
+            for (int r = 0; r < 8; ++r) e[r] = kn[r] * expf(L[r] - c);
+            *reinterpret_cast<float4*>(tk + lane * kLD + i0) = make_float4(e[0], e[1], e[2], e[3]);
+            *reinterpret_cast<float4*>(tk + lane * kLD + i0 + 4) = make_float4(e[4], e[5], e[6], e[7]);
 #pragma unroll
-            for (int r4 = 0; r4 < 4; ++r4) {
-                *reinterpret_cast<float4*>(tq + d * kLD + 16 * I + 4 * r4) =
-                    make_float4(qn[4 * r4] * e[4 * r4], qn[4 * r4 + 1] * e[4 * r4 + 1], qn[4 * r4 + 2] * e[4 * r4 + 2], qn[4 * r4 + 3] * e[4 * r4 + 3]);
-                *reinterpret_cast<float4*>(tk + d * kLD + 16 * I + 4 * r4) =
-                    make_float4(kn[4 * r4] * e[4 * r4], kn[4 * r4 + 1] * e[4 * r4 + 1], kn[4 * r4 + 2] * e[4 * r4 + 2], kn[4 * r4 + 3] * e[4 * r4 + 3]);
-            }
-#pragma unroll
-            for (int r = 0; r < 16; ++r) e[r] = kn[r] * expf(c - L[r]);
+            for (int r = 0; r < 8; ++r) e[r] = kn[r] * expf(c - L[r]);
             for (int T = I; T < 4; ++T) {
-                const float f = T == I ? 1.f : expf(cref[T * 64 + d] - cref[I * 64 + d]);
-                float* s = src + src_off(T) + d * src_ld(T) + 16 * I;
-#pragma unroll
-                for (int r4 = 0; r4 < 4; ++r4)
-                    *reinterpret_cast<float4*>(s + 4 * r4) = make_float4(e[4 * r4] * f, e[4 * r4 + 1] * f, e[4 * r4 + 2] * f, e[4 * r4 + 3] * f);
+                const float f = T == I ? 1.f : expf(cref[T * kHalf + lane] - cref[I * kHalf + lane]);
+                float* s = src + src_off(T) + lane * src_ld(T) + i0;
+                *reinterpret_cast<float4*>(s) = make_float4(e[0] * f, e[1] * f, e[2] * f, e[3] * f);
+                *reinterpret_cast<float4*>(s + 4) = make_float4(e[4] * f, e[5] * f, e[6] * f, e[7] * f);
             }
             __syncthreads();
-            mm_at(acc1, (r1 < 4 ? tq : tk) + 16 * t1 + 4 * (r1 & 3), kLD, src + src_off(t1) + 4 * c1, src_ld(t1), 64);
-            if (tid < 64) mm_at(acc2, (r2 < 4 ? tq : tk) + 48 + 4 * (r2 & 3), kLD, src + src_off(3) + 4 * c2, src_ld(3), 64);
+            mm_at(acc1, (r1 < 4 ? tq : tk) + 16 * t1 + 4 * (r1 & 3), kLD, src + src_off(t1) + 4 * c1, src_ld(t1), kHalf);
+            if (tid < 64) mm_at(acc2, (r2 < 4 ? tq : tk) + 48 + 4 * (r2 & 3), kLD, src + src_off(3) + 4 * c2, src_ld(3), kHalf);
         } else {
             float* Gs = src;                   // plain q, k, G columns
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                tq[d * kLD + 16 * I + r] = qn[r];
-                tk[d * kLD + 16 * I + r] = kn[r];
-                Gs[d * kLD + 16 * I + r] = pre + L[r];
+            for (int r = 0; r < 8; ++r) {
+                tk[lane * kLD + i0 + r] = kn[r];
+                Gs[lane * kLD + i0 + r] = pre + L[r];
             }
             __syncthreads();
-            auto pairs = [&](float (&acc)[4][4], int T, int rt, int ct) {
-                const float* x = (rt < 4 ? tq : tk);
+            auto pairs = [&](float (&acc)[4][4], int T, int rt4, int ct) {
+                const float* x = (rt4 < 4 ? tq : tk);
                 for (int r = 0; r < 4; ++r)
                     for (int s4 = 0; s4 < 4; ++s4) {
-                        const int i = 16 * T + 4 * (rt & 3) + r, s = 4 * ct + s4;
+                        const int i = 16 * T + 4 * (rt4 & 3) + r, s = 4 * ct + s4;
                         if (s > i) continue;
                         float a = 0.f;
-                        for (int e = 0; e < 64; ++e) a += x[e * kLD + i] * tk[e * kLD + s] * expf(Gs[e * kLD + i] - Gs[e * kLD + s]);
+                        for (int e = 0; e < kHalf; ++e) a += x[e * kLD + i] * tk[e * kLD + s] * expf(Gs[e * kLD + i] - Gs[e * kLD + s]);
 #pragma unroll
                         for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
@@ -481,8 +487,8 @@ __global__ void __launch_bounds__(256, 2) intra_fwd_kernel(Ws w, IntraArgs p) {
     float* Ms = sm;
     float* Ts = Ms + kTile;
     float* tmp = Ts + kTile;             // 32 rows
-    float* TT = tmp + 32 * kLD;          // [s][i] = T[i][s]
-    float* op = TT + kTile;              // operand tile
+    float* TT = Ms;                      // [s][i] = T[i][s], once M is done with
+    float* op = Ts;                      // operand tile, once T is out
     for (int idx = tid; idx < 2 * kTile / 4; idx += 256) reinterpret_cast<float4*>(sm)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     auto place = [&](const float (&acc)[4][4], int T, int rt, int ct) {
