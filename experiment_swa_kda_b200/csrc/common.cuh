@@ -25,6 +25,45 @@ __device__ __forceinline__ void st_io(void* p, size_t i, int bf16, float x) {
     else reinterpret_cast<float*>(p)[i] = x;
 }
 
+// Two float32 in a 64-bit register pair.  sm_100a executes one packed instruction for both at the same rate per value, so
+// kernels bound by instruction issue halve that part of their count; each half rounds like the scalar instruction.
+struct f2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 f2_get(f2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ f2 f2_all(float a) { return f2_make(a, a); }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// a bf16 pair in one word <-> two float32
+__device__ __forceinline__ f2 f2_from_bf16(unsigned u) { return f2_make(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+__device__ __forceinline__ unsigned f2_to_bf16(f2 a) {
+    const float2 x = f2_get(a);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
+    return *reinterpret_cast<const unsigned*>(&h);
+}
+
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);

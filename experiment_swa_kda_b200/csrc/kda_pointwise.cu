@@ -630,6 +630,62 @@ __device__ __forceinline__ void st_cvec(void* p, size_t i, const float (&s)[VEC]
     }
 }
 
+// The same as channel pairs
+template <int VEC, bool BF16>
+__device__ __forceinline__ void ld_c2(f2 (&d)[VEC / 2], const void* p, size_t i) {
+    if (BF16) {
+        const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(p) + i;
+        if (VEC == 2) {
+            d[0] = f2_from_bf16(__ldg(reinterpret_cast<const unsigned*>(b)));
+        } else {
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(b));
+            d[0] = f2_from_bf16(u.x);
+            d[VEC / 2 - 1] = f2_from_bf16(u.y);
+        }
+    } else {
+        float x[VEC];
+        ld_cvec<VEC, false>(x, p, i);
+#pragma unroll
+        for (int e = 0; e < VEC / 2; ++e) d[e] = f2_make(x[2 * e], x[2 * e + 1]);
+    }
+}
+template <int VEC, bool BF16>
+__device__ __forceinline__ void st_c2(void* p, size_t i, const f2 (&s)[VEC / 2]) {
+    if (BF16) {
+        __nv_bfloat16* b = reinterpret_cast<__nv_bfloat16*>(p) + i;
+        if (VEC == 2) *reinterpret_cast<unsigned*>(b) = f2_to_bf16(s[0]);
+        else *reinterpret_cast<uint2*>(b) = make_uint2(f2_to_bf16(s[0]), f2_to_bf16(s[VEC / 2 - 1]));
+    } else {
+        float x[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC / 2; ++e) {
+            const float2 v = f2_get(s[e]);
+            x[2 * e] = v.x;
+            x[2 * e + 1] = v.y;
+        }
+        st_cvec<VEC, false>(p, i, x);
+    }
+}
+template <bool FAST>
+__device__ __forceinline__ f2 sigmoid_2(f2 z) {
+    if (FAST) {
+        const f2 half = f2_all(0.5f);
+        const float2 h = f2_get(f2_mul(half, z));
+        float a, b;
+        asm("tanh.approx.f32 %0, %1;" : "=f"(a) : "f"(h.x));
+        asm("tanh.approx.f32 %0, %1;" : "=f"(b) : "f"(h.y));
+        return f2_fma(half, f2_make(a, b), half);
+    }
+    const float2 x = f2_get(z);
+    return f2_make(sigmoid_t<false>(x.x), sigmoid_t<false>(x.y));
+}
+// gy * d silu(z) / dz
+template <bool FAST>
+__device__ __forceinline__ f2 silu_vjp_2(f2 gy, f2 z) {
+    const f2 one = f2_all(1.f), s = sigmoid_2<FAST>(z);
+    return f2_mul(gy, f2_mul(s, f2_fma(z, f2_fma(s, f2_all(-1.f), one), one)));
+}
+
 // Gate activations, K % 4 == 0: a thread owns 4 adjacent channels (one head), so raw gate, bias, g and their gradients
 // move as 8- / 16-byte accesses and the head's exp(A_log) is computed once per 4 elements.
 template <bool BF16>
@@ -767,8 +823,8 @@ __device__ __forceinline__ T pick_item(T const (&a)[kConvItems], int i) {
 // grid: x = channel blocks of 32*VEC, y = blocks of 8 time groups x kConvPairT tokens, z = item * B + batch.  x rows are
 // ldx elements apart (a slice of a wider projection), y rows are dense.  WIN: a window is carried in or out; only the
 // threads at either end of a sequence touch it.  The kernel moves 2 x B x T x C elements and is bound by instruction issue
-// at 0.62 of the copy rate (131 us at 65,536 x 2,048 bf16); the windows used to go through a 4-token, 8-channel kernel
-// whose lanes read 16-byte pieces of strided rows: 78 us at 8,191 x 2,048, now 17.
+// at 0.65 of the copy rate (126 us at 65,536 x 2,048 bf16; long inputs take the streaming kernel below); the windows used
+// to go through a 4-token, 8-channel kernel whose lanes read 16-byte pieces of strided rows: 78 us at 8,191 x 2,048, now 22.
 template <int W, int VEC, bool BF16, bool WIN>
 __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C, int ldx, int silu, int wf32, ConvFwdItems items) {
     const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -781,31 +837,31 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
     void* __restrict__ y = pick_item(items.y, item);
     const bool cok = c < C;
     const int cl = cok ? c : 0;
-    float wv[W][VEC];
+    f2 wv[W][VEC / 2];
     {
         float flat[W * VEC];
         ld_wrun<W * VEC, BF16>(flat, wgt, (size_t)cl * W, wf32);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e)
+        for (int e = 0; e < VEC / 2; ++e)
 #pragma unroll
-            for (int m = 0; m < W; ++m) wv[m][e] = flat[e * W + m];
+            for (int m = 0; m < W; ++m) wv[m][e] = f2_make(flat[2 * e * W + m], flat[(2 * e + 1) * W + m]);
     }
     const size_t rowbase = (size_t)b * T;
-    float xin[kConvPairT + W - 1][VEC];
+    f2 xin[kConvPairT + W - 1][VEC / 2];
     if (t0 >= W - 1 && t0 + kConvPairT <= T) {
         // interior: plain address arithmetic, every load independent
         const size_t base = (rowbase + t0 - (W - 1)) * ldx + cl;
 #pragma unroll
-        for (int j = 0; j < kConvPairT + W - 1; ++j) ld_cvec<VEC, BF16>(xin[j], x, base + (size_t)j * ldx);
+        for (int j = 0; j < kConvPairT + W - 1; ++j) ld_c2<VEC, BF16>(xin[j], x, base + (size_t)j * ldx);
     } else {
 #pragma unroll
         for (int j = 0; j < kConvPairT + W - 1; ++j) {
             const int t = t0 - (W - 1) + j;
             const int tc = min(max(t, 0), T - 1);
-            ld_cvec<VEC, BF16>(xin[j], x, (rowbase + tc) * ldx + cl);
+            ld_c2<VEC, BF16>(xin[j], x, (rowbase + tc) * ldx + cl);
             if (t < 0 || t >= T) {
 #pragma unroll
-                for (int e = 0; e < VEC; ++e) xin[j][e] = 0.f;
+                for (int e = 0; e < VEC / 2; ++e) xin[j][e] = f2_all(0.f);
             }
         }
         if (WIN && t0 < W - 1) {
@@ -816,7 +872,10 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
                     const int t = t0 - (W - 1) + j;
                     if (t < 0) {
 #pragma unroll
-                        for (int e = 0; e < VEC; ++e) xin[j][e] = ld_io(cache, ((size_t)b * C + cl + e) * W + W + t, BF16);
+                        for (int e = 0; e < VEC / 2; ++e) {
+                            const size_t slot = ((size_t)b * C + cl + 2 * e) * W + W + t;
+                            xin[j][e] = f2_make(ld_io(cache, slot, BF16), ld_io(cache, slot + W, BF16));
+                        }
                     }
                 }
             }
@@ -824,15 +883,15 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
     }
 #pragma unroll
     for (int tt = 0; tt < kConvPairT; ++tt) {
-        float out[VEC];
+        f2 out[VEC / 2];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-            float z = 0.f;
+        for (int e = 0; e < VEC / 2; ++e) {
+            f2 z = f2_mul(wv[0][e], xin[tt][e]);
 #pragma unroll
-            for (int m = 0; m < W; ++m) z += wv[m][e] * xin[tt + m][e];
-            out[e] = silu ? z * sigmoid_t<BF16>(z) : z;
+            for (int m = 1; m < W; ++m) z = f2_fma(wv[m][e], xin[tt + m][e], z);
+            out[e] = silu ? f2_mul(z, sigmoid_2<BF16>(z)) : z;
         }
-        if (t0 + tt < T && cok) st_cvec<VEC, BF16>(y, (rowbase + t0 + tt) * C + c, out);
+        if (t0 + tt < T && cok) st_c2<VEC, BF16>(y, (rowbase + t0 + tt) * C + c, out);
     }
     if (WIN && cok && (t0 + kConvPairT > T - W || t0 == 0)) {
         void* fin = pick_item(items.fin, item);                    // slot s holds the input at time T - W + s
@@ -842,7 +901,11 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
                 const int t = t0 + tt, s = t - (T - W);
                 if (t < T && s >= 0) {
 #pragma unroll
-                    for (int e = 0; e < VEC; ++e) st_io(fin, ((size_t)b * C + c + e) * W + s, BF16, xin[tt + W - 1][e]);
+                    for (int e = 0; e < VEC / 2; ++e) {
+                        const float2 v = f2_get(xin[tt + W - 1][e]);
+                        st_io(fin, ((size_t)b * C + c + 2 * e) * W + s, BF16, v.x);
+                        st_io(fin, ((size_t)b * C + c + 2 * e + 1) * W + s, BF16, v.y);
+                    }
                 }
             }
             if (t0 == 0 && T < W) {                                // a sequence shorter than the window keeps what was carried in
@@ -855,6 +918,99 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
                     }
             }
         }
+    }
+}
+
+// The same for long bf16 inputs without carried windows, C % 128 == 0: a thread walks down a run of tokens, 8 rows at a
+// time, and loads the next 8 rows before it computes on the present ones, so that reads stay in flight and the W-1 halo
+// rows are read once per run instead of once per 8 tokens.  65,536 x 2,048: 129 -> 96 us (0.86 of the copy rate); with two
+// blocks per SM instead of three it takes 108.
+template <int W>
+__global__ void __launch_bounds__(256, W <= 4 ? 3 : 2) conv_fwd_stream_kernel(int B, int T, int C, int ldx, int run, int silu, int wf32, ConvFwdItems items) {
+    constexpr int R = 8;                                       // run is a multiple of 2 R
+    const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int c = (blockIdx.x * 32 + p) * 4;                   // C % 128 == 0: in range
+    const int item = blockIdx.z / B, b = blockIdx.z - item * B;
+    const int t0 = (blockIdx.y * 8 + g) * run;
+    if (t0 >= T) return;
+    const void* __restrict__ wgt = pick_item(items.w, item);
+    f2 wv[W][2];
+    {
+        float flat[W * 4];
+        ld_wrun<W * 4, true>(flat, wgt, (size_t)c * W, wf32);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int m = 0; m < W; ++m) wv[m][e] = f2_make(flat[2 * e * W + m], flat[(2 * e + 1) * W + m]);
+    }
+    const __nv_bfloat16* __restrict__ xp = static_cast<const __nv_bfloat16*>(pick_item(items.x, item)) + ((size_t)b * T + t0) * ldx + c;
+    __nv_bfloat16* __restrict__ yp = static_cast<__nv_bfloat16*>(pick_item(items.y, item)) + ((size_t)b * T + t0) * C + c;
+    const int n = min(run, T - t0);
+    f2 xw[W][2];                                               // rows t - (W-1) .. t as a circular buffer: row t in slot t % W
+#pragma unroll
+    for (int m = 1; m < W; ++m) {
+        xw[W - m][0] = xw[W - m][1] = f2_all(0.f);
+        if (t0 > 0) {                                          // then t0 >= run >= W: every halo row exists
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(xp - (size_t)m * ldx));
+            xw[W - m][0] = f2_from_bf16(u.x);
+            xw[W - m][1] = f2_from_bf16(u.y);
+        }
+    }
+    auto load = [&](uint2 (&d)[R], int i) {                    // rows i .. i + R - 1 of the run; past its end nothing
+        if (i + R <= n) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                d[r] = __ldg(reinterpret_cast<const uint2*>(xp));
+                xp += ldx;
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (i + r < n) {
+                    d[r] = __ldg(reinterpret_cast<const uint2*>(xp));
+                    xp += ldx;
+                }
+            }
+        }
+    };
+    auto rows = [&](const uint2 (&d)[R], int i, auto full) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!decltype(full)::value && i + r >= n) break;
+            const int s = r % W;
+            xw[s][0] = f2_from_bf16(d[r].x);
+            xw[s][1] = f2_from_bf16(d[r].y);
+            f2 out[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                f2 z = f2_mul(wv[0][e], xw[(s + 1) % W][e]);   // x[t - (W-1) + m]
+#pragma unroll
+                for (int m = 1; m < W; ++m) z = f2_fma(wv[m][e], xw[(s + 1 + m) % W][e], z);
+                out[e] = silu ? f2_mul(z, sigmoid_2<true>(z)) : z;
+            }
+            st_c2<4, true>(yp, 0, out);
+            yp += C;
+        }
+        if constexpr (R % W != 0) {                            // rotate, so that the next block starts at slot 0 again
+            f2 k[W][2];
+#pragma unroll
+            for (int m = 0; m < W; ++m) { k[m][0] = xw[(m + R) % W][0]; k[m][1] = xw[(m + R) % W][1]; }
+#pragma unroll
+            for (int m = 0; m < W; ++m) { xw[m][0] = k[m][0]; xw[m][1] = k[m][1]; }
+        }
+    };
+    auto block = [&](const uint2 (&d)[R], int i) {
+        if (i + R <= n) rows(d, i, std::true_type());
+        else rows(d, i, std::false_type());
+    };
+    uint2 da[R], db[R];
+    load(da, 0);
+#pragma unroll 1
+    for (int i = 0; i < n; i += 2 * R) {
+        load(db, i + R);
+        block(da, i);
+        load(da, i + 2 * R);
+        block(db, i + R);
     }
 }
 
@@ -1064,7 +1220,7 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
     typedef typename std::conditional<BF16, __nv_bfloat162, float2>::type xpair_t;
     __shared__ __align__(16) xpair_t xs[XR][32];
     __shared__ __align__(16) float2 gs[GR][32];
-    __shared__ float red[8][W][kConvTileC];
+    __shared__ __align__(16) float red[8][W][kConvTileC];
     const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int cb = blockIdx.x * kConvTileC;
     const int c = cb + 2 * p;
@@ -1076,15 +1232,12 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
     void* __restrict__ dx = pick_item(items.dx, item);
     const bool cok = c < C;
     const int cl = cok ? c : 0;                    // loads stay unconditional: out-of-range lanes read column 0 and are masked
-    float w0[W], w1[W];
+    f2 wv[W];
     {
         float flat[2 * W];
         ld_wrun<2 * W, BF16>(flat, wgt, (size_t)cl * W, wf32);
 #pragma unroll
-        for (int m = 0; m < W; ++m) {
-            w0[m] = flat[m];
-            w1[m] = flat[W + m];
-        }
+        for (int m = 0; m < W; ++m) wv[m] = f2_make(flat[m], flat[W + m]);
     }
     const size_t rowbase = (size_t)b * T;
     auto xload = [&](int tc) -> xpair_t {
@@ -1095,9 +1248,9 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
             return __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(x) + (rowbase + tc) * ldx + cl));
         }
     };
-    auto xwide = [](const xpair_t& v) -> float2 {
-        if constexpr (BF16) return __bfloat1622float2(v);
-        else return v;
+    auto xwide = [](const xpair_t& v) -> f2 {
+        if constexpr (BF16) return f2_from_bf16(*reinterpret_cast<const unsigned*>(&v));
+        else return f2_make(v.x, v.y);
     };
     if (t0 >= W - 1 && t0 + GR <= T && cb + kConvTileC <= C && (C & 3) == 0 && (ldx & 3) == 0) {
         // interior tile: no clamping, four channels per thread (sixteen threads cover a 64-channel row, a warp two rows),
@@ -1152,12 +1305,12 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
         }
     }
     __syncthreads();
-    float dw0[W], dw1[W];
+    f2 dw[W];
 #pragma unroll
-    for (int m = 0; m < W; ++m) dw0[m] = dw1[m] = 0.f;
+    for (int m = 0; m < W; ++m) dw[m] = f2_all(0.f);
     // dz for rows r0 .. r0+n-1, walking down with the x window in registers; dweight only from the tile's own rows
     auto dz_rows = [&](int r0, int n, bool own) {
-        float2 xw[W];
+        f2 xw[W];
 #pragma unroll
         for (int m = 0; m < W - 1; ++m) xw[m] = xwide(xs[r0 + m][p]);
 #pragma unroll
@@ -1165,25 +1318,18 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
             if (i < n) {
                 const int r = r0 + i;
                 xw[W - 1] = xwide(xs[r + W - 1][p]);
-                float2 gy = gs[r][p];
-                float z0 = 0.f, z1 = 0.f;
-#pragma unroll
-                for (int m = 0; m < W; ++m) {
-                    z0 += w0[m] * xw[m].x;
-                    z1 += w1[m] * xw[m].y;
-                }
+                f2* gp = reinterpret_cast<f2*>(&gs[r][p]);
+                f2 gy = *gp;
                 if (silu) {
-                    const float s0 = sigmoid_t<BF16>(z0), s1 = sigmoid_t<BF16>(z1);
-                    gy.x *= s0 * (1.f + z0 * (1.f - s0));
-                    gy.y *= s1 * (1.f + z1 * (1.f - s1));
+                    f2 z = f2_mul(wv[0], xw[0]);
+#pragma unroll
+                    for (int m = 1; m < W; ++m) z = f2_fma(wv[m], xw[m], z);
+                    gy = silu_vjp_2<BF16>(gy, z);
+                    *gp = gy;                      // dz; element (r, p) is touched by this thread only
                 }
-                gs[r][p] = gy;                     // dz; element (r, p) is touched by this thread only
                 if (own) {
 #pragma unroll
-                    for (int m = 0; m < W; ++m) {
-                        dw0[m] += gy.x * xw[m].x;
-                        dw1[m] += gy.y * xw[m].y;
-                    }
+                    for (int m = 0; m < W; ++m) dw[m] = f2_fma(gy, xw[m], dw[m]);
                 }
 #pragma unroll
                 for (int m = 0; m < W - 1; ++m) xw[m] = xw[m + 1];
@@ -1193,30 +1339,24 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
     dz_rows(g * RPW, RPW, true);
     if (g < W - 1) dz_rows(kConvTileT + g, 1, false);   // halo rows: their dweight belongs to the next block
 #pragma unroll
-    for (int m = 0; m < W; ++m) {
-        red[g][m][2 * p] = dw0[m];
-        red[g][m][2 * p + 1] = dw1[m];
-    }
+    for (int m = 0; m < W; ++m) *reinterpret_cast<f2*>(&red[g][m][2 * p]) = dw[m];
     __syncthreads();
     // dx[t] = sum_m w[m] dz[t + W-1-m], again with a register window over this warp's consecutive rows
     {
         const int r0 = g * RPW;
-        float2 dw_[W];
+        f2 dzw[W];
 #pragma unroll
-        for (int m = 0; m < W - 1; ++m) dw_[m] = gs[r0 + m][p];
+        for (int m = 0; m < W - 1; ++m) dzw[m] = *reinterpret_cast<const f2*>(&gs[r0 + m][p]);
 #pragma unroll
         for (int i = 0; i < RPW; ++i) {
             const int r = r0 + i, t = t0 + r;
-            dw_[W - 1] = gs[r + W - 1][p];
-            float a0 = 0.f, a1 = 0.f;
+            dzw[W - 1] = *reinterpret_cast<const f2*>(&gs[r + W - 1][p]);
+            f2 a[1] = {f2_mul(wv[0], dzw[W - 1])};
 #pragma unroll
-            for (int m = 0; m < W; ++m) {
-                a0 += w0[m] * dw_[W - 1 - m].x;
-                a1 += w1[m] * dw_[W - 1 - m].y;
-            }
-            if (t < T && cok) st_pair<BF16>(dx, (rowbase + t) * ldx + c, a0, a1);
+            for (int m = 1; m < W; ++m) a[0] = f2_fma(wv[m], dzw[W - 1 - m], a[0]);
+            if (t < T && cok) st_c2<2, BF16>(dx, (rowbase + t) * ldx + c, a);
 #pragma unroll
-            for (int m = 0; m < W - 1; ++m) dw_[m] = dw_[m + 1];
+            for (int m = 0; m < W - 1; ++m) dzw[m] = dzw[m + 1];
         }
     }
     if (threadIdx.x < kConvTileC && cb + threadIdx.x < C) {
@@ -1233,18 +1373,21 @@ __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C,
 
 // Backward, training path, bf16 with C % 128 == 0.  A thread owns 4 adjacent channels and a run of consecutive tokens
 // and streams down its rows once: x and dy rows arrive through a thread-private ring in shared memory filled by
-// asynchronous 8-byte copies kConvRingDepth rows ahead (no registers held for data in flight, no block-wide barrier in
-// the loop), the x window and the dz window live in registers as circular buffers with compile-time indices, and every
+// asynchronous 8-byte copies up to kConvRingDepth rows ahead (no registers held for data in flight, no block-wide barrier
+// in the loop), the x window and the dz window live in registers as circular buffers with compile-time indices, and every
 // pre-activation, SiLU derivative, dweight and dx multiply-add is done exactly once per element.  Only the W-1 rows
 // either side of a run are touched twice.  Block = 8 warps = 8 runs x 128 channels; one dweight partial per block.
+// Moves 3 x B x T x C elements and was bound by instruction issue (0.47 of the copy rate): channel pairs in packed
+// arithmetic, one copy group per W rows, pointers that walk, and two blocks per SM (at three, 80 registers a thread
+// spilled inside the loop): 266 -> 170 us at 65,536 x 2,048, 0.72 of the copy rate.  A ring of 24 rows gave 175.
 constexpr int kConvRingDepth = 16;
 
 template <int W>
-__global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int C, int ldx, int run, int silu, int wf32, ConvBwdItems items,
+__global__ void __launch_bounds__(256, 2) conv_bwd_ring_kernel(int B, int T, int C, int ldx, int run, int silu, int wf32, ConvBwdItems items,
                                                                float* __restrict__ dw_part) {
-    constexpr int D = kConvRingDepth;
+    constexpr int NG = kConvRingDepth / W;                     // groups of W rows in the ring
     extern __shared__ __align__(16) uint8_t ring_raw[];
-    uint2* ring = reinterpret_cast<uint2*>(ring_raw);          // [D][2: x | dy][256 threads]
+    uint2* ring = reinterpret_cast<uint2*>(ring_raw);          // [NG][W][2: x | dy][256 threads]
     float (*red)[W][128] = reinterpret_cast<float (*)[W][128]>(ring_raw);      // [8][W][128], once the ring is drained
     const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int c = (blockIdx.x * 32 + p) * 4;                   // C % 128 == 0: in range
@@ -1254,96 +1397,110 @@ __global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int
     const void* __restrict__ wgt = pick_item(items.w, item);
     const __nv_bfloat16* __restrict__ dy = static_cast<const __nv_bfloat16*>(pick_item(items.dy, item));
     __nv_bfloat16* __restrict__ dx = static_cast<__nv_bfloat16*>(pick_item(items.dx, item));
-    float wv[W][4];
+    f2 wv[W][2], dwv[W][2];
     {
         float flat[W * 4];
         ld_wrun<W * 4, true>(flat, wgt, (size_t)c * W, wf32);
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < 2; ++e)
 #pragma unroll
-            for (int m = 0; m < W; ++m) wv[m][e] = flat[e * W + m];
+            for (int m = 0; m < W; ++m) {
+                wv[m][e] = f2_make(flat[2 * e * W + m], flat[(2 * e + 1) * W + m]);
+                dwv[m][e] = f2_all(0.f);
+            }
     }
-    float dwv[W][4];
-#pragma unroll
-    for (int m = 0; m < W; ++m)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) dwv[m][e] = 0.f;
-    auto widen = [](const uint2& u, float (&f)[4]) {
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-        const float2 b2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-        f[0] = a.x; f[1] = a.y; f[2] = b2.x; f[3] = b2.y;
-    };
     if (t0 < T) {
         // stream step j handles token tx = t0 - (W-1) + j: x[tx] enters the window; from tx >= t0 on dz[tx] is formed;
         // from tx >= t0 + W-1 on dx[tx - (W-1)] leaves.  Steps run to a multiple of W so the circular indices are static.
         const int nr = ((run + 2 * (W - 1) + W - 1) / W) * W;
         const size_t rowbase = (size_t)b * T;
         const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(ring + threadIdx.x);
-        auto issue = [&](int j) {
-            if (j < nr) {
-                const int tx = min(max(t0 - (W - 1) + j, 0), T - 1);
-                const size_t row = rowbase + tx;
-                const uint32_t dst = slot0 + (uint32_t)((j % D) * 2) * 256u * 8u;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(x + row * ldx + c) : "memory");
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 256u * 8u), "l"(dy + row * C + c) : "memory");
+        // the source pointers walk down the rows: a row outside the sequence reads its nearest row inside and is masked
+        const __nv_bfloat16* xp = x + (rowbase + max(t0 - (W - 1), 0)) * ldx + c;
+        const __nv_bfloat16* gp = dy + (rowbase + max(t0 - (W - 1), 0)) * C + c;
+        __nv_bfloat16* dp = dx + (rowbase + t0) * ldx + c;
+        int jn = 0, sn = 0;                                    // next group to fetch: its first step, its slot
+        auto fetch = [&]() {
+            if (jn < nr) {
+                const uint32_t dst = slot0 + (uint32_t)sn * (W * 2 * 256 * 8);
+                const int tx = t0 - (W - 1) + jn;
+                const bool inner = tx >= 0 && tx + W < T;
+#pragma unroll
+                for (int u = 0; u < W; ++u) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + (2 * u) * 256 * 8), "l"(xp) : "memory");
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + (2 * u + 1) * 256 * 8), "l"(gp) : "memory");
+                    if (inner || (unsigned)(tx + u) < (unsigned)(T - 1)) {
+                        xp += ldx;
+                        gp += C;
+                    }
+                }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
+            jn += W;
+            sn = sn + 1 == NG ? 0 : sn + 1;
         };
 #pragma unroll 1
-        for (int j = 0; j < D - 1; ++j) issue(j);
-        float xc[W][4], dzc[W][4];
+        for (int i = 0; i < NG - 1; ++i) fetch();
+        f2 xc[W][2], dzc[W][2];
 #pragma unroll
         for (int m = 0; m < W; ++m)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) xc[m][e] = dzc[m][e] = 0.f;
-#pragma unroll 1
-        for (int jj = 0; jj < nr; jj += W) {
+            for (int e = 0; e < 2; ++e) xc[m][e] = dzc[m][e] = f2_all(0.f);
+        // EDGE: rows outside the sequence or the run need their masks; the steps in the middle of a run inside the sequence
+        // (all but the first and last few) run without them
+        auto step = [&](int jj, int slot, auto edge) {
+            constexpr bool EDGE = decltype(edge)::value;
+            const uint2* rp = ring + slot * (W * 2 * 256) + threadIdx.x;
 #pragma unroll
             for (int u = 0; u < W; ++u) {
-                const int j = jj + u;
-                issue(j + D - 1);                  // refills the slot whose row was consumed one step ago
-                asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
-                const int tx = t0 - (W - 1) + j;
-                const uint2 xr = ring[((j % D) * 2) * 256 + threadIdx.x];
-                const uint2 gr = ring[((j % D) * 2 + 1) * 256 + threadIdx.x];
-                widen(xr, xc[u]);
-                if (tx < 0 || tx >= T) {
+                const int tx = t0 - (W - 1) + jj + u;
+                const uint2 xr = rp[(2 * u) * 256];
+                const uint2 gr = rp[(2 * u + 1) * 256];
+                xc[u][0] = f2_from_bf16(xr.x);
+                xc[u][1] = f2_from_bf16(xr.y);
+                f2 gy[2] = {f2_from_bf16(gr.x), f2_from_bf16(gr.y)};
+                if (EDGE && (tx < 0 || tx >= T)) xc[u][0] = xc[u][1] = f2_all(0.f);
+                const bool live = !EDGE || (tx >= t0 && tx < T);              // dz[tx] exists and belongs to this run's window
+                const bool own = !EDGE || (live && tx < t0 + run);            // ... and its dweight is this run's
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) xc[u][e] = 0.f;
-                }
-                float gy[4];
-                widen(gr, gy);
-                const bool live = tx >= t0 && tx < T;             // dz[tx] exists and belongs to this run's window
-                const bool own = live && tx < t0 + run;           // ... and its dweight is this run's
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    float z = 0.f;
-#pragma unroll
-                    for (int m = 0; m < W; ++m) z += wv[m][e] * xc[(u + 1 + m) % W][e];      // x[tx - (W-1) + m]
-                    float dzv = gy[e];
+                for (int e = 0; e < 2; ++e) {
                     if (silu) {
-                        const float sg = sigmoid_t<true>(z);
-                        dzv *= sg * (1.f + z * (1.f - sg));
+                        f2 z = f2_mul(wv[0][e], xc[(u + 1) % W][e]);          // x[tx - (W-1) + m]
+#pragma unroll
+                        for (int m = 1; m < W; ++m) z = f2_fma(wv[m][e], xc[(u + 1 + m) % W][e], z);
+                        gy[e] = silu_vjp_2<true>(gy[e], z);
                     }
-                    dzv = live ? dzv : 0.f;
-                    dzc[u][e] = dzv;
+                    if (!live) gy[e] = f2_all(0.f);
+                    dzc[u][e] = gy[e];
                     if (own) {
 #pragma unroll
-                        for (int m = 0; m < W; ++m) dwv[m][e] += dzv * xc[(u + 1 + m) % W][e];
+                        for (int m = 0; m < W; ++m) dwv[m][e] = f2_fma(gy[e], xc[(u + 1 + m) % W][e], dwv[m][e]);
                     }
                 }
                 const int td = tx - (W - 1);
-                if (td >= t0 && td < t0 + run && td < T) {
-                    float a[4];
+                if (!EDGE || (td >= t0 && td < t0 + run && td < T)) {
+                    f2 a[2];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        a[e] = 0.f;
+                    for (int e = 0; e < 2; ++e) {
+                        a[e] = f2_mul(wv[0][e], dzc[u][e]);                   // dz[tx - m]
 #pragma unroll
-                        for (int m = 0; m < W; ++m) a[e] += wv[m][e] * dzc[(u - m + W) % W][e];  // dz[tx - m]
+                        for (int m = 1; m < W; ++m) a[e] = f2_fma(wv[m][e], dzc[(u - m + W) % W][e], a[e]);
                     }
-                    st_cvec<4, true>(dx, (rowbase + td) * ldx + c, a);
+                    st_c2<4, true>(dp, 0, a);
+                    dp += ldx;
                 }
             }
+        };
+        // rows tx of the steps jj .. jj + W - 1 and the outputs tx - (W-1) all inside [t0, min(T, t0 + run))
+        const int inner0 = 2 * (W - 1), inner1 = min(T - t0, run) + W - 1;
+        int slot = 0;
+#pragma unroll 1
+        for (int jj = 0; jj < nr; jj += W) {
+            fetch();                                           // refills the slot that the previous group was read from
+            asm volatile("cp.async.wait_group %0;" ::"n"(NG - 1) : "memory");
+            if (jj >= inner0 && jj + W <= inner1) step(jj, slot, std::false_type());
+            else step(jj, slot, std::true_type());
+            slot = slot + 1 == NG ? 0 : slot + 1;
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
@@ -1351,7 +1508,7 @@ __global__ void __launch_bounds__(256, 3) conv_bwd_ring_kernel(int B, int T, int
 #pragma unroll
     for (int m = 0; m < W; ++m)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) red[g][m][4 * p + e] = dwv[m][e];
+        for (int e = 0; e < 2; ++e) *reinterpret_cast<f2*>(&red[g][m][4 * p + 2 * e]) = dwv[m][e];
     __syncthreads();
     if (threadIdx.x < 128) {
         const size_t pblk = (size_t)blockIdx.z * gridDim.y + blockIdx.y;
@@ -1872,12 +2029,21 @@ namespace {
 inline bool conv_grid_ok(int n, int B, int T) { return ceil_div(T, 8 * pw::kConvPairT) <= 65535 && (long long)B * n <= 65535; }
 
 // n same-shaped convolutions in one launch; x rows ldx elements apart
+constexpr int kConvRun = 32;      // tokens per thread of the streaming forward
 template <int W>
 int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st) {
     const bool vec4 = C % 128 == 0 && ldx % 4 == 0;         // channels per thread: 4 when a warp's 128 channels fill a row segment
     const dim3 grid(ceil_div(C, vec4 ? 128 : 64), ceil_div(T, 8 * pw::kConvPairT), B * n);
     bool win = false;
     for (int i = 0; i < n; ++i) win = win || it.cache[i] != nullptr || it.fin[i] != nullptr;
+    // enough tokens that 32-token runs still give every SM three blocks several times over: the streaming kernel
+    if (vec4 && bf16 && !win) {
+        const dim3 sgrid(C / 128, ceil_div(T, 8 * kConvRun), B * n);
+        if ((long long)sgrid.x * sgrid.y * sgrid.z >= 148LL * 3 * 4) {
+            KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, silu, wf32, it));
+            return launch_status();
+        }
+    }
 #define KDA_CONV_FWD(VEC, BF, WIN) \
     KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, VEC, BF, WIN><<<grid, 256, 0, st>>>(B, T, C, ldx, silu, wf32, it))
     if (vec4 && bf16) { if (win) KDA_CONV_FWD(4, true, true); else KDA_CONV_FWD(4, true, false); }

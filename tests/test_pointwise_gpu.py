@@ -96,6 +96,22 @@ def test_conv_training_path_matches_oracle(B, T, C, dtype):
     assert O.rel_l2(got[1].squeeze(1).float(), want[1]) <= tol
 
 
+# from 1,776 blocks of 256 tokens x 128 channels on: ends within a group of 8 rows, a run of 32, a block; every window width class
+@pytest.mark.parametrize("W,B,T,C", [(4, 1, 28423, 2048), (2, 1, 28417, 2048), (3, 111, 511, 1024), (4, 1776, 5, 128), (1, 1776, 17, 128), (8, 222, 33, 1024)])
+def test_streaming_convolution_equals_short_pieces(W, B, T, C):
+    """Both kernels sum a window in the same order, so the long call equals calls on pieces of it to the bit."""
+    gen = torch.Generator(device=D0).manual_seed(T + W)
+    x = torch.randn(B, T, C, device=D0, generator=gen).bfloat16()
+    mod = _conv_mod(C, W, torch.randn(C, W, device=D0, generator=gen))
+    with torch.no_grad():
+        y, _ = mod(x)
+        for b in sorted({0, B // 2, B - 1}):
+            for t0 in range(0, T, 4096):
+                h = min(t0, W - 1)
+                piece, _ = mod(x[b:b + 1, t0 - h:t0 + 4096].contiguous())
+                assert torch.equal(y[b, t0:t0 + 4096], piece[0, h:])
+
+
 @pytest.mark.parametrize("B,T,C,dtype", [(2, 300, 384, torch.bfloat16), (1, 67, 20, torch.float32)])
 def test_short_convolutions_one_launch_equals_per_tensor_calls(B, T, C, dtype):
     """The batched q/k/v convolution entry points give bit-identical outputs and gradients to three separate calls."""
