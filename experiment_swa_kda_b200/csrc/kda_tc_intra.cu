@@ -32,6 +32,7 @@ int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
 namespace {
 
 constexpr int kLDs = 68;      // leading dimension (floats) of the 64x64 fp32 tiles of the inverse
+constexpr int kLDt = 36;      // ... and of its 32-row scratch
 constexpr int kNT = 256;
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -82,9 +83,9 @@ __device__ __forceinline__ float fast_rcp(float x) {
     return y;
 }
 
-// dst = alpha * A * B for NP independent S x S problems (row-major fp32, leading dimension kLDs), all 256 threads busy:
+// dst = alpha * A * B for NP independent S x S problems (row-major fp32, leading dimensions kLDs, LB, LD), all 256 threads busy:
 // a thread owns one row piece of CW adjacent columns of one product.
-template <int S, int NP, class PA, class PB, class PD>
+template <int S, int NP, int LB, int LD, class PA, class PB, class PD>
 __device__ __forceinline__ void tile_mm(PA pa, PB pb, PD pd, float alpha) {
     constexpr int CW = S * S * NP / kNT;          // columns per thread: 1 (8x8x4), 2 (16x16x2), 4 (32x32x1)
     constexpr int TPR = S / CW;                   // threads per row
@@ -100,21 +101,21 @@ __device__ __forceinline__ void tile_mm(PA pa, PB pb, PD pd, float alpha) {
     for (int t = 0; t < S; ++t) {
         const float a = A[t];
         if (CW == 4) {
-            const float4 b = *reinterpret_cast<const float4*>(B + t * kLDs);
+            const float4 b = *reinterpret_cast<const float4*>(B + t * LB);
             acc[0] += a * b.x; acc[1 % CW] += a * b.y; acc[2 % CW] += a * b.z; acc[3 % CW] += a * b.w;
         } else if (CW == 2) {
-            const float2 b = *reinterpret_cast<const float2*>(B + t * kLDs);
+            const float2 b = *reinterpret_cast<const float2*>(B + t * LB);
             acc[0] += a * b.x; acc[1 % CW] += a * b.y;
         } else {
-            acc[0] += a * B[t * kLDs];
+            acc[0] += a * B[t * LB];
         }
     }
-    float* D = pd(prob) + i * kLDs + j0;
+    float* D = pd(prob) + i * LD + j0;
 #pragma unroll
     for (int c = 0; c < CW; ++c) D[c] = alpha * acc[c];
 }
 
-// D = alpha * A * B for S x S fp32 tiles in shared memory (leading dimension kLDs) on the warp-level tensor-core path:
+// D = alpha * A * B for S x S fp32 tiles in shared memory (leading dimensions kLDs, LB, LD) on the warp-level tensor-core path:
 // mma.sync m16n8k8 with every operand split into two TF32 terms (hi + lo; lo*lo dropped), which keeps float32-class
 // accuracy - T feeds every later product - while one product costs a warp S/8 short steps instead of S dependent
 // shared-memory round trips.  These few 16..32-wide dependent products are latency-bound; a tcgen05 round trip
@@ -130,7 +131,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-template <int S, int NP, class PA, class PB, class PD>
+template <int S, int NP, int LB, int LD, class PA, class PB, class PD>
 __device__ __forceinline__ void warp_mm(PA pa, PB pb, PD pd, float alpha) {
     constexpr int TR = S / 16, TC = S / 8;         // output tiles per problem
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -139,7 +140,7 @@ __device__ __forceinline__ void warp_mm(PA pa, PB pb, PD pd, float alpha) {
     const int r0 = 16 * (tile / TC), c0 = 8 * (tile % TC);
     const int g = lane >> 2, tig = lane & 3;
     const float* A = pa(prob) + (r0 + g) * kLDs + tig;
-    const float* B = pb(prob) + tig * kLDs + c0 + g;
+    const float* B = pb(prob) + tig * LB + c0 + g;
     float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int ks = 0; ks < S / 8; ++ks) {
@@ -148,15 +149,15 @@ __device__ __forceinline__ void warp_mm(PA pa, PB pb, PD pd, float alpha) {
         split_tf32(A[8 * kLDs + 8 * ks], ah[1], al[1]);
         split_tf32(A[8 * ks + 4], ah[2], al[2]);
         split_tf32(A[8 * kLDs + 8 * ks + 4], ah[3], al[3]);
-        split_tf32(B[(8 * ks) * kLDs], bh[0], bl[0]);
-        split_tf32(B[(8 * ks + 4) * kLDs], bh[1], bl[1]);
+        split_tf32(B[(8 * ks) * LB], bh[0], bl[0]);
+        split_tf32(B[(8 * ks + 4) * LB], bh[1], bl[1]);
         mma_tf32(d, al, bh);
         mma_tf32(d, ah, bl);
         mma_tf32(d, ah, bh);
     }
-    float* D = pd(prob) + (r0 + g) * kLDs + c0 + 2 * tig;
+    float* D = pd(prob) + (r0 + g) * LD + c0 + 2 * tig;
     *reinterpret_cast<float2*>(D) = make_float2(alpha * d[0], alpha * d[1]);
-    *reinterpret_cast<float2*>(D + 8 * kLDs) = make_float2(alpha * d[2], alpha * d[3]);
+    *reinterpret_cast<float2*>(D + 8 * LD) = make_float2(alpha * d[2], alpha * d[3]);
 }
 
 // Ts = (I + Ms)^-1 for strictly lower-triangular Ms (64x64): 8x8 diagonal solves (a short dependent chain per thread),
@@ -185,21 +186,21 @@ __device__ __forceinline__ void unit_lower_inverse(const float* Ms, float* Ts, f
     }
     __syncthreads();
     // merges: tmp_p = C_p Ai_p ; T21_p = -Bi_p tmp_p
-    tile_mm<8, 4>([&](int p) { return Ms + (16 * p + 8) * kLDs + 16 * p; }, [&](int p) { return Ts + (16 * p) * kLDs + 16 * p; },
-                  [&](int p) { return tmp + p * 8 * kLDs; }, 1.f);
+    tile_mm<8, 4, kLDs, kLDt>([&](int p) { return Ms + (16 * p + 8) * kLDs + 16 * p; }, [&](int p) { return Ts + (16 * p) * kLDs + 16 * p; },
+                  [&](int p) { return tmp + p * 8 * kLDt; }, 1.f);
     __syncthreads();
-    tile_mm<8, 4>([&](int p) { return Ts + (16 * p + 8) * kLDs + 16 * p + 8; }, [&](int p) { return tmp + p * 8 * kLDs; },
+    tile_mm<8, 4, kLDt, kLDs>([&](int p) { return Ts + (16 * p + 8) * kLDs + 16 * p + 8; }, [&](int p) { return tmp + p * 8 * kLDt; },
                   [&](int p) { return Ts + (16 * p + 8) * kLDs + 16 * p; }, -1.f);
     __syncthreads();
-    warp_mm<16, 2>([&](int p) { return Ms + (32 * p + 16) * kLDs + 32 * p; }, [&](int p) { return Ts + (32 * p) * kLDs + 32 * p; },
-                   [&](int p) { return tmp + p * 16 * kLDs; }, 1.f);
+    warp_mm<16, 2, kLDs, kLDt>([&](int p) { return Ms + (32 * p + 16) * kLDs + 32 * p; }, [&](int p) { return Ts + (32 * p) * kLDs + 32 * p; },
+                   [&](int p) { return tmp + p * 16 * kLDt; }, 1.f);
     __syncthreads();
-    warp_mm<16, 2>([&](int p) { return Ts + (32 * p + 16) * kLDs + 32 * p + 16; }, [&](int p) { return tmp + p * 16 * kLDs; },
+    warp_mm<16, 2, kLDt, kLDs>([&](int p) { return Ts + (32 * p + 16) * kLDs + 32 * p + 16; }, [&](int p) { return tmp + p * 16 * kLDt; },
                    [&](int p) { return Ts + (32 * p + 16) * kLDs + 32 * p; }, -1.f);
     __syncthreads();
-    warp_mm<32, 1>([&](int) { return Ms + 32 * kLDs; }, [&](int) { return Ts; }, [&](int) { return tmp; }, 1.f);
+    warp_mm<32, 1, kLDs, kLDt>([&](int) { return Ms + 32 * kLDs; }, [&](int) { return Ts; }, [&](int) { return tmp; }, 1.f);
     __syncthreads();
-    warp_mm<32, 1>([&](int) { return Ts + 32 * kLDs + 32; }, [&](int) { return tmp; }, [&](int) { return Ts + 32 * kLDs; }, -1.f);
+    warp_mm<32, 1, kLDt, kLDs>([&](int) { return Ts + 32 * kLDs + 32; }, [&](int) { return tmp; }, [&](int) { return Ts + 32 * kLDs; }, -1.f);
     __syncthreads();
 }
 
@@ -219,16 +220,21 @@ struct IntraFwdArgs {
     ConvPrep conv;
 };
 
-// shared-memory map (bytes from a 1024-aligned base)
-constexpr int kFS = 0;             // 32 KB  source stack of the chain in flight: [2 target blocks][64 rows], 2 k-blocks of 16 KB
-constexpr int kFX = 32768;         // 32 KB  target stacks, chain pr at pr * 16 KB: rows (blk & 1) * 32 + {q: r, k: 16 + r}
-constexpr int kFV = 65536;         // 16 KB  v tile (TMA): MN-major A of U^T = v^T (T diag(beta))^T
-constexpr int kFQ = 81920;         // 16 KB  Q = beta e^G k: MN-major A of W^T = Q^T T^T
-constexpr int kFTab = 98304;       // floats: cref[4][128] eC[4][128] eEnd[4][128] fb[3][128] | gend[128] | bet[64]
-constexpr int kTabFloats = 15 * 128 + 128 + 64;
-// after the A / M~ chains the stacks are dead: Ms, Ts, tmp (fp32) and the two bf16 T operands live in [0, 64 KB)
-constexpr int kFMs = 0, kFTs = 64 * kLDs * 4, kFTmp = 2 * 64 * kLDs * 4, kFTb = 49152, kFTbb = 57344;
-static_assert(kFTmp + 32 * kLDs * 4 <= kFTb, "inverse scratch overlaps the T operands");
+// shared-memory map (bytes from a 1024-aligned base).  Source rows: a 16-row target block I needs the source rows of the
+// blocks <= I scaled to its own decay reference, 16 + 32 + 48 + 64 rows; blocks 3, 2 and 0 fill one 128-row stack exactly,
+// block 1 has its own, so that all of them exist at once and the two products run back to back.
+constexpr int kFSA = 0;            // 32 KB  sources of target blocks 3 | 2 | 0 (64 | 48 | 16 rows), 2 k-blocks of 16 KB
+constexpr int kFSB = 32768;        //  8 KB  sources of target block 1 (32 rows), 2 k-blocks of 4 KB
+constexpr int kFXA = 40960;        // 24 KB  targets 3 | 2 | 0 (32 rows each: 16 q~, 16 k~), 2 k-blocks of 12 KB
+constexpr int kFXB = 65536;        //  8 KB  targets 1, 2 k-blocks of 4 KB
+constexpr int kFQ = 73728;         // 16 KB  Q = beta e^G k: MN-major A of W^T = Q^T T^T
+constexpr int kFTab = 90112;       // floats: cref[4][128] eC[4][128] eEnd[4][128] fb[3][128] | gfirst[4][128] | bet[64]
+constexpr int kTabFloats = 15 * 128 + 4 * 128 + 64;
+// after the A / M~ products the stacks are dead: Ms, Ts (fp32), the two bf16 T operands and the value tile live in
+// [0, 72 KB), the inverse's scratch in the dead tables
+constexpr int kFMs = 0, kFTs = 64 * kLDs * 4, kFTb = 35840, kFTbb = 44032;
+constexpr int kFV = 53248;         // 16 KB  v tile (TMA): MN-major A of U^T = v^T (T diag(beta))^T
+static_assert(kFTs + 64 * kLDs * 4 <= kFTb && kFV + 16384 <= kFQ && 32 * kLDt <= 15 * 128, "shared-memory map");
 constexpr int kIntraFwdSmem = kFTab + kTabFloats * 4 + 1024;
 
 // y = silu(sum_m w[m] x[t - 3 + m]) for this thread's 4 rows x 8 channels from the 7 input rows it needs, in the
@@ -277,22 +283,21 @@ __global__ void __launch_bounds__(kNT, 2)
                         const __grid_constant__ CUtensorMap mTp, IntraFwdArgs p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
-    uint8_t* Sst = sm + kFS;
     uint8_t* vs = sm + kFV;
     uint8_t* Qs = sm + kFQ;
     float* cref = reinterpret_cast<float*>(sm + kFTab);      // [4][128] G at the first row of each 16-row block
     float* eC = cref + 512;                                  // [4][128] exp(cref)
     float* eEnd = eC + 512;                                  // [4][128] exp(G_end - cref)
     float* fbk = eEnd + 512;                                 // [3][128] exp(cref[I+1] - cref[I])
-    float* gends = fbk + 384;                                // [128]    G_end
-    float* bet = gends + 128;                                // [64]
-    float* wtot = reinterpret_cast<float*>(sm + kFS);        // [8][128] per-warp sums of g (dead before the stacks are written)
+    float* gfirst = fbk + 384;                               // [4][128] g of the first row of each block
+    float* bet = gfirst + 512;                               // [64]
+    float* wtot = reinterpret_cast<float*>(sm + kFSA);       // [8][128] per-warp sums of g (dead before the stacks are written)
     float* Ms = reinterpret_cast<float*>(sm + kFMs);
     float* Ts = reinterpret_cast<float*>(sm + kFTs);
-    float* tmp = reinterpret_cast<float*>(sm + kFTmp);
+    float* tmp = cref;
     uint8_t* Tb = sm + kFTb;                                 // [64 rows x 128 B] K-major B: T
     uint8_t* Tbb = sm + kFTbb;                               //                              T diag(beta)
-    __shared__ uint64_t bar_in, bar_am[2], bar_uw, bar_tr;
+    __shared__ uint64_t bar_in, bar_am, bar_uw, bar_tr;
     __shared__ uint32_t tmem_slot;
 
     const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
@@ -308,15 +313,10 @@ __global__ void __launch_bounds__(kNT, 2)
 
     if (tid == 0) {
         mbar_init(&bar_in, 1);
-        mbar_init(&bar_am[0], 1);
-        mbar_init(&bar_am[1], 1);
+        mbar_init(&bar_am, 2);
         mbar_init(&bar_uw, 1);
         mbar_init(&bar_tr, 1);
         mbar_fence_init();
-        if (!CONV) {
-            mbar_expect_tx(&bar_in, 16384);
-            for (int kb = 0; kb < 2; ++kb) tma_load_2d(vs + kb * 8192, &mv, &bar_in, h * 128 + kb * 64, tok0);
-        }
     }
     if (warp == 1) tmem_alloc(&tmem_slot, 256);
 
@@ -326,34 +326,25 @@ __global__ void __launch_bounds__(kNT, 2)
     float G[4][8];
     uint4 qraw[4], kraw[4];
     float brow[4];
-    if constexpr (CONV) {
-        // the three convolutions, one after the other (7 input rows for 4 output rows; the rows before the chunk belong to
-        // the previous chunk of the same sequence, or are the zero padding at a sequence start); v goes straight into the
-        // operand tile that TMA would have filled
+    // CONV: 7 input rows for 4 output rows; the rows before the chunk belong to the previous chunk of the same sequence, or
+    // are the zero padding at a sequence start
+    const size_t wbase = ((size_t)h * 128 + 8 * cg) * 4;
+    auto conv_rows = [&](const __nv_bfloat16* x, uint4 (&xr)[7]) {
         const bool first = p.w.seq_chunk0[p.w.chunk_seq[slot]] == slot;
-        const size_t wbase = ((size_t)h * 128 + 8 * cg) * 4;
-        auto rows = [&](const __nv_bfloat16* x, uint4 (&xr)[7]) {
 #pragma unroll
-            for (int jj = 0; jj < 7; ++jj) {
-                const int i = 4 * rq - 3 + jj;
-                const long long ic = min(i, len - 1);      // rows past the tail feed masked outputs only
-                xr[jj] = (i >= 0 || !first) ? __ldg(reinterpret_cast<const uint4*>(x + ((long long)tok0 + ic) * p.conv.x_ld + h * 128 + 8 * cg))
-                                            : make_uint4(0, 0, 0, 0);
-            }
-        };
-        uint4 xr[7];
-        rows(p.q, xr);
-        conv4_silu_rows(xr, p.conv.w[0], wbase, p.conv.wf32, qraw);
-        rows(p.k, xr);
-        conv4_silu_rows(xr, p.conv.w[1], wbase, p.conv.wf32, kraw);
-        rows(p.xv, xr);
-        uint4 vr[4];
-        conv4_silu_rows(xr, p.conv.w[2], wbase, p.conv.wf32, vr);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int i = 4 * rq + j;
-            *reinterpret_cast<uint4*>(vs + piece_off(i, cg, 8192)) = i < len ? vr[j] : make_uint4(0, 0, 0, 0);
+        for (int jj = 0; jj < 7; ++jj) {
+            const int i = 4 * rq - 3 + jj;
+            const long long ic = min(i, len - 1);      // rows past the tail feed masked outputs only
+            xr[jj] = (i >= 0 || !first) ? __ldg(reinterpret_cast<const uint4*>(x + ((long long)tok0 + ic) * p.conv.x_ld + h * 128 + 8 * cg))
+                                        : make_uint4(0, 0, 0, 0);
         }
+    };
+    if constexpr (CONV) {      // v's convolution follows once its operand tile is free
+        uint4 xr[7];
+        conv_rows(p.q, xr);
+        conv4_silu_rows(xr, p.conv.w[0], wbase, p.conv.wf32, qraw);
+        conv_rows(p.k, xr);
+        conv4_silu_rows(xr, p.conv.w[1], wbase, p.conv.wf32, kraw);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -372,6 +363,7 @@ __global__ void __launch_bounds__(kNT, 2)
             brow[j] = 0.f;
         }
     }
+    if ((rq & 3) == 0) sts8c(gfirst + J * 128 + 4 * cg, G[0]);
     // ---- cumulative log-decay: within the thread, across the two half-warps, then across warps through shared memory
 #pragma unroll
     for (int j = 1; j < 4; ++j)
@@ -419,171 +411,213 @@ __global__ void __launch_bounds__(kNT, 2)
         qi[j] *= p.scale;
     }
     tc_fence_before();
-    __syncthreads();                                   // (1) warp sums, TMEM slot
+    __syncthreads();                                   // (1) warp sums, first rows, TMEM slot
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     {
-        float gend[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) gend[c] = 0.f;
+        // per (block, channel) factors, two entries a thread, straight from the warp sums (two warps to a block).  The sums
+        // run in the order of a row's own G below, so that a block's first row has the factor 1 exactly.
+        const int pos = tid & 127;
+        float run[5], wsum = 0.f;                      // G at the first row of each block, then G_end
 #pragma unroll
         for (int w2 = 0; w2 < 8; ++w2) {
+            if ((w2 & 1) == 0) run[w2 >> 1] = gfirst[(w2 >> 1) * 128 + pos] + wsum;
+            wsum += wtot[w2 * 128 + pos];
+        }
+        run[4] = wsum;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if ((e & 1) == (tid >> 7)) {
+                cref[e * 128 + pos] = run[e];
+                eC[e * 128 + pos] = __expf(run[e]);
+                eEnd[e * 128 + pos] = __expf(wsum - run[e]);
+                if (e < 3) fbk[e * 128 + pos] = __expf(run[e + 1] - run[e]);
+            }
+        }
+        if (tid < 128)      // position -> channel
+            p.t.decay_end[ch * 128 + ((pos & 63) >> 2) * 8 + (pos >> 6) * 4 + (pos & 3)] = __expf(wsum);
+    }
+    {
+        for (int w2 = 0; w2 < warp; ++w2) {
             float t[8];
             lds8c(wtot + w2 * 128 + 4 * cg, t);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                gend[c] += t[c];
-                pre[c] += (w2 < warp) ? t[c] : 0.f;
-            }
+            for (int c = 0; c < 8; ++c) pre[c] += t[c];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int c = 0; c < 8; ++c) G[j][c] += pre[c];
-        if ((rq & 3) == 0) sts8c(cref + J * 128 + 4 * cg, G[0]);      // first row of block J
-        if (rq == 0) {
-            sts8c(gends + 4 * cg, gend);
-            float e[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) e[c] = __expf(gend[c]);
-            float* de = p.t.decay_end + ch * 128 + 8 * cg;
-            *reinterpret_cast<float4*>(de) = make_float4(e[0], e[1], e[2], e[3]);
-            *reinterpret_cast<float4*>(de + 4) = make_float4(e[4], e[5], e[6], e[7]);
-        }
     }
-    __syncthreads();                                   // (2) block references; wtot is dead from here
-    // per (block, channel) factors, 512 + 384 entries over 256 threads
-    for (int e = tid; e < 512; e += kNT) {
-        const int I = e >> 7, d = e & 127;
-        const float c = cref[e];
-        eC[e] = __expf(c);
-        eEnd[e] = __expf(gends[d] - c);
-        if (I < 3) fbk[e] = __expf(cref[e + 128] - c);
-    }
-    __syncthreads();                                   // (3) tables
+    __syncthreads();                                   // (2) tables; wtot is dead from here
 
-    // ---- operand panels, one row at a time: 16-byte pieces of the swizzled layouts
+    // ---- operand panels, one row at a time, four channels at a time in packed pairs: 16-byte pieces of the swizzled
+    // layouts.  Bound by instruction issue: two exponentials and reciprocals an element are 6 of its ~20 instructions.
+    uint32_t rw[4][4];                                 // R = q e^G, rows 4rq .. 4rq+3, channel pairs
     {
-        float cJ[8];
-        lds8c(cref + J * 128 + 4 * cg, cJ);
-        uint8_t* X = sm + kFX + (J >> 1) * 16384;
+        // row bases of target block b in the stacks: {3, 2, 0} share the first pair, {1} has the second
+        uint8_t* X = sm + (J == 1 ? kFXB : kFXA);
+        const uint32_t xkb = J == 1 ? 4096u : 12288u;
+        const int xr0 = J == 3 || J == 1 ? 0 : (J == 2 ? 32 : 64);
         __nv_bfloat16* Eg = p.t.E + ch * 8192 + 8 * cg;
-        uint32_t rt[8][2];                             // R^T: channel c, rows 4rq .. 4rq+3 as two bf16 pairs
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int i = 4 * rq + j, r16 = i & 15;
-            float fq[8], fk[8], ec[8], ee[8], f0[8], o8[8];
-            unpack_bf16x8(qraw[j], fq);
-            unpack_bf16x8(kraw[j], fk);
-            lds8c(eC + J * 128 + 4 * cg, ec);
-            lds8c(eEnd + J * 128 + 4 * cg, ee);
-            float tq[8], inv[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                tq[c] = __expf(G[j][c] - cJ[c]);       // e^{G - c_J} in (0, 1]
-                inv[c] = fast_rcp(tq[c]);              // e^{c_J - G}
-                fq[c] *= qi[j];
-                fk[c] *= ki[j];
-            }
-            const int xr = (J & 1) * 32 + r16;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) o8[c] = fq[c] * tq[c];
-            *reinterpret_cast<uint4*>(X + piece_off(xr, cg, 8192)) = pack8(o8);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) o8[c] = fk[c] * tq[c];
-            *reinterpret_cast<uint4*>(X + piece_off(xr + 16, cg, 8192)) = pack8(o8);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) f0[c] = fk[c] * inv[c];      // source row scaled to its own block
-            if (J <= 1) {                              // chain 0: target blocks 0, 1
-                if (J == 0) {
-                    *reinterpret_cast<uint4*>(Sst + piece_off(i, cg, 16384)) = pack8(f0);
-                    float fb[8];
-                    lds8c(fbk + 4 * cg, fb);
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) o8[c] = f0[c] * fb[c];
-                    *reinterpret_cast<uint4*>(Sst + piece_off(64 + i, cg, 16384)) = pack8(o8);
-                } else {
-                    *reinterpret_cast<uint4*>(Sst + piece_off(64 + i, cg, 16384)) = pack8(f0);
-                }
-            }
-            // E = k e^{G_end - G} (global, token-major), Q = beta e^G k, R = q e^G
-#pragma unroll
-            for (int c = 0; c < 8; ++c) o8[c] = f0[c] * ee[c];
-            *reinterpret_cast<uint4*>(Eg + (size_t)i * 128) = pack8(o8);
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float eg = tq[c] * ec[c];        // e^G
-                o8[c] = brow[j] * eg * fk[c];
-                const float r = fq[c] * eg;
-                if (j & 1) rt[c][j >> 1] = pack2(__uint_as_float(rt[c][j >> 1]), r);
-                else rt[c][j >> 1] = __float_as_uint(r);
-            }
-            *reinterpret_cast<uint4*>(Qs + piece_off(i, cg, 8192)) = pack8(o8);
-        }
-        __nv_bfloat16* Rg = p.t.RT + ch * 8192 + (size_t)(8 * cg) * 64 + 4 * rq;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint2*>(Rg + c * 64) = make_uint2(rt[c][0], rt[c][1]);
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();                                   // (4) chain-0 operands complete
-    auto issue_am = [&](int pr) {
-        tc_fence_after();
-        const uint32_t idesc = umma_idesc_bf16(128, 64, kMajorK, kMajorK);
-        const uint32_t a0 = smem_u32(Sst), b0 = smem_u32(sm + kFX + pr * 16384);
-#pragma unroll
-        for (int k16 = 0; k16 < 8; ++k16)
-            umma_bf16_ss(tmem + pr * 64, umma_smem_desc_sw128(a0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                         umma_smem_desc_sw128(b0 + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), idesc, k16 > 0);
-        umma_commit(&bar_am[pr]);
-    };
-    if (tid == 0) issue_am(0);
-    // ---- chain 1 (target blocks 2, 3): its source rows go into the same buffer once chain 0 has read it
-    bool ok = mbar_wait(&bar_am[0], 0, p.t.status, 31);
-    {
-        float c2[8];
-        lds8c(cref + 2 * 128 + 4 * cg, c2);
-        float fb2[8];
-        lds8c(fbk + 2 * 128 + 4 * cg, fb2);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int i = 4 * rq + j;
-            float fk[8], s2[8], s3[8];
-            unpack_bf16x8(kraw[j], fk);
-            if (J <= 2) {
-                // e^{c_2 - G} for rows of blocks 0..2 (for block 2 this is the own-block factor)
+            const uint32_t qw[4] = {qraw[j].x, qraw[j].y, qraw[j].z, qraw[j].w};
+            const uint32_t kw[4] = {kraw[j].x, kraw[j].y, kraw[j].z, kraw[j].w};
+            const f2 qi2 = f2_all(qi[j]), ki2 = f2_all(ki[j]), b2 = f2_all(brow[j]);
+            uint32_t xq[4], xk[4], src[4][4], ew[4], pw[4];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    s2[c] = fk[c] * ki[j] * __expf(c2[c] - G[j][c]);
-                    s3[c] = s2[c] * fb2[c];
+            for (int hf = 0; hf < 2; ++hf) {
+                const int to = J * 128 + 64 * hf + 4 * cg;
+                const float4 cJ = *reinterpret_cast<const float4*>(cref + to);
+                const float4 ec = *reinterpret_cast<const float4*>(eC + to);
+                const float4 ee = *reinterpret_cast<const float4*>(eEnd + to);
+                const f2 cj2[2] = {f2_make(cJ.x, cJ.y), f2_make(cJ.z, cJ.w)};
+                const f2 ec2[2] = {f2_make(ec.x, ec.y), f2_make(ec.z, ec.w)};
+                const f2 ee2[2] = {f2_make(ee.x, ee.y), f2_make(ee.z, ee.w)};
+                f2 f0[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int w = 2 * hf + e;
+                    const float2 x = f2_get(f2_fma(cj2[e], f2_all(-1.f), f2_make(G[j][2 * w], G[j][2 * w + 1])));
+                    const float t0 = __expf(x.x), t1 = __expf(x.y);        // e^{G - c_J} in (0, 1]
+                    const f2 tq = f2_make(t0, t1);
+                    const f2 q = f2_mul(f2_from_bf16(qw[w]), qi2), k = f2_mul(f2_from_bf16(kw[w]), ki2);
+                    xq[w] = f2_to_bf16(f2_mul(q, tq));
+                    xk[w] = f2_to_bf16(f2_mul(k, tq));
+                    const f2 eg = f2_mul(tq, ec2[e]);                      // e^G
+                    pw[w] = f2_to_bf16(f2_mul(f2_mul(b2, eg), k));         // Q = beta e^G k
+                    rw[j][w] = f2_to_bf16(f2_mul(q, eg));
+                    f0[e] = f2_mul(k, f2_make(fast_rcp(t0), fast_rcp(t1)));      // source row scaled to its own block
+                    ew[w] = f2_to_bf16(f2_mul(f0[e], ee2[e]));             // E = k e^{G_end - G}
+                    src[0][w] = f2_to_bf16(f0[e]);
                 }
-                *reinterpret_cast<uint4*>(Sst + piece_off(i, cg, 16384)) = pack8(s2);
-            } else {
-                float c3[8];
-                lds8c(cref + 3 * 128 + 4 * cg, c3);
+                // ... and to every later block
 #pragma unroll
-                for (int c = 0; c < 8; ++c) s3[c] = fk[c] * ki[j] * __expf(c3[c] - G[j][c]);
+                for (int v = 1; v < 4; ++v) {
+                    if (J + v < 4) {
+                        const float4 fb = *reinterpret_cast<const float4*>(fbk + (J + v - 1) * 128 + 64 * hf + 4 * cg);
+                        f0[0] = f2_mul(f0[0], f2_make(fb.x, fb.y));
+                        f0[1] = f2_mul(f0[1], f2_make(fb.z, fb.w));
+                        src[v][2 * hf] = f2_to_bf16(f0[0]);
+                        src[v][2 * hf + 1] = f2_to_bf16(f0[1]);
+                    }
+                }
             }
-            *reinterpret_cast<uint4*>(Sst + piece_off(64 + i, cg, 16384)) = pack8(s3);
+            auto put = [](uint8_t* dst, const uint32_t (&w)[4]) { *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]); };
+            put(X + piece_off(xr0 + (i & 15), cg, xkb), xq);
+            put(X + piece_off(xr0 + 16 + (i & 15), cg, xkb), xk);
+            put(Qs + piece_off(i, cg, 8192), pw);
+            put(reinterpret_cast<uint8_t*>(Eg + (size_t)i * 128), ew);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int b = J + v;                   // target block
+                if (b < 4) {
+                    if (b == 1) put(sm + kFSB + piece_off(i, cg, 4096), src[v]);
+                    else put(sm + kFSA + piece_off((b == 3 ? 0 : (b == 2 ? 64 : 112)) + i, cg, 16384), src[v]);
+                }
+            }
         }
     }
     fence_async_smem();
     tc_fence_before();
-    ok = __syncthreads_and(ok);                        // (5) chain-1 operands complete
-    if (tid == 0 && ok) issue_am(1);
-    ok = mbar_wait(&bar_am[1], 0, p.t.status, 31) && ok;
-    ok = __syncthreads_and(ok);                        // (6) both accumulators complete, stacks dead
+    __syncthreads();                                   // (3) operands complete
+    if (warp < 2 && lane == 0) {
+        // warp 0: targets 3, 2, 0 against the full stack.  warp 1: target 1; its stack has 32 rows, the product's other 96
+        // read the bytes behind them and are never looked at.
+        tc_fence_after();
+        const uint32_t idesc = umma_idesc_bf16(128, warp == 0 ? 96 : 32, kMajorK, kMajorK);
+        const uint32_t a0 = smem_u32(sm + (warp == 0 ? kFSA : kFSB)), b0 = smem_u32(sm + (warp == 0 ? kFXA : kFXB));
+        const uint32_t akb = warp == 0 ? 16384u : 4096u, bkb = warp == 0 ? 12288u : 4096u;
+#pragma unroll
+        for (int k16 = 0; k16 < 8; ++k16)
+            umma_bf16_ss(tmem + warp * 96, umma_smem_desc_sw128(a0 + (k16 >> 2) * akb + (k16 & 3) * 32, 16, 1024),
+                         umma_smem_desc_sw128(b0 + (k16 >> 2) * bkb + (k16 & 3) * 32, 16, 1024), idesc, k16 > 0);
+        umma_commit(&bar_am);
+    }
+    __syncwarp();
+    // in flight: R^T (channel-major: 4 tokens of 8 channels), v's convolution, the next block's inputs
+    {
+        __nv_bfloat16* Rg = p.t.RT + ch * 8192 + (size_t)(8 * cg) * 64 + 4 * rq;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            *reinterpret_cast<uint2*>(Rg + (2 * w) * 64) =
+                make_uint2(__byte_perm(rw[0][w], rw[1][w], 0x5410), __byte_perm(rw[2][w], rw[3][w], 0x5410));
+            *reinterpret_cast<uint2*>(Rg + (2 * w + 1) * 64) =
+                make_uint2(__byte_perm(rw[0][w], rw[1][w], 0x7632), __byte_perm(rw[2][w], rw[3][w], 0x7632));
+        }
+    }
+    uint4 vr[4];
+    if constexpr (CONV) {
+        uint4 xr[7];
+        conv_rows(p.xv, xr);
+        conv4_silu_rows(xr, p.conv.w[2], wbase, p.conv.wf32, vr);
+    }
+    if (warp == 7) {
+        // two blocks to an SM: the one that starts when this one ends is about 296 further on
+        const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + 296u;
+        if (nxt < gridDim.x * gridDim.y) {
+            const int ns = (int)(nxt % gridDim.x), nh = (int)(nxt / gridDim.x);
+            const int nlen = p.chunk_len[ns], nt0 = p.chunk_tok0[ns];
+            if (!CONV && nlen > 0 && lane < 2) tma_prefetch_2d(&mv, nh * 128 + lane * 64, nt0);
+            for (int i = lane; i < nlen; i += 32) {
+                const size_t o = ((size_t)(nt0 + i) * H + nh) * 128;
+#pragma unroll
+                for (int b = 0; b < 128; b += GBF16 ? 64 : 32)
+                    prefetch_l2(GBF16 ? static_cast<const void*>(static_cast<const __nv_bfloat16*>(p.g) + o + b)
+                                      : static_cast<const void*>(static_cast<const float*>(p.g) + o + b));
+                if constexpr (!CONV) {
+                    prefetch_l2(p.q + o);
+                    prefetch_l2(p.q + o + 64);
+                    prefetch_l2(p.k + o);
+                    prefetch_l2(p.k + o + 64);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    bool ok = mbar_wait(&bar_am, 0, p.t.status, 31);
+    ok = __syncthreads_and(ok);                        // (4) both accumulators complete, stacks dead
     tc_fence_after();
     if (ok) {
-        // ---- A^T panel, M~ panel and beta*M~ (fp32) from the two accumulators.  Lane = source row within a 64-row half;
-        // warps 0-3 read chain 0, warps 4-7 chain 1; 32 columns: 16 of A (q targets), 16 of M~ (k targets).
+        if constexpr (CONV) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = 4 * rq + j;
+                *reinterpret_cast<uint4*>(vs + piece_off(i, cg, 8192)) = i < len ? vr[j] : make_uint4(0, 0, 0, 0);
+            }
+        } else if (tid == 0) {
+            mbar_expect_tx(&bar_in, 16384);
+            for (int kb = 0; kb < 2; ++kb) tma_load_2d(vs + kb * 8192, &mv, &bar_in, h * 128 + kb * 64, tok0);
+        }
+        // ---- A^T panel, M~ panel and beta*M~ (fp32): a thread takes one source row s of one target block Ib, 16 columns
+        // of A (q targets) and 16 of M~ (k targets).  Accumulator lanes: block 3 in warps 0, 1, block 2 in warp 2 and half
+        // of warp 3, block 0 in the other half, block 1 in warp 4; warps 5 to 7 fill in the sources behind a target block.
         {
-            const int m = (warp & 3) * 32 + lane;
-            const int half = m >> 6, s = m & 63, pr = warp >> 2;
-            const int Ib = 2 * pr + half;              // target block held in these columns
+            int Ib, s;
             uint32_t t[32];
-            tmem_ld32(tmem + lane_base + pr * 64 + 32 * half, t);
-            tmem_ld_wait();
+            if (warp < 2) { Ib = 3; s = 32 * warp + lane; }
+            else if (warp == 2) { Ib = 2; s = lane; }
+            else if (warp == 3) { Ib = lane < 16 ? 2 : 0; s = lane < 16 ? 32 + lane : lane - 16; }
+            else if (warp == 4) { Ib = 1; s = lane; }
+            else if (warp == 5) { Ib = 1; s = 32 + lane; }
+            else if (warp == 6) { Ib = 0; s = 16 + lane; }
+            else { Ib = lane < 16 ? 0 : 2; s = 48 + (lane & 15); }
+            if (warp < 5) {
+                tmem_ld32(tmem + lane_base + (warp < 2 ? 0 : (warp == 4 ? 96 : 32)), t);
+                if (warp == 3) {
+                    uint32_t u[32];
+                    tmem_ld32(tmem + lane_base + 64, u);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) t[c] = lane < 16 ? t[c] : u[c];
+                }
+                tmem_ld_wait();
+            } else {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) t[c] = 0u;
+            }
             uint32_t at[8];
 #pragma unroll
             for (int c = 0; c < 16; c += 2) {
@@ -732,8 +766,8 @@ __global__ void __launch_bounds__(kNT, 2)
         if (ok) ok = mbar_wait(&bar_uw, 1, p.t.status, 34);      // no block-wide barrier: the staging below overwrites only what
         tc_fence_after();                                         // the completed products were the last to read
         if (ok) {
-            // both results leave through shared memory in the swizzled layout (Pn over the dead T operands and inverse
-            // scratch, Rm^T over the E tile the products have finished reading) and are stored by TMA
+            // both results leave through shared memory in the swizzled layout (Pn over the dead T operands and E tile, Rm^T
+            // over the A^T tile the products have finished reading) and are stored by TMA
             uint8_t* Pst = sm + 32768 + gt * 16384;          // [128 key rows][64 columns of half gt]
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
@@ -756,7 +790,7 @@ __global__ void __launch_bounds__(kNT, 2)
                 for (int c = 0; c < 4; ++c) {
                     float f[8];
                     unpack_bf16x8(rtv[c], f);
-                    *reinterpret_cast<uint4*>(vs + sw128_off(kt, 4 * gt + c)) =
+                    *reinterpret_cast<uint4*>(Qs + sw128_off(kt, 4 * gt + c)) =
                         make_uint4(pack2(f[0] - __uint_as_float(r[8 * c]), f[1] - __uint_as_float(r[8 * c + 1])),
                                    pack2(f[2] - __uint_as_float(r[8 * c + 2]), f[3] - __uint_as_float(r[8 * c + 3])),
                                    pack2(f[4] - __uint_as_float(r[8 * c + 4]), f[5] - __uint_as_float(r[8 * c + 5])),
@@ -768,14 +802,10 @@ __global__ void __launch_bounds__(kNT, 2)
         ok = __syncthreads_and(ok);
         if (tid == 0 && ok) {
             for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mP, sm + 32768 + nb * 16384, nb * 64, (int)(ch * 128));
-            if (!p.t.fwd_only) tma_store_2d(&mRm, vs, 0, (int)(ch * 128));
+            if (!p.t.fwd_only) tma_store_2d(&mRm, Qs, 0, (int)(ch * 128));
             tma_store_commit();
         }
         if (tid == 0) tma_store_wait_read();           // shared memory must outlive the reads of the bulk stores
-    } else {
-        // unwinding: the value tile must have landed before the block may exit
-        if (!CONV) mbar_wait(&bar_in, 0, nullptr, 0);
-        if (tid == 0) tma_store_wait_read();
     }
     tc_fence_before();
     __syncthreads();
