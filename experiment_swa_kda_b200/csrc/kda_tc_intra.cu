@@ -77,9 +77,9 @@ __device__ __forceinline__ void sts8c(float* p, const float (&f)[8]) {
     *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
     *reinterpret_cast<float4*>(p + 64) = make_float4(f[4], f[5], f[6], f[7]);
 }
-__device__ __forceinline__ float fast_rcp(float x) {
+__device__ __forceinline__ float fast_ex2(float x) {
     float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -301,9 +301,8 @@ __global__ void __launch_bounds__(kNT, 2)
     __shared__ uint32_t tmem_slot;
 
     const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
-    const int len = p.chunk_len[slot];
+    const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
     if (len == 0) return;
-    const int tok0 = p.chunk_tok0[slot];
     const size_t ch = (size_t)slot * H + h;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cg = lane & 15;                      // channels 8*cg .. 8*cg+7
@@ -480,16 +479,16 @@ __global__ void __launch_bounds__(kNT, 2)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int w = 2 * hf + e;
-                    const float2 x = f2_get(f2_fma(cj2[e], f2_all(-1.f), f2_make(G[j][2 * w], G[j][2 * w + 1])));
-                    const float t0 = __expf(x.x), t1 = __expf(x.y);        // e^{G - c_J} in (0, 1]
-                    const f2 tq = f2_make(t0, t1);
+                    const f2 dG = f2_fma(cj2[e], f2_all(-1.f), f2_make(G[j][2 * w], G[j][2 * w + 1]));
+                    const float2 x = f2_get(f2_mul(dG, f2_all(1.44269504f)));
+                    const f2 tq = f2_make(fast_ex2(x.x), fast_ex2(x.y));   // e^{G - c_J} in (0, 1]; its reciprocal does not wait for it
                     const f2 q = f2_mul(f2_from_bf16(qw[w]), qi2), k = f2_mul(f2_from_bf16(kw[w]), ki2);
                     xq[w] = f2_to_bf16(f2_mul(q, tq));
                     xk[w] = f2_to_bf16(f2_mul(k, tq));
                     const f2 eg = f2_mul(tq, ec2[e]);                      // e^G
                     pw[w] = f2_to_bf16(f2_mul(f2_mul(b2, eg), k));         // Q = beta e^G k
                     rw[j][w] = f2_to_bf16(f2_mul(q, eg));
-                    f0[e] = f2_mul(k, f2_make(fast_rcp(t0), fast_rcp(t1)));      // source row scaled to its own block
+                    f0[e] = f2_mul(k, f2_make(fast_ex2(-x.x), fast_ex2(-x.y)));  // source row scaled to its own block
                     ew[w] = f2_to_bf16(f2_mul(f0[e], ee2[e]));             // E = k e^{G_end - G}
                     src[0][w] = f2_to_bf16(f0[e]);
                 }

@@ -128,47 +128,36 @@ __global__ void __launch_bounds__(512, 1)
     float* tot = part + 1024;                              // [4][128] block sums of dG
     float* dots = tot + 512;                               // [2][4][64] row dots: q | k, channel quarter, row
     float* rowv = dots + 512;                              // [3][64]  qinv | kinv | beta
-    __shared__ uint64_t bar_in[2], bar_p1, bar_x, bar_q, bar_y, bar_m, bar_pb;
+    __shared__ uint64_t bar_in[2], bar_w, bar_p1, bar_x, bar_q, bar_y, bar_m, bar_pb;
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) float dA_diag[64];      // dA[i][i]: applied to dq, dk in float32, outside the pull-back products
 
     const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
-    const int len = p.chunk_len[slot];
+    const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
     if (len == 0) return;
-    const int tok0 = p.chunk_tok0[slot];
     const int ch = slot * H + h;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int I = warp >> 2;             // row block of this thread
     const int d = tid & 127;             // channel (and TMEM lane) of this thread
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
+    // The first barrier covers what the critical products and the work beside them need.  The loads are issued by warps 1-4,
+    // four each, after their gate loads: one thread issuing all of them held the block back.
     if (tid == 0) {
         mbar_init(&bar_in[0], 1);
         mbar_init(&bar_in[1], 1);
-        mbar_init(&bar_p1, 5);
+        mbar_init(&bar_w, 1);
+        mbar_init(&bar_p1, 4);
         mbar_init(&bar_x, 1);
         mbar_init(&bar_q, 1);
         mbar_init(&bar_y, 1);
         mbar_init(&bar_m, 1);
         mbar_init(&bar_pb, 4);
+        mbar_expect_tx(&bar_in[0], 32768 + 16384 * 4);
+        mbar_expect_tx(&bar_in[1], 32768 + 16384 * 2 + 8192 * 2);
         mbar_fence_init();
-        mbar_expect_tx(&bar_in[0], 32768 + 16384 * 3 + 8192);
-        mbar_expect_tx(&bar_in[1], 32768 + 16384 * 3 + 8192);
-        for (int mb = 0; mb < 2; ++mb) {
-            tma_load_2d(Hs + mb * 16384, &mH, &bar_in[0], mb * 64, ch * 128);
-            tma_load_2d(dOs + mb * 8192, &mdO, &bar_in[0], h * 128 + mb * 64, tok0);
-        }
-        tma_load_2d(dZTs, &mdZT, &bar_in[0], 0, ch * 128);
-        tma_load_2d(ZTs, &mZT, &bar_in[0], 0, ch * 128);
-        tma_load_2d(Ts, &mT, &bar_in[0], 0, ch * 64);
-        for (int mb = 0; mb < 2; ++mb) {
-            tma_load_2d(vs + mb * 8192, &mv, &bar_in[1], h * 128 + mb * 64, tok0);
-            tma_load_2d(dHs + mb * 16384, &mdH, &bar_in[1], mb * 64, ch * 128);
-            tma_load_2d(qs + mb * 8192, &mq, &bar_in[1], h * 128 + mb * 64, tok0);
-            tma_load_2d(ks + mb * 8192, &mk, &bar_in[1], h * 128 + mb * 64, tok0);
-        }
-        tma_load_2d(Mts, &mMt, &bar_in[1], 0, ch * 64);
     }
+    __syncthreads();
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
 
     // ---- per-row scalars and the cumulative log-decay of this thread's 16 rows
@@ -183,6 +172,26 @@ __global__ void __launch_bounds__(512, 1)
     {
 #pragma unroll
         for (int r = 0; r < 16; ++r) G[r] = ld_io(p.g, col + (size_t)min(16 * I + r, len - 1) * rstride, GB);
+        if (lane == 0) {
+            if (warp == 1) {
+                for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_in[0], mb * 64, ch * 128);
+                tma_load_2d(dZTs, &mdZT, &bar_in[0], 0, ch * 128);
+                tma_load_2d(Ts, &mT, &bar_in[1], 0, ch * 64);
+            } else if (warp == 2) {
+                for (int mb = 0; mb < 2; ++mb) {
+                    tma_load_2d(vs + mb * 8192, &mv, &bar_in[0], h * 128 + mb * 64, tok0);
+                    tma_load_2d(dOs + mb * 8192, &mdO, &bar_in[1], h * 128 + mb * 64, tok0);
+                }
+            } else if (warp == 3) {
+                for (int mb = 0; mb < 2; ++mb) tma_load_2d(ks + mb * 8192, &mk, &bar_in[0], h * 128 + mb * 64, tok0);
+                for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_in[1], mb * 64, ch * 128);
+            } else if (warp == 4) {
+                for (int mb = 0; mb < 2; ++mb) tma_load_2d(qs + mb * 8192, &mq, &bar_in[0], h * 128 + mb * 64, tok0);
+                tma_load_2d(ZTs, &mZT, &bar_in[1], 0, ch * 128);
+                tma_load_2d(Mts, &mMt, &bar_in[1], 0, ch * 64);
+            }
+        }
+        __syncwarp();
         float run = 0.f;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
@@ -237,56 +246,23 @@ __global__ void __launch_bounds__(512, 1)
     }
 
     // ================================================================ phase 1: state products
+    // dW and the first half of X are what the next product waits for: they go first.  The others follow from warps that
+    // have finished their share of the work beside them (a thread that issues into a full queue is held until it drains).
     ok = ok && mbar_wait(&bar_in[0], 0, p.status, 40);
-    if (ok && warp < 3 && lane == 0) {
+    if (ok && tid == 0) {
         tc_fence_after();
-        const uint32_t aH = smem_u32(Hs), bdO = smem_u32(dOs), bZ = smem_u32(ZTs), bdZ = smem_u32(dZTs), bT = smem_u32(Ts);
-        if (warp == 0) {
-            const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
-            const uint32_t id_k_mn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
+        const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
+        const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
+        const uint32_t aH = smem_u32(Hs), bdZ = smem_u32(dZTs), aV = smem_u32(vs);
 #pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dW^T = H dZ^T
-                umma_bf16_ss(tmem + cW, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
-                             umma_smem_desc_sw128(bdZ + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
+        for (int k16 = 0; k16 < 8; ++k16)     // dW^T = H dZ^T
+            umma_bf16_ss(tmem + cW, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
+                         umma_smem_desc_sw128(bdZ + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16)     // dP^T = dZ^T T
-                umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(bdZ + k16 * 32, 16, 1024),
-                             umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
-        } else if (warp == 1) {
-            const uint32_t id_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dR^T = H dO^T
-                umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
-                             umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), id_mn_k, k16 > 0);
-        } else {
-            const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dA = dO Z^T                      (M = 64)
-                umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
-        }
-        umma_commit(&bar_p1);
-    }
-    __syncwarp();
-    ok = ok && mbar_wait(&bar_in[1], 0, p.status, 40);
-    if (ok && (warp == 3 || warp == 4) && lane == 0) {
-        tc_fence_after();
-        if (warp == 3) {
-            const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
-            const uint32_t aV = smem_u32(vs), bdZ = smem_u32(dZTs);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // Xraw^T = v dZ^T  (first half)    (M = 64)
-                umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aV + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(bdZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
-        } else {
-            const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
-            const uint32_t adH = smem_u32(dHs), bZ = smem_u32(ZTs);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dE^T = dH' Z^T
-                umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(adH + k16 * 2048, 16384, 1024),
-                             umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
-        }
-        umma_commit(&bar_p1);
+        for (int k16 = 0; k16 < 8; ++k16)     // Xraw^T = v dZ^T  (first half)    (M = 64)
+            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aV + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
+                         umma_smem_desc_sw128(bdZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
+        umma_commit(&bar_w);
     }
     __syncwarp();
     // while the tensor core works: this thread's q and k, the Q' operand, and dD[d] = sum_v dH'[d][v] H[d][v]
@@ -325,6 +301,7 @@ __global__ void __launch_bounds__(512, 1)
         for (int e = 0; e < 8; ++e) w[e] = f2_mul(f2_mul(E[e], eCI), w[e]);
         *reinterpret_cast<uint4*>(Qp + sw128_off(d, 2 * I)) = pack_quad(w, 0);
         *reinterpret_cast<uint4*>(Qp + sw128_off(d, 2 * I + 1)) = pack_quad(w, 4);
+        ok = ok && mbar_wait(&bar_in[1], 0, p.status, 40);
         // two adjacent channels and 16 value rows a thread
         f2 acc = f2_all(0.f);
         const int d2 = 2 * (tid & 63), vg = tid >> 6;
@@ -338,7 +315,38 @@ __global__ void __launch_bounds__(512, 1)
         }
         *reinterpret_cast<float2*>(part + vg * 128 + d2) = f2_get(acc);
     }
-    ok = ok && mbar_wait(&bar_p1, 0, p.status, 41);
+    if (ok && (warp & 3) == 3 && lane == 0) {
+        tc_fence_after();
+        const uint32_t aH = smem_u32(Hs), adH = smem_u32(dHs), bdO = smem_u32(dOs), bZ = smem_u32(ZTs), bdZ = smem_u32(dZTs), bT = smem_u32(Ts);
+        if (warp == 3) {
+            const uint32_t id_k_mn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16)     // dP^T = dZ^T T
+                umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(bdZ + k16 * 32, 16, 1024),
+                             umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
+        } else if (warp == 7) {
+            const uint32_t id_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
+#pragma unroll
+            for (int k16 = 0; k16 < 8; ++k16)     // dR^T = H dO^T
+                umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
+                             umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), id_mn_k, k16 > 0);
+        } else if (warp == 11) {
+            const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
+#pragma unroll
+            for (int k16 = 0; k16 < 8; ++k16)     // dA = dO Z^T                      (M = 64)
+                umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
+                             umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
+        } else {
+            const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
+#pragma unroll
+            for (int k16 = 0; k16 < 8; ++k16)     // dE^T = dH' Z^T
+                umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(adH + k16 * 2048, 16384, 1024),
+                             umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
+        }
+        umma_commit(&bar_p1);
+    }
+    __syncwarp();
+    ok = ok && mbar_wait(&bar_w, 0, p.status, 41);
     tc_fence_after();
 
     // ================================================================ phase 2: X and dQ
@@ -387,6 +395,8 @@ __global__ void __launch_bounds__(512, 1)
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         unit_k(x, w);
     };
+    ok = ok && mbar_wait(&bar_p1, 0, p.status, 41);
+    tc_fence_after();
     f2 dqn[8], dG[8];
     {
         f2 t[8];
