@@ -807,7 +807,7 @@ struct ConvBwdItems {
     void* dx[kConvItems];
 };
 struct ColumnSumItems {
-    float* out[kConvItems];
+    void* out[kConvItems];
 };
 // Entry i of a kernel-parameter array by compile-time indices only: a run-time subscript would make every thread copy the
 // whole array to local memory first.
@@ -1764,12 +1764,12 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, int
     }
 }
 
-// out[i] = sum over b of part[b][i]: 32 columns per block, 32 row segments summed in a fixed order
+// out[i] = sum over b of part[b][i]: 32 columns per block, 32 row segments summed in a fixed order; bf16: rounded on the way out
 __global__ void __launch_bounds__(1024) column_sum_kernel(int nblk, int N, const float* __restrict__ part_all,
-                                                          ColumnSumItems outs) {
+                                                          ColumnSumItems outs, int bf16) {
     __shared__ float red[32][33];
     const float* __restrict__ part = part_all + (size_t)blockIdx.y * nblk * N;     // blockIdx.y = item
-    float* __restrict__ out = pick_item(outs.out, (int)blockIdx.y);
+    void* __restrict__ out = pick_item(outs.out, (int)blockIdx.y);
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     float a = 0.f;
@@ -1781,7 +1781,7 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(int nblk, int N, const
         float t = 0.f;
 #pragma unroll
         for (int r = 0; r < 32; ++r) t += red[r][lane];
-        out[i] = t;
+        st_io(out, i, bf16, t);
     }
 }
 
@@ -2056,7 +2056,7 @@ int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
 
 template <int W>
 int conv_bwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvBwdItems& it, float* const* dwgt,
-                  float* part, cudaStream_t st) {
+                  float* part, cudaStream_t st, int dwb = 0) {
     dim3 grid(ceil_div(C, pw::kConvTileC), ceil_div(T, pw::kConvTileT), B * n);
     // tokens per thread run of the streaming kernel: long runs amortise the W-1 halo rows; below ~12 warps per SM at
     // 32-token runs the tile kernel (64 tokens x 64 channels per block, more and smaller blocks) is the faster one
@@ -2072,7 +2072,7 @@ int conv_bwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
     const int nblk = grid.y * B;                  // partial rows per item
     pw::ColumnSumItems outs = {};
     for (int i = 0; i < n; ++i) outs.out[i] = dwgt[i];
-    KDA_LAUNCH("conv_dw_reduce_kernel", st, pw::column_sum_kernel<<<dim3(ceil_div(C * W, 32), n), 1024, 0, st>>>(nblk, C * W, part, outs));
+    KDA_LAUNCH("conv_dw_reduce_kernel", st, pw::column_sum_kernel<<<dim3(ceil_div(C * W, 32), n), 1024, 0, st>>>(nblk, C * W, part, outs, dwb));
     return launch_status();
 }
 
@@ -2098,7 +2098,7 @@ inline void conv_bwd_grid(int B, int T, int C, int vec, dim3& grid) {
 
 template <int W>
 int conv_bwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x, const void* w, const void* cache, const void* dy,
-               const void* dfin, void* dx, void* dcache, float* dwgt, float* part, cudaStream_t st) {
+               const void* dfin, void* dx, void* dcache, float* dwgt, int dwb, float* part, cudaStream_t st) {
     const bool al16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) % 16) == 0;
     dim3 grid, block(16, 16);
     if constexpr (W <= 4) {
@@ -2107,7 +2107,7 @@ int conv_bwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x,
         if (!cache && !dfin && !dcache && C % 2 == 0 && al16) {
             pw::ConvBwdItems it = {};
             it.x[0] = x; it.w[0] = w; it.dy[0] = dy; it.dx[0] = dx;
-            return conv_bwd_fast<W>(1, B, T, C, C, bf16, wf32, silu, it, &dwgt, part, st);
+            return conv_bwd_fast<W>(1, B, T, C, C, bf16, wf32, silu, it, &dwgt, part, st, dwb);
         }
     }
     // the vector path keeps W*VEC partials per thread in shared memory; wide windows use the scalar path
@@ -2138,7 +2138,7 @@ int conv_bwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x,
     const int nblk = grid.y * grid.z;
     pw::ColumnSumItems outs = {};
     outs.out[0] = dwgt;
-    KDA_LAUNCH("conv_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(C * W, 32), 1024, 0, st>>>(nblk, C * W, part, outs));
+    KDA_LAUNCH("conv_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(C * W, 32), 1024, 0, st>>>(nblk, C * W, part, outs, dwb));
     return launch_status();
 }
 
@@ -2177,7 +2177,7 @@ extern "C" size_t kda_conv_bwd_scratch_bytes(int32_t batch, int32_t seq_len, int
 
 extern "C" int kda_conv_bwd(int32_t batch, int32_t seq_len, int32_t channels, int32_t width, int32_t io_dtype,
                             int32_t silu, const void* x, const void* weight, const void* initial_state, const void* d_y,
-                            const void* d_final_state, void* dx, float* dweight, void* d_initial_state, void* scratch,
+                            const void* d_final_state, void* dx, void* dweight, void* d_initial_state, void* scratch,
                             size_t scratch_bytes, void* stream) {
     if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0) return KDA_ERR_BAD_SHAPE;
     if (!x || !weight || !d_y || !dx || !dweight) return KDA_ERR_NULL;
@@ -2187,7 +2187,7 @@ extern "C" int kda_conv_bwd(int32_t batch, int32_t seq_len, int32_t channels, in
     cudaStream_t st = (cudaStream_t)stream;
 #define CALL(WW)                                                                                                  \
     conv_bwd_w<WW>(batch, seq_len, channels, bf16, wf32, silu, x, weight, initial_state, d_y, d_final_state, dx,  \
-                   d_initial_state, dweight, static_cast<float*>(scratch), st)
+                   d_initial_state, static_cast<float*>(dweight), (io_dtype & KDA_DWEIGHT_BF16) != 0, static_cast<float*>(scratch), st)
     KDA_CONV_SWITCH(CALL)
 #undef CALL
 }
@@ -2380,7 +2380,7 @@ extern "C" int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype,
     }
     pw::ColumnSumItems outs = {};
     outs.out[0] = dweight;
-    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(dim, 32), 1024, 0, st>>>(nb, dim, part, outs));
+    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(dim, 32), 1024, 0, st>>>(nb, dim, part, outs, 0));
     return launch_status();
 }
 
@@ -2400,7 +2400,7 @@ extern "C" int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t
     else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false, true><<<nb, 256, 0, st>>>(rows, heads, gate_ld, x, gate, weight, inv_rms, d_y, dx, dgate, part));
     pw::ColumnSumItems outs = {};
     outs.out[0] = dweight;
-    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<4, 1024, 0, st>>>(nb, 128, part, outs));
+    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<4, 1024, 0, st>>>(nb, 128, part, outs, 0));
     return launch_status();
 }
 

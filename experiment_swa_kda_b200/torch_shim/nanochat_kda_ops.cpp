@@ -31,6 +31,10 @@ namespace {
 
 using namespace kda_host;
 
+// t itself where it is already what the kernels read: a call that does nothing still costs its trip through the dispatcher
+Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+Tensor dense_as(const Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? dense(t) : t.contiguous().to(type); }
+
 void check(int rc, const char* what) {
     TORCH_CHECK(rc == 0, "libkda_b200: ", what, " failed: ", kda_error_string(rc), " (", rc, ")");
 }
@@ -154,21 +158,21 @@ std::tuple<Tensor, OptTensor> chunk_forward(const Tensor& q_, const Tensor& k_, 
     const Dims d = validate_chunk_inputs(q_, k_, v_, raw_gate_, beta_logits_, A_log, dt_bias, initial_state, lower_bound, cu_seqlens);
     c10::cuda::CUDAGuard guard(q_.device());
     watch_status(q_.device().index());
-    const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), raw_gate = raw_gate_.contiguous(),
-                 beta_logits = beta_logits_.contiguous();
+    const Tensor q = dense(q_), k = dense(k_), v = dense(v_), raw_gate = dense(raw_gate_), beta_logits = dense(beta_logits_);
     // A call none of whose inputs takes part in a graph is inference / prefill: nothing is kept for a backward.
     bool needs_grad = false;
     for (const Tensor* t : {&q_, &k_, &v_, &raw_gate_, &beta_logits_, &A_log, &dt_bias}) needs_grad = needs_grad || t->requires_grad();
     if (has(initial_state)) needs_grad = needs_grad || initial_state->requires_grad();
     const KdaChunkShape sh = chunk_shape(d, scale, has(cu_seqlens), !needs_grad);
     const Layout l = layout_for(d, sh);
-    Tensor buf = at::empty({(int64_t)l.total}, q.options().dtype(at::kByte));
+    const Tensor buf = bytes(l.total, q);
     char* base = static_cast<char*>(buf.data_ptr());
-    Tensor output = buf.narrow(0, 0, (int64_t)l.out_bytes).view(at::kBFloat16).view({d.B, d.T, d.H, d.V});
+    Tensor output = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(buf.storage()), buf.key_set(), caffe2::TypeMeta::Make<c10::BFloat16>());
+    output.unsafeGetTensorImpl()->set_sizes_contiguous({d.B, d.T, d.H, d.V});
     float* g = reinterpret_cast<float*>(base + l.g_off);
     float* beta = reinterpret_cast<float*>(base + l.beta_off);
     OptTensor final_state;
-    if (output_final_state) final_state = at::empty({d.N, d.H, d.V, d.K}, q.options().dtype(at::kFloat));
+    if (output_final_state) final_state = empty({d.N, d.H, d.V, d.K}, at::kFloat, q);
     if (d.B * d.T > 0) {
         run_gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound, d, g, beta);
         check(kda_chunk_fwd(&sh, q.data_ptr(), k.data_ptr(), v.data_ptr(), g, beta, static_cast<const float*>(ptr(initial_state)),
@@ -204,8 +208,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
     }
     c10::cuda::CUDAGuard guard(q_.device());
     watch_status(q_.device().index());
-    const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), raw_gate = raw_gate_.contiguous(),
-                 beta_logits = beta_logits_.contiguous();
+    const Tensor q = dense(q_), k = dense(k_), v = dense(v_), raw_gate = dense(raw_gate_), beta_logits = dense(beta_logits_);
     const bool packed = has(cu_seqlens);
     KdaChunkShape sh = chunk_shape(d, scale, packed, false);
     Layout l = layout_for(d, sh);
@@ -222,7 +225,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
             base = static_cast<const char*>(output.data_ptr());
     }
     if (base == nullptr && d.B * d.T > 0) {
-        recomputed = at::empty({(int64_t)l.total}, q.options().dtype(at::kByte));
+        recomputed = bytes(l.total, q);
         char* b = static_cast<char*>(recomputed.data_ptr());
         Tensor scratch_out = recomputed.narrow(0, 0, (int64_t)l.out_bytes);
         run_gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound, d, reinterpret_cast<float*>(b + l.g_off),
@@ -233,22 +236,22 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
               "kda_chunk_fwd (recomputed for the backward)");
         base = b;
     }
-    const Tensor d_o = grad_output.contiguous().to(at::kBFloat16);
+    const Tensor d_o = dense_as(grad_output, at::kBFloat16);
     OptTensor dfs;
-    if (has(grad_final_state)) dfs = grad_final_state->contiguous().to(at::kFloat);
-    Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
-    Tensor dg = at::empty({d.B, d.T, d.H, d.K}, q.options().dtype(at::kFloat)), db = at::empty({d.B, d.T, d.H}, q.options().dtype(at::kFloat));
+    if (has(grad_final_state)) dfs = dense_as(*grad_final_state, at::kFloat);
+    Tensor dq = empty_as(q), dk = empty_as(k), dv = empty_as(v);
+    Tensor dg = empty({d.B, d.T, d.H, d.K}, at::kFloat, q), db = empty({d.B, d.T, d.H}, at::kFloat, q);
     OptTensor dh0;
-    if (has(initial_state)) dh0 = at::empty({d.N, d.H, d.V, d.K}, q.options().dtype(at::kFloat));
-    Tensor d_raw = at::empty_like(raw_gate), d_bl = at::empty_like(beta_logits);
-    Tensor dA = at::empty({d.H}, q.options().dtype(at::kFloat)), dbias = at::empty({d.H * d.K}, q.options().dtype(at::kFloat));
+    if (has(initial_state)) dh0 = empty({d.N, d.H, d.V, d.K}, at::kFloat, q);
+    Tensor d_raw = empty_as(raw_gate), d_bl = empty_as(beta_logits);
+    Tensor dA = empty({d.H}, at::kFloat, q), dbias = empty(dt_bias.sizes(), at::kFloat, q);
     if (d.B * d.T == 0) {
         dA.zero_(); dbias.zero_();
         if (dh0.has_value()) {
             if (dfs.has_value()) dh0->copy_(*dfs);
             else dh0->zero_();
         }
-        return {dq, dk, dv, d_raw, d_bl, dA, dbias.reshape(dt_bias.sizes()), dh0};
+        return {dq, dk, dv, d_raw, d_bl, dA, dbias, dh0};
     }
     Tensor scratch = bytes(kda_chunk_bwd_scratch_bytes(&sh), q);
     check(kda_chunk_bwd(&sh, q.data_ptr(), k.data_ptr(), v.data_ptr(), base + l.g_off, base + l.beta_off,
@@ -262,7 +265,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
                        d_raw.data_ptr(), d_bl.data_ptr(), dA.data_ptr<float>(), dbias.data_ptr<float>(), gscr.data_ptr(),
                        (size_t)gscr.numel(), stream_of(q)),
           "kda_gate_bwd");
-    return {dq, dk, dv, d_raw, d_bl, dA, dbias.reshape(dt_bias.sizes()), dh0};
+    return {dq, dk, dv, d_raw, d_bl, dA, dbias, dh0};
 }
 
 std::tuple<Tensor, OptTensor> recurrent_decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& raw_gate,
@@ -274,9 +277,9 @@ std::tuple<Tensor, OptTensor> recurrent_decode(const Tensor& q, const Tensor& k,
     TORCH_CHECK(q.is_contiguous() && k.is_contiguous() && v.is_contiguous() && raw_gate.is_contiguous() && beta_logits.is_contiguous(),
                 "all recurrent decode inputs must be contiguous");
     c10::cuda::CUDAGuard guard(q.device());
-    Tensor g = at::empty({d.B, 1, d.H, d.K}, q.options().dtype(at::kFloat)), beta = at::empty({d.B, 1, d.H}, q.options().dtype(at::kFloat));
+    Tensor g = empty({d.B, 1, d.H, d.K}, at::kFloat, q), beta = empty({d.B, 1, d.H}, at::kFloat, q);
     Tensor state = has(initial_state) ? *initial_state : at::zeros({d.B, d.H, d.V, d.K}, q.options().dtype(at::kFloat));
-    Tensor new_state = at::empty_like(state), o = at::empty_like(v);
+    Tensor new_state = at::empty_like(state), o = empty_as(v);
     if (d.B > 0) {
         run_gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound, d, g.data_ptr<float>(), beta.data_ptr<float>());
         check(kda_decode_step((int32_t)d.B, (int32_t)d.H, (int32_t)d.K, (int32_t)d.V, KDA_DTYPE_BF16, KDA_DTYPE_F32, 1, (float)scale,
@@ -316,12 +319,12 @@ std::tuple<Tensor, OptTensor> causal_convolution_forward(const Tensor& x, const 
     const ConvDims d = validate_conv(x, weight, initial_state, "initial_state");
     TORCH_CHECK(x.is_contiguous(), "nanochat_kda::causal_convolution_forward requires a contiguous input");
     c10::cuda::CUDAGuard guard(x.device());
-    const Tensor w = weight.contiguous().to(x.scalar_type());
+    const Tensor w = dense_as(weight, x.scalar_type());
     OptTensor s0;
     if (has(initial_state)) s0 = initial_state->contiguous().to(x.scalar_type());
-    Tensor y = at::empty_like(x);
+    Tensor y = empty_as(x);
     OptTensor fin;
-    if (output_final_state) fin = at::empty({d.B, d.C, d.W}, x.options());
+    if (output_final_state) fin = empty({d.B, d.C, d.W}, x.scalar_type(), x);
     if (d.T == 0 || d.B == 0 || d.C == 0) {
         if (fin.has_value()) {
             if (s0.has_value()) fin->copy_(*s0);
@@ -343,30 +346,31 @@ std::tuple<Tensor, Tensor, OptTensor> causal_convolution_backward(const Tensor& 
     TORCH_CHECK(grad_output.sizes() == x_.sizes(), "grad_output must have the shape of x");
     TORCH_CHECK(grad_output.is_cuda() && grad_output.device() == x_.device(), "grad_output must be on the same device as x");
     c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous();
-    const Tensor w = weight.contiguous().to(x.scalar_type());
+    const Tensor x = dense(x_);
+    const Tensor w = dense_as(weight, x.scalar_type());
     OptTensor s0, dfin, dinit;
     if (has(initial_state)) {
         s0 = initial_state->contiguous().to(x.scalar_type());
         dinit = at::empty_like(*s0);
     }
     if (has(grad_final_state)) dfin = grad_final_state->contiguous().to(x.scalar_type());
-    const Tensor dy = grad_output.contiguous().to(x.scalar_type());
-    Tensor dx = at::empty_like(x), dw = at::empty({d.C, d.W}, x.options().dtype(at::kFloat));
+    const Tensor dy = dense_as(grad_output, x.scalar_type());
+    Tensor dx = empty_as(x), dw = empty({d.C, d.W}, weight.scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kFloat, x);
     if (d.T == 0 || d.B == 0 || d.C == 0) {
         dw.zero_();
         if (dinit.has_value()) {
             if (dfin.has_value()) dinit->copy_(*dfin);
             else dinit->zero_();
         }
-        return {dx, dw.to(weight.scalar_type()), dinit};
+        return {dx, dense_as(dw, weight.scalar_type()), dinit};
     }
     Tensor scratch = bytes(kda_conv_bwd_scratch_bytes((int32_t)d.B, (int32_t)d.T, (int32_t)d.C, (int32_t)d.W), x);
-    check(kda_conv_bwd((int32_t)d.B, (int32_t)d.T, (int32_t)d.C, (int32_t)d.W, io_dtype_of(x), 1, x.data_ptr(), w.data_ptr(), ptr(s0),
-                       dy.data_ptr(), ptr(dfin), dx.data_ptr(), dw.data_ptr<float>(), dinit.has_value() ? dinit->data_ptr() : nullptr,
+    const int dw_bf16 = dw.scalar_type() == at::kBFloat16 ? KDA_DWEIGHT_BF16 : 0;
+    check(kda_conv_bwd((int32_t)d.B, (int32_t)d.T, (int32_t)d.C, (int32_t)d.W, io_dtype_of(x) | dw_bf16, 1, x.data_ptr(), w.data_ptr(), ptr(s0),
+                       dy.data_ptr(), ptr(dfin), dx.data_ptr(), dw.data_ptr(), dinit.has_value() ? dinit->data_ptr() : nullptr,
                        scratch.data_ptr(), (size_t)scratch.numel(), stream_of(x)),
           "kda_conv_bwd");
-    return {dx, dw.to(weight.scalar_type()), dinit};
+    return {dx, dense_as(dw, weight.scalar_type()), dinit};
 }
 
 // ------------------------------------------------------------------------------------------------ gated RMSNorm
@@ -384,9 +388,9 @@ int64_t validate_norm(const Tensor& x, const Tensor& gate, const Tensor& weight)
 std::tuple<Tensor, Tensor> rmsnorm_gate_forward(const Tensor& x_, const Tensor& gate_, const Tensor& weight, double epsilon) {
     const int64_t rows = validate_norm(x_, gate_, weight);
     c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous(), gate = gate_.contiguous().to(x_.scalar_type()), w = weight.contiguous().to(at::kFloat);
+    const Tensor x = dense(x_), gate = dense_as(gate_, x_.scalar_type()), w = dense_as(weight, at::kFloat);
     const int64_t D = x.size(-1);
-    Tensor y = at::empty_like(x), inv = at::empty({rows}, x.options().dtype(at::kFloat));
+    Tensor y = empty_as(x), inv = empty({rows}, at::kFloat, x);
     if (rows > 0)
         check(kda_rmsnorm_gate_fwd(rows, (int32_t)D, io_dtype_of(x), (float)epsilon, x.data_ptr(), gate.data_ptr(), w.data_ptr<float>(),
                                    y.data_ptr(), inv.data_ptr<float>(), stream_of(x)),
@@ -403,20 +407,20 @@ std::tuple<Tensor, Tensor, Tensor> rmsnorm_gate_backward(const Tensor& x_, const
     TORCH_CHECK(grad_output.sizes() == x_.sizes(), "grad_output must have the shape of x");
     TORCH_CHECK(grad_output.is_cuda() && grad_output.device() == x_.device(), "grad_output must be on the same device as x");
     c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous(), gate = gate_.contiguous().to(x_.scalar_type()), w = weight.contiguous().to(at::kFloat);
-    const Tensor inv = inverse_rms.contiguous(), dy = grad_output.contiguous().to(x_.scalar_type());
+    const Tensor x = dense(x_), gate = dense_as(gate_, x_.scalar_type()), w = dense_as(weight, at::kFloat);
+    const Tensor inv = dense(inverse_rms), dy = dense_as(grad_output, x_.scalar_type());
     const int64_t D = x.size(-1);
-    Tensor dx = at::empty_like(x), dgate = at::empty_like(gate), dw = at::empty({D}, x.options().dtype(at::kFloat));
+    Tensor dx = empty_as(x), dgate = empty_as(gate), dw = empty({D}, at::kFloat, x);
     if (rows == 0) {
         dw.zero_();
-        return {dx, dgate, dw.to(weight.scalar_type())};
+        return {dx, dgate, dense_as(dw, weight.scalar_type())};
     }
     Tensor scratch = bytes(kda_rmsnorm_gate_bwd_scratch_bytes(rows, (int32_t)D), x);
     check(kda_rmsnorm_gate_bwd(rows, (int32_t)D, io_dtype_of(x), x.data_ptr(), gate.data_ptr(), w.data_ptr<float>(), inv.data_ptr<float>(),
                                dy.data_ptr(), dx.data_ptr(), dgate.data_ptr(), dw.data_ptr<float>(), scratch.data_ptr(),
                                (size_t)scratch.numel(), stream_of(x)),
           "kda_rmsnorm_gate_bwd");
-    return {dx, dgate, dw.to(weight.scalar_type())};
+    return {dx, dgate, dense_as(dw, weight.scalar_type())};
 }
 
 }  // namespace

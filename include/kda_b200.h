@@ -40,6 +40,8 @@ extern "C" {
  * not; each weight is then rounded to the activation dtype as it is loaded (the result a cast of the weight tensor
  * would give) and no converted copy of the weights is needed. */
 #define KDA_WEIGHT_F32 0x100
+/* kda_conv_bwd only: OR this into io_dtype when `dweight` is bfloat16; the float32 sums are rounded as they are written. */
+#define KDA_DWEIGHT_BF16 0x200
 
 #define KDA_LANE_FP32 0 /* CUDA-core float32 arithmetic, any K, V <= 256 */
 #define KDA_LANE_TC 1   /* tcgen05 BF16 tensor-core tiles, float32 accumulation and state */
@@ -273,7 +275,7 @@ int kda_conv_fwd(int32_t batch, int32_t seq_len, int32_t channels, int32_t width
 size_t kda_conv_bwd_scratch_bytes(int32_t batch, int32_t seq_len, int32_t channels, int32_t width);
 int kda_conv_bwd(int32_t batch, int32_t seq_len, int32_t channels, int32_t width, int32_t io_dtype, int32_t silu,
                  const void* x, const void* weight, const void* initial_state, const void* d_y,
-                 const void* d_final_state, void* dx, float* dweight, void* d_initial_state, void* scratch,
+                 const void* d_final_state, void* dx, void* dweight, void* d_initial_state, void* scratch,
                  size_t scratch_bytes, void* stream);
 
 /* n_items (1..4) same-shaped convolutions in ONE launch each way - the q, k and v branches of a layer (the reference
