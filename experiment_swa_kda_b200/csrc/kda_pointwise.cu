@@ -167,7 +167,9 @@ struct RawGate {
 // gate from the low-rank projection, steps the state, and applies the gated RMSNorm to the head's output: three launches
 // of a token become one.  Each part repeats the stand-alone kernel's arithmetic, so both forms give the same bits.  The
 // block then owns all 128 rows of a state: 32 warps hold the whole 64 KB in flight when there are fewer blocks than SMs
-// (4.5 -> 3.4 us at one sequence and 3 heads), eight warps otherwise.
+// (8.5 us at one sequence and 3 heads, latency of the gate's weights and the state), eight warps otherwise.  Bound by the
+// state's bytes with many sequences: eight warps are held to 64 registers, four blocks an SM (256 x 16 states: 96 us, 0.86 of
+// the copy rate; with three blocks 101).
 struct TokenMix {
     const __nv_bfloat16* fa;       // [n_seq][128], rows ld apart
     const void* fb_w;              // [heads*128][128]
@@ -179,7 +181,7 @@ struct TokenMix {
 };
 
 template <int NV4, int R, int NW, bool FUSED>
-__global__ void __launch_bounds__(NW * 32, FUSED && NW == 8 ? 4 : 1) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
+__global__ void __launch_bounds__(NW * 32, NW > 8 ? 1 : (NV4 == 1 ? 4 : 2)) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
                                                      const void* __restrict__ q, const void* __restrict__ k,
                                                      const void* __restrict__ v, const void* __restrict__ g,
                                                      const void* __restrict__ beta, const float* s_in, float* s_out,

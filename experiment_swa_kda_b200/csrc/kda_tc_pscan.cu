@@ -337,16 +337,14 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
 // ---------------------------------------------------------------------------------------------
 struct ScanFixArgs {
     const int* seq_chunk0;
-    const int* chunk_seq;
-    const int* chunk_len;
     const float* seg_fin;      // [rec*units][128][128]
-    __nv_bfloat16* Hp;         // [nch][128][128]: local states in, true states out
     float* s_out;              // final state of the scan, V-first [n_seq][H][128][128], or null
-    int H, nseg, bwd, nslots;
+    int H, nseg, bwd, parts;
     int* status;
 };
 
-constexpr int kFixSmem = 3 * 32768 + 1024;          // S hi | S lo | P
+constexpr int kFixP = 65536, kFixL = 131072;        // S hi | S lo, then two P panels, then two local-state panels
+constexpr int kFixSmem = 196608 + 1024;
 
 // D[tmem] = (A_hi + A_lo) B: A K-major [128 v][128 k] in two bf16 terms, B = P [k][n] MN-major
 __device__ __forceinline__ void issue_hilo_product(uint32_t tmem, const uint8_t* a_hi, const uint8_t* b) {
@@ -362,65 +360,73 @@ __device__ __forceinline__ void issue_hilo_product(uint32_t tmem, const uint8_t*
     }
 }
 
-// Chunk-parallel fix-up of a split scan, one CTA per chunk-head of segments 1 .. nseg-1 (2 CTAs per SM).  The true state
-// at the start of segment k obeys S_1 = final state of segment 0, S_{j+1} = S_j Pfin_j + Lfin_j (final composite and final
-// local state of segment j); every CTA of segment k walks that short chain itself (k - 1 products; the panels sit in L2
-// and all CTAs run side by side, which costs less than a separate launch chaining them once on a handful of SMs), then
-// adds S_k Pp_c to the local state the scan published for its chunk.  S is carried between products as a bf16 hi + lo
-// pair in shared memory (the A operand), so the correction keeps float32-class accuracy.  When the caller wants the scan's
-// final state, one more CTA per (sequence, head) walks the last segment's chain and applies that segment's final maps:
-// the same number of products as a chunk of that segment, so it does not lengthen the launch.
+// Fix-up of a split scan, one CTA per part of a segment k >= 1 (a run of its chunks).  The true state at the start of
+// segment k obeys S_1 = final state of segment 0, S_{j+1} = S_j Pfin_j + Lfin_j (final composite and final local state of
+// segment j).  A CTA walks that short chain itself (k - 1 products), then adds S_k Pp_c to the local state the scan
+// published for each chunk c of its part; the last part of the last segment applies that segment's final maps as well when
+// the caller wants the scan's final state.  S is carried between products as a bf16 hi + lo pair in shared memory (the A
+// operand), so the correction keeps float32-class accuracy.
 // A thread owns one accumulator row (TMEM lane), so nothing it touches in global memory is addressed row-per-thread:
-// the float32 states come thread-major (see the scan kernel), the chunk's bf16 panel comes and goes by TMA through the
-// B-operand buffer, and the final state is transposed through shared memory.
-__global__ void __launch_bounds__(256, 2)
+// the float32 states come thread-major (see the scan kernel), a chunk's bf16 panel comes by TMA into a buffer, is corrected
+// there and leaves from it, and the final state is transposed through shared memory.
+// Bound by the latency of the chain, then by bytes (96 KB a chunk).  One CTA per SM, so that every input has a second
+// buffer: panels for product j + 2 load during j + 1, and the product of chunk c + 1 runs while chunk c is read out.  One
+// CTA per chunk, two to an SM, each walking the chain alone and waiting for its panels in turn, took 66 us at 16 recurrences
+// of 128 chunks and 17.5 us at 6 of 64.
+__global__ void __launch_bounds__(256, 1)
     tc_scan_fixup_kernel(const __grid_constant__ CUtensorMap mPp, const __grid_constant__ CUtensorMap mF,
                          const __grid_constant__ CUtensorMap mHp, ScanFixArgs p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
-    __shared__ uint64_t bar_in, bar_mma;
+    __shared__ uint64_t bar_p[2], bar_l[2], bar_mma[2];
     __shared__ uint32_t tmem_slot;
-    const int h = blockIdx.y, H = p.H, units = 2 * p.nseg - 1;
-    // blocks past the chunk slots (launched only when the caller wants the scan's final state) form that state, one per
-    // sequence: the chain of the last segment plus one product, the same length as a chunk's work in that segment
-    const bool fin = (int)blockIdx.x >= p.nslots;
-    const int slot = fin ? 0 : blockIdx.x;
-    if (!fin && p.chunk_len[slot] == 0) return;
-    const int seq = fin ? (int)blockIdx.x - p.nslots : p.chunk_seq[slot];
-    const int c_begin = p.seq_chunk0[seq], c_end = p.seq_chunk0[seq + 1];
-    const int n_total = c_end - c_begin;         // 0 for an empty sequence: its final state is its initial state, which the
-    int k = p.nseg - 1;                          // chain below reproduces (identity composites, zero local states)
-    if (!fin) {
-        const int step = p.bwd ? c_end - 1 - slot : slot - c_begin;
-        while (k > 0 && step < seg_begin(k, p.nseg, n_total)) --k;
-        if (k == 0) return;                         // segment 0 holds true states already
-    }
-    const int rec = seq * H + h;
-    const int ch = slot * H + h;
-    // products 0 .. k-2 walk the chain S_1 -> S_k; product k-1 is the chunk's own (S_k Pp_c) or, in a final-state block,
-    // S_k Pfin_k
-    const int nprod = k;
+    const int units = 2 * p.nseg - 1, rec = blockIdx.y, seq = rec / p.H, h = rec - seq * p.H;
+    const int k = 1 + (int)blockIdx.x / p.parts, part = (int)blockIdx.x % p.parts;
+    const int c_begin = p.seq_chunk0[seq], c_end = p.seq_chunk0[seq + 1], n_total = c_end - c_begin;
+    const int s0 = seg_begin(k, p.nseg, n_total), sn = seg_begin(k + 1, p.nseg, n_total) - s0;
+    const int b0 = s0 + (int)((long long)part * sn / p.parts), nc = s0 + (int)((long long)(part + 1) * sn / p.parts) - b0;
+    // an empty sequence's final state is its initial state, which the chain reproduces (identity composites, zero local states)
+    const bool fin = p.s_out != nullptr && k == p.nseg - 1 && part == p.parts - 1;
+    if (nc == 0 && !fin) return;
+    // products 0 .. j0-1 walk the chain S_1 -> S_k, j0 .. j0+nc-1 are the chunks' own, the last one the final state's
+    const int j0 = k - 1, np = j0 + nc + (fin ? 1 : 0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = warp >> 2;                        // key half handled by this warpgroup
     const int v = (warp & 3) * 32 + lane;           // value row = TMEM lane;  tid == g * 128 + v
-    uint8_t* Pbuf = sm + 65536;
-    uint32_t inph = 0;                              // completed phases of bar_in (uniform)
-    auto load_panel = [&](const CUtensorMap* map, int row) {
-        mbar_expect_tx(&bar_in, 32768);
-        for (int nb = 0; nb < 2; ++nb) tma_load_2d(Pbuf + nb * 16384, map, &bar_in, nb * 64, row);
+    auto chunk_row = [&](int j) {                   // panel row of chunk product j
+        const int step = b0 + j - j0;
+        return ((p.bwd ? c_end - 1 - step : c_begin + step) * p.H + h) * 128;
     };
-    auto load_p = [&](int t) {                      // B operand of product t
-        if (t == k - 1 && !fin) load_panel(&mPp, ch * 128);
-        else load_panel(&mF, (rec * units + 2 * (t + 1)) * 128);
+    auto is_chunk = [&](int j) { return j >= j0 && j < j0 + nc; };
+    // loads, by thread 0: phase j >> 1 of stage j & 1 for the P panels, phase (j - j0) >> 1 for the local states
+    int p_end = 0, l_end = j0;                      // loads issued so far (products below these)
+    auto load_p = [&]() {
+        if (p_end >= np) return;
+        const int j = p_end++;
+        uint8_t* dst = sm + kFixP + (j & 1) * 32768;
+        mbar_expect_tx(&bar_p[j & 1], 32768);
+        for (int nb = 0; nb < 2; ++nb)
+            tma_load_2d(dst + nb * 16384, is_chunk(j) ? &mPp : &mF, &bar_p[j & 1], nb * 64,
+                        is_chunk(j) ? chunk_row(j) : (rec * units + 2 * (j < j0 ? j + 1 : k)) * 128);
+    };
+    auto load_l = [&]() {
+        if (l_end >= j0 + nc) return;
+        const int j = l_end++;
+        uint8_t* dst = sm + kFixL + (j & 1) * 32768;
+        mbar_expect_tx(&bar_l[j & 1], 32768);
+        for (int nb = 0; nb < 2; ++nb) tma_load_2d(dst + nb * 16384, &mHp, &bar_l[j & 1], nb * 64, chunk_row(j));
     };
     if (tid == 0) {
-        mbar_init(&bar_in, 1);
-        mbar_init(&bar_mma, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&bar_p[s], 1);
+            mbar_init(&bar_l[s], 1);
+            mbar_init(&bar_mma[s], 1);
+        }
         mbar_fence_init();
-        if (k == 1 && !fin) load_panel(&mHp, ch * 128);     // the first product is the chunk's own: its local state comes first
-        else load_p(0);
+        load_p(); load_p();
+        load_l(); load_l();
     }
-    if (warp == 1) tmem_alloc(&tmem_slot, 128);
+    if (warp == 1) tmem_alloc(&tmem_slot, 256);
     auto split_store = [&](const float (&x)[32], int b) {      // 32 keys starting at 64 g + 32 b -> hi / lo operand panels
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -444,12 +450,12 @@ __global__ void __launch_bounds__(256, 2)
             x[4 * c] = a.x; x[4 * c + 1] = a.y; x[4 * c + 2] = a.z; x[4 * c + 3] = a.w;
         }
     };
-    // S_1 = final state of segment 0
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-        float x[32];
-        load_f32(p.seg_fin + (size_t)rec * units * 16384, x, b);
-        split_store(x, b);
+    {   // S_1 = final state of segment 0
+        float x[2][32];
+        load_f32(p.seg_fin + (size_t)rec * units * 16384, x[0], 0);
+        load_f32(p.seg_fin + (size_t)rec * units * 16384, x[1], 1);
+        split_store(x[0], 0);
+        split_store(x[1], 1);
     }
     fence_async_smem();
     tc_fence_before();
@@ -458,96 +464,115 @@ __global__ void __launch_bounds__(256, 2)
     const uint32_t tmem = tmem_slot;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     bool ok = true;
-    for (int t = 0; t < nprod && ok; ++t) {
-        const bool own = t == k - 1 && !fin;
-        const bool final_state = t == k - 1 && fin;
-        float add[2][32];                           // what is added to the product
-        if (own) {
-            // the chunk's local state sits in the B-operand buffer (TMA): take this thread's row, then make room for P
-            ok = mbar_wait(&bar_in, inph & 1, p.status, 82);
-            ++inph;
-            if (ok) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    float l[8];
-                    unpack_bf16x8(*reinterpret_cast<const uint4*>(Pbuf + g * 16384 + sw128_off(v, c)), l);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) add[c >> 2][8 * (c & 3) + e] = l[e];
+    int issued = 0;
+    for (int j = 0; j < np && ok; ++j) {
+        const int st = j & 1;
+        const bool own = is_chunk(j);
+        if (tid == 0) {
+            // this product and, when it leaves S alone, the next: its accumulator was read out an iteration ago
+            while (ok && issued < np && (issued <= j || (issued == j + 1 && j >= j0))) {
+                ok = mbar_wait(&bar_p[issued & 1], (issued >> 1) & 1, p.status, 80);
+                if (ok) {
+                    tc_fence_after();
+                    issue_hilo_product(tmem + 128 * (issued & 1), sm, sm + kFixP + (issued & 1) * 32768);
+                    umma_commit(&bar_mma[issued & 1]);
+                    ++issued;
                 }
             }
-            fence_async_smem();
-            ok = __syncthreads_and(ok);
-            if (ok && tid == 0) load_p(t);
-        } else {
-            // the final local state of the segment this chain step crosses (float32, thread-major): flies during the product
-            const float* L = p.seg_fin + (size_t)(rec * units + 2 * (t + 1) - 1) * 16384;
+        }
+        __syncwarp();
+        float add[2][32];                           // what is added to the product
+        if (!own) {
+            // the final local state of the segment this step crosses (float32, thread-major): flies during the product
+            const float* L = p.seg_fin + (size_t)(rec * units + 2 * (j < j0 ? j + 1 : k) - 1) * 16384;
             load_f32(L, add[0], 0);
             load_f32(L, add[1], 1);
+        } else {
+            ok = mbar_wait(&bar_l[st], ((j - j0) >> 1) & 1, p.status, 82) && ok;
         }
+        ok = mbar_wait(&bar_mma[st], (j >> 1) & 1, p.status, 81) && ok;
+        tc_fence_after();
         if (tid == 0 && ok) {
-            ok = mbar_wait(&bar_in, inph & 1, p.status, 80);
-            if (ok) {
-                tc_fence_after();
-                issue_hilo_product(tmem, sm, Pbuf);
-                umma_commit(&bar_mma);
+            load_p();                               // product j + 2 into the panel this one has read
+            if (j > j0) {
+                tma_store_wait_read();              // chunk j - 1 has left its buffer: chunk j + 1 into it
+                load_l();
             }
         }
-        ++inph;
-        if (ok) ok = mbar_wait(&bar_mma, (uint32_t)t & 1, p.status, 81);
-        ok = __syncthreads_and(ok);                 // the product has read both operand buffers
-        tc_fence_after();
-        if (ok && tid == 0 && t + 1 < nprod) {      // next panel into the free buffer while this result is read out
-            if (t + 1 == k - 1 && !fin) load_panel(&mHp, ch * 128);
-            else load_p(t + 1);
-        }
-        if (ok) {
+        if (own) {
+            // the chunk's true state, in place in its buffer
+            uint8_t* Lb = sm + kFixL + st * 32768 + g * 16384;
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 uint32_t r[32];
-                tmem_ld32(tmem + lane_base + 64 * g + 32 * b, r);
+                tmem_ld32(tmem + lane_base + 128 * st + 64 * g + 32 * b, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint4* at = reinterpret_cast<uint4*>(Lb + sw128_off(v, 4 * b + c));
+                    const uint4 l = *at;
+                    const uint32_t lw[4] = {l.x, l.y, l.z, l.w};
+                    uint32_t w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        w[e] = f2_to_bf16(f2_add(f2_make(__uint_as_float(r[8 * c + 2 * e]), __uint_as_float(r[8 * c + 2 * e + 1])), f2_from_bf16(lw[e])));
+                    *at = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+        } else {
+            const bool final_state = j >= j0;
+            if (final_state) {                      // the rows go through the panel buffers: their stores must have read them
+                if (tid == 0) tma_store_wait_read();
+                ok = __syncthreads_and(ok);
+            }
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                uint32_t r[32];
+                tmem_ld32(tmem + lane_base + 128 * st + 64 * g + 32 * b, r);
                 tmem_ld_wait();
                 float x[32];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]) + add[b][j];
-                if (own) {                          // the chunk's true state -> B-operand buffer -> TMA store; S_k stays put
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        *reinterpret_cast<uint4*>(Pbuf + g * 16384 + sw128_off(v, 4 * b + c)) =
-                            make_uint4(pack_bf16(x[8 * c], x[8 * c + 1]), pack_bf16(x[8 * c + 2], x[8 * c + 3]),
-                                       pack_bf16(x[8 * c + 4], x[8 * c + 5]), pack_bf16(x[8 * c + 6], x[8 * c + 7]));
-                } else if (final_state) {
-                    // the scan's final state, row-major for the caller: rows through the dead operand panels (16-byte
-                    // pieces XOR-swizzled by row so that the stores spread over the banks), written out below
+                for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(r[i]) + add[b][i];
+                if (final_state) {
+                    // row-major for the caller (16-byte pieces XOR-swizzled by row so that the stores spread over the
+                    // banks), written out below
 #pragma unroll
                     for (int c = 0; c < 8; ++c)
-                        *reinterpret_cast<float4*>(sm + v * 512 + (((16 * g + 8 * b + c) ^ (v & 7)) << 4)) =
+                        *reinterpret_cast<float4*>(sm + kFixL + v * 512 + (((16 * g + 8 * b + c) ^ (v & 7)) << 4)) =
                             make_float4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
                 } else {
-                    split_store(x, b);              // S_{t+2}: the next product's A operand
+                    split_store(x, b);              // S_{j+2}: the next product's A operand
                 }
             }
         }
         fence_async_smem();
         tc_fence_before();
-        __syncthreads();                            // operand panels rewritten, accumulator read: next product may go
+        ok = __syncthreads_and(ok);                 // operands rewritten, accumulator read
         tc_fence_after();
         if (ok && own && tid == 0) {
-            for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mHp, Pbuf + nb * 16384, nb * 64, ch * 128);
+            for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mHp, sm + kFixL + st * 32768 + nb * 16384, nb * 64, chunk_row(j));
             tma_store_commit();
         }
-        if (ok && final_state) {
+        if (ok && !own && j >= j0) {
             float4* dst = reinterpret_cast<float4*>(p.s_out + (size_t)rec * 16384);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int f = i * 256 + tid, row = f >> 5, c16 = f & 31;       // float4 f of the row-major 128 x 128 tile
-                dst[f] = *reinterpret_cast<const float4*>(sm + row * 512 + ((c16 ^ (row & 7)) << 4));
+                dst[f] = *reinterpret_cast<const float4*>(sm + kFixL + row * 512 + ((c16 ^ (row & 7)) << 4));
             }
         }
     }
-    if (tid == 0) tma_store_wait_read();            // shared memory must outlive the reads of the bulk store
+    if (tid == 0) {
+        if (!ok) {      // unwinding: copies and products in flight must end before the block may exit
+            for (int j = p_end > 2 ? p_end - 2 : 0; j < p_end; ++j) mbar_wait(&bar_p[j & 1], (j >> 1) & 1, nullptr, 0);
+            for (int j = l_end > j0 + 2 ? l_end - 2 : j0; j < l_end; ++j) mbar_wait(&bar_l[j & 1], ((j - j0) >> 1) & 1, nullptr, 0);
+            for (int j = issued > 2 ? issued - 2 : 0; j < issued; ++j) mbar_wait(&bar_mma[j & 1], (j >> 1) & 1, nullptr, 0);
+        }
+        tma_store_wait_read();            // shared memory must outlive the reads of the bulk store
+    }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, 128);
+    if (warp == 1) tmem_dealloc(tmem, 256);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -847,12 +872,15 @@ static int scan_fixup(const simt::Ws& w, const tc::TcWs& t, int n_seq, __nv_bflo
     using namespace tc;
     if (set_smem_limit(tc_scan_fixup_kernel, kFixSmem))
         return KDA_ERR_CUDA;
+    // one CTA per SM: as many parts to a segment as fill the GPU once, none of them without a chunk
+    const int rec = n_seq * w.H, per_seg = (w.nslots / n_seq + t.nseg - 1) / t.nseg;
+    const int parts = std::max(1, std::min(148 / (rec * (t.nseg - 1)), per_seg));
     ScanFixArgs f;
-    f.seq_chunk0 = w.seq_chunk0; f.chunk_seq = w.chunk_seq; f.chunk_len = w.chunk_len; f.seg_fin = t.seg_fin;
-    f.Hp = panels; f.s_out = s_out; f.H = w.H; f.nseg = t.nseg; f.bwd = bwd; f.nslots = w.nslots; f.status = t.status;
+    f.seq_chunk0 = w.seq_chunk0; f.seg_fin = t.seg_fin; f.s_out = s_out; f.H = w.H; f.nseg = t.nseg; f.bwd = bwd; f.parts = parts;
+    f.status = t.status;
     CUtensorMap mHp;
     if (make_map_bf16(&mHp, panels, (uint64_t)w.nslots * w.H * 128, 128, 64, 128)) return KDA_ERR_CUDA;
-    KDA_LAUNCH("tc_scan_fixup_kernel", st, tc_scan_fixup_kernel<<<dim3(w.nslots + (s_out != nullptr ? n_seq : 0), w.H), 256, kFixSmem, st>>>(mPp, mF, mHp, f));
+    KDA_LAUNCH("tc_scan_fixup_kernel", st, tc_scan_fixup_kernel<<<dim3(parts * (t.nseg - 1), rec), 256, kFixSmem, st>>>(mPp, mF, mHp, f));
     return launch_status();
 }
 
