@@ -160,13 +160,11 @@ __device__ __forceinline__ void warp_mm(PA pa, PB pb, PD pd, float alpha) {
     *reinterpret_cast<float2*>(D + 8 * LD) = make_float2(alpha * d[2], alpha * d[3]);
 }
 
-// Ts = (I + Ms)^-1 for strictly lower-triangular Ms (64x64): 8x8 diagonal solves (a short dependent chain per thread),
+// Ts = (I + Ms)^-1 for strictly lower-triangular Ms (64x64), Ts zero on entry: 8x8 diagonal solves (a short dependent chain per thread),
 // then merges to 16 (CUDA cores), 32 and 64 (warp-level tensor cores) with
 //   inv([[A,0],[C,B]]) = [[Ai,0],[-Bi C Ai, Bi]].
 __device__ __forceinline__ void unit_lower_inverse(const float* Ms, float* Ts, float* tmp) {
     const int tid = threadIdx.x;
-    for (int idx = tid; idx < 64 * kLDs / 4; idx += kNT) reinterpret_cast<float4*>(Ts)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
     if (tid < 64) {
         const int b = tid >> 3, j = tid & 7;          // diagonal block, column of the inverse
         const float* Lb = Ms + (8 * b) * kLDs + 8 * b;
@@ -300,10 +298,11 @@ __global__ void __launch_bounds__(kNT, 2)
     __shared__ uint64_t bar_in, bar_am, bar_uw, bar_tr;
     __shared__ uint32_t tmem_slot;
 
-    const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
+    // heads fastest: blocks that run side by side read neighbouring pieces of the same token rows
+    const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;
     const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
     if (len == 0) return;
-    const size_t ch = (size_t)slot * H + h;
+    const size_t ch = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cg = lane & 15;                      // channels 8*cg .. 8*cg+7
     const int rq = 2 * warp + (lane >> 4);         // rows 4*rq .. 4*rq+3
@@ -555,9 +554,9 @@ __global__ void __launch_bounds__(kNT, 2)
     }
     if (warp == 7) {
         // two blocks to an SM: the one that starts when this one ends is about 296 further on
-        const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + 296u;
-        if (nxt < gridDim.x * gridDim.y) {
-            const int ns = (int)(nxt % gridDim.x), nh = (int)(nxt / gridDim.x);
+        const unsigned nxt = blockIdx.x + 296u;
+        if (nxt < gridDim.x) {
+            const int ns = (int)(nxt / H), nh = (int)(nxt % H);
             const int nlen = p.chunk_len[ns], nt0 = p.chunk_tok0[ns];
             if (!CONV && nlen > 0 && lane < 2) tma_prefetch_2d(&mv, nh * 128 + lane * 64, nt0);
             for (int i = lane; i < nlen; i += 32) {
@@ -637,6 +636,7 @@ __global__ void __launch_bounds__(kNT, 2)
                 *reinterpret_cast<__nv_bfloat16*>(Mts + sw128_off(tt, s >> 3) + (s & 7) * 2) = __float2bfloat16(mt);
             }
         }
+        for (int idx = tid; idx < 64 * kLDs / 4; idx += kNT) reinterpret_cast<float4*>(Ts)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
@@ -675,7 +675,6 @@ __global__ void __launch_bounds__(kNT, 2)
             }
         }
         fence_async_smem();
-        // the E rows this block wrote with plain stores long ago come back by a bulk load below: order them for it
         __threadfence();
         asm volatile("fence.proxy.async.global;" ::: "memory");
         tc_fence_before();
@@ -838,7 +837,7 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
     auto kern = conv != nullptr ? (gbf16 ? tc_intra_fwd_kernel<true, true> : tc_intra_fwd_kernel<false, true>)
                                 : (gbf16 ? tc_intra_fwd_kernel<true, false> : tc_intra_fwd_kernel<false, false>);
     if (set_smem_limit(kern, kIntraFwdSmem)) return KDA_ERR_CUDA;
-    KDA_LAUNCH("tc_intra_fwd_kernel", st, kern<<<dim3(w.nslots, w.H), kNT, kIntraFwdSmem, st>>>(mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp, a));
+    KDA_LAUNCH("tc_intra_fwd_kernel", st, kern<<<(unsigned)nch, kNT, kIntraFwdSmem, st>>>(mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp, a));
     return launch_status();
 }
 

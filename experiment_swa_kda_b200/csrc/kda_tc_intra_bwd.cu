@@ -763,6 +763,13 @@ __global__ void __launch_bounds__(512, 1)
         dots[(lane & 1) * 256 + (warp & 3) * 64 + 16 * I + (lane >> 1)] = vals[0];
     }
     __syncthreads();
+    if (p.l2norm) {
+        if (tid < 128) {      // the four quadrants of the channels -> one number, in place
+            float* q4 = dots + (tid >> 6) * 256 + (tid & 63);
+            q4[0] = (q4[0] + q4[64]) + (q4[128] + q4[192]);
+        }
+        __syncthreads();
+    }
     {
         float run = gsum[d] + gsum[128 + d] + gsum[256 + d] + gsum[384 + d];
         {
@@ -785,12 +792,7 @@ __global__ void __launch_bounds__(512, 1)
             const int i = 16 * I + 2 * e;
             f2 dqv = f2_mul(dqn[e], f2_all(p.scale)), dkv = dkn[e];
             if (p.l2norm) {
-                f2 pq = ld_2(dots + i), pk = ld_2(dots + 256 + i);
-#pragma unroll
-                for (int w = 1; w < 4; ++w) {          // the four quadrants of the channels
-                    pq = f2_add(pq, ld_2(dots + 64 * w + i));
-                    pk = f2_add(pk, ld_2(dots + 256 + 64 * w + i));
-                }
+                const f2 pq = ld_2(dots + i), pk = ld_2(dots + 256 + i);
                 dqv = f2_mul(ld_2(rowv + i), f2_fma(f2_mul(qn[e], f2_all(-inv_scale)), pq, dqv));
                 dkv = f2_mul(ld_2(rowv + 64 + i), f2_fma(neg_2(kn[e]), pk, dkv));
             }

@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(256, 2)
     __nv_bfloat16* Ot = reinterpret_cast<__nv_bfloat16*>(sm + kOutO);   // [64 tokens][128 values]
     __shared__ uint64_t bar_in, bar_mma1, bar_mma2;
     __shared__ uint32_t tmem_slot;
-    const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
+    const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;      // heads fastest, as in the intra-chunk kernels
     const int len = p.chunk_len[slot];
     if (len == 0) return;
     const int tok0 = p.chunk_tok0[slot];
@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(256, 3)
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
     __shared__ uint64_t bar_in, bar_mma;
     __shared__ uint32_t tmem_slot;
-    const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
+    const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;      // heads fastest, as in the intra-chunk kernels
     const int len = p.chunk_len[slot];
     if (len == 0) return;
     const int tok0 = p.chunk_tok0[slot];
@@ -930,7 +930,7 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
     oa.status = t.status;
     oa.norm = norm;
     KDA_LAUNCH("tc_chunk_out_kernel", st,
-               tc_chunk_out_kernel<<<dim3(w.nslots, w.H), 256, out_smem, st>>>(mH, mW, mR, mUT, mAT, mG, mZT, oa));
+               tc_chunk_out_kernel<<<(unsigned)nch, 256, out_smem, st>>>(mH, mW, mR, mUT, mAT, mG, mZT, oa));
     return launch_status();
 }
 
@@ -974,7 +974,7 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
     ChunkDzArgs da;
     da.chunk_tok0 = w.chunk_tok0; da.chunk_len = w.chunk_len; da.dZT = t.dZT; da.H = w.H; da.status = t.status;
     KDA_LAUNCH("tc_chunk_dz_kernel", st,
-               tc_chunk_dz_kernel<<<dim3(w.nslots, w.H), 256, kChunkDzSmem, st>>>(mdH, mE, mdO, mAT, mdZT, da));
+               tc_chunk_dz_kernel<<<(unsigned)nch, 256, kChunkDzSmem, st>>>(mdH, mE, mdO, mAT, mdZT, da));
     return launch_status();
 }
 
