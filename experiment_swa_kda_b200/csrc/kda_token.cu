@@ -29,7 +29,7 @@ struct RowsArgs {
     const void* conv_w[3];         // [channels][width]
     void* cache[3];                // [m][channels][width] bf16, shifted in place
     __nv_bfloat16* act;            // [3][m][channels]
-    int width, conv_wf32;
+    int width, conv_wf32, conv_vec;      // conv_vec: width 4, windows and weights aligned for one access each
 };
 
 __device__ __forceinline__ uint32_t pk(float a, float b) {
@@ -117,6 +117,32 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
 #pragma unroll
     for (int i = 0; i < D - 1; ++i) issue(i);
     load_x(0);
+    // A thread's outputs all belong to one weight row (ROWS divides the block), so its convolution windows and weights can
+    // come in now, behind the product, instead of one after another at the end (32 tokens, 16 heads: 24.0 -> 21 us).
+    constexpr int NOUT = (ROWS * NT * 8 + NTH - 1) / NTH;
+    const int orow = row0 + threadIdx.x % ROWS;
+    const bool early = CONV && p.conv_vec && orow < p.end[2];
+    const int citem = orow < p.end[0] ? 0 : (orow < p.end[1] ? 1 : 2), cc = orow - citem * p.end[0];      // the three have the same channels
+    uint2* const win_at = CONV ? static_cast<uint2*>(citem == 0 ? p.cache[0] : (citem == 1 ? p.cache[1] : p.cache[2])) : nullptr;
+    const void* const cw = citem == 0 ? p.conv_w[0] : (citem == 1 ? p.conv_w[1] : p.conv_w[2]);
+    uint2 win[CONV ? NOUT : 1];
+    float cwt[4];
+    if (early) {
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) {
+            const int m = (threadIdx.x + o * NTH) / ROWS;
+            if (m < p.m) win[o] = win_at[(size_t)m * p.end[0] + cc];
+        }
+        if (p.conv_wf32) {
+            const float4 u = __ldg(static_cast<const float4*>(cw) + cc);
+            cwt[0] = __bfloat162float(__float2bfloat16(u.x)); cwt[1] = __bfloat162float(__float2bfloat16(u.y));
+            cwt[2] = __bfloat162float(__float2bfloat16(u.z)); cwt[3] = __bfloat162float(__float2bfloat16(u.w));
+        } else {
+            const uint2 u = __ldg(static_cast<const uint2*>(cw) + cc);
+            cwt[0] = __uint_as_float(u.x << 16); cwt[1] = __uint_as_float(u.x & 0xffff0000u);
+            cwt[2] = __uint_as_float(u.y << 16); cwt[3] = __uint_as_float(u.y & 0xffff0000u);
+        }
+    }
 #pragma unroll 1
     for (int i = 0; i < mine; ++i) {
         issue(i + D - 1);
@@ -160,35 +186,45 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
             d[8 * LD + 1] = acc[r][t][3];
         }
     __syncthreads();
-    for (int i = threadIdx.x; i < ROWS * p.m; i += NTH) {
-        const int r = i % ROWS, m = i / ROWS, row = row0 + r;
-        if (row >= p.end[p.n_items - 1]) continue;
+    if (orow >= p.end[p.n_items - 1]) return;
+#pragma unroll
+    for (int o = 0; o < NOUT; ++o) {
+        const int m = (threadIdx.x + o * NTH) / ROWS;
+        if (m >= p.m) break;
         float y = 0.f;
 #pragma unroll
-        for (int k = 0; k < kWarps; ++k) y += red[(size_t)(k * ROWS + r) * LD + m];
+        for (int k = 0; k < kWarps; ++k) y += red[(size_t)(k * ROWS + threadIdx.x % ROWS) * LD + m];
         const __nv_bfloat16 yb = __float2bfloat16(y);
-        if (CONV && row < p.end[2]) {
+        if (CONV && orow < p.end[2]) {
             // one token of the short convolution + SiLU, the arithmetic of the stand-alone step: the window drops its oldest
             // value and takes y; the cache is rewritten in place
-            const int item = row < p.end[0] ? 0 : (row < p.end[1] ? 1 : 2);
-            void* cache = item == 0 ? p.cache[0] : (item == 1 ? p.cache[1] : p.cache[2]);
-            const void* cw = item == 0 ? p.conv_w[0] : (item == 1 ? p.conv_w[1] : p.conv_w[2]);
-            const int C = p.end[0], c = row - item * C;      // the three have the same channels
-            const size_t base = ((size_t)m * C + c) * p.width;
+            const int C = p.end[0];
             float z = 0.f;
-            for (int j = 0; j < p.width; ++j) {
-                const float v = j + 1 < p.width ? ld_io(cache, base + j + 1, 1) : __bfloat162float(yb);
-                float wj;
-                if (p.conv_wf32) wj = __bfloat162float(__float2bfloat16(static_cast<const float*>(cw)[(size_t)c * p.width + j]));
-                else wj = ld_io(cw, (size_t)c * p.width + j, 1);
-                z += wj * v;
-                st_io(cache, base + j, 1, v);
+            if (early) {
+                const uint32_t yw = (uint32_t)*reinterpret_cast<const uint16_t*>(&yb) << 16;
+                const uint2 next = make_uint2((win[o].x >> 16) | (win[o].y << 16), (win[o].y >> 16) | yw);
+                z += cwt[0] * __uint_as_float(next.x << 16);
+                z += cwt[1] * __uint_as_float(next.x & 0xffff0000u);
+                z += cwt[2] * __uint_as_float(next.y << 16);
+                z += cwt[3] * __uint_as_float(yw);
+                win_at[(size_t)m * C + cc] = next;
+            } else {
+                void* cache = win_at;
+                const size_t base = ((size_t)m * C + cc) * p.width;
+                for (int j = 0; j < p.width; ++j) {
+                    const float v = j + 1 < p.width ? ld_io(cache, base + j + 1, 1) : __bfloat162float(yb);
+                    float wj;
+                    if (p.conv_wf32) wj = __bfloat162float(__float2bfloat16(static_cast<const float*>(cw)[(size_t)cc * p.width + j]));
+                    else wj = ld_io(cw, (size_t)cc * p.width + j, 1);
+                    z += wj * v;
+                    st_io(cache, base + j, 1, v);
+                }
             }
             float th;
             asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(0.5f * z));
-            p.act[((size_t)item * p.m + m) * C + c] = __float2bfloat16(z * fmaf(0.5f, th, 0.5f));
+            p.act[((size_t)citem * p.m + m) * C + cc] = __float2bfloat16(z * fmaf(0.5f, th, 0.5f));
         } else {
-            p.out[(size_t)m * p.ldo + row] = yb;
+            p.out[(size_t)m * p.ldo + orow] = yb;
         }
     }
 }
@@ -265,6 +301,12 @@ extern "C" int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t we
     p.act = static_cast<__nv_bfloat16*>(conv->act);
     p.width = conv->width;
     p.conv_wf32 = conv->weight_dtype == KDA_DTYPE_F32;
+    uintptr_t cal = 0, wal = 0;
+    for (int i = 0; i < 3; ++i) {
+        cal |= reinterpret_cast<uintptr_t>(conv->cache[i]);
+        wal |= reinterpret_cast<uintptr_t>(conv->weight[i]);
+    }
+    p.conv_vec = conv->width == 4 && cal % 8 == 0 && wal % 16 == 0;
     return f32 ? tok::launch_rows<true, true>(p, st) : tok::launch_rows<false, true>(p, st);
 }
 

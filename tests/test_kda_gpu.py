@@ -109,6 +109,31 @@ def test_strong_decay_fp32():
     run_case(1, 130, 2, 64, 64, dtype=torch.float32, seed=7, tol=FP32_TOL, gate_scale=40.0)
 
 
+@pytest.mark.parametrize("K,V,T", [(32, 16, 65), (64, 64, 130), (128, 72, 63), (8, 256, 70)])
+def test_decay_past_the_factored_range_fp32(K, V, T):
+    """About -12 a token in every other channel: the decay over 8 rows leaves e^80, so products of factored exponentials
+    would overflow and the float32 lane takes its pairwise branch.  Both sides evaluate e^(G_t - G_s) in float32 from sums of
+    up to 64 gates, |G| <= 800: an exponent is off by at most |G| 2^-24 = 5e-5, so 1e-4 relative.  The other channels decay
+    slowly: the gate gradient of a fast channel is what e^-12 leaves of the difference of O(1) terms, and float32 holds none
+    of its digits (2^-24 / e^-12 = 1e-2 of it a term), so a norm over fast channels alone would measure rounding only."""
+    d = O.make_inputs(1, T, 2, K, V, seed=K + T, with_state=True)
+    d["g"][..., ::2] = -12.0 - torch.rand(d["g"][..., ::2].shape, generator=torch.Generator().manual_seed(T))
+    d["g"][..., 1::2] *= 0.1
+    m = kda_mod()
+    x = to_dev(d)
+    for n in x:
+        x[n].requires_grad_(True)
+    o, s = m.chunk_kda(x["q"], x["k"], x["v"], x["g"], x["beta"], initial_state=x["h0"], output_final_state=True, lane="fp32")
+    gen = torch.Generator().manual_seed(K)
+    do, ds = torch.randn(o.shape, generator=gen).to(dev()), torch.randn(s.shape, generator=gen).to(dev())
+    names = ["q", "k", "v", "g", "beta", "h0"]
+    grads = torch.autograd.grad((o, s), [x[n] for n in names], (do, ds))
+    eo, es, eg = oracle_grads({n: x[n] for n in names}, do, ds)
+    errs = {"o": O.rel_l2(o, eo), "s": O.rel_l2(s, es)}
+    errs.update({"d" + n: O.rel_l2(gr, eg[n]) for n, gr in zip(names, grads)})
+    assert all(e <= 1e-4 for e in errs.values()), errs
+
+
 # ---------------------------------------------------------------------------------- packed sequences
 def test_varlen_ragged_fp32():
     cu = [0, 5, 69, 69, 200, 263]       # includes an empty segment and ragged tails
