@@ -455,18 +455,9 @@ class KimiDeltaAttention(nn.Module):
     def _plain_weights(self):
         """The layer's parameters in the native path's order, or None when a submodule is not the plain one this class built
         (replaced, hooked, parametrised, given a bias): such a layer runs its modules one by one."""
-        mods, weights = self._modules, []
         if torch.nn.modules.module._has_any_global_hook():
             return None
-        for name, cls in self._PLAIN:
-            m = mods[name]
-            if (type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-                    or "forward" in m.__dict__ or m._parameters.get("bias") is not None):
-                return None
-            weights.append(m._parameters.get("weight"))
-        own = self._parameters
-        weights[-1:] = (own.get("A_log"), own.get("dt_bias"), weights[-1])
-        return weights if all(type(w) in (nn.Parameter, Tensor) for w in weights) else None
+        return _native.load().plain_weights(self._modules, self._parameters, self._PLAIN, (nn.Parameter, Tensor))
 
     def decode_token(self, hidden_states: Tensor, state: KDAState) -> Tensor:
         """One decode token with the state updated IN PLACE (inference only).
@@ -478,18 +469,18 @@ class KimiDeltaAttention(nn.Module):
         their epilogue, the decode step with the gate projection before and the gated norm behind it, and the output
         projection.  The projections read the parameters as they are, no cast or copy is kept.  Same arithmetic, same
         results as the non-mutating path.  Batches above 64 run the modules one by one."""
-        if hidden_states.ndim != 3 or hidden_states.shape[1] != 1 or hidden_states.shape[-1] != self.hidden_size:
-            raise ValueError(f"hidden_states must have shape [B,1,{self.hidden_size}]")
-        if not hidden_states.is_cuda:
-            raise RuntimeError("project CUDA KDA backend unavailable: project KDA requires CUDA")
         x = hidden_states
-        if self.head_dim == 128 and type(x) is Tensor:
+        if self.head_dim == 128 and type(x) is Tensor and x.is_cuda:
             weights = self._plain_weights()
             if weights is not None:
                 out = _native.load().token(x, weights, self.num_heads, self._modules["o_norm"].eps, self.lower_bound,
                                            (state.memory, state.q_conv, state.k_conv, state.v_conv), True)
                 if out is not None:
                     return out[0]
+        if x.ndim != 3 or x.shape[1] != 1 or x.shape[-1] != self.hidden_size:
+            raise ValueError(f"hidden_states must have shape [B,1,{self.hidden_size}]")
+        if not x.is_cuda:
+            raise RuntimeError("project CUDA KDA backend unavailable: project KDA requires CUDA")
         return self._decode_modules(x, state)
 
     @torch.no_grad()

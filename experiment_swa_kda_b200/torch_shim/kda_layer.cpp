@@ -497,6 +497,47 @@ LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     return out;
 }
 
+// The layer's parameters in the order above, or None when a submodule is not the plain one the class built.  A token is three
+// launches, and these few dozen lookups as Python statements took as long as two of them.  plain: ((name, class), ...), the
+// norm last; types: what a parameter's type may be.
+pybind11::object plain_weights(const pybind11::dict& modules, const pybind11::dict& own, const pybind11::tuple& plain, const pybind11::tuple& types) {
+    namespace py = pybind11;
+    static PyObject* const hooks[4] = {PyUnicode_InternFromString("_forward_hooks"), PyUnicode_InternFromString("_forward_pre_hooks"),
+                                       PyUnicode_InternFromString("_backward_hooks"), PyUnicode_InternFromString("_backward_pre_hooks")};
+    static PyObject *const s_forward = PyUnicode_InternFromString("forward"), *const s_params = PyUnicode_InternFromString("_parameters"),
+                    *const s_bias = PyUnicode_InternFromString("bias"), *const s_weight = PyUnicode_InternFromString("weight"),
+                    *const s_A = PyUnicode_InternFromString("A_log"), *const s_dt = PyUnicode_InternFromString("dt_bias");
+    py::list out;
+    bool ok = true;
+    auto add = [&](PyObject* w) {
+        if (w != nullptr && (reinterpret_cast<PyObject*>(Py_TYPE(w)) == types[0].ptr() || reinterpret_cast<PyObject*>(Py_TYPE(w)) == types[1].ptr()))
+            out.append(py::handle(w));
+        else ok = false;
+    };
+    const py::ssize_t n = PyTuple_GET_SIZE(plain.ptr());
+    for (py::ssize_t i = 0; i < n && ok; ++i) {
+        if (i == n - 1) {
+            add(PyDict_GetItem(own.ptr(), s_A));
+            add(PyDict_GetItem(own.ptr(), s_dt));
+        }
+        PyObject* const item = PyTuple_GET_ITEM(plain.ptr(), i);
+        PyObject* const m = PyDict_GetItem(modules.ptr(), PyTuple_GET_ITEM(item, 0));
+        if (m == nullptr || reinterpret_cast<PyObject*>(Py_TYPE(m)) != PyTuple_GET_ITEM(item, 1)) return py::none();
+        const py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(m, nullptr));
+        if (!d) throw py::error_already_set();
+        for (PyObject* h : hooks) {
+            PyObject* const v = PyDict_GetItem(d.ptr(), h);
+            if (v == nullptr || PyObject_Size(v) != 0) return py::none();
+        }
+        PyObject* const params = PyDict_GetItem(d.ptr(), s_params);
+        if (params == nullptr || !PyDict_Check(params) || PyDict_GetItem(d.ptr(), s_forward) != nullptr) return py::none();
+        PyObject* const bias = PyDict_GetItem(params, s_bias);
+        if (bias != nullptr && bias != Py_None) return py::none();
+        add(PyDict_GetItem(params, s_weight));
+    }
+    return ok ? py::object(out) : py::none();
+}
+
 }  // namespace
 
 void bind_layer(pybind11::module_& m) {
@@ -504,6 +545,7 @@ void bind_layer(pybind11::module_& m) {
     using nogil = py::call_guard<py::gil_scoped_release>;
     m.def("layer", &layer, nogil());
     m.def("token", &token, nogil());
+    m.def("plain_weights", &plain_weights);
 }
 
 }  // namespace kda_host
