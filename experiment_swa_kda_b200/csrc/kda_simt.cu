@@ -11,7 +11,7 @@
 // Substituting Z, the recurrence is affine in H with coefficients that do not depend on it:
 //   H' = exp(G_end) . H - (E^T W) H + E^T U        dH = exp(G_end) . dH' - (E^T W)^T dH' + (R - A W)^T dO
 // so everything but one K x K product per step is formed for all chunks side by side, and the scans carry a quarter of
-// the work they would with Z inside: at K = V = 64 and 32 chunks 303 + 533 us became 17 + 17.
+// the work they would with Z inside: at K = V = 64 and 32 chunks 303 + 533 us became 36 + 36.
 // The equations restate reference chunk_wy_forward.cu:125-405, 761-858, 940-1275, 1498-1588
 // and, for the adjoints, chunk_wy_backward.cu:2445-2562, 2818-3331, 3337-3552, 3787-3894.
 //
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(256, 3) intra_fwd_kernel(Ws w, IntraArgs p) {
 // its decay) comes through a ring filled by asynchronous copies three tiles ahead; four groups of two warps share the
 // contraction and meet in shared memory, laid out so that no access of the step has a bank conflict.  The strip lives in
 // registers (thread = row x 4 columns) and, for the products, in shared memory.  1.9 us a step at K = 64 while B was loaded
-// one step ahead into registers and the partial sums conflicted; 0.7 now, a chain of four barriers and 16 x 18 instructions.
+// one step ahead into registers and the partial sums conflicted; 1.1 now, a chain of four barriers and 16 x 18 instructions.
 // ---------------------------------------------------------------------------------------------
 constexpr int kVS = 16, kScanStages = 4;
 constexpr int kStageFloats = 4096 + 64 * kVS + 64;      // tile, strip of B, decay of one 64-row block

@@ -98,8 +98,11 @@ constexpr int kIntraBwdSmem = kSmall + ((4 + 4 + 8 + 4) * 128 + 64 * 8 + 3 * 64)
 // Bound by latency: 225 KB of shared memory allow one CTA per SM, and its products depend on one another (state products
 // -> X -> Y -> dM -> pull-back).  So (1) only the operand of the next product is read out before that product is issued,
 // and everything else - dv, the dR / dE / dQ contributions, the pull-back's decay panels - runs while it is in flight;
-// (2) the six state products are issued by five warps as soon as their inputs have landed; (3) a warp fetches the inputs
+// (2) of the six state products the two that the next phase needs are issued first, the others by warps that have finished
+// their share of the work beside them; (3) a warp fetches the inputs
 // of the CTA that this SM is likely to run next into L2; (4) token pairs go through packed float32 arithmetic.
+// 16,384 chunk-heads: 2,262 -> 1,733 us (7 % of it the prefetch), 384: 81 -> 61 us.  A persistent form that loads the next
+// chunk-head's panels during the gradient assembly took 1,830: the loads are not what it waits for any more.
 template <bool GB>
 __global__ void __launch_bounds__(512, 1)
     tc_intra_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,

@@ -6,7 +6,7 @@
 // projection in place, and the backward forms the gradient of the input as one GEMM over all six and the six weight
 // gradients as another, both accumulated in float32.  Columns of the projection P [tokens][n]:
 //     q | k | v | output gate (hidden each) | f_a (128) | b (heads) | zero padding to a multiple of 8
-// B2 T2045 width 768, forward and backward: 1,141 us and 65 launches -> 420 us and 27.
+// B2 T2045 width 768, forward and backward: 1,141 us and 65 launches -> 406 us and 27.
 
 #include <torch/extension.h>
 
