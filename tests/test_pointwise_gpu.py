@@ -112,6 +112,28 @@ def test_streaming_convolution_equals_short_pieces(W, B, T, C):
                 assert torch.equal(y[b, t0:t0 + 4096], piece[0, h:])
 
 
+# 2,048 channels: 36 blocks of 64 tokens take the tile kernel, 37 the streaming one, both with ragged ends
+@pytest.mark.parametrize("T", [36 * 64 - 1, 36 * 64 + 1])
+def test_conv_backward_either_side_of_the_streaming_line(T):
+    test_conv_training_path_matches_oracle(1, T, 2048, torch.bfloat16)
+
+
+# the even, the odd (one channel a thread) and the final-state paths each end in the reduction that rounds
+@pytest.mark.parametrize("B,T,C,W,state", [(2, 70, 384, 4, False), (1, 33, 17, 4, False), (2, 65, 24, 3, True), (1, 5, 8, 6, False)])
+def test_bf16_weight_gradient_is_the_float32_one_rounded(B, T, C, W, state):
+    from experiment_swa_kda_b200 import nanochat_ops
+    nanochat_ops.register()
+    ops = torch.ops.nanochat_kda
+    gen = torch.Generator(device=D0).manual_seed(T + C)
+    draw = lambda *n: torch.randn(*n, device=D0, generator=gen).bfloat16()
+    x, dy, w = draw(B, T, C), draw(B, T, C), draw(C, W)
+    s0, dfin = (draw(B, C, W), draw(B, C, W)) if state else (None, None)
+    dx, dw, _ = ops.causal_convolution_backward(x, w, s0, x, None, dy, dfin)
+    dx32, dw32, _ = ops.causal_convolution_backward(x, w.float(), s0, x, None, dy, dfin)
+    assert dw.dtype == torch.bfloat16 and dw32.dtype == torch.float32
+    assert torch.equal(dx, dx32) and torch.equal(dw, dw32.bfloat16())
+
+
 @pytest.mark.parametrize("B,T,C,dtype", [(2, 300, 384, torch.bfloat16), (1, 67, 20, torch.float32)])
 def test_short_convolutions_one_launch_equals_per_tensor_calls(B, T, C, dtype):
     """The batched q/k/v convolution entry points give bit-identical outputs and gradients to three separate calls."""
