@@ -420,7 +420,10 @@ __device__ __forceinline__ float ld_w(const void* w, size_t i, bool bf16, int wf
     return ld_io(w, i, bf16);
 }
 
-// weights of VEC adjacent channels: W*VEC contiguous elements starting at c0*W
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// weights of VEC adjacent channels: W*VEC contiguous elements starting at c0*W.  A weight may be a view into a flat
+// parameter buffer at any element offset, so it is the address, not the index, that allows a 16-byte load.
 template <int W, int VEC, bool BF16>
 __device__ __forceinline__ void ld_weights(float (&wv)[W][VEC], const void* wgt, int c0, int wf32) {
     float flat[W * VEC];
@@ -429,7 +432,7 @@ __device__ __forceinline__ void ld_weights(float (&wv)[W][VEC], const void* wgt,
     if (wf32) {
 #pragma unroll
         for (int j = 0; j < N; ++j) flat[j] = ld_w(wgt, base + j, BF16, 1);
-    } else if (BF16 && N % 8 == 0 && (base % 8) == 0) {
+    } else if (BF16 && N % 8 == 0 && aligned16(reinterpret_cast<const __nv_bfloat16*>(wgt) + base)) {
 #pragma unroll
         for (int j = 0; j < N / 8; ++j) {
             float t[8];
@@ -437,7 +440,7 @@ __device__ __forceinline__ void ld_weights(float (&wv)[W][VEC], const void* wgt,
 #pragma unroll
             for (int e = 0; e < 8; ++e) flat[8 * j + e] = t[e];
         }
-    } else if (!BF16 && N % 4 == 0 && (base % 4) == 0) {
+    } else if (!BF16 && N % 4 == 0 && aligned16(reinterpret_cast<const float*>(wgt) + base)) {
 #pragma unroll
         for (int j = 0; j < N / 4; ++j) {
             float t[4];
@@ -572,7 +575,8 @@ __device__ __forceinline__ void st_pair(void* p, size_t i, float a, float b) {
 }
 
 // N consecutive weights starting at element `base` (the W taps of N / W adjacent channels), with 16-byte loads when the
-// run is 16-byte aligned: a warp then reads one contiguous span instead of 32 scattered words per tap.
+// run is 16-byte aligned: a warp then reads one contiguous span instead of 32 scattered words per tap.  The weights
+// themselves are 16-byte aligned: the host sends any other to the kernels that read them with ld_weights.
 template <int N, bool BF16>
 __device__ __forceinline__ void ld_wrun(float (&flat)[N], const void* wgt, size_t base, int wf32) {
     const bool f32 = wf32 || !BF16;
@@ -2081,7 +2085,7 @@ int conv_bwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
 template <int W>
 int conv_fwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x, const void* w, const void* cache, void* y,
                void* fin, cudaStream_t st) {
-    const bool al16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16) == 0;
+    const bool al16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) % 16) == 0;
     if (C % 2 == 0 && al16 && conv_grid_ok(1, B, T)) {
         pw::ConvFwdItems it = {};
         it.x[0] = x; it.w[0] = w; it.y[0] = y; it.cache[0] = cache; it.fin[0] = fin;
@@ -2106,7 +2110,7 @@ int conv_bwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x,
     if constexpr (W <= 4) {
         // no carried-in window and no final-state cotangent: the tiled kernel (same partial layout: one row of
         // partials per 64-token tile and batch entry)
-        if (!cache && !dfin && !dcache && C % 2 == 0 && al16) {
+        if (!cache && !dfin && !dcache && C % 2 == 0 && al16 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
             pw::ConvBwdItems it = {};
             it.x[0] = x; it.w[0] = w; it.dy[0] = dy; it.dx[0] = dx;
             return conv_bwd_fast<W>(1, B, T, C, C, bf16, wf32, silu, it, &dwgt, part, st, dwb);
@@ -2198,11 +2202,12 @@ extern "C" int kda_conv_bwd(int32_t batch, int32_t seq_len, int32_t channels, in
 // and row stride, 16-byte aligned tensors; anything else returns KDA_ERR_UNSUPPORTED and the caller issues the per-tensor
 // calls.
 namespace {
-bool conv_multi_ok(int n, int channels, int width, const void* const* a, const void* const* b, const void* const* c) {
+bool conv_multi_ok(int n, int channels, int width, const void* const* w, const void* const* a, const void* const* b, const void* const* c) {
     if (n < 1 || n > pw::kConvItems || width > 4 || channels % 2 != 0) return false;
     for (int i = 0; i < n; ++i) {
         if (!a[i] || !b[i] || (c && !c[i])) return false;
-        if ((reinterpret_cast<uintptr_t>(a[i]) | reinterpret_cast<uintptr_t>(b[i]) | (c ? reinterpret_cast<uintptr_t>(c[i]) : 0)) % 16) return false;
+        if ((reinterpret_cast<uintptr_t>(w[i]) | reinterpret_cast<uintptr_t>(a[i]) | reinterpret_cast<uintptr_t>(b[i]) |
+             (c ? reinterpret_cast<uintptr_t>(c[i]) : 0)) % 16) return false;
     }
     return true;
 }
@@ -2214,7 +2219,7 @@ extern "C" int kda_conv_fwd_rows(int32_t n_items, int32_t batch, int32_t seq_len
     if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0 || x_ld < channels) return KDA_ERR_BAD_SHAPE;
     if (!x || !weight || !y) return KDA_ERR_NULL;
     if (x_ld % 2 != 0 || !conv_grid_ok(n_items, batch, seq_len) ||
-        !conv_multi_ok(n_items, channels, width, x, const_cast<const void* const*>(y), nullptr))
+        !conv_multi_ok(n_items, channels, width, weight, x, const_cast<const void* const*>(y), nullptr))
         return KDA_ERR_UNSUPPORTED;
     const int wf32 = (io_dtype & KDA_WEIGHT_F32) != 0;
     const int bf16 = (io_dtype & 0xff) == KDA_DTYPE_BF16;
@@ -2279,7 +2284,7 @@ extern "C" int kda_conv_bwd_rows(int32_t n_items, int32_t batch, int32_t seq_len
                                  size_t scratch_bytes, void* stream) {
     if (batch <= 0 || seq_len <= 0 || channels <= 0 || width <= 0 || x_ld < channels) return KDA_ERR_BAD_SHAPE;
     if (!x || !weight || !d_y || !dx || !dweight) return KDA_ERR_NULL;
-    if (x_ld % 2 != 0 || !conv_grid_ok(n_items, batch, seq_len) || !conv_multi_ok(n_items, channels, width, x, d_y, const_cast<const void* const*>(dx))) return KDA_ERR_UNSUPPORTED;
+    if (x_ld % 2 != 0 || !conv_grid_ok(n_items, batch, seq_len) || !conv_multi_ok(n_items, channels, width, weight, x, d_y, const_cast<const void* const*>(dx))) return KDA_ERR_UNSUPPORTED;
     if (!scratch || scratch_bytes < kda_conv_bwd_multi_scratch_bytes(n_items, batch, seq_len, channels, width)) return KDA_ERR_WORKSPACE;
     const int wf32 = (io_dtype & KDA_WEIGHT_F32) != 0;
     const int bf16 = (io_dtype & 0xff) == KDA_DTYPE_BF16;

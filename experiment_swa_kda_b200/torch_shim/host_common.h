@@ -28,6 +28,8 @@ inline Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& li
     return Tensor(at::detail::empty_cuda(sizes, type, like.device(), c10::nullopt));
 }
 inline Tensor empty_as(const Tensor& t) { return empty(t.sizes(), t.scalar_type(), t); }
+// t itself, or a copy where its address would rule out 16-byte accesses (a view at an odd offset of a larger buffer)
+inline Tensor aligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0 ? t : t.clone(); }
 inline Tensor bytes(size_t n, const Tensor& like) { return empty({(int64_t)(n < 256 ? 256 : n)}, at::kByte, like); }
 
 // One allocation cut into 256-byte aligned tensors: a call's temporaries cost one trip to the allocator.

@@ -382,9 +382,9 @@ ChunkResult kda_raw(const Tensor& q, const Tensor& k, const Tensor& v, const Ten
 }
 
 // ------------------------------------------------------------------------------------------------ short convolution
-// weight of a convolution as the kernels take it: [C, W] dense, float32 or the activations' type
+// weight of a convolution as the fast kernels take it: [C, W] dense and 16-byte aligned, float32 or the activations' type
 Tensor conv_weight(const Tensor& w, const Tensor& x) {
-    return w.scalar_type() == at::kFloat ? dense(w) : dense_as(w, x.scalar_type());
+    return aligned(w.scalar_type() == at::kFloat ? dense(w) : dense_as(w, x.scalar_type()));
 }
 
 Tensor grad_like(const Tensor& dw, at::ScalarType type, const std::vector<int64_t>& shape) {

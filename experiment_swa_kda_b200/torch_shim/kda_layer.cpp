@@ -322,11 +322,12 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     const int64_t h = z.hid, M = z.M, n = z.n;
     const KdaChunkShape sh = layer_shape(z, !tracked);
     Kept kept(z, sh, tracked, !few, !fuse_conv);
-    Tensor x, nw, y, mem, win[3], cache[3], h0;
+    Tensor x, nw, y, mem, win[3], cache[3], h0, taps[3];
     {
         at::AutoDispatchBelowADInplaceOrView below;
         x = dense(x_);
         nw = dense_as(w[kNorm], at::kFloat);
+        for (int i = 0; i < 3; ++i) taps[i] = aligned(w[kCq + i]);
         kept.slab.make(x);
         y = empty({z.B, z.T, h}, at::kBFloat16, x);
         if (want_state) {
@@ -355,7 +356,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         void *yp[3], *fp[3];
         for (int i = 0; i < 3; ++i) {
             xp[i] = at_col(P, i * h);
-            wp[i] = w[kCq + i].data_ptr();
+            wp[i] = taps[i].data_ptr();
             yp[i] = const_cast<char*>(qkv[i]);
             cp[i] = cache[i].defined() ? cache[i].data_ptr() : nullptr;
             fp[i] = want_state ? win[i].data_ptr() : nullptr;
@@ -378,7 +379,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     if (fuse_conv) {
         for (int i = 0; i < 3; ++i) {
             qkv[i] = at_col(P, i * h);
-            ex.conv_weight[i] = w[kCq + i].data_ptr();
+            ex.conv_weight[i] = taps[i].data_ptr();
         }
         ex.conv_width = 4;
         ex.conv_weight_dtype = dt(w[kCq]);
@@ -417,7 +418,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         node->dt_shape = w[kDt].sizes().vec();
         node->has_state = !state.empty();
         const Tensor all = kept.slab.tensor();
-        for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &w[kCq], &w[kCk], &w[kCv], &w[kAlog], &w[kDt], &nw, &all}) node->keep(*t);
+        for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &taps[0], &taps[1], &taps[2], &w[kAlog], &w[kDt], &nw, &all}) node->keep(*t);
         if (!state.empty())
             for (auto& t : cache) node->keep(t);
         torch::autograd::set_history(y, node);
@@ -470,13 +471,14 @@ LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         out.push_back(mem);
         const void *xp[3], *wp[3], *cp[3];
         void *yp[3], *fp[3];
-        Tensor cache[3];
+        Tensor cache[3], taps[3];
         for (int i = 0; i < 3; ++i) {
+            taps[i] = aligned(w[kCq + i]);
             cache[i] = dense_as(state[1 + i], at::kBFloat16);
             const Tensor win = empty_as(cache[i]);
             out.push_back(win);
             xp[i] = at_col(P, i * h);
-            wp[i] = w[kCq + i].data_ptr();
+            wp[i] = taps[i].data_ptr();
             yp[i] = q + i * act;
             cp[i] = cache[i].data_ptr();
             fp[i] = win.data_ptr();

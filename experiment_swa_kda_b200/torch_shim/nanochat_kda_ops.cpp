@@ -319,7 +319,7 @@ std::tuple<Tensor, OptTensor> causal_convolution_forward(const Tensor& x, const 
     const ConvDims d = validate_conv(x, weight, initial_state, "initial_state");
     TORCH_CHECK(x.is_contiguous(), "nanochat_kda::causal_convolution_forward requires a contiguous input");
     c10::cuda::CUDAGuard guard(x.device());
-    const Tensor w = dense_as(weight, x.scalar_type());
+    const Tensor w = aligned(dense_as(weight, x.scalar_type()));
     OptTensor s0;
     if (has(initial_state)) s0 = initial_state->contiguous().to(x.scalar_type());
     Tensor y = empty_as(x);
@@ -347,7 +347,7 @@ std::tuple<Tensor, Tensor, OptTensor> causal_convolution_backward(const Tensor& 
     TORCH_CHECK(grad_output.is_cuda() && grad_output.device() == x_.device(), "grad_output must be on the same device as x");
     c10::cuda::CUDAGuard guard(x_.device());
     const Tensor x = dense(x_);
-    const Tensor w = dense_as(weight, x.scalar_type());
+    const Tensor w = aligned(dense_as(weight, x.scalar_type()));
     OptTensor s0, dfin, dinit;
     if (has(initial_state)) {
         s0 = initial_state->contiguous().to(x.scalar_type());

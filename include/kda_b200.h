@@ -262,7 +262,7 @@ int kda_decode_steps(int32_t n_steps, int32_t n_seq, int32_t heads, int32_t key_
                      const void* g, const void* beta, float* state, void* o, void* stream);
 
 /* ---- short causal depthwise convolution + SiLU --------------------------------
- * x,y [B,T,C]; weight [C,W] in io_dtype; cache [B,C,W] in io_dtype holds the last W
+ * x,y [B,T,C]; weight [C,W] in io_dtype, at any element address; cache [B,C,W] in io_dtype holds the last W
  * inputs including the current token.  Stands in for
  * nanochat_kda::causal_convolution_forward / _backward
  * (reference causal_convolution_forward.cu:149-237, causal_convolution_backward.cu:303-451).
@@ -280,7 +280,7 @@ int kda_conv_bwd(int32_t batch, int32_t seq_len, int32_t channels, int32_t width
 
 /* n_items (1..4) same-shaped convolutions in ONE launch each way - the q, k and v branches of a layer (the reference
  * issues three separate operator calls, nanochat/mixers/kda.py:758-766; there is no batched counterpart there).
- * Training path only: no carried-in window, no final state, width <= 4, even channel count, 16-byte aligned tensors;
+ * Training path only: no carried-in window, no final state, width <= 4, even channel count, 16-byte aligned tensors and weights;
  * any other case returns KDA_ERR_UNSUPPORTED and the caller issues the per-tensor calls.  x, weight, y, d_y, dx, dweight
  * are HOST arrays of n_items device pointers; io_dtype may carry KDA_WEIGHT_F32.  scratch:
  * kda_conv_bwd_multi_scratch_bytes. */

@@ -254,3 +254,43 @@ def test_layer_forward_backward_finite_and_matches_composed_oracle():
         ye = lin("o_proj", o.reshape(2, 70, 256))
     assert O.rel_l2(y.float(), ye) <= 3e-2      # several bf16 GEMMs in series
     assert O.rel_l2(st.memory, mem) <= 3e-2
+
+
+# A weight that is a view into a flat parameter buffer (1, 2, 3 or 6 elements before it) allows no 16-byte loads: every
+# entry point gives what it gives for an aligned copy.  Widths and types whose taps are read in 16-byte pieces otherwise; a
+# carried window, none, and the channel counts of the pair (2), streaming (128) and one-channel kernels.
+@pytest.mark.parametrize("B,T,C,W,dtype,wdtype", [(2, 70, 384, 4, torch.bfloat16, torch.float32), (1, 33, 130, 4, torch.bfloat16, torch.bfloat16),
+                                                  (2, 65, 24, 4, torch.float32, torch.float32), (1, 9, 16, 8, torch.bfloat16, torch.bfloat16),
+                                                  (1, 7, 5, 8, torch.float32, torch.float32), (1, 28423, 2048, 4, torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("state", [False, True])
+@pytest.mark.parametrize("offset", [1, 6])
+def test_convolution_weights_at_any_element_offset(B, T, C, W, dtype, wdtype, state, offset):
+    from experiment_swa_kda_b200 import ops
+    gen = torch.Generator(device=D0).manual_seed(T + C + offset)
+    draw = lambda *n: torch.randn(*n, device=D0, generator=gen).to(dtype)
+    x, dy = draw(B, T, C), draw(B, T, C)
+    s0, dfin = (draw(B, C, W), draw(B, C, W)) if state else (None, None)
+    w = torch.randn(C, W, device=D0, generator=gen).to(wdtype)
+    flat = torch.empty(offset + C * W, device=D0, dtype=wdtype)
+    view = flat[offset:].view(C, W).copy_(w)
+    assert view.data_ptr() % 16 != 0 and w.data_ptr() % 16 == 0
+    # the library itself: the one-channel kernels sum in the same order as the fast ones, up to the width of an fma
+    tol = 1e-2 if dtype == torch.bfloat16 else 1e-5
+    for a, b in zip((*ops.conv_fwd(x, view, s0, state), *ops.conv_bwd(x, view, s0, dy, dfin)),
+                    (*ops.conv_fwd(x, w, s0, state), *ops.conv_bwd(x, w, s0, dy, dfin))):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert O.rel_l2(a.float(), b.float()) <= tol
+    # the operators: an aligned copy of the weight on the fast kernels, to the bit
+    results = []
+    for weight in (view, w):
+        leaf = weight.detach().requires_grad_(True)
+        assert leaf.data_ptr() == weight.data_ptr()
+        xs = x.detach().clone().requires_grad_(True)
+        y, fin = ops.conv(xs, leaf, s0, state)
+        outs = [y, fin] if state else [y]
+        results.append([*outs, *torch.autograd.grad(outs, [xs, leaf], [dy, dfin][:len(outs)])])
+        if not state and W <= 4:
+            ys = ops.ConvMultiFunction.apply(True, 2, xs, xs, leaf, leaf)
+            results[-1] += [*ys, *torch.autograd.grad(ys, [xs, leaf], [dy, dy])]
+    assert all(torch.equal(a, b) for a, b in zip(*results))
