@@ -2,6 +2,7 @@
 
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -47,6 +48,13 @@ static int check_shape(const KdaChunkShape* s, const int32_t* cu) {
     return KDA_OK;
 }
 
+// The tensor-core lane moves its tensors by TMA and in 16-byte accesses; beta and dbeta alone are read element by element.
+static bool off16(std::initializer_list<const void*> ps) {
+    uintptr_t a = 0;
+    for (const void* p : ps) a |= reinterpret_cast<uintptr_t>(p);
+    return a % 16 != 0;
+}
+
 extern "C" const char* kda_error_string(int code) {
     switch (code) {
         case KDA_OK: return "ok";
@@ -87,6 +95,7 @@ extern "C" int kda_chunk_fwd(const KdaChunkShape* shape, const void* q, const vo
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0 ||
         workspace_bytes < kda_chunk_workspace_bytes(shape))
         return KDA_ERR_WORKSPACE;
+    if (shape->lane == KDA_LANE_TC && off16({q, k, v, g, h0, o, final_state})) return KDA_ERR_UNSUPPORTED;
     return simt_chunk_fwd(shape, q, k, v, g, beta, h0, cu_seqlens, o, final_state, workspace, (cudaStream_t)stream, nullptr);
 }
 
@@ -110,14 +119,10 @@ extern "C" int kda_chunk_fwd_ex(const KdaChunkShape* shape, const KdaChunkExtras
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0 || workspace_bytes < kda_chunk_workspace_bytes(shape))
         return KDA_ERR_WORKSPACE;
     const int64_t hk = (int64_t)shape->heads * shape->key_dim, gate_ld = ex->gate_ld ? ex->gate_ld : hk, x_ld = ex->x_ld ? ex->x_ld : hk;
-    if (norm && (gate_ld < hk || gate_ld % 8 != 0 ||
-                 (reinterpret_cast<uintptr_t>(ex->gate) | reinterpret_cast<uintptr_t>(ex->y) | reinterpret_cast<uintptr_t>(ex->norm_weight)) % 16 != 0))
-        return KDA_ERR_UNSUPPORTED;
-    if (conv && (x_ld < hk || x_ld % 8 != 0 ||
-                 (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
-                  reinterpret_cast<uintptr_t>(ex->conv_weight[0]) | reinterpret_cast<uintptr_t>(ex->conv_weight[1]) |
-                  reinterpret_cast<uintptr_t>(ex->conv_weight[2])) % 16 != 0))
-        return KDA_ERR_UNSUPPORTED;
+    // the norm's epilogue writes o in 8-byte pieces
+    if (off16({q, k, v, g, h0, final_state}) || reinterpret_cast<uintptr_t>(o) % (norm ? 8 : 16) != 0) return KDA_ERR_UNSUPPORTED;
+    if (norm && (gate_ld < hk || gate_ld % 8 != 0 || off16({ex->gate, ex->y, ex->norm_weight}))) return KDA_ERR_UNSUPPORTED;
+    if (conv && (x_ld < hk || x_ld % 8 != 0 || off16({ex->conv_weight[0], ex->conv_weight[1], ex->conv_weight[2]}))) return KDA_ERR_UNSUPPORTED;
     tc::ConvPrep cp{{ex->conv_weight[0], ex->conv_weight[1], ex->conv_weight[2]}, ex->conv_weight_dtype == KDA_DTYPE_F32 ? 1 : 0, x_ld};
     tc::NormEpilogue ep{static_cast<const __nv_bfloat16*>(ex->gate), ex->norm_weight, ex->eps, static_cast<__nv_bfloat16*>(ex->y), ex->inv_rms, gate_ld};
     return simt_chunk_fwd(shape, q, k, v, g, beta, h0, cu_seqlens, o, final_state, workspace, (cudaStream_t)stream, norm ? &ep : nullptr,
@@ -160,6 +165,7 @@ extern "C" int kda_chunk_bwd(const KdaChunkShape* shape, const void* q, const vo
     if (!scratch || (reinterpret_cast<uintptr_t>(scratch) % 256) != 0 ||
         scratch_bytes < kda_chunk_bwd_scratch_bytes(shape))
         return KDA_ERR_WORKSPACE;
+    if (shape->lane == KDA_LANE_TC && off16({q, k, v, g, d_o, d_final_state, dq, dk, dv, dg, dh0})) return KDA_ERR_UNSUPPORTED;
     return simt_chunk_bwd(shape, q, k, v, g, beta, cu_seqlens, d_o, d_final_state, workspace, scratch, dq, dk, dv, dg,
                           dbeta, dh0, (cudaStream_t)stream);
 }

@@ -132,8 +132,8 @@ struct ChunkNode : public HostNode {
         const Tensor &q = t[0], &k = t[1], &v = t[2], &g = t[3], &beta = t[4], &ws = t[5];
         c10::cuda::CUDAGuard guard(q.device());
         watch_status(q.device().index());
-        const Tensor d_o = grads[0].defined() ? dense(grads[0]) : at::zeros_like(v);
-        const Tensor dfs = grads[1].defined() ? dense_as(grads[1], at::kFloat) : Tensor();
+        const Tensor d_o = grads[0].defined() ? aligned(dense(grads[0])) : at::zeros_like(v);
+        const Tensor dfs = grads[1].defined() ? aligned(dense_as(grads[1], at::kFloat)) : Tensor();
         ChunkGrads r = run_chunk_bwd(sh, q, k, v, g, beta, cu, d_o, dfs, ws, has_h0);
         return {r.dq, r.dk, r.dv, r.dg, r.db, r.dh0};
     }
@@ -154,8 +154,8 @@ ChunkOut run_chunk(const Tensor& q_, const Tensor& k_, const Tensor& v_, const T
     ChunkOut out;
     {
         at::AutoDispatchBelowADInplaceOrView below;
-        q = dense(q_), k = dense(k_), v = dense(v_), g = dense(g_), beta = dense(beta_);
-        if (has(h0_)) h0 = dense(*h0_);
+        q = aligned(dense(q_)), k = aligned(dense(k_)), v = aligned(dense(v_)), g = aligned(dense(g_)), beta = dense(beta_);
+        if (has(h0_)) h0 = aligned(dense(*h0_));
         if (has(cu_)) cu = dense(*cu_);
         sh = chunk_shape(q, g, d, cu.defined(), scale, l2norm, lane, !tracked);
         out.o = empty(v.sizes(), v.scalar_type(), q);
@@ -211,8 +211,8 @@ struct ChunkNormNode : public HostNode {
         const Tensor &q = t[0], &k = t[1], &v = t[2], &g = t[3], &beta = t[4], &ws = t[5], &o = t[6], &gate = t[7], &w32 = t[8], &inv = t[9];
         c10::cuda::CUDAGuard guard(q.device());
         watch_status(q.device().index());
-        const Tensor dy = grads[0].defined() ? dense_as(grads[0], o.scalar_type()) : at::zeros_like(o);
-        const Tensor dfs = grads[1].defined() ? dense_as(grads[1], at::kFloat) : Tensor();
+        const Tensor dy = grads[0].defined() ? aligned(dense_as(grads[0], o.scalar_type())) : at::zeros_like(o);
+        const Tensor dfs = grads[1].defined() ? aligned(dense_as(grads[1], at::kFloat)) : Tensor();
         const int64_t D = o.size(3), rows = o.numel() / D;
         Tensor d_o = empty_as(o), dgate = empty_as(gate), dw = empty({D}, at::kFloat, o);
         Tensor nscr = bytes(kda_rmsnorm_gate_bwd_scratch_bytes(rows, (int32_t)D), o);
@@ -240,12 +240,12 @@ ChunkResult chunk_kda_norm(const Tensor& q_, const Tensor& k_, const Tensor& v_,
     KdaChunkShape sh;
     {
         at::AutoDispatchBelowADInplaceOrView below;
-        q = dense(q_), k = dense(k_), v = dense(v_), g = dense(g_), beta = dense(beta_);
-        if (has(h0_)) h0 = dense(*h0_);
+        q = aligned(dense(q_)), k = aligned(dense(k_)), v = aligned(dense(v_)), g = aligned(dense(g_)), beta = dense(beta_);
+        if (has(h0_)) h0 = aligned(dense(*h0_));
         if (has(cu_)) cu = dense(*cu_);
         sh = chunk_shape(q, g, d, cu.defined(), sc, l2norm, KDA_LANE_TC, !tracked);
-        gate = dense_as(gate_, v.scalar_type());
-        w32 = dense_as(nw_, at::kFloat);
+        gate = aligned(dense_as(gate_, v.scalar_type()));
+        w32 = aligned(dense_as(nw_, at::kFloat));
         o = empty(v.sizes(), v.scalar_type(), q);
         y = empty(v.sizes(), v.scalar_type(), q);
         inv = empty({d.B * d.T * d.H}, at::kFloat, q);

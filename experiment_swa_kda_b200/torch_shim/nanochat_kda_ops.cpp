@@ -158,7 +158,8 @@ std::tuple<Tensor, OptTensor> chunk_forward(const Tensor& q_, const Tensor& k_, 
     const Dims d = validate_chunk_inputs(q_, k_, v_, raw_gate_, beta_logits_, A_log, dt_bias, initial_state, lower_bound, cu_seqlens);
     c10::cuda::CUDAGuard guard(q_.device());
     watch_status(q_.device().index());
-    const Tensor q = dense(q_), k = dense(k_), v = dense(v_), raw_gate = dense(raw_gate_), beta_logits = dense(beta_logits_);
+    const Tensor q = aligned(dense(q_)), k = aligned(dense(k_)), v = aligned(dense(v_)), raw_gate = dense(raw_gate_), beta_logits = dense(beta_logits_);
+    const OptTensor h0 = has(initial_state) ? OptTensor(aligned(*initial_state)) : OptTensor();
     // A call none of whose inputs takes part in a graph is inference / prefill: nothing is kept for a backward.
     bool needs_grad = false;
     for (const Tensor* t : {&q_, &k_, &v_, &raw_gate_, &beta_logits_, &A_log, &dt_bias}) needs_grad = needs_grad || t->requires_grad();
@@ -175,7 +176,7 @@ std::tuple<Tensor, OptTensor> chunk_forward(const Tensor& q_, const Tensor& k_, 
     if (output_final_state) final_state = empty({d.N, d.H, d.V, d.K}, at::kFloat, q);
     if (d.B * d.T > 0) {
         run_gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound, d, g, beta);
-        check(kda_chunk_fwd(&sh, q.data_ptr(), k.data_ptr(), v.data_ptr(), g, beta, static_cast<const float*>(ptr(initial_state)),
+        check(kda_chunk_fwd(&sh, q.data_ptr(), k.data_ptr(), v.data_ptr(), g, beta, static_cast<const float*>(ptr(h0)),
                             static_cast<const int32_t*>(ptr(cu_seqlens)), output.data_ptr(),
                             output_final_state ? final_state->data_ptr<float>() : nullptr, base + l.ws_off, l.ws_bytes, stream_of(q)),
               "kda_chunk_fwd");
@@ -208,7 +209,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
     }
     c10::cuda::CUDAGuard guard(q_.device());
     watch_status(q_.device().index());
-    const Tensor q = dense(q_), k = dense(k_), v = dense(v_), raw_gate = dense(raw_gate_), beta_logits = dense(beta_logits_);
+    const Tensor q = aligned(dense(q_)), k = aligned(dense(k_)), v = aligned(dense(v_)), raw_gate = dense(raw_gate_), beta_logits = dense(beta_logits_);
+    const OptTensor h0 = has(initial_state) ? OptTensor(aligned(*initial_state)) : OptTensor();
     const bool packed = has(cu_seqlens);
     KdaChunkShape sh = chunk_shape(d, scale, packed, false);
     Layout l = layout_for(d, sh);
@@ -231,14 +233,14 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> ch
         run_gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound, d, reinterpret_cast<float*>(b + l.g_off),
                  reinterpret_cast<float*>(b + l.beta_off));
         check(kda_chunk_fwd(&sh, q.data_ptr(), k.data_ptr(), v.data_ptr(), b + l.g_off, b + l.beta_off,
-                            static_cast<const float*>(ptr(initial_state)), static_cast<const int32_t*>(ptr(cu_seqlens)),
+                            static_cast<const float*>(ptr(h0)), static_cast<const int32_t*>(ptr(cu_seqlens)),
                             scratch_out.data_ptr(), nullptr, b + l.ws_off, l.ws_bytes, stream_of(q)),
               "kda_chunk_fwd (recomputed for the backward)");
         base = b;
     }
-    const Tensor d_o = dense_as(grad_output, at::kBFloat16);
+    const Tensor d_o = aligned(dense_as(grad_output, at::kBFloat16));
     OptTensor dfs;
-    if (has(grad_final_state)) dfs = dense_as(*grad_final_state, at::kFloat);
+    if (has(grad_final_state)) dfs = aligned(dense_as(*grad_final_state, at::kFloat));
     Tensor dq = empty_as(q), dk = empty_as(k), dv = empty_as(v);
     Tensor dg = empty({d.B, d.T, d.H, d.K}, at::kFloat, q), db = empty({d.B, d.T, d.H}, at::kFloat, q);
     OptTensor dh0;

@@ -78,6 +78,7 @@ const char* kda_build_arch(void);
  * workspace: kda_chunk_workspace_bytes(shape) bytes, 256-byte aligned.  The
  * forward leaves in it everything the backward needs; keep it untouched until
  * kda_chunk_bwd has run.  h0 and final_state may be NULL.
+ * The tensor-core lane takes 16-byte aligned tensors (beta and dbeta at any address), else KDA_ERR_UNSUPPORTED.
  * With shape->forward_only set this is the no-grad prefill path (the reference
  * sends such calls to its token loop, chunk.cu:1694-1698).
  */
