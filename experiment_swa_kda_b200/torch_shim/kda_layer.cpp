@@ -163,7 +163,7 @@ struct LayerNode : public HostNode {
         Tensor small = empty({kHead + H + h + 3 * h * z.W}, at::kFloat, x);      // gradients of the vectors and the taps
         float *dnw = small.data_ptr<float>(), *dA = dnw + kHead, *dbias = dA + H, *dcw = dbias + h;
 
-        const Tensor dy = grads[0].defined() ? dense_as(grads[0], at::kBFloat16) : at::zeros({M, h}, x.options());
+        const Tensor dy = grads[0].defined() ? aligned(dense_as(grads[0], at::kBFloat16)) : at::zeros({M, h}, x.options());
         if (want(1 + kO)) out[1 + kO] = linear_dw(dy.data_ptr(), h, base + kept.mixed, h, M, h, h, wtype, x);
         linear_dx(dy.data_ptr(), h, packed_o(pack, z), h, dmix, h, M, h, h);
 
@@ -175,7 +175,7 @@ struct LayerNode : public HostNode {
         out[1 + kNorm] = ntype == at::kFloat ? g_nw : g_nw.to(ntype);
 
         // chunked operator
-        const Tensor dmem = grads[1].defined() ? dense_as(grads[1], at::kFloat) : Tensor();
+        const Tensor dmem = grads[1].defined() ? aligned(dense_as(grads[1], at::kFloat)) : Tensor();
         Tensor dh0;
         if (has_state) dh0 = empty({z.B, H, kHead, kHead}, at::kFloat, x);
         must(kda_chunk_bwd(&sh, base + kept.q, base + kept.k, base + kept.v, base + kept.g, base + kept.beta, nullptr, tmp.at(t_do),
@@ -254,6 +254,9 @@ struct LayerNode : public HostNode {
 
 // ------------------------------------------------------------------------------------------------ forward
 // The plain case: bf16 input, 128-wide heads, weights of one type (float32 masters or bf16), everything dense on one GPU.
+// A call that passes must not be declined by a kernel any more: what the kernels need aligned is tested here (the
+// projections, read as they are) or copied where it is not (the input, the vectors, the taps, the incoming memory), and
+// the convolutions' grid limits are tested by fits_grid.
 bool layer_sizes(const Tensor& x, const std::vector<Tensor>& w, int64_t heads, const std::vector<Tensor>& state, Sizes& z) {
     if (w.size() != kParams || x.dim() != 3 || !x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.numel() == 0 || heads < 1) return false;
     z.B = x.size(0), z.T = x.size(1), z.H = heads, z.M = z.B * z.T, z.hid = heads * kHead;
@@ -288,6 +291,9 @@ bool layer_sizes(const Tensor& x, const std::vector<Tensor>& w, int64_t heads, c
     return !at::autocast::is_autocast_enabled(at::kCUDA);
 }
 
+// kda_conv_*_rows: `items` convolutions share a launch whose grid has items x batch and 64-token tiles as its y and z
+bool fits_grid(const Sizes& z, int64_t items) { return z.B * items <= 65535 && (z.T + 63) / 64 <= 65535; }
+
 constexpr int64_t kFewRows = 64;
 
 // products of at most kFewRows rows with `count` consecutive weights of the list, straight from the parameters
@@ -313,6 +319,9 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     bool tracked = torch::autograd::compute_requires_grad(x_);
     for (const auto& t : w) tracked = tracked || torch::autograd::compute_requires_grad(t);
     for (const auto& t : state) tracked = tracked || torch::autograd::compute_requires_grad(t);
+    // a call that carries windows issues its convolutions one by one; a backward may take all three at once
+    const int conv_step = (want_state || !state.empty()) ? 1 : 3;
+    if (!fits_grid(z, tracked ? 3 : conv_step)) return c10::nullopt;
     fuse_conv = fuse_conv && !tracked && state.empty() && z.W == 4;
     // without a backward, up to 64 rows go straight to the float32 masters (kda_rows_linear): nothing to pack
     const bool few = !tracked && z.M <= kFewRows;
@@ -322,11 +331,12 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     const int64_t h = z.hid, M = z.M, n = z.n;
     const KdaChunkShape sh = layer_shape(z, !tracked);
     Kept kept(z, sh, tracked, !few, !fuse_conv);
-    Tensor x, nw, y, mem, win[3], cache[3], h0, taps[3];
+    Tensor x, nw, dt_bias, y, mem, win[3], cache[3], h0, taps[3];
     {
         at::AutoDispatchBelowADInplaceOrView below;
-        x = dense(x_);
-        nw = dense_as(w[kNorm], at::kFloat);
+        x = aligned(dense(x_));
+        nw = aligned(dense_as(w[kNorm], at::kFloat));
+        dt_bias = aligned(w[kDt]);
         for (int i = 0; i < 3; ++i) taps[i] = aligned(w[kCq + i]);
         kept.slab.make(x);
         y = empty({z.B, z.T, h}, at::kBFloat16, x);
@@ -335,7 +345,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
             for (auto& t : win) t = empty({z.B, h, z.W}, at::kBFloat16, x);
         }
         if (!state.empty()) {
-            h0 = dense(state[0]);
+            h0 = aligned(dense(state[0]));
             for (int i = 0; i < 3; ++i) cache[i] = dense_as(state[1 + i], at::kBFloat16);
         }
     }
@@ -349,7 +359,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         linear(x.data_ptr(), h, pack, h, P, n, M, n, h);
         linear(at_col(P, z.fa()), n, packed_fb(pack, z), kHead, raw, h, M, h, kHead);
     }
-    // convolutions on their slices of P: one launch; a call that carries windows issues them one by one
+    // convolutions on their slices of P
     const char* qkv[3] = {sl.at(kept.q), sl.at(kept.k), sl.at(kept.v)};
     if (!fuse_conv) {
         const void *xp[3], *wp[3], *cp[3];
@@ -361,13 +371,13 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
             cp[i] = cache[i].defined() ? cache[i].data_ptr() : nullptr;
             fp[i] = want_state ? win[i].data_ptr() : nullptr;
         }
-        const int io = KDA_DTYPE_BF16 | wflag(x, w[kCq]), step = (want_state || !state.empty()) ? 1 : 3;
-        for (int i = 0; i < 3; i += step)
-            must(kda_conv_fwd_rows(step, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xp + i, (int32_t)n, wp + i, cp + i, yp + i, fp + i, st),
+        const int io = KDA_DTYPE_BF16 | wflag(x, w[kCq]);
+        for (int i = 0; i < 3; i += conv_step)
+            must(kda_conv_fwd_rows(conv_step, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xp + i, (int32_t)n, wp + i, cp + i, yp + i, fp + i, st),
                  "kda_conv_fwd_rows");
     }
     must(kda_gate_fwd_rows((int32_t)M, (int32_t)heads, (int32_t)kHead, KDA_DTYPE_BF16, raw, at_col(P, z.b()), (int32_t)n, w[kAlog].data_ptr<float>(),
-                           w[kDt].data_ptr<float>(), (float)lb, sl.f32(kept.g), sl.f32(kept.beta), st),
+                           dt_bias.data_ptr<float>(), (float)lb, sl.f32(kept.g), sl.f32(kept.beta), st),
          "kda_gate_fwd_rows");
     KdaChunkExtras ex = {};
     ex.gate = at_col(P, 3 * h);
@@ -418,7 +428,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         node->dt_shape = w[kDt].sizes().vec();
         node->has_state = !state.empty();
         const Tensor all = kept.slab.tensor();
-        for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &taps[0], &taps[1], &taps[2], &w[kAlog], &w[kDt], &nw, &all}) node->keep(*t);
+        for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &taps[0], &taps[1], &taps[2], &w[kAlog], &dt_bias, &nw, &all}) node->keep(*t);
         if (!state.empty())
             for (auto& t : cache) node->keep(t);
         torch::autograd::set_history(y, node);
@@ -435,12 +445,14 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
 LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads, double eps, double lb, const std::vector<Tensor>& state, bool in_place) {
     Sizes z;
     if (state.size() != 4 || !layer_sizes(x_, w, heads, state, z) || z.T != 1 || z.M > kFewRows || !(lb >= -5.0 && lb < 0.0)) return c10::nullopt;
+    // updated where it lies: bf16 windows, and a memory whose rows are read and written in 16-byte pieces
     if (in_place)
         for (int i = 0; i < 4; ++i)
-            if (!state[i].is_contiguous() || (i > 0 && state[i].scalar_type() != at::kBFloat16)) return c10::nullopt;
+            if (!state[i].is_contiguous() || (i > 0 ? state[i].scalar_type() != at::kBFloat16 : reinterpret_cast<uintptr_t>(state[i].data_ptr()) % 16 != 0))
+                return c10::nullopt;
     at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = dense(x_), nw = dense_as(w[kNorm], at::kFloat);
+    const Tensor x = aligned(dense(x_)), nw = aligned(dense_as(w[kNorm], at::kFloat));
     void* st = stream_of(x);
     const int64_t h = z.hid, M = z.M, n = z.n;
     const size_t act = 2 * (size_t)(M * h);
@@ -467,7 +479,7 @@ LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
                            (float)eps, state[0].data_ptr<float>(), state[0].data_ptr<float>(), mixed, st),
              "kda_token_mix");
     } else {
-        const Tensor mem_in = dense(state[0]), mem = empty_as(mem_in);
+        const Tensor mem_in = aligned(dense(state[0])), mem = empty_as(mem_in);
         out.push_back(mem);
         const void *xp[3], *wp[3], *cp[3];
         void *yp[3], *fp[3];

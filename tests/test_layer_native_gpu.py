@@ -97,3 +97,97 @@ def test_training_step_equals_the_modules(batch, T, heads, carried, wdtype):
             assert (a - b).abs().max() <= 5e-2 * b.abs().max() + 2e-2, n
         else:
             assert O.rel_l2(a.float(), b.float()) <= 2e-2, n
+
+
+def _shifted(t):
+    """The same values one element into a larger buffer: dense, at an address that allows no 16-byte access."""
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    view = flat[1:].view(t.shape).copy_(t.detach())
+    assert view.data_ptr() % 16 != 0
+    return view
+
+
+def _shifted_state(state):
+    from experiment_swa_kda_b200 import KDAState
+    return KDAState(*[_shifted(t) for t in (state.memory, state.q_conv, state.k_conv, state.v_conv)])
+
+
+def _shift_vectors(layer):
+    """dt_bias, the norm weight and the taps as a flat parameter buffer behind a 3-element A_log would hold them."""
+    for p in (layer.dt_bias, layer.o_norm.weight, layer.q_conv1d.weight, layer.k_conv1d.weight, layer.v_conv1d.weight):
+        p.data = _shifted(p.data)
+    assert layer._plain_weights() is not None
+    return layer
+
+
+# few rows straight from the parameters and packed ones, with and without an incoming state; the convolutions in the kernel
+@pytest.mark.parametrize("T,carried,fuse", [(5, False, False), (5, True, False), (70, True, False), (70, False, True)])
+def test_prefill_with_tensors_at_odd_addresses(T, carried, fuse):
+    gen = torch.Generator().manual_seed(T)
+    layer, x, results = _layer(3, 2), torch.randn(2, T, 384, generator=gen).bfloat16().to(D0), []
+    layer.fuse_prefill_conv = fuse
+    state = _state(2, 3, gen) if carried else None
+    for put in (False, True):
+        if put:
+            layer, x, state = _shift_vectors(layer), _shifted(x), _shifted_state(state) if carried else None
+        with torch.no_grad():
+            y, st = layer(x, state=state, output_final_state=True)
+        results.append((y, st.memory, st.q_conv, st.k_conv, st.v_conv))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("carried", [False, True])
+def test_training_step_with_tensors_at_odd_addresses(carried):
+    from experiment_swa_kda_b200 import KDAState
+    gen = torch.Generator().manual_seed(9)
+    layer, x = _layer(3, 2), torch.randn(2, 70, 384, generator=gen).bfloat16().to(D0)
+    dy, init, results = torch.randn(2, 70, 384, generator=gen).bfloat16().to(D0), _state(2, 3, gen), []
+    for put in (lambda t: t.clone(), _shifted):
+        if put is _shifted:
+            _shift_vectors(layer)
+        xs = put(x).requires_grad_(True)
+        parts = [put(t).requires_grad_(True) for t in (init.memory, init.q_conv, init.k_conv, init.v_conv)] if carried else []
+        y, st = layer(xs, state=KDAState(*parts) if carried else None, output_final_state=carried)
+        outs = [y] + ([st.memory, st.q_conv, st.k_conv, st.v_conv] if carried else [])
+        results.append([*outs, *torch.autograd.grad(outs, [xs, *layer.parameters(), *parts], [put(dy)] + [put(t.detach()) for t in outs[1:]])])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_token_step_with_tensors_at_odd_addresses():
+    """A memory at an odd address cannot be stepped by the fused kernel: the call is declined before anything has moved and
+    runs module by module, so the windows advance once."""
+    gen = torch.Generator().manual_seed(8)
+    layer, x, state = _layer(3, 1), torch.randn(2, 1, 384, generator=gen).bfloat16().to(D0), _state(2, 3, gen)
+    aligned, shifted = state.clone(), _shifted_state(state)
+    want = layer.decode_token(x, aligned)
+    with torch.no_grad():
+        y, st = layer(_shifted(x), state=shifted, output_final_state=True, mode="project_recurrent")
+    assert torch.equal(y, want) and torch.equal(st.memory, aligned.memory) and torch.equal(st.q_conv, aligned.q_conv)
+    got = _shift_vectors(layer).decode_token(_shifted(x), shifted)
+    assert O.rel_l2(got.float(), want.float()) <= 1e-2
+    for a, b in ((shifted.memory, aligned.memory), (shifted.q_conv, aligned.q_conv), (shifted.k_conv, aligned.k_conv), (shifted.v_conv, aligned.v_conv)):
+        assert O.rel_l2(a.float(), b.float()) <= 1e-2
+    whole = aligned.clone()       # everything but the memory at odd addresses: the fused step, to the bit
+    odd = _shifted_state(aligned)
+    odd.memory = aligned.memory.clone()
+    assert torch.equal(layer.decode_token(x, whole), layer.decode_token(_shifted(x), odd))
+    assert torch.equal(whole.memory, odd.memory) and torch.equal(whole.v_conv, odd.v_conv)
+
+
+# three convolutions of 21,845 sequences fill a grid; one more sequence runs module by module, forward and backward
+@pytest.mark.parametrize("batch", [21845, 21846])
+def test_more_sequences_than_the_batched_convolutions_grid_holds(batch):
+    gen = torch.Generator().manual_seed(batch)
+    layer = _layer(1, 4)
+    x = torch.randn(batch, 1, 128, generator=gen).bfloat16().to(D0).requires_grad_(True)
+    dy = torch.randn(batch, 1, 128, generator=gen).bfloat16().to(D0)
+    results = []
+    for _ in range(2):
+        with torch.no_grad():
+            y0, _ = layer(x)
+        y, _ = layer(x)
+        assert O.rel_l2(y0.float(), y.detach().float()) <= 1e-2
+        results.append((y, *torch.autograd.grad(y, [x, layer.q_proj.weight, layer.v_conv1d.weight], dy)))
+        _modules_one_by_one(layer)
+    for a, b in zip(*results):
+        assert O.rel_l2(a.detach().float(), b.detach().float()) <= 2e-2
