@@ -27,6 +27,21 @@ inline bool on(const Tensor& t, const Tensor& like) { return t.is_cuda() && t.de
 inline Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 inline Tensor dense_as(const Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? dense(t) : t.to(type).contiguous(); }
 
+// The nodes below are reverse-mode only: a dual tensor's tangent is refused, not dropped.
+inline void refuse_tangent(const Tensor& t) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "KDA operators have no forward-mode derivative");
+}
+inline void refuse_tangent(const OptTensor& t) {
+    if (has(t)) refuse_tangent(*t);
+}
+inline void refuse_tangent(const std::vector<Tensor>& ts) {
+    for (const auto& t : ts) refuse_tangent(t);
+}
+template <class... Ts>
+void refuse_tangents(const Ts&... ts) {
+    (refuse_tangent(ts), ...);
+}
+
 // A backward node: saved inputs, released with the graph.  Derived classes hold their sizes as plain fields.
 struct HostNode : public Node {
     std::vector<SavedVariable> saved;

@@ -146,6 +146,7 @@ struct ChunkOut {
 
 ChunkOut run_chunk(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, const OptTensor& h0_,
                    bool want_final, const OptTensor& cu_, double scale, bool l2norm, int lane, const Dims& d) {
+    refuse_tangents(q_, k_, v_, g_, beta_, h0_);
     const bool tracked = torch::autograd::compute_requires_grad(q_, k_, v_, g_, beta_, has(h0_) ? *h0_ : Tensor());
     c10::cuda::CUDAGuard guard(q_.device());
     watch_status(q_.device().index());
@@ -232,6 +233,7 @@ ChunkResult chunk_kda_norm(const Tensor& q_, const Tensor& k_, const Tensor& v_,
     if (!chunk_dims(q_, k_, v_, g_, beta_, h0_, cu_, d) || !tc_shape(q_, d)) return c10::nullopt;
     if (gate_.sizes() != v_.sizes() || nw_.dim() != 1 || nw_.numel() != d.V || !on(gate_, q_) || !on(nw_, q_)) return c10::nullopt;
     const double sc = scale.has_value() ? *scale : 1.0 / std::sqrt((double)d.K);
+    refuse_tangents(q_, k_, v_, g_, beta_, gate_, nw_, h0_);
     const bool tracked = torch::autograd::compute_requires_grad(q_, k_, v_, g_, beta_, gate_, nw_, has(h0_) ? *h0_ : Tensor());
     c10::cuda::CUDAGuard guard(q_.device());
     watch_status(q_.device().index());
@@ -308,6 +310,7 @@ TensorPair gate(const Tensor& raw_, const Tensor& bl_, const Tensor& A_, const T
         return c10::nullopt;
     const int64_t B = raw_.size(0), T = raw_.size(1), H = raw_.size(2), K = raw_.size(3);
     if (A_.numel() != H || bias_.numel() != H * K || B * T >= (int64_t(1) << 31)) return c10::nullopt;
+    refuse_tangents(raw_, bl_, A_, bias_);
     const bool tracked = torch::autograd::compute_requires_grad(raw_, bl_, A_, bias_);
     c10::cuda::CUDAGuard guard(raw_.device());
     Tensor g, beta, raw, bl, A, bias;
@@ -434,6 +437,7 @@ ChunkResult conv(const Tensor& x_, const Tensor& w_, const OptTensor& s0_, bool 
     const int64_t want[3] = {B, C, W};
     if (B * T >= (int64_t(1) << 31) || C >= (int64_t(1) << 31)) return c10::nullopt;
     if (has(s0_) && (s0_->sizes() != at::IntArrayRef(want, 3) || !on(*s0_, x_))) return c10::nullopt;
+    refuse_tangents(x_, w_, s0_);
     const bool tracked = torch::autograd::compute_requires_grad(x_, w_, has(s0_) ? *s0_ : Tensor());
     c10::cuda::CUDAGuard guard(x_.device());
     Tensor x, w, s0, y;
@@ -525,6 +529,7 @@ c10::optional<std::vector<Tensor>> conv_multi(const std::vector<Tensor>& xs_, co
             return c10::nullopt;
     const int64_t B = x0.size(0), T = x0.size(1), C = x0.size(2), W = ws_[0].numel() / C;
     if (W == 0 || B * T >= (int64_t(1) << 31)) return c10::nullopt;
+    refuse_tangents(xs_, ws_);
     bool tracked = false;
     for (size_t i = 0; i < n; ++i) tracked = tracked || torch::autograd::compute_requires_grad(xs_[i], ws_[i]);
     c10::cuda::CUDAGuard guard(x0.device());
@@ -595,6 +600,7 @@ OptTensor rmsnorm(const Tensor& x_, const Tensor& gate_, const Tensor& w_, doubl
     if (x_.dim() < 1 || x_.numel() == 0 || !x_.is_cuda() || !is_io(x_) || !on(gate_, x_) || !on(w_, x_) || gate_.sizes() != x_.sizes()) return c10::nullopt;
     const int64_t D = x_.size(-1), rows = x_.numel() / D;
     if (w_.numel() != D) return c10::nullopt;
+    refuse_tangents(x_, gate_, w_);
     const bool tracked = torch::autograd::compute_requires_grad(x_, gate_, w_);
     c10::cuda::CUDAGuard guard(x_.device());
     Tensor x, gate, w, y, inv;

@@ -316,6 +316,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
                   bool want_state, bool fuse_conv) {
     Sizes z;
     if (!layer_sizes(x_, w, heads, state, z) || !(lb >= -5.0 && lb < 0.0)) return c10::nullopt;
+    refuse_tangents(x_, w, state);
     bool tracked = torch::autograd::compute_requires_grad(x_);
     for (const auto& t : w) tracked = tracked || torch::autograd::compute_requires_grad(t);
     for (const auto& t : state) tracked = tracked || torch::autograd::compute_requires_grad(t);
@@ -445,6 +446,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
 LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads, double eps, double lb, const std::vector<Tensor>& state, bool in_place) {
     Sizes z;
     if (state.size() != 4 || !layer_sizes(x_, w, heads, state, z) || z.T != 1 || z.M > kFewRows || !(lb >= -5.0 && lb < 0.0)) return c10::nullopt;
+    if (!in_place) refuse_tangents(x_, w, state);
     // updated where it lies: bf16 windows, and a memory whose rows are read and written in 16-byte pieces
     if (in_place)
         for (int i = 0; i < 4; ++i)
