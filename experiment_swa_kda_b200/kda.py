@@ -176,6 +176,10 @@ def chunk_kda(q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor, *, initi
     lane_id = _LANES.get(lane)
     if lane_id is not None and q.is_cuda:
         out = _native.load().chunk_kda(q, k, v, g, beta, initial_state, bool(output_final_state), cu_seqlens, scale, bool(use_qk_l2norm), lane_id)
+        if out is None:
+            out = ops.traced(lambda q, k, v, g, beta, h0, cu: _native.load().chunk_kda(q, k, v, g, beta, h0, bool(output_final_state), cu, scale,
+                                                                                       bool(use_qk_l2norm), lane_id),
+                             (q, k, v, g, beta, initial_state, cu_seqlens))
         if out is not None:
             return out
     # not the plain valid case: say why
@@ -217,6 +221,11 @@ def chunk_kda_norm(q: Tensor, k: Tensor, v: Tensor, g: Tensor, beta: Tensor, gat
     if q.is_cuda:
         out = _native.load().chunk_kda_norm(q, k, v, g, beta, gate, norm_weight, eps, initial_state, bool(output_final_state), cu_seqlens,
                                             scale, bool(use_qk_l2norm))
+        if out is None:
+            out = ops.traced(lambda q, k, v, g, beta, gate, w, h0, cu: _native.load().chunk_kda_norm(q, k, v, g, beta, gate, w, eps, h0,
+                                                                                                     bool(output_final_state), cu, scale,
+                                                                                                     bool(use_qk_l2norm)),
+                             (q, k, v, g, beta, gate, norm_weight, initial_state, cu_seqlens))
         if out is not None:
             return out
     n_states = _packed_states(q, cu_seqlens)
@@ -268,6 +277,10 @@ def kda(q: Tensor, k: Tensor, v: Tensor, raw_gate: Tensor, beta_logits: Tensor, 
     if mode == "project_chunk" and lane_id is not None and q.is_cuda:
         out = _native.load().kda_raw(q, k, v, raw_gate, beta_logits, A_log, dt_bias, initial_state, bool(output_final_state), lower_bound,
                                      scale, cu_seqlens, lane_id)
+        if out is None:
+            out = ops.traced(lambda q, k, v, raw, bl, A, bias, h0, cu: _native.load().kda_raw(q, k, v, raw, bl, A, bias, h0, bool(output_final_state),
+                                                                                              lower_bound, scale, cu, lane_id),
+                             (q, k, v, raw_gate, beta_logits, A_log, dt_bias, initial_state, cu_seqlens))
         if out is not None:
             return out
     n_states = None if cu_seqlens is None else cu_seqlens.numel() - 1

@@ -8,6 +8,7 @@ ctypes are its thin binding for callers that manage workspaces themselves.
 
 from __future__ import annotations
 
+import contextlib
 from typing import Optional, Tuple
 
 import torch
@@ -50,6 +51,68 @@ def _need_cuda(*ts):
 
 def _bytes(n: int, dev) -> Tensor:
     return torch.empty(max(int(n), 256), dtype=torch.uint8, device=dev)
+
+
+# --------------------------------------------------------------------------------------------
+# torch.jit traces
+# --------------------------------------------------------------------------------------------
+
+@contextlib.contextmanager
+def _untraced():
+    state = torch._C._get_tracing_state()
+    torch._C._set_tracing_state(None)
+    try:
+        yield
+    finally:
+        torch._C._set_tracing_state(state)
+
+
+class _TracedCall(torch.autograd.Function):
+    """A native call as one node of a trace: the tracer records Python autograd functions, and the C++ graph that the call
+    builds is kept inside and differentiated by the backward."""
+
+    @staticmethod
+    def forward(ctx, call, *tensors):
+        with _untraced(), torch.enable_grad():
+            leaves = [t.detach().requires_grad_(wanted) for t, wanted in zip(tensors, ctx.needs_input_grad[1:])]
+            outs = call(*leaves)
+            like = [(tuple(o.shape), o.dtype, o.device) for o in outs]
+        ctx.inner = leaves, outs
+        results = tuple(torch.empty(shape, dtype=dtype, device=device) for shape, dtype, device in like)      # the tracer has to have seen them
+        with _untraced():
+            for r, o in zip(results, outs):
+                r.copy_(o)
+        return results
+
+    @staticmethod
+    def backward(ctx, *grads):
+        leaves, outs = ctx.inner
+        pairs = [(o, g) for o, g in zip(outs, grads) if o.requires_grad]
+        wanted = [t for t in leaves if t.requires_grad]
+        got = iter(torch.autograd.grad([o for o, _ in pairs], wanted, [g for _, g in pairs], retain_graph=True, allow_unused=True))
+        return (None, *[next(got) if t.requires_grad else None for t in leaves])
+
+
+def traced(call, tensors):
+    """call(*tensors) -> tuple of tensors and Nones, as one node of the torch.jit trace in progress.  None outside of a trace,
+    and where the call itself declines its inputs (answers None)."""
+    if torch._C._get_tracing_state() is None:
+        return None
+    at = [i for i, t in enumerate(tensors) if t is not None]
+
+    def bound(*given):
+        full = [None] * len(tensors)
+        for i, t in zip(at, given):
+            full[i] = t
+        return call(*full)
+
+    given = [tensors[i] for i in at]
+    with _untraced(), torch.no_grad():
+        first = bound(*given)
+    if first is None:
+        return None
+    outs = iter(_TracedCall.apply(lambda *ts: [o for o in bound(*ts) if o is not None], *given))
+    return tuple(None if o is None else next(outs) for o in first)
 
 
 # --------------------------------------------------------------------------------------------
@@ -170,6 +233,8 @@ class GateFunction:
     @staticmethod
     def apply(raw_gate, beta_logits, A_log, dt_bias, lower_bound):
         out = _native.load().gate(raw_gate, beta_logits, A_log, dt_bias, lower_bound)
+        if out is None:
+            out = traced(lambda *ts: _native.load().gate(*ts, lower_bound), (raw_gate, beta_logits, A_log, dt_bias))
         if out is None:
             _need_cuda(raw_gate, beta_logits, A_log, dt_bias)
             _dt(raw_gate)
@@ -331,6 +396,8 @@ class ConvMultiFunction:
     def apply(silu, n, *tensors):
         xs, ws = list(tensors[:n]), list(tensors[n:])
         ys = _native.load().conv_multi(xs, ws, bool(silu))
+        if ys is None:
+            ys = traced(lambda *ts: _native.load().conv_multi(list(ts[:n]), list(ts[n:]), bool(silu)), tensors)
         return tuple(ys) if ys is not None else tuple(conv(x, w, None, False, silu)[0] for x, w in zip(xs, ws))
 
 
@@ -338,6 +405,8 @@ def conv(x, weight, initial_state, output_final_state, silu=True):
     """Causal depthwise convolution (+ SiLU) with an explicit cache, differentiable (role of the reference's
     _ProjectConvolutionAutograd, nanochat/mixers/kda.py:439-466).  weight [C,W] or [C,1,W]."""
     out = _native.load().conv(x, weight, initial_state, bool(output_final_state), bool(silu))
+    if out is None:
+        out = traced(lambda *ts: _native.load().conv(*ts, bool(output_final_state), bool(silu)), (x, weight, initial_state))
     if out is None:
         _need_cuda(x, weight, initial_state)
         _dt(x)
@@ -382,6 +451,8 @@ def rmsnorm_gated(x, gate, weight, eps):
     """y = rms_norm(x; w, eps) * sigmoid(gate), differentiable
     (role of the reference's _ProjectRMSNormGateAutograd, nanochat/mixers/kda.py:418-436)."""
     y = _native.load().rmsnorm(x, gate, weight, eps)
+    if y is None:
+        y, = traced(lambda *ts: None if (out := _native.load().rmsnorm(*ts, eps)) is None else (out,), (x, gate, weight)) or (None,)
     if y is None:
         _need_cuda(x, gate, weight)
         _dt(x)

@@ -1,6 +1,7 @@
 // Helpers of the native host path and the base of its backward nodes.
 #pragma once
 
+#include <ATen/TracerMode.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -26,6 +27,10 @@ inline int wflag(const Tensor& x, const Tensor& w) {
 inline bool on(const Tensor& t, const Tensor& like) { return t.is_cuda() && t.device() == like.device(); }
 inline Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 inline Tensor dense_as(const Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? dense(t) : t.to(type).contiguous(); }
+
+// A torch.jit trace records dispatched operators and Python autograd functions, not these calls: inside one the entries
+// answer None, and the Python side makes the call through an autograd function (ops.traced) that the tracer can see.
+inline bool tracing() { return at::tracer::impl::is_dispatch_enabled(); }
 
 // The nodes below are reverse-mode only: a dual tensor's tangent is refused, not dropped.
 inline void refuse_tangent(const Tensor& t) {

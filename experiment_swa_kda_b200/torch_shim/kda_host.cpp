@@ -59,7 +59,7 @@ struct Dims {
 // The plain valid case of chunk_kda's inputs (raw: kda's, whose activations must be bf16 and whose gate is raw).
 bool chunk_dims(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const OptTensor& h0, const OptTensor& cu,
                 Dims& d) {
-    if (q.dim() != 4 || v.dim() != 4 || beta.dim() != 3 || !q.is_cuda()) return false;
+    if (tracing() || q.dim() != 4 || v.dim() != 4 || beta.dim() != 3 || !q.is_cuda()) return false;
     if (k.sizes() != q.sizes() || g.sizes() != q.sizes() || v.sizes().slice(0, 3) != q.sizes().slice(0, 3) || beta.sizes() != q.sizes().slice(0, 3))
         return false;
     d = Dims{q.size(0), q.size(1), q.size(2), q.size(3), v.size(3), q.size(0)};
@@ -305,7 +305,7 @@ using TensorPair = c10::optional<std::tuple<Tensor, Tensor>>;
 
 // (raw gate, beta logits, A_log, dt_bias) -> (g, beta) in float32
 TensorPair gate(const Tensor& raw_, const Tensor& bl_, const Tensor& A_, const Tensor& bias_, double lb) {
-    if (raw_.dim() != 4 || bl_.dim() != 3 || bl_.sizes() != raw_.sizes().slice(0, 3) || !raw_.is_cuda() || !on(bl_, raw_) || !on(A_, raw_) ||
+    if (tracing() || raw_.dim() != 4 || bl_.dim() != 3 || bl_.sizes() != raw_.sizes().slice(0, 3) || !raw_.is_cuda() || !on(bl_, raw_) || !on(A_, raw_) ||
         !on(bias_, raw_) || !is_io(raw_))
         return c10::nullopt;
     const int64_t B = raw_.size(0), T = raw_.size(1), H = raw_.size(2), K = raw_.size(3);
@@ -431,7 +431,7 @@ struct ConvNode : public HostNode {
 
 // x [B,T,C], weight [C,1,W] or [C,W], state [B,C,W] or none
 ChunkResult conv(const Tensor& x_, const Tensor& w_, const OptTensor& s0_, bool want_final, bool silu) {
-    if (x_.dim() != 3 || !x_.is_cuda() || !is_io(x_) || !on(w_, x_) || w_.dim() < 2 || w_.size(0) != x_.size(2) || w_.numel() == 0 || x_.numel() == 0)
+    if (tracing() || x_.dim() != 3 || !x_.is_cuda() || !is_io(x_) || !on(w_, x_) || w_.dim() < 2 || w_.size(0) != x_.size(2) || w_.numel() == 0 || x_.numel() == 0)
         return c10::nullopt;
     const int64_t B = x_.size(0), T = x_.size(1), C = x_.size(2), W = w_.numel() / C;
     const int64_t want[3] = {B, C, W};
@@ -520,7 +520,7 @@ struct ConvMultiNode : public HostNode {
 
 c10::optional<std::vector<Tensor>> conv_multi(const std::vector<Tensor>& xs_, const std::vector<Tensor>& ws_, bool silu) {
     const size_t n = xs_.size();
-    if (n < 1 || n > 4 || ws_.size() != n) return c10::nullopt;
+    if (tracing() || n < 1 || n > 4 || ws_.size() != n) return c10::nullopt;
     const Tensor& x0 = xs_[0];
     if (x0.dim() != 3 || !x0.is_cuda() || !is_io(x0) || x0.numel() == 0) return c10::nullopt;
     for (size_t i = 0; i < n; ++i)
@@ -597,7 +597,7 @@ struct NormNode : public HostNode {
 };
 
 OptTensor rmsnorm(const Tensor& x_, const Tensor& gate_, const Tensor& w_, double eps) {
-    if (x_.dim() < 1 || x_.numel() == 0 || !x_.is_cuda() || !is_io(x_) || !on(gate_, x_) || !on(w_, x_) || gate_.sizes() != x_.sizes()) return c10::nullopt;
+    if (tracing() || x_.dim() < 1 || x_.numel() == 0 || !x_.is_cuda() || !is_io(x_) || !on(gate_, x_) || !on(w_, x_) || gate_.sizes() != x_.sizes()) return c10::nullopt;
     const int64_t D = x_.size(-1), rows = x_.numel() / D;
     if (w_.numel() != D) return c10::nullopt;
     refuse_tangents(x_, gate_, w_);

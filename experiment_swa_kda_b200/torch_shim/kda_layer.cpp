@@ -258,7 +258,7 @@ struct LayerNode : public HostNode {
 // projections, read as they are) or copied where it is not (the input, the vectors, the taps, the incoming memory), and
 // the convolutions' grid limits are tested by fits_grid.
 bool layer_sizes(const Tensor& x, const std::vector<Tensor>& w, int64_t heads, const std::vector<Tensor>& state, Sizes& z) {
-    if (w.size() != kParams || x.dim() != 3 || !x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.numel() == 0 || heads < 1) return false;
+    if (tracing() || w.size() != kParams || x.dim() != 3 || !x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.numel() == 0 || heads < 1) return false;
     z.B = x.size(0), z.T = x.size(1), z.H = heads, z.M = z.B * z.T, z.hid = heads * kHead;
     z.pad = (8 - heads % 8) % 8;
     z.n = 4 * z.hid + kHead + heads + z.pad;

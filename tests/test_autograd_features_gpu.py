@@ -43,3 +43,26 @@ def test_forward_mode_is_refused(name, tracked):
     with fw.dual_level(), pytest.raises(RuntimeError, match="forward-mode|forward AD"):
         call(fw.make_dual(a.clone().requires_grad_(tracked), torch.ones_like(a)))
     call(a)      # outside of the level the same call runs
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("tracked", [False, True])
+@pytest.mark.parametrize("name", NAMES)
+def test_a_traced_call_follows_its_inputs(name, tracked):
+    """torch.jit.trace of a call, run on other inputs, equals the call; so do its gradients."""
+    call, a = _calls()[name]
+    if name in ("conv", "convs", "norm", "layer"):      # parameters in a closure are constants that the tracer takes without gradients only
+        for cell in call.__closure__:
+            if isinstance(cell.cell_contents, torch.nn.Module):
+                cell.cell_contents.requires_grad_(False)
+    with torch.set_grad_enabled(tracked):
+        other = (a * 0.5 + 1).to(a.dtype).requires_grad_(tracked)
+        trace = torch.jit.trace(call, (a.clone().requires_grad_(tracked),), check_trace=False)
+        got, want = trace(other), call(other)
+        assert torch.equal(got, want)
+        if tracked:
+            dy = torch.randn(want.shape, generator=torch.Generator().manual_seed(1)).to(D0, want.dtype)
+            assert torch.equal(*(torch.autograd.grad(o, other, dy)[0] for o in (got, want))) or name == "layer"
+            for o in (got, want):
+                assert o.requires_grad
+    call(a)
