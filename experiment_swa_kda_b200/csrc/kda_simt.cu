@@ -441,6 +441,19 @@ __global__ void __launch_bounds__(256, 3) intra_fwd_kernel(Ws w, IntraArgs p) {
         for (int r = 0; r < 8; ++r) far = far || !(fabsf(L[r] - c) <= kMaxExponent);
         const bool pairwise = __syncthreads_or(far);           // every warp has read the block sums and the rows' g
         if (!(warp & 1)) cref[I * kHalf + lane] = pre + c;
+        {
+            // e^{G_end - G} from the rows' own sum to the chunk's end: G_end and G are both as large as the chunk's whole decay
+            // (300 at the gate's lowest), and their difference keeps that size's rounding, 1e-5 of the last tokens' weight in
+            // the state.  g once more (L1): eight registers to hold it would cost the third CTA.
+            float run = 0.f;
+            for (int J = 7; J > warp; --J) run += bsum[J * kHalf + lane];
+            float* ed = w.Ed + (ch * 64 + i0) * Kp + dd;
+#pragma unroll
+            for (int r = 7; r >= 0; --r) {
+                ed[(size_t)r * Kp] = expf(run);
+                run += (i0 + r < len && in) ? ld_io(p.g, col + (size_t)(i0 + r) * rstep, p.gbf16) : 0.f;
+            }
+        }
         __syncthreads();
         float kn[8];
         float* rt = w.RT + (ch * Kp + dd) * 64 + i0;           // R^T: 8 rows of this channel
@@ -577,10 +590,8 @@ __global__ void __launch_bounds__(256, 3) intra_fwd_kernel(Ws w, IntraArgs p) {
         for (int idx = tid; idx < 1024; idx += 256) {
             const int r = idx >> 4, c4 = (idx & 15) << 2;
             const float4 k4 = *reinterpret_cast<const float4*>(kn_g + (size_t)r * Kp + kt * 64 + c4);
-            const float4 g4 = *reinterpret_cast<const float4*>(G_g + (size_t)r * Kp + kt * 64 + c4);
-            const float4 e4 = *reinterpret_cast<const float4*>(ge + kt * 64 + c4);
-            *reinterpret_cast<float4*>(Es + r * kLD + c4) =
-                make_float4(k4.x * expf(e4.x - g4.x), k4.y * expf(e4.y - g4.y), k4.z * expf(e4.z - g4.z), k4.w * expf(e4.w - g4.w));
+            const float4 e4 = *reinterpret_cast<const float4*>(w.Ed + (ch * 64 + r) * Kp + kt * 64 + c4);
+            *reinterpret_cast<float4*>(Es + r * kLD + c4) = make_float4(k4.x * e4.x, k4.y * e4.y, k4.z * e4.z, k4.w * e4.w);
         }
         if (tid < 64) w.dec[ch * Kp + kt * 64 + tid] = expf(ge[kt * 64 + tid]);
         for (int k2 = 0; k2 < KT; ++k2) {
@@ -850,6 +861,7 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, d = tid & 63, I = tid >> 6;
     const float* kn_g = w.kn + ch * 64 * Kp;
     const float* G_g = w.G + ch * 64 * Kp;
+    const float* Ed_g = w.Ed + ch * 64 * Kp;
     const float* qn_g = w.qn + ch * 64 * Kp;
     const size_t vrow = (size_t)H * V, krow = (size_t)H * K;
     if (tid < 64) {
@@ -883,11 +895,10 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
             ld_tile_io<true>(t0, p.d_o, p.bf16, voff, vrow, len, nc, p.vec_v);
             float e[16];
             auto source_col = [&](int kt) {      // column of E^T
-                const float ge = G_g[(size_t)63 * Kp + kt * 64 + d];
 #pragma unroll
                 for (int r = 0; r < 16; ++r) {
                     const size_t o = (size_t)(16 * I + r) * Kp + kt * 64 + d;
-                    e[r] = kn_g[o] * expf(ge - G_g[o]);
+                    e[r] = kn_g[o] * Ed_g[o];
                 }
             };
             source_col(0);
@@ -979,18 +990,17 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
             }
         }
         {
-            const float4 e4 = *reinterpret_cast<const float4*>(G_g + (size_t)63 * Kp + kt * 64 + 4 * tx);
-            const float ea[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const size_t o = (size_t)(4 * ty + r) * Kp + kt * 64 + 4 * tx;
                 const float4 g4 = *reinterpret_cast<const float4*>(G_g + o), q4 = *reinterpret_cast<const float4*>(qn_g + o),
-                             k4 = *reinterpret_cast<const float4*>(kn_g + o);
-                const float ga[4] = {g4.x, g4.y, g4.z, g4.w}, qa[4] = {q4.x, q4.y, q4.z, q4.w}, ka[4] = {k4.x, k4.y, k4.z, k4.w};
+                             k4 = *reinterpret_cast<const float4*>(kn_g + o), e4 = *reinterpret_cast<const float4*>(Ed_g + o);
+                const float ga[4] = {g4.x, g4.y, g4.z, g4.w}, qa[4] = {q4.x, q4.y, q4.z, q4.w}, ka[4] = {k4.x, k4.y, k4.z, k4.w},
+                            ea[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     acc[r][c] *= expf(ga[c]);                  // dq = dR e^G
-                    dk[r][c] *= expf(ea[c] - ga[c]);           // dE e^{G_end - G}
+                    dk[r][c] *= ea[c];                         // dE e^{G_end - G}
                     const float eE = dk[r][c] * ka[c];
                     dG[r][c] = acc[r][c] * qa[c] - eE;
                     colE[c] += eE;

@@ -11,8 +11,9 @@ namespace simt {
 struct Ws {
     int *chunk_seq, *chunk_tok0, *chunk_len, *seq_chunk0;
     int* seq_order;             // [n_seq] sequences by falling chunk count: the order the state scans start them in
-    // float32 lane, per chunk-head.  R = qn e^G, E = kn e^{G_end - G}; ...T arrays are transposed
+    // float32 lane, per chunk-head.  R = qn e^G, E = kn Ed; ...T arrays are transposed
     float *kn, *G;              // [64][Kp]   unit k, cumulative log-decay
+    float* Ed;                  // [64][Kp]   e^{G_end - G}, from sums that start at the chunk's end
     float *qn, *Rm;             // [64][Kp]   scaled unit q; R - A W (backward only)
     float *W, *WT, *RT;         // [64][Kp], [Kp][64], [Kp][64]
     float* Z;                   // [64][Vp]   U after the intra-chunk step, Z after the output kernel
@@ -74,6 +75,7 @@ inline Ws carve_ws(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr) 
     const size_t bw = sh.forward_only ? 0 : big;      // arrays only a backward reads
     w.kn = c.take<float>(big * nch * 64 * w.Kp);
     w.G = c.take<float>(big * nch * 64 * w.Kp);
+    w.Ed = c.take<float>(big * nch * 64 * w.Kp);
     w.qn = c.take<float>(bw * nch * 64 * w.Kp);
     w.Rm = c.take<float>(bw * nch * 64 * w.Kp);
     w.W = c.take<float>(big * nch * 64 * w.Kp);

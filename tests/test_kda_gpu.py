@@ -134,6 +134,29 @@ def test_decay_past_the_factored_range_fp32(K, V, T):
     assert all(e <= 1e-4 for e in errs.values()), errs
 
 
+@pytest.mark.parametrize("K,V,T", [(64, 64, 128), (32, 48, 100), (128, 128, 128)])
+def test_tokens_at_a_chunks_end_keep_float32_weight_under_strong_decay(K, V, T):
+    """Gates over the whole of [-5, 0]: G_end is near -160, and its last tokens enter the state with e^(G_end - G), exponents near 0
+    that must not carry the rounding of G's size (1e-5).  An exponent x <= 0 rounded at its own size moves e^x by at most
+    |x| e^x 2^-24 < 2^-25; behind it are sums of up to 256 products, whose roundings add up like 16 (the square root) of 2^-24:
+    1e-6 relative L2 (measured: 0.7 to 5.6e-7; with e^(G_end - G) as a difference 1.5 to 2.2e-6)."""
+    d = O.make_inputs(1, T, 2, K, V, seed=K + T, with_state=True)
+    d["g"] = -5 * torch.sigmoid(2 * torch.randn(d["g"].shape, generator=torch.Generator().manual_seed(V)))
+    m = kda_mod()
+    x = {n: t.requires_grad_(True) for n, t in to_dev(d).items()}
+    o, s = m.chunk_kda(x["q"], x["k"], x["v"], x["g"], x["beta"], initial_state=x["h0"], output_final_state=True, lane="fp32")
+    gen = torch.Generator().manual_seed(K)
+    do, ds = torch.randn(o.shape, generator=gen), torch.randn(s.shape, generator=gen)
+    names = ["q", "k", "v", "g", "beta", "h0"]
+    grads = dict(zip(names, torch.autograd.grad((o, s), [x[n] for n in names], (do.to(dev()), ds.to(dev())))))
+    e = {n: x[n].detach().double().cpu().requires_grad_(True) for n in names}
+    eo, es = O.kda_recurrence(e["q"], e["k"], e["v"], e["g"], e["beta"], initial_state=e["h0"], compute_dtype=torch.float64)
+    want = dict(zip(names, torch.autograd.grad((eo, es), [e[n] for n in names], (do.double(), ds.double()))))
+    far = lambda a, b: ((a.double().cpu() - b).norm() / b.norm()).item()
+    errs = {"s": far(s, es), **{n: far(grads[n], want[n]) for n in ("k", "v", "beta", "h0")}}
+    assert all(v <= 1e-6 for v in errs.values()), errs
+
+
 # ---------------------------------------------------------------------------------- packed sequences
 def test_varlen_ragged_fp32():
     cu = [0, 5, 69, 69, 200, 263]       # includes an empty segment and ragged tails
