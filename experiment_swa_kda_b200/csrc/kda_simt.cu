@@ -335,8 +335,10 @@ __device__ void unit_lower_inverse(const float* Ms, float* Ts, float* tmp) {
 // so that the masked products are plain tile products.  Within the block both exponents are at most eight tokens' decay
 // (40 at the gate's lowest), for earlier sources the factor only shrinks.  The blocks' sums are kept apart from the prefix
 // (L, counted from the block's first row), so a factor's exponent is rounded at its own size, not at G's.  A chunk whose
-// decay exceeds kMaxExponent inside a block takes the pairwise exponentials instead (log-decays below -10 per token).
-constexpr float kMaxExponent = 80.f;
+// decay exceeds kMaxExponent inside a block takes the pairwise exponentials instead (log-decays below -5.5 per token).  The
+// line lies just above the gate's 40: sums of cotangents times a source's factor are formed before the target's factor
+// brings them down, and from e^44 = 1e19 they have another 1e19 to float32's end (from e^80, 6e3: gradients of 1e4 overflowed).
+constexpr float kMaxExponent = 44.f;
 constexpr int kSrcCols = 16 + 32 + 48 + 64;
 // source array of block I in the forward: [32 d][16 (I + 1)] with 4 floats of padding, after the two target stacks
 constexpr int kHalf = 32;

@@ -134,6 +134,27 @@ def test_decay_past_the_factored_range_fp32(K, V, T):
     assert all(e <= 1e-4 for e in errs.values()), errs
 
 
+@pytest.mark.parametrize("decay", [-5.4, -5.6, -9.5])
+@pytest.mark.parametrize("K,V,T", [(64, 64, 130), (128, 72, 63)])
+def test_large_cotangents_either_side_of_the_factored_range_fp32(K, V, T, decay):
+    """8 tokens of -5.4 leave e^43 (factored exponentials), of -5.6 e^45 (pairwise), of -9.5 e^76; cotangents of 1e7, as a scaled
+    loss gives, must not overflow between a source's factor and its target's.  Tolerance and slow channels as in the
+    test above: |G| <= 608."""
+    d = O.make_inputs(1, T, 2, K, V, seed=K + T, with_state=True)
+    d["g"][..., ::2] = decay
+    d["g"][..., 1::2] *= 0.1
+    m = kda_mod()
+    x = {n: t.requires_grad_(True) for n, t in to_dev(d).items()}
+    o, s = m.chunk_kda(x["q"], x["k"], x["v"], x["g"], x["beta"], initial_state=x["h0"], output_final_state=True, lane="fp32")
+    gen = torch.Generator().manual_seed(K)
+    do, ds = 1e7 * torch.randn(o.shape, generator=gen).to(dev()), 1e7 * torch.randn(s.shape, generator=gen).to(dev())
+    names = ["q", "k", "v", "g", "beta", "h0"]
+    grads = torch.autograd.grad((o, s), [x[n] for n in names], (do, ds))
+    eo, es, eg = oracle_grads({n: x[n] for n in names}, do, ds)
+    errs = {"o": O.rel_l2(o, eo), "s": O.rel_l2(s, es), **{"d" + n: O.rel_l2(gr, eg[n]) for n, gr in zip(names, grads)}}
+    assert all(v <= 1e-4 for v in errs.values()), errs
+
+
 @pytest.mark.parametrize("K,V,T", [(64, 64, 128), (32, 48, 100), (128, 128, 128)])
 def test_tokens_at_a_chunks_end_keep_float32_weight_under_strong_decay(K, V, T):
     """Gates over the whole of [-5, 0]: G_end is near -160, and its last tokens enter the state with e^(G_end - G), exponents near 0
