@@ -876,7 +876,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     a.dq = static_cast<__nv_bfloat16*>(dq); a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
     a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.scale = scale; a.status = t.status;
     auto kern = gbf16 ? tc_intra_bwd_kernel<true> : tc_intra_bwd_kernel<false>;
-    if (set_smem_limit(kern, kIntraBwdSmem)) return launch_status();
+    if (set_smem_limit(kern, kIntraBwdSmem)) return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_intra_bwd_kernel", st,
                kern<<<dim3(w.nslots, w.H), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, a));
     return launch_status();

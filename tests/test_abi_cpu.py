@@ -146,3 +146,16 @@ def test_forward_only_shapes_need_less_workspace_and_refuse_a_backward():
     bad = _lib.ChunkShape(2, 4096, 8192, 3, 128, 128, 1, 0, 1, 1, 0.0884, 7)
     assert lib.kda_chunk_fwd(bad, *([None] * 10), 0, None) == -1
     assert lib.kda_status_word_code(0) == 0 and lib.kda_status_word_code(10) == -7 and lib.kda_status_word_code(53) == -6
+
+
+def test_a_kernel_that_cannot_have_its_shared_memory_is_an_error():
+    """set_smem_limit can fail without a pending CUDA error (the device's limit is below the request); a launch site that answered
+    with the last CUDA error would then report success and skip its kernel."""
+    csrc = os.path.join(ROOT, "experiment_swa_kda_b200", "csrc")
+    found = []
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith(".cu"):
+            text = open(os.path.join(csrc, name)).read()
+            found += [(name, m.group(1)) for m in re.finditer(r"if \(set_smem(?:_limit)?\(.*?return ([^;]+);", text, re.S)]
+    assert len(found) >= 10
+    assert all(code == "KDA_ERR_CUDA" for _, code in found), found
