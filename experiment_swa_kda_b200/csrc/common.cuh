@@ -138,9 +138,11 @@ void end(cudaStream_t st);
     } while (0)
 
 // Dynamic shared memory limit of a kernel: the attribute is a driver call, so it is set once per kernel and device.
+// Kernels that share a signature share this function's statics; one past their number pays the driver calls every time.
+constexpr int kSmemKernels = 64;
 template <class Kern>
 inline int set_smem_limit(Kern kern, size_t bytes) {
-    constexpr int kDevices = 64, kKernels = 8;      // kernels that share a signature share this function's statics
+    constexpr int kDevices = 64, kKernels = kSmemKernels;
     static std::atomic<const void*> done[kDevices][kKernels];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return KDA_ERR_CUDA;

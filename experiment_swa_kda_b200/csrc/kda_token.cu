@@ -229,6 +229,8 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
     }
 }
 
+// 4 counts of row tiles x 2 weight types x with and without convolutions x 2 heights: one signature
+static_assert(kSmemKernels >= 4 * 2 * 2 * 2, "set_smem_limit would forget instantiations of rows_kernel");
 template <int NT, bool F32W, bool CONV, int RT>
 int launch_tile(const RowsArgs& p, cudaStream_t st) {
     constexpr size_t ring = (size_t)kDepth<RT> * RT * (F32W ? 4 : 2) * kWarps * 32 * 16, red = (size_t)kWarps * kRows * RT * (NT * 8 + 1) * 4;
