@@ -56,14 +56,26 @@ void bind_context(int device) {
     bound = device;
 }
 
+// torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction, as torch's own products take it; its third setting (no
+// split of k either) has no cuBLAS equivalent, and such a layer runs its modules.
+cublasMath_t product_math() {
+    return at::globalContext().allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK
+               ? CUBLAS_DEFAULT_MATH
+               : CUBLAS_MATH_DISALLOW_REDUCED_PRECISION_REDUCTION;
+}
+
 // Row-major products with row strides, bf16 operands and float32 accumulation.  cuBLAS directly: at::mm spends as long in
 // dispatch and views as the call itself takes, and these operands are slices.
 void gemm(cublasOperation_t ta, cublasOperation_t tb, int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, const void* b, int64_t ldb,
           void* c, int64_t ldc, at::ScalarType ctype) {
     const float one = 1.f, zero = 0.f;
-    const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), ta, tb, (int)m, (int)n, (int)k, &one, a, CUDA_R_16BF, (int)lda, b,
+    const cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();      // in the default mode, in which it goes back
+    const cublasMath_t math = product_math();
+    if (math != CUBLAS_DEFAULT_MATH) cublasSetMathMode(handle, math);
+    const cublasStatus_t rc = cublasGemmEx(handle, ta, tb, (int)m, (int)n, (int)k, &one, a, CUDA_R_16BF, (int)lda, b,
                                            CUDA_R_16BF, (int)ldb, &zero, c, ctype == at::kFloat ? CUDA_R_32F : CUDA_R_16BF, (int)ldc,
                                            CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+    if (math != CUBLAS_DEFAULT_MATH) cublasSetMathMode(handle, CUBLAS_DEFAULT_MATH);
     TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed (", (int)rc, ")");
 }
 // y [m][n] = x [m][k] w^T, w [n][k]
@@ -288,7 +300,8 @@ bool layer_sizes(const Tensor& x, const std::vector<Tensor>& w, int64_t heads, c
         for (int i = 1; i < 4; ++i)
             if (state[i].sizes() != at::IntArrayRef(win, 3) || !on(state[i], x)) return false;
     }
-    return !at::autocast::is_autocast_enabled(at::kCUDA);
+    return !at::autocast::is_autocast_enabled(at::kCUDA) &&
+           at::globalContext().allowBF16ReductionCuBLAS() != at::CuBLASReductionOption::DisallowReducedPrecisionDisallowSplitK;
 }
 
 // kda_conv_*_rows: `items` convolutions share a launch whose grid has items x batch and 64-token tiles as its y and z
@@ -562,6 +575,7 @@ void bind_layer(pybind11::module_& m) {
     m.def("layer", &layer, nogil());
     m.def("token", &token, nogil());
     m.def("plain_weights", &plain_weights);
+    m.def("product_math", [] { return (int)product_math(); });      // the mode the layer's products would run in now
 }
 
 }  // namespace kda_host

@@ -159,3 +159,16 @@ def test_a_kernel_that_cannot_have_its_shared_memory_is_an_error():
             found += [(name, m.group(1)) for m in re.finditer(r"if \(set_smem(?:_limit)?\(.*?return ([^;]+);", text, re.S)]
     assert len(found) >= 10
     assert all(code == "KDA_ERR_CUDA" for _, code in found), found
+
+
+def test_the_layers_products_follow_the_reduced_precision_setting():
+    """They call cuBLAS directly, where torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction is a mode of the handle:
+    0 by default, CUBLAS_MATH_DISALLOW_REDUCED_PRECISION_REDUCTION (16) when the user forbids bf16 reductions."""
+    from experiment_swa_kda_b200 import _native
+    flag = torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction
+    try:
+        for allowed, mode in ((True, 0), (False, 16)):
+            torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = allowed
+            assert _native.load().product_math() == mode
+    finally:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = flag
