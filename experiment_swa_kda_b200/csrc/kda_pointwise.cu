@@ -1579,7 +1579,9 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(long long rows, int D,
 //           dx = inv * (dn - n * mean(dn*n)).
 // dweight: every warp accumulates its rows into its own shared-memory row, the block sums the
 // eight rows in fixed order and writes one partial per block.
-template <bool BF16, bool VEC4>
+// What a launch writes: everything, or one half of it in a call that has no memory of its own for the partials.
+enum RmsParts { kRmsAll, kRmsWeight, kRmsInputs };
+template <bool BF16, bool VEC4, int PARTS>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(long long rows, int D, const void* __restrict__ x,
                                                           const void* __restrict__ gate, const float* __restrict__ w,
                                                           const float* __restrict__ inv_rms, const void* __restrict__ dy,
@@ -1627,20 +1629,25 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(long long rows, int D,
                     ox[e] = inv * (du * wa[e] - n * dot);
                     mine[d + e] += du * n;
                 }
-                st4<BF16>(dx, base + d, ox);
-                st4<BF16>(dgate, base + d, og);
+                if (PARTS != kRmsWeight) {
+                    st4<BF16>(dx, base + d, ox);
+                    st4<BF16>(dgate, base + d, og);
+                }
             }
         } else {
             for (int d = lane; d < D; d += 32) {
                 const float n = ld_io(x, base + d, BF16) * inv, s = sigmoid_t<BF16>(ld_io(gate, base + d, BF16));
                 const float gyv = ld_io(dy, base + d, BF16);
                 const float du = gyv * s;
-                st_io(dgate, base + d, BF16, gyv * n * w[d] * s * (1.f - s));
-                st_io(dx, base + d, BF16, inv * (du * w[d] - n * dot));
+                if (PARTS != kRmsWeight) {
+                    st_io(dgate, base + d, BF16, gyv * n * w[d] * s * (1.f - s));
+                    st_io(dx, base + d, BF16, inv * (du * w[d] - n * dot));
+                }
                 mine[d] += du * n;
             }
         }
     }
+    if (PARTS == kRmsInputs) return;
     __syncthreads();
     for (int d = threadIdx.x; d < D; d += 256) {
         float a = 0.f;
@@ -1698,7 +1705,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd128_kernel(long long rows, int
 
 // ROWS: gate and dgate are the [token][head][128] part of wider rows gate_ld elements apart (a slice of the layer's
 // projection), heads rows to a token.
-template <bool BF16, bool ROWS>
+template <bool BF16, bool ROWS, int PARTS = kRmsAll>
 __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, int heads, int gate_ld, const void* __restrict__ x,
                                                              const void* __restrict__ gate, const float* __restrict__ w,
                                                              const float* __restrict__ inv_rms, const void* __restrict__ dy,
@@ -1754,11 +1761,14 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, int
                     dwa[e] += du * n;
                 }
                 const size_t base = (size_t)(row0 + r) * 128 + 4 * lane;
-                st4<BF16>(dx, base, ox);
-                st4<BF16>(dgate, ROWS ? gate_at(row0 + r) : base, og);
+                if (PARTS != kRmsWeight) {
+                    st4<BF16>(dx, base, ox);
+                    st4<BF16>(dgate, ROWS ? gate_at(row0 + r) : base, og);
+                }
             }
         }
     }
+    if (PARTS == kRmsInputs) return;
 #pragma unroll
     for (int e = 0; e < 4; ++e) dws[wid][4 * lane + e] = dwa[e];
     __syncthreads();
@@ -2359,6 +2369,34 @@ extern "C" size_t kda_rmsnorm_gate_bwd_scratch_bytes(int64_t rows, int32_t dim) 
     return align_up((size_t)rms_blocks(rows > 0 ? rows : 1) * dim * sizeof(float), 256);
 }
 
+namespace {
+// part: one row of partials per block
+template <int PARTS>
+void rms_bwd_launch(int nb, int64_t rows, int32_t dim, int32_t io_dtype, const void* x, const void* gate, const float* weight, const float* inv_rms,
+                    const void* d_y, void* dx, void* dgate, float* part, cudaStream_t st) {
+    const size_t smem = (size_t)8 * dim * sizeof(float);
+    const bool vec = dim % 128 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(d_y) |
+                       reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate) | reinterpret_cast<uintptr_t>(weight)) % 16) == 0;
+    const bool bf16 = io_dtype == KDA_DTYPE_BF16;
+    if (vec && dim == 128) {
+        if (bf16) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<true, false, PARTS><<<nb, 256, 0, st>>>(rows, 1, 128, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+        else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false, false, PARTS><<<nb, 256, 0, st>>>(rows, 1, 128, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+    } else if (bf16) {
+        if (vec) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<true, true, PARTS><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+        else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<true, false, PARTS><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+    } else {
+        if (vec) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<false, true, PARTS><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+        else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<false, false, PARTS><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
+    }
+}
+void rms_dw_launch(int nb, int32_t dim, const float* part, float* dweight, cudaStream_t st) {
+    pw::ColumnSumItems outs = {};
+    outs.out[0] = dweight;
+    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(dim, 32), 1024, 0, st>>>(nb, dim, part, outs, 0));
+}
+}  // namespace
+
 extern "C" int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype, const void* x, const void* gate,
                                     const float* weight, const float* inv_rms, const void* d_y, void* dx, void* dgate,
                                     float* dweight, void* scratch, size_t scratch_bytes, void* stream) {
@@ -2369,25 +2407,8 @@ extern "C" int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype,
     cudaStream_t st = (cudaStream_t)stream;
     const int nb = rows > 0 ? rms_blocks(rows) : 0;
     float* part = static_cast<float*>(scratch);
-    const size_t smem = (size_t)8 * dim * sizeof(float);
-    const bool vec = dim % 128 == 0 &&
-                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(d_y) |
-                       reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate) | reinterpret_cast<uintptr_t>(weight)) % 16) == 0;
-    if (nb > 0 && vec && dim == 128) {
-        if (io_dtype == KDA_DTYPE_BF16) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<true, false><<<nb, 256, 0, st>>>(rows, 1, 128, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-        else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false, false><<<nb, 256, 0, st>>>(rows, 1, 128, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-    } else if (nb > 0) {
-        if (io_dtype == KDA_DTYPE_BF16) {
-            if (vec) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<true, true><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-            else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<true, false><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-        } else {
-            if (vec) KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<false, true><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-            else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<false, false><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
-        }
-    }
-    pw::ColumnSumItems outs = {};
-    outs.out[0] = dweight;
-    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(dim, 32), 1024, 0, st>>>(nb, dim, part, outs, 0));
+    if (nb > 0) rms_bwd_launch<pw::kRmsAll>(nb, rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, part, st);
+    rms_dw_launch(nb, dim, part, dweight, st);
     return launch_status();
 }
 
@@ -2418,30 +2439,29 @@ extern "C" int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t
 // weight gradient.  Some callers have nowhere to get one: code running against a frozen memory plan
 // (a serving engine that sized all of its device memory at start-up), a plugin that is handed tensors
 // but no allocator, or anything that must not call cudaMalloc because that call synchronises the
-// device.  For them the partials live in a fixed array inside the library image.
-namespace {
-constexpr int kStaticMaxDim = 256;                 // widest row the static variant accepts
-constexpr int kStaticMaxBlocks = 148 * 8;          // the backward never launches more blocks than this
-constexpr int kMaxDevices = 64;
-static __device__ __align__(256) float g_rms_static_scratch[(size_t)kStaticMaxBlocks * kStaticMaxDim];   // 1.2 MB per GPU
-float* g_rms_static_ptr[kMaxDevices] = {nullptr};  // device address of the array, per device ordinal
-}  // namespace
-
+// device.  For them dx holds the partials first - at most ceil(rows / 8) rows of dim floats, about a
+// quarter of it in bf16 and an eighth in float32 - and is written after they have been summed.  The
+// inputs are read twice for it; in return nothing is shared between calls, so they may overlap on
+// different streams and in graphs.  Up to 8 rows need no partials: their one block writes the
+// gradient itself.
 extern "C" int kda_rmsnorm_gate_bwd_static(int64_t rows, int32_t dim, int32_t io_dtype, const void* x, const void* gate,
                                            const float* weight, const float* inv_rms, const void* d_y, void* dx,
                                            void* dgate, float* dweight, void* stream) {
+    constexpr int kStaticMaxDim = 256;
     if (rows < 0 || dim <= 0) return KDA_ERR_BAD_SHAPE;
-    if (dim > kStaticMaxDim) return KDA_ERR_UNSUPPORTED;   // beyond the built-in scratch: use kda_rmsnorm_gate_bwd
-    int device = -1;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return KDA_ERR_CUDA;
-    if (g_rms_static_ptr[device] == nullptr) {
-        // In host code the array's name is only a handle; the kernels need its address on the current device.
-        void* p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_rms_static_scratch) != cudaSuccess || p == nullptr) return KDA_ERR_CUDA;
-        g_rms_static_ptr[device] = static_cast<float*>(p);
+    if (dim > kStaticMaxDim) return KDA_ERR_UNSUPPORTED;
+    if (!weight || !dweight) return KDA_ERR_NULL;
+    if (rows > 0 && (!x || !gate || !inv_rms || !d_y || !dx || !dgate)) return KDA_ERR_NULL;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (rows == 0) {
+        rms_dw_launch(0, dim, nullptr, dweight, st);
+        return launch_status();
     }
-    const size_t bytes = (size_t)kStaticMaxBlocks * kStaticMaxDim * sizeof(float);
-    return kda_rmsnorm_gate_bwd(rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, dweight,
-                                g_rms_static_ptr[device], bytes, stream);
+    const int nb = rms_blocks(rows);
+    // bf16 rows may start at an odd element, floats may not: 2 bytes of slack, and more than 8 rows have room for it
+    float* part = nb == 1 ? dweight : reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(dx) + 3) / 4 * 4);
+    rms_bwd_launch<pw::kRmsWeight>(nb, rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, part, st);
+    if (nb > 1) rms_dw_launch(nb, dim, part, dweight, st);
+    rms_bwd_launch<pw::kRmsInputs>(nb, rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, nullptr, st);
+    return launch_status();
 }
-
