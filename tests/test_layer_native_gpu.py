@@ -191,3 +191,8 @@ def test_more_sequences_than_the_batched_convolutions_grid_holds(batch):
         _modules_one_by_one(layer)
     for a, b in zip(*results):
         assert O.rel_l2(a.detach().float(), b.detach().float()) <= 2e-2
+
+
+def test_training_step_long_enough_for_the_streaming_convolutions():
+    """2 x 1,100 tokens of 6 heads: 3 x 6 x 36 runs, past the line (592) from which slices of the projection are streamed."""
+    test_training_step_equals_the_modules(2, 1100, 6, False, torch.float32)

@@ -294,3 +294,46 @@ def test_convolution_weights_at_any_element_offset(B, T, C, W, dtype, wdtype, st
             ys = ops.ConvMultiFunction.apply(True, 2, xs, xs, leaf, leaf)
             results[-1] += [*ys, *torch.autograd.grad(ys, [xs, leaf], [dy, dy])]
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+# Three convolutions on slices of one wide matrix, as the layer keeps its projections, either side of every dispatch line:
+# backward tile | ring (592 runs of 64 tokens x 128 channels: 65 and 66 tiles at 3 x 384), ring runs of 32 | 64 tokens (147 and 148
+# tiles at 3 x 2,048), forward pair | streaming (36 and 37 blocks of 256 tokens at 3 x 2,048); ragged ends, several sequences.
+@pytest.mark.parametrize("B,T,C,W", [(1, 4160, 384, 4), (1, 4161, 384, 4), (3, 1431, 384, 3), (1, 9216, 2048, 4), (1, 9217, 2048, 4), (1, 9408, 2048, 4),
+                                     (1, 9409, 2048, 4), (2, 4801, 2048, 2), (2, 70, 130, 4)])
+def test_convolutions_on_slices_equal_those_on_dense_copies(B, T, C, W):
+    """The same kernels with another row stride: equal to the bit, with NaN in the columns that are not theirs and every column
+    of the gradient's matrix outside the slices untouched."""
+    import ctypes
+    from experiment_swa_kda_b200 import _lib
+    lib, n = _lib.load(), 3
+    step = (C + 15) // 8 * 8                                # slices at 16-byte addresses, a few columns between them
+    first, ld = [0, step, 2 * step], 4 * C + 144 + C % 8
+    gen = torch.Generator(device=D0).manual_seed(T + C)
+    dense = lambda *shape: torch.randn(*shape, device=D0, generator=gen).bfloat16()
+    xs, dys = [dense(B * T, C) for _ in range(n)], [dense(B * T, C) for _ in range(n)]
+    ws = [torch.randn(C, W, device=D0, generator=gen) for _ in range(n)]
+    P = torch.full((B * T, ld), float("nan"), device=D0, dtype=torch.bfloat16)
+    for f, x in zip(first, xs):
+        P[:, f:f + C] = x
+    arr = lambda ps: ctypes.cast((ctypes.c_void_p * n)(*ps), ctypes.c_void_p)
+    ptrs = lambda ts: [t.data_ptr() for t in ts]
+    at = lambda m: [m.data_ptr() + 2 * f for f in first]
+    stream, io = torch.cuda.current_stream().cuda_stream, _lib.DTYPE_BF16 | 0x100
+    scr = torch.empty(lib.kda_conv_bwd_multi_scratch_bytes(n, B, T, C, W), dtype=torch.uint8, device=D0)
+
+    def run(x_at, x_ld, dx_at):
+        ys, dws = [torch.empty_like(x) for x in xs], [torch.empty(C, W, device=D0) for _ in range(n)]
+        _lib.check(lib.kda_conv_fwd_rows(n, B, T, C, W, io, 1, arr(x_at), x_ld, arr(ptrs(ws)), None, arr(ptrs(ys)), None, stream), "forward")
+        _lib.check(lib.kda_conv_bwd_rows(n, B, T, C, W, io, 1, arr(x_at), x_ld, arr(ptrs(ws)), arr(ptrs(dys)), arr(dx_at), arr(ptrs(dws)),
+                                         scr.data_ptr(), scr.numel(), stream), "backward")
+        return [*ys, *dws]
+
+    dxs, dP = [torch.empty_like(x) for x in xs], torch.full_like(P, 7.0)
+    want, got = run(ptrs(xs), C, ptrs(dxs)), run(at(P), ld, at(dP))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    outside = torch.ones(ld, dtype=torch.bool, device=D0)
+    for f, dx in zip(first, dxs):
+        assert torch.equal(dP[:, f:f + C], dx)
+        outside[f:f + C] = False
+    assert outside.any() and (dP[:, outside] == 7.0).all()
