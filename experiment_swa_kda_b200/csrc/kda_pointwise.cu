@@ -829,7 +829,7 @@ __device__ __forceinline__ T pick_item(T const (&a)[kConvItems], int i) {
 // grid: x = channel blocks of 32*VEC, y = blocks of 8 time groups x kConvPairT tokens, z = item * B + batch.  x rows are
 // ldx elements apart (a slice of a wider projection), y rows are dense.  WIN: a window is carried in or out; only the
 // threads at either end of a sequence touch it.  The kernel moves 2 x B x T x C elements and is bound by instruction issue
-// at 0.65 of the copy rate (126 us at 65,536 x 2,048 bf16; long inputs take the streaming kernel below); the windows used
+// at 0.63 of the copy rate (129 us at 65,536 x 2,048 bf16; long inputs take the streaming kernel below); the windows used
 // to go through a 4-token, 8-channel kernel whose lanes read 16-byte pieces of strided rows: 78 us at 8,191 x 2,048, now 22.
 template <int W, int VEC, bool BF16, bool WIN>
 __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C, int ldx, int silu, int wf32, ConvFwdItems items) {

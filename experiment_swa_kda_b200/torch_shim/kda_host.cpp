@@ -115,8 +115,9 @@ ChunkGrads run_chunk_bwd(const KdaChunkShape& sh, const Tensor& q, const Tensor&
 }
 
 // Backward of chunk_kda: the gradients of (q, k, v, g, beta, h0) from the cotangents of (o, final state).  The workspace
-// rides with the saved tensors: it lives exactly as long as the graph does, and the backward kernels only read it, so a
-// second backward through a retained graph finds it intact.
+// rides with the saved tensors: it lives exactly as long as the graph does.  A backward of the tensor-core lane writes its
+// own panels there (adjoint states, dZ, the split scan's maps) and nothing the forward left for it, so a second one through
+// a retained graph finds all it reads.
 struct ChunkNode : public HostNode {
     KdaChunkShape sh;
     Tensor cu;

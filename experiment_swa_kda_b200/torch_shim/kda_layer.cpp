@@ -307,6 +307,9 @@ bool layer_sizes(const Tensor& x, const std::vector<Tensor>& w, int64_t heads, c
 // kda_conv_*_rows: `items` convolutions share a launch whose grid has items x batch and 64-token tiles as its y and z
 bool fits_grid(const Sizes& z, int64_t items) { return z.B * items <= 65535 && (z.T + 63) / 64 <= 65535; }
 
+// Rows that one launch of the rows product takes.  A no-grad layer of 16 heads, on the device with a cold L2: 76 us at 8 rows, 80
+// at 32 and 94 at 64, through the packed matrix 84, 84 and 88; with 3 heads 54, 57 and 59 against 57.  A token of more
+// sequences runs module by module (16 heads, by the host: 83 us at 64 sequences, 292 at 65).
 constexpr int64_t kFewRows = 64;
 
 // products of at most kFewRows rows with `count` consecutive weights of the list, straight from the parameters
