@@ -15,7 +15,7 @@
 // 256-byte row segment) and needs two exponentials per element.  Only the source rows up to a target block's own end are
 // built, 160 instead of 256, so all of them fit at once; the value tile takes their place when the products are done.  97 KB
 // and <= 128 registers let two CTAs share an SM and fill each other's waits: the kernel is a chain of short phases between
-// barriers, at 40 % of its issue slots.  16,384 chunk-heads: 1,372 -> 1,165 us, 384: 49 -> 43 us.
+// barriers, at 40 % of its issue slots.  16,384 chunk-heads: 1,372 -> 1,156 us, 384: 49 -> 43 us.
 // Restates reference chunk_wy_forward.cu:125-405 and 761-858.
 
 #include <cstdio>
