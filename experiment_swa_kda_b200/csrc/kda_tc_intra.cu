@@ -7,15 +7,18 @@
 //       (restates the per-tile decay centre of reference chunk_wy_forward.cu:312-376, 447-450)
 //   T = (I + beta M~)^-1                                                       fp32, block forward substitution
 //   U^T = P^T T^T,  W^T = Q^T T^T   (P = beta v, Q = beta e^G k)                tcgen05, M=128 N=64 K=64, MN-major A
-//   R^T = (q e^G)^T, E = k e^{G_end-G}, e^{G_end}, A^T, T                       panels for the scans / backward
+//   R = q e^G, E = k e^{G_end-G}, e^{G_end}, A^T, T                            panels for the scans / backward
 //   Pn = W^T E,  Rm^T = R^T - W^T A^T   (the chunk's state transition)         tcgen05, M=128 N=128|64 K=64, at the end:
-//       W^T is still staged in shared memory for its store, E and A^T come back by TMA into the dead value / Q tiles
+//       W^T is staged in shared memory for its store, R, E and A^T are still there as they left
 // Every operand panel is written as 16-byte pieces of the 128-byte-swizzled layout the UMMA descriptors read: a thread
 // owns 8 adjacent channels of 4 consecutive rows, takes q, k, g straight from global memory (a half-warp reads one
 // 256-byte row segment) and needs two exponentials per element.  Only the source rows up to a target block's own end are
-// built, 160 instead of 256, so all of them fit at once; the value tile takes their place when the products are done.  97 KB
-// and <= 128 registers let two CTAs share an SM and fill each other's waits: the kernel is a chain of short phases between
-// barriers, at 40 % of its issue slots.  16,384 chunk-heads: 1,372 -> 1,156 us, 384: 49 -> 43 us.
+// built, 160 instead of 256, so all of them fit at once; the second half's tiles take their place when the products are done.
+// 113 KB and <= 128 registers let two CTAs share an SM and fill each other's waits: the kernel is a chain of short phases
+// between barriers.  Every panel leaves by TMA from the tile the products read, and nothing comes back: R^T stored from
+// registers in 8-byte pieces (32 sectors a warp store), E and A^T fetched again for the transition, with a fence in front,
+// and R^T read row by row had taken a fifth of a block's cycles.  16,384 chunk-heads: 1,157 -> 960 us, 384: 46 -> 41 us,
+// 2,048 forward-only: 148 -> 130 us.
 // Restates reference chunk_wy_forward.cu:125-405 and 761-858.
 
 #include <cstdio>
@@ -161,22 +164,29 @@ __device__ __forceinline__ void warp_mm(PA pa, PB pb, PD pd, float alpha) {
     *reinterpret_cast<float2*>(D + 8 * LD) = make_float2(alpha * d[2], alpha * d[3]);
 }
 
-// Ts = (I + Ms)^-1 for strictly lower-triangular Ms (64x64), Ts zero on entry: 8x8 diagonal solves (a short dependent chain per thread),
-// then merges to 16 (CUDA cores), 32 and 64 (warp-level tensor cores) with
+// Ms = (I + Ms)^-1 in place for strictly lower-triangular Ms (64x64, zero on and above the diagonal): 8x8 diagonal solves (a
+// short dependent chain per thread), then merges to 16 (CUDA cores), 32 and 64 (warp-level tensor cores) with
 //   inv([[A,0],[C,B]]) = [[Ai,0],[-Bi C Ai, Bi]].
-__device__ __forceinline__ void unit_lower_inverse(const float* Ms, float* Ts, float* tmp) {
+// A merge reads all of C into its scratch before it writes over it.
+__device__ __forceinline__ void unit_lower_inverse(float* Ms, float* tmp) {
     const int tid = threadIdx.x;
+    float* Ts = Ms;
     if (tid < 64) {
         const int b = tid >> 3, j = tid & 7;          // diagonal block, column of the inverse
         const float* Lb = Ms + (8 * b) * kLDs + 8 * b;
-        float x[8];
+        float x[8], L[28];
+#pragma unroll
+        for (int i = 1; i < 8; ++i)
+#pragma unroll
+            for (int t = 0; t < i; ++t) L[i * (i - 1) / 2 + t] = Lb[i * kLDs + t];
+        __syncwarp();                                 // a block's eight threads sit in one warp: all have read it
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = (i == j) ? 1.f : 0.f;
 #pragma unroll
         for (int i = 1; i < 8; ++i) {
             float s = 0.f;
 #pragma unroll
-            for (int t = 0; t < i; ++t) s += Lb[i * kLDs + t] * x[t];
+            for (int t = 0; t < i; ++t) s += L[i * (i - 1) / 2 + t] * x[t];
             x[i] = (i > j) ? -s : x[i];
         }
         float* Tb = Ts + (8 * b) * kLDs + 8 * b;
@@ -227,14 +237,20 @@ constexpr int kFSB = 32768;        //  8 KB  sources of target block 1 (32 rows)
 constexpr int kFXA = 40960;        // 24 KB  targets 3 | 2 | 0 (32 rows each: 16 q~, 16 k~), 2 k-blocks of 12 KB
 constexpr int kFXB = 65536;        //  8 KB  targets 1, 2 k-blocks of 4 KB
 constexpr int kFQ = 73728;         // 16 KB  Q = beta e^G k: MN-major A of W^T = Q^T T^T
-constexpr int kFTab = 90112;       // floats: cref[4][128] eC[4][128] eEnd[4][128] fb[3][128] | gfirst[4][128] | bet[64]
-constexpr int kTabFloats = 15 * 128 + 4 * 128 + 64;
-// after the A / M~ products the stacks are dead: Ms, Ts (fp32), the two bf16 T operands and the value tile live in
-// [0, 72 KB), the inverse's scratch in the dead tables
-constexpr int kFMs = 0, kFTs = 64 * kLDs * 4, kFTb = 35840, kFTbb = 44032;
-constexpr int kFV = 53248;         // 16 KB  v tile (TMA): MN-major A of U^T = v^T (T diag(beta))^T
-static_assert(kFTs + 64 * kLDs * 4 <= kFTb && kFV + 16384 <= kFQ && 32 * kLDt <= 15 * 128, "shared-memory map");
+constexpr int kFE = 90112;         // 16 KB  E = k e^{G_end-G}: the panel's store and the B operand of Pn = W^T E
+constexpr int kFTab = 106496;      // floats: cref[4][128] eC[4][128] eEnd[4][128] fb[3][128] | bet[64]
+constexpr int kTabFloats = 15 * 128 + 64;
+// After the A / M~ products the stacks are dead and [0, 72 KB) holds the second half's tiles; the inverse's scratch lies in
+// the dead tables.
+constexpr int kFMs = 0;            // 17 KB  beta M~, then its inverse (fp32); the two bf16 T operands take its place
+constexpr int kFTb = 0, kFTbb = 8192;
+constexpr int kFAT = 18432;        //  8 KB  A^T: the panel's store and the B operand of W^T A^T
+constexpr int kFMt = 26624;        //  8 KB  M~ panel on its way out, then the identity that adds R^T to the transition
+constexpr int kFR = 34816;         // 16 KB  R = q e^G: the panel's store and an A operand of the transition, then Rm^T on its way out
+constexpr int kFV = 51200;         // 16 KB  v tile (TMA): MN-major A of U^T = v^T (T diag(beta))^T, then U^T on its way out
+static_assert(kFMs + 64 * kLDs * 4 <= kFAT && kFV + 16384 <= kFQ && 32 * kLDt <= 15 * 128, "shared-memory map");
 constexpr int kIntraFwdSmem = kFTab + kTabFloats * 4 + 1024;
+static_assert(2 * (kIntraFwdSmem + 64 + 1024) <= 228 * 1024, "two CTAs share an SM");
 
 // y = silu(sum_m w[m] x[t - 3 + m]) for this thread's 4 rows x 8 channels from the 7 input rows it needs, in the
 // arithmetic of the stand-alone convolution kernel (float32 accumulation in tap order, hardware-tanh sigmoid, one
@@ -279,7 +295,7 @@ __global__ void __launch_bounds__(kNT, 2)
                         const __grid_constant__ CUtensorMap mWT, const __grid_constant__ CUtensorMap mAT,
                         const __grid_constant__ CUtensorMap mMt, const __grid_constant__ CUtensorMap mE,
                         const __grid_constant__ CUtensorMap mP, const __grid_constant__ CUtensorMap mRm,
-                        const __grid_constant__ CUtensorMap mTp, IntraFwdArgs p) {
+                        const __grid_constant__ CUtensorMap mTp, const __grid_constant__ CUtensorMap mR, IntraFwdArgs p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
     uint8_t* vs = sm + kFV;
@@ -288,15 +304,12 @@ __global__ void __launch_bounds__(kNT, 2)
     float* eC = cref + 512;                                  // [4][128] exp(cref)
     float* eEnd = eC + 512;                                  // [4][128] exp(G_end - cref)
     float* fbk = eEnd + 512;                                 // [3][128] exp(cref[I+1] - cref[I])
-    float* gfirst = fbk + 384;                               // [4][128] g of the first row of each block
-    float* bet = gfirst + 512;                               // [64]
+    float* bet = fbk + 384;                                  // [64]
     float* wtot = reinterpret_cast<float*>(sm + kFSA);       // [8][128] per-warp sums of g (dead before the stacks are written)
+    float* gfirst = wtot + 1024;                             // [4][128] g of the first row of each block (dead with them)
     float* Ms = reinterpret_cast<float*>(sm + kFMs);
-    float* Ts = reinterpret_cast<float*>(sm + kFTs);
     float* tmp = cref;
-    uint8_t* Tb = sm + kFTb;                                 // [64 rows x 128 B] K-major B: T
-    uint8_t* Tbb = sm + kFTbb;                               //                              T diag(beta)
-    __shared__ uint64_t bar_in, bar_am, bar_uw, bar_tr;
+    __shared__ uint64_t bar_in, bar_am, bar_uw;
     __shared__ uint32_t tmem_slot;
 
     // heads fastest: blocks that run side by side read neighbouring pieces of the same token rows
@@ -314,7 +327,6 @@ __global__ void __launch_bounds__(kNT, 2)
         mbar_init(&bar_in, 1);
         mbar_init(&bar_am, 2);
         mbar_init(&bar_uw, 1);
-        mbar_init(&bar_tr, 1);
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(&tmem_slot, 256);
@@ -452,13 +464,12 @@ __global__ void __launch_bounds__(kNT, 2)
 
     // ---- operand panels, one row at a time, four channels at a time in packed pairs: 16-byte pieces of the swizzled
     // layouts.  Bound by instruction issue: two exponentials and reciprocals an element are 6 of its ~20 instructions.
-    uint32_t rw[4][4];                                 // R = q e^G, rows 4rq .. 4rq+3, channel pairs
+    uint32_t rw[4][4];                                 // R = q e^G, rows 4rq .. 4rq+3, channel pairs (stored once the stacks are dead)
     {
         // row bases of target block b in the stacks: {3, 2, 0} share the first pair, {1} has the second
         uint8_t* X = sm + (J == 1 ? kFXB : kFXA);
         const uint32_t xkb = J == 1 ? 4096u : 12288u;
         const int xr0 = J == 3 || J == 1 ? 0 : (J == 2 ? 32 : 64);
-        __nv_bfloat16* Eg = p.t.E + ch * 8192 + 8 * cg;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int i = 4 * rq + j;
@@ -508,7 +519,7 @@ __global__ void __launch_bounds__(kNT, 2)
             put(X + piece_off(xr0 + (i & 15), cg, xkb), xq);
             put(X + piece_off(xr0 + 16 + (i & 15), cg, xkb), xk);
             put(Qs + piece_off(i, cg, 8192), pw);
-            put(reinterpret_cast<uint8_t*>(Eg + (size_t)i * 128), ew);
+            put(sm + kFE + piece_off(i, cg, 8192), ew);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 const int b = J + v;                   // target block
@@ -536,16 +547,10 @@ __global__ void __launch_bounds__(kNT, 2)
         umma_commit(&bar_am);
     }
     __syncwarp();
-    // in flight: R^T (channel-major: 4 tokens of 8 channels), v's convolution, the next block's inputs
-    {
-        __nv_bfloat16* Rg = p.t.RT + ch * 8192 + (size_t)(8 * cg) * 64 + 4 * rq;
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            *reinterpret_cast<uint2*>(Rg + (2 * w) * 64) =
-                make_uint2(__byte_perm(rw[0][w], rw[1][w], 0x5410), __byte_perm(rw[2][w], rw[3][w], 0x5410));
-            *reinterpret_cast<uint2*>(Rg + (2 * w + 1) * 64) =
-                make_uint2(__byte_perm(rw[0][w], rw[1][w], 0x7632), __byte_perm(rw[2][w], rw[3][w], 0x7632));
-        }
+    // in flight: the E panel leaves, v's convolution, the next block's inputs
+    if (tid == 0) {
+        for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mE, sm + kFE + nb * 8192, nb * 64, (int)(ch * 64));
+        tma_store_commit();
     }
     uint4 vr[4];
     if constexpr (CONV) {
@@ -590,6 +595,8 @@ __global__ void __launch_bounds__(kNT, 2)
             mbar_expect_tx(&bar_in, 16384);
             for (int kb = 0; kb < 2; ++kb) tma_load_2d(vs + kb * 8192, &mv, &bar_in, h * 128 + kb * 64, tok0);
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(sm + kFR + piece_off(4 * rq + j, cg, 8192)) = make_uint4(rw[j][0], rw[j][1], rw[j][2], rw[j][3]);
         // ---- A^T panel, M~ panel and beta*M~ (fp32): a thread takes one source row s of one target block Ib, 16 columns
         // of A (q targets) and 16 of M~ (k targets).  Accumulator lanes: block 3 in warps 0, 1, block 2 in warp 2 and half
         // of warp 3, block 0 in the other half, block 1 in warp 4; warps 5 to 7 fill in the sources behind a target block.
@@ -624,9 +631,9 @@ __global__ void __launch_bounds__(kNT, 2)
                 const float a1 = (s <= 16 * Ib + c + 1) ? __uint_as_float(t[c + 1]) : 0.f;
                 at[c >> 1] = pack2(a0, a1);
             }
-            // both panels leave through shared memory (the T operands' region is still free) as one TMA store each
-            uint8_t* ATs = sm + kFTb;              // [64 s][64 i]  bf16, 128-byte swizzle
-            uint8_t* Mts = sm + kFTb + 8192;       // [64 tt][64 s]
+            // both panels leave through shared memory as one TMA store each
+            uint8_t* ATs = sm + kFAT;              // [64 s][64 i]  bf16, 128-byte swizzle
+            uint8_t* Mts = sm + kFMt;              // [64 tt][64 s]
             *reinterpret_cast<uint4*>(ATs + sw128_off(s, 2 * Ib)) = make_uint4(at[0], at[1], at[2], at[3]);
             *reinterpret_cast<uint4*>(ATs + sw128_off(s, 2 * Ib + 1)) = make_uint4(at[4], at[5], at[6], at[7]);
 #pragma unroll
@@ -637,34 +644,45 @@ __global__ void __launch_bounds__(kNT, 2)
                 *reinterpret_cast<__nv_bfloat16*>(Mts + sw128_off(tt, s >> 3) + (s & 7) * 2) = __float2bfloat16(mt);
             }
         }
-        for (int idx = tid; idx < 64 * kLDs / 4; idx += kNT) reinterpret_cast<float4*>(Ts)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
-            tma_store_2d(&mAT, sm + kFTb, 0, (int)(ch * 64));
-            if (!p.t.fwd_only) tma_store_2d(&mMt, sm + kFTb + 8192, 0, (int)(ch * 64));
+            tma_store_2d(&mAT, sm + kFAT, 0, (int)(ch * 64));
+            for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mR, sm + kFR + nb * 8192, nb * 64, (int)(ch * 64));
+            if (!p.t.fwd_only) tma_store_2d(&mMt, sm + kFMt, 0, (int)(ch * 64));
             tma_store_commit();
         }
-        unit_lower_inverse(Ms, Ts, tmp);
-        if (tid == 0) tma_store_wait_read();       // the staging region becomes the T operands below
-        __syncthreads();
+        unit_lower_inverse(Ms, tmp);
         // ---- T: bf16 K-major B operands (plain and column-scaled by beta); 32 bytes of a row each, lanes on
         // consecutive rows (272 bytes apart: every 16-byte access of a quarter-warp lands in its own banks).  The plain
         // operand tile is the T panel as TMA lays it out, so the panel is stored from it below.
         {
             const int i = tid & 63, seg = tid >> 6;
-            const float* src = Ts + i * kLDs + 16 * seg;
+            const float* src = Ms + i * kLDs + 16 * seg;
             const float* bb = bet + 16 * seg;
+            uint4 u[2], ub[2];
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 float x[8], b8[8];
                 lds8(src + 8 * hh, x);
                 lds8(bb + 8 * hh, b8);
-                const uint4 u = pack8(x);
-                *reinterpret_cast<uint4*>(Tb + sw128_off(i, 2 * seg + hh)) = u;
+                u[hh] = pack8(x);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) x[c] *= b8[c];
-                *reinterpret_cast<uint4*>(Tbb + sw128_off(i, 2 * seg + hh)) = pack8(x);
+                ub[hh] = pack8(x);
+            }
+            if (tid == 0) tma_store_wait_read();       // the M~ panel has left: the identity takes its place
+            __syncthreads();                           // everyone has its piece of T: the operands take its place
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const uint32_t off = sw128_off(i, 2 * seg + hh);
+                *reinterpret_cast<uint4*>(sm + kFTb + off) = u[hh];
+                *reinterpret_cast<uint4*>(sm + kFTbb + off) = ub[hh];
+                if (!p.t.fwd_only) {
+                    const int one = i - 16 * seg - 8 * hh;         // this row's element on the diagonal, if it is in these 8
+                    const uint32_t w = (one & 1) ? 0x3f800000u : 0x3f80u;
+                    *reinterpret_cast<uint4*>(sm + kFMt + off) = make_uint4((one >> 1) == 0 ? w : 0u, (one >> 1) == 1 ? w : 0u, (one >> 1) == 2 ? w : 0u, (one >> 1) == 3 ? w : 0u);
+                }
             }
         }
         // the value tile: wait for it, blank the rows past a ragged tail (they hold other tokens)
@@ -676,18 +694,16 @@ __global__ void __launch_bounds__(kNT, 2)
             }
         }
         fence_async_smem();
-        __threadfence();
-        asm volatile("fence.proxy.async.global;" ::: "memory");
         tc_fence_before();
         ok = __syncthreads_and(ok);
         if (tid == 0 && ok) {
             if (!p.t.fwd_only) {                   // kept for the backward only
-                tma_store_2d(&mTp, Tb, 0, (int)(ch * 64));
+                tma_store_2d(&mTp, sm + kFTb, 0, (int)(ch * 64));
                 tma_store_commit();
             }
             tc_fence_after();
             const uint32_t idesc = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
-            const uint32_t b0 = smem_u32(Tb), b1 = smem_u32(Tbb);
+            const uint32_t b0 = smem_u32(sm + kFTb), b1 = smem_u32(sm + kFTbb);
 #pragma unroll
             for (int k16 = 0; k16 < 4; ++k16)     // U^T = v^T (T diag(beta))^T
                 umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(smem_u32(vs) + k16 * 2048, 8192, 1024),
@@ -700,27 +716,13 @@ __global__ void __launch_bounds__(kNT, 2)
         }
         if (ok) ok = mbar_wait(&bar_uw, 0, p.t.status, 32);
         tc_fence_after();
-        // ---- chunk transition, fused: Pn = W^T E and Rm^T = R^T - W^T A^T need W^T (about to be staged below), E and
-        // A^T.  The value and Q tiles are dead now: E and A^T come back into them by TMA while the panels are read out.
         const int kt = (warp & 3) * 32 + lane, gt = warp >> 2;      // transition read-out: key row, column half
-        uint4 rtv[4];
-        if (tid == 0 && ok) {
-            tma_store_wait_all();                  // the A^T panel stored above is complete in global memory
-            mbar_expect_tx(&bar_tr, 16384 + (p.t.fwd_only ? 0 : 8192));
-            for (int nb = 0; nb < 2; ++nb) tma_load_2d(vs + nb * 8192, &mE, &bar_tr, nb * 64, (int)(ch * 64));
-            if (!p.t.fwd_only) tma_load_2d(Qs, &mAT, &bar_tr, 0, (int)(ch * 64));
-        }
-        if (ok && !p.t.fwd_only) {
-            const uint4* src = reinterpret_cast<const uint4*>(p.t.RT + ch * 8192 + (size_t)kt * 64 + 32 * gt);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) rtv[j] = src[j];
-        }
         if (ok) {
             // lane = value channel (U^T, warps 0-3) / key channel (W^T, warps 4-7): one 128-byte panel row per thread,
-            // staged in the swizzled layout (the inverse's scratch is dead) and stored by TMA, 16 KB per panel
+            // staged in the swizzled layout over the dead v and Q tiles and stored by TMA, 16 KB per panel
             const int which = warp >> 2;
             const int d = (warp & 3) * 32 + lane;
-            uint8_t* stg = sm + which * 16384;
+            uint8_t* stg = which ? Qs : vs;
 #pragma unroll
             for (int hb = 0; hb < 2; ++hb) {
                 uint32_t r[32];
@@ -739,35 +741,41 @@ __global__ void __launch_bounds__(kNT, 2)
         tc_fence_before();
         ok = __syncthreads_and(ok);
         if (tid == 0 && ok) {
-            tma_store_2d(&mUT, sm, 0, (int)(ch * 128));
-            tma_store_2d(&mWT, sm + 16384, 0, (int)(ch * 128));
+            tma_store_2d(&mUT, vs, 0, (int)(ch * 128));
+            tma_store_2d(&mWT, Qs, 0, (int)(ch * 128));
             tma_store_commit();
-            ok = mbar_wait(&bar_tr, 0, p.t.status, 33);
-            if (ok) {
-                tc_fence_after();
-                // every accumulator column has been read out: Pn takes columns 0..127, (A W)^T columns 128..191
-                const uint32_t a0 = smem_u32(sm + 16384), bE = smem_u32(vs), bA = smem_u32(Qs);
-                const uint32_t id128 = umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
-                const uint32_t id64 = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
+            // ---- chunk transition, fused: Pn = W^T E and Rm^T = R^T - W^T A^T from the tiles that are still here.  Every
+            // accumulator column has been read out: Pn takes columns 0..127, Rm^T columns 128..191.  R lies token by token,
+            // so the product with an identity brings it in transposed (exactly: one term a sum).
+            tc_fence_after();
+            const uint32_t a0 = smem_u32(Qs), bE = smem_u32(sm + kFE);
+            const uint32_t id128 = umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
 #pragma unroll
-                for (int k16 = 0; k16 < 4; ++k16)     // Pn = W^T E
-                    umma_bf16_ss(tmem, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
-                                 umma_smem_desc_sw128(bE + k16 * 2048, 8192, 1024), id128, k16 > 0);
-                if (!p.t.fwd_only) {
+            for (int k16 = 0; k16 < 4; ++k16)     // Pn = W^T E
+                umma_bf16_ss(tmem, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
+                             umma_smem_desc_sw128(bE + k16 * 2048, 8192, 1024), id128, k16 > 0);
+            if (!p.t.fwd_only) {
+                const uint32_t idn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN, 1), idr = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
+                const uint32_t aR = smem_u32(sm + kFR), bA = smem_u32(sm + kFAT), bI = smem_u32(sm + kFMt);
 #pragma unroll
-                    for (int k16 = 0; k16 < 4; ++k16)     // (A W)^T = W^T A^T
-                        umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
-                                     umma_smem_desc_sw128(bA + k16 * 2048, 8192, 1024), id64, k16 > 0);
-                }
-                umma_commit(&bar_uw);
+                for (int k16 = 0; k16 < 4; ++k16)     // -(A W)^T = -W^T A^T
+                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
+                                 umma_smem_desc_sw128(bA + k16 * 2048, 8192, 1024), idn, k16 > 0);
+#pragma unroll
+                for (int k16 = 0; k16 < 4; ++k16)     // + R^T I
+                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(aR + k16 * 2048, 8192, 1024),
+                                 umma_smem_desc_sw128(bI + k16 * 32, 16, 1024), idr, 1);
             }
+            // the staging below overwrites E, R and T: their stores must have been read, all but the newest group's
+            tma_store_wait_read_but1();
+            umma_commit(&bar_uw);
         }
         if (ok) ok = mbar_wait(&bar_uw, 1, p.t.status, 34);      // no block-wide barrier: the staging below overwrites only what
         tc_fence_after();                                         // the completed products were the last to read
         if (ok) {
-            // both results leave through shared memory in the swizzled layout (Pn over the dead T operands and E tile, Rm^T
-            // over the A^T tile the products have finished reading) and are stored by TMA
-            uint8_t* Pst = sm + 32768 + gt * 16384;          // [128 key rows][64 columns of half gt]
+            // both results leave through shared memory in the swizzled layout (Pn over the T operands and the E tile, Rm^T
+            // over the R tile, all of them read for the last time) and are stored by TMA
+            uint8_t* Pst = sm + (gt ? kFE : kFTb);           // [128 key rows][64 columns of half gt]
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 uint32_t r[32];
@@ -786,22 +794,19 @@ __global__ void __launch_bounds__(kNT, 2)
                 tmem_ld32(tmem + lane_base + 128 + 32 * gt, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float f[8];
-                    unpack_bf16x8(rtv[c], f);
-                    *reinterpret_cast<uint4*>(Qs + sw128_off(kt, 4 * gt + c)) =
-                        make_uint4(pack2(f[0] - __uint_as_float(r[8 * c]), f[1] - __uint_as_float(r[8 * c + 1])),
-                                   pack2(f[2] - __uint_as_float(r[8 * c + 2]), f[3] - __uint_as_float(r[8 * c + 3])),
-                                   pack2(f[4] - __uint_as_float(r[8 * c + 4]), f[5] - __uint_as_float(r[8 * c + 5])),
-                                   pack2(f[6] - __uint_as_float(r[8 * c + 6]), f[7] - __uint_as_float(r[8 * c + 7])));
-                }
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(sm + kFR + sw128_off(kt, 4 * gt + c)) =
+                        make_uint4(pack2(__uint_as_float(r[8 * c]), __uint_as_float(r[8 * c + 1])),
+                                   pack2(__uint_as_float(r[8 * c + 2]), __uint_as_float(r[8 * c + 3])),
+                                   pack2(__uint_as_float(r[8 * c + 4]), __uint_as_float(r[8 * c + 5])),
+                                   pack2(__uint_as_float(r[8 * c + 6]), __uint_as_float(r[8 * c + 7])));
             }
         }
         fence_async_smem();
         ok = __syncthreads_and(ok);
         if (tid == 0 && ok) {
-            for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mP, sm + 32768 + nb * 16384, nb * 64, (int)(ch * 128));
-            if (!p.t.fwd_only) tma_store_2d(&mRm, Qs, 0, (int)(ch * 128));
+            for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mP, sm + (nb ? kFE : kFTb), nb * 64, (int)(ch * 128));
+            if (!p.t.fwd_only) tma_store_2d(&mRm, sm + kFR, 0, (int)(ch * 128));
             tma_store_commit();
         }
         if (tid == 0) tma_store_wait_read();           // shared memory must outlive the reads of the bulk stores
@@ -824,13 +829,14 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
     a.conv = conv != nullptr ? *conv : tc::ConvPrep{{nullptr, nullptr, nullptr}, 0, 0};
     if (conv != nullptr && !t.fwd_only) return KDA_ERR_UNSUPPORTED;      // a backward would need q, k, v in memory
     const uint64_t nch = (uint64_t)w.nslots * w.H;
-    CUtensorMap mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp;
+    CUtensorMap mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp, mR;
     int rc = make_map_bf16(&mv, v, (uint64_t)tokens, (uint64_t)w.H * 128, 64, 64);
     rc |= make_map_bf16(&mUT, t.UT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mWT, t.WT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mAT, t.AT, nch * 64, 64, 64, 64);
     rc |= make_map_bf16(&mMt, t.fwd_only ? t.AT : t.Mt, nch * 64, 64, 64, 64);      // not stored in a forward-only call
     rc |= make_map_bf16(&mE, t.E, nch * 64, 128, 64, 64);
+    rc |= make_map_bf16(&mR, t.R, nch * 64, 128, 64, 64);
     rc |= make_map_bf16(&mTp, t.fwd_only ? t.AT : t.Tp, nch * 64, 64, 64, 64);      // not stored in a forward-only call
     rc |= make_map_bf16(&mP, t.Pn, nch * 128, 128, 64, 128);
     rc |= make_map_bf16(&mRm, t.fwd_only ? t.WT : t.RmT, nch * 128, 64, 64, 128);      // not stored in a forward-only call
@@ -838,7 +844,7 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
     auto kern = conv != nullptr ? (gbf16 ? tc_intra_fwd_kernel<true, true> : tc_intra_fwd_kernel<false, true>)
                                 : (gbf16 ? tc_intra_fwd_kernel<true, false> : tc_intra_fwd_kernel<false, false>);
     if (set_smem_limit(kern, kIntraFwdSmem)) return KDA_ERR_CUDA;
-    KDA_LAUNCH("tc_intra_fwd_kernel", st, kern<<<(unsigned)nch, kNT, kIntraFwdSmem, st>>>(mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp, a));
+    KDA_LAUNCH("tc_intra_fwd_kernel", st, kern<<<(unsigned)nch, kNT, kIntraFwdSmem, st>>>(mv, mUT, mWT, mAT, mMt, mE, mP, mRm, mTp, mR, a));
     return launch_status();
 }
 

@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(256, 1)
 
 // ---------------------------------------------------------------------------------------------
 // chunk output (forward), one CTA per chunk-head, from the chunk-start state the scan stored:
-//     [ (W H)^T | (R H)^T ] = H^T [ W^T | R^T ]      M=128, N=128, K=128
+//     (W H)^T = H^T W^T,  (R H)^T = H^T R^T           M=128, N=64 each, K=128
 //     Z^T = U^T - (W H)^T                             registers -> bf16 panel (kept for the backward) and A operand
 //     (A Z)^T = Z^T A^T                               M=128, N=64,  K=64
 //     O^T = (R H)^T + (A Z)^T                         transposed through shared memory into o[token][head][value]
@@ -593,8 +593,8 @@ struct ChunkOutArgs {
     NormEpilogue norm;
 };
 
-// Z^T reuses the [W^T|R^T] tile and the output tile reuses the state tile: both are dead once the first UMMA chain has
-// completed, and the smaller footprint lets two CTAs share an SM.
+// Z^T reuses the W^T tile and the output tile reuses the state tile: the one is dead once the first UMMA chain has
+// completed, the other after the last, and the smaller footprint lets two CTAs share an SM.
 constexpr int kOutH = 0, kOutWR = 32768, kOutU = 65536, kOutA = 81920, kOutZ = kOutWR, kOutO = kOutH, kOutG = 90112;
 constexpr int kChunkOutSmem = kOutA + 8192 + 1024;
 constexpr int kChunkOutNormSmem = kOutG + 16384 + 1024;      // + the norm gate's tile when the epilogue is on
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(256, 2)
             for (int kb = 0; kb < 2; ++kb) tma_load_2d(sm + kOutG + kb * 8192, &mG, &bar_in, h * 128 + kb * 64, tok0);
         for (int kb = 0; kb < 2; ++kb) tma_load_2d(sm + kOutH + kb * 16384, &mH, &bar_in, kb * 64, ch * 128);
         tma_load_2d(sm + kOutWR, &mW, &bar_in, 0, ch * 128);
-        tma_load_2d(sm + kOutWR + 16384, &mR, &bar_in, 0, ch * 128);
+        for (int kb = 0; kb < 2; ++kb) tma_load_2d(sm + kOutWR + 16384 + kb * 8192, &mR, &bar_in, kb * 64, ch * 64);
         tma_load_2d(sm + kOutU, &mUT, &bar_in, 0, ch * 128);
         tma_load_2d(sm + kOutA, &mAT, &bar_in, 0, ch * 64);
     }
@@ -644,12 +644,16 @@ __global__ void __launch_bounds__(256, 2)
         if (ok) {
             tc_fence_after();
             const uint32_t a0 = smem_u32(sm + kOutH), b0 = smem_u32(sm + kOutWR);
-            const uint32_t idesc = umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
+            const uint32_t idw = umma_idesc_bf16(128, 64, kMajorK, kMajorMN), idr = umma_idesc_bf16(128, 64, kMajorK, kMajorK);
 #pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)
+            for (int k16 = 0; k16 < 8; ++k16)     // W^T lies key by key ...
                 umma_bf16_ss(tmem, umma_smem_desc_sw128(a0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(b0 + k16 * 2048, 16384, 1024), idesc, k16 > 0);
+                             umma_smem_desc_sw128(b0 + k16 * 2048, 8192, 1024), idw, k16 > 0);
             umma_commit(&bar_mma1);
+#pragma unroll
+            for (int k16 = 0; k16 < 8; ++k16)     // ... R token by token; needed with the last product only (the commit behind that covers it)
+                umma_bf16_ss(tmem + 64, umma_smem_desc_sw128(a0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
+                             umma_smem_desc_sw128(b0 + 16384 + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), idr, k16 > 0);
         }
     }
     ok = mbar_wait(&bar_mma1, 0, p.status, 61) && ok;
@@ -891,7 +895,7 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
     CUtensorMap mW, mR, mE, mAT, mUT, mH, mP, mG, mZT;
     int rc = 0;
     rc |= make_map_bf16(&mW, t.WT, nch * 128, 64, 64, 128);
-    rc |= make_map_bf16(&mR, t.RT, nch * 128, 64, 64, 128);
+    rc |= make_map_bf16(&mR, t.R, nch * 64, 128, 64, 64);
     rc |= make_map_bf16(&mE, t.E, nch * 64, 128, 64, 64);
     rc |= make_map_bf16(&mAT, t.AT, nch * 64, 64, 64, 64);
     rc |= make_map_bf16(&mUT, t.UT, nch * 128, 64, 64, 128);

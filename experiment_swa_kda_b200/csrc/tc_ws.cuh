@@ -17,8 +17,8 @@ struct ConvPrep {
 };
 
 struct TcWs {
-    __nv_bfloat16 *WT, *RT;     // [nch][128][64]   rows = key, cols = token
-    __nv_bfloat16* E;           // [nch][64][128]   rows = token, cols = key
+    __nv_bfloat16* WT;          // [nch][128][64]   rows = key, cols = token
+    __nv_bfloat16 *R, *E;       // [nch][64][128]   rows = token, cols = key
     __nv_bfloat16* AT;          // [nch][64][64]    A transposed: [source s][target i]
     __nv_bfloat16* UT;          // [nch][128][64]   U transposed: [value][token]
     __nv_bfloat16* Tp;          // [nch][64][64]    T = (I + M)^-1, row-major
@@ -71,7 +71,7 @@ inline TcWs carve_tc(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr
     const size_t bw = sh.forward_only ? 0 : 1;      // panels only the backward reads
     simt::Carver c(mem);
     t.WT = c.take<__nv_bfloat16>(nch * 8192);
-    t.RT = c.take<__nv_bfloat16>(nch * 8192);
+    t.R = c.take<__nv_bfloat16>(nch * 8192);
     t.E = c.take<__nv_bfloat16>(nch * 8192);
     t.AT = c.take<__nv_bfloat16>(nch * 4096);
     t.UT = c.take<__nv_bfloat16>(nch * 8192);
