@@ -1,7 +1,8 @@
 // Tensor-core lane, chunk-parallel part of the backward: one CTA (512 threads) per (chunk, head) turns the
 // adjoints published by the reverse scan into dq, dk, dv, dg, dbeta.  K = V = 128, 64 tokens per chunk, bf16
-// UMMA operands, fp32 accumulation.  Thread (I, d) owns channel d and the 16 tokens of row block I, so every
-// "channel x token" accumulator row (TMEM lane d) is read by the four threads that share that lane.
+// UMMA operands, fp32 accumulation.  Warp (I, w) owns the 16 tokens of row block I and channels 32w .. 32w+31, spread over its
+// lanes in 8 x 8 pieces: lane l holds channels l/4 + {0, 8, 16, 24} and tokens 2(l%4) + {0, 1, 8, 9}.  That is what
+// tcgen05.ld.16x256b reads, ldmatrix.trans takes from a [token][channel] tile and stmatrix puts back, transposed or not.
 //
 // Products (all on tcgen05; "^T" = channel-major result, M = 128; token x token results use M = 64):
 //   dR^T = H dO^T          dW^T = H dZ^T          dE^T = dH' Z^T            (H, dH' V-first panels: MN-major A)
@@ -27,30 +28,55 @@ int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
 
 namespace {
 
-__device__ __forceinline__ uint32_t pk2(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
 // one MUFU: the operands here are decay factors in [e^-75, 1], far from the flush-to-zero and overflow ends
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float ld16(const uint8_t* base, uint32_t off) {
-    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + off));
-}
-// element (row r, column d) of a 128-byte-swizzled panel whose 64-column blocks are blk_bytes apart
-__device__ __forceinline__ uint32_t eoff(int r, int d, uint32_t blk_bytes) {
-    return (uint32_t)(d >> 6) * blk_bytes + sw128_off(r, (d & 63) >> 3) + (uint32_t)(d & 7) * 2;
-}
-// 32 lanes x 16 consecutive columns, as pairs of adjacent columns (here: adjacent tokens)
-__device__ __forceinline__ void tmem_ld_pairs(uint32_t taddr, f2 (&f)[8]) {
-    uint32_t r[16];
-    tmem_ld16(taddr, r);
+// Eight 8 x 8 pieces a lane, as pairs of adjacent columns (tokens): x[2c + n] is row l/4 + 8c, columns 8n + 2(l%4) + {0, 1}
+__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, f2* x) {      // 16 lanes x 16 columns: x[0..3]
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
     tmem_ld_wait();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = f2_make(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) x[2 * hf + n] = f2_make(__uint_as_float(r[4 * n + 2 * hf]), __uint_as_float(r[4 * n + 2 * hf + 1]));
+}
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, f2 (&x)[8]) {      // 32 lanes x 16 columns
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+                 "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr), "r"(taddr + (16u << 16))
+                 : "memory");
+    tmem_ld_wait();
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf)
+                x[4 * m + 2 * hf + n] = f2_make(__uint_as_float(r[8 * m + 4 * n + 2 * hf]), __uint_as_float(r[8 * m + 4 * n + 2 * hf + 1]));
+}
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t* w) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t* w) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void stsm_x4(uint32_t addr, const uint32_t* w) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+__device__ __forceinline__ void stsm_x4_t(uint32_t addr, const uint32_t* w) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
 __device__ __forceinline__ f2 rcp_2(f2 a) {
     const float2 x = f2_get(a);
@@ -62,8 +88,18 @@ __device__ __forceinline__ f2 ld_2(const float* p) {
     const float2 v = *reinterpret_cast<const float2*>(p);
     return f2_make(v.x, v.y);
 }
-__device__ __forceinline__ uint4 pack_quad(const f2 (&a)[8], int e) {
-    return make_uint4(f2_to_bf16(a[e]), f2_to_bf16(a[e + 1]), f2_to_bf16(a[e + 2]), f2_to_bf16(a[e + 3]));
+// Sum over the lanes of a quad that come before this one (0 in the first), and after it (0 in the last)
+__device__ __forceinline__ float quad_before(float p, int c4) {
+    float a = __shfl_up_sync(0xffffffffu, p, 1, 4);
+    a = c4 >= 1 ? a : 0.f;
+    const float b = __shfl_up_sync(0xffffffffu, a + p, 2, 4);
+    return c4 >= 2 ? a + b : a;
+}
+__device__ __forceinline__ float quad_after(float p, int c4) {
+    float a = __shfl_down_sync(0xffffffffu, p, 1, 4);
+    a = c4 <= 2 ? a : 0.f;
+    const float b = __shfl_down_sync(0xffffffffu, a + p, 2, 4);
+    return c4 <= 1 ? a + b : a;
 }
 
 }  // namespace
@@ -87,22 +123,25 @@ constexpr int kR1 = 0;         // 64 KB  H | dH' panels            -> later: k~_
 constexpr int kR2 = 65536;     // 16 KB  dO tile                   -> later: X^T tile (8 KB) | Y tile (8 KB)
 constexpr int kR3 = 81920;     // 16 KB  Z^T panel                 -> later: target stacks I = 0,1 (2 x 8 KB)
 constexpr int kR4 = 98304;     // 16 KB  dZ^T panel                -> later: target stacks I = 2,3
-constexpr int kR5 = 114688;    // 48 KB  q | k | v tiles
+constexpr int kR5 = 114688;    // 48 KB  q | k | v tiles           -> later: dv in the v tile
 constexpr int kR6 = 163840;    //  8 KB  T
 constexpr int kR7 = 172032;    // 16 KB  dW^T                      -> later: [dA_I ; beta dM_I] tiles (4 x 4 KB)
-constexpr int kR8 = 188416;    // 16 KB  Q' = e^G k
+constexpr int kR8 = 188416;    // 16 KB  g tile (bf16 gates)       -> later: Q' = e^G k
 constexpr int kRM = 204800;    //  8 KB  M~ (before beta), row-major [target][source]
-constexpr int kSmall = 212992; // floats: gsum[4][128] cref[4][128] part[8][128] tot[4][128] dots[64][8] rowv[3][64]
-constexpr int kIntraBwdSmem = kSmall + ((4 + 4 + 8 + 4) * 128 + 64 * 8 + 3 * 64) * 4 + 1024;
+// floats: gfirst[4][128] gsum[4][128] eC[4][128] eEnd[4][128] fb[4][128] part[4][128] egend[128] dots[2][4][64] rowv[3][64] rowb[2][64]
+constexpr int kSmall = 212992;
+constexpr int kIntraBwdSmem = kSmall + (24 * 128 + 128 + 512 + 3 * 64 + 2 * 64) * 4 + 1024;
 
 // Bound by latency: 225 KB of shared memory allow one CTA per SM, and its products depend on one another (state products
 // -> X -> Y -> dM -> pull-back).  So (1) only the operand of the next product is read out before that product is issued,
 // and everything else - dv, the dR / dE / dQ contributions, the pull-back's decay panels - runs while it is in flight;
 // (2) of the six state products the two that the next phase needs are issued first, the others by warps that have finished
 // their share of the work beside them; (3) a warp fetches the inputs
-// of the CTA that this SM is likely to run next into L2; (4) token pairs go through packed float32 arithmetic.
-// 16,384 chunk-heads: 2,262 -> 1,733 us (7 % of it the prefetch), 384: 81 -> 61 us.  A persistent form that loads the next
-// chunk-head's panels during the gradient assembly took 1,830: the loads are not what it waits for any more.
+// of the CTA that this SM is likely to run next into L2; (4) token pairs go through packed float32 arithmetic; (5) a lane's
+// elements lie in 8 x 8 pieces, so that tiles are read and written by ldmatrix / stmatrix, four pieces an instruction, a row
+// scalar serves eight of its elements and a row dot takes 7 shuffles: with a channel and 16 tokens a lane, its 2-byte accesses, row
+// scalars and 31 shuffles had been a quarter of a block's cycles.
+// 16,384 chunk-heads: 1,725 -> 1,490 us, 384: 65 -> 56 us (2,262 and 81 before (1) to (4)).
 template <bool GB>
 __global__ void __launch_bounds__(512, 1)
     tc_intra_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
@@ -110,7 +149,7 @@ __global__ void __launch_bounds__(512, 1)
                         const __grid_constant__ CUtensorMap mT, const __grid_constant__ CUtensorMap mH,
                         const __grid_constant__ CUtensorMap mdH, const __grid_constant__ CUtensorMap mZT,
                         const __grid_constant__ CUtensorMap mdZT, const __grid_constant__ CUtensorMap mMt,
-                        IntraBwdArgs p) {
+                        const __grid_constant__ CUtensorMap mg, IntraBwdArgs p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
     uint8_t* Hs = sm + kR1;
@@ -125,13 +164,19 @@ __global__ void __launch_bounds__(512, 1)
     uint8_t* dWs = sm + kR7;
     uint8_t* Qp = sm + kR8;
     uint8_t* Mts = sm + kRM;
-    float* gsum = reinterpret_cast<float*>(sm + kSmall);   // [4][128] block sums of g
-    float* cref = gsum + 512;                              // [4][128] G at the first row of each block
-    float* part = cref + 512;                              // [8][128] partial sums of dD
-    float* tot = part + 1024;                              // [4][128] block sums of dG
-    float* dots = tot + 512;                               // [2][4][64] row dots: q | k, channel quarter, row
-    float* rowv = dots + 512;                              // [3][64]  qinv | kinv | beta
-    __shared__ uint64_t bar_in[2], bar_w, bar_p1, bar_x, bar_q, bar_y, bar_m, bar_pb;
+    float* gfirst = reinterpret_cast<float*>(sm + kSmall); // [4][128] g of the first row of each block
+    float* gsum = gfirst + 512;                            // [4][128] sum of g over a block's other rows
+    float* eC = gsum + 512;                                // [4][128] e^{c_I}, c_I = G at the first row of block I
+    float* eEnd = eC + 512;                                // [4][128] e^{G_end - c_I}
+    float* fbk = eEnd + 512;                               // [3][128] e^{c_{I+1} - c_I}
+    float* part = fbk + 512;                               // [4][128] partial sums of dD
+    float* egend = part + 512;                             // [128]
+    float* dots = egend + 128;                             // [2][4][64] row dots: q | k, channel quarter, row
+    float* rowv = dots + 512;                              // [3][64]  qinv * scale | kinv | beta
+    float* rowb = rowv + 192;                              // [2][64]  what the row dots take off q and k, per unit row
+    float* tot = gsum;                                     // [4][128] block sums of dG (the sums of g are done with)
+    float* ge = gfirst;                                    // [4][128] block sums of dE * E
+    __shared__ uint64_t bar_g, bar_in[2], bar_w, bar_x, bar_q, bar_y, bar_r, bar_m, bar_pb;
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) float dA_diag[64];      // dA[i][i]: applied to dq, dk in float32, outside the pull-back products
 
@@ -140,22 +185,52 @@ __global__ void __launch_bounds__(512, 1)
     if (len == 0) return;
     const int ch = slot * H + h;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int I = warp >> 2;             // row block of this thread
-    const int d = tid & 127;             // channel (and TMEM lane) of this thread
+    const int I = warp >> 2, wq = warp & 3;       // row block and channel quarter of this warp
+    const int c4 = lane & 3, r8 = lane >> 2;      // token pair and channel inside an 8 x 8 piece
+    const int mi = lane >> 3, mr = lane & 7;      // the piece and row whose address this lane gives to ldmatrix / stmatrix
+    const int tb = 16 * I + 2 * c4;               // this lane's tokens: tb + {0, 1, 8, 9}
+    const int cb = 32 * wq + r8;                  // this lane's channels: cb + {0, 8, 16, 24}
+    const uint32_t sb = smem_u32(sm);
+    // offsets of the pieces: [token][channel] tile (channels + 16: ^ 32), [channel][token] panel (channels + 16: + 2048), tile of
+    // 64 rows whose 16 rows 16wq .. belong to this warp; `chunk` is the 16-byte column of the block's first eight tokens
+    const uint32_t tile_off = (uint32_t)(wq >> 1) * 8192 + sw128_off(16 * I + 8 * (mi & 1) + mr, 4 * (wq & 1) + (mi >> 1));
+    auto panel_off = [&](int chunk) { return sw128_off(32 * wq + 8 * (mi >> 1) + mr, chunk + (mi & 1)); };
+    const uint32_t row_off = sw128_off(16 * wq + 8 * (mi >> 1) + mr, 2 * I + (mi & 1));
+    auto put_panel = [&](uint32_t panel, int chunk, const f2 (&x)[8]) {
+        uint32_t w[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = f2_to_bf16(x[e]);
+        const uint32_t a = panel + panel_off(chunk);
+        stsm_x4(a, w);
+        stsm_x4(a + 2048, w + 4);
+    };
+    auto put_tile = [&](uint32_t tile, const f2 (&x)[8]) {
+        uint32_t w[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = f2_to_bf16(x[e]);
+        stsm_x4_t(tile + tile_off, w);
+        stsm_x4_t(tile + (tile_off ^ 32u), w + 4);
+    };
+    auto get_tile = [&](uint32_t tile, uint32_t (&w)[8]) {
+        ldsm_x4_t(tile + tile_off, w);
+        ldsm_x4_t(tile + (tile_off ^ 32u), w + 4);
+    };
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
-    // The first barrier covers what the critical products and the work beside them need.  The loads are issued by warps 1-4,
-    // four each, after their gate loads: one thread issuing all of them held the block back.
+    // The gates come first, then what the critical products and the work beside them need.  The loads are issued by warps 1-4,
+    // a few each: one thread issuing all of them held the block back.
     if (tid == 0) {
+        mbar_init(&bar_g, 1);
         mbar_init(&bar_in[0], 1);
         mbar_init(&bar_in[1], 1);
         mbar_init(&bar_w, 1);
-        mbar_init(&bar_p1, 4);
+        mbar_init(&bar_r, 1);
         mbar_init(&bar_x, 1);
         mbar_init(&bar_q, 1);
         mbar_init(&bar_y, 1);
         mbar_init(&bar_m, 1);
         mbar_init(&bar_pb, 4);
+        if (GB) mbar_expect_tx(&bar_g, 16384);
         mbar_expect_tx(&bar_in[0], 32768 + 16384 * 4);
         mbar_expect_tx(&bar_in[1], 32768 + 16384 * 2 + 8192 * 2);
         mbar_fence_init();
@@ -163,96 +238,130 @@ __global__ void __launch_bounds__(512, 1)
     __syncthreads();
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
 
-    // ---- per-row scalars and the cumulative log-decay of this thread's 16 rows
+    if (warp >= 1 && warp <= 4 && lane == 0) {
+        if (warp == 1) {
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_in[0], mb * 64, ch * 128);
+            tma_load_2d(dZTs, &mdZT, &bar_in[0], 0, ch * 128);
+            tma_load_2d(Ts, &mT, &bar_in[1], 0, ch * 64);
+        } else if (warp == 2) {
+            for (int mb = 0; mb < 2; ++mb) {
+                tma_load_2d(vs + mb * 8192, &mv, &bar_in[0], h * 128 + mb * 64, tok0);
+                tma_load_2d(dOs + mb * 8192, &mdO, &bar_in[1], h * 128 + mb * 64, tok0);
+            }
+        } else if (warp == 3) {
+            if (GB)
+                for (int mb = 0; mb < 2; ++mb) tma_load_2d(Qp + mb * 8192, &mg, &bar_g, h * 128 + mb * 64, tok0);
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(ks + mb * 8192, &mk, &bar_in[0], h * 128 + mb * 64, tok0);
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_in[1], mb * 64, ch * 128);
+        } else {
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(qs + mb * 8192, &mq, &bar_in[0], h * 128 + mb * 64, tok0);
+            tma_load_2d(ZTs, &mZT, &bar_in[1], 0, ch * 128);
+            tma_load_2d(Mts, &mMt, &bar_in[1], 0, ch * 64);
+        }
+    }
+    __syncwarp();
+    // ---- per-row scalars and the log-decay relative to the block's first row
     if (tid < 64) {
-        rowv[tid] = p.qinv[ch * 64 + tid];
+        rowv[tid] = p.qinv[ch * 64 + tid] * p.scale;
         rowv[64 + tid] = p.kinv[ch * 64 + tid];
         rowv[128 + tid] = p.beta[ch * 64 + tid];
     }
-    const size_t rstride = (size_t)H * 128;
-    const size_t col = ((size_t)tok0 * H + h) * 128 + d;
-    float G[16];
-    {
+    bool ok = true;
+    f2 E[8];
+    if constexpr (GB) {
+        uint32_t w[8];
+        ok = mbar_wait(&bar_g, 0, p.status, 40);
+        get_tile(sb + kR8, w);
 #pragma unroll
-        for (int r = 0; r < 16; ++r) G[r] = ld_io(p.g, col + (size_t)min(16 * I + r, len - 1) * rstride, GB);
-        if (lane == 0) {
-            if (warp == 1) {
-                for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_in[0], mb * 64, ch * 128);
-                tma_load_2d(dZTs, &mdZT, &bar_in[0], 0, ch * 128);
-                tma_load_2d(Ts, &mT, &bar_in[1], 0, ch * 64);
-            } else if (warp == 2) {
-                for (int mb = 0; mb < 2; ++mb) {
-                    tma_load_2d(vs + mb * 8192, &mv, &bar_in[0], h * 128 + mb * 64, tok0);
-                    tma_load_2d(dOs + mb * 8192, &mdO, &bar_in[1], h * 128 + mb * 64, tok0);
-                }
-            } else if (warp == 3) {
-                for (int mb = 0; mb < 2; ++mb) tma_load_2d(ks + mb * 8192, &mk, &bar_in[0], h * 128 + mb * 64, tok0);
-                for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_in[1], mb * 64, ch * 128);
-            } else if (warp == 4) {
-                for (int mb = 0; mb < 2; ++mb) tma_load_2d(qs + mb * 8192, &mq, &bar_in[0], h * 128 + mb * 64, tok0);
-                tma_load_2d(ZTs, &mZT, &bar_in[1], 0, ch * 128);
-                tma_load_2d(Mts, &mMt, &bar_in[1], 0, ch * 64);
-            }
+        for (int e = 0; e < 8; ++e) {
+            const float2 x = f2_get(f2_from_bf16(w[e]));
+            const int i = tb + 8 * (e & 1);
+            E[e] = f2_make(i < len ? x.x : 0.f, i + 1 < len ? x.y : 0.f);
         }
-        __syncwarp();
-        float run = 0.f;
+    } else {
+        const float* gp = static_cast<const float*>(p.g) + ((size_t)tok0 * H + h) * 128 + cb;
+        const size_t rstride = (size_t)H * 128;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            run += (16 * I + r < len) ? G[r] : 0.f;
-            G[r] = run;
+        for (int e = 0; e < 8; ++e) {
+            const int i = tb + 8 * (e & 1);
+            const float a = gp[(size_t)min(i, len - 1) * rstride + 8 * (e >> 1)], b = gp[(size_t)min(i + 1, len - 1) * rstride + 8 * (e >> 1)];
+            E[e] = f2_make(i < len ? a : 0.f, i + 1 < len ? b : 0.f);
         }
-        gsum[I * 128 + d] = run;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        float2 g0 = f2_get(E[2 * c]), g1 = f2_get(E[2 * c + 1]);
+        if (c4 == 0) {
+            gfirst[I * 128 + cb + 8 * c] = g0.x;
+            g0.x = 0.f;
+        }
+        const float p0 = g0.x + g0.y, p1 = g1.x + g1.y;
+        const float b0 = quad_before(p0, c4);
+        const float b1 = quad_before(p1, c4) + __shfl_sync(0xffffffffu, b0 + p0, 3, 4);
+        if (c4 == 3) gsum[I * 128 + cb + 8 * c] = b1 + p1;
+        E[2 * c] = f2_make(b0 + g0.x, b0 + p0);
+        E[2 * c + 1] = f2_make(b1 + g1.x, b1 + p1);
     }
     tc_fence_before();
-    __syncthreads();
+    ok = __syncthreads_and(ok);
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    // Only decay factors relative to this thread's own block reference cI = G[first row of the block] are needed:
-    // E[r] = e^{G[r] - cI} (in (0, 1], at least e^-75), its reciprocal, and the two per-thread scalars that move the
-    // reference to the chunk start (e^{cI}) and to the chunk end (e^{gend - cI}).  One exponential per row instead of
-    // eight, and the operand panels and the gradient assembly use bit-identical factors by construction.
-    float egend, eEndI;
-    f2 eCI, E[8];
+    // Only decay factors relative to a block's own reference c_I = G[first row of the block] are needed per element:
+    // E = e^{G - c_I} (in (0, 1], at least e^-75) and its reciprocal; per block and channel there are the factors that move the
+    // reference to the chunk start, the chunk end and the next block.  The operand panels and the gradient assembly use
+    // bit-identical factors by construction.
     {
-        const float s0 = gsum[d], s1 = gsum[128 + d], s2 = gsum[256 + d], s3 = gsum[384 + d];
-        const float pre = I == 0 ? 0.f : (I == 1 ? s0 : (I == 2 ? s0 + s1 : s0 + s1 + s2));
-        const float gend = s0 + s1 + s2 + s3;
+        const int dd = tid & 127;
+        float after = 0.f, before = 0.f;           // log-decay from the next block's first row to the end; before this block
 #pragma unroll
-        for (int r = 0; r < 16; ++r) G[r] += pre;
-        const float cI = G[0];
-        cref[I * 128 + d] = cI;
-        egend = __expf(gend);
-        eEndI = __expf(gend - cI);
-        eCI = f2_all(__expf(cI));
-#pragma unroll
-        for (int e = 0; e < 8; ++e) E[e] = f2_make(__expf(G[2 * e] - cI), __expf(G[2 * e + 1] - cI));
+        for (int j = 0; j < 4; ++j) {
+            const float sj = gfirst[j * 128 + dd] + gsum[j * 128 + dd];
+            before += j < I ? sj : 0.f;
+            after += j > I ? sj : 0.f;
+        }
+        const float first = gfirst[I * 128 + dd], rest = gsum[I * 128 + dd];
+        eC[tid] = __expf(before + first);
+        eEnd[tid] = __expf(rest + after);
+        fbk[tid] = I < 3 ? __expf(rest + gfirst[min(I + 1, 3) * 128 + dd]) : 0.f;
+        if (I == 0) egend[dd] = __expf(first + rest + after);
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float2 x = f2_get(E[e]);
+        E[e] = f2_make(__expf(x.x), __expf(x.y));
+    }
+    auto chan4 = [&](float (&x)[4], const float* tbl) {      // a [128] table at this lane's channels
+#pragma unroll
+        for (int c = 0; c < 4; ++c) x[c] = tbl[cb + 8 * c];
+    };
 
     // TMEM columns
-    constexpr uint32_t cR = 0, cW = 64, cA = 128, cP = 192, cX = 256, cE = 384, cQ = 448, cY = cP, cM = cW;
+    constexpr uint32_t cR = 0, cW = 64, cA = 128, cP = 192, cX = 256, cY = 320, cE = 384, cQ = 448, cM = cW;
 
-    bool ok = true;
     if (len < 64) {
-        // rows past a ragged tail hold the next sequence's tokens: blank them in the dO and v tiles, which feed UMMAs
-        // as they are (0 x Inf would otherwise reach this sequence's gradients)
-        ok = mbar_wait(&bar_in[0], 0, p.status, 40) && mbar_wait(&bar_in[1], 0, p.status, 40);
+        // rows past a ragged tail hold the next sequence's tokens: blank them (0 x Inf would otherwise reach this sequence's
+        // gradients)
+        ok = ok && mbar_wait(&bar_in[0], 0, p.status, 40) && mbar_wait(&bar_in[1], 0, p.status, 40);
         if (ok) {
             for (int idx = tid; idx < (64 - len) * 16; idx += 512) {
                 const int r = len + (idx >> 4), c = idx & 15;
                 const uint32_t off = (uint32_t)(c >> 3) * 8192 + sw128_off(r, c & 7);
                 *reinterpret_cast<uint4*>(dOs + off) = make_uint4(0, 0, 0, 0);
                 *reinterpret_cast<uint4*>(vs + off) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(qs + off) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(ks + off) = make_uint4(0, 0, 0, 0);
             }
         }
         fence_async_smem();
-        ok = __syncthreads_and(ok);
     }
+    ok = __syncthreads_and(ok);                    // tables; the g tile has been read
 
     // ================================================================ phase 1: state products
-    // dW and the first half of X are what the next product waits for: they go first.  The others follow from warps that
-    // have finished their share of the work beside them (a thread that issues into a full queue is held until it drains).
+    // One thread issues the products, and they run in that order: dW and the first half of X, what the next link of the chain
+    // X -> Y -> dM waits for, go first; the five others (~300 cycles each of operand reads) go where the chain's next product
+    // is still being prepared.  Issued all at once from four warps they held those warps, and with them the block, back.
     ok = ok && mbar_wait(&bar_in[0], 0, p.status, 40);
-    if (ok && tid == 0) {
+    if (ok && tid == 384) {
         tc_fence_after();
         const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
         const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
@@ -269,84 +378,74 @@ __global__ void __launch_bounds__(512, 1)
     }
     __syncwarp();
     // while the tensor core works: this thread's q and k, the Q' operand, and dD[d] = sum_v dH'[d][v] H[d][v]
-    uint32_t qw[8], kw[8];
-    // unit k and scaled unit q of this thread's rows from their bf16 words
-    auto unit_k = [&](f2 (&x)[8], const uint32_t (&w)[8]) {
+    // Unit k and scaled unit q of this lane's elements come from their tiles each time they are needed: at 128 registers a
+    // thread q, k, the decay factors and three gradients do not fit together, and beside 226 KB of shared memory too little
+    // L1 is left to spill into (it goes to L2).
+    auto unit = [&](f2 (&x)[8], uint32_t tile, const float* row) {
+        uint32_t w[8];
+        get_tile(sb + tile, w);
+        const f2 s[2] = {ld_2(row + tb), ld_2(row + tb + 8)};
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = f2_mul(f2_from_bf16(w[e]), ld_2(rowv + 64 + 16 * I + 2 * e));
+        for (int e = 0; e < 8; ++e) x[e] = f2_mul(f2_from_bf16(w[e]), s[e & 1]);
     };
-    auto unit_q = [&](f2 (&x)[8], const uint32_t (&w)[8]) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = f2_mul(f2_from_bf16(w[e]), f2_mul(ld_2(rowv + 16 * I + 2 * e), f2_all(p.scale)));
-    };
+    constexpr uint32_t kQt = kR5, kKt = kR5 + 16384;
     {
-        const int nv = ok ? len - 16 * I : 0;            // this thread's rows inside the chunk
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int i = 16 * I + 2 * e;
-            uint32_t q0 = 0, q1 = 0, k0 = 0, k1 = 0;
-            if (2 * e < nv) {
-                q0 = *reinterpret_cast<const uint16_t*>(qs + eoff(i, d, 8192));
-                k0 = *reinterpret_cast<const uint16_t*>(ks + eoff(i, d, 8192));
-            }
-            if (2 * e + 1 < nv) {
-                q1 = *reinterpret_cast<const uint16_t*>(qs + eoff(i + 1, d, 8192));
-                k1 = *reinterpret_cast<const uint16_t*>(ks + eoff(i + 1, d, 8192));
-            }
-            qw[e] = q0 | (q1 << 16);
-            kw[e] = k0 | (k1 << 16);
-        }
-        // Q' = e^G k for Xraw^T -= Q' dW^T, stored [key d][token] (MN-major A): this thread's 16 tokens are 32
-        // contiguous bytes of row d
+        // Q' = e^G k for Xraw^T -= Q' dW^T, stored [key d][token] (MN-major A)
         f2 w[8];
-        unit_k(w, kw);
+        float ec[4];
+        chan4(ec, eC + I * 128);
+        unit(w, kKt, rowv + 64);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = f2_mul(f2_mul(E[e], eCI), w[e]);
-        *reinterpret_cast<uint4*>(Qp + sw128_off(d, 2 * I)) = pack_quad(w, 0);
-        *reinterpret_cast<uint4*>(Qp + sw128_off(d, 2 * I + 1)) = pack_quad(w, 4);
+        for (int e = 0; e < 8; ++e) w[e] = f2_mul(f2_mul(E[e], f2_all(ec[e >> 1])), w[e]);
+        put_panel(sb + kR8, 2 * I, w);
         ok = ok && mbar_wait(&bar_in[1], 0, p.status, 40);
-        // two adjacent channels and 16 value rows a thread
-        f2 acc = f2_all(0.f);
-        const int d2 = 2 * (tid & 63), vg = tid >> 6;
+        // eight adjacent channels of four value rows a lane; the warp's eight lanes that share them add up by halving
+        const int cg = 4 * wq + mi;
+        f2 acc[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] = f2_all(0.f);
         if (ok) {
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const uint32_t off = eoff(16 * vg + r, d2, 16384);
-                acc = f2_fma(f2_from_bf16(*reinterpret_cast<const uint32_t*>(Hs + off)),
-                             f2_from_bf16(*reinterpret_cast<const uint32_t*>(dHs + off)), acc);
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t off = (uint32_t)(cg >> 3) * 16384 + sw128_off(32 * I + 8 * j + mr, cg & 7);
+                const uint4 a = *reinterpret_cast<const uint4*>(Hs + off), b = *reinterpret_cast<const uint4*>(dHs + off);
+                acc[0] = f2_fma(f2_from_bf16(a.x), f2_from_bf16(b.x), acc[0]);
+                acc[1] = f2_fma(f2_from_bf16(a.y), f2_from_bf16(b.y), acc[1]);
+                acc[2] = f2_fma(f2_from_bf16(a.z), f2_from_bf16(b.z), acc[2]);
+                acc[3] = f2_fma(f2_from_bf16(a.w), f2_from_bf16(b.w), acc[3]);
             }
         }
-        *reinterpret_cast<float2*>(part + vg * 128 + d2) = f2_get(acc);
-    }
-    if (ok && (warp & 3) == 3 && lane == 0) {
-        tc_fence_after();
-        const uint32_t aH = smem_u32(Hs), adH = smem_u32(dHs), bdO = smem_u32(dOs), bZ = smem_u32(ZTs), bdZ = smem_u32(dZTs), bT = smem_u32(Ts);
-        if (warp == 3) {
-            const uint32_t id_k_mn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
+        float v8[8];
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16)     // dP^T = dZ^T T
-                umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(bdZ + k16 * 32, 16, 1024),
-                             umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
-        } else if (warp == 7) {
-            const uint32_t id_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dR^T = H dO^T
-                umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
-                             umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), id_mn_k, k16 > 0);
-        } else if (warp == 11) {
-            const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dA = dO Z^T                      (M = 64)
-                umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
-        } else {
-            const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
-#pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16)     // dE^T = dH' Z^T
-                umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(adH + k16 * 2048, 16384, 1024),
-                             umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
+        for (int e = 0; e < 4; ++e) {
+            const float2 x = f2_get(acc[e]);
+            v8[2 * e] = x.x;
+            v8[2 * e + 1] = x.y;
         }
-        umma_commit(&bar_p1);
+#pragma unroll
+        for (int o = 4; o >= 1; o >>= 1) {
+            const bool up = (mr & o) != 0;
+#pragma unroll
+            for (int j = 0; j < o; ++j) {
+                const float send = up ? v8[j] : v8[j + o], keep = up ? v8[j + o] : v8[j];
+                v8[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        part[I * 128 + 8 * cg + mr] = v8[0];
+    }
+    if (ok && tid == 384) {
+        tc_fence_after();
+        const uint32_t aH = smem_u32(Hs), bdO = smem_u32(dOs), bZ = smem_u32(ZTs);
+        const uint32_t id_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
+        const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
+#pragma unroll
+        for (int k16 = 0; k16 < 8; ++k16)     // dR^T = H dO^T
+            umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
+                         umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), id_mn_k, k16 > 0);
+#pragma unroll
+        for (int k16 = 0; k16 < 8; ++k16)     // dA = dO Z^T                      (M = 64)
+            umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
+                         umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
     }
     __syncwarp();
     ok = ok && mbar_wait(&bar_w, 0, p.status, 41);
@@ -354,15 +453,14 @@ __global__ void __launch_bounds__(512, 1)
 
     // ================================================================ phase 2: X and dQ
     {
-        f2 t[8];      // dW^T -> bf16 operand (row = channel d, 16 of its 64 tokens)
-        tmem_ld_pairs(tmem + lane_base + cW + 16 * I, t);
-        *reinterpret_cast<uint4*>(dWs + sw128_off(d, 2 * I)) = pack_quad(t, 0);
-        *reinterpret_cast<uint4*>(dWs + sw128_off(d, 2 * I + 1)) = pack_quad(t, 4);
+        f2 t[8];      // dW^T -> bf16 operand (row = channel d)
+        tmem_ld_32x16(tmem + lane_base + cW + 16 * I, t);
+        put_panel(sb + kR7, 2 * I, t);
     }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (ok && tid == 0) {
+    if (ok && tid == 384) {
         tc_fence_after();
         const uint32_t id64_neg = umma_idesc_bf16(64, 64, kMajorMN, kMajorMN, 1);
         const uint32_t id_k_mn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
@@ -376,152 +474,129 @@ __global__ void __launch_bounds__(512, 1)
         for (int k16 = 0; k16 < 4; ++k16)     // (T^T dW)^T = dW^T T ;  dQ = -that
             umma_bf16_ss(tmem + cQ, umma_smem_desc_sw128(aW + k16 * 32, 16, 1024),
                          umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
+#pragma unroll
+        for (int k16 = 0; k16 < 4; ++k16)     // dP^T = dZ^T T
+            umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(smem_u32(dZTs) + k16 * 32, 16, 1024),
+                         umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
         umma_commit(&bar_q);
     }
     __syncwarp();
-    // The q and k tiles have been read by everyone: they become thread-private slots for these words.  At 128 registers a
-    // thread q, k, the decay factors and three gradients do not fit together, and beside 225 KB of shared memory too little
-    // L1 is left to spill into (it went to L2).
-    uint4* qslot = reinterpret_cast<uint4*>(qs) + tid;
-    uint4* kslot = reinterpret_cast<uint4*>(ks) + tid;
-    qslot[0] = make_uint4(qw[0], qw[1], qw[2], qw[3]);
-    qslot[512] = make_uint4(qw[4], qw[5], qw[6], qw[7]);
-    kslot[0] = make_uint4(kw[0], kw[1], kw[2], kw[3]);
-    kslot[512] = make_uint4(kw[4], kw[5], kw[6], kw[7]);
-    auto get_q = [&](f2 (&x)[8]) {
-        const uint4 a = qslot[0], b = qslot[512];
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        unit_q(x, w);
-    };
-    auto get_k = [&](f2 (&x)[8]) {
-        const uint4 a = kslot[0], b = kslot[512];
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        unit_k(x, w);
-    };
-    ok = ok && mbar_wait(&bar_p1, 0, p.status, 41);
-    tc_fence_after();
-    f2 dqn[8], dG[8];
-    {
-        f2 t[8];
-        // in flight: dv = beta dP, staged [token][channel] in the value tile (only the completed products read it) so that
-        // it leaves as 16-byte row segments, and the dR part of dq
-        tmem_ld_pairs(tmem + lane_base + cP + 16 * I, t);
-        __nv_bfloat16* tv = reinterpret_cast<__nv_bfloat16*>(vs) + 16 * I * 128 + d;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const uint32_t u = f2_to_bf16(f2_mul(ld_2(rowv + 128 + 16 * I + 2 * e), t[e]));
-            const __nv_bfloat162 b2 = *reinterpret_cast<const __nv_bfloat162*>(&u);
-            tv[2 * e * 128] = b2.x;
-            tv[(2 * e + 1) * 128] = b2.y;
-        }
-        tmem_ld_pairs(tmem + lane_base + cR + 16 * I, t);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            dqn[e] = f2_mul(t[e], f2_mul(E[e], eCI));
-        }
-        unit_q(t, qw);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) dG[e] = f2_mul(dqn[e], t[e]);
-    }
     ok = ok && mbar_wait(&bar_x, 0, p.status, 42);
     tc_fence_after();
 
     // ================================================================ phase 3: Y, dM
-    // M = 64 accumulators keep row (16*w + l) in lane l < 16 of warp w < 4.  tcgen05.ld is warp-collective, so all 32
-    // lanes of those warps run the loads; lanes >= 16 mirror a row and never store.  All four warp groups see the same lanes, so each takes 16 of the 64 columns.
-    const bool rowown = lane < 16;
-    const int row = 16 * (warp & 3) + (lane & 15);
-    uint8_t* XT = sm + kR2;           // [64 rows s][64 i]   K-major B
-    uint8_t* Yt = sm + kR2 + 8192;    // [64 rows j][64 s]   K-major A
-    float dbeta_acc = 0.f;
+    // M = 64 accumulators keep row (16*w + l) in lane l < 16 of warp w < 4: a 16-lane read takes them whole.  All four warp groups
+    // see the same lanes, so each takes 16 of the 64 columns; a lane holds rows row0 and row0 + 8, x[2 hf + n].
+    const int row0 = 16 * wq + r8;
+    constexpr uint32_t kXT = kR2;           // [64 rows s][64 i]   K-major B
+    constexpr uint32_t kYt = kR2 + 8192;    // [64 rows j][64 s]   K-major A
+    auto put_rows = [&](uint32_t tile, const f2 (&x)[4]) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = f2_to_bf16(x[e]);
+        stsm_x4(tile + row_off, w);
+    };
+    float dbeta_acc[2];
     float* dbp = reinterpret_cast<float*>(Qp);      // [4][64] partial dbeta per column group (Q' has been read once X is complete)
     {
-        const f2 bs = f2_all(rowv[128 + row]);
-        f2 t[8], acc = f2_all(0.f);
-        tmem_ld_pairs(tmem + lane_base + cX + 16 * I, t);
+        f2 t[4];
+        tmem_ld_16x16(tmem + lane_base + cX + 16 * I, t);
+        uint32_t tw[4];                             // T[i][s] in the accumulator's order (rows s)
+        ldsm_x4_t(sb + kR6 + sw128_off(16 * I + 8 * (mi & 1) + mr, 2 * wq + (mi >> 1)), tw);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int i = 16 * I + 2 * e;
-            acc = f2_fma(f2_make(ld16(Ts, sw128_off(i, row >> 3) + (row & 7) * 2), ld16(Ts, sw128_off(i + 1, row >> 3) + (row & 7) * 2)),
-                         t[e], acc);                                                   // T[i][s] * Xraw[i][s]
-            t[e] = f2_mul(bs, t[e]);
+        for (int hf = 0; hf < 2; ++hf) {
+            const f2 bs = f2_all(rowv[128 + row0 + 8 * hf]);
+            const float2 a = f2_get(f2_fma(f2_from_bf16(tw[2 * hf]), t[2 * hf], f2_mul(f2_from_bf16(tw[2 * hf + 1]), t[2 * hf + 1])));   // T * Xraw
+            dbeta_acc[hf] = a.x + a.y;
+            t[2 * hf] = f2_mul(bs, t[2 * hf]);
+            t[2 * hf + 1] = f2_mul(bs, t[2 * hf + 1]);
         }
-        const float2 a = f2_get(acc);
-        dbeta_acc = a.x + a.y;
-        if (rowown) {
-            *reinterpret_cast<uint4*>(XT + sw128_off(row, 2 * I)) = pack_quad(t, 0);
-            *reinterpret_cast<uint4*>(XT + sw128_off(row, 2 * I + 1)) = pack_quad(t, 4);
-        }
+        put_rows(sb + kXT, t);
     }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (ok && tid == 0) {
+    if (ok && tid == 384) {
         tc_fence_after();
         const uint32_t id = umma_idesc_bf16(64, 64, kMajorMN, kMajorK);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)     // Y = T^T X : A[m=j][k=i] = T[i][j] (MN-major), B[n=s][k=i] = X^T rows
             umma_bf16_ss(tmem + cY, umma_smem_desc_sw128(smem_u32(Ts) + k16 * 2048, 8192, 1024),
-                         umma_smem_desc_sw128(smem_u32(XT) + k16 * 32, 16, 1024), id, k16 > 0);
+                         umma_smem_desc_sw128(sb + kXT + k16 * 32, 16, 1024), id, k16 > 0);
         umma_commit(&bar_y);
+        const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
+#pragma unroll
+        for (int k16 = 0; k16 < 8; ++k16)     // dE^T = dH' Z^T
+            umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(smem_u32(dHs) + k16 * 2048, 16384, 1024),
+                         umma_smem_desc_sw128(smem_u32(ZTs) + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
+        umma_commit(&bar_r);
     }
     __syncwarp();
+    ok = ok && mbar_wait(&bar_q, 0, p.status, 42);
+    tc_fence_after();
+    {
+        // in flight: dv = beta dP, staged [token][channel] in the value tile (only the completed products read it) so that
+        // it leaves as 16-byte row segments
+        f2 t[8];
+        tmem_ld_32x16(tmem + lane_base + cP + 16 * I, t);
+        const f2 bt[2] = {ld_2(rowv + 128 + tb), ld_2(rowv + 128 + tb + 8)};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) t[e] = f2_mul(bt[e & 1], t[e]);
+        put_tile(sb + kR5 + 32768, t);
+    }
+    ok = ok && mbar_wait(&bar_y, 0, p.status, 43);
+    tc_fence_after();
+    {
+        f2 t[4];
+        tmem_ld_16x16(tmem + lane_base + cY + 16 * I, t);
+        put_rows(sb + kYt, t);
+    }
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (ok && tid == 384) {
+        tc_fence_after();
+        const uint32_t id = umma_idesc_bf16(64, 64, kMajorK, kMajorK);
+#pragma unroll
+        for (int k16 = 0; k16 < 4; ++k16)     // Y T^T : B[n=l][k=s] = T[l][s]
+            umma_bf16_ss(tmem + cM, umma_smem_desc_sw128(sb + kYt + k16 * 32, 16, 1024),
+                         umma_smem_desc_sw128(smem_u32(Ts) + k16 * 32, 16, 1024), id, k16 > 0);
+        umma_commit(&bar_m);
+    }
+    __syncwarp();
+
     if (ok) {      // in flight: the dv rows leave
-        const __nv_bfloat16* tv = reinterpret_cast<const __nv_bfloat16*>(vs);
         const int c = tid & 15;
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
             const int i = pass * 32 + (tid >> 4);
             if (i < len)
                 *reinterpret_cast<uint4*>(p.dv + ((size_t)(tok0 + i) * H + h) * 128 + 8 * c) =
-                    *reinterpret_cast<const uint4*>(tv + i * 128 + 8 * c);
+                    *reinterpret_cast<const uint4*>(vs + (c >> 3) * 8192 + sw128_off(i, c & 7));
         }
     }
-    ok = ok && mbar_wait(&bar_y, 0, p.status, 43);
+    ok = ok && mbar_wait(&bar_r, 0, p.status, 42);       // every product up to dE is complete: its operands' tiles are free
     tc_fence_after();
-    {
-        f2 t[8];
-        tmem_ld_pairs(tmem + lane_base + cY + 16 * I, t);
-        if (rowown) {
-            *reinterpret_cast<uint4*>(Yt + sw128_off(row, 2 * I)) = pack_quad(t, 0);
-            *reinterpret_cast<uint4*>(Yt + sw128_off(row, 2 * I + 1)) = pack_quad(t, 4);
-        }
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (ok && tid == 0) {
-        tc_fence_after();
-        const uint32_t id = umma_idesc_bf16(64, 64, kMajorK, kMajorK);
-#pragma unroll
-        for (int k16 = 0; k16 < 4; ++k16)     // Y T^T : B[n=l][k=s] = T[l][s]
-            umma_bf16_ss(tmem + cM, umma_smem_desc_sw128(smem_u32(Yt) + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(smem_u32(Ts) + k16 * 32, 16, 1024), id, k16 > 0);
-        umma_commit(&bar_m);
-    }
-    __syncwarp();
 
     // ================================================================ phase 4: pull-back operands
     uint8_t* Sk = sm + kR1;           // k~_I source panels: [I][128 rows d][64 s], rows of blocks <= I only  K-major A
     uint8_t* Xk = sm + kR3;           // target stacks: [I / 2][128 rows d][32 rows of I even | 32 of I odd] K-major A
     uint8_t* DAt = sm + kR7;          // [I][32 rows: 16 dA rows, 16 beta*dM rows][64 s]   K-major / MN-major B
-    const int jb = row >> 4, jr = row & 15;
+    // this warp's 16 rows of dA or dM go to the tile of row block wq
+    const uint32_t da_off = kR7 + wq * 4096 + sw128_off(8 * (mi >> 1) + mr, 2 * I + (mi & 1));
     {
-        // in flight: the decay panels.  Both operand families are stored transposed, [channel d][row], so that this
-        // thread's 16 rows are contiguous bytes of row d and leave as 16-byte stores (K-major A operands).
-        uint8_t* X = Xk + (I >> 1) * 16384;      // two target blocks share a panel: 32 stack rows each
+        // in flight: the decay panels.  Both operand families are stored transposed, [channel d][row] (K-major A operands).
+        const uint32_t X = sb + kR3 + (I >> 1) * 16384;      // two target blocks share a panel: 32 stack rows each
         const int xc = (I & 1) * 4;
         f2 w[8], x[8];
-        get_q(w);
+        unit(w, kQt, rowv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = f2_mul(w[e], E[e]);       // q~ rows of this block
-        *reinterpret_cast<uint4*>(X + sw128_off(d, xc)) = pack_quad(w, 0);
-        *reinterpret_cast<uint4*>(X + sw128_off(d, xc + 1)) = pack_quad(w, 4);
-        get_k(x);
+        put_panel(X, xc, w);
+        unit(x, kKt, rowv + 64);
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = f2_mul(x[e], E[e]);       // k~ rows of this block
-        *reinterpret_cast<uint4*>(X + sw128_off(d, xc + 2)) = pack_quad(w, 0);
-        *reinterpret_cast<uint4*>(X + sw128_off(d, xc + 3)) = pack_quad(w, 4);
+        put_panel(X, xc + 2, w);
         // these rows as sources of their own and every later block (block I's product sums over the blocks <= I only)
         f2 ei[8];
 #pragma unroll
@@ -529,82 +604,87 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll 1
         for (int ver = I; ver < 4; ++ver) {
             if (ver > I) {
-                const f2 fb = f2_all(__expf(cref[ver * 128 + d] - cref[(ver - 1) * 128 + d]));
+                float fb[4];
+                chan4(fb, fbk + (ver - 1) * 128);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) ei[e] = f2_mul(ei[e], fb);
+                for (int e = 0; e < 8; ++e) ei[e] = f2_mul(ei[e], f2_all(fb[e >> 1]));
             }
 #pragma unroll
             for (int e = 0; e < 8; ++e) w[e] = f2_mul(x[e], ei[e]);
-            *reinterpret_cast<uint4*>(Sk + ver * 16384 + sw128_off(d, 2 * I)) = pack_quad(w, 0);
-            *reinterpret_cast<uint4*>(Sk + ver * 16384 + sw128_off(d, 2 * I + 1)) = pack_quad(w, 4);
+            put_panel(sb + kR1 + ver * 16384, 2 * I, w);
         }
     }
-    ok = ok && mbar_wait(&bar_q, 0, p.status, 42);       // the dW^T panel is free from here: it becomes the DAt tiles
-    tc_fence_after();
     {   // still in flight: the rows of dA
-        f2 t[8];
+        f2 t[4];
+        uint32_t w[4];
         // row j of dA = tril(dO Z^T), 16 source columns per warp group.  The diagonal of dA adds q k dA to dG through the
         // row part and takes the same amount away through the column part; left inside two bf16 products those O(1) terms
         // cancel only to bf16 accuracy, which swamps dg when the decay is strong.  It goes to dq and dk directly instead
         // (decay factor 1, no dG term).
-        tmem_ld_pairs(tmem + lane_base + cA + 16 * I, t);
-        const int nd = row - 16 * I;                     // columns before the diagonal, relative to this group's first
+        tmem_ld_16x16(tmem + lane_base + cA + 16 * I, t);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
+        for (int e = 0; e < 4; ++e) {
+            const int row = row0 + 8 * (e >> 1), nd = row - (tb + 8 * (e & 1));     // columns before the diagonal, from this pair on
             const float2 a = f2_get(t[e]);
-            if (rowown && 2 * e == nd) dA_diag[row] = a.x;
-            if (rowown && 2 * e + 1 == nd) dA_diag[row] = a.y;
-            t[e] = f2_make(2 * e < nd ? a.x : 0.f, 2 * e + 1 < nd ? a.y : 0.f);
+            if (nd == 0) dA_diag[row] = a.x;
+            if (nd == 1) dA_diag[row] = a.y;
+            w[e] = f2_to_bf16(f2_make(nd > 0 ? a.x : 0.f, nd > 1 ? a.y : 0.f));
         }
-        if (rowown) {
-            *reinterpret_cast<uint4*>(DAt + jb * 4096 + sw128_off(jr, 2 * I)) = pack_quad(t, 0);
-            *reinterpret_cast<uint4*>(DAt + jb * 4096 + sw128_off(jr, 2 * I + 1)) = pack_quad(t, 4);
-        }
+        stsm_x4(sb + da_off, w);
     }
     ok = ok && mbar_wait(&bar_m, 0, p.status, 44);
     tc_fence_after();
     {
         // row j of dM = -stril(Y T^T); dbeta gets sum_l dM[j][l] M~[j][l]
-        const int nd = row - 16 * I;
-        f2 t[8], acc = f2_all(0.f);
-        tmem_ld_pairs(tmem + lane_base + cM + 16 * I, t);
-        const uint4 m0 = *reinterpret_cast<const uint4*>(Mts + sw128_off(row, 2 * I));
-        const uint4 m1 = *reinterpret_cast<const uint4*>(Mts + sw128_off(row, 2 * I + 1));
-        const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-        const f2 bj = f2_all(rowv[128 + row]);
+        f2 t[4];
+        uint32_t mw[4], w[4];
+        tmem_ld_16x16(tmem + lane_base + cM + 16 * I, t);
+        ldsm_x4(sb + kRM + row_off, mw);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const float2 a = f2_get(t[e]);
-            const f2 dm = f2_make(2 * e < nd ? -a.x : 0.f, 2 * e + 1 < nd ? -a.y : 0.f);
-            acc = f2_fma(dm, f2_from_bf16(mw[e]), acc);
-            t[e] = f2_mul(bj, dm);
+        for (int hf = 0; hf < 2; ++hf) {
+            const int row = row0 + 8 * hf;
+            const f2 bj = f2_all(rowv[128 + row]);
+            f2 acc = f2_all(0.f);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int nd = row - (tb + 8 * n);
+                const float2 a = f2_get(t[2 * hf + n]);
+                const f2 dm = f2_make(nd > 0 ? -a.x : 0.f, nd > 1 ? -a.y : 0.f);
+                acc = f2_fma(dm, f2_from_bf16(mw[2 * hf + n]), acc);
+                w[2 * hf + n] = f2_to_bf16(f2_mul(bj, dm));
+            }
+            const float2 a = f2_get(acc);
+            dbeta_acc[hf] += a.x + a.y;
         }
-        const float2 a = f2_get(acc);
-        dbeta_acc += a.x + a.y;
-        if (rowown) {
-            *reinterpret_cast<uint4*>(DAt + jb * 4096 + sw128_off(16 + jr, 2 * I)) = pack_quad(t, 0);
-            *reinterpret_cast<uint4*>(DAt + jb * 4096 + sw128_off(16 + jr, 2 * I + 1)) = pack_quad(t, 4);
-            dbp[I * 64 + row] = dbeta_acc;
+        stsm_x4(sb + da_off + 2048, w);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            float x = dbeta_acc[hf];
+            x += __shfl_xor_sync(0xffffffffu, x, 1);
+            x += __shfl_xor_sync(0xffffffffu, x, 2);
+            if (c4 == 0) dbp[I * 64 + row0 + 8 * hf] = x;
         }
     }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    // accumulator columns of the pull-back: RP_I (32 columns each) and CP_I (64 columns each)
-    constexpr uint32_t cRP = 0, cCP = 128;
-    if (ok && warp < 4 && lane == 0) {     // warp = target block
+    // accumulator columns of the pull-back: RP_I (32 columns each) and CP_I (16 columns for each source block up to I), beside
+    // those of dR, dE and dQ
+    constexpr uint32_t cRP = 64;
+    auto cCP = [](int b) { return 192u + 8u * (uint32_t)(b * (b + 1)); };
+    if (ok && warp >= 12 && lane == 0) {     // wq = target block; the warps with the least work of their own
         tc_fence_after();
         const uint32_t id_rp = umma_idesc_bf16(128, 32, kMajorK, kMajorK);
-        const uint32_t id_cp = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
-        const uint32_t aS = smem_u32(Sk + warp * 16384), aX = smem_u32(Xk + (warp >> 1) * 16384) + (warp & 1) * 64;
-        const uint32_t bD = smem_u32(DAt + warp * 4096);
+        const uint32_t id_cp = umma_idesc_bf16(128, 16, kMajorK, kMajorMN) + ((uint32_t)(2 * wq) << 17);      // N = 16 (wq + 1)
+        const uint32_t aS = smem_u32(Sk + wq * 16384), aX = smem_u32(Xk + (wq >> 1) * 16384) + (wq & 1) * 64;
+        const uint32_t bD = smem_u32(DAt + wq * 4096);
 #pragma unroll 1
-        for (int k16 = 0; k16 <= warp; ++k16)     // RP_I^T[d][n] = sum_{s in blocks <= I} k~_I[s][d] * rows_I[n][s]
-            umma_bf16_ss(tmem + cRP + 32 * warp, umma_smem_desc_sw128(aS + k16 * 32, 16, 1024),
+        for (int k16 = 0; k16 <= wq; ++k16)     // RP_I^T[d][n] = sum_{s in blocks <= I} k~_I[s][d] * rows_I[n][s]
+            umma_bf16_ss(tmem + cRP + 32 * wq, umma_smem_desc_sw128(aS + k16 * 32, 16, 1024),
                          umma_smem_desc_sw128(bD + k16 * 32, 16, 1024), id_rp, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 2; ++k16)     // CP_I^T[d][s] = sum_{n<32} stack_I[n][d] * rows_I[n][s]
-            umma_bf16_ss(tmem + cCP + 64 * warp, umma_smem_desc_sw128(aX + k16 * 32, 16, 1024),
+            umma_bf16_ss(tmem + cCP(wq), umma_smem_desc_sw128(aX + k16 * 32, 16, 1024),
                          umma_smem_desc_sw128(bD + k16 * 2048, 4096, 1024), id_cp, k16 > 0);
         umma_commit(&bar_pb);
     }
@@ -613,7 +693,7 @@ __global__ void __launch_bounds__(512, 1)
         const int i = tid - 128;
         st_io(p.dbeta, (size_t)(tok0 + i) * H + h, GB, dbp[i] + dbp[64 + i] + dbp[128 + i] + dbp[192 + i]);
     }
-    if (warp == 15) {
+    if (warp == 11) {
         // the inputs of the block that starts when this one ends, 148 further on, into L2
         const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + 148u;
         if (nxt < gridDim.x * gridDim.y) {
@@ -627,48 +707,68 @@ __global__ void __launch_bounds__(512, 1)
                     tma_prefetch_2d(&mq, nh * 128 + lane * 64, nt0);
                     tma_prefetch_2d(&mk, nh * 128 + lane * 64, nt0);
                     tma_prefetch_2d(&mv, nh * 128 + lane * 64, nt0);
+                    if (GB) tma_prefetch_2d(&mg, nh * 128 + lane * 64, nt0);
                 } else if (lane == 2) {
                     tma_prefetch_2d(&mZT, 0, nch * 128);
                     tma_prefetch_2d(&mdZT, 0, nch * 128);
                     tma_prefetch_2d(&mT, 0, nch * 64);
                     tma_prefetch_2d(&mMt, 0, nch * 64);
                 }
-                for (int i = lane; i < nlen; i += 32) {
-                    const char* gp = static_cast<const char*>(p.g) + (((size_t)(nt0 + i) * H + nh) * 128) * (GB ? 2 : 4);
+                if (!GB) {
+                    for (int i = lane; i < nlen; i += 32) {
+                        const char* gp = static_cast<const char*>(p.g) + (((size_t)(nt0 + i) * H + nh) * 128) * 4;
 #pragma unroll
-                    for (int b = 0; b < (GB ? 256 : 512); b += 128) prefetch_l2(gp + b);
+                        for (int b = 0; b < 512; b += 128) prefetch_l2(gp + b);
+                    }
                 }
             }
         }
         __syncwarp();
     }
-    // in flight: the dE and dQ parts of dk, the diagonal of dA
-    f2 dkn[8], kn[8];
-    f2 ge2 = f2_all(0.f);
-    get_k(kn);
+    // in flight: the dR part of dq, the dE and dQ parts of dk, the diagonal of dA
+    f2 dqn[8], dkn[8], kn[8], dG[8];
+    float ge4[4];      // sum of dE * E over this lane's tokens, per channel
     {
         f2 t[8];
-        tmem_ld_pairs(tmem + lane_base + cE + 16 * I, t);
+        float x4[4];
+        tmem_ld_32x16(tmem + lane_base + cR + 16 * I, t);
+        chan4(x4, eC + I * 128);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dqn[e] = f2_mul(t[e], f2_mul(E[e], f2_all(x4[e >> 1])));
+        unit(t, kQt, rowv);
+        const f2 dd[2] = {ld_2(dA_diag + tb), ld_2(dA_diag + tb + 8)};
+        unit(kn, kKt, rowv + 64);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            dkn[e] = f2_mul(t[e], f2_mul(rcp_2(E[e]), f2_all(eEndI)));
-            const f2 eE = f2_mul(dkn[e], kn[e]);    // dE * E
-            dG[e] = f2_add(dG[e], neg_2(eE));
-            ge2 = f2_add(ge2, eE);
+            dG[e] = f2_mul(dqn[e], t[e]);
+            dqn[e] = f2_fma(dd[e & 1], kn[e], dqn[e]);
+            dkn[e] = f2_mul(dd[e & 1], t[e]);
         }
-        tmem_ld_pairs(tmem + lane_base + cQ + 16 * I, t);
+        tmem_ld_32x16(tmem + lane_base + cE + 16 * I, t);
+        chan4(x4, eEnd + I * 128);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            f2 s;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int e = 2 * c + n;
+                const f2 dE = f2_mul(t[e], f2_mul(rcp_2(E[e]), f2_all(x4[c])));
+                const f2 eE = f2_mul(dE, kn[e]);        // dE * E
+                dkn[e] = f2_add(dkn[e], dE);
+                dG[e] = f2_fma(eE, f2_all(-1.f), dG[e]);
+                s = n == 0 ? eE : f2_add(s, eE);
+            }
+            const float2 s2 = f2_get(s);
+            ge4[c] = s2.x + s2.y;
+        }
+        tmem_ld_32x16(tmem + lane_base + cQ + 16 * I, t);
+        chan4(x4, eC + I * 128);
+        const f2 nb[2] = {neg_2(ld_2(rowv + 128 + tb)), neg_2(ld_2(rowv + 128 + tb + 8))};
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const f2 dQ = neg_2(f2_mul(f2_mul(t[e], ld_2(rowv + 128 + 16 * I + 2 * e)), f2_mul(E[e], eCI)));   // dQ * beta * e^G
+            const f2 dQ = f2_mul(f2_mul(t[e], nb[e & 1]), f2_mul(E[e], f2_all(x4[e >> 1])));   // dQ * beta * e^G
             dkn[e] = f2_add(dkn[e], dQ);
             dG[e] = f2_fma(dQ, kn[e], dG[e]);
-        }
-        get_q(t);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const f2 dd = ld_2(dA_diag + 16 * I + 2 * e);
-            dqn[e] = f2_fma(dd, kn[e], dqn[e]);
-            dkn[e] = f2_fma(dd, t[e], dkn[e]);
         }
     }
     ok = ok && mbar_wait(&bar_pb, 0, p.status, 45);
@@ -677,167 +777,165 @@ __global__ void __launch_bounds__(512, 1)
     // ================================================================ phase 5: assemble the gradients
     {
         f2 t[8];
-        // decay factors of this thread's rows relative to its own block reference: E = e^{G - c_own} (<= 1) for the
+        // decay factors relative to the block's own reference: E = e^{G - c_own} (<= 1) for the
         // row parts, 1 / E for the column parts (a later block I' contributes e^{c_I' - c_own} / E)
         // The decay gradient is a telescoping sum: a pair (i, s) adds its summand to dG at row i (row part) and takes the
         // same summand away at row s (column part), and only the rows in between keep it after the reverse cumulative
         // sum.  The two parts come from different UMMAs, so they cancel exactly only if both are built from the SAME
         // rounded factors: dG therefore uses the bf16 values that sit in the operand panels (target rows q~, k~ and
         // source rows k-), while dq and dk keep the float32 factors.
-        tmem_ld_pairs(tmem + lane_base + cRP + 32 * I + 16, t);     // row part through beta*dM
+        tmem_ld_32x16(tmem + lane_base + cRP + 32 * I + 16, t);     // row part through beta*dM
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             dkn[e] = f2_fma(E[e], t[e], dkn[e]);
             dG[e] = f2_fma(round_bf16_2(f2_mul(kn[e], E[e])), t[e], dG[e]);
+            kn[e] = neg_2(kn[e]);                                   // -k from here on: the column part is taken away
         }
-        tmem_ld_pairs(tmem + lane_base + cRP + 32 * I, t);          // row part through dA
+        tmem_ld_32x16(tmem + lane_base + cRP + 32 * I, t);          // row part through dA
         {
-            const uint4 a = qslot[0], b = qslot[512];
-            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            f2 q[8];
+            unit(q, kQt, rowv);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const f2 q = f2_mul(f2_from_bf16(w[e]), f2_mul(ld_2(rowv + 16 * I + 2 * e), f2_all(p.scale)));
                 dqn[e] = f2_fma(E[e], t[e], dqn[e]);
-                dG[e] = f2_fma(round_bf16_2(f2_mul(q, E[e])), t[e], dG[e]);
+                dG[e] = f2_fma(round_bf16_2(f2_mul(q[e], E[e])), t[e], dG[e]);
             }
         }
         // column part: sources of block I receive from target blocks I' >= I, each with its own decay reference; the
         // source factor is rebuilt exactly as the panel code built it
 #pragma unroll
         for (int e = 0; e < 8; ++e) E[e] = rcp_2(E[e]);
-        float cprev = cref[I * 128 + d];
 #pragma unroll 1
         for (int Ib = I; Ib < 4; ++Ib) {
-            tmem_ld_pairs(tmem + lane_base + cCP + 64 * Ib + 16 * I, t);
+            tmem_ld_32x16(tmem + lane_base + cCP(Ib) + 16 * I, t);
             if (Ib > I) {
-                const float cn = cref[Ib * 128 + d];
-                const f2 fb = f2_all(__expf(cn - cprev));
-                cprev = cn;
+                float fb[4];
+                chan4(fb, fbk + (Ib - 1) * 128);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) E[e] = f2_mul(E[e], fb);
+                for (int e = 0; e < 8; ++e) E[e] = f2_mul(E[e], f2_all(fb[e >> 1]));
             }
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 dkn[e] = f2_fma(E[e], t[e], dkn[e]);
-                dG[e] = f2_fma(neg_2(round_bf16_2(f2_mul(kn[e], E[e]))), t[e], dG[e]);
+                dG[e] = f2_fma(round_bf16_2(f2_mul(kn[e], E[e])), t[e], dG[e]);
             }
         }
     }
-    // chunk-end term and reverse cumulative sum of dG over the 64 rows of this channel
-    {
-        f2 local = dG[0];
+    // reverse cumulative sum of dG inside the block; the block's sums go to the other blocks' lanes through shared memory
 #pragma unroll
-        for (int e = 1; e < 8; ++e) local = f2_add(local, dG[e]);
-        const float2 l2 = f2_get(local), g2 = f2_get(ge2);
-        tot[I * 128 + d] = l2.x + l2.y;
-        gsum[I * 128 + d] = g2.x + g2.y;   // gsum is free again
+    for (int c = 0; c < 4; ++c) {
+        const float2 g0 = f2_get(dG[2 * c]), g1 = f2_get(dG[2 * c + 1]);
+        const float p0 = g0.x + g0.y, p1 = g1.x + g1.y;
+        const float a1 = quad_after(p1, c4);
+        const float a0 = quad_after(p0, c4) + __shfl_sync(0xffffffffu, a1 + p1, 0, 4);
+        if (c4 == 0) tot[I * 128 + cb + 8 * c] = a0 + p0;
+        dG[2 * c] = f2_make(a0 + p0, a0 + g0.y);
+        dG[2 * c + 1] = f2_make(a1 + p1, a1 + g1.y);
     }
-    // L2-normalisation VJP needs per-row dots over the channels: unit k is kn, unit q is qn / scale
-    const float inv_scale = p.scale != 0.f ? 1.0f / p.scale : 0.f;
+    {
+        // sums of dE * E over the quad by halving: lane c4 ends with channel c4's
+        const bool u2 = (c4 & 2) != 0, u1 = (c4 & 1) != 0;
+        const float a = (u2 ? ge4[2] : ge4[0]) + __shfl_xor_sync(0xffffffffu, u2 ? ge4[0] : ge4[2], 2);
+        const float b = (u2 ? ge4[3] : ge4[1]) + __shfl_xor_sync(0xffffffffu, u2 ? ge4[1] : ge4[3], 2);
+        ge[I * 128 + cb + 8 * c4] = (u1 ? b : a) + __shfl_xor_sync(0xffffffffu, u1 ? a : b, 1);
+    }
+    // L2-normalisation VJP needs per-row dots over the channels: unit k is -kn, unit q is qn / scale
     f2 qn[8];
-    get_q(qn);
+    unit(qn, kQt, rowv);
     {
-        // 32 per-row products (q and k of 16 rows) summed over the 32 channels of this warp with 31 shuffles: each
-        // step halves the values a lane carries, so lane L ends with the warp's total of value L.
-        float vals[16];
-        {
-            const bool up = (lane & 16) != 0;      // first step straight from the operands: value j pairs with value j + 16
+        // q and k of four rows, summed over this lane's four channels, then over the eight lanes with the same rows by halving
+        float v8[8];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {          // value 2 * row + {q, k}
-                const float2 qa = f2_get(f2_mul(qn[e], dqn[e])), ka = f2_get(f2_mul(kn[e], dkn[e]));
-                const float2 qb = f2_get(f2_mul(qn[4 + e], dqn[4 + e])), kb = f2_get(f2_mul(kn[4 + e], dkn[4 + e]));
-                vals[4 * e] = (up ? qb.x : qa.x) + __shfl_xor_sync(0xffffffffu, up ? qa.x : qb.x, 16);
-                vals[4 * e + 1] = (up ? kb.x : ka.x) + __shfl_xor_sync(0xffffffffu, up ? ka.x : kb.x, 16);
-                vals[4 * e + 2] = (up ? qb.y : qa.y) + __shfl_xor_sync(0xffffffffu, up ? qa.y : qb.y, 16);
-                vals[4 * e + 3] = (up ? kb.y : ka.y) + __shfl_xor_sync(0xffffffffu, up ? ka.y : kb.y, 16);
+        for (int n = 0; n < 2; ++n) {
+            f2 a = f2_mul(qn[n], dqn[n]), b = f2_mul(kn[n], dkn[n]);
+#pragma unroll
+            for (int c = 1; c < 4; ++c) {
+                a = f2_fma(qn[2 * c + n], dqn[2 * c + n], a);
+                b = f2_fma(kn[2 * c + n], dkn[2 * c + n], b);
             }
+            const float2 x = f2_get(a), y = f2_get(b);
+            v8[2 * n] = x.x;
+            v8[2 * n + 1] = x.y;
+            v8[4 + 2 * n] = y.x;
+            v8[4 + 2 * n + 1] = y.y;
         }
 #pragma unroll
-        for (int o = 8; o >= 1; o >>= 1) {
-            const bool up = (lane & o) != 0;
+        for (int o = 4; o >= 1; o >>= 1) {
+            const bool up = (r8 & o) != 0;
 #pragma unroll
             for (int j = 0; j < o; ++j) {
-                const float send = up ? vals[j] : vals[j + o];
-                const float keep = up ? vals[j + o] : vals[j];
-                vals[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                const float send = up ? v8[j] : v8[j + o], keep = up ? v8[j + o] : v8[j];
+                v8[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * o);
             }
         }
-        // lane L holds value L = (row L/2, q or k): quadrant partial
-        dots[(lane & 1) * 256 + (warp & 3) * 64 + 16 * I + (lane >> 1)] = vals[0];
+        // lane (r8, c4) holds value r8 = (q or k, n, which of the pair)
+        dots[(r8 >> 2) * 256 + wq * 64 + tb + 8 * ((r8 >> 1) & 1) + (r8 & 1)] = v8[0];
     }
     __syncthreads();
-    if (p.l2norm) {
-        if (tid < 128) {      // the four quadrants of the channels -> one number, in place
-            float* q4 = dots + (tid >> 6) * 256 + (tid & 63);
-            q4[0] = (q4[0] + q4[64]) + (q4[128] + q4[192]);
-        }
-        __syncthreads();
+    if (tid < 128) {      // the four quarters of the channels -> what a row's dot takes off its gradient, per unit of q or -k
+        const float* q4 = dots + (tid >> 6) * 256 + (tid & 63);
+        const float dot = (q4[0] + q4[64]) + (q4[128] + q4[192]);
+        const float inv_scale = p.scale != 0.f ? 1.0f / p.scale : 0.f;
+        const float f = tid < 64 ? -inv_scale * inv_scale : -1.f;
+        rowb[tid] = p.l2norm ? f * dot * rowv[tid] : 0.f;
     }
     {
-        float run = gsum[d] + gsum[128 + d] + gsum[256 + d] + gsum[384 + d];
-        {
-            float dD = 0.f;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) dD += part[r * 128 + d];
-            run += egend * dD;
-        }
+        // what the rows of (I, channel) get from the later blocks and from the chunk's end
+        const int dd = tid & 127;
+        float run = (ge[dd] + ge[128 + dd]) + (ge[256 + dd] + ge[384 + dd]);
+        run = fmaf(egend[dd], (part[dd] + part[128 + dd]) + (part[256 + dd] + part[384 + dd]), run);
 #pragma unroll
         for (int Ib = 3; Ib > 0; --Ib)
-            if (Ib > I) run += tot[Ib * 128 + d];
-        // The gradients of this thread's 16 rows go through shared memory (the source-panel region is free now), so
-        // that they leave as 16-byte row segments instead of one 2-byte store per row, tensor and thread.
-        __nv_bfloat16* tq = reinterpret_cast<__nv_bfloat16*>(sm + kR1) + 16 * I * 128 + d;      // [64][128] dq
-        __nv_bfloat16* tk = tq + 64 * 128;                                                       // [64][128] dk
-        __nv_bfloat16* tgb = tk + 64 * 128;                                                      // [64][128] dg when the gate dtype is bf16
-        float* tgf = reinterpret_cast<float*>(sm + kR1 + 32768) + 16 * I * 128 + d;              // [64][128] dg when it is float32
+            if (Ib > I) run += tot[Ib * 128 + dd];
+        eC[tid] = run;
+    }
+    __syncthreads();
+    {
+        // The gradients go through shared memory (the source-panel region is free now), so that they leave as 16-byte row
+        // segments.
+        const f2 qa[2] = {ld_2(rowv + tb), ld_2(rowv + tb + 8)}, qb[2] = {ld_2(rowb + tb), ld_2(rowb + tb + 8)};
 #pragma unroll
-        for (int e = 7; e >= 0; --e) {
-            const int i = 16 * I + 2 * e;
-            f2 dqv = f2_mul(dqn[e], f2_all(p.scale)), dkv = dkn[e];
-            if (p.l2norm) {
-                const f2 pq = ld_2(dots + i), pk = ld_2(dots + 256 + i);
-                dqv = f2_mul(ld_2(rowv + i), f2_fma(f2_mul(qn[e], f2_all(-inv_scale)), pq, dqv));
-                dkv = f2_mul(ld_2(rowv + 64 + i), f2_fma(neg_2(kn[e]), pk, dkv));
-            }
-            const uint32_t uq = f2_to_bf16(dqv), uk = f2_to_bf16(dkv);
-            const __nv_bfloat162 bq = *reinterpret_cast<const __nv_bfloat162*>(&uq), bk = *reinterpret_cast<const __nv_bfloat162*>(&uk);
-            tq[2 * e * 128] = bq.x;
-            tq[(2 * e + 1) * 128] = bq.y;
-            tk[2 * e * 128] = bk.x;
-            tk[(2 * e + 1) * 128] = bk.y;
-            const float2 g2 = f2_get(dG[e]);
-            const float r1 = run + g2.y, r0 = r1 + g2.x;
-            run = r0;
-            if (GB) {
-                tgb[2 * e * 128] = __float2bfloat16(r0);
-                tgb[(2 * e + 1) * 128] = __float2bfloat16(r1);
-            } else {
-                tgf[2 * e * 128] = r0;
-                tgf[(2 * e + 1) * 128] = r1;
+        for (int e = 0; e < 8; ++e) dqn[e] = f2_fma(qn[e], qb[e & 1], f2_mul(dqn[e], qa[e & 1]));
+        put_tile(sb + kR1, dqn);
+        const f2 ka[2] = {ld_2(rowv + 64 + tb), ld_2(rowv + 64 + tb + 8)}, kb[2] = {ld_2(rowb + 64 + tb), ld_2(rowb + 64 + tb + 8)};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dkn[e] = f2_fma(kn[e], kb[e & 1], f2_mul(dkn[e], ka[e & 1]));
+        put_tile(sb + kR1 + 16384, dkn);
+        float run[4];
+        chan4(run, eC + I * 128);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dG[e] = f2_add(dG[e], f2_all(run[e >> 1]));
+        if (GB) {
+            put_tile(sb + kR1 + 32768, dG);
+        } else {
+            float* tg = reinterpret_cast<float*>(sm + kR1 + 32768);      // [64][128], 16-byte columns turned by the row pair
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float2 x = f2_get(dG[e]);
+                const int i = tb + 8 * (e & 1), d = cb + 8 * (e >> 1), sw = (d & 3) + ((((d >> 2) ^ (i >> 1)) & 31) << 2);
+                tg[i * 128 + sw] = x.x;
+                tg[(i + 1) * 128 + sw] = x.y;
             }
         }
     }
     __syncthreads();
     if (ok) {
-        const __nv_bfloat16* tq = reinterpret_cast<const __nv_bfloat16*>(sm + kR1);
-        const __nv_bfloat16* tk = tq + 64 * 128;
-        const __nv_bfloat16* tgb = tk + 64 * 128;
-        const float* tgf = reinterpret_cast<const float*>(sm + kR1 + 32768);
         const int c = tid & 15;
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
             const int i = pass * 32 + (tid >> 4);
             if (i < len) {
                 const size_t o = ((size_t)(tok0 + i) * H + h) * 128;
-                *reinterpret_cast<uint4*>(p.dq + o + 8 * c) = *reinterpret_cast<const uint4*>(tq + i * 128 + 8 * c);
-                *reinterpret_cast<uint4*>(p.dk + o + 8 * c) = *reinterpret_cast<const uint4*>(tk + i * 128 + 8 * c);
+                const uint8_t* src = sm + kR1 + (c >> 3) * 8192 + sw128_off(i, c & 7);
+                *reinterpret_cast<uint4*>(p.dq + o + 8 * c) = *reinterpret_cast<const uint4*>(src);
+                *reinterpret_cast<uint4*>(p.dk + o + 8 * c) = *reinterpret_cast<const uint4*>(src + 16384);
                 if (GB) {
-                    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dg) + o + 8 * c) =
-                        *reinterpret_cast<const uint4*>(tgb + i * 128 + 8 * c);
+                    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dg) + o + 8 * c) = *reinterpret_cast<const uint4*>(src + 32768);
                 } else {
+                    const float* tg = reinterpret_cast<const float*>(sm + kR1 + 32768) + i * 128;
                     float* dgp = reinterpret_cast<float*>(p.dg) + o;
-                    *reinterpret_cast<uint4*>(dgp + 4 * c) = *reinterpret_cast<const uint4*>(tgf + i * 128 + 4 * c);
-                    *reinterpret_cast<uint4*>(dgp + 64 + 4 * c) = *reinterpret_cast<const uint4*>(tgf + i * 128 + 64 + 4 * c);
+                    *reinterpret_cast<uint4*>(dgp + 4 * c) = *reinterpret_cast<const uint4*>(tg + ((c ^ (i >> 1)) & 31) * 4);
+                    *reinterpret_cast<uint4*>(dgp + 64 + 4 * c) = *reinterpret_cast<const uint4*>(tg + (((16 + c) ^ (i >> 1)) & 31) * 4);
                 }
             }
         }
@@ -855,7 +953,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     using namespace tc;
     const uint64_t nch = (uint64_t)w.nslots * w.H;
     const uint64_t cols = (uint64_t)w.H * 128;
-    CUtensorMap mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt;
+    CUtensorMap mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg;
     int rc = 0;
     rc |= make_map_bf16(&mq, q, (uint64_t)tokens, cols, 64, 64);
     rc |= make_map_bf16(&mk, k, (uint64_t)tokens, cols, 64, 64);
@@ -867,6 +965,8 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     rc |= make_map_bf16(&mZT, t.ZT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mdZT, t.dZT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mMt, t.Mt, nch * 64, 64, 64, 64);
+    if (gbf16) rc |= make_map_bf16(&mg, g, (uint64_t)tokens, cols, 64, 64);
+    else mg = mq;      // float32 gates are read by the threads
     if (rc) return KDA_ERR_CUDA;
     IntraBwdArgs a;
     a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len;
@@ -878,7 +978,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     auto kern = gbf16 ? tc_intra_bwd_kernel<true> : tc_intra_bwd_kernel<false>;
     if (set_smem_limit(kern, kIntraBwdSmem)) return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_intra_bwd_kernel", st,
-               kern<<<dim3(w.nslots, w.H), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, a));
+               kern<<<dim3(w.nslots, w.H), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg, a));
     return launch_status();
 }
 
