@@ -17,8 +17,8 @@
 // 113 KB and <= 128 registers let two CTAs share an SM and fill each other's waits: the kernel is a chain of short phases
 // between barriers.  Every panel leaves by TMA from the tile the products read, and nothing comes back: R^T stored from
 // registers in 8-byte pieces (32 sectors a warp store), E and A^T fetched again for the transition, with a fence in front,
-// and R^T read row by row had taken a fifth of a block's cycles.  16,384 chunk-heads: 1,157 -> 960 us, 384: 46 -> 41 us,
-// 2,048 forward-only: 148 -> 130 us.
+// and R^T read row by row had taken a fifth of a block's cycles.  16,384 chunk-heads: 1,157 -> 916 us, 384: 46 -> 39 us,
+// 2,048 forward-only: 148 -> 126 us.
 // Restates reference chunk_wy_forward.cu:125-405 and 761-858.
 
 #include <cstdio>
@@ -317,13 +317,13 @@ __global__ void __launch_bounds__(kNT, 2)
     const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
     if (len == 0) return;
     const size_t ch = blockIdx.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int cg = lane & 15;                      // channels 8*cg .. 8*cg+7
     const int rq = 2 * warp + (lane >> 4);         // rows 4*rq .. 4*rq+3
     const int J = warp >> 1;                       // 16-row block of this thread's rows
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         mbar_init(&bar_in, 1);
         mbar_init(&bar_am, 2);
         mbar_init(&bar_uw, 1);
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kNT, 2)
     fence_async_smem();
     tc_fence_before();
     __syncthreads();                                   // (3) operands complete
-    if (warp < 2 && lane == 0) {
+    if (warp < 2 && elect_one()) {
         // warp 0: targets 3, 2, 0 against the full stack.  warp 1: target 1; its stack has 32 rows, the product's other 96
         // read the bytes behind them and are never looked at.
         tc_fence_after();
@@ -542,13 +542,13 @@ __global__ void __launch_bounds__(kNT, 2)
         const uint32_t akb = warp == 0 ? 16384u : 4096u, bkb = warp == 0 ? 12288u : 4096u;
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)
-            umma_bf16_ss(tmem + warp * 96, umma_smem_desc_sw128(a0 + (k16 >> 2) * akb + (k16 & 3) * 32, 16, 1024),
-                         umma_smem_desc_sw128(b0 + (k16 >> 2) * bkb + (k16 & 3) * 32, 16, 1024), idesc, k16 > 0);
+            umma_bf16_ss(tmem + warp * 96, umma_smem_desc_sw128(a0, 16, 1024) + ((k16 >> 2) * akb + (k16 & 3) * 32),
+                         umma_smem_desc_sw128(b0, 16, 1024) + ((k16 >> 2) * bkb + (k16 & 3) * 32), idesc, k16 > 0);
         umma_commit(&bar_am);
     }
     __syncwarp();
     // in flight: the E panel leaves, v's convolution, the next block's inputs
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mE, sm + kFE + nb * 8192, nb * 64, (int)(ch * 64));
         tma_store_commit();
     }
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kNT, 2)
                 const int i = 4 * rq + j;
                 *reinterpret_cast<uint4*>(vs + piece_off(i, cg, 8192)) = i < len ? vr[j] : make_uint4(0, 0, 0, 0);
             }
-        } else if (tid == 0) {
+        } else if (warp == 0 && elect_one()) {
             mbar_expect_tx(&bar_in, 16384);
             for (int kb = 0; kb < 2; ++kb) tma_load_2d(vs + kb * 8192, &mv, &bar_in, h * 128 + kb * 64, tok0);
         }
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(kNT, 2)
         }
         fence_async_smem();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tma_store_2d(&mAT, sm + kFAT, 0, (int)(ch * 64));
             for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mR, sm + kFR + nb * 8192, nb * 64, (int)(ch * 64));
             if (!p.t.fwd_only) tma_store_2d(&mMt, sm + kFMt, 0, (int)(ch * 64));
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kNT, 2)
                 for (int c = 0; c < 8; ++c) x[c] *= b8[c];
                 ub[hh] = pack8(x);
             }
-            if (tid == 0) tma_store_wait_read();       // the M~ panel has left: the identity takes its place
+            if (warp == 0 && elect_one()) tma_store_wait_read();       // the M~ panel has left: the identity takes its place
             __syncthreads();                           // everyone has its piece of T: the operands take its place
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(kNT, 2)
         fence_async_smem();
         tc_fence_before();
         ok = __syncthreads_and(ok);
-        if (tid == 0 && ok) {
+        if (warp == 0 && elect_one() && ok) {
             if (!p.t.fwd_only) {                   // kept for the backward only
                 tma_store_2d(&mTp, sm + kFTb, 0, (int)(ch * 64));
                 tma_store_commit();
@@ -706,12 +706,12 @@ __global__ void __launch_bounds__(kNT, 2)
             const uint32_t b0 = smem_u32(sm + kFTb), b1 = smem_u32(sm + kFTbb);
 #pragma unroll
             for (int k16 = 0; k16 < 4; ++k16)     // U^T = v^T (T diag(beta))^T
-                umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(smem_u32(vs) + k16 * 2048, 8192, 1024),
-                             umma_smem_desc_sw128(b1 + k16 * 32, 16, 1024), idesc, k16 > 0);
+                umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(smem_u32(vs), 8192, 1024) + (k16 * 2048),
+                             umma_smem_desc_sw128(b1, 16, 1024) + (k16 * 32), idesc, k16 > 0);
 #pragma unroll
             for (int k16 = 0; k16 < 4; ++k16)     // W^T = Q^T T^T
-                umma_bf16_ss(tmem + 192, umma_smem_desc_sw128(smem_u32(Qs) + k16 * 2048, 8192, 1024),
-                             umma_smem_desc_sw128(b0 + k16 * 32, 16, 1024), idesc, k16 > 0);
+                umma_bf16_ss(tmem + 192, umma_smem_desc_sw128(smem_u32(Qs), 8192, 1024) + (k16 * 2048),
+                             umma_smem_desc_sw128(b0, 16, 1024) + (k16 * 32), idesc, k16 > 0);
             umma_commit(&bar_uw);
         }
         if (ok) ok = mbar_wait(&bar_uw, 0, p.t.status, 32);
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kNT, 2)
         fence_async_smem();
         tc_fence_before();
         ok = __syncthreads_and(ok);
-        if (tid == 0 && ok) {
+        if (warp == 0 && elect_one() && ok) {
             tma_store_2d(&mUT, vs, 0, (int)(ch * 128));
             tma_store_2d(&mWT, Qs, 0, (int)(ch * 128));
             tma_store_commit();
@@ -752,19 +752,19 @@ __global__ void __launch_bounds__(kNT, 2)
             const uint32_t id128 = umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
 #pragma unroll
             for (int k16 = 0; k16 < 4; ++k16)     // Pn = W^T E
-                umma_bf16_ss(tmem, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
-                             umma_smem_desc_sw128(bE + k16 * 2048, 8192, 1024), id128, k16 > 0);
+                umma_bf16_ss(tmem, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
+                             umma_smem_desc_sw128(bE, 8192, 1024) + (k16 * 2048), id128, k16 > 0);
             if (!p.t.fwd_only) {
                 const uint32_t idn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN, 1), idr = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
                 const uint32_t aR = smem_u32(sm + kFR), bA = smem_u32(sm + kFAT), bI = smem_u32(sm + kFMt);
 #pragma unroll
                 for (int k16 = 0; k16 < 4; ++k16)     // -(A W)^T = -W^T A^T
-                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
-                                 umma_smem_desc_sw128(bA + k16 * 2048, 8192, 1024), idn, k16 > 0);
+                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
+                                 umma_smem_desc_sw128(bA, 8192, 1024) + (k16 * 2048), idn, k16 > 0);
 #pragma unroll
                 for (int k16 = 0; k16 < 4; ++k16)     // + R^T I
-                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(aR + k16 * 2048, 8192, 1024),
-                                 umma_smem_desc_sw128(bI + k16 * 32, 16, 1024), idr, 1);
+                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(aR, 8192, 1024) + (k16 * 2048),
+                                 umma_smem_desc_sw128(bI, 16, 1024) + (k16 * 32), idr, 1);
             }
             // the staging below overwrites E, R and T: their stores must have been read, all but the newest group's
             tma_store_wait_read_but1();
@@ -804,12 +804,12 @@ __global__ void __launch_bounds__(kNT, 2)
         }
         fence_async_smem();
         ok = __syncthreads_and(ok);
-        if (tid == 0 && ok) {
+        if (warp == 0 && elect_one() && ok) {
             for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mP, sm + (nb ? kFE : kFTb), nb * 64, (int)(ch * 128));
             if (!p.t.fwd_only) tma_store_2d(&mRm, sm + kFR, 0, (int)(ch * 128));
             tma_store_commit();
         }
-        if (tid == 0) tma_store_wait_read();           // shared memory must outlive the reads of the bulk stores
+        if (warp == 0 && elect_one()) tma_store_wait_read();           // shared memory must outlive the reads of the bulk stores
     }
     tc_fence_before();
     __syncthreads();

@@ -141,7 +141,8 @@ constexpr int kIntraBwdSmem = kSmall + (24 * 128 + 128 + 512 + 3 * 64 + 2 * 64) 
 // elements lie in 8 x 8 pieces, so that tiles are read and written by ldmatrix / stmatrix, four pieces an instruction, a row
 // scalar serves eight of its elements and a row dot takes 7 shuffles: with a channel and 16 tokens a lane, its 2-byte accesses, row
 // scalars and 31 shuffles had been a quarter of a block's cycles.
-// 16,384 chunk-heads: 1,725 -> 1,490 us, 384: 65 -> 56 us (2,262 and 81 before (1) to (4)).
+// 16,384 chunk-heads: 1,725 -> 1,380 us, 384: 65 -> 52 us (2,262 and 81 before (1) to (4)); the last 110 us of it are cheaper
+// issue of the products (elect_one).
 template <bool GB>
 __global__ void __launch_bounds__(512, 1)
     tc_intra_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(512, 1)
     const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
     if (len == 0) return;
     const int ch = slot * H + h;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int I = warp >> 2, wq = warp & 3;       // row block and channel quarter of this warp
     const int c4 = lane & 3, r8 = lane >> 2;      // token pair and channel inside an 8 x 8 piece
     const int mi = lane >> 3, mr = lane & 7;      // the piece and row whose address this lane gives to ldmatrix / stmatrix
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(512, 1)
     __syncthreads();
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
 
-    if (warp >= 1 && warp <= 4 && lane == 0) {
+    if (warp >= 1 && warp <= 4 && elect_one()) {
         if (warp == 1) {
             for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_in[0], mb * 64, ch * 128);
             tma_load_2d(dZTs, &mdZT, &bar_in[0], 0, ch * 128);
@@ -361,19 +362,19 @@ __global__ void __launch_bounds__(512, 1)
     // X -> Y -> dM waits for, go first; the five others (~300 cycles each of operand reads) go where the chain's next product
     // is still being prepared.  Issued all at once from four warps they held those warps, and with them the block, back.
     ok = ok && mbar_wait(&bar_in[0], 0, p.status, 40);
-    if (ok && tid == 384) {
+    if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
         const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
         const uint32_t aH = smem_u32(Hs), bdZ = smem_u32(dZTs), aV = smem_u32(vs);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dW^T = H dZ^T
-            umma_bf16_ss(tmem + cW, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
-                         umma_smem_desc_sw128(bdZ + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
+            umma_bf16_ss(tmem + cW, umma_smem_desc_sw128(aH, 16384, 1024) + (k16 * 2048),
+                         umma_smem_desc_sw128(bdZ, 8192, 1024) + (k16 * 2048), id_mn_mn, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // Xraw^T = v dZ^T  (first half)    (M = 64)
-            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aV + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
-                         umma_smem_desc_sw128(bdZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aV, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32),
+                         umma_smem_desc_sw128(bdZ, 8192, 1024) + (k16 * 2048), id64_k_mn, k16 > 0);
         umma_commit(&bar_w);
     }
     __syncwarp();
@@ -433,19 +434,19 @@ __global__ void __launch_bounds__(512, 1)
         }
         part[I * 128 + 8 * cg + mr] = v8[0];
     }
-    if (ok && tid == 384) {
+    if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t aH = smem_u32(Hs), bdO = smem_u32(dOs), bZ = smem_u32(ZTs);
         const uint32_t id_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
         const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dR^T = H dO^T
-            umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH + k16 * 2048, 16384, 1024),
-                         umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), id_mn_k, k16 > 0);
+            umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH, 16384, 1024) + (k16 * 2048),
+                         umma_smem_desc_sw128(bdO, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), id_mn_k, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dA = dO Z^T                      (M = 64)
-            umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024),
-                         umma_smem_desc_sw128(bZ + k16 * 2048, 8192, 1024), id64_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32),
+                         umma_smem_desc_sw128(bZ, 8192, 1024) + (k16 * 2048), id64_k_mn, k16 > 0);
     }
     __syncwarp();
     ok = ok && mbar_wait(&bar_w, 0, p.status, 41);
@@ -460,24 +461,24 @@ __global__ void __launch_bounds__(512, 1)
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (ok && tid == 384) {
+    if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t id64_neg = umma_idesc_bf16(64, 64, kMajorMN, kMajorMN, 1);
         const uint32_t id_k_mn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
         const uint32_t aQ = smem_u32(Qp), aW = smem_u32(dWs), bT = smem_u32(Ts);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // Xraw^T -= Q' dW^T   (dW^T panel read as MN-major B: [key][token])
-            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aQ + k16 * 2048, 8192, 1024),
-                         umma_smem_desc_sw128(aW + k16 * 2048, 8192, 1024), id64_neg, 1);
+            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aQ, 8192, 1024) + (k16 * 2048),
+                         umma_smem_desc_sw128(aW, 8192, 1024) + (k16 * 2048), id64_neg, 1);
         umma_commit(&bar_x);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)     // (T^T dW)^T = dW^T T ;  dQ = -that
-            umma_bf16_ss(tmem + cQ, umma_smem_desc_sw128(aW + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cQ, umma_smem_desc_sw128(aW, 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(bT, 8192, 1024) + (k16 * 2048), id_k_mn, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)     // dP^T = dZ^T T
-            umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(smem_u32(dZTs) + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(bT + k16 * 2048, 8192, 1024), id_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(smem_u32(dZTs), 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(bT, 8192, 1024) + (k16 * 2048), id_k_mn, k16 > 0);
         umma_commit(&bar_q);
     }
     __syncwarp();
@@ -516,19 +517,19 @@ __global__ void __launch_bounds__(512, 1)
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (ok && tid == 384) {
+    if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t id = umma_idesc_bf16(64, 64, kMajorMN, kMajorK);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)     // Y = T^T X : A[m=j][k=i] = T[i][j] (MN-major), B[n=s][k=i] = X^T rows
-            umma_bf16_ss(tmem + cY, umma_smem_desc_sw128(smem_u32(Ts) + k16 * 2048, 8192, 1024),
-                         umma_smem_desc_sw128(sb + kXT + k16 * 32, 16, 1024), id, k16 > 0);
+            umma_bf16_ss(tmem + cY, umma_smem_desc_sw128(smem_u32(Ts), 8192, 1024) + (k16 * 2048),
+                         umma_smem_desc_sw128(sb + kXT, 16, 1024) + (k16 * 32), id, k16 > 0);
         umma_commit(&bar_y);
         const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dE^T = dH' Z^T
-            umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(smem_u32(dHs) + k16 * 2048, 16384, 1024),
-                         umma_smem_desc_sw128(smem_u32(ZTs) + k16 * 2048, 8192, 1024), id_mn_mn, k16 > 0);
+            umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(smem_u32(dHs), 16384, 1024) + (k16 * 2048),
+                         umma_smem_desc_sw128(smem_u32(ZTs), 8192, 1024) + (k16 * 2048), id_mn_mn, k16 > 0);
         umma_commit(&bar_r);
     }
     __syncwarp();
@@ -554,13 +555,13 @@ __global__ void __launch_bounds__(512, 1)
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (ok && tid == 384) {
+    if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t id = umma_idesc_bf16(64, 64, kMajorK, kMajorK);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)     // Y T^T : B[n=l][k=s] = T[l][s]
-            umma_bf16_ss(tmem + cM, umma_smem_desc_sw128(sb + kYt + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(smem_u32(Ts) + k16 * 32, 16, 1024), id, k16 > 0);
+            umma_bf16_ss(tmem + cM, umma_smem_desc_sw128(sb + kYt, 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(smem_u32(Ts), 16, 1024) + (k16 * 32), id, k16 > 0);
         umma_commit(&bar_m);
     }
     __syncwarp();
@@ -672,7 +673,7 @@ __global__ void __launch_bounds__(512, 1)
     // those of dR, dE and dQ
     constexpr uint32_t cRP = 64;
     auto cCP = [](int b) { return 192u + 8u * (uint32_t)(b * (b + 1)); };
-    if (ok && warp >= 12 && lane == 0) {     // wq = target block; the warps with the least work of their own
+    if (warp >= 12 && elect_one() && ok) {     // wq = target block; the warps with the least work of their own
         tc_fence_after();
         const uint32_t id_rp = umma_idesc_bf16(128, 32, kMajorK, kMajorK);
         const uint32_t id_cp = umma_idesc_bf16(128, 16, kMajorK, kMajorMN) + ((uint32_t)(2 * wq) << 17);      // N = 16 (wq + 1)
@@ -680,12 +681,12 @@ __global__ void __launch_bounds__(512, 1)
         const uint32_t bD = smem_u32(DAt + wq * 4096);
 #pragma unroll 1
         for (int k16 = 0; k16 <= wq; ++k16)     // RP_I^T[d][n] = sum_{s in blocks <= I} k~_I[s][d] * rows_I[n][s]
-            umma_bf16_ss(tmem + cRP + 32 * wq, umma_smem_desc_sw128(aS + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(bD + k16 * 32, 16, 1024), id_rp, k16 > 0);
+            umma_bf16_ss(tmem + cRP + 32 * wq, umma_smem_desc_sw128(aS, 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(bD, 16, 1024) + (k16 * 32), id_rp, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 2; ++k16)     // CP_I^T[d][s] = sum_{n<32} stack_I[n][d] * rows_I[n][s]
-            umma_bf16_ss(tmem + cCP(wq), umma_smem_desc_sw128(aX + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(bD + k16 * 2048, 4096, 1024), id_cp, k16 > 0);
+            umma_bf16_ss(tmem + cCP(wq), umma_smem_desc_sw128(aX, 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(bD, 4096, 1024) + (k16 * 2048), id_cp, k16 > 0);
         umma_commit(&bar_pb);
     }
     __syncwarp();

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int v = (warp & 3) * 32 + lane;          // value row = TMEM lane
     const bool split = p.nseg > 1;
     const int units = 2 * p.nseg - 1;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
     const int unit = (seq * H + h) * units + role;
     auto slot_of = [&](int c) { return kBwd ? c_end - 1 - (step0 + c) : c_begin + step0 + c; };   // chunk slot of step c
 
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         mbar_init(&bar_full[0], 1);
         mbar_init(&bar_full[1], 1);
         mbar_init(&bar_free[0], 1);
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
 
     if (warp == 4 * kScanGroups) {
         // ------------------------------------------------------------------ load warp
-        if (lane == 0) {
+        if (elect_one()) {
             auto issue_loads = [&](int c) {
                 const int st = c & 1;
                 const int slot = slot_of(c);
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                 __syncwarp();
             }
         }
-        if (lane == 0 && n == 0 && split) {
+        if (n == 0 && split && elect_one()) {
             if (mbar_wait(&bar_pan, 0, p.status, 55)) {
                 tma_store_2d(&mF, Sop, 0, unit * 128);
                 tma_store_2d(&mF, Sop + 16384, 64, unit * 128);
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
             }
             tma_store_wait_all();
         }
-        if (lane == 0 && n > 0) {
+        if (n > 0 && elect_one()) {
             // state-independent product:  forward U^T E (A K-major, B MN-major), backward dO^T Rm (A MN-major, B K-major)
             const uint32_t id_ind = kBwd ? umma_idesc_bf16(128, 128, kMajorMN, kMajorK) : umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
             // state product, negated:  forward -S Pn (B MN-major: rows of Pn are the contraction index),
@@ -190,11 +190,11 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
 #pragma unroll
                 for (int k16 = 0; k16 < 4; ++k16) {
                     if (!kBwd)
-                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 32768 + k16 * 32, 16, 1024),
-                                     umma_smem_desc_sw128(s0 + 49152 + k16 * 2048, 8192, 1024), id_ind, k16 > 0);
+                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 32768, 16, 1024) + (k16 * 32),
+                                     umma_smem_desc_sw128(s0 + 49152, 8192, 1024) + (k16 * 2048), id_ind, k16 > 0);
                     else
-                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 49152 + k16 * 2048, 8192, 1024),
-                                     umma_smem_desc_sw128(s0 + 32768 + k16 * 32, 16, 1024), id_ind, k16 > 0);
+                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 49152, 8192, 1024) + (k16 * 2048),
+                                     umma_smem_desc_sw128(s0 + 32768, 16, 1024) + (k16 * 32), id_ind, k16 > 0);
                 }
             };
             const CUtensorMap* mstore = composite ? &mS2 : &mS;      // composites go to their own panel array
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                 tc_fence_after();
 #pragma unroll
                 for (int k16 = 0; k16 < 8; ++k16) {   // A = the packed state in tensor memory, 8 columns per K = 16
-                    const uint64_t bd = kBwd ? umma_smem_desc_sw128(s0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024)
-                                             : umma_smem_desc_sw128(s0 + k16 * 2048, 16384, 1024);
+                    const UmmaDesc bd = kBwd ? umma_smem_desc_sw128(s0, 16, 1024) + ((k16 >> 2) * 16384 + (k16 & 3) * 32)
+                                             : umma_smem_desc_sw128(s0, 16384, 1024) + (k16 * 2048);
                     umma_bf16_ts(tmem + 128 * st, tmem + kScanPanelCol + 8 * k16, bd, id_st, (composite && k16 == 0) ? 0u : 1u);
                 }
                 // The store of panel c-1 has read its buffer before this commit lets the state threads write panel c+1
@@ -355,8 +355,8 @@ __device__ __forceinline__ void issue_hilo_product(uint32_t tmem, const uint8_t*
         const uint32_t a0 = smem_u32(a_hi + part * 32768);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)
-            umma_bf16_ss(tmem, umma_smem_desc_sw128(a0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                         umma_smem_desc_sw128(b0 + k16 * 2048, 16384, 1024), idesc, (part | k16) != 0);
+            umma_bf16_ss(tmem, umma_smem_desc_sw128(a0, 16, 1024) + ((k16 >> 2) * 16384 + (k16 & 3) * 32),
+                         umma_smem_desc_sw128(b0, 16384, 1024) + (k16 * 2048), idesc, (part | k16) != 0);
     }
 }
 
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256, 1)
     if (nc == 0 && !fin) return;
     // products 0 .. j0-1 walk the chain S_1 -> S_k, j0 .. j0+nc-1 are the chunks' own, the last one the final state's
     const int j0 = k - 1, np = j0 + nc + (fin ? 1 : 0);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;                        // key half handled by this warpgroup
     const int v = (warp & 3) * 32 + lane;           // value row = TMEM lane;  tid == g * 128 + v
     auto chunk_row = [&](int j) {                   // panel row of chunk product j
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(256, 1)
         mbar_expect_tx(&bar_l[j & 1], 32768);
         for (int nb = 0; nb < 2; ++nb) tma_load_2d(dst + nb * 16384, &mHp, &bar_l[j & 1], nb * 64, chunk_row(j));
     };
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bar_p[s], 1);
             mbar_init(&bar_l[s], 1);
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(256, 1)
     for (int j = 0; j < np && ok; ++j) {
         const int st = j & 1;
         const bool own = is_chunk(j);
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             // this product and, when it leaves S alone, the next: its accumulator was read out an iteration ago
             while (ok && issued < np && (issued <= j || (issued == j + 1 && j >= j0))) {
                 ok = mbar_wait(&bar_p[issued & 1], (issued >> 1) & 1, p.status, 80);
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(256, 1)
         }
         ok = mbar_wait(&bar_mma[st], (j >> 1) & 1, p.status, 81) && ok;
         tc_fence_after();
-        if (tid == 0 && ok) {
+        if (warp == 0 && elect_one() && ok) {
             load_p();                               // product j + 2 into the panel this one has read
             if (j > j0) {
                 tma_store_wait_read();              // chunk j - 1 has left its buffer: chunk j + 1 into it
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(256, 1)
         } else {
             const bool final_state = j >= j0;
             if (final_state) {                      // the rows go through the panel buffers: their stores must have read them
-                if (tid == 0) tma_store_wait_read();
+                if (warp == 0 && elect_one()) tma_store_wait_read();
                 ok = __syncthreads_and(ok);
             }
 #pragma unroll
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(256, 1)
         tc_fence_before();
         ok = __syncthreads_and(ok);                 // operands rewritten, accumulator read
         tc_fence_after();
-        if (ok && own && tid == 0) {
+        if (warp == 0 && elect_one() && ok && own) {
             for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mHp, sm + kFixL + st * 32768 + nb * 16384, nb * 64, chunk_row(j));
             tma_store_commit();
         }
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(256, 1)
             }
         }
     }
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         if (!ok) {      // unwinding: copies and products in flight must end before the block may exit
             for (int j = p_end > 2 ? p_end - 2 : 0; j < p_end; ++j) mbar_wait(&bar_p[j & 1], (j >> 1) & 1, nullptr, 0);
             for (int j = l_end > j0 + 2 ? l_end - 2 : j0; j < l_end; ++j) mbar_wait(&bar_l[j & 1], ((j - j0) >> 1) & 1, nullptr, 0);
@@ -615,10 +615,10 @@ __global__ void __launch_bounds__(256, 2)
     if (len == 0) return;
     const int tok0 = p.chunk_tok0[slot];
     const int ch = slot * H + h;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
     const int v = (warp & 3) * 32 + lane;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         mbar_init(&bar_in, 1);
         mbar_init(&bar_mma1, 1);
         mbar_init(&bar_mma2, 1);
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(256, 2)
     const uint32_t tmem = tmem_slot;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     bool ok = true;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         ok = mbar_wait(&bar_in, 0, p.status, 60);
         if (ok) {
             tc_fence_after();
@@ -647,13 +647,13 @@ __global__ void __launch_bounds__(256, 2)
             const uint32_t idw = umma_idesc_bf16(128, 64, kMajorK, kMajorMN), idr = umma_idesc_bf16(128, 64, kMajorK, kMajorK);
 #pragma unroll
             for (int k16 = 0; k16 < 8; ++k16)     // W^T lies key by key ...
-                umma_bf16_ss(tmem, umma_smem_desc_sw128(a0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(b0 + k16 * 2048, 8192, 1024), idw, k16 > 0);
+                umma_bf16_ss(tmem, umma_smem_desc_sw128(a0, 16, 1024) + ((k16 >> 2) * 16384 + (k16 & 3) * 32),
+                             umma_smem_desc_sw128(b0, 8192, 1024) + (k16 * 2048), idw, k16 > 0);
             umma_commit(&bar_mma1);
 #pragma unroll
             for (int k16 = 0; k16 < 8; ++k16)     // ... R token by token; needed with the last product only (the commit behind that covers it)
-                umma_bf16_ss(tmem + 64, umma_smem_desc_sw128(a0 + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(b0 + 16384 + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), idr, k16 > 0);
+                umma_bf16_ss(tmem + 64, umma_smem_desc_sw128(a0, 16, 1024) + ((k16 >> 2) * 16384 + (k16 & 3) * 32),
+                             umma_smem_desc_sw128(b0 + 16384, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), idr, k16 > 0);
         }
     }
     ok = mbar_wait(&bar_mma1, 0, p.status, 61) && ok;
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(256, 2)
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
         if (p.ZT != nullptr) {                      // kept for the backward only: the operand tile is the panel, as TMA lays it out
             tma_store_2d(&mZT, Zop, 0, ch * 128);
             tma_store_commit();
@@ -691,8 +691,8 @@ __global__ void __launch_bounds__(256, 2)
         const uint32_t idesc = umma_idesc_bf16(128, 64, kMajorK, kMajorMN);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)
-            umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0 + k16 * 32, 16, 1024),
-                         umma_smem_desc_sw128(b0 + k16 * 2048, 8192, 1024), idesc, k16 > 0);
+            umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(b0, 8192, 1024) + (k16 * 2048), idesc, k16 > 0);
         umma_commit(&bar_mma2);
     }
     if (ok) ok = mbar_wait(&bar_mma2, 0, p.status, 62);
@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(256, 2)
             }
         }
     }
-    if (tid == 0) tma_store_wait_read();            // the Z^T tile must outlive the reads of its bulk store
+    if (warp == 0 && elect_one()) tma_store_wait_read();            // the Z^T tile must outlive the reads of its bulk store
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 256);
@@ -785,10 +785,10 @@ __global__ void __launch_bounds__(256, 3)
     if (len == 0) return;
     const int tok0 = p.chunk_tok0[slot];
     const int ch = slot * H + h;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
     const int v = (warp & 3) * 32 + lane;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         mbar_init(&bar_in, 1);
         mbar_init(&bar_mma, 1);
         mbar_fence_init();
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(256, 3)
         }
         ok = __syncthreads_and(ok);
     }
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
         ok = mbar_wait(&bar_in, 0, p.status, 70);
         if (ok) {
             tc_fence_after();
@@ -828,12 +828,12 @@ __global__ void __launch_bounds__(256, 3)
             const uint32_t idb = umma_idesc_bf16(128, 64, kMajorK, kMajorK);
 #pragma unroll
             for (int k16 = 0; k16 < 4; ++k16)     // dO^T A
-                umma_bf16_ss(tmem, umma_smem_desc_sw128(s0 + kDzO + k16 * 2048, 8192, 1024),
-                             umma_smem_desc_sw128(s0 + kDzA + k16 * 32, 16, 1024), ida, k16 > 0);
+                umma_bf16_ss(tmem, umma_smem_desc_sw128(s0 + kDzO, 8192, 1024) + (k16 * 2048),
+                             umma_smem_desc_sw128(s0 + kDzA, 16, 1024) + (k16 * 32), ida, k16 > 0);
 #pragma unroll
             for (int k16 = 0; k16 < 8; ++k16)     // + dH'^T E^T
-                umma_bf16_ss(tmem, umma_smem_desc_sw128(s0 + kDzH + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024),
-                             umma_smem_desc_sw128(s0 + kDzE + (k16 >> 2) * 8192 + (k16 & 3) * 32, 16, 1024), idb, 1);
+                umma_bf16_ss(tmem, umma_smem_desc_sw128(s0 + kDzH, 16, 1024) + ((k16 >> 2) * 16384 + (k16 & 3) * 32),
+                             umma_smem_desc_sw128(s0 + kDzE, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), idb, 1);
             umma_commit(&bar_mma);
         }
     }
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(256, 3)
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
         tma_store_2d(&mdZT, sm + kDzH, 0, ch * 128);
         tma_store_commit();
         tma_store_wait_read();

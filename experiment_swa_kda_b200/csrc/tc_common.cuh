@@ -151,6 +151,19 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------------- UMMA
+// One lane of a converged warp, the same one every time.  Products and bulk copies are issued by the lane this picks in a warp
+// whose index is known to be uniform: the instruction takes its operands from uniform registers, and the compiler computes
+// them there only where it can see that a single lane of the warp runs.  Behind `tid == 0` every operand was moved over first:
+// 16 products took 1,500 cycles to issue, with one addition a descriptor 1,180, behind this 860.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok));
+    return ok != 0;
+}
 constexpr uint32_t kMajorK = 0, kMajorMN = 1;
 
 // kind::f16 instruction descriptor: BF16 operands, FP32 accumulator, dense.
@@ -163,35 +176,37 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N, uint32_t a_
 // Shared-memory matrix descriptor, 128-byte swizzle.  K-major: rows of 128 bytes (64 bf16), sbo = bytes
 // between 8-row groups (1024 when rows are packed), lbo unused (encoded as 16 bytes).  MN-major: lbo =
 // bytes between 64-element blocks along M/N, sbo = bytes between 8-row groups along K.
-__device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= 1ull << 46;   // descriptor version for sm_100
-    d |= 2ull << 61;   // SWIZZLE_128B
-    return d;
+// Adding bytes moves the start address within the tile: one 32-bit addition a step (shared addresses stay below 2^18, so the
+// address field never carries).
+struct UmmaDesc {
+    uint32_t lo, hi;
+};
+__device__ __forceinline__ UmmaDesc operator+(UmmaDesc d, uint32_t bytes) { return UmmaDesc{d.lo + (bytes >> 4), d.hi}; }
+__device__ __forceinline__ UmmaDesc umma_smem_desc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+    // descriptor version for sm_100 at bit 46, SWIZZLE_128B at bit 61
+    return UmmaDesc{(saddr >> 4) | (lbo_bytes >> 4) << 16, (sbo_bytes >> 4) | 1u << 14 | 2u << 29};
 }
 
 // D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
+__device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, UmmaDesc a, UmmaDesc b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %2};\n\t"
+        "mov.b64 b, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand lives in tensor memory, lane = row, 16-bit elements packed two per
 // 32-bit column (K = 16 per instruction is 8 columns).  Issued by ONE thread.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, UmmaDesc b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // All previously issued UMMAs of this thread arrive on `bar` when complete (implies fence::before_thread_sync).
