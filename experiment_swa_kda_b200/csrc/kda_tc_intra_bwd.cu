@@ -14,7 +14,7 @@
 //     RP_I^T = k~_I^T [dA_I ; beta dM_I]^T      CP_I^T = [q~_I ; k-_I]^T [dA_I ; beta dM_I]
 // Restates reference chunk_wy_backward.cu:2818-3331 (local VJP), 3337-3552 (pull-back), 3787-3894 (finalize).
 
-#include <cstdio>
+#include <algorithm>
 
 #include "common.cuh"
 #include "simt_ws.cuh"
@@ -113,7 +113,7 @@ struct IntraBwdArgs {
     const __nv_bfloat16* Mt;          // [nch][64][64] M~ (before beta)
     __nv_bfloat16 *dq, *dk, *dv;
     void *dg, *dbeta;                 // gate dtype
-    int l2norm, H;
+    int l2norm, H, nslots;
     float scale;
     int* status;
 };
@@ -123,26 +123,27 @@ constexpr int kR1 = 0;         // 64 KB  H | dH' panels            -> later: k~_
 constexpr int kR2 = 65536;     // 16 KB  dO tile                   -> later: X^T tile (8 KB) | Y tile (8 KB)
 constexpr int kR3 = 81920;     // 16 KB  Z^T panel                 -> later: target stacks I = 0,1 (2 x 8 KB)
 constexpr int kR4 = 98304;     // 16 KB  dZ^T panel                -> later: target stacks I = 2,3
-constexpr int kR5 = 114688;    // 48 KB  q | k | v tiles           -> later: dv in the v tile
+constexpr int kR5 = 114688;    // 48 KB  q | k | v tiles           -> later: dq | dk | dv, on their way out
 constexpr int kR6 = 163840;    //  8 KB  T
-constexpr int kR7 = 172032;    // 16 KB  dW^T                      -> later: [dA_I ; beta dM_I] tiles (4 x 4 KB)
+constexpr int kR7 = 172032;    // 16 KB  dW^T                      -> later: [dA_I ; beta dM_I] tiles (4 x 4 KB), dg on its way out
 constexpr int kR8 = 188416;    // 16 KB  g tile (bf16 gates)       -> later: Q' = e^G k
 constexpr int kRM = 204800;    //  8 KB  M~ (before beta), row-major [target][source]
-// floats: gfirst[4][128] gsum[4][128] eC[4][128] eEnd[4][128] fb[4][128] part[4][128] egend[128] dots[2][4][64] rowv[3][64] rowb[2][64]
+// floats: gfirst[4][128] gsum[4][128] eC[4][128] eEnd[4][128] fb[4][128] part[4][128] egend[128] dots[2][4][64] rowb[2][64]
+//         rowv[2][3][64] (this chunk-head's and the next one's)
 constexpr int kSmall = 212992;
-constexpr int kIntraBwdSmem = kSmall + (24 * 128 + 128 + 512 + 3 * 64 + 2 * 64) * 4 + 1024;
-
+constexpr int kIntraBwdSmem = kSmall + (24 * 128 + 128 + 512 + 2 * 64 + 2 * 3 * 64) * 4 + 1024;
+constexpr int kBwdCtas = 148;      // one to an SM
 // Bound by latency: 225 KB of shared memory allow one CTA per SM, and its products depend on one another (state products
 // -> X -> Y -> dM -> pull-back).  So (1) only the operand of the next product is read out before that product is issued,
 // and everything else - dv, the dR / dE / dQ contributions, the pull-back's decay panels - runs while it is in flight;
-// (2) of the six state products the two that the next phase needs are issued first, the others by warps that have finished
-// their share of the work beside them; (3) a warp fetches the inputs
-// of the CTA that this SM is likely to run next into L2; (4) token pairs go through packed float32 arithmetic; (5) a lane's
-// elements lie in 8 x 8 pieces, so that tiles are read and written by ldmatrix / stmatrix, four pieces an instruction, a row
-// scalar serves eight of its elements and a row dot takes 7 shuffles: with a channel and 16 tokens a lane, its 2-byte accesses, row
-// scalars and 31 shuffles had been a quarter of a block's cycles.
-// 16,384 chunk-heads: 1,725 -> 1,380 us, 384: 65 -> 52 us (2,262 and 81 before (1) to (4)); the last 110 us of it are cheaper
-// issue of the products (elect_one).
+// (2) the products that the chain does not wait for are issued where it leaves a gap; (3) a CTA walks over chunk-heads: a tile's
+// next contents are loaded as soon as its last reader is done, all but q, k and the gates behind the pull-back, so that the next
+// chunk-head starts without a launch, without an allocation and with its operands there; (4) token pairs go through packed
+// float32 arithmetic; (5) a lane's elements lie in 8 x 8 pieces, so that tiles are read and written by ldmatrix / stmatrix, four
+// pieces an instruction, a row scalar serves eight of its elements and a row dot takes 7 shuffles: with a channel and 16 tokens a
+// lane, its 2-byte accesses, row scalars and 31 shuffles had been a quarter of a block's cycles.
+// 16,384 chunk-heads: 1,725 -> 1,207 us (1,490 by (2) and (5), 1,380 with cheaper issue, see elect_one; 2,262 before (1) and (4)),
+// 384: 65 -> 50 us.
 template <bool GB>
 __global__ void __launch_bounds__(512, 1)
     tc_intra_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
@@ -150,7 +151,9 @@ __global__ void __launch_bounds__(512, 1)
                         const __grid_constant__ CUtensorMap mT, const __grid_constant__ CUtensorMap mH,
                         const __grid_constant__ CUtensorMap mdH, const __grid_constant__ CUtensorMap mZT,
                         const __grid_constant__ CUtensorMap mdZT, const __grid_constant__ CUtensorMap mMt,
-                        const __grid_constant__ CUtensorMap mg, IntraBwdArgs p) {
+                        const __grid_constant__ CUtensorMap mg, const __grid_constant__ CUtensorMap mdq,
+                        const __grid_constant__ CUtensorMap mdk, const __grid_constant__ CUtensorMap mdv,
+                        const __grid_constant__ CUtensorMap mdg, IntraBwdArgs p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
     uint8_t* Hs = sm + kR1;
@@ -173,18 +176,23 @@ __global__ void __launch_bounds__(512, 1)
     float* part = fbk + 512;                               // [4][128] partial sums of dD
     float* egend = part + 512;                             // [128]
     float* dots = egend + 128;                             // [2][4][64] row dots: q | k, channel quarter, row
-    float* rowv = dots + 512;                              // [3][64]  qinv * scale | kinv | beta
-    float* rowb = rowv + 192;                              // [2][64]  what the row dots take off q and k, per unit row
+    float* rowb = dots + 512;                              // [2][64]  what the row dots take off q and k, per unit row
+    float* rowv2 = rowb + 128;                             // [2][3][64]  qinv * scale | kinv | beta
     float* tot = gsum;                                     // [4][128] block sums of dG (the sums of g are done with)
     float* ge = gfirst;                                    // [4][128] block sums of dE * E
-    __shared__ uint64_t bar_g, bar_in[2], bar_w, bar_x, bar_q, bar_y, bar_r, bar_m, bar_pb;
+    __shared__ uint64_t bar_g, bar_a, bar_qk, bar_w, bar_x, bar_q, bar_y, bar_r, bar_m, bar_pb;
     __shared__ uint32_t tmem_slot;
+    __shared__ int next[3];                         // the next chunk-head: index (past the end: none), length, first token
     __shared__ __align__(8) float dA_diag[64];      // dA[i][i]: applied to dq, dk in float32, outside the pull-back products
 
-    const int slot = blockIdx.x, h = blockIdx.y, H = p.H;
-    const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
-    if (len == 0) return;
-    const int ch = slot * H + h;
+    const int H = p.H, total = p.nslots * H;
+    int work = blockIdx.x, len = 0, tok0 = 0;       // chunk-heads blockIdx.x, + gridDim.x, ...; heads slowest; empty slots are skipped
+    for (; work < total; work += gridDim.x) {
+        len = p.chunk_len[work % p.nslots];
+        if (len > 0) break;
+    }
+    if (work >= total) return;
+    tok0 = p.chunk_tok0[work % p.nslots];
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int I = warp >> 2, wq = warp & 3;       // row block and channel quarter of this warp
     const int c4 = lane & 3, r8 = lane >> 2;      // token pair and channel inside an 8 x 8 piece
@@ -218,12 +226,13 @@ __global__ void __launch_bounds__(512, 1)
     };
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
+    constexpr uint32_t kBytesA = 65536 + 3 * 16384 + 2 * 8192;      // H, dH', Z^T, dZ^T, dO, T, M~
     // The gates come first, then what the critical products and the work beside them need.  The loads are issued by warps 1-4,
     // a few each: one thread issuing all of them held the block back.
     if (tid == 0) {
         mbar_init(&bar_g, 1);
-        mbar_init(&bar_in[0], 1);
-        mbar_init(&bar_in[1], 1);
+        mbar_init(&bar_a, 2);
+        mbar_init(&bar_qk, 1);
         mbar_init(&bar_w, 1);
         mbar_init(&bar_r, 1);
         mbar_init(&bar_x, 1);
@@ -232,46 +241,59 @@ __global__ void __launch_bounds__(512, 1)
         mbar_init(&bar_m, 1);
         mbar_init(&bar_pb, 4);
         if (GB) mbar_expect_tx(&bar_g, 16384);
-        mbar_expect_tx(&bar_in[0], 32768 + 16384 * 4);
-        mbar_expect_tx(&bar_in[1], 32768 + 16384 * 2 + 8192 * 2);
+        mbar_expect_tx(&bar_a, kBytesA);
+        mbar_expect_tx(&bar_a, 16384);              // v
+        mbar_expect_tx(&bar_qk, 32768);
         mbar_fence_init();
     }
     __syncthreads();
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
 
     if (warp >= 1 && warp <= 4 && elect_one()) {
+        const int h = work / p.nslots, ch = (work - h * p.nslots) * H + h;
         if (warp == 1) {
-            for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_in[0], mb * 64, ch * 128);
-            tma_load_2d(dZTs, &mdZT, &bar_in[0], 0, ch * 128);
-            tma_load_2d(Ts, &mT, &bar_in[1], 0, ch * 64);
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_a, mb * 64, ch * 128);
+            tma_load_2d(dZTs, &mdZT, &bar_a, 0, ch * 128);
+            tma_load_2d(Ts, &mT, &bar_a, 0, ch * 64);
         } else if (warp == 2) {
             for (int mb = 0; mb < 2; ++mb) {
-                tma_load_2d(vs + mb * 8192, &mv, &bar_in[0], h * 128 + mb * 64, tok0);
-                tma_load_2d(dOs + mb * 8192, &mdO, &bar_in[1], h * 128 + mb * 64, tok0);
+                tma_load_2d(vs + mb * 8192, &mv, &bar_a, h * 128 + mb * 64, tok0);
+                tma_load_2d(dOs + mb * 8192, &mdO, &bar_a, h * 128 + mb * 64, tok0);
             }
         } else if (warp == 3) {
             if (GB)
                 for (int mb = 0; mb < 2; ++mb) tma_load_2d(Qp + mb * 8192, &mg, &bar_g, h * 128 + mb * 64, tok0);
-            for (int mb = 0; mb < 2; ++mb) tma_load_2d(ks + mb * 8192, &mk, &bar_in[0], h * 128 + mb * 64, tok0);
-            for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_in[1], mb * 64, ch * 128);
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(ks + mb * 8192, &mk, &bar_qk, h * 128 + mb * 64, tok0);
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_a, mb * 64, ch * 128);
         } else {
-            for (int mb = 0; mb < 2; ++mb) tma_load_2d(qs + mb * 8192, &mq, &bar_in[0], h * 128 + mb * 64, tok0);
-            tma_load_2d(ZTs, &mZT, &bar_in[1], 0, ch * 128);
-            tma_load_2d(Mts, &mMt, &bar_in[1], 0, ch * 64);
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(qs + mb * 8192, &mq, &bar_qk, h * 128 + mb * 64, tok0);
+            tma_load_2d(ZTs, &mZT, &bar_a, 0, ch * 128);
+            tma_load_2d(Mts, &mMt, &bar_a, 0, ch * 64);
         }
     }
     __syncwarp();
+    // the row scalars of a chunk-head, 64 threads
+    auto load_rows = [&](float* dst, int ch) {
+        const float* src[3] = {p.qinv, p.kinv, p.beta};
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + 64 * j + tid)), "l"(src[j] + (size_t)ch * 64 + tid) : "memory");
+    };
+    if (tid < 64) load_rows(rowv2, (work % p.nslots) * H + work / p.nslots);
+    bool ok = true;
+#pragma unroll 1
+    for (uint32_t ph = 0;; ph ^= 1) {       // every barrier below completes once a round
+    const int h = work / p.nslots;
+    float* rowv = rowv2 + 192 * ph;
     // ---- per-row scalars and the log-decay relative to the block's first row
     if (tid < 64) {
-        rowv[tid] = p.qinv[ch * 64 + tid] * p.scale;
-        rowv[64 + tid] = p.kinv[ch * 64 + tid];
-        rowv[128 + tid] = p.beta[ch * 64 + tid];
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        rowv[tid] *= p.scale;
     }
-    bool ok = true;
     f2 E[8];
     if constexpr (GB) {
         uint32_t w[8];
-        ok = mbar_wait(&bar_g, 0, p.status, 40);
+        ok = mbar_wait(&bar_g, ph, p.status, 40);
         get_tile(sb + kR8, w);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -342,7 +364,7 @@ __global__ void __launch_bounds__(512, 1)
     if (len < 64) {
         // rows past a ragged tail hold the next sequence's tokens: blank them (0 x Inf would otherwise reach this sequence's
         // gradients)
-        ok = ok && mbar_wait(&bar_in[0], 0, p.status, 40) && mbar_wait(&bar_in[1], 0, p.status, 40);
+        ok = ok && mbar_wait(&bar_a, ph, p.status, 40) && mbar_wait(&bar_qk, ph, p.status, 40);
         if (ok) {
             for (int idx = tid; idx < (64 - len) * 16; idx += 512) {
                 const int r = len + (idx >> 4), c = idx & 15;
@@ -361,7 +383,7 @@ __global__ void __launch_bounds__(512, 1)
     // One thread issues the products, and they run in that order: dW and the first half of X, what the next link of the chain
     // X -> Y -> dM waits for, go first; the five others (~300 cycles each of operand reads) go where the chain's next product
     // is still being prepared.  Issued all at once from four warps they held those warps, and with them the block, back.
-    ok = ok && mbar_wait(&bar_in[0], 0, p.status, 40);
+    ok = ok && mbar_wait(&bar_a, ph, p.status, 40);
     if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
@@ -390,6 +412,7 @@ __global__ void __launch_bounds__(512, 1)
         for (int e = 0; e < 8; ++e) x[e] = f2_mul(f2_from_bf16(w[e]), s[e & 1]);
     };
     constexpr uint32_t kQt = kR5, kKt = kR5 + 16384;
+    ok = ok && mbar_wait(&bar_qk, ph, p.status, 40);
     {
         // Q' = e^G k for Xraw^T -= Q' dW^T, stored [key d][token] (MN-major A)
         f2 w[8];
@@ -399,7 +422,6 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = f2_mul(f2_mul(E[e], f2_all(ec[e >> 1])), w[e]);
         put_panel(sb + kR8, 2 * I, w);
-        ok = ok && mbar_wait(&bar_in[1], 0, p.status, 40);
         // eight adjacent channels of four value rows a lane; the warp's eight lanes that share them add up by halving
         const int cg = 4 * wq + mi;
         f2 acc[4];
@@ -449,7 +471,7 @@ __global__ void __launch_bounds__(512, 1)
                          umma_smem_desc_sw128(bZ, 8192, 1024) + (k16 * 2048), id64_k_mn, k16 > 0);
     }
     __syncwarp();
-    ok = ok && mbar_wait(&bar_w, 0, p.status, 41);
+    ok = ok && mbar_wait(&bar_w, ph, p.status, 41);
     tc_fence_after();
 
     // ================================================================ phase 2: X and dQ
@@ -482,7 +504,7 @@ __global__ void __launch_bounds__(512, 1)
         umma_commit(&bar_q);
     }
     __syncwarp();
-    ok = ok && mbar_wait(&bar_x, 0, p.status, 42);
+    ok = ok && mbar_wait(&bar_x, ph, p.status, 42);
     tc_fence_after();
 
     // ================================================================ phase 3: Y, dM
@@ -533,7 +555,7 @@ __global__ void __launch_bounds__(512, 1)
         umma_commit(&bar_r);
     }
     __syncwarp();
-    ok = ok && mbar_wait(&bar_q, 0, p.status, 42);
+    ok = ok && mbar_wait(&bar_q, ph, p.status, 42);
     tc_fence_after();
     {
         // in flight: dv = beta dP, staged [token][channel] in the value tile (only the completed products read it) so that
@@ -545,7 +567,7 @@ __global__ void __launch_bounds__(512, 1)
         for (int e = 0; e < 8; ++e) t[e] = f2_mul(bt[e & 1], t[e]);
         put_tile(sb + kR5 + 32768, t);
     }
-    ok = ok && mbar_wait(&bar_y, 0, p.status, 43);
+    ok = ok && mbar_wait(&bar_y, ph, p.status, 43);
     tc_fence_after();
     {
         f2 t[4];
@@ -563,10 +585,14 @@ __global__ void __launch_bounds__(512, 1)
             umma_bf16_ss(tmem + cM, umma_smem_desc_sw128(sb + kYt, 16, 1024) + (k16 * 32),
                          umma_smem_desc_sw128(smem_u32(Ts), 16, 1024) + (k16 * 32), id, k16 > 0);
         umma_commit(&bar_m);
+        if (len == 64) {      // in flight: the dv rows leave
+            for (int mb = 0; mb < 2; ++mb) tma_store_2d(&mdv, vs + mb * 8192, h * 128 + mb * 64, tok0);
+            tma_store_commit();
+        }
     }
     __syncwarp();
 
-    if (ok) {      // in flight: the dv rows leave
+    if (len < 64 && ok) {      // the rows past a ragged tail are not this sequence's: the others one by one
         const int c = tid & 15;
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
@@ -576,7 +602,7 @@ __global__ void __launch_bounds__(512, 1)
                     *reinterpret_cast<const uint4*>(vs + (c >> 3) * 8192 + sw128_off(i, c & 7));
         }
     }
-    ok = ok && mbar_wait(&bar_r, 0, p.status, 42);       // every product up to dE is complete: its operands' tiles are free
+    ok = ok && mbar_wait(&bar_r, ph, p.status, 42);       // every product up to dE is complete: its operands' tiles are free
     tc_fence_after();
 
     // ================================================================ phase 4: pull-back operands
@@ -585,6 +611,12 @@ __global__ void __launch_bounds__(512, 1)
     uint8_t* DAt = sm + kR7;          // [I][32 rows: 16 dA rows, 16 beta*dM rows][64 s]   K-major / MN-major B
     // this warp's 16 rows of dA or dM go to the tile of row block wq
     const uint32_t da_off = kR7 + wq * 4096 + sw128_off(8 * (mi >> 1) + mr, 2 * I + (mi & 1));
+    // the next chunk-head of this CTA: one warp looks it up
+    int nwork = work + gridDim.x, nlen = 0, ntok0 = 0;
+    if (warp == 15 && nwork < total) {
+        nlen = p.chunk_len[nwork % p.nslots];
+        ntok0 = p.chunk_tok0[nwork % p.nslots];
+    }
     {
         // in flight: the decay panels.  Both operand families are stored transposed, [channel d][row] (K-major A operands).
         const uint32_t X = sb + kR3 + (I >> 1) * 16384;      // two target blocks share a panel: 32 stack rows each
@@ -633,7 +665,21 @@ __global__ void __launch_bounds__(512, 1)
         }
         stsm_x4(sb + da_off, w);
     }
-    ok = ok && mbar_wait(&bar_m, 0, p.status, 44);
+    if (warp == 15) {
+        while (nwork < total && nlen == 0) {
+            nwork += gridDim.x;
+            if (nwork < total) {
+                nlen = p.chunk_len[nwork % p.nslots];
+                ntok0 = p.chunk_tok0[nwork % p.nslots];
+            }
+        }
+        if (lane == 0) {
+            next[0] = nwork;
+            next[1] = nlen;
+            next[2] = ntok0;
+        }
+    }
+    ok = ok && mbar_wait(&bar_m, ph, p.status, 44);
     tc_fence_after();
     {
         // row j of dM = -stril(Y T^T); dbeta gets sum_l dM[j][l] M~[j][l]
@@ -694,38 +740,10 @@ __global__ void __launch_bounds__(512, 1)
         const int i = tid - 128;
         st_io(p.dbeta, (size_t)(tok0 + i) * H + h, GB, dbp[i] + dbp[64 + i] + dbp[128 + i] + dbp[192 + i]);
     }
-    if (warp == 11) {
-        // the inputs of the block that starts when this one ends, 148 further on, into L2
-        const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + 148u;
-        if (nxt < gridDim.x * gridDim.y) {
-            const int ns = (int)(nxt % gridDim.x), nh = (int)(nxt / gridDim.x);
-            const int nlen = p.chunk_len[ns], nt0 = p.chunk_tok0[ns], nch = ns * H + nh;
-            if (nlen > 0) {
-                if (lane < 2) {
-                    tma_prefetch_2d(&mH, lane * 64, nch * 128);
-                    tma_prefetch_2d(&mdH, lane * 64, nch * 128);
-                    tma_prefetch_2d(&mdO, nh * 128 + lane * 64, nt0);
-                    tma_prefetch_2d(&mq, nh * 128 + lane * 64, nt0);
-                    tma_prefetch_2d(&mk, nh * 128 + lane * 64, nt0);
-                    tma_prefetch_2d(&mv, nh * 128 + lane * 64, nt0);
-                    if (GB) tma_prefetch_2d(&mg, nh * 128 + lane * 64, nt0);
-                } else if (lane == 2) {
-                    tma_prefetch_2d(&mZT, 0, nch * 128);
-                    tma_prefetch_2d(&mdZT, 0, nch * 128);
-                    tma_prefetch_2d(&mT, 0, nch * 64);
-                    tma_prefetch_2d(&mMt, 0, nch * 64);
-                }
-                if (!GB) {
-                    for (int i = lane; i < nlen; i += 32) {
-                        const char* gp = static_cast<const char*>(p.g) + (((size_t)(nt0 + i) * H + nh) * 128) * 4;
-#pragma unroll
-                        for (int b = 0; b < 512; b += 128) prefetch_l2(gp + b);
-                    }
-                }
-            }
-        }
-        __syncwarp();
-    }
+    nwork = next[0];
+    const bool more = nwork < total;
+    const int nh = more ? nwork / p.nslots : 0, nch = more ? (nwork - nh * p.nslots) * H + nh : 0;
+    if (more && tid < 64) load_rows(rowv2 + 192 * (ph ^ 1), nch);
     // in flight: the dR part of dq, the dE and dQ parts of dk, the diagonal of dA
     f2 dqn[8], dkn[8], kn[8], dG[8];
     float ge4[4];      // sum of dE * E over this lane's tokens, per channel
@@ -772,8 +790,31 @@ __global__ void __launch_bounds__(512, 1)
             dG[e] = f2_fma(dQ, kn[e], dG[e]);
         }
     }
-    ok = ok && mbar_wait(&bar_pb, 0, p.status, 45);
+    ok = ok && mbar_wait(&bar_pb, ph, p.status, 45);
     tc_fence_after();
+    // The products are done with every operand: the next chunk-head's take their places.
+    if (warp == 15 && elect_one() && ok && more) {
+        const int nt0 = next[2];
+        mbar_expect_tx(&bar_a, kBytesA);
+        for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_a, mb * 64, nch * 128);
+        tma_load_2d(dZTs, &mdZT, &bar_a, 0, nch * 128);
+        for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_a, mb * 64, nch * 128);
+        for (int mb = 0; mb < 2; ++mb) tma_load_2d(dOs + mb * 8192, &mdO, &bar_a, nh * 128 + mb * 64, nt0);
+        tma_load_2d(ZTs, &mZT, &bar_a, 0, nch * 128);
+        tma_load_2d(Ts, &mT, &bar_a, 0, nch * 64);
+        tma_load_2d(Mts, &mMt, &bar_a, 0, nch * 64);
+        for (int mb = 0; mb < 2; ++mb) {            // into L2 only: their tiles are still in use
+            if (GB) tma_prefetch_2d(&mg, nh * 128 + mb * 64, nt0);
+            tma_prefetch_2d(&mk, nh * 128 + mb * 64, nt0);
+            tma_prefetch_2d(&mq, nh * 128 + mb * 64, nt0);
+        }
+    }
+    if (warp == 12 && elect_one() && ok && more) {
+        tma_store_wait_read();                      // dv has left the value tile
+        mbar_expect_tx(&bar_a, 16384);
+        for (int mb = 0; mb < 2; ++mb) tma_load_2d(vs + mb * 8192, &mv, &bar_a, nh * 128 + mb * 64, next[2]);
+    }
+    __syncwarp();
 
     // ================================================================ phase 5: assemble the gradients
     {
@@ -873,6 +914,11 @@ __global__ void __launch_bounds__(512, 1)
         dots[(r8 >> 2) * 256 + wq * 64 + tb + 8 * ((r8 >> 1) & 1) + (r8 & 1)] = v8[0];
     }
     __syncthreads();
+    if (GB && warp == 14 && elect_one() && ok && more) {      // Q' and the dbeta sums have been read
+        mbar_expect_tx(&bar_g, 16384);
+        for (int mb = 0; mb < 2; ++mb) tma_load_2d(Qp + mb * 8192, &mg, &bar_g, nh * 128 + mb * 64, next[2]);
+    }
+    __syncwarp();
     if (tid < 128) {      // the four quarters of the channels -> what a row's dot takes off its gradient, per unit of q or -k
         const float* q4 = dots + (tid >> 6) * 256 + (tid & 63);
         const float dot = (q4[0] + q4[64]) + (q4[128] + q4[192]);
@@ -892,24 +938,24 @@ __global__ void __launch_bounds__(512, 1)
     }
     __syncthreads();
     {
-        // The gradients go through shared memory (the source-panel region is free now), so that they leave as 16-byte row
-        // segments.
+        // The gradients go through shared memory, so that they leave as whole rows: dq and dk over q and k, of which a warp
+        // overwrites only the pieces that it alone has read, dg over the dead tiles of the pull-back.
         const f2 qa[2] = {ld_2(rowv + tb), ld_2(rowv + tb + 8)}, qb[2] = {ld_2(rowb + tb), ld_2(rowb + tb + 8)};
 #pragma unroll
         for (int e = 0; e < 8; ++e) dqn[e] = f2_fma(qn[e], qb[e & 1], f2_mul(dqn[e], qa[e & 1]));
-        put_tile(sb + kR1, dqn);
+        put_tile(sb + kQt, dqn);
         const f2 ka[2] = {ld_2(rowv + 64 + tb), ld_2(rowv + 64 + tb + 8)}, kb[2] = {ld_2(rowb + 64 + tb), ld_2(rowb + 64 + tb + 8)};
 #pragma unroll
         for (int e = 0; e < 8; ++e) dkn[e] = f2_fma(kn[e], kb[e & 1], f2_mul(dkn[e], ka[e & 1]));
-        put_tile(sb + kR1 + 16384, dkn);
+        put_tile(sb + kKt, dkn);
         float run[4];
         chan4(run, eC + I * 128);
 #pragma unroll
         for (int e = 0; e < 8; ++e) dG[e] = f2_add(dG[e], f2_all(run[e >> 1]));
         if (GB) {
-            put_tile(sb + kR1 + 32768, dG);
+            put_tile(sb + kR7, dG);
         } else {
-            float* tg = reinterpret_cast<float*>(sm + kR1 + 32768);      // [64][128], 16-byte columns turned by the row pair
+            float* tg = reinterpret_cast<float*>(sm + kR7);      // [64][128] (over Q' too), 16-byte columns turned by the row pair
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float2 x = f2_get(dG[e]);
@@ -919,31 +965,72 @@ __global__ void __launch_bounds__(512, 1)
             }
         }
     }
-    __syncthreads();
-    if (ok) {
+    if (tid < 64) asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    if (len < 64 || !GB) {
         const int c = tid & 15;
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
             const int i = pass * 32 + (tid >> 4);
             if (i < len) {
                 const size_t o = ((size_t)(tok0 + i) * H + h) * 128;
-                const uint8_t* src = sm + kR1 + (c >> 3) * 8192 + sw128_off(i, c & 7);
-                *reinterpret_cast<uint4*>(p.dq + o + 8 * c) = *reinterpret_cast<const uint4*>(src);
-                *reinterpret_cast<uint4*>(p.dk + o + 8 * c) = *reinterpret_cast<const uint4*>(src + 16384);
+                const uint32_t off = (c >> 3) * 8192 + sw128_off(i, c & 7);
+                if (len < 64) {
+                    *reinterpret_cast<uint4*>(p.dq + o + 8 * c) = *reinterpret_cast<const uint4*>(qs + off);
+                    *reinterpret_cast<uint4*>(p.dk + o + 8 * c) = *reinterpret_cast<const uint4*>(ks + off);
+                }
                 if (GB) {
-                    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dg) + o + 8 * c) = *reinterpret_cast<const uint4*>(src + 32768);
+                    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dg) + o + 8 * c) = *reinterpret_cast<const uint4*>(sm + kR7 + off);
                 } else {
-                    const float* tg = reinterpret_cast<const float*>(sm + kR1 + 32768) + i * 128;
+                    const float* tg = reinterpret_cast<const float*>(sm + kR7) + i * 128;
                     float* dgp = reinterpret_cast<float*>(p.dg) + o;
                     *reinterpret_cast<uint4*>(dgp + 4 * c) = *reinterpret_cast<const uint4*>(tg + ((c ^ (i >> 1)) & 31) * 4);
                     *reinterpret_cast<uint4*>(dgp + 64 + 4 * c) = *reinterpret_cast<const uint4*>(tg + (((16 + c) ^ (i >> 1)) & 31) * 4);
                 }
             }
         }
+        __syncthreads();
     }
+    if (warp == 15 && elect_one()) {
+        if (len == 64) {
+            for (int mb = 0; mb < 2; ++mb) {
+                tma_store_2d(&mdq, qs + mb * 8192, h * 128 + mb * 64, tok0);
+                tma_store_2d(&mdk, ks + mb * 8192, h * 128 + mb * 64, tok0);
+                if (GB) tma_store_2d(&mdg, sm + kR7 + mb * 8192, h * 128 + mb * 64, tok0);
+            }
+            tma_store_commit();
+        }
+        tma_store_wait_read();
+        if (more) {
+            const int nt0 = next[2];
+            mbar_expect_tx(&bar_qk, 32768);
+            for (int mb = 0; mb < 2; ++mb) {
+                tma_load_2d(ks + mb * 8192, &mk, &bar_qk, nh * 128 + mb * 64, nt0);
+                tma_load_2d(qs + mb * 8192, &mq, &bar_qk, nh * 128 + mb * 64, nt0);
+            }
+        }
+    }
+    __syncwarp();
+    if (!more) break;
+    work = nwork;
+    len = next[1];
+    tok0 = next[2];
+    }
+    if (!ok && tid == 0) {       // unwinding: copies in flight must land before the block may exit
+        for (uint32_t par = 0; par < 2; ++par) {
+            mbar_poll(&bar_a, par, kSpinLimit / 8);
+            mbar_poll(&bar_qk, par, kSpinLimit / 8);
+            mbar_poll(&bar_g, par, kSpinLimit / 8);
+        }
+    }
+    if (warp == 12 && elect_one()) tma_store_wait_read();      // shared memory must outlive the reads of the bulk stores
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 512);
+    if (warp == 0) tmem_dealloc(tmem_slot, 512);
 }
 
 }  // namespace tc
@@ -954,7 +1041,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     using namespace tc;
     const uint64_t nch = (uint64_t)w.nslots * w.H;
     const uint64_t cols = (uint64_t)w.H * 128;
-    CUtensorMap mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg;
+    CUtensorMap mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg, mdq, mdk, mdv, mdg;
     int rc = 0;
     rc |= make_map_bf16(&mq, q, (uint64_t)tokens, cols, 64, 64);
     rc |= make_map_bf16(&mk, k, (uint64_t)tokens, cols, 64, 64);
@@ -966,8 +1053,11 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     rc |= make_map_bf16(&mZT, t.ZT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mdZT, t.dZT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mMt, t.Mt, nch * 64, 64, 64, 64);
-    if (gbf16) rc |= make_map_bf16(&mg, g, (uint64_t)tokens, cols, 64, 64);
-    else mg = mq;      // float32 gates are read by the threads
+    rc |= make_map_bf16(&mdq, dq, (uint64_t)tokens, cols, 64, 64);
+    rc |= make_map_bf16(&mdk, dk, (uint64_t)tokens, cols, 64, 64);
+    rc |= make_map_bf16(&mdv, dv, (uint64_t)tokens, cols, 64, 64);
+    if (gbf16) rc |= make_map_bf16(&mg, g, (uint64_t)tokens, cols, 64, 64) | make_map_bf16(&mdg, dg, (uint64_t)tokens, cols, 64, 64);
+    else mg = mdg = mq;      // float32 gates and their gradients go through the threads
     if (rc) return KDA_ERR_CUDA;
     IntraBwdArgs a;
     a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len;
@@ -975,11 +1065,11 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     a.v = static_cast<const __nv_bfloat16*>(v); a.g = g;
     a.qinv = w.qinv; a.kinv = w.kinv; a.beta = w.beta; a.Mt = t.Mt;
     a.dq = static_cast<__nv_bfloat16*>(dq); a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
-    a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.scale = scale; a.status = t.status;
+    a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.nslots = w.nslots; a.scale = scale; a.status = t.status;
     auto kern = gbf16 ? tc_intra_bwd_kernel<true> : tc_intra_bwd_kernel<false>;
     if (set_smem_limit(kern, kIntraBwdSmem)) return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_intra_bwd_kernel", st,
-               kern<<<dim3(w.nslots, w.H), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg, a));
+               kern<<<(unsigned)std::min<uint64_t>(nch, kBwdCtas), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg, mdq, mdk, mdv, mdg, a));
     return launch_status();
 }
 

@@ -200,6 +200,30 @@ def test_split_scans_agree_with_the_single_chain_and_the_oracle(T):
     _run_activated(d)                           # the split path against the oracle
 
 
+@pytest.mark.parametrize("gate", [torch.bfloat16, torch.float32])
+def test_blocks_that_walk_over_many_chunk_heads_equal_blocks_with_one(gate):
+    """The backward's blocks walk over chunk-heads, one block to an SM.  A head's results do not depend on the others', so a
+    batch with several chunk-heads to a block - full, ragged, one-token and unused ones in turn - has to give the bits of the
+    same heads in groups so small that every block has one."""
+    m = _kda_mod()
+    lens, H, group = [200, 64, 1, 0, 129, 320, 63], 40, 8
+    T = sum(lens)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=D0)
+    d = {n: t.bfloat16().to(D0) for n, t in O.make_inputs(1, T, H, 128, 128, seed=77).items()}
+    d["g"], d["beta"] = d["g"].to(gate), d["beta"].to(gate)
+    do = torch.randn(d["v"].shape, generator=torch.Generator().manual_seed(8)).bfloat16().to(D0)
+
+    def run(heads):
+        x = [d[n][:, :, heads].contiguous().requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+        o, _ = m.chunk_kda(*x, cu_seqlens=cu, lane="tc")
+        return [o, *torch.autograd.grad(o, x, do[:, :, heads].contiguous())]
+
+    whole = run(slice(0, H))
+    for h0 in range(0, H, group):
+        for a, b in zip(whole, run(slice(h0, h0 + group))):
+            assert torch.equal(a[:, :, h0:h0 + group], b)
+
+
 @pytest.mark.parametrize("lens,H", [([64 * 40 + 5, 30, 64 * 70 + 1], 2),          # 6 recurrences, mean 37 chunks -> 4 segments
                                     ([64 * 60 + 3, 0, 64 * 99, 1], 3),             # 12 recurrences, mean 39 chunks -> 4 segments
                                     ([64 * 50, 64 * 3 + 9, 0, 64 * 19 + 63], 4)])  # 16 recurrences, mean 18 chunks -> 2 segments
