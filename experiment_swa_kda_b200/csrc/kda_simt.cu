@@ -191,7 +191,7 @@ __device__ __forceinline__ float row_sum16(float x) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// chunk table: which tokens each 64-token chunk slot covers
+// chunk table of a packed batch (or of one without tokens): which tokens each 64-token chunk slot covers
 // ---------------------------------------------------------------------------------------------
 // A packed batch is described by cu_seqlens, which the caller controls: every segment is checked against the token
 // count and the slot budget before it enters the tables, so that no later kernel can be steered outside the tensors.
@@ -201,14 +201,15 @@ __device__ __forceinline__ float row_sum16(float x) {
 constexpr int kStatusBadCuSeqlens = 10;
 constexpr int kScanOrderMax = 512;      // batches up to this many sequences get a longest-first scan order
 
-__global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_seq, int seq_len, int tokens, int* status, int* mirror) {
+__global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_seq, int tokens, int* status, int* mirror) {
+    const ChunkTable& t = w.tab;
     __shared__ int total;
     if (threadIdx.x == 0) {
         int flag = 0;
         int acc = 0, prev_end = 0;
         for (int s = 0; s < n_seq; ++s) {
-            w.seq_chunk0[s] = acc;
-            int len = seq_len;
+            t.seq_chunk0[s] = acc;
+            int len = 0;
             if (cu) {
                 const int t0 = cu[s], t1 = cu[s + 1];
                 len = t1 - t0;
@@ -220,21 +221,20 @@ __global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_s
             acc += nc;
         }
         if (cu && (cu[0] != 0 || prev_end != tokens)) flag = 1;
-        w.seq_chunk0[n_seq] = acc;
+        t.seq_chunk0[n_seq] = acc;
         total = acc;
-        *status = 0;                                   // every forward starts with a clean status word
-        *reinterpret_cast<int**>(status + 2) = mirror;
+        start_status(status, mirror);
         if (flag) raise_status(status, kStatusBadCuSeqlens);
     }
     __syncthreads();
     for (int s = threadIdx.x; s < n_seq; s += blockDim.x) {
-        const int c0 = w.seq_chunk0[s], nc = w.seq_chunk0[s + 1] - c0;
-        const int t0 = cu ? cu[s] : s * seq_len;
-        const int len = cu ? (cu[s + 1] - cu[s]) : seq_len;
+        const int c0 = t.seq_chunk0[s], nc = t.seq_chunk0[s + 1] - c0;
+        const int t0 = cu ? cu[s] : 0;
+        const int len = cu ? cu[s + 1] - cu[s] : 0;
         for (int j = 0; j < nc; ++j) {
-            w.chunk_seq[c0 + j] = s;
-            w.chunk_tok0[c0 + j] = t0 + j * kChunk;
-            w.chunk_len[c0 + j] = min(kChunk, len - j * kChunk);
+            t.seq[c0 + j] = s;
+            t.tok0[c0 + j] = t0 + j * kChunk;
+            t.len[c0 + j] = min(kChunk, len - j * kChunk);
         }
     }
     // Scan order: the scans run one CTA per (sequence, head) with one CTA per SM, so starting the longest chains first
@@ -243,19 +243,19 @@ __global__ void chunk_table_kernel(Ws w, const int32_t* __restrict__ cu, int n_s
     for (int s = threadIdx.x; s < n_seq; s += blockDim.x) {
         int rank = s;
         if (n_seq <= kScanOrderMax) {
-            const int nc = w.seq_chunk0[s + 1] - w.seq_chunk0[s];
+            const int nc = t.seq_chunk0[s + 1] - t.seq_chunk0[s];
             rank = 0;
             for (int j = 0; j < n_seq; ++j) {
-                const int ncj = w.seq_chunk0[j + 1] - w.seq_chunk0[j];
+                const int ncj = t.seq_chunk0[j + 1] - t.seq_chunk0[j];
                 rank += (ncj > nc || (ncj == nc && j < s)) ? 1 : 0;
             }
         }
-        w.seq_order[rank] = s;
+        t.seq_order[rank] = s;
     }
     for (int c = total + threadIdx.x; c < w.nslots; c += blockDim.x) {
-        w.chunk_seq[c] = -1;
-        w.chunk_tok0[c] = 0;
-        w.chunk_len[c] = 0;
+        t.seq[c] = -1;
+        t.tok0[c] = 0;
+        t.len[c] = 0;
     }
 }
 
@@ -353,6 +353,8 @@ struct IntraArgs {
     const void *q, *k, *v, *g, *beta;
     int bf16, gbf16, l2norm, vec_v, backward;
     float scale;
+    int* mirror;
+    int clear_status;      // no table kernel ran before this one
 };
 // 46 KB and at most 80 registers, so that three CTAs share an SM: the kernel alternates between loads, short products and
 // barriers, and two CTAs (64-wide factor tiles, 83 KB) left the issue slots 60 % idle.
@@ -371,9 +373,11 @@ __global__ void __launch_bounds__(256, 3) intra_fwd_kernel(Ws w, IntraArgs p) {
     float* bsum = bet + 64;              // [8][32] sums of g over 8 rows
     float* cref = bsum + 8 * kHalf;      // [4][32] G at row 8 of each block
     const int slot = blockIdx.x, h = blockIdx.y;
-    const int len = w.chunk_len[slot];
+    if (p.clear_status && slot == 0 && h == 0 && threadIdx.x == 0) start_status(w.status, p.mirror);
+    int len, tok0;
+    w.tab.span(slot, tok0, len);
     if (len == 0) return;
-    const int tok0 = w.chunk_tok0[slot], K = w.K, Kp = w.Kp, V = w.V, Vp = w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
+    const int K = w.K, Kp = w.Kp, V = w.V, Vp = w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
     const size_t ch = (size_t)slot * H + h;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -667,7 +671,7 @@ __global__ void __launch_bounds__(256) scan_kernel(Ws w, ScanArgs p) {
     float* S = reinterpret_cast<float*>(part + 16 * kPartBlock);      // [Kp][kSLD]
     const int Kp = 64 * KT, Vp = w.Vp, K = w.K, V = w.V, H = w.H;
     const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kVS, tid = threadIdx.x;
-    const int c0 = w.seq_chunk0[seq], c1 = w.seq_chunk0[seq + 1], n = c1 - c0;
+    const int c0 = w.tab.first_chunk(seq), c1 = w.tab.first_chunk(seq + 1), n = c1 - c0;
     const int row = tid & 63, cq = tid >> 6;                          // the state element group this thread owns in every 64-row block
     const int l = tid & 15, pq = (tid >> 4) & 3, kg = tid >> 6;       // product: rows 4 l .., column quad, contraction group
     const int grow = tid >> 2, gc = (tid & 3) << 2;                   // global rows of 64 bytes
@@ -770,7 +774,8 @@ __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, in
     extern __shared__ __align__(16) float sm[];
     float *Wt = sm, *Rt = sm + kTile, *Bs = sm + 2 * kTile;
     const int slot = blockIdx.x, h = blockIdx.y, vt = blockIdx.z;
-    const int len = w.chunk_len[slot];
+    int len, tok0;
+    w.tab.span(slot, tok0, len);
     if (len == 0) return;
     const size_t ch = (size_t)slot * w.H + h;
     const int Kp = w.Kp, Vp = w.Vp;
@@ -799,7 +804,7 @@ __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, in
     st_nat(Bs, kLD, u);
     __syncthreads();
     mm64(ao, Wt, Bs);
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15, tok0 = w.chunk_tok0[slot];
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int i = 4 * ty + r;
@@ -818,11 +823,12 @@ __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, in
 __global__ void __launch_bounds__(256) adjoint_term_kernel(Ws w, Scr s, const void* __restrict__ d_o, int bf16, int vec_v) {
     extern __shared__ __align__(16) float sm[];
     const int slot = blockIdx.x, h = blockIdx.y, VT = w.Vp / 64, kt = blockIdx.z / VT, vt = blockIdx.z % VT;
-    const int len = w.chunk_len[slot];
+    int len, tok0;
+    w.tab.span(slot, tok0, len);
     if (len == 0) return;
     const size_t ch = (size_t)slot * w.H + h;
     ld_nat(sm, w.Rm + ch * 64 * w.Kp + kt * 64, w.Kp);
-    ld_tile_io<false>(sm + kTile, d_o, bf16, ((size_t)w.chunk_tok0[slot] * w.H + h) * w.V + vt * 64, (size_t)w.H * w.V, len, w.V - vt * 64, vec_v);
+    ld_tile_io<false>(sm + kTile, d_o, bf16, ((size_t)tok0 * w.H + h) * w.V + vt * 64, (size_t)w.H * w.V, len, w.V - vt * 64, vec_v);
     __syncthreads();
     float acc[4][4];
     zero_acc(acc);
@@ -856,9 +862,10 @@ __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArg
     float* tot = cref + 256;             // [4][64] scratch
     float* gend = tot + 256;             // [Kp]    d G_end
     const int slot = blockIdx.x, h = blockIdx.y;
-    const int len = w.chunk_len[slot];
+    int len, tok0;
+    w.tab.span(slot, tok0, len);
     if (len == 0) return;
-    const int tok0 = w.chunk_tok0[slot], K = w.K, Kp = ONE ? 64 : w.Kp, V = w.V, Vp = ONE ? 64 : w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
+    const int K = w.K, Kp = ONE ? 64 : w.Kp, V = w.V, Vp = ONE ? 64 : w.Vp, H = w.H, KT = Kp / 64, VT = Vp / 64;
     const size_t ch = (size_t)slot * H + h;
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, d = tid & 63, I = tid >> 6;
     const float* kn_g = w.kn + ch * 64 * Kp;
@@ -1381,6 +1388,12 @@ static int launch_scan(const Ws& w, int n_seq, const simt::ScanArgs& a, const ch
     return launch_status();
 }
 
+static int chunk_table(const KdaChunkShape* sh, const Ws& w, const int32_t* cu, cudaStream_t st) {
+    if (w.tab.per_seq > 0) return KDA_OK;
+    KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->tokens, w.status, status_mirror()));
+    return launch_status();
+}
+
 int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const void* v, const void* g, const void* beta,
                    const float* h0, const int32_t* cu, void* o, float* final_state, void* workspace, cudaStream_t st,
                    const tc::NormEpilogue* norm, const tc::ConvPrep* conv) {
@@ -1395,7 +1408,7 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         simt::carve_ws(*sh, nullptr, &ws_bytes);
         tc::TcWs t = tc::carve_tc(*sh, static_cast<char*>(workspace) + ws_bytes);
         t.status = w.status;      // one status word per workspace, shared by both lanes
-        KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status, status_mirror()));
+        if (int rc = chunk_table(sh, w, cu, st)) return rc;
         if (w.nslots > 0) {
             int rc = tc_intra_forward(w, t, q, k, v, g, beta, gbf16, sh->l2norm, sh->scale, sh->tokens, conv, st);
             if (rc) return rc;
@@ -1405,10 +1418,10 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         }
         return launch_status();
     }
-    KDA_LAUNCH("chunk_table_kernel", st, simt::chunk_table_kernel<<<1, 256, 0, st>>>(w, cu, sh->n_seq, sh->seq_len, sh->tokens, w.status, status_mirror()));
+    if (int rc = chunk_table(sh, w, cu, st)) return rc;
     const dim3 gch(w.nslots, w.H);
     if (w.nslots > 0) {
-        const simt::IntraArgs a{q, k, v, g, beta, bf16, gbf16, sh->l2norm, vec4(v, sh->value_dim), sh->forward_only ? 0 : 1, sh->scale};
+        const simt::IntraArgs a{q, k, v, g, beta, bf16, gbf16, sh->l2norm, vec4(v, sh->value_dim), sh->forward_only ? 0 : 1, sh->scale, status_mirror(), w.tab.per_seq > 0};
         if (set_smem(simt::intra_fwd_kernel, simt::kIntraSmem)) return KDA_ERR_CUDA;
         KDA_LAUNCH("intra_fwd_kernel", st, simt::intra_fwd_kernel<<<gch, 256, simt::kIntraSmem, st>>>(w, a));
     }

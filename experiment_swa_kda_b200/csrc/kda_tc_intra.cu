@@ -216,8 +216,7 @@ __device__ __forceinline__ void unit_lower_inverse(float* Ms, float* tmp) {
 }  // namespace
 
 struct IntraFwdArgs {
-    const int* chunk_tok0;
-    const int* chunk_len;
+    simt::ChunkTable tab;
     const __nv_bfloat16 *q, *k;       // [tokens][H][128]
     const void* g;                    // [tokens][H][128], gate dtype
     const void* beta;                 // [tokens][H]
@@ -225,6 +224,8 @@ struct IntraFwdArgs {
     float scale;
     TcWs t;
     simt::Ws w;                       // per-row scalars (inverse norms, beta) kept for the backward
+    int* mirror;
+    int clear_status;                 // no table kernel ran before this one
     const __nv_bfloat16* xv;          // CONV only: the v convolution's input (q, k above are the q, k convolutions' inputs)
     ConvPrep conv;
 };
@@ -314,7 +315,9 @@ __global__ void __launch_bounds__(kNT, 2)
 
     // heads fastest: blocks that run side by side read neighbouring pieces of the same token rows
     const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;
-    const int len = p.chunk_len[slot], tok0 = p.chunk_tok0[slot];
+    if (p.clear_status && blockIdx.x == 0 && threadIdx.x == 0) simt::start_status(p.t.status, p.mirror);
+    int len, tok0;
+    p.tab.span(slot, tok0, len);
     if (len == 0) return;
     const size_t ch = blockIdx.x;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -341,7 +344,7 @@ __global__ void __launch_bounds__(kNT, 2)
     // are the zero padding at a sequence start
     const size_t wbase = ((size_t)h * 128 + 8 * cg) * 4;
     auto conv_rows = [&](const __nv_bfloat16* x, uint4 (&xr)[7]) {
-        const bool first = p.w.seq_chunk0[p.w.chunk_seq[slot]] == slot;
+        const bool first = p.tab.starts_sequence(slot);
 #pragma unroll
         for (int jj = 0; jj < 7; ++jj) {
             const int i = 4 * rq - 3 + jj;
@@ -563,7 +566,8 @@ __global__ void __launch_bounds__(kNT, 2)
         const unsigned nxt = blockIdx.x + 296u;
         if (nxt < gridDim.x) {
             const int ns = (int)(nxt / H), nh = (int)(nxt % H);
-            const int nlen = p.chunk_len[ns], nt0 = p.chunk_tok0[ns];
+            int nlen, nt0;
+            p.tab.span(ns, nt0, nlen);
             if (!CONV && nlen > 0 && lane < 2) tma_prefetch_2d(&mv, nh * 128 + lane * 64, nt0);
             for (int i = lane; i < nlen; i += 32) {
                 const size_t o = ((size_t)(nt0 + i) * H + nh) * 128;
@@ -822,7 +826,7 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
                      const void* beta, int gbf16, int l2norm, float scale, int tokens, const tc::ConvPrep* conv, cudaStream_t st) {
     using namespace tc;
     IntraFwdArgs a;
-    a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len;
+    a.tab = w.tab; a.mirror = status_mirror(); a.clear_status = w.tab.per_seq > 0;
     a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
     a.g = g; a.beta = beta; a.gbf16 = gbf16; a.l2norm = l2norm; a.H = w.H; a.scale = scale; a.t = t; a.w = w;
     a.xv = static_cast<const __nv_bfloat16*>(v);

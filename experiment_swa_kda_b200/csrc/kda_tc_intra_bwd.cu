@@ -105,8 +105,7 @@ __device__ __forceinline__ float quad_after(float p, int c4) {
 }  // namespace
 
 struct IntraBwdArgs {
-    const int* chunk_tok0;
-    const int* chunk_len;
+    simt::ChunkTable tab;
     const __nv_bfloat16 *q, *k, *v;   // caller tensors [tokens][H][128]
     const void* g;                    // gate dtype
     const float *qinv, *kinv, *beta;  // [nch][64] from the forward
@@ -188,11 +187,10 @@ __global__ void __launch_bounds__(512, 1)
     const int H = p.H, total = p.nslots * H;
     int work = blockIdx.x, len = 0, tok0 = 0;       // chunk-heads blockIdx.x, + gridDim.x, ...; heads slowest; empty slots are skipped
     for (; work < total; work += gridDim.x) {
-        len = p.chunk_len[work % p.nslots];
+        p.tab.span(work % p.nslots, tok0, len);
         if (len > 0) break;
     }
     if (work >= total) return;
-    tok0 = p.chunk_tok0[work % p.nslots];
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int I = warp >> 2, wq = warp & 3;       // row block and channel quarter of this warp
     const int c4 = lane & 3, r8 = lane >> 2;      // token pair and channel inside an 8 x 8 piece
@@ -613,10 +611,7 @@ __global__ void __launch_bounds__(512, 1)
     const uint32_t da_off = kR7 + wq * 4096 + sw128_off(8 * (mi >> 1) + mr, 2 * I + (mi & 1));
     // the next chunk-head of this CTA: one warp looks it up
     int nwork = work + gridDim.x, nlen = 0, ntok0 = 0;
-    if (warp == 15 && nwork < total) {
-        nlen = p.chunk_len[nwork % p.nslots];
-        ntok0 = p.chunk_tok0[nwork % p.nslots];
-    }
+    if (warp == 15 && nwork < total) p.tab.span(nwork % p.nslots, ntok0, nlen);
     {
         // in flight: the decay panels.  Both operand families are stored transposed, [channel d][row] (K-major A operands).
         const uint32_t X = sb + kR3 + (I >> 1) * 16384;      // two target blocks share a panel: 32 stack rows each
@@ -668,10 +663,7 @@ __global__ void __launch_bounds__(512, 1)
     if (warp == 15) {
         while (nwork < total && nlen == 0) {
             nwork += gridDim.x;
-            if (nwork < total) {
-                nlen = p.chunk_len[nwork % p.nslots];
-                ntok0 = p.chunk_tok0[nwork % p.nslots];
-            }
+            if (nwork < total) p.tab.span(nwork % p.nslots, ntok0, nlen);
         }
         if (lane == 0) {
             next[0] = nwork;
@@ -1060,7 +1052,7 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     else mg = mdg = mq;      // float32 gates and their gradients go through the threads
     if (rc) return KDA_ERR_CUDA;
     IntraBwdArgs a;
-    a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len;
+    a.tab = w.tab;
     a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
     a.v = static_cast<const __nv_bfloat16*>(v); a.g = g;
     a.qinv = w.qinv; a.kinv = w.kinv; a.beta = w.beta; a.Mt = t.Mt;

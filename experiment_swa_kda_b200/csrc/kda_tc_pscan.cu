@@ -39,10 +39,8 @@ int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
 // panel c has a whole step to read it before it is written again.
 // ---------------------------------------------------------------------------------------------
 struct AffineScanArgs {
-    const int* seq_chunk0;
-    const int* seq_order;     // unsplit scans: grid = (heads, sequences), block (h, r) walks sequence seq_order[r]
-    const int* chunk_tok0;
-    const int* chunk_len;
+    simt::ChunkTable tab;
+    int heads_first;          // unsplit scans of several sequences: grid = (heads, sequences); 2: block (h, r) walks sequence tab.seq_order[r]
     const float* decay_end;   // [nch][128] exp(G_end)
     const float* s_in;        // V-first initial state (forward: h0, backward: cotangent of the final state), or null
     float* s_out;             // V-first final state of the scan (forward: final state, backward: dh0), or null
@@ -90,12 +88,12 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
     const int v = (warp & 3) * 32 + lane;          // value row = TMEM lane
     const bool split = p.nseg > 1;
     const int units = 2 * p.nseg - 1;
-    // split: grid (sequences x units, heads); unsplit with an order table: grid (heads, sequences), longest first, so that
-    // the blocks the hardware starts first are the longest chains
-    const bool lpt = !split && p.seq_order != nullptr;
-    const int seq = split ? blockIdx.x / units : (lpt ? p.seq_order[blockIdx.y] : blockIdx.x), role = split ? blockIdx.x % units : 0;
-    const int h = lpt ? blockIdx.x : blockIdx.y, H = p.H;
-    const int c_begin = p.seq_chunk0[seq], c_end = p.seq_chunk0[seq + 1];
+    // split: grid (sequences x units, heads); unsplit: grid (heads, sequences), a packed batch longest first, so that the blocks
+    // the hardware starts first are the longest chains
+    const bool heads_first = !split && p.heads_first;
+    const int seq = split ? blockIdx.x / units : (heads_first ? (p.heads_first == 2 ? p.tab.seq_order[blockIdx.y] : blockIdx.y) : blockIdx.x), role = split ? blockIdx.x % units : 0;
+    const int h = heads_first ? blockIdx.x : blockIdx.y, H = p.H;
+    const int c_begin = p.tab.first_chunk(seq), c_end = p.tab.first_chunk(seq + 1);
     const int n_total = c_end - c_begin;
     const int seg = (role + 1) >> 1;                             // segment this unit walks
     const int step0 = seg_begin(seg, p.nseg, n_total);           // its first step, in the sequence's scan order
@@ -138,7 +136,8 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                 if (!kBwd) {
                     for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + 49152 + nb * 8192, &mY, &bar_full[st], nb * 64, ch * 64);
                 } else {
-                    const int tok0 = p.chunk_tok0[slot];
+                    int tok0, len;
+                    p.tab.span(slot, tok0, len);
                     for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + 49152 + nb * 8192, &mY, &bar_full[st], h * 128 + nb * 64, tok0);
                 }
             };
@@ -158,7 +157,8 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
         if (kBwd && n > 0 && !composite && step0 == 0) {
             // Only a sequence's last chunk (the adjoint scan's first step) can be ragged; the dO rows past its tail
             // belong to the next sequence and are blanked by the whole warp before lane 0 issues the product on them.
-            const int len0 = p.chunk_len[slot_of(0)];
+            int tok0, len0;
+            p.tab.span(slot_of(0), tok0, len0);
             if (len0 < 64) {
                 if (mbar_wait(&bar_full[0], 0, p.status, 51)) {
                     for (int idx = lane; idx < (64 - len0) * 16; idx += 32) {
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
 // split scans, second pass: from the units' local states to the true states (see tc_scan_fixup_kernel)
 // ---------------------------------------------------------------------------------------------
 struct ScanFixArgs {
-    const int* seq_chunk0;
+    simt::ChunkTable tab;
     const float* seg_fin;      // [rec*units][128][128]
     float* s_out;              // final state of the scan, V-first [n_seq][H][128][128], or null
     int H, nseg, bwd, parts;
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(256, 1)
     __shared__ uint32_t tmem_slot;
     const int units = 2 * p.nseg - 1, rec = blockIdx.y, seq = rec / p.H, h = rec - seq * p.H;
     const int k = 1 + (int)blockIdx.x / p.parts, part = (int)blockIdx.x % p.parts;
-    const int c_begin = p.seq_chunk0[seq], c_end = p.seq_chunk0[seq + 1], n_total = c_end - c_begin;
+    const int c_begin = p.tab.first_chunk(seq), c_end = p.tab.first_chunk(seq + 1), n_total = c_end - c_begin;
     const int s0 = seg_begin(k, p.nseg, n_total), sn = seg_begin(k + 1, p.nseg, n_total) - s0;
     const int b0 = s0 + (int)((long long)part * sn / p.parts), nc = s0 + (int)((long long)(part + 1) * sn / p.parts) - b0;
     // an empty sequence's final state is its initial state, which the chain reproduces (identity composites, zero local states)
@@ -584,8 +584,7 @@ __global__ void __launch_bounds__(256, 1)
 // 256 threads: thread (g, v) handles value row v, tokens 32g .. 32g+31.
 // ---------------------------------------------------------------------------------------------
 struct ChunkOutArgs {
-    const int* chunk_tok0;
-    const int* chunk_len;
+    simt::ChunkTable tab;
     __nv_bfloat16* ZT;
     __nv_bfloat16* o;          // [tokens][H][128]; nullptr with the norm's epilogue when only y is wanted
     int H;
@@ -611,9 +610,9 @@ __global__ void __launch_bounds__(256, 2)
     __shared__ uint64_t bar_in, bar_mma1, bar_mma2;
     __shared__ uint32_t tmem_slot;
     const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;      // heads fastest, as in the intra-chunk kernels
-    const int len = p.chunk_len[slot];
+    int len, tok0;
+    p.tab.span(slot, tok0, len);
     if (len == 0) return;
-    const int tok0 = p.chunk_tok0[slot];
     const int ch = slot * H + h;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
@@ -762,8 +761,7 @@ __global__ void __launch_bounds__(256, 2)
 //     dZ^T = dO^T A + dH'^T E^T          M=128, N=64: K=64 (MN-major A) then K=128
 // ---------------------------------------------------------------------------------------------
 struct ChunkDzArgs {
-    const int* chunk_tok0;
-    const int* chunk_len;
+    simt::ChunkTable tab;
     __nv_bfloat16* dZT;
     int H;
     int* status;
@@ -781,9 +779,9 @@ __global__ void __launch_bounds__(256, 3)
     __shared__ uint64_t bar_in, bar_mma;
     __shared__ uint32_t tmem_slot;
     const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;      // heads fastest, as in the intra-chunk kernels
-    const int len = p.chunk_len[slot];
+    int len, tok0;
+    p.tab.span(slot, tok0, len);
     if (len == 0) return;
-    const int tok0 = p.chunk_tok0[slot];
     const int ch = slot * H + h;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
@@ -880,7 +878,7 @@ static int scan_fixup(const simt::Ws& w, const tc::TcWs& t, int n_seq, __nv_bflo
     const int rec = n_seq * w.H, per_seg = (w.nslots / n_seq + t.nseg - 1) / t.nseg;
     const int parts = std::max(1, std::min(148 / (rec * (t.nseg - 1)), per_seg));
     ScanFixArgs f;
-    f.seq_chunk0 = w.seq_chunk0; f.seg_fin = t.seg_fin; f.s_out = s_out; f.H = w.H; f.nseg = t.nseg; f.bwd = bwd; f.parts = parts;
+    f.tab = w.tab; f.seg_fin = t.seg_fin; f.s_out = s_out; f.H = w.H; f.nseg = t.nseg; f.bwd = bwd; f.parts = parts;
     f.status = t.status;
     CUtensorMap mHp;
     if (make_map_bf16(&mHp, panels, (uint64_t)w.nslots * w.H * 128, 128, 64, 128)) return KDA_ERR_CUDA;
@@ -911,12 +909,11 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
         set_smem_limit(tc_chunk_out_kernel, kChunkOutNormSmem))
         return KDA_ERR_CUDA;
     AffineScanArgs a;
-    a.seq_chunk0 = w.seq_chunk0; a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len; a.decay_end = t.decay_end; a.s_in = h0; a.s_out = final_state;
+    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = h0; a.s_out = final_state;
     a.H = w.H; a.status = t.status; a.nseg = t.nseg; a.seg_fin = t.seg_fin;
     const int units = 2 * t.nseg - 1;
-    const bool lpt = t.nseg == 1 && n_seq > 1 && n_seq <= 65535;
-    a.seq_order = lpt ? w.seq_order : nullptr;
-    const dim3 scan_grid = lpt ? dim3(w.H, n_seq) : dim3(n_seq * units, w.H);
+    a.heads_first = t.nseg == 1 && n_seq > 1 && n_seq <= 65535 ? (w.tab.per_seq > 0 ? 1 : 2) : 0;      // equal lengths need no order
+    const dim3 scan_grid = a.heads_first ? dim3(w.H, n_seq) : dim3(n_seq * units, w.H);
     CUtensorMap mPp = mH, mF = mH;
     if (t.nseg > 1) {
         if (make_map_bf16(&mPp, t.Pp, nch * 128, 128, 64, 128) ||
@@ -930,7 +927,7 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
         if (int e = scan_fixup(w, t, n_seq, t.Hp, final_state, 0, mPp, mF, st)) return e;
     }
     ChunkOutArgs oa;
-    oa.chunk_tok0 = w.chunk_tok0; oa.chunk_len = w.chunk_len; oa.ZT = t.fwd_only ? nullptr : t.ZT; oa.o = static_cast<__nv_bfloat16*>(o); oa.H = w.H;
+    oa.tab = w.tab; oa.ZT = t.fwd_only ? nullptr : t.ZT; oa.o = static_cast<__nv_bfloat16*>(o); oa.H = w.H;
     oa.status = t.status;
     oa.norm = norm;
     KDA_LAUNCH("tc_chunk_out_kernel", st,
@@ -957,12 +954,11 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
         set_smem_limit(tc_chunk_dz_kernel, kChunkDzSmem))
         return KDA_ERR_CUDA;
     AffineScanArgs a;
-    a.seq_chunk0 = w.seq_chunk0; a.chunk_tok0 = w.chunk_tok0; a.chunk_len = w.chunk_len; a.decay_end = t.decay_end; a.s_in = d_final; a.s_out = dh0;
+    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = d_final; a.s_out = dh0;
     a.H = w.H; a.status = t.status; a.nseg = t.nseg; a.seg_fin = t.seg_fin;
     const int units = 2 * t.nseg - 1;
-    const bool lpt = t.nseg == 1 && n_seq > 1 && n_seq <= 65535;
-    a.seq_order = lpt ? w.seq_order : nullptr;
-    const dim3 scan_grid = lpt ? dim3(w.H, n_seq) : dim3(n_seq * units, w.H);
+    a.heads_first = t.nseg == 1 && n_seq > 1 && n_seq <= 65535 ? (w.tab.per_seq > 0 ? 1 : 2) : 0;      // equal lengths need no order
+    const dim3 scan_grid = a.heads_first ? dim3(w.H, n_seq) : dim3(n_seq * units, w.H);
     CUtensorMap mPp = mdH, mF = mdH;
     if (t.nseg > 1) {
         if (make_map_bf16(&mPp, t.Pp, nch * 128, 128, 64, 128) ||
@@ -976,7 +972,7 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
         if (int e = scan_fixup(w, t, n_seq, t.dHp, dh0, 1, mPp, mF, st)) return e;
     }
     ChunkDzArgs da;
-    da.chunk_tok0 = w.chunk_tok0; da.chunk_len = w.chunk_len; da.dZT = t.dZT; da.H = w.H; da.status = t.status;
+    da.tab = w.tab; da.dZT = t.dZT; da.H = w.H; da.status = t.status;
     KDA_LAUNCH("tc_chunk_dz_kernel", st,
                tc_chunk_dz_kernel<<<(unsigned)nch, 256, kChunkDzSmem, st>>>(mdH, mE, mdO, mAT, mdZT, da));
     return launch_status();
