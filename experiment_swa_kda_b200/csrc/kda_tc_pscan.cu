@@ -31,12 +31,17 @@ int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
 //     backward   S = dH'^T [v][k]:   S' = dec . S - S Pn^T + dO^T Rm         stores S (adjoint of the chunk's outgoing state)
 // Threads are specialised by warp; they meet only through mbarriers:
 //   state warpgroups (kScanGroups of them): thread (g, v) owns S[v][g*kScanCols .. (g+1)*kScanCols) in registers
-//   next warp   one lane issues the TMA loads, two chunks ahead
-//   last warp   one lane issues every UMMA and the TMA stores of the state panels
+//   next warp   one lane issues the TMA loads, as far ahead as the ring reaches
+//   next warp   one lane issues every UMMA
+//   last warp   one lane issues the TMA stores of the state panels
+// The loads of a step are two 32 KB items of one ring, the state-independent operands and then Pn, each handed back when
+// its own product is complete: five slots reach two steps ahead.  With two whole steps in the ring a load
+// could start only when the step before the last had ended, and 1,700 of a step's 2,600 cycles went by waiting for it
+// (16 recurrences in 4 segments of 32 steps: 60 -> 51 us; 6 of 16: 27 -> 24.5).
 // TMEM: the accumulator is double-buffered (columns 0 / 128) so that the state-independent product of step c+1 is
 // issued while the state threads still read the accumulator of step c; the bf16 state panel the state product reads as
-// its A operand sits at column 256.  Its shared-memory copy (for the TMA store) is double-buffered, so the store of
-// panel c has a whole step to read it before it is written again.
+// its A operand sits at column 256.  Its copy in shared memory, for the TMA store, is written behind the arrival that releases
+// the product and has the rest of the step to leave.
 // ---------------------------------------------------------------------------------------------
 struct AffineScanArgs {
     simt::ChunkTable tab;
@@ -60,29 +65,38 @@ struct AffineScanArgs {
 // first scan step of segment k of a sequence of n steps
 __host__ __device__ __forceinline__ int seg_begin(int k, int nseg, int n) { return (int)(((long long)k * n) / nseg); }
 
-constexpr int kPStage = 65536;                              // Pn 32 KB | X 16 KB (U^T or Rm^T) | Y 16 KB (E or dO)
-constexpr int kPStageBytes = kPStage + 512;                 // + exp(G_end), which lands in a ring of its own
-constexpr int kAffineScanSmem = 2 * kPStage + 2 * 32768 + 1024;
+constexpr int kScanItem = 32768;                            // Pn, or X 16 KB (U^T or Rm^T) | Y 16 KB (E or dO)
+constexpr int kScanSlots = 5;
+constexpr int kScanMapSlots = 3;                            // composites load Pn only; more would outrun the ring of decays
+constexpr int kScanPanel = kScanSlots * kScanItem;          // 2 x 32 KB  bf16 state panel of step c in c % 2, [2 k-blocks][128 rows x 128 B]
+constexpr int kScanDec = kScanPanel + 65536;                // exp(G_end) of step c in slot c % 4: [4][128] floats
+constexpr int kScanBars = kScanDec + 2048;
+constexpr int kAffineScanSmem = kScanBars + 256;            // 1 KB less than the limit: the base has to be 1024-aligned as it is
 constexpr int kScanGroups = 2;                              // state warpgroups: each thread owns 128 / kScanGroups columns of a row
 constexpr int kScanCols = 128 / kScanGroups;
 constexpr uint32_t kScanPanelCol = 256;                     // TMEM column of the bf16 state panel (64 columns: 128 keys as pairs)
-constexpr int kAffineScanThreads = (4 * kScanGroups + 2) * 32;
+constexpr int kAffineScanThreads = (4 * kScanGroups + 3) * 32;
 
 template <bool kBwd>
 __global__ void __launch_bounds__(kAffineScanThreads, 1)
     tc_affine_scan_kernel(const __grid_constant__ CUtensorMap mP, const __grid_constant__ CUtensorMap mX,
                           const __grid_constant__ CUtensorMap mY, const __grid_constant__ CUtensorMap mS,
                           const __grid_constant__ CUtensorMap mS2, const __grid_constant__ CUtensorMap mF, AffineScanArgs p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
-    uint8_t* Sop = sm + 2 * kPStage;               // 2 x [2 k-blocks][128 rows x 128 B]: bf16 state panel of step c in c % 2
-    __shared__ __align__(16) float dec_ring[4][128];   // exp(G_end) of step c in slot c % 4
-    // full: a stage has landed.  free: every product that reads a stage is complete (one per stage, so that the load
-    // thread can never miss a phase).  sop: all state threads have packed the state panel.  mma: the step's
-    // accumulator is complete.
-    __shared__ uint64_t bar_full[2], bar_free[2], bar_sop, bar_pan, bar_mma;
-    __shared__ uint32_t tmem_slot;
-    __shared__ volatile int abort_flag;
+    extern __shared__ __align__(1024) uint8_t sm[];
+    uint8_t* Sop = sm + kScanPanel;
+    float (*dec_ring)[128] = reinterpret_cast<float (*)[128]>(sm + kScanDec);
+    // full: an item has landed.  free: the product that reads it is complete.  sop: all state threads have packed the state panel
+    // into tensor memory, pan: into shared memory.  out: the store has read that panel (one per buffer).  mma: the step's accumulator is complete.
+    uint64_t* bar_full = reinterpret_cast<uint64_t*>(sm + kScanBars);
+    uint64_t* bar_free = bar_full + kScanSlots;
+    uint64_t &bar_sop = bar_free[kScanSlots], &bar_pan = bar_free[kScanSlots + 1], &bar_mma = bar_free[kScanSlots + 2];
+    uint64_t* bar_out = bar_free + kScanSlots + 3;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bar_free + kScanSlots + 5);
+    volatile int& abort_flag = *reinterpret_cast<volatile int*>(bar_free + kScanSlots + 6);
+    if (smem_u32(sm) & 1023u) {      // the swizzled tiles would be misread
+        if (threadIdx.x == 0) raise_status(p.status, 56);
+        return;
+    }
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int v = (warp & 3) * 32 + lane;          // value row = TMEM lane
@@ -103,12 +117,14 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
     auto slot_of = [&](int c) { return kBwd ? c_end - 1 - (step0 + c) : c_begin + step0 + c; };   // chunk slot of step c
 
     if (warp == 0 && elect_one()) {
-        mbar_init(&bar_full[0], 1);
-        mbar_init(&bar_full[1], 1);
-        mbar_init(&bar_free[0], 1);
-        mbar_init(&bar_free[1], 1);
+        for (int i = 0; i < kScanSlots; ++i) {
+            mbar_init(&bar_full[i], 1);
+            mbar_init(&bar_free[i], 1);
+        }
         mbar_init(&bar_sop, 4 * kScanGroups);      // one arrival per state warp
         mbar_init(&bar_pan, 4 * kScanGroups);
+        mbar_init(&bar_out[0], 1);
+        mbar_init(&bar_out[1], 1);
         mbar_init(&bar_mma, 1);
         mbar_fence_init();
         abort_flag = 0;
@@ -119,41 +135,47 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    // item 2c of the ring is X | Y of step c, item 2c + 1 its Pn; a composite's Pn is item c of a shorter ring
+    auto slot_xy = [&](int c) { return (2 * c) % kScanSlots; };
+    auto parity_xy = [&](int c) { return (uint32_t)(2 * c / kScanSlots) & 1u; };
+    auto slot_p = [&](int c) { return composite ? c % kScanMapSlots : (2 * c + 1) % kScanSlots; };
+    auto parity_p = [&](int c) { return (uint32_t)(composite ? c / kScanMapSlots : (2 * c + 1) / kScanSlots) & 1u; };
 
     if (warp == 4 * kScanGroups) {
         // ------------------------------------------------------------------ load warp
         if (elect_one()) {
-            auto issue_loads = [&](int c) {
-                const int st = c & 1;
-                const int slot = slot_of(c);
-                const int ch = slot * H + h;
-                uint8_t* b = sm + st * kPStage;
-                mbar_expect_tx(&bar_full[st], composite ? 32768 + 512 : kPStageBytes);
-                bulk_load_1d(dec_ring[c & 3], p.decay_end + (size_t)ch * 128, 512, &bar_full[st]);
-                for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + nb * 16384, &mP, &bar_full[st], nb * 64, ch * 128);
-                if (composite) return;
-                tma_load_2d(b + 32768, &mX, &bar_full[st], 0, ch * 128);                  // U^T / Rm^T: [128][64]
-                if (!kBwd) {
-                    for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + 49152 + nb * 8192, &mY, &bar_full[st], nb * 64, ch * 64);
+            const int depth = composite ? kScanMapSlots : kScanSlots, items = composite ? n : 2 * n;
+            auto slot_item = [&](int i) { return i % depth; };
+            auto parity_item = [&](int i) { return (uint32_t)(i / depth) & 1u; };
+            auto issue_load = [&](int i) {
+                const int c = composite ? i : i >> 1, cs = slot_of(c), ch = cs * H + h, sl = slot_item(i);
+                uint8_t* b = sm + sl * kScanItem;
+                uint64_t* bar = &bar_full[sl];
+                if (composite || (i & 1)) {
+                    mbar_expect_tx(bar, 32768 + 512);
+                    bulk_load_1d(dec_ring[c & 3], p.decay_end + (size_t)ch * 128, 512, bar);
+                    for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + nb * 16384, &mP, bar, nb * 64, ch * 128);
                 } else {
-                    int tok0, len;
-                    p.tab.span(slot, tok0, len);
-                    for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + 49152 + nb * 8192, &mY, &bar_full[st], h * 128 + nb * 64, tok0);
+                    mbar_expect_tx(bar, 32768);
+                    tma_load_2d(b, &mX, bar, 0, ch * 128);                  // U^T / Rm^T: [128][64]
+                    int tok0 = 0, len;
+                    if (kBwd) p.tab.span(cs, tok0, len);
+                    for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + 16384 + nb * 8192, &mY, bar, kBwd ? h * 128 + nb * 64 : nb * 64, kBwd ? tok0 : ch * 64);
                 }
             };
             int issued = 0;
-            for (; issued < 2 && issued < n; ++issued) issue_loads(issued);
+            for (; issued < depth && issued < items; ++issued) issue_load(issued);
             bool ok = true;
-            for (int c = 0; c + 2 < n && ok; ++c) {     // stage c % 2 is free once every product of step c is complete
-                ok = mbar_wait(&bar_free[c & 1], (c >> 1) & 1, p.status, 50);
-                if (ok) { issue_loads(c + 2); issued = c + 3; }
+            while (issued < items && ok) {     // a slot is free once the product that reads its item is complete
+                ok = mbar_wait(&bar_free[slot_item(issued)], parity_item(issued) ^ 1u, p.status, 50);
+                if (ok) issue_load(issued++);
                 else abort_flag = 1;
             }
             if (!ok)   // unwinding: the copies in flight must land before the block may exit
-                for (int c = issued > 2 ? issued - 2 : 0; c < issued; ++c) mbar_wait(&bar_full[c & 1], (c >> 1) & 1, nullptr, 0);
+                for (int i = issued > depth ? issued - depth : 0; i < issued; ++i) mbar_wait(&bar_full[slot_item(i)], parity_item(i), nullptr, 0);
         }
     } else if (warp == 4 * kScanGroups + 1) {
-        // ------------------------------------------------------------------ UMMA / panel-store thread
+        // ------------------------------------------------------------------ UMMA thread
         if (kBwd && n > 0 && !composite && step0 == 0) {
             // Only a sequence's last chunk (the adjoint scan's first step) can be ragged; the dO rows past its tail
             // belong to the next sequence and are blanked by the whole warp before lane 0 issues the product on them.
@@ -163,20 +185,12 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                 if (mbar_wait(&bar_full[0], 0, p.status, 51)) {
                     for (int idx = lane; idx < (64 - len0) * 16; idx += 32) {
                         const int r = len0 + (idx >> 4), c = idx & 15;
-                        *reinterpret_cast<uint4*>(sm + 49152 + (c >> 3) * 8192 + sw128_off(r, c & 7)) = make_uint4(0, 0, 0, 0);
+                        *reinterpret_cast<uint4*>(sm + 16384 + (c >> 3) * 8192 + sw128_off(r, c & 7)) = make_uint4(0, 0, 0, 0);
                     }
                     fence_async_smem();
                 }
                 __syncwarp();
             }
-        }
-        if (n == 0 && split && elect_one()) {
-            if (mbar_wait(&bar_pan, 0, p.status, 55)) {
-                tma_store_2d(&mF, Sop, 0, unit * 128);
-                tma_store_2d(&mF, Sop + 16384, 64, unit * 128);
-                tma_store_commit();
-            }
-            tma_store_wait_all();
         }
         if (n > 0 && elect_one()) {
             // state-independent product:  forward U^T E (A K-major, B MN-major), backward dO^T Rm (A MN-major, B K-major)
@@ -185,28 +199,34 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
             //                          backward -S Pn^T (B K-major: rows of Pn are the output index)
             const uint32_t id_st = umma_idesc_bf16(128, 128, kMajorK, kBwd ? kMajorK : kMajorMN, 1);
             auto issue_independent = [&](int c) {
-                const uint32_t s0 = smem_u32(sm + (c & 1) * kPStage);
+                const uint32_t s0 = smem_u32(sm + slot_xy(c) * kScanItem);
                 const uint32_t d = tmem + 128 * (c & 1);
 #pragma unroll
                 for (int k16 = 0; k16 < 4; ++k16) {
                     if (!kBwd)
-                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 32768, 16, 1024) + (k16 * 32),
-                                     umma_smem_desc_sw128(s0 + 49152, 8192, 1024) + (k16 * 2048), id_ind, k16 > 0);
+                        umma_bf16_ss(d, umma_smem_desc_sw128(s0, 16, 1024) + (k16 * 32),
+                                     umma_smem_desc_sw128(s0 + 16384, 8192, 1024) + (k16 * 2048), id_ind, k16 > 0);
                     else
-                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 49152, 8192, 1024) + (k16 * 2048),
-                                     umma_smem_desc_sw128(s0 + 32768, 16, 1024) + (k16 * 32), id_ind, k16 > 0);
+                        umma_bf16_ss(d, umma_smem_desc_sw128(s0 + 16384, 8192, 1024) + (k16 * 2048),
+                                     umma_smem_desc_sw128(s0, 16, 1024) + (k16 * 32), id_ind, k16 > 0);
                 }
+                umma_commit(&bar_free[slot_xy(c)]);
             };
-            const CUtensorMap* mstore = composite ? &mS2 : &mS;      // composites go to their own panel array
-            bool ok = mbar_wait(&bar_full[0], 0, p.status, 51);
-            if (ok) {
+            auto ready = [&](int sl, uint32_t parity) {
+                if (mbar_wait(&bar_full[sl], parity, p.status, 51)) return true;
+                abort_flag = 1;
+                return false;
+            };
+            const bool ok = composite || ready(slot_xy(0), 0u);
+            if (ok && !composite) {
                 tc_fence_after();
-                if (!composite) issue_independent(0);
-            } else abort_flag = 1;
+                issue_independent(0);
+            }
             for (int c = 0; c < n && ok; ++c) {
                 const int st = c & 1;
-                const int ch = slot_of(c) * H + h;
-                const uint32_t s0 = smem_u32(sm + st * kPStage);
+                const int sl = slot_p(c);
+                const uint32_t s0 = smem_u32(sm + sl * kScanItem);
+                if (!ready(sl, parity_p(c))) break;
                 if (!mbar_wait(&bar_sop, c & 1, p.status, 52)) { abort_flag = 1; break; }
                 tc_fence_after();
 #pragma unroll
@@ -215,30 +235,28 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                                              : umma_smem_desc_sw128(s0, 16384, 1024) + (k16 * 2048);
                     umma_bf16_ts(tmem + 128 * st, tmem + kScanPanelCol + 8 * k16, bd, id_st, (composite && k16 == 0) ? 0u : 1u);
                 }
-                // The store of panel c-1 has read its buffer before this commit lets the state threads write panel c+1
-                // into it.
-                tma_store_wait_read();
                 umma_commit(&bar_mma);
-                umma_commit(&bar_free[st]);
-                // the copy of the panel in shared memory (written after the tensor-memory one, off the critical path)
-                if (!mbar_wait(&bar_pan, c & 1, p.status, 55)) { abort_flag = 1; break; }
-                tma_store_2d(mstore, Sop + st * 32768, 0, ch * 128);
-                tma_store_2d(mstore, Sop + st * 32768 + 16384, 64, ch * 128);
-                tma_store_commit();
-                if (c + 1 < n) {
+                umma_commit(&bar_free[sl]);
+                if (c + 1 < n && !composite) {
                     // accumulator (c+1) % 2 was last read by the state threads in step c-1, before they packed panel c
-                    if (!mbar_wait(&bar_full[(c + 1) & 1], ((c + 1) >> 1) & 1, p.status, 51)) { abort_flag = 1; break; }
+                    if (!ready(slot_xy(c + 1), parity_xy(c + 1))) break;
                     tc_fence_after();
-                    if (!composite) issue_independent(c + 1);
+                    issue_independent(c + 1);
                 }
             }
-            if (ok && split && abort_flag == 0) {
-                // the unit's final state as one more bf16 panel (the state threads pack it after their last step)
-                if (mbar_wait(&bar_pan, n & 1, p.status, 55)) {
-                    tma_store_2d(&mF, Sop + (n & 1) * 32768, 0, unit * 128);
-                    tma_store_2d(&mF, Sop + (n & 1) * 32768 + 16384, 64, unit * 128);
-                    tma_store_commit();
-                }
+        }
+    } else if (warp == 4 * kScanGroups + 2) {
+        // ------------------------------------------------------------------ panel-store thread: the chunk-start states, and for a
+        // unit of a split scan its final state as one more panel
+        if (elect_one()) {
+            for (int c = 0; c < n + (split ? 1 : 0); ++c) {
+                if (!mbar_wait(&bar_pan, c & 1, p.status, 55)) { abort_flag = 1; break; }
+                const CUtensorMap* m = c == n ? &mF : (composite ? &mS2 : &mS);      // composites go to their own panel array
+                const int row = c == n ? unit * 128 : (slot_of(c) * H + h) * 128;
+                for (int nb = 0; nb < 2; ++nb) tma_store_2d(m, Sop + (c & 1) * 32768 + nb * 16384, nb * 64, row);
+                tma_store_commit();
+                tma_store_wait_read();
+                mbar_arrive(&bar_out[c & 1]);
             }
             tma_store_wait_all();
         }
@@ -265,12 +283,12 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
         // thread - into the shared-memory panel that the TMA store sends to the chunk-parallel kernels.
         static_assert(kScanCols == 64, "the tensor-memory panel is written with one 32-column store per thread");
         const int kh = col0 / 64;
-        // The stage of step c is observed HERE, before the arrival that lets the UMMA thread run step c: the commit of
-        // step c frees the stage for the loads of step c + 2, so a state warp that looked at the stage barrier only
+        // Pn and the decays of step c are observed HERE, before the arrival that lets the UMMA thread run step c: the commit of
+        // step c frees the slot for a later load, so a state warp that looked at the slot's barrier only
         // after that commit could find it two phases on and read the parity as "not yet complete".
         auto pack_state = [&](int c) -> bool {
             const bool last = c >= n;      // the final state's panel: shared-memory copy only, nothing consumes it on chip
-            if (!last && !mbar_wait(&bar_full[c & 1], (c >> 1) & 1, p.status, 54)) return false;
+            if (!last && !mbar_wait(&bar_full[slot_p(c)], parity_p(c), p.status, 54)) return false;
             uint32_t w[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) w[j] = pack_bf16(s[2 * j], s[2 * j + 1]);
@@ -280,6 +298,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                 tc_fence_before();
                 warp_arrive(&bar_sop, lane);
             }
+            if (c > 1 && !mbar_wait(&bar_out[c & 1], ((c - 2) >> 1) & 1, p.status, 57)) return false;      // the panel before the last has left
             uint8_t* dst = Sop + (c & 1) * 32768 + kh * 16384;
 #pragma unroll
             for (int q = 0; q < 8; ++q)
