@@ -941,16 +941,33 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
     }
 }
 
-// The same for long bf16 inputs without carried windows, C % 128 == 0: a thread walks down a run of tokens, 8 rows at a
+// The same for long bf16 inputs, C % 128 == 0: a thread walks down a run of tokens, 8 rows at a
 // time, and loads the next 8 rows before it computes on the present ones, so that reads stay in flight and the W-1 halo
 // rows are read once per run instead of once per 8 tokens.  65,536 x 2,048: 129 -> 96 us (0.86 of the copy rate); with two
-// blocks per SM instead of three it takes 108.
+// blocks per SM instead of three it takes 108.  A window that is only carried out
+// (a prompt from an empty state) is a copy of the last W rows, by one more block row of the grid (fin_row; -1: none); in the
+// runs themselves it cost every thread registers (49 -> 57 us at 3 x 8,191 x 2,048).
 template <int W>
-__global__ void __launch_bounds__(256, W <= 4 ? 3 : 2) conv_fwd_stream_kernel(int B, int T, int C, int ldx, int run, int silu, int wf32, ConvFwdItems items) {
+__global__ void __launch_bounds__(256, W <= 4 ? 3 : 2) conv_fwd_stream_kernel(int B, int T, int C, int ldx, int run, int fin_row, int silu, int wf32, ConvFwdItems items) {
     constexpr int R = 8;                                       // run is a multiple of 2 R
     const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int c = (blockIdx.x * 32 + p) * 4;                   // C % 128 == 0: in range
     const int item = blockIdx.z / B, b = blockIdx.z - item * B;
+    if ((int)blockIdx.y == fin_row) {                          // slot s holds the input at time T - W + s
+        const int t = T - W + g;
+        __nv_bfloat16* fin = static_cast<__nv_bfloat16*>(pick_item(items.fin, item));
+        if (g < W && fin != nullptr) {
+            uint2 u = make_uint2(0u, 0u);
+            if (t >= 0) u = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(pick_item(items.x, item)) + ((size_t)b * T + t) * ldx + c));
+            const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&u.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&u.y);
+            __nv_bfloat16* o = fin + ((size_t)b * C + c) * W + g;
+            o[0] = lo.x;
+            o[W] = lo.y;
+            o[2 * W] = hi.x;
+            o[3 * W] = hi.y;
+        }
+        return;
+    }
     const int t0 = (blockIdx.y * 8 + g) * run;
     if (t0 >= T) return;
     const void* __restrict__ wgt = pick_item(items.w, item);
@@ -2068,17 +2085,23 @@ inline bool conv_grid_ok(int n, int B, int T) { return ceil_div(T, 8 * pw::kConv
 
 // n same-shaped convolutions in one launch; x rows ldx elements apart
 constexpr int kConvRun = 32;      // tokens per thread of the streaming forward
+constexpr long long kConvStreamBlocks = 148 * 3 / 2;
 template <int W>
 int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st) {
     const bool vec4 = C % 128 == 0 && ldx % 4 == 0;         // channels per thread: 4 when a warp's 128 channels fill a row segment
     const dim3 grid(ceil_div(C, vec4 ? 128 : 64), ceil_div(T, 8 * pw::kConvPairT), B * n);
-    bool win = false;
-    for (int i = 0; i < n; ++i) win = win || it.cache[i] != nullptr || it.fin[i] != nullptr;
-    // enough tokens that 32-token runs still give every SM three blocks several times over: the streaming kernel
-    if (vec4 && bf16 && !win) {
-        const dim3 sgrid(C / 128, ceil_div(T, 8 * kConvRun), B * n);
-        if ((long long)sgrid.x * sgrid.y * sgrid.z >= 148LL * 3 * 4) {
-            KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, silu, wf32, it));
+    bool win = false, carried = false;
+    for (int i = 0; i < n; ++i) {
+        win = win || it.cache[i] != nullptr || it.fin[i] != nullptr;
+        carried = carried || it.cache[i] != nullptr;
+    }
+    // The streaming kernel from one and a half blocks of 32-token runs per SM on (3 x 2 x 4,096 x 384, 288 blocks: 16.4 -> 14.3 us;
+    // 3 x 4,096 x 2,048: 34.8 -> 28.8; 144 blocks: 12.3 and 12.4; 72: 8.3 and 12.3), unless a window is carried in.
+    if (vec4 && bf16 && !carried) {
+        const int runs = ceil_div(T, 8 * kConvRun);
+        const dim3 sgrid(C / 128, runs + (win ? 1 : 0), B * n);
+        if ((long long)sgrid.x * runs * sgrid.z >= kConvStreamBlocks && sgrid.y <= 65535) {
+            KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, win ? runs : -1, silu, wf32, it));
             return launch_status();
         }
     }

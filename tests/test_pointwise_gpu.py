@@ -296,6 +296,29 @@ def test_convolution_weights_at_any_element_offset(B, T, C, W, dtype, wdtype, st
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
+# either side of the line between the kernel of short runs and the streaming one (222 blocks of 256 tokens x 128 channels, three
+# convolutions: 216 and 240 here), a last run of one token, several sequences
+@pytest.mark.parametrize("B,T,C,W", [(1, 2303, 1024, 4), (1, 2305, 1024, 4), (3, 1025, 768, 2), (1, 10241, 256, 3)])
+def test_windows_carried_out_are_the_last_inputs(B, T, C, W):
+    import ctypes
+    from experiment_swa_kda_b200 import _lib
+    lib, n = _lib.load(), 3
+    gen = torch.Generator(device=D0).manual_seed(T)
+    xs = [torch.randn(B, T, C, device=D0, generator=gen).bfloat16() for _ in range(n)]
+    ws = [torch.randn(C, W, device=D0, generator=gen) for _ in range(n)]
+    arr = lambda ts: ctypes.cast((ctypes.c_void_p * n)(*[t.data_ptr() for t in ts]), ctypes.c_void_p)
+    stream, io = torch.cuda.current_stream().cuda_stream, _lib.DTYPE_BF16 | 0x100
+
+    def run(fins):
+        ys = [torch.empty_like(x) for x in xs]
+        _lib.check(lib.kda_conv_fwd_rows(n, B, T, C, W, io, 1, arr(xs), C, arr(ws), None, arr(ys), arr(fins) if fins else None, stream), "forward")
+        return ys
+
+    fins = [torch.full((B, C, W), 9.0, device=D0, dtype=torch.bfloat16) for _ in range(n)]
+    assert all(torch.equal(a, b) for a, b in zip(run(fins), run(None)))
+    assert all(torch.equal(f, x[:, T - W:].transpose(1, 2)) for f, x in zip(fins, xs))
+
+
 # Three convolutions on slices of one wide matrix, as the layer keeps its projections, either side of every dispatch line:
 # backward tile | ring (592 runs of 64 tokens x 128 channels: 65 and 66 tiles at 3 x 384), ring runs of 32 | 64 tokens (147 and 148
 # tiles at 3 x 2,048), forward pair | streaming (36 and 37 blocks of 256 tokens at 3 x 2,048); ragged ends, several sequences.
