@@ -338,7 +338,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     for (const auto& t : state) tracked = tracked || torch::autograd::compute_requires_grad(t);
     // one launch for the three convolutions; a short call that carries windows issues them one by one, which is what the form with
     // the convolutions inside the forward kernel is compared with (8,191 x 2,048: 3 x 25 us one by one, 49 at once)
-    const int conv_step = (want_state || !state.empty()) && z.M < 1024 ? 1 : 3;
+    const int conv_step = (want_state || !state.empty()) && (z.M < 1024 || !fits_grid(z, 3)) ? 1 : 3;
     if (!fits_grid(z, tracked ? 3 : conv_step)) return c10::nullopt;
     fuse_conv = fuse_conv && !tracked && state.empty() && z.W == 4;
     // without a backward, up to 64 rows go straight to the float32 masters (kda_rows_linear): nothing to pack
