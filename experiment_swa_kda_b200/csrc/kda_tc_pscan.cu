@@ -86,13 +86,15 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
     uint8_t* Sop = sm + kScanPanel;
     float (*dec_ring)[128] = reinterpret_cast<float (*)[128]>(sm + kScanDec);
     // full: an item has landed.  free: the product that reads it is complete.  sop: all state threads have packed the state panel
-    // into tensor memory, pan: into shared memory.  out: the store has read that panel (one per buffer).  mma: the step's accumulator is complete.
+    // into tensor memory, pan: into shared memory.  out: the store has read that panel.  Both have one barrier per buffer: the store
+    // warp gives `out` of panel c - 1 before it looks for panel c, and by then a barrier of both buffers could have counted panels c
+    // and c + 1, which reads like none; panel c + 2 waits for `out` of panel c.  mma: the step's accumulator is complete.
     uint64_t* bar_full = reinterpret_cast<uint64_t*>(sm + kScanBars);
     uint64_t* bar_free = bar_full + kScanSlots;
-    uint64_t &bar_sop = bar_free[kScanSlots], &bar_pan = bar_free[kScanSlots + 1], &bar_mma = bar_free[kScanSlots + 2];
-    uint64_t* bar_out = bar_free + kScanSlots + 3;
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bar_free + kScanSlots + 5);
-    volatile int& abort_flag = *reinterpret_cast<volatile int*>(bar_free + kScanSlots + 6);
+    uint64_t &bar_sop = bar_free[kScanSlots], &bar_mma = bar_free[kScanSlots + 1];
+    uint64_t *bar_pan = bar_free + kScanSlots + 2, *bar_out = bar_pan + 2;
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bar_out + 2);
+    volatile int& abort_flag = *reinterpret_cast<volatile int*>(bar_out + 3);
     if (smem_u32(sm) & 1023u) {      // the swizzled tiles would be misread
         if (threadIdx.x == 0) raise_status(p.status, 56);
         return;
@@ -122,9 +124,10 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
             mbar_init(&bar_free[i], 1);
         }
         mbar_init(&bar_sop, 4 * kScanGroups);      // one arrival per state warp
-        mbar_init(&bar_pan, 4 * kScanGroups);
-        mbar_init(&bar_out[0], 1);
-        mbar_init(&bar_out[1], 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bar_pan[i], 4 * kScanGroups);
+            mbar_init(&bar_out[i], 1);
+        }
         mbar_init(&bar_mma, 1);
         mbar_fence_init();
         abort_flag = 0;
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
         // unit of a split scan its final state as one more panel
         if (elect_one()) {
             for (int c = 0; c < n + (split ? 1 : 0); ++c) {
-                if (!mbar_wait(&bar_pan, c & 1, p.status, 55)) { abort_flag = 1; break; }
+                if (!mbar_wait(&bar_pan[c & 1], (c >> 1) & 1, p.status, 55)) { abort_flag = 1; break; }
                 const CUtensorMap* m = c == n ? &mF : (composite ? &mS2 : &mS);      // composites go to their own panel array
                 const int row = c == n ? unit * 128 : (slot_of(c) * H + h) * 128;
                 for (int nb = 0; nb < 2; ++nb) tma_store_2d(m, Sop + (c & 1) * 32768 + nb * 16384, nb * 64, row);
@@ -304,7 +307,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
             for (int q = 0; q < 8; ++q)
                 *reinterpret_cast<uint4*>(dst + sw128_off(v, q)) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
             fence_async_smem();
-            warp_arrive(&bar_pan, lane);
+            warp_arrive(&bar_pan[c & 1], lane);
             return true;
         };
         bool ok = true;
