@@ -694,41 +694,63 @@ __device__ __forceinline__ f2 silu_vjp_2(f2 gy, f2 z) {
 
 // Gate activations, K % 4 == 0: a thread owns 4 adjacent channels (one head), so raw gate, bias, g and their gradients
 // move as 8- / 16-byte accesses and the head's exp(A_log) is computed once for all of a thread's rows.
-// Forward: grid x = blocks of 128 columns (lane = 4 channels), y = blocks of 32 tokens; warp w takes rows w, w + 8, w + 16,
-// w + 24 with all four loads in flight.  Bound by issue (an exponential and a division an element) and bytes in about equal
-// parts; walking the elements one quad at a time, with an index division, the bias and exp(A_log) for each, it took 31 us
-// at 8,191 x 2,048 bf16, now 27 (100 MB: 15 at the copy rate).
-constexpr int kGateFwdRows = 32;
+// Forward: quads of channels in memory order; n_thr is a multiple of a row's quads, and a thread takes quads i, i + n_thr, ..., four
+// at most and all in its column, with every load in flight.  No lane is idle whatever the width: with blocks of 128 columns,
+// narrower rows left lanes without work (200,000 x 8: 29 us, now 4.6).  Bound by issue (an exponential and a division an element)
+// and bytes in about equal parts; one quad at a time, with an index division, the bias and exp(A_log) for each, it took 26.7 us at
+// 8,191 x 2,048 bf16, now 21.0 (100 MB: 15 at the copy rate).  The four in one block of 32 rows: 22.6.
 template <bool BF16>
-__global__ void __launch_bounds__(256) gate_fwd4_kernel(int tokens, int H, int K, const void* __restrict__ raw,
+__global__ void __launch_bounds__(256) gate_fwd4_kernel(unsigned n_thr, size_t n4, int tokens, int H, int K, const void* __restrict__ raw,
                                                         const void* __restrict__ bl, int bl_ld, const float* __restrict__ A_log,
                                                         const float* __restrict__ dt_bias, float lb, float* __restrict__ g,
                                                         float* __restrict__ beta) {
-    const int hk = H * K, t0 = blockIdx.y * kGateFwdRows, warp = threadIdx.x >> 5;
-    const int c = (blockIdx.x * 32 + (threadIdx.x & 31)) * 4;
-    if (c < hk) {
-        float r[kGateFwdRows / 8][4];
+    const unsigned i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= n_thr) return;
+    constexpr size_t quad = BF16 ? 8 : 16;
+    const char* rp = static_cast<const char*>(raw) + i * quad;
+    float* gp = g + (size_t)i * 4;
+    const bool four = i + 3 * (size_t)n_thr < n4;
+    float r[4][4];
+    if (four) {
 #pragma unroll
-        for (int j = 0; j < kGateFwdRows / 8; ++j) ld_cvec<4, BF16>(r[j], raw, (size_t)min(t0 + warp + 8 * j, tokens - 1) * hk + c);
-        const float ea = expf(A_log[c / K]);
-        const float4 bias = *reinterpret_cast<const float4*>(dt_bias + c);
+        for (int j = 0; j < 4; ++j) ld_cvec<4, BF16>(r[j], rp + j * (n_thr * quad), 0);
+    } else {
 #pragma unroll
-        for (int j = 0; j < kGateFwdRows / 8; ++j) {
-            const int t = t0 + warp + 8 * j;
-            float4 o;
-            o.x = lb * sigmoidf_(ea * (r[j][0] + bias.x));
-            o.y = lb * sigmoidf_(ea * (r[j][1] + bias.y));
-            o.z = lb * sigmoidf_(ea * (r[j][2] + bias.z));
-            o.w = lb * sigmoidf_(ea * (r[j][3] + bias.w));
-            if (t < tokens) *reinterpret_cast<float4*>(g + (size_t)t * hk + c) = o;
-        }
+        for (int j = 0; j < 3; ++j)
+            if (i + j * (size_t)n_thr < n4) ld_cvec<4, BF16>(r[j], rp + j * (n_thr * quad), 0);
     }
-    if (blockIdx.x == 0) {                  // beta of this block's rows
-        const int nb = min(kGateFwdRows, tokens - t0) * H;
-        for (int i = threadIdx.x; i < nb; i += 256) {
-            const int t = t0 + i / H, h = i % H;
-            beta[(size_t)t * H + h] = sigmoidf_(ld_io(bl, (size_t)t * bl_ld + h, BF16));
-        }
+    // n_thr is a multiple of H too: a thread's beta logits, if it has any, belong to one head
+    const bool has_beta = i < (size_t)tokens * H;
+    unsigned bt = 0, bh = 0;
+    float b0 = 0.f;
+    if (has_beta) {
+        bt = i / (unsigned)H;
+        bh = i - bt * H;
+        b0 = ld_io(bl, (size_t)bt * bl_ld + bh, BF16);
+    }
+    const unsigned c = i % ((unsigned)(H * K) >> 2) * 4;
+    const float ea = expf(A_log[c / (unsigned)K]);
+    const float4 bias = *reinterpret_cast<const float4*>(dt_bias + c);
+    auto put = [&](int j) {
+        float4 o;
+        o.x = lb * sigmoidf_(ea * (r[j][0] + bias.x));
+        o.y = lb * sigmoidf_(ea * (r[j][1] + bias.y));
+        o.z = lb * sigmoidf_(ea * (r[j][2] + bias.z));
+        o.w = lb * sigmoidf_(ea * (r[j][3] + bias.w));
+        *reinterpret_cast<float4*>(gp + j * ((size_t)n_thr * 4)) = o;
+    };
+    if (four) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) put(j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (i + j * (size_t)n_thr < n4) put(j);
+    }
+    if (has_beta) {
+        beta[i] = sigmoidf_(b0);
+        const unsigned rows = n_thr / (unsigned)H;
+        for (size_t t = (size_t)bt + rows; t < (size_t)tokens; t += rows) beta[t * H + bh] = sigmoidf_(ld_io(bl, t * bl_ld + bh, BF16));
     }
 }
 
@@ -1908,21 +1930,16 @@ extern "C" int kda_gate_fwd_rows(int32_t tokens, int32_t heads, int32_t key_dim,
     const size_t n = (size_t)tokens * heads * key_dim;
     cudaStream_t fst = (cudaStream_t)stream;
     const bool al = ((reinterpret_cast<uintptr_t>(raw_gate) | reinterpret_cast<uintptr_t>(dt_bias) | reinterpret_cast<uintptr_t>(g_out)) % 16) == 0;
-    // the grid's y bounds the rows: longer inputs in pieces
-    if (key_dim % 4 == 0 && al && (long long)heads * key_dim < (1ll << 31)) {
-        constexpr int piece = 65535 * pw::kGateFwdRows;
-        const size_t row = (size_t)heads * key_dim, eb = io_dtype == KDA_DTYPE_BF16 ? 2 : 4;
-        for (int t0 = 0; t0 < tokens; t0 += piece) {
-            const int nt = std::min(piece, tokens - t0);
-            const dim3 grid(ceil_div((int)row, 128), ceil_div(nt, pw::kGateFwdRows));
-            const void* rp = static_cast<const char*>(raw_gate) + t0 * row * eb;
-            const void* bp = static_cast<const char*>(beta_logits) + (size_t)t0 * bl_ld * eb;
-            float *gp = g_out + t0 * row, *op = beta_out + (size_t)t0 * heads;
-            if (io_dtype == KDA_DTYPE_BF16)
-                KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<true><<<grid, 256, 0, fst>>>(nt, heads, key_dim, rp, bp, bl_ld, A_log, dt_bias, lower_bound, gp, op));
-            else
-                KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<false><<<grid, 256, 0, fst>>>(nt, heads, key_dim, rp, bp, bl_ld, A_log, dt_bias, lower_bound, gp, op));
-        }
+    // quads a thread: one up to four blocks a SM, two up to eight (77 rows of 2,048: 2.6, 2.9 and 3.5 us with 1, 2 and 4; 450:
+    // 3.8, 3.5, 3.6; 8,191: 39, 28, 21)
+    const int quads = n / 4 <= 148 * 4 * 256 ? 1 : (n / 4 <= 148 * 8 * 256 ? 2 : 4);
+    const long long n_thr = (long long)heads * key_dim / 4 * ceil_div(tokens, quads);
+    if (key_dim % 4 == 0 && al && (long long)heads * key_dim < (1ll << 31) && n_thr < (1ll << 31)) {      // 2^31 threads: 137 GB of g
+        const unsigned thr = (unsigned)n_thr, blocks4 = (thr + 255) / 256;
+        if (io_dtype == KDA_DTYPE_BF16)
+            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<true><<<blocks4, 256, 0, fst>>>(thr, n / 4, tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
+        else
+            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<false><<<blocks4, 256, 0, fst>>>(thr, n / 4, tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
         return launch_status();
     }
     if (bl_ld != heads) return KDA_ERR_UNSUPPORTED;      // strided beta logits: the vector path only

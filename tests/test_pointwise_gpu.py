@@ -225,6 +225,29 @@ def test_gate_matches_reference_vectors_and_gradients(golden_dir):
         torch.testing.assert_close(a.double().cpu(), b, atol=1e-5, rtol=1e-4)
 
 
+# one quad of channels a thread up to 151,552 of them (296 rows of 2,048), two up to 303,104 (592), then four; rows narrower and wider
+# than a block, row counts that four does not divide, fewer rows than that; beta logits in rows of their own and in wider ones
+@pytest.mark.parametrize("tokens,H,K", [(1, 1, 4), (3, 2, 4), (5, 3, 12), (33, 3, 44), (296, 16, 128), (297, 16, 128), (592, 16, 128), (593, 16, 128),
+                                        (4099, 3, 132), (200001, 1, 8), (70003, 8, 4)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gate_activations_at_every_width(tokens, H, K, dtype):
+    from experiment_swa_kda_b200 import _lib
+    lib = _lib.load()
+    gen = torch.Generator(device=D0).manual_seed(tokens + K)
+    raw = (3 * torch.randn(1, tokens, H, K, device=D0, generator=gen)).to(dtype)
+    A_log, bias = 0.5 * torch.randn(H, device=D0, generator=gen), torch.randn(H * K, device=D0, generator=gen)
+    want = O.decay_gate(raw.double(), A_log.double(), bias.double())
+    for ld in (H, H + 3):
+        logits = torch.randn(tokens, ld, device=D0, generator=gen).to(dtype)
+        g, beta = torch.full((tokens * H * K + 8,), 9.0, device=D0), torch.full((tokens * H + 8,), 9.0, device=D0)
+        _lib.check(lib.kda_gate_fwd_rows(tokens, H, K, _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_F32, raw.data_ptr(), logits.data_ptr(), ld,
+                                         A_log.data_ptr(), bias.data_ptr(), -5.0, g.data_ptr(), beta.data_ptr(), torch.cuda.current_stream().cuda_stream), "gate")
+        assert (g[-8:] == 9.0).all() and (beta[-8:] == 9.0).all()
+        # float32 arithmetic on arguments of up to 60: their rounding, 2^-24 of them, times the slope's bound of 5 / 4
+        torch.testing.assert_close(g[:-8].view_as(want).double(), want, atol=5e-6, rtol=1e-5)
+        torch.testing.assert_close(beta[:-8].view(tokens, H).double(), torch.sigmoid(logits[:, :H].double()), atol=1e-6, rtol=1e-5)
+
+
 def test_layer_forward_backward_finite_and_matches_composed_oracle():
     from experiment_swa_kda_b200 import KimiDeltaAttention
     torch.manual_seed(0)
