@@ -2102,7 +2102,6 @@ inline bool conv_grid_ok(int n, int B, int T) { return ceil_div(T, 8 * pw::kConv
 
 // n same-shaped convolutions in one launch; x rows ldx elements apart
 constexpr int kConvRun = 32;      // tokens per thread of the streaming forward
-constexpr long long kConvStreamBlocks = 148 * 3 / 2;
 template <int W>
 int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st) {
     const bool vec4 = C % 128 == 0 && ldx % 4 == 0;         // channels per thread: 4 when a warp's 128 channels fill a row segment
@@ -2112,12 +2111,20 @@ int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
         win = win || it.cache[i] != nullptr || it.fin[i] != nullptr;
         carried = carried || it.cache[i] != nullptr;
     }
-    // The streaming kernel from one and a half blocks of 32-token runs per SM on (3 x 2 x 4,096 x 384, 288 blocks: 16.4 -> 14.3 us;
-    // 3 x 4,096 x 2,048: 34.8 -> 28.8; 144 blocks: 12.3 and 12.4; 72: 8.3 and 12.3), unless a window is carried in.
+    // The streaming kernel unless a window is carried in, where its blocks of eight 32-token runs are many enough.  Filled to four fifths:
+    // one and a half a SM, two where a window is carried out (224 blocks: 1.09 and 0.91 times the speed of the other kernel, 288: 1.24
+    // and 1.00, 4,000: 1.26 and 1.2).  Where the last block of a sequence leaves more warps idle: filled to a half, and six a SM
+    // (5 of 8 runs: 0.8 to 1.1 at 450 to 600 blocks, 1.0 to 1.2 at 864; 1 or 2 of 8: 0.5 to 0.8 at any number; 3 of 8: 0.9 to 1.05).
+    // Up to 8 tokens a thread has one step to go, and the copy of the windows is what counts (1.0 to 1.3 up to twelve blocks a SM,
+    // 0.9 at 27, 0.7 at 83).
     if (vec4 && bf16 && !carried) {
         const int runs = ceil_div(T, 8 * kConvRun);
         const dim3 sgrid(C / 128, runs + (win ? 1 : 0), B * n);
-        if ((long long)sgrid.x * runs * sgrid.z >= kConvStreamBlocks && sgrid.y <= 65535) {
+        const long long blocks = (long long)sgrid.x * runs * sgrid.z;
+        const long long room = 8LL * kConvRun * runs;      // tokens a sequence's blocks could take
+        const bool filled = 5LL * T >= 4 * room ? blocks >= (win ? 2 * 148 : 148 * 3 / 2) : 2LL * T >= room && blocks >= 148 * 6;
+        const bool copied = win && T <= 8 && blocks >= 148 * 3 / 2 && blocks <= 148 * 12;
+        if ((filled || copied) && sgrid.y <= 65535) {
             KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, win ? runs : -1, silu, wf32, it));
             return launch_status();
         }

@@ -4,6 +4,8 @@ Each compares a shape that a dispatch or a walk over the work can serve badly wi
 times taken in turn.  The bounds lie between what the shape costs by nature and what it cost when it was served badly; both figures
 stand beside them."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -51,3 +53,23 @@ def test_gate_activations_of_narrow_rows():
     narrow, wide = _times([_gate(1 << 21, 2, 4), _gate(1 << 17, 1, 128)], 10)
     assert narrow < 3 * wide
 
+
+def _convolutions(n, B, T, C, windows):
+    from experiment_swa_kda_b200 import _lib
+    lib = _lib.load()
+    xs, ws = [torch.randn(B, T, C, device=D0).bfloat16() for _ in range(n)], [torch.randn(C, 4, device=D0) for _ in range(n)]
+    ys, fins = [torch.empty_like(x) for x in xs], [torch.empty(B, C, 4, device=D0, dtype=torch.bfloat16) for _ in range(n)]
+    held = [(ctypes.c_void_p * n)(*[t.data_ptr() for t in ts]) for ts in (xs, ws, ys, fins)]
+    a = [ctypes.cast(h, ctypes.c_void_p) for h in held]
+
+    def call(keep=(xs, ws, ys, fins, held)):
+        _lib.check(lib.kda_conv_fwd_rows(n, B, T, C, 4, _lib.DTYPE_BF16 | 0x100, 1, a[0], C, a[1], None, a[2], a[3] if windows else None,
+                                         torch.cuda.current_stream().cuda_stream), "convolution")
+    return call
+
+
+# by nature 1.43 and 1.27 (halo rows and windows of every sequence); 1.91 and 1.59 with most warps of the streaming kernel without a run
+@pytest.mark.parametrize("T,windows,bound", [(32, False, 1.67), (64, True, 1.43)])
+def test_convolutions_of_short_sequences(T, windows, bound):
+    short, long = _times([_convolutions(3, 8192 // T, T, 2048, windows), _convolutions(3, 1, 8192, 2048, windows)], 10)
+    assert short < bound * long
