@@ -1356,7 +1356,7 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
                      const void* beta, int gbf16, int l2norm, float scale, int tokens, const tc::ConvPrep* conv, cudaStream_t st);
 int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, int n_seq, int tokens, const void* d_o,
                      const float* d_final, float* dh0, cudaStream_t st);
-int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const void* q, const void* k, const void* v,
+int tc_intra_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, int n_seq, int tokens, const void* q, const void* k, const void* v,
                       const void* g, const void* d_o, int gbf16, int l2norm, float scale, void* dq, void* dk, void* dv,
                       void* dg, void* dbeta, cudaStream_t st);
 
@@ -1474,7 +1474,7 @@ int simt_chunk_bwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         if (w.nslots > 0) {
             int rc = tc_scan_backward(w, s, t, sh->n_seq, sh->tokens, d_o, d_final, dh0, st);
             if (rc) return rc;
-            rc = tc_intra_backward(w, t, sh->tokens, q, k, v, g, d_o, gbf16, sh->l2norm, sh->scale, dq, dk, dv, dg, dbeta, st);
+            rc = tc_intra_backward(w, s, t, sh->n_seq, sh->tokens, q, k, v, g, d_o, gbf16, sh->l2norm, sh->scale, dq, dk, dv, dg, dbeta, st);
             return rc ? rc : launch_status();
         } else if (dh0) {
             return KDA_ERR_UNSUPPORTED;

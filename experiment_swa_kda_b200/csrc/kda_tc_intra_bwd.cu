@@ -1,4 +1,4 @@
-// Tensor-core lane, chunk-parallel part of the backward: one CTA (512 threads) per (chunk, head) turns the
+// Tensor-core lane, chunk-parallel part of the backward: CTAs of 512 threads, one to an SM, walk over the (chunk, head)s and turn the
 // adjoints published by the reverse scan into dq, dk, dv, dg, dbeta.  K = V = 128, 64 tokens per chunk, bf16
 // UMMA operands, fp32 accumulation.  Warp (I, w) owns the 16 tokens of row block I and channels 32w .. 32w+31, spread over its
 // lanes in 8 x 8 pieces: lane l holds channels l/4 + {0, 8, 16, 24} and tokens 2(l%4) + {0, 1, 8, 9}.  That is what
@@ -112,9 +112,10 @@ struct IntraBwdArgs {
     const __nv_bfloat16* Mt;          // [nch][64][64] M~ (before beta)
     __nv_bfloat16 *dq, *dk, *dv;
     void *dg, *dbeta;                 // gate dtype
-    int l2norm, H, nslots;
+    int l2norm, H, n_seq, nslots;
     float scale;
     int* status;
+    int* next;                        // chunk-heads handed out beyond the blocks' first ones; zeroed by the kernel before this one
 };
 
 // shared-memory map (bytes, 1024-aligned base)
@@ -184,13 +185,14 @@ __global__ void __launch_bounds__(512, 1)
     __shared__ int next[3];                         // the next chunk-head: index (past the end: none), length, first token
     __shared__ __align__(8) float dA_diag[64];      // dA[i][i]: applied to dq, dk in float32, outside the pull-back products
 
-    const int H = p.H, total = p.nslots * H;
-    int work = blockIdx.x, len = 0, tok0 = 0;       // chunk-heads blockIdx.x, + gridDim.x, ...; heads slowest; empty slots are skipped
-    for (; work < total; work += gridDim.x) {
-        p.tab.span(work % p.nslots, tok0, len);
-        if (len > 0) break;
-    }
+    // Chunk-heads in order, heads slowest: the block's own first, then one at a time as blocks become free.  Dealt out in advance,
+    // the unused slots of a packed batch could all fall to the same blocks (74 sequences of 64 tokens, 148 slots, 16 heads: 184 us, now
+    // 115), and a block that had to wait for an SM kept its share (backward of 8,192 chunk-heads while another stream's kernel holds 12
+    // SMs: 1,630 us, now 1,127; alone 1,040 both).
+    const int H = p.H, used = p.tab.per_seq > 0 ? p.nslots : p.tab.seq_chunk0[p.n_seq], total = used * H;
+    int work = blockIdx.x, len = 0, tok0 = 0;
     if (work >= total) return;
+    p.tab.span(work % used, tok0, len);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int I = warp >> 2, wq = warp & 3;       // row block and channel quarter of this warp
     const int c4 = lane & 3, r8 = lane >> 2;      // token pair and channel inside an 8 x 8 piece
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(512, 1)
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
 
     if (warp >= 1 && warp <= 4 && elect_one()) {
-        const int h = work / p.nslots, ch = (work - h * p.nslots) * H + h;
+        const int h = work / used, ch = (work - h * used) * H + h;
         if (warp == 1) {
             for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_a, mb * 64, ch * 128);
             tma_load_2d(dZTs, &mdZT, &bar_a, 0, ch * 128);
@@ -277,11 +279,11 @@ __global__ void __launch_bounds__(512, 1)
         for (int j = 0; j < 3; ++j)
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + 64 * j + tid)), "l"(src[j] + (size_t)ch * 64 + tid) : "memory");
     };
-    if (tid < 64) load_rows(rowv2, (work % p.nslots) * H + work / p.nslots);
+    if (tid < 64) load_rows(rowv2, (work % used) * H + work / used);
     bool ok = true;
 #pragma unroll 1
     for (uint32_t ph = 0;; ph ^= 1) {       // every barrier below completes once a round
-    const int h = work / p.nslots;
+    const int h = work / used;
     float* rowv = rowv2 + 192 * ph;
     // ---- per-row scalars and the log-decay relative to the block's first row
     if (tid < 64) {
@@ -502,7 +504,12 @@ __global__ void __launch_bounds__(512, 1)
         umma_commit(&bar_q);
     }
     __syncwarp();
+    // The answer is on its way behind the product and goes to shared memory: held in a register up to where it is used it was
+    // spilled, and the spill waited for it (323 -> 352 us at 4,096 chunk-heads).
+    int taken = 0;
+    if (warp == 15 && lane == 0) taken = atomicAdd(p.next, 1);
     ok = ok && mbar_wait(&bar_x, ph, p.status, 42);
+    if (warp == 15 && lane == 0) next[0] = gridDim.x + taken;
     tc_fence_after();
 
     // ================================================================ phase 3: Y, dM
@@ -609,9 +616,12 @@ __global__ void __launch_bounds__(512, 1)
     uint8_t* DAt = sm + kR7;          // [I][32 rows: 16 dA rows, 16 beta*dM rows][64 s]   K-major / MN-major B
     // this warp's 16 rows of dA or dM go to the tile of row block wq
     const uint32_t da_off = kR7 + wq * 4096 + sw128_off(8 * (mi >> 1) + mr, 2 * I + (mi & 1));
-    // the next chunk-head of this CTA: one warp looks it up
-    int nwork = work + gridDim.x, nlen = 0, ntok0 = 0;
-    if (warp == 15 && nwork < total) p.tab.span(nwork % p.nslots, ntok0, nlen);
+    // where the next chunk-head of this CTA lies: on its way behind the panels
+    int nlen = 0, ntok0 = 0;
+    if (warp == 15) {
+        __syncwarp();
+        if (next[0] < total) p.tab.span(next[0] % used, ntok0, nlen);
+    }
     {
         // in flight: the decay panels.  Both operand families are stored transposed, [channel d][row] (K-major A operands).
         const uint32_t X = sb + kR3 + (I >> 1) * 16384;      // two target blocks share a panel: 32 stack rows each
@@ -660,16 +670,9 @@ __global__ void __launch_bounds__(512, 1)
         }
         stsm_x4(sb + da_off, w);
     }
-    if (warp == 15) {
-        while (nwork < total && nlen == 0) {
-            nwork += gridDim.x;
-            if (nwork < total) p.tab.span(nwork % p.nslots, ntok0, nlen);
-        }
-        if (lane == 0) {
-            next[0] = nwork;
-            next[1] = nlen;
-            next[2] = ntok0;
-        }
+    if (warp == 15 && lane == 0) {
+        next[1] = nlen;
+        next[2] = ntok0;
     }
     ok = ok && mbar_wait(&bar_m, ph, p.status, 44);
     tc_fence_after();
@@ -732,9 +735,9 @@ __global__ void __launch_bounds__(512, 1)
         const int i = tid - 128;
         st_io(p.dbeta, (size_t)(tok0 + i) * H + h, GB, dbp[i] + dbp[64 + i] + dbp[128 + i] + dbp[192 + i]);
     }
-    nwork = next[0];
+    const int nwork = next[0];
     const bool more = nwork < total;
-    const int nh = more ? nwork / p.nslots : 0, nch = more ? (nwork - nh * p.nslots) * H + nh : 0;
+    const int nh = more ? nwork / used : 0, nch = more ? (nwork - nh * used) * H + nh : 0;
     if (more && tid < 64) load_rows(rowv2 + 192 * (ph ^ 1), nch);
     // in flight: the dR part of dq, the dE and dQ parts of dk, the diagonal of dA
     f2 dqn[8], dkn[8], kn[8], dG[8];
@@ -1027,7 +1030,7 @@ __global__ void __launch_bounds__(512, 1)
 
 }  // namespace tc
 
-int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const void* q, const void* k, const void* v,
+int tc_intra_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, int n_seq, int tokens, const void* q, const void* k, const void* v,
                       const void* g, const void* d_o, int gbf16, int l2norm, float scale, void* dq, void* dk, void* dv,
                       void* dg, void* dbeta, cudaStream_t st) {
     using namespace tc;
@@ -1057,7 +1060,8 @@ int tc_intra_backward(const simt::Ws& w, const tc::TcWs& t, int tokens, const vo
     a.v = static_cast<const __nv_bfloat16*>(v); a.g = g;
     a.qinv = w.qinv; a.kinv = w.kinv; a.beta = w.beta; a.Mt = t.Mt;
     a.dq = static_cast<__nv_bfloat16*>(dq); a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
-    a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.nslots = w.nslots; a.scale = scale; a.status = t.status;
+    a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.n_seq = n_seq; a.nslots = w.nslots; a.scale = scale; a.status = t.status;
+    a.next = s.next;
     auto kern = gbf16 ? tc_intra_bwd_kernel<true> : tc_intra_bwd_kernel<false>;
     if (set_smem_limit(kern, kIntraBwdSmem)) return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_intra_bwd_kernel", st,

@@ -787,6 +787,7 @@ struct ChunkDzArgs {
     __nv_bfloat16* dZT;
     int H;
     int* status;
+    int* next;                 // zeroed here for the kernel after this one (tc_intra_bwd_kernel)
 };
 
 constexpr int kDzH = 0, kDzE = 32768, kDzO = 49152, kDzA = 65536;
@@ -801,6 +802,7 @@ __global__ void __launch_bounds__(256, 3)
     __shared__ uint64_t bar_in, bar_mma;
     __shared__ uint32_t tmem_slot;
     const int H = p.H, slot = blockIdx.x / H, h = blockIdx.x - slot * H;      // heads fastest, as in the intra-chunk kernels
+    if (blockIdx.x == 0 && threadIdx.x == 0) *p.next = 0;
     int len, tok0;
     p.tab.span(slot, tok0, len);
     if (len == 0) return;
@@ -960,7 +962,6 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
 int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, int n_seq, int tokens, const void* d_o,
                      const float* d_final, float* dh0, cudaStream_t st) {
     using namespace tc;
-    (void)s;
     const uint64_t nch = (uint64_t)w.nslots * w.H;
     CUtensorMap mE, mAT, mdO, mdH, mP, mRm, mdZT;
     int rc = 0;
@@ -994,7 +995,7 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
         if (int e = scan_fixup(w, t, n_seq, t.dHp, dh0, 1, mPp, mF, st)) return e;
     }
     ChunkDzArgs da;
-    da.tab = w.tab; da.dZT = t.dZT; da.H = w.H; da.status = t.status;
+    da.tab = w.tab; da.dZT = t.dZT; da.H = w.H; da.status = t.status; da.next = s.next;
     KDA_LAUNCH("tc_chunk_dz_kernel", st,
                tc_chunk_dz_kernel<<<(unsigned)nch, 256, kChunkDzSmem, st>>>(mdH, mE, mdO, mAT, mdZT, da));
     return launch_status();

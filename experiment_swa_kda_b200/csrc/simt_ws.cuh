@@ -59,6 +59,7 @@ struct Scr {
     float *dqn, *dkn, *dG;  // [nch][64][Kp]
     float* dA;              // [nch][64][64]
     float* dZ;              // [nch][64][Vp]   only when V > 64 (one value tile stays on chip)
+    int* next;              // tensor-core lane: chunk-heads handed out by the intra-chunk backward
 };
 
 inline int slots_for(const KdaChunkShape& sh, bool varlen_hint) {
@@ -138,6 +139,7 @@ inline Scr carve_scr(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr
     s.dG = c.take<float>(nch * 64 * Kp);
     s.dA = c.take<float>(nch * 4096);
     s.dZ = c.take<float>(Vp > 64 ? nch * 64 * Vp : 0);
+    s.next = c.take<int>(sh.lane == KDA_LANE_TC ? 64 : 0);
     if (bytes) *bytes = align_up(c.off, 256);
     return s;
 }
