@@ -75,13 +75,13 @@ def test_convolutions_of_short_sequences(T, windows, bound):
     assert short < bound * long
 
 
-def _backward(packed, n, length, heads):
+def _backward(packed, n, length, heads, gates=torch.bfloat16):
     from experiment_swa_kda_b200 import _lib, ops
     B, T = (1, n * length) if packed else (n, length)
     gen = torch.Generator(device=D0).manual_seed(n)
     draw = lambda *s: torch.randn(*s, device=D0, generator=gen)
     q, k, v, do = (draw(B, T, heads, 128).bfloat16() for _ in range(4))
-    g, beta = (-0.1 * draw(B, T, heads, 128).abs()).bfloat16(), torch.sigmoid(draw(B, T, heads)).bfloat16()
+    g, beta = (-0.1 * draw(B, T, heads, 128).abs()).to(gates), torch.sigmoid(draw(B, T, heads)).to(gates)
     cu = torch.arange(0, n * length + 1, length, device=D0, dtype=torch.int32) if packed else None
     _, _, saved = ops.chunk_kda_fwd(q, k, v, g, beta, None, cu, 128 ** -0.5, True, False, lane=_lib.LANE_TC)
     return lambda: ops.chunk_kda_bwd(q, k, v, g, beta, cu, do, None, saved, False)
@@ -94,3 +94,24 @@ def _backward(packed, n, length, heads):
 def test_backward_of_packed_sequences_equals_a_fixed_batch(n, length, bound):
     packed, fixed = _times([_backward(True, n, length, 16), _backward(False, n, length, 16)], 4)
     assert packed < bound * fixed
+
+
+# 1.12 by nature (twice the bytes, through the threads); 1.21 without the next chunk-head's rows on their way into L2
+def test_backward_with_float32_gates():
+    from experiment_swa_kda_b200 import _lib
+    calls = [_backward(False, 1, 16384, 16, gates) for gates in (torch.float32, torch.bfloat16)]
+    best = [float("inf")] * 2
+    for _ in range(6):
+        for i, call in enumerate(calls):
+            call()
+            torch.cuda.synchronize()
+            _lib.profile_report()
+            _lib.profile(True)
+            try:
+                for _ in range(4):
+                    call()
+            finally:
+                _lib.profile(False)
+            launches, ms = _lib.profile_report()["tc_intra_bwd_kernel"]
+            best[i] = min(best[i], ms / launches)
+    assert best[0] < 1.165 * best[1]
