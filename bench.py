@@ -64,7 +64,7 @@ def kda_kernel_flops(K, V, C=64):
 def chain_kernel_bytes(cfg):
     B, T, H, D = cfg["B"], cfg["T"], cfg["H"], cfg["D"]
     n = B * T * H * D * 2      # one bf16 tensor
-    return {"conv_fwd_kernel": 2 * n, "conv_bwd_kernel": 3 * n, "rmsnorm_fwd_kernel": 3 * n, "rmsnorm_bwd_kernel": 5 * n}
+    return {"conv_fwd_kernel": 2 * n, "conv_fwd_stream_kernel": 2 * n, "conv_bwd_kernel": 3 * n, "rmsnorm_fwd_kernel": 3 * n, "rmsnorm_bwd_kernel": 5 * n}
 
 
 # ----------------------------------------------------------------------------------------------

@@ -2125,7 +2125,7 @@ int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
         const bool filled = 5LL * T >= 4 * room ? blocks >= (win ? 2 * 148 : 148 * 3 / 2) : 2LL * T >= room && blocks >= 148 * 6;
         const bool copied = win && T <= 8 && blocks >= 148 * 3 / 2 && blocks <= 148 * 12;
         if ((filled || copied) && sgrid.y <= 65535) {
-            KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, win ? runs : -1, silu, wf32, it));
+            KDA_LAUNCH("conv_fwd_stream_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, win ? runs : -1, silu, wf32, it));
             return launch_status();
         }
     }

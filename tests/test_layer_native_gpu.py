@@ -57,8 +57,10 @@ def test_token_step_equals_the_modules(batch, heads, wdtype):
         assert O.rel_l2(a.float(), b.float()) <= 1e-2
 
 
-# up to 64 rows straight from the parameters, more through the packed matrix; odd head counts pad the projection
-@pytest.mark.parametrize("batch,T,heads,carried", [(1, 5, 1, False), (2, 32, 3, True), (1, 65, 3, True), (2, 130, 8, False)])
+# up to 64 rows straight from the parameters, more through the packed matrix; odd head counts pad the projection; from 1,024 rows on
+# the three convolutions in one launch, with windows carried in, out, and out of the streaming kernel
+@pytest.mark.parametrize("batch,T,heads,carried", [(1, 5, 1, False), (2, 32, 3, True), (1, 65, 3, True), (2, 130, 8, False), (1, 1023, 3, True), (2, 512, 3, True),
+                                                   (2, 601, 3, False), (4, 1100, 6, False), (520, 2, 1, True), (520, 2, 1, False)])
 def test_prefill_equals_the_modules(batch, T, heads, carried):
     gen = torch.Generator().manual_seed(T)
     layer = _layer(heads, 2)
@@ -196,3 +198,8 @@ def test_more_sequences_than_the_batched_convolutions_grid_holds(batch):
 def test_training_step_long_enough_for_the_streaming_convolutions():
     """2 x 1,100 tokens of 6 heads: 3 x 6 x 36 runs, past the line (592) from which slices of the projection are streamed."""
     test_training_step_equals_the_modules(2, 1100, 6, False, torch.float32)
+
+
+@pytest.mark.parametrize("batch,T,heads", [(2, 512, 3), (2, 1100, 6)])
+def test_training_step_whose_windows_go_through_one_launch(batch, T, heads):
+    test_training_step_equals_the_modules(batch, T, heads, True, torch.float32)

@@ -96,20 +96,57 @@ def test_conv_training_path_matches_oracle(B, T, C, dtype):
     assert O.rel_l2(got[1].squeeze(1).float(), want[1]) <= tol
 
 
-# from 1,776 blocks of 256 tokens x 128 channels on: ends within a group of 8 rows, a run of 32, a block; every window width class
-@pytest.mark.parametrize("W,B,T,C", [(4, 1, 28423, 2048), (2, 1, 28417, 2048), (3, 111, 511, 1024), (4, 1776, 5, 128), (1, 1776, 17, 128), (8, 222, 33, 1024)])
+def _forward_kernels(call):
+    """Which forward convolution kernels a call launches: {"conv_fwd_stream_kernel"} or {"conv_fwd_kernel"}."""
+    from experiment_swa_kda_b200 import _lib
+    torch.cuda.synchronize()
+    _lib.profile_report()
+    _lib.profile(True)
+    try:
+        call()
+    finally:
+        _lib.profile(False)
+    return {name for name in _lib.profile_report() if name.startswith("conv_fwd")}
+
+
+# ends within a group of 8 rows, a run of 32, a block; sequences that fill their last block by half or more; every window width
+@pytest.mark.parametrize("W,B,T,C", [(4, 1, 28423, 2048), (4, 1, 3549, 2048), (2, 1, 28417, 2048), (2, 222, 229, 128), (3, 111, 511, 1024), (4, 888, 133, 128),
+                                     (1, 888, 161, 128), (4, 444, 197, 256)])
 def test_streaming_convolution_equals_short_pieces(W, B, T, C):
     """Both kernels sum a window in the same order, so the long call equals calls on pieces of it to the bit."""
     gen = torch.Generator(device=D0).manual_seed(T + W)
     x = torch.randn(B, T, C, device=D0, generator=gen).bfloat16()
     mod = _conv_mod(C, W, torch.randn(C, W, device=D0, generator=gen))
+    out = []
     with torch.no_grad():
-        y, _ = mod(x)
+        assert _forward_kernels(lambda: out.append(mod(x)[0])) == {"conv_fwd_stream_kernel"}
         for b in sorted({0, B // 2, B - 1}):
-            for t0 in range(0, T, 4096):
+            for t0 in range(0, T, 2048):
                 h = min(t0, W - 1)
-                piece, _ = mod(x[b:b + 1, t0 - h:t0 + 4096].contiguous())
-                assert torch.equal(y[b, t0:t0 + 4096], piece[0, h:])
+                piece = x[b:b + 1, t0 - h:t0 + 2048].contiguous()
+                assert _forward_kernels(lambda: out.append(mod(piece)[0])) == {"conv_fwd_kernel"}
+                assert torch.equal(out[0][b, t0:t0 + 2048], out.pop()[0, h:])
+
+
+# Either side of every line of the forward's dispatch: blocks of 256 tokens x 128 channels, how well a sequence fills its own, windows
+# carried out
+@pytest.mark.parametrize("n,B,T,C,W,windows,streams", [(3, 1, 1024, 2048, 4, False, False), (3, 1, 1281, 2048, 4, False, True), (1, 221, 256, 128, 4, False, False),
+                                                       (1, 222, 205, 128, 4, False, True), (1, 222, 204, 128, 4, False, False), (1, 888, 128, 128, 4, False, True),
+                                                       (1, 888, 127, 128, 4, False, False), (1, 887, 128, 128, 3, False, False), (1, 295, 256, 128, 4, True, False),
+                                                       (1, 296, 256, 128, 4, True, True), (1, 221, 8, 128, 4, True, False), (1, 222, 8, 128, 4, True, True),
+                                                       (1, 222, 9, 128, 4, True, False), (1, 1777, 1, 128, 4, True, False), (1, 1776, 1, 128, 4, True, True),
+                                                       (1, 296, 8, 128, 4, False, False)])
+def test_the_forward_kernel_by_size(n, B, T, C, W, windows, streams):
+    import ctypes
+    from experiment_swa_kda_b200 import _lib
+    lib = _lib.load()
+    xs, ws = [torch.randn(B, T, C, device=D0).bfloat16() for _ in range(n)], [torch.randn(C, W, device=D0) for _ in range(n)]
+    ys, fins = [torch.empty_like(x) for x in xs], [torch.empty(B, C, W, device=D0, dtype=torch.bfloat16) for _ in range(n)]
+    arr = lambda ts: ctypes.cast((ctypes.c_void_p * n)(*[t.data_ptr() for t in ts]), ctypes.c_void_p)
+    a = [arr(ts) for ts in (xs, ws, ys, fins)]
+    call = lambda: _lib.check(lib.kda_conv_fwd_rows(n, B, T, C, W, _lib.DTYPE_BF16 | 0x100, 1, a[0], C, a[1], None, a[2], a[3] if windows else None,
+                                                    torch.cuda.current_stream().cuda_stream), "forward")
+    assert _forward_kernels(call) == {"conv_fwd_stream_kernel" if streams else "conv_fwd_kernel"}
 
 
 # 2,048 channels: 36 blocks of 64 tokens take the tile kernel, 37 the streaming one, both with ragged ends
@@ -319,10 +356,11 @@ def test_convolution_weights_at_any_element_offset(B, T, C, W, dtype, wdtype, st
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
-# either side of the line between the kernel of short runs and the streaming one (222 blocks of 256 tokens x 128 channels, three
-# convolutions: 216 and 240 here), a last run of one token, several sequences
-@pytest.mark.parametrize("B,T,C,W", [(1, 2303, 1024, 4), (1, 2305, 1024, 4), (3, 1025, 768, 2), (1, 10241, 256, 3)])
-def test_windows_carried_out_are_the_last_inputs(B, T, C, W):
+# either side of the line between the kernel of short runs and the streaming one (296 blocks of 256 tokens x 128 channels, three
+# convolutions: 288 and 312 here), a last run of one token, several sequences, fewer tokens than the window holds
+@pytest.mark.parametrize("B,T,C,W,streams", [(1, 3071, 1024, 4, False), (1, 3073, 1024, 4, True), (3, 1281, 768, 2, True), (1, 12801, 256, 3, True), (80, 2, 128, 4, True),
+                                             (40, 1, 256, 4, True), (40, 8, 256, 3, True), (20, 3, 128, 4, False)])
+def test_windows_carried_out_are_the_last_inputs(B, T, C, W, streams):
     import ctypes
     from experiment_swa_kda_b200 import _lib
     lib, n = _lib.load(), 3
@@ -337,15 +375,18 @@ def test_windows_carried_out_are_the_last_inputs(B, T, C, W):
         _lib.check(lib.kda_conv_fwd_rows(n, B, T, C, W, io, 1, arr(xs), C, arr(ws), None, arr(ys), arr(fins) if fins else None, stream), "forward")
         return ys
 
-    fins = [torch.full((B, C, W), 9.0, device=D0, dtype=torch.bfloat16) for _ in range(n)]
-    assert all(torch.equal(a, b) for a, b in zip(run(fins), run(None)))
-    assert all(torch.equal(f, x[:, T - W:].transpose(1, 2)) for f, x in zip(fins, xs))
+    fins, got = [torch.full((B, C, W), 9.0, device=D0, dtype=torch.bfloat16) for _ in range(n)], []
+    assert _forward_kernels(lambda: got.extend(run(fins))) == {"conv_fwd_stream_kernel" if streams else "conv_fwd_kernel"}
+    assert all(torch.equal(a, b) for a, b in zip(got, run(None)))
+    padded = [torch.nn.functional.pad(x, (0, 0, W, 0)) for x in xs]      # zeros before the first token
+    assert all(torch.equal(f, x[:, T:].transpose(1, 2)) for f, x in zip(fins, padded))
 
 
 # Three convolutions on slices of one wide matrix, as the layer keeps its projections, either side of every dispatch line:
 # backward tile | ring (592 runs of 64 tokens x 128 channels: 65 and 66 tiles at 3 x 384), ring runs of 32 | 64 tokens (147 and 148
-# tiles at 3 x 2,048), forward pair | streaming (36 and 37 blocks of 256 tokens at 3 x 2,048); ragged ends, several sequences.
-@pytest.mark.parametrize("B,T,C,W", [(1, 4160, 384, 4), (1, 4161, 384, 4), (3, 1431, 384, 3), (1, 9216, 2048, 4), (1, 9217, 2048, 4), (1, 9408, 2048, 4),
+# tiles at 3 x 2,048), forward pair | streaming (222 blocks of 256 tokens x 128 channels: 192 and 240 at 3 x 2,048); ragged ends,
+# several sequences.
+@pytest.mark.parametrize("B,T,C,W", [(1, 4160, 384, 4), (1, 4161, 384, 4), (3, 1431, 384, 3), (1, 1024, 2048, 4), (1, 1027, 2048, 4), (1, 9408, 2048, 4),
                                      (1, 9409, 2048, 4), (2, 4801, 2048, 2), (2, 70, 130, 4)])
 def test_convolutions_on_slices_equal_those_on_dense_copies(B, T, C, W):
     """The same kernels with another row stride: equal to the bit, with NaN in the columns that are not theirs and every column
