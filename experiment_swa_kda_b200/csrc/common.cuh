@@ -104,7 +104,7 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf
 // Device status of a workspace: int 0 is the status word, ints 2 and 3 hold the address of a page-locked host word that
 // mirrors it (null: none), left there by the forward's first kernel.  Only a failure writes either, so a call that goes
 // well pays nothing for being watched: the host reads its own memory at the next call.
-// Out of line: inlined at every wait it cost the intra-chunk kernels registers (forward 56 bytes of spills, now 28).
+// Out of line: inlined at every wait it cost the intra-chunk kernels registers (forward 56 bytes of spills, now 24).
 static __device__ __noinline__ void raise_status(int* status, int code) {
     // The thread that sets the word tells the host, nobody else: an expired wait is met by hundreds of threads over a long
     // time, and one that came after the host had read and cleared its word would blame the next, healthy call.

@@ -1401,7 +1401,7 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
     if (conv != nullptr && (sh->lane != KDA_LANE_TC || !sh->forward_only)) return KDA_ERR_UNSUPPORTED;
     if (norm != nullptr && norm->gate != nullptr && sh->lane != KDA_LANE_TC) return KDA_ERR_UNSUPPORTED;
     const int bf16 = sh->io_dtype == KDA_DTYPE_BF16, gbf16 = sh->gate_dtype == KDA_DTYPE_BF16;
-    const int KT = w.Kp / 64, VT = w.Vp / 64;
+    const int VT = w.Vp / 64;
     if (sh->lane == KDA_LANE_TC) {
         // chunk-parallel operand panels and transitions on tcgen05, the affine state scan, then the chunk outputs
         size_t ws_bytes = 0;

@@ -64,10 +64,6 @@ __device__ __forceinline__ void lds8(const float* p, float (&f)[8]) {
     const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
-__device__ __forceinline__ void sts8(float* p, const float (&f)[8]) {
-    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
-    *reinterpret_cast<float4*>(p + 4) = make_float4(f[4], f[5], f[6], f[7]);
-}
 // Per-channel tables (rows of 128 floats read 8 channels per lane): channel ch sits at ((ch >> 2) & 1) * 64 +
 // (ch >> 3) * 4 + (ch & 3), i.e. the two float4 halves of a lane's 8 channels live in separate 64-float halves of the
 // row, so that each of the two 16-byte accesses has a 16-byte lane stride (32 bytes would use half the banks).

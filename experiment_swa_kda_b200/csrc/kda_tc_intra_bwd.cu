@@ -106,10 +106,8 @@ __device__ __forceinline__ float quad_after(float p, int c4) {
 
 struct IntraBwdArgs {
     simt::ChunkTable tab;
-    const __nv_bfloat16 *q, *k, *v;   // caller tensors [tokens][H][128]
-    const void* g;                    // gate dtype
+    const void* g;                    // [tokens][H][128], gate dtype
     const float *qinv, *kinv, *beta;  // [nch][64] from the forward
-    const __nv_bfloat16* Mt;          // [nch][64][64] M~ (before beta)
     __nv_bfloat16 *dq, *dk, *dv;
     void *dg, *dbeta;                 // gate dtype
     int l2norm, H, n_seq, nslots;
@@ -1061,9 +1059,8 @@ int tc_intra_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, 
     if (rc) return KDA_ERR_CUDA;
     IntraBwdArgs a;
     a.tab = w.tab;
-    a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k);
-    a.v = static_cast<const __nv_bfloat16*>(v); a.g = g;
-    a.qinv = w.qinv; a.kinv = w.kinv; a.beta = w.beta; a.Mt = t.Mt;
+    a.g = g;
+    a.qinv = w.qinv; a.kinv = w.kinv; a.beta = w.beta;
     a.dq = static_cast<__nv_bfloat16*>(dq); a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
     a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.n_seq = n_seq; a.nslots = w.nslots; a.scale = scale; a.status = t.status;
     a.next = s.next;

@@ -71,7 +71,7 @@ constexpr int kScanMapSlots = 3;                            // composites load P
 constexpr int kScanPanel = kScanSlots * kScanItem;          // 2 x 32 KB  bf16 state panel of step c in c % 2, [2 k-blocks][128 rows x 128 B]
 constexpr int kScanDec = kScanPanel + 65536;                // exp(G_end) of step c in slot c % 4: [4][128] floats
 constexpr int kScanBars = kScanDec + 2048;
-constexpr int kAffineScanSmem = kScanBars + 256;            // 1 KB less than the limit: the base has to be 1024-aligned as it is
+constexpr int kAffineScanSmem = kScanBars + 256;            // 768 bytes below the limit: no room to align the base, which has to be 1024-aligned as it is
 constexpr int kScanGroups = 2;                              // state warpgroups: each thread owns 128 / kScanGroups columns of a row
 constexpr int kScanCols = 128 / kScanGroups;
 constexpr uint32_t kScanPanelCol = 256;                     // TMEM column of the bf16 state panel (64 columns: 128 keys as pairs)
@@ -784,7 +784,6 @@ __global__ void __launch_bounds__(256, 2)
 // ---------------------------------------------------------------------------------------------
 struct ChunkDzArgs {
     simt::ChunkTable tab;
-    __nv_bfloat16* dZT;
     int H;
     int* status;
     int* next;                 // zeroed here for the kernel after this one (tc_intra_bwd_kernel)
@@ -995,7 +994,7 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
         if (int e = scan_fixup(w, t, n_seq, t.dHp, dh0, 1, mPp, mF, st)) return e;
     }
     ChunkDzArgs da;
-    da.tab = w.tab; da.dZT = t.dZT; da.H = w.H; da.status = t.status; da.next = s.next;
+    da.tab = w.tab; da.H = w.H; da.status = t.status; da.next = s.next;
     KDA_LAUNCH("tc_chunk_dz_kernel", st,
                tc_chunk_dz_kernel<<<(unsigned)nch, 256, kChunkDzSmem, st>>>(mdH, mE, mdO, mAT, mdZT, da));
     return launch_status();

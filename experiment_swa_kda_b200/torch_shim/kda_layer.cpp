@@ -336,8 +336,9 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     bool tracked = torch::autograd::compute_requires_grad(x_);
     for (const auto& t : w) tracked = tracked || torch::autograd::compute_requires_grad(t);
     for (const auto& t : state) tracked = tracked || torch::autograd::compute_requires_grad(t);
-    // one launch for the three convolutions; a short call that carries windows issues them one by one, which is what the form with
-    // the convolutions inside the forward kernel is compared with (8,191 x 2,048: 3 x 25 us one by one, 49 at once)
+    // One launch for the three convolutions (8,191 x 2,048: 3 x 25 us one by one, 49 at once).  Below 1,024 rows a call that carries
+    // windows still issues them one by one, not for speed (77 rows of 384: 72 us, 62 at once): the form with the convolutions inside
+    // the forward kernel is defined, and tested, as this one without those three launches.
     const int conv_step = (want_state || !state.empty()) && (z.M < 1024 || !fits_grid(z, 3)) ? 1 : 3;
     if (!fits_grid(z, tracked ? 3 : conv_step)) return c10::nullopt;
     fuse_conv = fuse_conv && !tracked && state.empty() && z.W == 4;
