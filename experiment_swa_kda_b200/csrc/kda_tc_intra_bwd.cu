@@ -922,7 +922,8 @@ __global__ void __launch_bounds__(512, 1)
         const float dot = (q4[0] + q4[64]) + (q4[128] + q4[192]);
         const float inv_scale = p.scale != 0.f ? 1.0f / p.scale : 0.f;
         const float f = tid < 64 ? -inv_scale * inv_scale : -1.f;
-        rowb[tid] = p.l2norm ? f * dot * rowv[tid] : 0.f;
+        const bool far = tid < 64 && !(fabsf(inv_scale) > 1e-15f && fabsf(inv_scale) < 1e15f);      // its square leaves float32
+        rowb[tid] = !p.l2norm ? 0.f : (far ? -(dot * inv_scale) * (inv_scale * rowv[tid]) : f * dot * rowv[tid]);
     }
     {
         // what the rows of (I, channel) get from the later blocks and from the chunk's end

@@ -223,6 +223,20 @@ def test_blocks_that_walk_over_many_chunk_heads_equal_blocks_with_one(gate):
         for a, b in zip(whole, run(slice(h0, h0 + group))):
             assert torch.equal(a[:, :, h0:h0 + group], b)
 
+@pytest.mark.parametrize("scale", [2.0 ** -80, 2.0 ** 70])
+def test_gradients_at_scales_whose_square_leaves_float32(scale):
+    """Every product is linear in the scale and a power of two is exact, so outputs and gradients are those of scale 1 times it, to
+    the bit."""
+    m = _kda_mod()
+    d = {n: t.bfloat16().to(D0) for n, t in O.make_inputs(1, 130, 2, 128, 128, seed=5).items()}
+    do = torch.randn(d["v"].shape, generator=torch.Generator().manual_seed(6)).bfloat16().to(D0)
+    results = []
+    for s in (1.0, scale):
+        x = [d[n].clone().requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+        o, _ = m.chunk_kda(*x, scale=s, lane="tc")
+        results.append([t.float() for t in (o, *torch.autograd.grad(o, x, do))])
+    assert all(torch.equal(a * scale, b) for a, b in zip(*results))
+
 
 @pytest.mark.parametrize("lens,H", [([64 * 40 + 5, 30, 64 * 70 + 1], 2),          # 6 recurrences, mean 37 chunks -> 4 segments
                                     ([64 * 60 + 3, 0, 64 * 99, 1], 3),             # 12 recurrences, mean 39 chunks -> 4 segments
