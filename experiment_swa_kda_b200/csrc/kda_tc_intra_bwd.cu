@@ -941,7 +941,10 @@ __global__ void __launch_bounds__(512, 1)
         // overwrites only the pieces that it alone has read, dg over the dead tiles of the pull-back.
         const f2 qa[2] = {ld_2(rowv + tb), ld_2(rowv + tb + 8)}, qb[2] = {ld_2(rowb + tb), ld_2(rowb + tb + 8)};
 #pragma unroll
-        for (int e = 0; e < 8; ++e) dqn[e] = f2_fma(qn[e], qb[e & 1], f2_mul(dqn[e], qa[e & 1]));
+        for (int e = 0; e < 8; ++e) {
+            dqn[e] = f2_mul(dqn[e], qa[e & 1]);
+            if (p.l2norm) dqn[e] = f2_fma(qn[e], qb[e & 1], dqn[e]);      // without it dq does not depend on q: an infinite one stays out
+        }
         put_tile(sb + kQt, dqn);
         const f2 ka[2] = {ld_2(rowv + 64 + tb), ld_2(rowv + 64 + tb + 8)}, kb[2] = {ld_2(rowb + 64 + tb), ld_2(rowb + 64 + tb + 8)};
 #pragma unroll

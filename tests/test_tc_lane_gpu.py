@@ -238,6 +238,23 @@ def test_gradients_at_scales_whose_square_leaves_float32(scale):
     assert all(torch.equal(a * scale, b) for a, b in zip(*results))
 
 
+def test_without_the_norm_the_gradient_of_q_does_not_depend_on_q():
+    """An infinite q spoils what it enters - the outputs of its token, the gradients of k, v, g and beta - and nothing of dq."""
+    m = _kda_mod()
+    d = {n: t.bfloat16().to(D0) for n, t in O.make_inputs(1, 130, 2, 128, 128, seed=5).items()}
+    d["q"], d["k"] = (torch.nn.functional.normalize(d[n].float(), dim=-1).bfloat16() for n in ("q", "k"))
+    do = torch.randn(d["v"].shape, generator=torch.Generator().manual_seed(6)).bfloat16().to(D0)
+    results = []
+    for infinite in (False, True):
+        x = [d[n].clone() for n in ("q", "k", "v", "g", "beta")]
+        if infinite:
+            x[0][0, 70, 1, 5] = float("inf")
+        x = [t.requires_grad_(True) for t in x]
+        o, _ = m.chunk_kda(*x, use_qk_l2norm=False, lane="tc")
+        results.append(torch.autograd.grad(o, x, do)[0])
+    assert torch.equal(*results)
+
+
 @pytest.mark.parametrize("lens,H", [([64 * 40 + 5, 30, 64 * 70 + 1], 2),          # 6 recurrences, mean 37 chunks -> 4 segments
                                     ([64 * 60 + 3, 0, 64 * 99, 1], 3),             # 12 recurrences, mean 39 chunks -> 4 segments
                                     ([64 * 50, 64 * 3 + 9, 0, 64 * 19 + 63], 4)])  # 16 recurrences, mean 18 chunks -> 2 segments
