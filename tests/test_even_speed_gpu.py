@@ -96,10 +96,10 @@ def test_backward_of_packed_sequences_equals_a_fixed_batch(n, length, bound):
     assert packed < bound * fixed
 
 
-# 1.12 by nature (twice the bytes, through the threads); 1.21 without the next chunk-head's rows on their way into L2
+# 1.14 to 1.16 by nature (twice the bytes, through the threads); 1.27 without the next chunk-head's rows on their way into L2
 def test_backward_with_float32_gates():
     from experiment_swa_kda_b200 import _lib
-    calls = [_backward(False, 1, 16384, 16, gates) for gates in (torch.float32, torch.bfloat16)]
+    calls = [_backward(False, 22, 3000, 16, gates) for gates in (torch.float32, torch.bfloat16)]
     best = [float("inf")] * 2
     for _ in range(6):
         for i, call in enumerate(calls):
@@ -114,4 +114,4 @@ def test_backward_with_float32_gates():
                 _lib.profile(False)
             launches, ms = _lib.profile_report()["tc_intra_bwd_kernel"]
             best[i] = min(best[i], ms / launches)
-    assert best[0] < 1.165 * best[1]
+    assert best[0] < 1.215 * best[1]
