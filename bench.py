@@ -54,6 +54,8 @@ def kda_kernel_flops(K, V, C=64):
         "tc_chunk_out_kernel": 2 * C * K * V + C * C * V,
         "tc_affine_scan_bwd_kernel": K * K * V + C * K * V,
         "tc_chunk_dz_kernel": C * C * V + C * K * V,
+        "tc_walk_fwd_kernel": 3 * C * K * V + C * C * V,
+        "tc_walk_bwd_kernel": 3 * C * K * V + C * C * V,
         "tc_intra_bwd_kernel": bwd["bwd_local_kernel"] + bwd["pullback_kernel"],
     }
     out = {k: 2.0 * v for k, v in {**fwd, **bwd, **tcl}.items()}     # FLOP = 2 * MAC

@@ -1737,11 +1737,14 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd128_kernel(long long rows, int
             ld4<BF16>(gt[r], gate, ROWS ? gate_at(min(row0 + r, rows - 1)) : base);
         }
 #pragma unroll
-        for (int r = 0; r < kRmsRows; ++r) ss[r] = a[r][0] * a[r][0] + a[r][1] * a[r][1] + a[r][2] * a[r][2] + a[r][3] * a[r][3];
+        for (int r = 0; r < kRmsRows; ++r) ss[r] = fmaf(a[r][3], a[r][3], fmaf(a[r][2], a[r][2], fmaf(a[r][1], a[r][1], a[r][0] * a[r][0])));
+        // the halves of a row last: the operator's fused norm (tc_walk_kernel) has them in two blocks and gives the same bits
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
             for (int r = 0; r < kRmsRows; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], o);
+#pragma unroll
+        for (int r = 0; r < kRmsRows; ++r) ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 16);
 #pragma unroll
         for (int r = 0; r < kRmsRows; ++r) {
             if (row0 + r < rows) {

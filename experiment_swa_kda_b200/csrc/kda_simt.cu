@@ -1352,6 +1352,10 @@ using simt::Ws;
 
 int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens, const float* h0, float* final_state, void* o,
                     const tc::NormEpilogue& norm, cudaStream_t st);
+int tc_walk_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens, const float* h0, float* final_state, void* o,
+                    const tc::NormEpilogue& norm, cudaStream_t st);
+int tc_walk_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, int n_seq, int tokens, const void* d_o,
+                     const float* d_final, float* dh0, cudaStream_t st);
 int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const void* k, const void* v, const void* g,
                      const void* beta, int gbf16, int l2norm, float scale, int tokens, const tc::ConvPrep* conv, cudaStream_t st);
 int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, int n_seq, int tokens, const void* d_o,
@@ -1412,8 +1416,9 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         if (w.nslots > 0) {
             int rc = tc_intra_forward(w, t, q, k, v, g, beta, gbf16, sh->l2norm, sh->scale, sh->tokens, conv, st);
             if (rc) return rc;
-            rc = tc_scan_forward(w, t, sh->n_seq, sh->tokens, h0, final_state, o,
-                                 norm != nullptr ? *norm : tc::NormEpilogue{nullptr, nullptr, 0.f, nullptr, nullptr, 0}, st);
+            const auto recurrence = t.nseg > 1 ? tc_scan_forward : tc_walk_forward;
+            rc = recurrence(w, t, sh->n_seq, sh->tokens, h0, final_state, o,
+                            norm != nullptr ? *norm : tc::NormEpilogue{nullptr, nullptr, 0.f, nullptr, nullptr, 0}, st);
             if (rc) return rc;
         }
         return launch_status();
@@ -1472,7 +1477,7 @@ int simt_chunk_bwd(const KdaChunkShape* sh, const void* q, const void* k, const 
         tc::TcWs t = tc::carve_tc(*sh, static_cast<char*>(const_cast<void*>(workspace)) + ws_bytes);
         t.status = w.status;
         if (w.nslots > 0) {
-            int rc = tc_scan_backward(w, s, t, sh->n_seq, sh->tokens, d_o, d_final, dh0, st);
+            int rc = (t.nseg > 1 ? tc_scan_backward : tc_walk_backward)(w, s, t, sh->n_seq, sh->tokens, d_o, d_final, dh0, st);
             if (rc) return rc;
             rc = tc_intra_backward(w, s, t, sh->n_seq, sh->tokens, q, k, v, g, d_o, gbf16, sh->l2norm, sh->scale, dq, dk, dv, dg, dbeta, st);
             return rc ? rc : launch_status();

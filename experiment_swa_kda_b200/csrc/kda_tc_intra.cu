@@ -8,7 +8,8 @@
 //   T = (I + beta M~)^-1                                                       fp32, block forward substitution
 //   U^T = P^T T^T,  W^T = Q^T T^T   (P = beta v, Q = beta e^G k)                tcgen05, M=128 N=64 K=64, MN-major A
 //   R = q e^G, E = k e^{G_end-G}, e^{G_end}, A^T, T                            panels for the scans / backward
-//   Pn = W^T E,  Rm^T = R^T - W^T A^T   (the chunk's state transition)         tcgen05, M=128 N=128|64 K=64, at the end:
+//   Pn = W^T E,  Rm^T = R^T - W^T A^T   (the chunk's state transition,         tcgen05, M=128 N=128|64 K=64, at the end:
+//                                        for split scans only)
 //       W^T is staged in shared memory for its store, R, E and A^T are still there as they left
 // Every operand panel is written as 16-byte pieces of the 128-byte-swizzled layout the UMMA descriptors read: a thread
 // owns 8 adjacent channels of 4 consecutive rows, takes q, k, g straight from global memory (a half-warp reads one
@@ -18,7 +19,7 @@
 // between barriers.  Every panel leaves by TMA from the tile the products read, and nothing comes back: R^T stored from
 // registers in 8-byte pieces (32 sectors a warp store), E and A^T fetched again for the transition, with a fence in front,
 // and R^T read row by row had taken a fifth of a block's cycles.  16,384 chunk-heads: 1,157 -> 916 us, 384: 46 -> 39 us,
-// 2,048 forward-only: 148 -> 126 us.
+// 2,048 forward-only: 148 -> 126 us; without the transition 798, 34 and 115.
 // Restates reference chunk_wy_forward.cu:125-405 and 761-858.
 
 #include <cstdio>
@@ -321,6 +322,7 @@ __global__ void __launch_bounds__(kNT, 2)
     const int rq = 2 * warp + (lane >> 4);         // rows 4*rq .. 4*rq+3
     const int J = warp >> 1;                       // 16-row block of this thread's rows
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const bool trans = p.t.nseg > 1;               // the split scans walk over maps of whole chunks, formed at the end
 
     if (warp == 0 && elect_one()) {
         mbar_init(&bar_in, 1);
@@ -671,14 +673,14 @@ __global__ void __launch_bounds__(kNT, 2)
                 for (int c = 0; c < 8; ++c) x[c] *= b8[c];
                 ub[hh] = pack8(x);
             }
-            if (warp == 0 && elect_one()) tma_store_wait_read();       // the M~ panel has left: the identity takes its place
+            if (trans && warp == 0 && elect_one()) tma_store_wait_read();       // the M~ panel has left: the identity takes its place
             __syncthreads();                           // everyone has its piece of T: the operands take its place
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 const uint32_t off = sw128_off(i, 2 * seg + hh);
                 *reinterpret_cast<uint4*>(sm + kFTb + off) = u[hh];
                 *reinterpret_cast<uint4*>(sm + kFTbb + off) = ub[hh];
-                if (!p.t.fwd_only) {
+                if (trans && !p.t.fwd_only) {
                     const int one = i - 16 * seg - 8 * hh;         // this row's element on the diagonal, if it is in these 8
                     const uint32_t w = (one & 1) ? 0x3f800000u : 0x3f80u;
                     *reinterpret_cast<uint4*>(sm + kFMt + off) = make_uint4((one >> 1) == 0 ? w : 0u, (one >> 1) == 1 ? w : 0u, (one >> 1) == 2 ? w : 0u, (one >> 1) == 3 ? w : 0u);
@@ -744,70 +746,74 @@ __global__ void __launch_bounds__(kNT, 2)
             tma_store_2d(&mUT, vs, 0, (int)(ch * 128));
             tma_store_2d(&mWT, Qs, 0, (int)(ch * 128));
             tma_store_commit();
-            // ---- chunk transition, fused: Pn = W^T E and Rm^T = R^T - W^T A^T from the tiles that are still here.  Every
-            // accumulator column has been read out: Pn takes columns 0..127, Rm^T columns 128..191.  R lies token by token,
-            // so the product with an identity brings it in transposed (exactly: one term a sum).
-            tc_fence_after();
-            const uint32_t a0 = smem_u32(Qs), bE = smem_u32(sm + kFE);
-            const uint32_t id128 = umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
+            if (trans) {
+                // ---- chunk transition, fused: Pn = W^T E and Rm^T = R^T - W^T A^T from the tiles that are still here.  Every
+                // accumulator column has been read out: Pn takes columns 0..127, Rm^T columns 128..191.  R lies token by token,
+                // so the product with an identity brings it in transposed (exactly: one term a sum).
+                tc_fence_after();
+                const uint32_t a0 = smem_u32(Qs), bE = smem_u32(sm + kFE);
+                const uint32_t id128 = umma_idesc_bf16(128, 128, kMajorK, kMajorMN);
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16)     // Pn = W^T E
-                umma_bf16_ss(tmem, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
-                             umma_smem_desc_sw128(bE, 8192, 1024) + (k16 * 2048), id128, k16 > 0);
-            if (!p.t.fwd_only) {
-                const uint32_t idn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN, 1), idr = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
-                const uint32_t aR = smem_u32(sm + kFR), bA = smem_u32(sm + kFAT), bI = smem_u32(sm + kFMt);
+                for (int k16 = 0; k16 < 4; ++k16)     // Pn = W^T E
+                    umma_bf16_ss(tmem, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
+                                 umma_smem_desc_sw128(bE, 8192, 1024) + (k16 * 2048), id128, k16 > 0);
+                if (!p.t.fwd_only) {
+                    const uint32_t idn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN, 1), idr = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
+                    const uint32_t aR = smem_u32(sm + kFR), bA = smem_u32(sm + kFAT), bI = smem_u32(sm + kFMt);
 #pragma unroll
-                for (int k16 = 0; k16 < 4; ++k16)     // -(A W)^T = -W^T A^T
-                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
-                                 umma_smem_desc_sw128(bA, 8192, 1024) + (k16 * 2048), idn, k16 > 0);
+                    for (int k16 = 0; k16 < 4; ++k16)     // -(A W)^T = -W^T A^T
+                        umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(a0, 16, 1024) + (k16 * 32),
+                                     umma_smem_desc_sw128(bA, 8192, 1024) + (k16 * 2048), idn, k16 > 0);
 #pragma unroll
-                for (int k16 = 0; k16 < 4; ++k16)     // + R^T I
-                    umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(aR, 8192, 1024) + (k16 * 2048),
-                                 umma_smem_desc_sw128(bI, 16, 1024) + (k16 * 32), idr, 1);
-            }
-            // the staging below overwrites E, R and T: their stores must have been read, all but the newest group's
-            tma_store_wait_read_but1();
-            umma_commit(&bar_uw);
-        }
-        if (ok) ok = mbar_wait(&bar_uw, 1, p.t.status, 34);      // no block-wide barrier: the staging below overwrites only what
-        tc_fence_after();                                         // the completed products were the last to read
-        if (ok) {
-            // both results leave through shared memory in the swizzled layout (Pn over the T operands and the E tile, Rm^T
-            // over the R tile, all of them read for the last time) and are stored by TMA
-            uint8_t* Pst = sm + (gt ? kFE : kFTb);           // [128 key rows][64 columns of half gt]
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                uint32_t r[32];
-                tmem_ld32(tmem + lane_base + 64 * gt + 32 * b, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(Pst + sw128_off(kt, 4 * b + c)) =
-                        make_uint4(pack2(__uint_as_float(r[8 * c]), __uint_as_float(r[8 * c + 1])),
-                                   pack2(__uint_as_float(r[8 * c + 2]), __uint_as_float(r[8 * c + 3])),
-                                   pack2(__uint_as_float(r[8 * c + 4]), __uint_as_float(r[8 * c + 5])),
-                                   pack2(__uint_as_float(r[8 * c + 6]), __uint_as_float(r[8 * c + 7])));
-            }
-            if (!p.t.fwd_only) {     // the adjoint scan's operand is not needed in a forward-only call
-                uint32_t r[32];
-                tmem_ld32(tmem + lane_base + 128 + 32 * gt, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(sm + kFR + sw128_off(kt, 4 * gt + c)) =
-                        make_uint4(pack2(__uint_as_float(r[8 * c]), __uint_as_float(r[8 * c + 1])),
-                                   pack2(__uint_as_float(r[8 * c + 2]), __uint_as_float(r[8 * c + 3])),
-                                   pack2(__uint_as_float(r[8 * c + 4]), __uint_as_float(r[8 * c + 5])),
-                                   pack2(__uint_as_float(r[8 * c + 6]), __uint_as_float(r[8 * c + 7])));
+                    for (int k16 = 0; k16 < 4; ++k16)     // + R^T I
+                        umma_bf16_ss(tmem + 128, umma_smem_desc_sw128(aR, 8192, 1024) + (k16 * 2048),
+                                     umma_smem_desc_sw128(bI, 16, 1024) + (k16 * 32), idr, 1);
+                }
+                // the staging below overwrites E, R and T: their stores must have been read, all but the newest group's
+                tma_store_wait_read_but1();
+                umma_commit(&bar_uw);
             }
         }
-        fence_async_smem();
-        ok = __syncthreads_and(ok);
-        if (warp == 0 && elect_one() && ok) {
-            for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mP, sm + (nb ? kFE : kFTb), nb * 64, (int)(ch * 128));
-            if (!p.t.fwd_only) tma_store_2d(&mRm, sm + kFR, 0, (int)(ch * 128));
-            tma_store_commit();
+        if (trans) {
+            if (ok) ok = mbar_wait(&bar_uw, 1, p.t.status, 34);      // no block-wide barrier: the staging below overwrites only what
+            tc_fence_after();                                         // the completed products were the last to read
+            if (ok) {
+                // both results leave through shared memory in the swizzled layout (Pn over the T operands and the E tile, Rm^T
+                // over the R tile, all of them read for the last time) and are stored by TMA
+                uint8_t* Pst = sm + (gt ? kFE : kFTb);           // [128 key rows][64 columns of half gt]
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    uint32_t r[32];
+                    tmem_ld32(tmem + lane_base + 64 * gt + 32 * b, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<uint4*>(Pst + sw128_off(kt, 4 * b + c)) =
+                            make_uint4(pack2(__uint_as_float(r[8 * c]), __uint_as_float(r[8 * c + 1])),
+                                       pack2(__uint_as_float(r[8 * c + 2]), __uint_as_float(r[8 * c + 3])),
+                                       pack2(__uint_as_float(r[8 * c + 4]), __uint_as_float(r[8 * c + 5])),
+                                       pack2(__uint_as_float(r[8 * c + 6]), __uint_as_float(r[8 * c + 7])));
+                }
+                if (!p.t.fwd_only) {     // the adjoint scan's operand is not needed in a forward-only call
+                    uint32_t r[32];
+                    tmem_ld32(tmem + lane_base + 128 + 32 * gt, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<uint4*>(sm + kFR + sw128_off(kt, 4 * gt + c)) =
+                            make_uint4(pack2(__uint_as_float(r[8 * c]), __uint_as_float(r[8 * c + 1])),
+                                       pack2(__uint_as_float(r[8 * c + 2]), __uint_as_float(r[8 * c + 3])),
+                                       pack2(__uint_as_float(r[8 * c + 4]), __uint_as_float(r[8 * c + 5])),
+                                       pack2(__uint_as_float(r[8 * c + 6]), __uint_as_float(r[8 * c + 7])));
+                }
+            }
+            fence_async_smem();
+            ok = __syncthreads_and(ok);
+            if (warp == 0 && elect_one() && ok) {
+                for (int nb = 0; nb < 2; ++nb) tma_store_2d(&mP, sm + (nb ? kFE : kFTb), nb * 64, (int)(ch * 128));
+                if (!p.t.fwd_only) tma_store_2d(&mRm, sm + kFR, 0, (int)(ch * 128));
+                tma_store_commit();
+            }
         }
         if (warp == 0 && elect_one()) tma_store_wait_read();           // shared memory must outlive the reads of the bulk stores
     }
@@ -838,8 +844,8 @@ int tc_intra_forward(const simt::Ws& w, const tc::TcWs& t, const void* q, const 
     rc |= make_map_bf16(&mE, t.E, nch * 64, 128, 64, 64);
     rc |= make_map_bf16(&mR, t.R, nch * 64, 128, 64, 64);
     rc |= make_map_bf16(&mTp, t.fwd_only ? t.AT : t.Tp, nch * 64, 64, 64, 64);      // not stored in a forward-only call
-    rc |= make_map_bf16(&mP, t.Pn, nch * 128, 128, 64, 128);
-    rc |= make_map_bf16(&mRm, t.fwd_only ? t.WT : t.RmT, nch * 128, 64, 64, 128);      // not stored in a forward-only call
+    rc |= t.nseg > 1 ? make_map_bf16(&mP, t.Pn, nch * 128, 128, 64, 128) : (mP = mE, 0);      // the split scans' alone
+    rc |= t.nseg > 1 && !t.fwd_only ? make_map_bf16(&mRm, t.RmT, nch * 128, 64, 64, 128) : (mRm = mWT, 0);
     if (rc) return KDA_ERR_CUDA;
     auto kern = conv != nullptr ? (gbf16 ? tc_intra_fwd_kernel<true, true> : tc_intra_fwd_kernel<false, true>)
                                 : (gbf16 ? tc_intra_fwd_kernel<true, false> : tc_intra_fwd_kernel<false, false>);

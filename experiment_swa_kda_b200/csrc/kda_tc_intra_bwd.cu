@@ -142,7 +142,9 @@ constexpr int kBwdCtas = 148;      // one to an SM
 // lane, its 2-byte accesses, row scalars and 31 shuffles had been a quarter of a block's cycles.
 // 16,384 chunk-heads: 1,725 -> 1,207 us (1,490 by (2) and (5), 1,380 with cheaper issue, see elect_one; 2,262 before (1) and (4)),
 // 384: 65 -> 50 us.
-template <bool GB>
+// KV: the panels are the walk's, states [key][value] and Z, dZ [token][value]; otherwise the split scans', states [value][key] and Z, dZ
+// [value][token].
+template <bool GB, bool KV>
 __global__ void __launch_bounds__(512, 1)
     tc_intra_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                         const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mdO,
@@ -247,11 +249,26 @@ __global__ void __launch_bounds__(512, 1)
     __syncthreads();
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
 
+    auto load_z = [&](uint8_t* dst, const CUtensorMap& m, int c) {
+        if (KV)
+            for (int mb = 0; mb < 2; ++mb) tma_load_2d(dst + mb * 8192, &m, &bar_a, mb * 64, c * 64);
+        else
+            tma_load_2d(dst, &m, &bar_a, 0, c * 128);
+    };
+    // operands out of the panels at step k16 of a product: a state as A (rows: keys, contracted over values), Z or dZ as B (columns:
+    // tokens, contracted over values)
+    auto state_a = [&](uint32_t a, int k16) {
+        return KV ? umma_smem_desc_sw128(a, 16, 1024) + ((k16 >> 2) * 16384 + (k16 & 3) * 32) : umma_smem_desc_sw128(a, 16384, 1024) + (k16 * 2048);
+    };
+    auto z_b = [&](uint32_t b, int k16) {
+        return KV ? umma_smem_desc_sw128(b, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32) : umma_smem_desc_sw128(b, 8192, 1024) + (k16 * 2048);
+    };
+    constexpr uint32_t kSt = KV ? kMajorK : kMajorMN;       // how states, Z and dZ lie as these operands
     if (warp >= 1 && warp <= 4 && elect_one()) {
         const int h = work / used, ch = (work - h * used) * H + h;
         if (warp == 1) {
             for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_a, mb * 64, ch * 128);
-            tma_load_2d(dZTs, &mdZT, &bar_a, 0, ch * 128);
+            load_z(dZTs, mdZT, ch);
             tma_load_2d(Ts, &mT, &bar_a, 0, ch * 64);
         } else if (warp == 2) {
             for (int mb = 0; mb < 2; ++mb) {
@@ -265,7 +282,7 @@ __global__ void __launch_bounds__(512, 1)
             for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_a, mb * 64, ch * 128);
         } else {
             for (int mb = 0; mb < 2; ++mb) tma_load_2d(qs + mb * 8192, &mq, &bar_qk, h * 128 + mb * 64, tok0);
-            tma_load_2d(ZTs, &mZT, &bar_a, 0, ch * 128);
+            load_z(ZTs, mZT, ch);
             tma_load_2d(Mts, &mMt, &bar_a, 0, ch * 64);
         }
     }
@@ -384,17 +401,15 @@ __global__ void __launch_bounds__(512, 1)
     ok = ok && mbar_wait(&bar_a, ph, p.status, 40);
     if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
-        const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
-        const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
+        const uint32_t id_st = umma_idesc_bf16(128, 64, kSt, kSt);
+        const uint32_t id64_k_z = umma_idesc_bf16(64, 64, kMajorK, kSt);
         const uint32_t aH = smem_u32(Hs), bdZ = smem_u32(dZTs), aV = smem_u32(vs);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dW^T = H dZ^T
-            umma_bf16_ss(tmem + cW, umma_smem_desc_sw128(aH, 16384, 1024) + (k16 * 2048),
-                         umma_smem_desc_sw128(bdZ, 8192, 1024) + (k16 * 2048), id_mn_mn, k16 > 0);
+            umma_bf16_ss(tmem + cW, state_a(aH, k16), z_b(bdZ, k16), id_st, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // Xraw^T = v dZ^T  (first half)    (M = 64)
-            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aV, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32),
-                         umma_smem_desc_sw128(bdZ, 8192, 1024) + (k16 * 2048), id64_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cX, umma_smem_desc_sw128(aV, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), z_b(bdZ, k16), id64_k_z, k16 > 0);
         umma_commit(&bar_w);
     }
     __syncwarp();
@@ -420,53 +435,69 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = f2_mul(f2_mul(E[e], f2_all(ec[e >> 1])), w[e]);
         put_panel(sb + kR8, 2 * I, w);
-        // eight adjacent channels of four value rows a lane; the warp's eight lanes that share them add up by halving
-        const int cg = 4 * wq + mi;
-        f2 acc[4];
+        if constexpr (KV) {      // a key row and a quarter of its values a thread
+            f2 acc = f2_all(0.f);
+            if (ok) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[e] = f2_all(0.f);
-        if (ok) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t off = (uint32_t)(cg >> 3) * 16384 + sw128_off(32 * I + 8 * j + mr, cg & 7);
-                const uint4 a = *reinterpret_cast<const uint4*>(Hs + off), b = *reinterpret_cast<const uint4*>(dHs + off);
-                acc[0] = f2_fma(f2_from_bf16(a.x), f2_from_bf16(b.x), acc[0]);
-                acc[1] = f2_fma(f2_from_bf16(a.y), f2_from_bf16(b.y), acc[1]);
-                acc[2] = f2_fma(f2_from_bf16(a.z), f2_from_bf16(b.z), acc[2]);
-                acc[3] = f2_fma(f2_from_bf16(a.w), f2_from_bf16(b.w), acc[3]);
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t off = (uint32_t)(I >> 1) * 16384 + sw128_off(tid & 127, 4 * (I & 1) + j);
+                    const uint4 a = *reinterpret_cast<const uint4*>(Hs + off), b = *reinterpret_cast<const uint4*>(dHs + off);
+                    acc = f2_fma(f2_from_bf16(a.x), f2_from_bf16(b.x), acc);
+                    acc = f2_fma(f2_from_bf16(a.y), f2_from_bf16(b.y), acc);
+                    acc = f2_fma(f2_from_bf16(a.z), f2_from_bf16(b.z), acc);
+                    acc = f2_fma(f2_from_bf16(a.w), f2_from_bf16(b.w), acc);
+                }
             }
-        }
-        float v8[8];
+            const float2 x = f2_get(acc);
+            part[tid] = x.x + x.y;
+        } else {
+            // eight adjacent channels of four value rows a lane; the warp's eight lanes that share them add up by halving
+            const int cg = 4 * wq + mi;
+            f2 acc[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 x = f2_get(acc[e]);
-            v8[2 * e] = x.x;
-            v8[2 * e + 1] = x.y;
-        }
+            for (int e = 0; e < 4; ++e) acc[e] = f2_all(0.f);
+            if (ok) {
 #pragma unroll
-        for (int o = 4; o >= 1; o >>= 1) {
-            const bool up = (mr & o) != 0;
-#pragma unroll
-            for (int j = 0; j < o; ++j) {
-                const float send = up ? v8[j] : v8[j + o], keep = up ? v8[j + o] : v8[j];
-                v8[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t off = (uint32_t)(cg >> 3) * 16384 + sw128_off(32 * I + 8 * j + mr, cg & 7);
+                    const uint4 a = *reinterpret_cast<const uint4*>(Hs + off), b = *reinterpret_cast<const uint4*>(dHs + off);
+                    acc[0] = f2_fma(f2_from_bf16(a.x), f2_from_bf16(b.x), acc[0]);
+                    acc[1] = f2_fma(f2_from_bf16(a.y), f2_from_bf16(b.y), acc[1]);
+                    acc[2] = f2_fma(f2_from_bf16(a.z), f2_from_bf16(b.z), acc[2]);
+                    acc[3] = f2_fma(f2_from_bf16(a.w), f2_from_bf16(b.w), acc[3]);
+                }
             }
+            float v8[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 x = f2_get(acc[e]);
+                v8[2 * e] = x.x;
+                v8[2 * e + 1] = x.y;
+            }
+#pragma unroll
+            for (int o = 4; o >= 1; o >>= 1) {
+                const bool up = (mr & o) != 0;
+#pragma unroll
+                for (int j = 0; j < o; ++j) {
+                    const float send = up ? v8[j] : v8[j + o], keep = up ? v8[j + o] : v8[j];
+                    v8[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            part[I * 128 + 8 * cg + mr] = v8[0];
         }
-        part[I * 128 + 8 * cg + mr] = v8[0];
     }
     if (warp == 12 && elect_one() && ok) {
         tc_fence_after();
         const uint32_t aH = smem_u32(Hs), bdO = smem_u32(dOs), bZ = smem_u32(ZTs);
-        const uint32_t id_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK);
-        const uint32_t id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
+        const uint32_t id_st_k = umma_idesc_bf16(128, 64, kSt, kMajorK);
+        const uint32_t id64_k_z = umma_idesc_bf16(64, 64, kMajorK, kSt);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dR^T = H dO^T
-            umma_bf16_ss(tmem + cR, umma_smem_desc_sw128(aH, 16384, 1024) + (k16 * 2048),
-                         umma_smem_desc_sw128(bdO, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), id_mn_k, k16 > 0);
+            umma_bf16_ss(tmem + cR, state_a(aH, k16),
+                         umma_smem_desc_sw128(bdO, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), id_st_k, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dA = dO Z^T                      (M = 64)
-            umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32),
-                         umma_smem_desc_sw128(bZ, 8192, 1024) + (k16 * 2048), id64_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cA, umma_smem_desc_sw128(bdO, 16, 1024) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), z_b(bZ, k16), id64_k_z, k16 > 0);
     }
     __syncwarp();
     ok = ok && mbar_wait(&bar_w, ph, p.status, 41);
@@ -497,8 +528,8 @@ __global__ void __launch_bounds__(512, 1)
                          umma_smem_desc_sw128(bT, 8192, 1024) + (k16 * 2048), id_k_mn, k16 > 0);
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)     // dP^T = dZ^T T
-            umma_bf16_ss(tmem + cP, umma_smem_desc_sw128(smem_u32(dZTs), 16, 1024) + (k16 * 32),
-                         umma_smem_desc_sw128(bT, 8192, 1024) + (k16 * 2048), id_k_mn, k16 > 0);
+            umma_bf16_ss(tmem + cP, KV ? umma_smem_desc_sw128(smem_u32(dZTs), 8192, 1024) + (k16 * 2048) : umma_smem_desc_sw128(smem_u32(dZTs), 16, 1024) + (k16 * 32),
+                         umma_smem_desc_sw128(bT, 8192, 1024) + (k16 * 2048), KV ? umma_idesc_bf16(128, 64, kMajorMN, kMajorMN) : id_k_mn, k16 > 0);
         umma_commit(&bar_q);
     }
     __syncwarp();
@@ -550,11 +581,10 @@ __global__ void __launch_bounds__(512, 1)
             umma_bf16_ss(tmem + cY, umma_smem_desc_sw128(smem_u32(Ts), 8192, 1024) + (k16 * 2048),
                          umma_smem_desc_sw128(sb + kXT, 16, 1024) + (k16 * 32), id, k16 > 0);
         umma_commit(&bar_y);
-        const uint32_t id_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN);
+        const uint32_t id_st = umma_idesc_bf16(128, 64, kSt, kSt);
 #pragma unroll
         for (int k16 = 0; k16 < 8; ++k16)     // dE^T = dH' Z^T
-            umma_bf16_ss(tmem + cE, umma_smem_desc_sw128(smem_u32(dHs), 16384, 1024) + (k16 * 2048),
-                         umma_smem_desc_sw128(smem_u32(ZTs), 8192, 1024) + (k16 * 2048), id_mn_mn, k16 > 0);
+            umma_bf16_ss(tmem + cE, state_a(smem_u32(dHs), k16), z_b(smem_u32(ZTs), k16), id_st, k16 > 0);
         umma_commit(&bar_r);
     }
     __syncwarp();
@@ -790,10 +820,10 @@ __global__ void __launch_bounds__(512, 1)
         const int nt0 = next[2];
         mbar_expect_tx(&bar_a, kBytesA);
         for (int mb = 0; mb < 2; ++mb) tma_load_2d(Hs + mb * 16384, &mH, &bar_a, mb * 64, nch * 128);
-        tma_load_2d(dZTs, &mdZT, &bar_a, 0, nch * 128);
+        load_z(dZTs, mdZT, nch);
         for (int mb = 0; mb < 2; ++mb) tma_load_2d(dHs + mb * 16384, &mdH, &bar_a, mb * 64, nch * 128);
         for (int mb = 0; mb < 2; ++mb) tma_load_2d(dOs + mb * 8192, &mdO, &bar_a, nh * 128 + mb * 64, nt0);
-        tma_load_2d(ZTs, &mZT, &bar_a, 0, nch * 128);
+        load_z(ZTs, mZT, nch);
         tma_load_2d(Ts, &mT, &bar_a, 0, nch * 64);
         tma_load_2d(Mts, &mMt, &bar_a, 0, nch * 64);
         for (int mb = 0; mb < 2; ++mb) {            // into L2 only: their tiles are still in use
@@ -1052,8 +1082,9 @@ int tc_intra_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, 
     rc |= make_map_bf16(&mT, t.Tp, nch * 64, 64, 64, 64);
     rc |= make_map_bf16(&mH, t.Hp, nch * 128, 128, 64, 128);
     rc |= make_map_bf16(&mdH, t.dHp, nch * 128, 128, 64, 128);
-    rc |= make_map_bf16(&mZT, t.ZT, nch * 128, 64, 64, 128);
-    rc |= make_map_bf16(&mdZT, t.dZT, nch * 128, 64, 64, 128);
+    const bool kv = t.nseg == 1;      // who left the panels
+    rc |= kv ? make_map_bf16(&mZT, t.ZT, nch * 64, 128, 64, 64) : make_map_bf16(&mZT, t.ZT, nch * 128, 64, 64, 128);
+    rc |= kv ? make_map_bf16(&mdZT, t.dZT, nch * 64, 128, 64, 64) : make_map_bf16(&mdZT, t.dZT, nch * 128, 64, 64, 128);
     rc |= make_map_bf16(&mMt, t.Mt, nch * 64, 64, 64, 64);
     rc |= make_map_bf16(&mdq, dq, (uint64_t)tokens, cols, 64, 64);
     rc |= make_map_bf16(&mdk, dk, (uint64_t)tokens, cols, 64, 64);
@@ -1068,7 +1099,8 @@ int tc_intra_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, 
     a.dq = static_cast<__nv_bfloat16*>(dq); a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
     a.dg = dg; a.dbeta = dbeta; a.l2norm = l2norm; a.H = w.H; a.n_seq = n_seq; a.nslots = w.nslots; a.scale = scale; a.status = t.status;
     a.next = s.next;
-    auto kern = gbf16 ? tc_intra_bwd_kernel<true> : tc_intra_bwd_kernel<false>;
+    auto kern = kv ? (gbf16 ? tc_intra_bwd_kernel<true, true> : tc_intra_bwd_kernel<false, true>)
+                   : (gbf16 ? tc_intra_bwd_kernel<true, false> : tc_intra_bwd_kernel<false, false>);
     if (set_smem_limit(kern, kIntraBwdSmem)) return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_intra_bwd_kernel", st,
                kern<<<(unsigned)std::min<uint64_t>(nch, kBwdCtas), 512, kIntraBwdSmem, st>>>(mq, mk, mv, mdO, mT, mH, mdH, mZT, mdZT, mMt, mg, mdq, mdk, mdv, mdg, a));

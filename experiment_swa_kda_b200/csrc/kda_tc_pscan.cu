@@ -1,4 +1,5 @@
-// Tensor-core lane (K = V = 128): the state recurrences as affine scans.
+// Tensor-core lane (K = V = 128): the state recurrences as affine scans, for batches of so few and so long sequences that their steps
+// are cut into segments that run side by side (scan_segments; the others walk, kda_tc_walk.cu).
 //
 // With Z = U - W H substituted, one chunk maps its incoming state H to
 //     H' = exp(G_end) . H  -  (W^T E)^T-contracted H  +  E^T U          i.e.  H'^T = dec . H^T - H^T Pn + U^T E
@@ -26,7 +27,7 @@ int make_map_bf16_ld(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t co
 int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
 
 // ---------------------------------------------------------------------------------------------
-// affine scan: one CTA per (sequence, head) walks the chunks in order (forward) or in reverse (backward)
+// affine scan: one CTA per unit of a (sequence, head) walks its chunks in order (forward) or in reverse (backward)
 //     forward    S = H^T   [v][k]:   S' = dec . S - S Pn   + U^T E           stores S (chunk-start state) per chunk
 //     backward   S = dH'^T [v][k]:   S' = dec . S - S Pn^T + dO^T Rm         stores S (adjoint of the chunk's outgoing state)
 // Threads are specialised by warp; they meet only through mbarriers:
@@ -45,20 +46,18 @@ int make_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
 // ---------------------------------------------------------------------------------------------
 struct AffineScanArgs {
     simt::ChunkTable tab;
-    int heads_first;          // unsplit scans of several sequences: grid = (heads, sequences); 2: block (h, r) walks sequence tab.seq_order[r]
     const float* decay_end;   // [nch][128] exp(G_end)
     const float* s_in;        // V-first initial state (forward: h0, backward: cotangent of the final state), or null
-    float* s_out;             // V-first final state of the scan (forward: final state, backward: dh0), or null
     int H;
     int* status;
-    // Split scans (few long sequences: most SMs would idle behind a handful of 64-step chains).  The steps of every
+    // Few long sequences: most SMs would idle behind a handful of 64-step chains.  The steps of every
     // (sequence, head) are cut into nseg segments that run side by side as 2 nseg - 1 units: unit 0 walks segment 0 from
     // s_in; for every later segment k, unit 2k-1 walks it from a zero state (its "local" states L) and unit 2k walks its
     // state-to-state map alone, from the identity and without the state-independent term (the composites P of the
     // affine maps).  The true state at a chunk of segment k is S_k P + L with S_k the state at the segment's start;
     // tc_scan_fixup_kernel forms the S_k (a chain of nseg - 1 small products) and then the chunk states, chunk-parallel.
     // Units leave their final state as float32 (seg_fin) and as a bf16 panel (through mF).
-    int nseg;                 // 1: no split
+    int nseg;
     float* seg_fin;           // [n_seq*H*(2 nseg - 1)][128][128]
 };
 
@@ -102,13 +101,8 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int v = (warp & 3) * 32 + lane;          // value row = TMEM lane
-    const bool split = p.nseg > 1;
-    const int units = 2 * p.nseg - 1;
-    // split: grid (sequences x units, heads); unsplit: grid (heads, sequences), a packed batch longest first, so that the blocks
-    // the hardware starts first are the longest chains
-    const bool heads_first = !split && p.heads_first;
-    const int seq = split ? blockIdx.x / units : (heads_first ? (p.heads_first == 2 ? p.tab.seq_order[blockIdx.y] : blockIdx.y) : blockIdx.x), role = split ? blockIdx.x % units : 0;
-    const int h = heads_first ? blockIdx.x : blockIdx.y, H = p.H;
+    const int units = 2 * p.nseg - 1;             // grid (sequences x units, heads)
+    const int seq = blockIdx.x / units, role = blockIdx.x % units, h = blockIdx.y, H = p.H;
     const int c_begin = p.tab.first_chunk(seq), c_end = p.tab.first_chunk(seq + 1);
     const int n_total = c_end - c_begin;
     const int seg = (role + 1) >> 1;                             // segment this unit walks
@@ -249,10 +243,10 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
             }
         }
     } else if (warp == 4 * kScanGroups + 2) {
-        // ------------------------------------------------------------------ panel-store thread: the chunk-start states, and for a
-        // unit of a split scan its final state as one more panel
+        // ------------------------------------------------------------------ panel-store thread: the chunk-start states, and the
+        // unit's final state as one more panel
         if (elect_one()) {
-            for (int c = 0; c < n + (split ? 1 : 0); ++c) {
+            for (int c = 0; c < n + 1; ++c) {
                 if (!mbar_wait(&bar_pan[c & 1], (c >> 1) & 1, p.status, 55)) { abort_flag = 1; break; }
                 const CUtensorMap* m = c == n ? &mF : (composite ? &mS2 : &mS);      // composites go to their own panel array
                 const int row = c == n ? unit * 128 : (slot_of(c) * H + h) * 128;
@@ -311,7 +305,7 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
             return true;
         };
         bool ok = true;
-        if ((n > 0 || split) && !pack_state(0)) { abort_flag = 1; ok = false; }
+        if (!pack_state(0)) { abort_flag = 1; ok = false; }
         for (int c = 0; c < n && ok; ++c) {
             if (!mbar_wait(&bar_mma, c & 1, p.status, 53)) {
                 abort_flag = 1; ok = false;
@@ -336,17 +330,14 @@ __global__ void __launch_bounds__(kAffineScanThreads, 1)
                     }
             }
             tc_fence_before();
-            if ((c + 1 < n || split) && !pack_state(c + 1)) { abort_flag = 1; ok = false; }
+            if (!pack_state(c + 1)) { abort_flag = 1; ok = false; }
         }
-        float* fin = split ? p.seg_fin + (size_t)unit * 16384 : (p.s_out ? p.s_out + ((size_t)seq * H + h) * 16384 : nullptr);
-        if (ok && abort_flag == 0 && fin) {
-            // split units leave their final state thread-major (float4 j of state thread tid at [j][tid]: every warp
-            // store is one contiguous 512-byte run, and the fix-up's threads own the same elements); the scan's final
-            // state goes out in the caller's row-major layout
-            float4* dst = split ? reinterpret_cast<float4*>(fin) + tid : reinterpret_cast<float4*>(fin + (size_t)v * 128 + col0);
-            const int dstep = split ? 256 : 1;
+        if (ok && abort_flag == 0) {
+            // thread-major (float4 j of state thread tid at [j][tid]): every warp store is one contiguous 512-byte run, and the
+            // fix-up's threads own the same elements
+            float4* dst = reinterpret_cast<float4*>(p.seg_fin + (size_t)unit * 16384) + tid;
 #pragma unroll
-            for (int j = 0; j < kScanCols / 4; ++j) dst[j * dstep] = make_float4(s[4 * j], s[4 * j + 1], s[4 * j + 2], s[4 * j + 3]);
+            for (int j = 0; j < kScanCols / 4; ++j) dst[j * 256] = make_float4(s[4 * j], s[4 * j + 1], s[4 * j + 2], s[4 * j + 3]);
         }
     }
     tc_fence_before();
@@ -753,9 +744,10 @@ __global__ void __launch_bounds__(256, 2)
             const float2 o01 = __bfloat1622float2(oh[0]), o23 = __bfloat1622float2(oh[1]);
             const float2 g01 = __bfloat1622float2(gh[0]), g23 = __bfloat1622float2(gh[1]);
             const float a[4] = {o01.x, o01.y, o23.x, o23.y}, gt[4] = {g01.x, g01.y, g23.x, g23.y};
-            float ss = a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
+            float ss = fmaf(a[3], a[3], fmaf(a[2], a[2], fmaf(a[1], a[1], a[0] * a[0])));
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            for (int off = 8; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            ss += __shfl_xor_sync(0xffffffffu, ss, 16);
             if (i < len) {
                 const float inv = rsqrtf(ss * (1.0f / 128.0f) + p.norm.eps);
                 if (lane == 0 && p.norm.inv_rms != nullptr) p.norm.inv_rms[row] = inv;
@@ -932,23 +924,18 @@ int tc_scan_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
         set_smem_limit(tc_chunk_out_kernel, kChunkOutNormSmem))
         return KDA_ERR_CUDA;
     AffineScanArgs a;
-    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = h0; a.s_out = final_state;
+    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = h0;
     a.H = w.H; a.status = t.status; a.nseg = t.nseg; a.seg_fin = t.seg_fin;
     const int units = 2 * t.nseg - 1;
-    a.heads_first = t.nseg == 1 && n_seq > 1 && n_seq <= 65535 ? (w.tab.per_seq > 0 ? 1 : 2) : 0;      // equal lengths need no order
-    const dim3 scan_grid = a.heads_first ? dim3(w.H, n_seq) : dim3(n_seq * units, w.H);
-    CUtensorMap mPp = mH, mF = mH;
-    if (t.nseg > 1) {
-        if (make_map_bf16(&mPp, t.Pp, nch * 128, 128, 64, 128) ||
-            make_map_bf16(&mF, t.fin_panel, (uint64_t)n_seq * w.H * units * 128, 128, 64, 128))
-            return KDA_ERR_CUDA;
-    }
+    const dim3 scan_grid(n_seq * units, w.H);
+    CUtensorMap mPp, mF;
+    if (make_map_bf16(&mPp, t.Pp, nch * 128, 128, 64, 128) ||
+        make_map_bf16(&mF, t.fin_panel, (uint64_t)n_seq * w.H * units * 128, 128, 64, 128))
+        return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_affine_scan_fwd_kernel", st,
                tc_affine_scan_kernel<false><<<scan_grid, kAffineScanThreads, kAffineScanSmem, st>>>(mP, mUT, mE, mH, mPp, mF, a));
     if (int e = launch_status()) return e;
-    if (t.nseg > 1) {
-        if (int e = scan_fixup(w, t, n_seq, t.Hp, final_state, 0, mPp, mF, st)) return e;
-    }
+    if (int e = scan_fixup(w, t, n_seq, t.Hp, final_state, 0, mPp, mF, st)) return e;
     ChunkOutArgs oa;
     oa.tab = w.tab; oa.ZT = t.fwd_only ? nullptr : t.ZT; oa.o = static_cast<__nv_bfloat16*>(o); oa.H = w.H;
     oa.status = t.status;
@@ -976,23 +963,18 @@ int tc_scan_backward(const simt::Ws& w, const simt::Scr& s, const tc::TcWs& t, i
         set_smem_limit(tc_chunk_dz_kernel, kChunkDzSmem))
         return KDA_ERR_CUDA;
     AffineScanArgs a;
-    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = d_final; a.s_out = dh0;
+    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = d_final;
     a.H = w.H; a.status = t.status; a.nseg = t.nseg; a.seg_fin = t.seg_fin;
     const int units = 2 * t.nseg - 1;
-    a.heads_first = t.nseg == 1 && n_seq > 1 && n_seq <= 65535 ? (w.tab.per_seq > 0 ? 1 : 2) : 0;      // equal lengths need no order
-    const dim3 scan_grid = a.heads_first ? dim3(w.H, n_seq) : dim3(n_seq * units, w.H);
-    CUtensorMap mPp = mdH, mF = mdH;
-    if (t.nseg > 1) {
-        if (make_map_bf16(&mPp, t.Pp, nch * 128, 128, 64, 128) ||
-            make_map_bf16(&mF, t.fin_panel, (uint64_t)n_seq * w.H * units * 128, 128, 64, 128))
-            return KDA_ERR_CUDA;
-    }
+    const dim3 scan_grid(n_seq * units, w.H);
+    CUtensorMap mPp, mF;
+    if (make_map_bf16(&mPp, t.Pp, nch * 128, 128, 64, 128) ||
+        make_map_bf16(&mF, t.fin_panel, (uint64_t)n_seq * w.H * units * 128, 128, 64, 128))
+        return KDA_ERR_CUDA;
     KDA_LAUNCH("tc_affine_scan_bwd_kernel", st,
                tc_affine_scan_kernel<true><<<scan_grid, kAffineScanThreads, kAffineScanSmem, st>>>(mP, mRm, mdO, mdH, mPp, mF, a));
     if (int e = launch_status()) return e;
-    if (t.nseg > 1) {
-        if (int e = scan_fixup(w, t, n_seq, t.dHp, dh0, 1, mPp, mF, st)) return e;
-    }
+    if (int e = scan_fixup(w, t, n_seq, t.dHp, dh0, 1, mPp, mF, st)) return e;
     ChunkDzArgs da;
     da.tab = w.tab; da.H = w.H; da.status = t.status; da.next = s.next;
     KDA_LAUNCH("tc_chunk_dz_kernel", st,

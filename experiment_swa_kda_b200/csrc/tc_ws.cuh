@@ -23,16 +23,17 @@ struct TcWs {
     __nv_bfloat16* UT;          // [nch][128][64]   U transposed: [value][token]
     __nv_bfloat16* Tp;          // [nch][64][64]    T = (I + M)^-1, row-major
     __nv_bfloat16* Mt;          // [nch][64][64]    M before the beta scaling, strictly lower, row-major
-    __nv_bfloat16* Hp;          // [nch][128][128]  chunk-start state, V-first [value][key]
-    __nv_bfloat16* ZT;          // [nch][128][64]   Z transposed: [value][token]
-    __nv_bfloat16* dHp;         // [nch][128][128]  adjoint of each chunk's outgoing state, V-first
-    __nv_bfloat16* dZT;         // [nch][128][64]   dZ transposed
+    __nv_bfloat16* Hp;          // [nch][128][128]  chunk-start state: [key][value] from a walk, [value][key] from split scans
+    __nv_bfloat16* ZT;          // [nch][8192]      Z: [token][value], [value][token]
+    __nv_bfloat16* dHp;         // [nch][128][128]  adjoint of each chunk's outgoing state, as Hp
+    __nv_bfloat16* dZT;         // [nch][8192]      dZ, as ZT
+    // split scans only
     __nv_bfloat16* Pn;          // [nch][128][128]  W^T E: [key k][key k'], the state-to-state part of the chunk transition
     __nv_bfloat16* RmT;         // [nch][128][64]   (R - A W)^T: [key][token]
-    __nv_bfloat16* Pp;          // [nch][128][128]  split scans only: composite state-to-state maps at each chunk start
-    __nv_bfloat16* fin_panel;   // [n_seq*H*units][128][128]  split scans only: final state of every scan unit as a bf16 panel
-    float* seg_fin;             // [n_seq*H*units][128][128]  split scans only: the same in float32
-    int nseg;                   // scan segments per (sequence, head): 1 (no split), 2 or 4; units = 2 * nseg - 1
+    __nv_bfloat16* Pp;          // [nch][128][128]  composite state-to-state maps at each chunk start
+    __nv_bfloat16* fin_panel;   // [n_seq*H*units][128][128]  final state of every scan unit as a bf16 panel
+    float* seg_fin;             // [n_seq*H*units][128][128]  the same in float32
+    int nseg;                   // scan_segments(): 1 - no split scans -, or their segments per (sequence, head); units = 2 * nseg - 1
     float* decay_end;           // [nch][128]       exp(G_end)
     int* status;                // device status word (0 = ok); points at the workspace's word (simt::Ws::status)
     int fwd_only;               // 1: the backward-only panels (T, M~, Z^T, dH', dZ^T, Rm^T) have no storage and are not written
@@ -50,19 +51,21 @@ struct NormEpilogue {
     long long gate_ld;
 };
 
-// Scans are split when a batch has so few (sequence, head) recurrences that most SMs would idle behind them, and the
-// sequences are long enough for a shorter chain to outweigh the fix-up pass.  The decision uses the shape alone (a packed
-// batch is judged by its mean sequence length: the lengths themselves live on the device), so the forward and the
-// backward of a call agree; every sequence of the batch is cut into the same number of segments, short ones into
-// segments of one chunk or none.
+// How a batch goes through its recurrences: 1 - walks (kda_tc_walk.cu), two blocks to a (sequence, head) -, or the number of segments of
+// split scans (kda_tc_pscan.cu).  The decision uses the shape alone (a packed batch is judged by its mean sequence length: the lengths
+// themselves live on the device), so the forward and the backward of a call agree; split, every sequence of the batch is cut into the
+// same number of segments, short ones into segments of one chunk or none.
+// A walk's step takes about 1.1 us each way and has everything behind it done; split scans take a quarter of a step's 0.8 us for the
+// chain, but 48 + 176 KB more of memory traffic for every chunk of every recurrence, and three more launches each way.  So the walk
+// falls behind where there are few recurrences and many chunks.  Forward and backward in us, split / walk, by recurrences x chunks:
+// 2 x 16: 72 / 64, 2 x 32: 79 / 94, 12 x 32: 146 / 144, 12 x 128: 415 / 481, 16 x 32: 174 / 160, 16 x 128: 515 / 540, 32 x 128: 921 / 815.
+// Two segments (17 to 49 recurrences, or 16 to 31 chunks, of the measured split side) are behind the walk wherever they were chosen.
 inline int scan_segments(const KdaChunkShape& sh) {
     if (sh.n_seq <= 0) return 1;
     const bool fixed = sh.seq_len > 0 && (long long)sh.n_seq * sh.seq_len == sh.tokens;
     const long long rec = (long long)sh.n_seq * sh.heads;
     const long long chunks = fixed ? (sh.seq_len + 63) / 64 : (sh.tokens / 64) / sh.n_seq;
-    if (rec * 7 <= 148 && chunks >= 32) return 4;
-    if (rec * 3 <= 148 && chunks >= 16) return 2;
-    return 1;
+    return rec < 21 && chunks * (21 - rec) > 350 ? 4 : 1;      // at most 7 x 20 scan units, one to an SM
 }
 
 inline TcWs carve_tc(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr) {
@@ -77,15 +80,16 @@ inline TcWs carve_tc(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr
     t.UT = c.take<__nv_bfloat16>(nch * 8192);
     t.Tp = c.take<__nv_bfloat16>(bw * nch * 4096);
     t.Mt = c.take<__nv_bfloat16>(bw * nch * 4096);
-    t.Hp = c.take<__nv_bfloat16>(nch * 16384);
+    t.nseg = scan_segments(sh);
+    const size_t split = t.nseg > 1 ? 1 : 0;         // panels of the split scans and what follows them
+    t.Hp = c.take<__nv_bfloat16>((bw | split) * nch * 16384);
     t.ZT = c.take<__nv_bfloat16>(bw * nch * 8192);
     t.dHp = c.take<__nv_bfloat16>(bw * nch * 16384);
     t.dZT = c.take<__nv_bfloat16>(bw * nch * 8192);
-    t.Pn = c.take<__nv_bfloat16>(nch * 16384);
-    t.RmT = c.take<__nv_bfloat16>(bw * nch * 8192);
-    t.nseg = scan_segments(sh);
-    const size_t units = t.nseg > 1 ? (size_t)sh.n_seq * sh.heads * (2 * t.nseg - 1) : 0;
-    t.Pp = c.take<__nv_bfloat16>(t.nseg > 1 ? nch * 16384 : 0);
+    t.Pn = c.take<__nv_bfloat16>(split * nch * 16384);
+    t.RmT = c.take<__nv_bfloat16>(split * bw * nch * 8192);
+    const size_t units = split * sh.n_seq * sh.heads * (2 * t.nseg - 1);
+    t.Pp = c.take<__nv_bfloat16>(split * nch * 16384);
     t.fin_panel = c.take<__nv_bfloat16>(units * 16384);
     t.seg_fin = c.take<float>(units * 16384);
     t.decay_end = c.take<float>(nch * 128);
