@@ -341,9 +341,10 @@ __global__ void __launch_bounds__(NW * 32, NW > 8 ? 1 : (NV4 == 1 ? 4 : 2)) deco
             ld4<true>(gt, mix.gate, (size_t)(bh / H) * mix.ld + (bh % H) * 128 + 4 * lane);
             const float4 ww = *reinterpret_cast<const float4*>(mix.norm_w + 4 * lane);
             const float wa[4] = {ww.x, ww.y, ww.z, ww.w};
-            float ss = a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
+            float ss = fmaf(a[3], a[3], fmaf(a[2], a[2], fmaf(a[1], a[1], a[0] * a[0])));
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            for (int off = 8; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            ss += __shfl_xor_sync(0xffffffffu, ss, 16);
             const float inv = rsqrtf(ss * (1.0f / 128.0f) + mix.eps);
 #pragma unroll
             for (int e = 0; e < 4; ++e) out[e] = a[e] * inv * wa[e] * sigmoid_t<true>(gt[e]);
