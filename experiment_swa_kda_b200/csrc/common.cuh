@@ -70,10 +70,67 @@ __device__ __forceinline__ float warp_sum(float x) {
     return x;
 }
 
-// One output of a 128-wide product: lane holds x[4 lane .. 4 lane + 3] in xv; weights (float32 masters are rounded to
+// A kernel that may start while the one before it in its stream still runs (programmatic dependent launch).  Kernels launched
+// this way wait (dependency_wait) before they touch anything a kernel of the same call writes, and none of them holds tensor memory.
+template <class... P, class... A>
+inline cudaError_t launch_early(void (*kern)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool early, int cluster, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (early) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+// All of the kernel this one depends on has ended and its writes are visible; at once in a kernel launched the usual way.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What the kernel before may have written is read behind dependency_wait() by these: a load the compiler takes for one of constant
+// memory (__ldg, or through a const __restrict__ pointer) may be moved ahead of the wait, and was.
+__device__ __forceinline__ uint4 ld_after16(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
+__device__ __forceinline__ uint2 ld_after8(const void* p) {
+    uint2 r;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p) : "memory");
+    return r;
+}
+__device__ __forceinline__ float ld_after_bf16(const void* p, size_t i) {
+    unsigned short r;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(r) : "l"(static_cast<const __nv_bfloat16*>(p) + i) : "memory");
+    return __uint_as_float((unsigned)r << 16);
+}
+// All blocks of the cluster have come here, and what they wrote to shared memory, each other's included, is there.
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p = x in block `rank` of the cluster
+__device__ __forceinline__ void st_cluster(float* p, int rank, float x) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
+}
+// The kernel after this one may start once every block has said so or ended.
+__device__ __forceinline__ void dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// One output of a 128-wide product: lane holds x[4 lane .. 4 lane + 3] (u) in xv; weights (float32 masters are rounded to
 // bf16, as a cast of the matrix would) start at w[base].  Every lane gets the sum.
-__device__ __forceinline__ void narrow_x(const __nv_bfloat16* x, int lane, float (&xv)[4]) {
-    const uint2 u = *reinterpret_cast<const uint2*>(x + 4 * lane);
+__device__ __forceinline__ void narrow_x(uint2 u, float (&xv)[4]) {
     const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
     const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
     xv[0] = a.x; xv[1] = a.y; xv[2] = b.x; xv[3] = b.y;

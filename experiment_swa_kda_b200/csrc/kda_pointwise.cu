@@ -166,10 +166,14 @@ struct RawGate {
 // FUSED: the layer's decode step around the recurrence (K = V = 128, bf16, raw gate).  The kernel forms its head's raw
 // gate from the low-rank projection, steps the state, and applies the gated RMSNorm to the head's output: three launches
 // of a token become one.  Each part repeats the stand-alone kernel's arithmetic, so both forms give the same bits.  The
-// block then owns all 128 rows of a state: 32 warps hold the whole 64 KB in flight when there are fewer blocks than SMs
-// (8.5 us at one sequence and 3 heads, latency of the gate's weights and the state), eight warps otherwise.  Bound by the
-// state's bytes with many sequences: eight warps are held to 64 registers, four blocks an SM (256 x 16 states: 96 us, 0.86 of
-// the copy rate; with three blocks 101).
+// block then owns all 128 rows of a state: 32 warps hold the whole 64 KB in flight when there are fewer blocks than SMs,
+// eight warps otherwise.  Bound by the state's bytes with many sequences: eight warps are held to 64 registers, four blocks an SM (256 x
+// 16 states without the rest: 96 us, 0.86 of the copy rate; with three blocks 101).
+// With few, by a chain: the projections' outputs, the gate's weights (64 KB a block out of L2, which at 512 blocks it gave in 4.7 us),
+// the head's scalars, rows, norm.  So the gate's weights and the first rows are loaded while the launch before still runs, the blocks of
+// one head in four sequences form a cluster and share out the gate's rows, and the scalars are worked out once a block instead of in
+// every warp.  From the end of the projections to the end of the kernel: 512 states 17.2 -> 14.6 us, 3 states 5.3 -> 4.3; a whole token of
+// 32 x 16 heads 53.8 -> 45.8, of 1 x 3 18.4 -> 14.6 (9.6 in a graph, was 14.3).
 struct TokenMix {
     const __nv_bfloat16* fa;       // [n_seq][128], rows ld apart
     const void* fb_w;              // [heads*128][128]
@@ -177,23 +181,32 @@ struct TokenMix {
     const float* norm_w;           // [128]
     long long ld;
     float eps;
-    int fb_f32;
+    int fb_f32, n_seq;
 };
 
-template <int NV4, int R, int NW, bool FUSED>
-__global__ void __launch_bounds__(NW * 32, NW > 8 ? 1 : (NV4 == 1 ? 4 : 2)) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
+template <int NV4, int R, int NW, bool FUSED, int CL>
+__global__ void __launch_bounds__(NW * 32, NW > 8 ? 32 / NW : (NV4 == 1 ? 4 : 2)) decode_kernel(int H, int K, int V, int bf16, int gbf16, int l2norm, float scale,
                                                      const void* __restrict__ q, const void* __restrict__ k,
                                                      const void* __restrict__ v, const void* __restrict__ g,
                                                      const void* __restrict__ beta, const float* s_in, float* s_out,
                                                      void* __restrict__ o, int rows_per_cta, RawGate raw, TokenMix mix) {
     __shared__ __align__(16) float raw_s[FUSED ? 128 : 4];
+    __shared__ __align__(16) float head_s[FUSED ? 388 : 4];      // scaled unit q, unit k, decay, then q.k and beta
     __shared__ __align__(16) __nv_bfloat16 o_s[FUSED ? 128 : 8];
     constexpr int NE = NV4 > 0 ? 4 * NV4 : 8;     // state elements per lane per row
-    const int bh = blockIdx.x;                    // sequence * H + head
+    const int rank = blockIdx.x % CL, first = blockIdx.x - rank, last = CL > 1 ? mix.n_seq * H - 1 : 0;
+    const int at = CL > 1 ? min((int)blockIdx.x, last) : blockIdx.x;
+    const int head = CL > 1 ? at / mix.n_seq : at % H, seq = CL > 1 ? at - head * mix.n_seq : at / H;
+    const bool shared = CL > 1 && first / mix.n_seq == min(first + CL - 1, last) / mix.n_seq;
+    const int bh = seq * H + head;
     const int v_base = blockIdx.y * rows_per_cta;
     const int v_end = min(V, v_base + rows_per_cta);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto key_of = [&](int e) { return NV4 > 0 ? (128 * (e >> 2) + 4 * lane + (e & 3)) : (lane + 32 * e); };
+    auto load_v = [&](int r0, float (&vv)[R]) {      // FUSED: v is the work of the kernel before
+#pragma unroll
+        for (int j = 0; j < R; ++j) vv[j] = ld_after_bf16(v, (size_t)bh * V + min(r0 + j, v_end - 1));
+    };
     auto load_rows = [&](int r0, float (&s)[R][NE], float (&vv)[R]) {
 #pragma unroll
         for (int j = 0; j < R; ++j) {
@@ -210,76 +223,150 @@ __global__ void __launch_bounds__(NW * 32, NW > 8 ? 1 : (NV4 == 1 ? 4 : 2)) deco
 #pragma unroll
                 for (int e = 0; e < NE; ++e) s[j][e] = src[min(lane + 32 * e, K - 1)];
             }
-            vv[j] = ld_io(v, (size_t)bh * V + row, bf16);
+            if (!FUSED) vv[j] = ld_io(v, (size_t)bh * V + row, bf16);
         }
     };
     // first row group goes out before the per-(sequence, head) scalars are needed
     float s[R][NE], vv[R];
+    float qe[NE], ke[NE], dec[NE], bt, qk;
     int r0 = v_base + warp * R;
     if (r0 < v_end) load_rows(r0, s, vv);
     if (FUSED) {
-        const int hh = bh % H;
-        float xv[4];
-        narrow_x(mix.fa + (size_t)(bh / H) * mix.ld, lane, xv);
-        constexpr int PER = 128 / NW, G = 4;                        // gate rows per warp, G weight rows in flight
-#pragma unroll 1
-        for (int i0 = 0; i0 < PER; i0 += G) {
-            float wv[G][4], y[G];
+        dependents_go();
+        // Everything with an address of its own is on its way before the first of it is needed: the state and the gate's weights ahead
+        // of the launch this one may have started beside, the projections' outputs right behind its end.
+        constexpr int GR = 128 / (CL * NW), G = GR < 4 ? GR : 4;    // gate rows a warp, and how many at once, NW apart
+        float wv[G][4], xv[CL][4];
+        auto load_w = [&](int r0) {
 #pragma unroll
             for (int i = 0; i < G; ++i) {
-                const size_t base = ((size_t)hh * 128 + (i0 + i) * NW + warp) * 128;
+                const size_t base = ((size_t)head * 128 + r0 + NW * i + warp) * 128;
                 if (mix.fb_f32) narrow_w<true>(mix.fb_w, base, lane, wv[i]);
                 else narrow_w<false>(mix.fb_w, base, lane, wv[i]);
             }
+        };
+        load_w(shared ? GR * NW * rank : 0);
+        float ea = 0.f, db = 0.f;
+        if (threadIdx.x < 128) {
+            ea = expf(raw.A_log[head]);
+            db = raw.dt_bias[head * 128 + threadIdx.x];
+        }
+        if (CL > 1) cluster_sync();                                 // the other blocks have started: their shared memory is there
+        dependency_wait();
 #pragma unroll
-            for (int i = 0; i < G; ++i) y[i] = narrow_sum(xv, wv[i]);
-            if (lane == 0) {
+        for (int i = 0; i < CL; ++i) narrow_x(ld_after8(mix.fa + (size_t)(shared ? min(first + i, last) - head * mix.n_seq : seq) * mix.ld + 4 * lane), xv[i]);
+        if (warp == 0) {
+            bt = ld_after_bf16(beta, (size_t)seq * raw.bl_ld + head);
 #pragma unroll
-                for (int i = 0; i < G; ++i) raw_s[(i0 + i) * NW + warp] = __bfloat162float(__float2bfloat16(y[i]));
+            for (int e = 0; e < 4; ++e) {
+                qe[e] = ld_after_bf16(q, (size_t)bh * 128 + 4 * lane + e);
+                ke[e] = ld_after_bf16(k, (size_t)bh * 128 + 4 * lane + e);
             }
         }
+        load_v(r0, vv);
+        auto gate_rows = [&](const float (&x)[4], int r0, int to) {
+            float y[G];
+#pragma unroll
+            for (int i = 0; i < G; ++i) y[i] = narrow_sum(x, wv[i]);
+            if (lane == 0) {
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    const float r = __bfloat162float(__float2bfloat16(y[i]));
+                    if (CL > 1) st_cluster(raw_s + r0 + NW * i + warp, to, r);
+                    else raw_s[r0 + NW * i + warp] = r;
+                }
+            }
+        };
+        if (shared) {
+            static_assert(CL == 1 || G == GR, "a shared block's rows go at once");
+#pragma unroll
+            for (int c = 0; c < CL; ++c) gate_rows(xv[c], G * NW * rank, c);
+        } else {
+#pragma unroll 1
+            for (int r0 = 0;;) {
+                gate_rows(xv[0], r0, rank);
+                if ((r0 += G * NW) >= 128) break;
+                load_w(r0);
+            }
+        }
+        if (warp == 0) {                                            // the head's q, k and scalars, once for all warps
+            float sq = 0.f, sk = 0.f, qk = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sq += qe[e] * qe[e];
+                sk += ke[e] * ke[e];
+            }
+            sq = warp_sum(sq);
+            sk = warp_sum(sk);
+            const float qi = 1.f / fmaxf(sqrtf(sq), 1e-12f) * scale, ki = 1.f / fmaxf(sqrtf(sk), 1e-12f);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                qe[e] *= qi;
+                ke[e] *= ki;
+                qk += qe[e] * ke[e];
+            }
+            qk = warp_sum(qk);
+            *reinterpret_cast<float4*>(head_s + 4 * lane) = make_float4(qe[0], qe[1], qe[2], qe[3]);
+            *reinterpret_cast<float4*>(head_s + 128 + 4 * lane) = make_float4(ke[0], ke[1], ke[2], ke[3]);
+            if (lane == 0) {
+                head_s[384] = qk;
+                head_s[385] = sigmoidf_(bt);
+            }
+        }
+        if (CL > 1) cluster_sync();
+        else __syncthreads();
+        if (CL > 1 && (int)blockIdx.x > last) return;               // there for its share of the gate
+        if (threadIdx.x < 128) head_s[256 + threadIdx.x] = expf(raw.lb * sigmoidf_(ea * (raw_s[threadIdx.x] + db)));
         __syncthreads();
-    }
-
-    float qe[NE], ke[NE], dec[NE];
+        auto get4 = [&](float (&x)[NE], int at) {
+            const float4 f = *reinterpret_cast<const float4*>(head_s + at + 4 * lane);
+            x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
+        };
+        get4(qe, 0);
+        get4(ke, 128);
+        get4(dec, 256);
+        qk = head_s[384];
+        bt = head_s[385];
+    } else {
 #pragma unroll
-    for (int e = 0; e < NE; ++e) {
-        const size_t i = (size_t)bh * K + min(key_of(e), K - 1);
-        qe[e] = ld_io(q, i, bf16);
-        ke[e] = ld_io(k, i, bf16);
-        dec[e] = FUSED ? raw_s[key_of(e)] : ld_io(g, i, gbf16);
-    }
-    float bt = ld_io(beta, raw.A_log != nullptr ? (size_t)(bh / H) * raw.bl_ld + bh % H : (size_t)bh, gbf16);
-    if (raw.A_log != nullptr) {
-        const int hh = bh % H;
-        const float ea = expf(raw.A_log[hh]);
-        bt = sigmoidf_(bt);
+        for (int e = 0; e < NE; ++e) {
+            const size_t i = (size_t)bh * K + min(key_of(e), K - 1);
+            qe[e] = ld_io(q, i, bf16);
+            ke[e] = ld_io(k, i, bf16);
+            dec[e] = ld_io(g, i, gbf16);
+        }
+        bt = ld_io(beta, raw.A_log != nullptr ? (size_t)(bh / H) * raw.bl_ld + bh % H : (size_t)bh, gbf16);
+        if (raw.A_log != nullptr) {
+            const int hh = bh % H;
+            const float ea = expf(raw.A_log[hh]);
+            bt = sigmoidf_(bt);
 #pragma unroll
-        for (int e = 0; e < NE; ++e)
-            dec[e] = raw.lb * sigmoidf_(ea * (dec[e] + raw.dt_bias[hh * K + min(key_of(e), K - 1)]));
-    }
-    float sq = 0.f, sk = 0.f;
+            for (int e = 0; e < NE; ++e)
+                dec[e] = raw.lb * sigmoidf_(ea * (dec[e] + raw.dt_bias[hh * K + min(key_of(e), K - 1)]));
+        }
+        float sq = 0.f, sk = 0.f;
 #pragma unroll
-    for (int e = 0; e < NE; ++e) {
-        const bool in = key_of(e) < K;
-        qe[e] = in ? qe[e] : 0.f;
-        ke[e] = in ? ke[e] : 0.f;
-        dec[e] = in ? expf(dec[e]) : 0.f;
-        sq += qe[e] * qe[e];
-        sk += ke[e] * ke[e];
-    }
-    sq = warp_sum(sq);
-    sk = warp_sum(sk);
-    const float qi = (l2norm ? 1.f / fmaxf(sqrtf(sq), 1e-12f) : 1.f) * scale;
-    const float ki = l2norm ? 1.f / fmaxf(sqrtf(sk), 1e-12f) : 1.f;
-    float qk = 0.f;
+        for (int e = 0; e < NE; ++e) {
+            const bool in = key_of(e) < K;
+            qe[e] = in ? qe[e] : 0.f;
+            ke[e] = in ? ke[e] : 0.f;
+            dec[e] = in ? expf(dec[e]) : 0.f;
+            sq += qe[e] * qe[e];
+            sk += ke[e] * ke[e];
+        }
+        sq = warp_sum(sq);
+        sk = warp_sum(sk);
+        const float qi = (l2norm ? 1.f / fmaxf(sqrtf(sq), 1e-12f) : 1.f) * scale;
+        const float ki = l2norm ? 1.f / fmaxf(sqrtf(sk), 1e-12f) : 1.f;
+        qk = 0.f;
 #pragma unroll
-    for (int e = 0; e < NE; ++e) {
-        qe[e] *= qi;
-        ke[e] *= ki;
-        qk += qe[e] * ke[e];
+        for (int e = 0; e < NE; ++e) {
+            qe[e] *= qi;
+            ke[e] *= ki;
+            qk += qe[e] * ke[e];
+        }
+        qk = warp_sum(qk);
     }
-    qk = warp_sum(qk);
 
     for (; r0 < v_end; r0 += NW * R) {
         float a[R], b[R];
@@ -331,14 +418,17 @@ __global__ void __launch_bounds__(NW * 32, NW > 8 ? 1 : (NV4 == 1 ? 4 : 2)) deco
                 }
             }
         }
-        if (r0 + NW * R < v_end) load_rows(r0 + NW * R, s, vv);
+        if (r0 + NW * R < v_end) {
+            load_rows(r0 + NW * R, s, vv);
+            if (FUSED) load_v(r0 + NW * R, vv);
+        }
     }
     if (FUSED) {
         __syncthreads();
         if (warp == 0) {      // the head's 128 outputs: lane = 4 adjacent values, as in the stand-alone norm
             float a[4], gt[4], out[4];
             ld4<true>(a, o_s, 4 * lane);
-            ld4<true>(gt, mix.gate, (size_t)(bh / H) * mix.ld + (bh % H) * 128 + 4 * lane);
+            narrow_x(ld_after8(mix.gate + (size_t)seq * mix.ld + head * 128 + 4 * lane), gt);
             const float4 ww = *reinterpret_cast<const float4*>(mix.norm_w + 4 * lane);
             const float wa[4] = {ww.x, ww.y, ww.z, ww.w};
             float ss = fmaf(a[3], a[3], fmaf(a[2], a[2], fmaf(a[1], a[1], a[0] * a[0])));
@@ -2015,7 +2105,7 @@ static int decode_launch(int n_seq, int heads, int key_dim, int value_dim, int b
                      ((reinterpret_cast<uintptr_t>(state_in) | reinterpret_cast<uintptr_t>(state_out)) % 16 == 0);
     const pw::TokenMix none = {};
 #define KDA_DECODE(NV4) \
-    KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<NV4, 4, 8, false><<<grid, 256, 0, st>>>(heads, key_dim, value_dim, bf16, gbf16, l2norm, scale, q, k, v, g, beta, state_in, state_out, o, rows_per_cta, raw, none))
+    KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<NV4, 4, 8, false, 1><<<grid, 256, 0, st>>>(heads, key_dim, value_dim, bf16, gbf16, l2norm, scale, q, k, v, g, beta, state_in, state_out, o, rows_per_cta, raw, none))
     if (vec && key_dim <= 128) KDA_DECODE(1);
     else if (vec) KDA_DECODE(2);
     else KDA_DECODE(0);
@@ -2048,6 +2138,8 @@ extern "C" int kda_token_mix(int32_t n_seq, int32_t heads, float scale, const vo
                              const void* beta_logits, const void* gate, int64_t ld, const void* fb_weight, int32_t fb_dtype, const float* A_log,
                              const float* dt_bias, float lower_bound, const float* norm_weight, float eps, const float* state_in,
                              float* state_out, void* mixed, void* stream) {
+    const bool early = (fb_dtype & KDA_BEHIND_OWN_LAUNCH) != 0;
+    fb_dtype &= ~KDA_BEHIND_OWN_LAUNCH;
     if (n_seq < 0 || heads <= 0 || ld < heads) return KDA_ERR_BAD_SHAPE;
     if (n_seq == 0) return KDA_OK;
     if (!q || !k || !v || !fa || !beta_logits || !gate || !fb_weight || !A_log || !dt_bias || !norm_weight || !state_in || !state_out || !mixed)
@@ -2057,14 +2149,22 @@ extern "C" int kda_token_mix(int32_t n_seq, int32_t heads, float scale, const vo
         (reinterpret_cast<uintptr_t>(fa) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(mixed)) % 8 != 0)
         return KDA_ERR_UNSUPPORTED;
     const pw::TokenMix mix{static_cast<const __nv_bfloat16*>(fa), fb_weight, static_cast<const __nv_bfloat16*>(gate), norm_weight, ld, eps,
-                           fb_dtype == KDA_DTYPE_F32 ? 1 : 0};
+                           fb_dtype == KDA_DTYPE_F32 ? 1 : 0, n_seq};
     const pw::RawGate raw{A_log, dt_bias, lower_bound, ld};
     cudaStream_t st = (cudaStream_t)stream;
     const int blocks = n_seq * heads;
-    if (blocks <= 148)
-        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<1, 4, 32, true><<<blocks, 1024, 0, st>>>(heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits, state_in, state_out, mixed, 128, raw, mix));
-    else
-        KDA_LAUNCH("decode_kernel", st, pw::decode_kernel<1, 4, 8, true><<<blocks, 256, 0, st>>>(heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits, state_in, state_out, mixed, 128, raw, mix));
+    cudaError_t e = cudaSuccess;
+    // Blocks of 32, 16 and 8 warps go one, two and four to an SM.  Clusters are placed whole, and unevenly, so blocks that would fill the
+    // SMs just once, or by halves, are on their own (a token's three launches in us before / clusters / alone: 37 x 16 states 58.2 / 61.9 /
+    // 54.2, 28 x 16 43.7 / 39.9 / -, 48 x 12 44.0 / 46.2 / 40.1).  And blocks that start beside the projections' take the SMs these leave
+    // free, four to one and none to the next: with two to an SM in the end, where that counts, they start behind them (24 x 12 28.7 / 29.8
+    // early / 25.9, 48 x 6 28.1 / 29.7 / 26.4).
+    const int nw = blocks <= 148 ? 32 : (blocks <= 256 ? 16 : 8), cluster = nw == 16 || (blocks > 340 && blocks <= 548) || blocks > 592 ? 4 : 1;
+    const auto kern = nw == 32 ? pw::decode_kernel<1, 4, 32, true, 1>
+                               : (nw == 16 ? pw::decode_kernel<1, 4, 16, true, 4> : (cluster == 4 ? pw::decode_kernel<1, 4, 8, true, 4> : pw::decode_kernel<1, 4, 8, true, 1>));
+    KDA_LAUNCH("decode_kernel", st, e = launch_early(kern, dim3(ceil_div(blocks, cluster) * cluster), 32u * nw, 0, st, early && (blocks <= 256 || blocks > 384), cluster, heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits,
+                                                     state_in, state_out, mixed, 128, raw, mix));
+    if (e != cudaSuccess) return KDA_ERR_CUDA;
     return launch_status();
 }
 

@@ -47,17 +47,29 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 // Weights arrive through a thread-private ring in shared memory filled by 16-byte asynchronous copies, 96 KB per CTA in
 // flight and no registers held for it (register-staged loads reached 2.3 TB/s at 2,048 x 8,336 and 32 rows, 68 MB of
 // masters); x, which L2 serves, is loaded one step ahead.
-template <int RT>
-constexpr int kDepth = RT == 1 ? 6 : 3;
+// DEEP: no more CTAs than SMs and no convolution, the output projection: the ring takes 192 KB, so that up to 3,072 columns are all on
+// their way while the kernel before it still runs.
+template <int RT, bool DEEP>
+constexpr int kDepth = DEEP ? 12 : (RT == 1 ? 6 : 3);
+// Leading dimension of the partial sums: odd for the reads (lanes over rows), and 9 modulo 32 leaves two lanes at most on a bank in the
+// writes (lanes over 8 rows x 4 pairs; four lanes at 1 modulo 32).
+template <int NT>
+constexpr int kLdRed = NT >= 4 ? NT * 8 + 9 : NT * 8 + 1;
+// Steps x is loaded ahead.  With one tile of weights a CTA there are few CTAs, latency counts, and registers are there for it (output
+// projection of 32 tokens, 2,048 wide, from the end of the kernel before it: 9.0 us with one step ahead and six stages, 8.5 with two,
+// 6.4 with the deep ring as well).
+template <int RT, int NT>
+constexpr int kDepthX = RT == 2 ? 1 : (NT == 1 ? 6 : (NT == 2 ? 3 : 2));
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-template <int NT, bool F32W, bool CONV, int RT>
+template <int NT, bool F32W, bool CONV, int RT, bool DEEP>
 __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
-    constexpr int D = kDepth<RT>, PIECES = F32W ? 4 : 2, NTH = kWarps * 32, ROWS = kRows * RT, LD = NT * 8 + 1;
+    constexpr int D = kDepth<RT, DEEP>, PIECES = F32W ? 4 : 2, NTH = kWarps * 32, ROWS = kRows * RT, LD = kLdRed<NT>;
     extern __shared__ __align__(16) uint8_t smem[];
+    dependents_go();
     uint4* ring = reinterpret_cast<uint4*>(smem);                    // [D][RT][PIECES][threads]
     float* red = reinterpret_cast<float*>(smem);                     // [warps][ROWS][LD], once the ring is drained
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
@@ -91,18 +103,19 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    uint4 xb[NT];
-    auto load_x = [&](int i) {
+    constexpr int XD = kDepthX<RT, NT>;
+    uint4 xb[XD][NT];
+    auto load_x = [&](int i, uint4 (&x)[NT]) {
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            xb[t] = make_uint4(0, 0, 0, 0);
+            x[t] = make_uint4(0, 0, 0, 0);
             if (i < mine && t * 8 + g < p.m) {
                 const __nv_bfloat16* xr = p.x + (size_t)(t * 8 + g) * p.ldx + (size_t)(warp + kWarps * i) * kStep;
                 if (F32W) {
-                    const uint2 u = __ldg(reinterpret_cast<const uint2*>(xr + 4 * tig)), v = __ldg(reinterpret_cast<const uint2*>(xr + 16 + 4 * tig));
-                    xb[t] = make_uint4(u.x, u.y, v.x, v.y);
+                    const uint2 u = ld_after8(xr + 4 * tig), v = ld_after8(xr + 16 + 4 * tig);
+                    x[t] = make_uint4(u.x, u.y, v.x, v.y);
                 } else {
-                    xb[t] = __ldg(reinterpret_cast<const uint4*>(xr + 8 * tig));
+                    x[t] = ld_after16(xr + 8 * tig);
                 }
             }
         }
@@ -116,7 +129,9 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
             for (int e = 0; e < 4; ++e) acc[r][t][e] = 0.f;
 #pragma unroll
     for (int i = 0; i < D - 1; ++i) issue(i);
-    load_x(0);
+    dependency_wait();                                               // weights are nobody's output; x may be the kernel's before
+#pragma unroll
+    for (int i = 0; i < XD; ++i) load_x(i, xb[i]);
     // A thread's outputs all belong to one weight row (ROWS divides the block), so its convolution windows and weights can
     // come in now, behind the product, instead of one after another at the end (32 tokens, 16 heads: 24.0 -> 21 us).
     constexpr int NOUT = (ROWS * NT * 8 + NTH - 1) / NTH;
@@ -144,12 +159,16 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
         }
     }
 #pragma unroll 1
-    for (int i = 0; i < mine; ++i) {
+    for (int i0 = 0; i0 < mine; i0 += XD)
+#pragma unroll
+    for (int d = 0; d < XD; ++d) {
+        const int i = i0 + d;
+        if (XD > 1 && i >= mine) break;
         issue(i + D - 1);
         uint4 xc[NT];
 #pragma unroll
-        for (int t = 0; t < NT; ++t) xc[t] = xb[t];
-        load_x(i + 1);
+        for (int t = 0; t < NT; ++t) xc[t] = xb[d][t];
+        load_x(i + XD, xb[d]);
         asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
@@ -229,24 +248,25 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(RowsArgs p) {
     }
 }
 
-// 4 counts of row tiles x 2 weight types x with and without convolutions x 2 heights: one signature
-static_assert(kSmemKernels >= 4 * 2 * 2 * 2, "set_smem_limit would forget instantiations of rows_kernel");
-template <int NT, bool F32W, bool CONV, int RT>
-int launch_tile(const RowsArgs& p, cudaStream_t st) {
-    constexpr size_t ring = (size_t)kDepth<RT> * RT * (F32W ? 4 : 2) * kWarps * 32 * 16, red = (size_t)kWarps * kRows * RT * (NT * 8 + 1) * 4;
+// 4 counts of row tiles x 2 weight types x (with and without convolutions x 2 heights, deep): one signature
+static_assert(kSmemKernels >= 4 * 2 * 5, "set_smem_limit would forget instantiations of rows_kernel");
+template <int NT, bool F32W, bool CONV, int RT, bool DEEP = false>
+int launch_tile(const RowsArgs& p, bool early, cudaStream_t st) {
+    constexpr size_t ring = (size_t)kDepth<RT, DEEP> * RT * (F32W ? 4 : 2) * kWarps * 32 * 16, red = (size_t)kWarps * kRows * RT * kLdRed<NT> * 4;
     constexpr size_t bytes = ring > red ? ring : red;
-    if (set_smem_limit(rows_kernel<NT, F32W, CONV, RT>, bytes)) return KDA_ERR_CUDA;
-    KDA_LAUNCH("rows_kernel", st, rows_kernel<NT, F32W, CONV, RT><<<ceil_div(p.end[p.n_items - 1], kRows * RT), kWarps * 32, bytes, st>>>(p));
-    return launch_status();
+    if (set_smem_limit(rows_kernel<NT, F32W, CONV, RT, DEEP>, bytes)) return KDA_ERR_CUDA;
+    cudaError_t e = cudaSuccess;
+    KDA_LAUNCH("rows_kernel", st, e = launch_early(rows_kernel<NT, F32W, CONV, RT, DEEP>, dim3(ceil_div(p.end[p.n_items - 1], kRows * RT)), kWarps * 32, bytes, st, early, 1, p));
+    return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
 }
 
 template <bool F32W, bool CONV>
-int launch_rows(const RowsArgs& p, cudaStream_t st) {
+int launch_rows(const RowsArgs& p, bool early, cudaStream_t st) {
     const bool wide = p.end[p.n_items - 1] >= 148 * kRows * 2;       // at least one CTA of two tiles for every SM
-    if (p.m <= 8) return wide ? launch_tile<1, F32W, CONV, 2>(p, st) : launch_tile<1, F32W, CONV, 1>(p, st);
-    if (p.m <= 16) return wide ? launch_tile<2, F32W, CONV, 2>(p, st) : launch_tile<2, F32W, CONV, 1>(p, st);
-    if (p.m <= 32) return wide ? launch_tile<4, F32W, CONV, 2>(p, st) : launch_tile<4, F32W, CONV, 1>(p, st);
-    return wide ? launch_tile<8, F32W, CONV, 2>(p, st) : launch_tile<8, F32W, CONV, 1>(p, st);
+    const bool deep = !CONV && p.end[p.n_items - 1] <= 148 * kRows;  // one CTA of one tile at most
+#define KDA_ROWS(NT) (wide ? launch_tile<NT, F32W, CONV, 2>(p, early, st) : (!CONV && deep ? launch_tile<NT, F32W, false, 1, true>(p, early, st) : launch_tile<NT, F32W, CONV, 1>(p, early, st)))
+    return p.m <= 8 ? KDA_ROWS(1) : (p.m <= 16 ? KDA_ROWS(2) : (p.m <= 32 ? KDA_ROWS(4) : KDA_ROWS(8)));
+#undef KDA_ROWS
 }
 
 // y[m][n] for one 128-wide product (the low-rank gate projection), a warp per (row of x, weight row): the form the decode
@@ -258,7 +278,7 @@ __global__ void __launch_bounds__(256) narrow_kernel(int m, int n, const __nv_bf
     if (i >= (long long)m * n) return;
     const int lane = threadIdx.x & 31, row = (int)(i % n), mm = (int)(i / n);
     float xv[4], wv[4];
-    narrow_x(x + (size_t)mm * ldx, lane, xv);
+    narrow_x(*reinterpret_cast<const uint2*>(x + (size_t)mm * ldx + 4 * lane), xv);
     narrow_w<F32W>(w, (size_t)row * 128, lane, wv);
     const float y = narrow_sum(xv, wv);
     if (lane == 0) out[(size_t)mm * n + row] = __float2bfloat16(y);
@@ -273,6 +293,8 @@ extern "C" int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t we
                                const int32_t* rows, void* out, int64_t out_ld, const KdaTokenConv* conv, void* stream) {
     if (m < 1 || m > tok::kMaxRows || k < 1 || n_items < 1 || n_items > tok::kItems || x_ld < k) return KDA_ERR_BAD_SHAPE;
     if (!x || !weight || !rows || !out) return KDA_ERR_NULL;
+    const bool early = (weight_dtype & KDA_BEHIND_OWN_LAUNCH) != 0;
+    weight_dtype &= ~KDA_BEHIND_OWN_LAUNCH;
     if (k % tok::kStep != 0 || x_ld % 8 != 0 || (weight_dtype != KDA_DTYPE_F32 && weight_dtype != KDA_DTYPE_BF16)) return KDA_ERR_UNSUPPORTED;
     tok::RowsArgs p = {};
     p.x = static_cast<const __nv_bfloat16*>(x);
@@ -293,7 +315,7 @@ extern "C" int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t we
     if (al % 16 != 0 || out_ld < (conv ? 0 : end)) return KDA_ERR_UNSUPPORTED;
     cudaStream_t st = (cudaStream_t)stream;
     const bool f32 = weight_dtype == KDA_DTYPE_F32;
-    if (!conv) return f32 ? tok::launch_rows<true, false>(p, st) : tok::launch_rows<false, false>(p, st);
+    if (!conv) return f32 ? tok::launch_rows<true, false>(p, early, st) : tok::launch_rows<false, false>(p, early, st);
     if (n_items < 3 || rows[1] != rows[0] || rows[2] != rows[0] || conv->width < 1 || conv->width > 4 || !conv->act) return KDA_ERR_BAD_SHAPE;
     for (int i = 0; i < 3; ++i) {
         if (!conv->weight[i] || !conv->cache[i]) return KDA_ERR_NULL;
@@ -309,7 +331,7 @@ extern "C" int kda_rows_linear(int32_t m, int32_t k, int32_t n_items, int32_t we
         wal |= reinterpret_cast<uintptr_t>(conv->weight[i]);
     }
     p.conv_vec = conv->width == 4 && cal % 8 == 0 && wal % 16 == 0;
-    return f32 ? tok::launch_rows<true, true>(p, st) : tok::launch_rows<false, true>(p, st);
+    return f32 ? tok::launch_rows<true, true>(p, early, st) : tok::launch_rows<false, true>(p, early, st);
 }
 
 extern "C" int kda_narrow_linear(int32_t m, int32_t n, int32_t weight_dtype, const void* x, int64_t x_ld, const void* weight, void* out, void* stream) {

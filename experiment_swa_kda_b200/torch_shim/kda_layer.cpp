@@ -314,14 +314,14 @@ constexpr int64_t kFewRows = 64;
 
 // products of at most kFewRows rows with `count` consecutive weights of the list, straight from the parameters
 void few_rows(const std::vector<Tensor>& w, int first, int count, const Sizes& z, const void* x, int64_t ldx, int64_t k, char* out, int64_t ldo,
-              const KdaTokenConv* conv, void* st) {
+              const KdaTokenConv* conv, void* st, int32_t flags = 0) {
     const void* wp[6];
     int32_t rows[6];
     for (int i = 0; i < count; ++i) {
         wp[i] = w[first + i].data_ptr();
         rows[i] = (int32_t)w[first + i].size(0);
     }
-    must(kda_rows_linear((int32_t)z.M, (int32_t)k, count, dt(w[first]), x, ldx, wp, rows, out, ldo, conv, st), "kda_rows_linear");
+    must(kda_rows_linear((int32_t)z.M, (int32_t)k, count, dt(w[first]) | flags, x, ldx, wp, rows, out, ldo, conv, st), "kda_rows_linear");
 }
 
 using LayerResult = c10::optional<std::vector<c10::optional<Tensor>>>;
@@ -495,7 +495,7 @@ LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         cv.weight_dtype = dt(w[kCq]);
         few_rows(w, kQ, 6, z, x.data_ptr(), h, h, P, n, &cv, st);
         must(kda_token_mix((int32_t)M, (int32_t)heads, scale, q, q + act, q + 2 * act, at_col(P, z.fa()), at_col(P, z.b()), at_col(P, 3 * h), n,
-                           w[kFb].data_ptr(), dt(w[kFb]), w[kAlog].data_ptr<float>(), w[kDt].data_ptr<float>(), (float)lb, nw.data_ptr<float>(),
+                           w[kFb].data_ptr(), dt(w[kFb]) | KDA_BEHIND_OWN_LAUNCH, w[kAlog].data_ptr<float>(), w[kDt].data_ptr<float>(), (float)lb, nw.data_ptr<float>(),
                            (float)eps, state[0].data_ptr<float>(), state[0].data_ptr<float>(), mixed, st),
              "kda_token_mix");
     } else {
@@ -527,7 +527,7 @@ LayerResult token(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
                                        nw.data_ptr<float>(), mixed, tmp.f32(oinv), st),
              "kda_rmsnorm_gate_fwd_rows");
     }
-    few_rows(w, kO, 1, z, mixed, h, h, static_cast<char*>(y.data_ptr()), h, nullptr, st);
+    few_rows(w, kO, 1, z, mixed, h, h, static_cast<char*>(y.data_ptr()), h, nullptr, st, in_place ? KDA_BEHIND_OWN_LAUNCH : 0);
     return out;
 }
 

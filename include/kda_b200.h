@@ -40,6 +40,10 @@ extern "C" {
  * not; each weight is then rounded to the activation dtype as it is loaded (the result a cast of the weight tensor
  * would give) and no converted copy of the weights is needed. */
 #define KDA_WEIGHT_F32 0x100
+/* Added to the weight_dtype of kda_rows_linear or the fb_dtype of kda_token_mix: the launch before this one in the stream is one of
+ * these two calls' (of the same token), which write no weights and no memory state.  The kernel may then start beside that launch
+ * and read weights and state before it has ended. */
+#define KDA_BEHIND_OWN_LAUNCH 0x400
 /* kda_conv_bwd only: OR this into io_dtype when `dweight` is bfloat16; the float32 sums are rounded as they are written. */
 #define KDA_DWEIGHT_BF16 0x200
 

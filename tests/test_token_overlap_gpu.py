@@ -1,0 +1,62 @@
+"""A token's three launches overlap: weights, state and the gate's weights are read while the launch before still runs, and above 148
+states the blocks of four sequences form a cluster.  Many tokens in a row have to give the bits of the launches one by one."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+D0 = "cuda:0"
+
+
+def _layer(heads, seed):
+    import experiment_swa_kda_b200 as m
+    torch.manual_seed(seed)
+    layer = m.KimiDeltaAttention(hidden_size=heads * 128, num_heads=heads, head_dim=128, conv_size=4, norm_eps=1e-6).to(D0).eval()
+    with torch.no_grad():
+        for p in layer.parameters():
+            if p.dim() > 1:
+                torch.nn.init.normal_(p, std=p.shape[-1] ** -0.5)
+    return m, layer
+
+
+# one block a state up to 148 states; clusters with 0, 1, 2 and 3 sequences over; output projections of one and of two tiles a CTA
+@pytest.mark.parametrize("batch,heads", [(1, 1), (9, 16), (10, 16), (13, 12), (50, 3), (40, 4), (7, 40)])
+def test_overlapping_launches_give_the_bits_of_separate_ones(batch, heads):
+    m, layer = _layer(heads, batch)
+    x = torch.randn(24, batch, 1, heads * 128, generator=torch.Generator().manual_seed(heads)).bfloat16().to(D0)
+    a = m.KDAState.zeros(batch, heads, 128, 4, D0)
+    a.memory.normal_(generator=torch.Generator(device=D0).manual_seed(1)).mul_(0.02)
+    b = a.clone()
+    with torch.no_grad():
+        got = [layer.decode_token(t, a) for t in x]
+        want = []
+        for t in x:
+            y, b = layer(t, state=b, output_final_state=True, mode="project_recurrent")
+            want.append(y)
+    assert all(torch.equal(p, q) for p, q in zip(got, want))
+    assert torch.equal(a.memory, b.memory) and torch.equal(a.q_conv, b.q_conv) and torch.equal(a.v_conv, b.v_conv)
+
+
+@pytest.mark.parametrize("batch,heads", [(2, 3), (13, 16)])
+def test_overlapping_launches_in_a_graph(batch, heads):
+    m, layer = _layer(heads, 5)
+    xs = torch.randn(8, batch, 1, heads * 128, device=D0).bfloat16()
+    eager, state = (m.KDAState.zeros(batch, heads, 128, 4, D0) for _ in range(2))
+    x, stream, graph = xs[0].clone(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.no_grad():
+        want = [layer.decode_token(t, eager) for t in xs]
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            layer.decode_token(x, state)
+        torch.cuda.current_stream().wait_stream(stream)
+        for t in (state.memory, state.q_conv, state.k_conv, state.v_conv):
+            t.zero_()
+        with torch.cuda.graph(graph):
+            y = layer.decode_token(x, state)
+        for t in (state.memory, state.q_conv, state.k_conv, state.v_conv):
+            t.zero_()
+        for t, w in zip(xs, want):
+            x.copy_(t)
+            graph.replay()
+            assert torch.equal(y, w)
+    assert torch.equal(state.memory, eager.memory)
