@@ -125,6 +125,11 @@ __device__ __forceinline__ void st_cluster(float* p, int rank, float x) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(x) : "memory");
 }
+__device__ __forceinline__ float ld_after_f32(const float* p) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p) : "memory");
+    return r;
+}
 // The kernel after this one may start once every block has said so or ended.
 __device__ __forceinline__ void dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -75,6 +75,7 @@ __global__ void gate_bwd_kernel(int tokens, int H, int K, int bf16, const void* 
                                 const float* __restrict__ dt_bias, float lb, const float* __restrict__ dg,
                                 const float* __restrict__ dbeta, void* __restrict__ d_raw, void* __restrict__ d_bl,
                                 float* __restrict__ part_b, float* __restrict__ part_a) {
+    dependents_go();
     const int HK = H * K;
     const int t0 = blockIdx.x * kGateRows, t1 = min(tokens, t0 + kGateRows);
     for (int c = threadIdx.x; c < HK; c += blockDim.x) {
@@ -111,14 +112,15 @@ __global__ void __launch_bounds__(1024) gate_bwd_reduce_kernel(int nblk, int H, 
     __shared__ float wsum[4];
     const int h = blockIdx.x, HK = H * K;
     const int col = threadIdx.x & 127, seg = threadIdx.x >> 7;
+    dependency_wait();                     // the kernel before wrote the partial sums
     float accA = 0.f;                      // segment 0 only: this column's share of sum_k (dr * x), over all column groups
     for (int k0 = 0; k0 < K; k0 += 128) {
         const int kk = k0 + col, c = h * K + kk;
         float sb = 0.f, sa = 0.f;
         if (kk < K)
             for (int b = seg; b < nblk; b += 8) {
-                sb += part_b[(size_t)b * HK + c];
-                sa += part_a[(size_t)b * HK + c];
+                sb += ld_after_f32(part_b + (size_t)b * HK + c);
+                sa += ld_after_f32(part_a + (size_t)b * HK + c);
             }
         redb[seg][col] = sb;
         reda[seg][col] = sa;
@@ -796,6 +798,7 @@ __global__ void __launch_bounds__(256) gate_fwd4_kernel(unsigned n_thr, size_t n
                                                         const float* __restrict__ dt_bias, float lb, float* __restrict__ g,
                                                         float* __restrict__ beta) {
     const unsigned i = blockIdx.x * 256u + threadIdx.x;
+    dependents_go();
     if (i >= n_thr) return;
     constexpr size_t quad = BF16 ? 8 : 16;
     const char* rp = static_cast<const char*>(raw) + i * quad;
@@ -843,6 +846,7 @@ __global__ void __launch_bounds__(256) gate_fwd4_kernel(unsigned n_thr, size_t n
         const unsigned rows = n_thr / (unsigned)H;
         for (size_t t = (size_t)bt + rows; t < (size_t)tokens; t += rows) beta[t * H + bh] = sigmoidf_(ld_io(bl, t * bl_ld + bh, BF16));
     }
+    dependency_wait();      // not to end before a launch this one ran beside
 }
 
 // grid: x = blocks of 128 columns (lane = 4 channels), y = blocks of kGateRows tokens; warp w takes rows w, w + 8, ...
@@ -853,6 +857,7 @@ __global__ void __launch_bounds__(256) gate_bwd4_kernel(int tokens, int H, int K
                                                         const float* __restrict__ dbeta, void* __restrict__ d_raw,
                                                         void* __restrict__ d_bl, float* __restrict__ part_b,
                                                         float* __restrict__ part_a) {
+    dependents_go();
     constexpr int RPW = kGateRows / 8;
     __shared__ float red[2][8][128];
     const int HK = H * K;
@@ -964,6 +969,7 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
     const int c = (blockIdx.x * 32 + p) * VEC;
     const int item = blockIdx.z / B;
     const int t0 = (blockIdx.y * 8 + g) * kConvPairT, b = blockIdx.z - item * B;
+    dependents_go();
     if (t0 >= T) return;
     const void* __restrict__ x = pick_item(items.x, item);
     const void* __restrict__ wgt = pick_item(items.w, item);
@@ -1052,6 +1058,7 @@ __global__ void __launch_bounds__(256) conv_fwd_pair_kernel(int B, int T, int C,
             }
         }
     }
+    dependency_wait();                         // not to end before a launch this one ran beside
 }
 
 // The same for long bf16 inputs, C % 128 == 0: a thread walks down a run of tokens, 8 rows at a
@@ -1066,6 +1073,7 @@ __global__ void __launch_bounds__(256, W <= 4 ? 3 : 2) conv_fwd_stream_kernel(in
     const int p = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int c = (blockIdx.x * 32 + p) * 4;                   // C % 128 == 0: in range
     const int item = blockIdx.z / B, b = blockIdx.z - item * B;
+    dependents_go();
     if ((int)blockIdx.y == fin_row) {                          // slot s holds the input at time T - W + s
         const int t = T - W + g;
         __nv_bfloat16* fin = static_cast<__nv_bfloat16*>(pick_item(items.fin, item));
@@ -1162,6 +1170,7 @@ __global__ void __launch_bounds__(256, W <= 4 ? 3 : 2) conv_fwd_stream_kernel(in
         load(da, i + 2 * R);
         block(db, i + R);
     }
+    dependency_wait();                                         // not to end before a launch this one ran beside
 }
 
 // Backward.  blockDim = (16 channel groups, 16 time tiles).  Each thread recomputes the
@@ -1176,6 +1185,7 @@ __global__ void __launch_bounds__(256) conv_bwd_kernel(int B, int T, int C, int 
                                                        const void* __restrict__ dy, const void* __restrict__ dfin,
                                                        void* __restrict__ dx, void* __restrict__ dcache,
                                                        float* __restrict__ dw_part) {
+    dependents_go();
     __shared__ float red[16][16][W * VEC];
     const int ncg = C / VEC, ntile = (T + kConvBT - 1) / kConvBT;
     const int cg = blockIdx.x * 16 + threadIdx.x;
@@ -1363,6 +1373,7 @@ constexpr int kConvTileT = 64, kConvTileC = 64;
 template <int W, bool BF16>
 __global__ void __launch_bounds__(256) conv_bwd_tile_kernel(int B, int T, int C, int ldx, int silu, int wf32, ConvBwdItems items,
                                                             float* __restrict__ dw_part) {
+    dependents_go();
     constexpr int XR = kConvTileT + 2 * (W - 1);   // x rows  t0-(W-1) .. t0+63+(W-1)
     constexpr int GR = kConvTileT + W - 1;         // dy rows t0 .. t0+63+(W-1)
     constexpr int RPW = kConvTileT / 8;            // consecutive rows per warp
@@ -1535,6 +1546,7 @@ constexpr int kConvRingDepth = 16;
 template <int W>
 __global__ void __launch_bounds__(256, 2) conv_bwd_ring_kernel(int B, int T, int C, int ldx, int run, int silu, int wf32, ConvBwdItems items,
                                                                float* __restrict__ dw_part) {
+    dependents_go();
     constexpr int NG = kConvRingDepth / W;                     // groups of W rows in the ring
     extern __shared__ __align__(16) uint8_t ring_raw[];
     uint2* ring = reinterpret_cast<uint2*>(ring_raw);          // [NG][W][2: x | dy][256 threads]
@@ -1731,6 +1743,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(long long rows, int D,
                                                           const float* __restrict__ inv_rms, const void* __restrict__ dy,
                                                           void* __restrict__ dx, void* __restrict__ dgate,
                                                           float* __restrict__ dw_part) {
+    dependents_go();
     extern __shared__ float dws[];   // [8][D]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float* mine = dws + (size_t)wid * D;
@@ -1858,6 +1871,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd128_kernel(long long rows, int
                                                              const float* __restrict__ inv_rms, const void* __restrict__ dy,
                                                              void* __restrict__ dx, void* __restrict__ dgate,
                                                              float* __restrict__ dw_part) {
+    dependents_go();
     __shared__ float dws[8][128];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long warp0 = (long long)blockIdx.x * 8 + wid;
@@ -1936,8 +1950,9 @@ __global__ void __launch_bounds__(1024) column_sum_kernel(int nblk, int N, const
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     float a = 0.f;
+    dependency_wait();                    // the kernel before wrote the partial sums
     if (i < N)
-        for (int b = seg; b < nblk; b += 32) a += part[(size_t)b * N + i];
+        for (int b = seg; b < nblk; b += 32) a += ld_after_f32(part + (size_t)b * N + i);
     red[seg][lane] = a;
     __syncthreads();
     if (seg == 0 && i < N) {
@@ -2018,6 +2033,8 @@ extern "C" int kda_pack_bf16(int32_t n_items, int32_t src_dtype, const void* con
 extern "C" int kda_gate_fwd_rows(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
                                  const void* beta_logits, int32_t bl_ld, const float* A_log, const float* dt_bias, float lower_bound,
                             float* g_out, float* beta_out, void* stream) {
+    const bool beside = (io_dtype & KDA_BESIDE_OWN_LAUNCH) != 0;
+    io_dtype &= ~KDA_BESIDE_OWN_LAUNCH;
     if (tokens < 0 || heads <= 0 || key_dim <= 0 || bl_ld < heads) return KDA_ERR_BAD_SHAPE;
     if (tokens == 0) return KDA_OK;
     if (!raw_gate || !beta_logits || !A_log || !dt_bias || !g_out || !beta_out) return KDA_ERR_NULL;
@@ -2030,11 +2047,10 @@ extern "C" int kda_gate_fwd_rows(int32_t tokens, int32_t heads, int32_t key_dim,
     const long long n_thr = (long long)heads * key_dim / 4 * ceil_div(tokens, quads);
     if (key_dim % 4 == 0 && al && (long long)heads * key_dim < (1ll << 31) && n_thr < (1ll << 31)) {      // 2^31 threads: 137 GB of g
         const unsigned thr = (unsigned)n_thr, blocks4 = (thr + 255) / 256;
-        if (io_dtype == KDA_DTYPE_BF16)
-            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<true><<<blocks4, 256, 0, fst>>>(thr, n / 4, tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
-        else
-            KDA_LAUNCH("gate_fwd_kernel", fst, pw::gate_fwd4_kernel<false><<<blocks4, 256, 0, fst>>>(thr, n / 4, tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
-        return launch_status();
+        cudaError_t e = cudaSuccess;
+        const auto kern = io_dtype == KDA_DTYPE_BF16 ? pw::gate_fwd4_kernel<true> : pw::gate_fwd4_kernel<false>;
+        KDA_LAUNCH("gate_fwd_kernel", fst, e = launch_early(kern, dim3(blocks4), 256, 0, fst, beside, 1, thr, n / 4, tokens, heads, key_dim, raw_gate, beta_logits, bl_ld, A_log, dt_bias, lower_bound, g_out, beta_out));
+        return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
     }
     if (bl_ld != heads) return KDA_ERR_UNSUPPORTED;      // strided beta logits: the vector path only
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
@@ -2081,8 +2097,9 @@ extern "C" int kda_gate_bwd_rows(int32_t tokens, int32_t heads, int32_t key_dim,
         KDA_LAUNCH("gate_bwd_kernel", st, pw::gate_bwd_kernel<<<nblk, 256, 0, st>>>(tokens, heads, key_dim, io_dtype == KDA_DTYPE_BF16, raw_gate,
                                                   beta_logits, A_log, dt_bias, lower_bound, dg, dbeta, d_raw_gate,
                                                   d_beta_logits, part_b, part_a));
-    KDA_LAUNCH("gate_bwd_reduce_kernel", st, pw::gate_bwd_reduce_kernel<<<heads, 1024, 0, st>>>(nblk, heads, key_dim, part_b, part_a, ddt_bias, dA_log));
-    return launch_status();
+    cudaError_t e = cudaSuccess;
+    KDA_LAUNCH("gate_bwd_reduce_kernel", st, e = launch_early(pw::gate_bwd_reduce_kernel, dim3(heads), 1024, 0, st, nblk > 0, 1, nblk, heads, key_dim, part_b, part_a, ddt_bias, dA_log));
+    return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
 }
 
 extern "C" int kda_gate_bwd(int32_t tokens, int32_t heads, int32_t key_dim, int32_t io_dtype, const void* raw_gate,
@@ -2202,12 +2219,21 @@ extern "C" int kda_decode_steps(int32_t n_steps, int32_t n_seq, int32_t heads, i
 
 namespace {
 
+// Sums of the partial rows the launch before this one left: early, so that a few small blocks stand ready when its last ones end
+// (with the gap a launch of their own cost: norm 4.1 + 2.1 us behind a 8.2 us kernel, convolutions 2.3 + 2.4).
+int column_sums(const char* name, int n, int nblk, int N, const float* part, const pw::ColumnSumItems& outs, int bf16, cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    KDA_LAUNCH(name, st, e = launch_early(pw::column_sum_kernel, dim3(ceil_div(N, 32), n), 1024, 0, st, nblk > 0, 1, nblk, N, part, outs, bf16));
+    return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
+}
+
 inline bool conv_grid_ok(int n, int B, int T) { return ceil_div(T, 8 * pw::kConvPairT) <= 65535 && (long long)B * n <= 65535; }
 
 // n same-shaped convolutions in one launch; x rows ldx elements apart
 constexpr int kConvRun = 32;      // tokens per thread of the streaming forward
 template <int W>
-int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st) {
+int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int silu, const pw::ConvFwdItems& it, cudaStream_t st, bool beside = false) {
+    cudaError_t e = cudaSuccess;
     const bool vec4 = C % 128 == 0 && ldx % 4 == 0;         // channels per thread: 4 when a warp's 128 channels fill a row segment
     const dim3 grid(ceil_div(C, vec4 ? 128 : 64), ceil_div(T, 8 * pw::kConvPairT), B * n);
     bool win = false, carried = false;
@@ -2229,18 +2255,18 @@ int conv_fwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
         const bool filled = 5LL * T >= 4 * room ? blocks >= (win ? 2 * 148 : 148 * 3 / 2) : 2LL * T >= room && blocks >= 148 * 6;
         const bool copied = win && T <= 8 && blocks >= 148 * 3 / 2 && blocks <= 148 * 12;
         if ((filled || copied) && sgrid.y <= 65535) {
-            KDA_LAUNCH("conv_fwd_stream_kernel", st, pw::conv_fwd_stream_kernel<W><<<sgrid, 256, 0, st>>>(B, T, C, ldx, kConvRun, win ? runs : -1, silu, wf32, it));
-            return launch_status();
+            KDA_LAUNCH("conv_fwd_stream_kernel", st, e = launch_early(pw::conv_fwd_stream_kernel<W>, sgrid, 256, 0, st, beside, 1, B, T, C, ldx, kConvRun, win ? runs : -1, silu, wf32, it));
+            return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
         }
     }
 #define KDA_CONV_FWD(VEC, BF, WIN) \
-    KDA_LAUNCH("conv_fwd_kernel", st, pw::conv_fwd_pair_kernel<W, VEC, BF, WIN><<<grid, 256, 0, st>>>(B, T, C, ldx, silu, wf32, it))
+    KDA_LAUNCH("conv_fwd_kernel", st, e = launch_early(pw::conv_fwd_pair_kernel<W, VEC, BF, WIN>, grid, 256, 0, st, beside, 1, B, T, C, ldx, silu, wf32, it))
     if (vec4 && bf16) { if (win) KDA_CONV_FWD(4, true, true); else KDA_CONV_FWD(4, true, false); }
     else if (vec4) { if (win) KDA_CONV_FWD(4, false, true); else KDA_CONV_FWD(4, false, false); }
     else if (bf16) { if (win) KDA_CONV_FWD(2, true, true); else KDA_CONV_FWD(2, true, false); }
     else { if (win) KDA_CONV_FWD(2, false, true); else KDA_CONV_FWD(2, false, false); }
 #undef KDA_CONV_FWD
-    return launch_status();
+    return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
 }
 
 template <int W>
@@ -2261,8 +2287,7 @@ int conv_bwd_fast(int n, int B, int T, int C, int ldx, int bf16, int wf32, int s
     const int nblk = grid.y * B;                  // partial rows per item
     pw::ColumnSumItems outs = {};
     for (int i = 0; i < n; ++i) outs.out[i] = dwgt[i];
-    KDA_LAUNCH("conv_dw_reduce_kernel", st, pw::column_sum_kernel<<<dim3(ceil_div(C * W, 32), n), 1024, 0, st>>>(nblk, C * W, part, outs, dwb));
-    return launch_status();
+    return column_sums("conv_dw_reduce_kernel", n, nblk, C * W, part, outs, dwb, st);
 }
 
 template <int W>
@@ -2327,8 +2352,7 @@ int conv_bwd_w(int B, int T, int C, int bf16, int wf32, int silu, const void* x,
     const int nblk = grid.y * grid.z;
     pw::ColumnSumItems outs = {};
     outs.out[0] = dwgt;
-    KDA_LAUNCH("conv_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(C * W, 32), 1024, 0, st>>>(nblk, C * W, part, outs, dwb));
-    return launch_status();
+    return column_sums("conv_dw_reduce_kernel", 1, nblk, C * W, part, outs, dwb, st);
 }
 
 }  // namespace
@@ -2406,6 +2430,7 @@ extern "C" int kda_conv_fwd_rows(int32_t n_items, int32_t batch, int32_t seq_len
         return KDA_ERR_UNSUPPORTED;
     const int wf32 = (io_dtype & KDA_WEIGHT_F32) != 0;
     const int bf16 = (io_dtype & 0xff) == KDA_DTYPE_BF16;
+    const bool beside = (io_dtype & KDA_BESIDE_OWN_LAUNCH) != 0;
     pw::ConvFwdItems it = {};
     for (int i = 0; i < n_items; ++i) {
         if (!weight[i]) return KDA_ERR_NULL;
@@ -2415,10 +2440,10 @@ extern "C" int kda_conv_fwd_rows(int32_t n_items, int32_t batch, int32_t seq_len
     }
     cudaStream_t st = (cudaStream_t)stream;
     switch (width) {
-        case 1: return conv_fwd_fast<1>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
-        case 2: return conv_fwd_fast<2>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
-        case 3: return conv_fwd_fast<3>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
-        default: return conv_fwd_fast<4>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st);
+        case 1: return conv_fwd_fast<1>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st, beside);
+        case 2: return conv_fwd_fast<2>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st, beside);
+        case 3: return conv_fwd_fast<3>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st, beside);
+        default: return conv_fwd_fast<4>(n_items, batch, seq_len, channels, x_ld, bf16, wf32, silu, it, st, beside);
     }
 }
 
@@ -2563,10 +2588,10 @@ void rms_bwd_launch(int nb, int64_t rows, int32_t dim, int32_t io_dtype, const v
         else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<false, false, PARTS><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
     }
 }
-void rms_dw_launch(int nb, int32_t dim, const float* part, float* dweight, cudaStream_t st) {
+int rms_dw_launch(int nb, int32_t dim, const float* part, float* dweight, cudaStream_t st) {
     pw::ColumnSumItems outs = {};
     outs.out[0] = dweight;
-    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<ceil_div(dim, 32), 1024, 0, st>>>(nb, dim, part, outs, 0));
+    return column_sums("rmsnorm_dw_reduce_kernel", 1, nb, dim, part, outs, 0, st);
 }
 }  // namespace
 
@@ -2601,8 +2626,7 @@ extern "C" int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t
     else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd128_kernel<false, true><<<nb, 256, 0, st>>>(rows, heads, gate_ld, x, gate, weight, inv_rms, d_y, dx, dgate, part));
     pw::ColumnSumItems outs = {};
     outs.out[0] = dweight;
-    KDA_LAUNCH("rmsnorm_dw_reduce_kernel", st, pw::column_sum_kernel<<<4, 1024, 0, st>>>(nb, 128, part, outs, 0));
-    return launch_status();
+    return column_sums("rmsnorm_dw_reduce_kernel", 1, nb, 128, part, outs, 0, st);
 }
 
 // =============================================================================================

@@ -372,7 +372,7 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
     char *P = sl.at(kept.P), *raw = sl.at(kept.raw), *pack = sl.at(kept.pack);
     if (few) {
         few_rows(w, kQ, 6, z, x.data_ptr(), h, h, P, n, nullptr, st);
-        few_rows(w, kFb, 1, z, at_col(P, z.fa()), n, kHead, raw, h, nullptr, st);
+        few_rows(w, kFb, 1, z, at_col(P, z.fa()), n, kHead, raw, h, nullptr, st, KDA_BEHIND_OWN_LAUNCH);
     } else {
         pack_weights(w, z, pack, st);
         linear(x.data_ptr(), h, pack, h, P, n, M, n, h);
@@ -392,10 +392,12 @@ LayerResult layer(const Tensor& x_, const std::vector<Tensor>& w, int64_t heads,
         }
         const int io = KDA_DTYPE_BF16 | wflag(x, w[kCq]);
         for (int i = 0; i < 3; i += conv_step)
-            must(kda_conv_fwd_rows(conv_step, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, io, 1, xp + i, (int32_t)n, wp + i, cp + i, yp + i, fp + i, st),
+            must(kda_conv_fwd_rows(conv_step, (int32_t)z.B, (int32_t)z.T, (int32_t)h, (int32_t)z.W, i > 0 ? io | KDA_BESIDE_OWN_LAUNCH : io, 1, xp + i, (int32_t)n, wp + i,
+                                   cp + i, yp + i, fp + i, st),
                  "kda_conv_fwd_rows");
     }
-    must(kda_gate_fwd_rows((int32_t)M, (int32_t)heads, (int32_t)kHead, KDA_DTYPE_BF16, raw, at_col(P, z.b()), (int32_t)n, w[kAlog].data_ptr<float>(),
+    // beside the convolutions: neither needs the other
+    must(kda_gate_fwd_rows((int32_t)M, (int32_t)heads, (int32_t)kHead, fuse_conv ? KDA_DTYPE_BF16 : KDA_DTYPE_BF16 | KDA_BESIDE_OWN_LAUNCH, raw, at_col(P, z.b()), (int32_t)n, w[kAlog].data_ptr<float>(),
                            dt_bias.data_ptr<float>(), (float)lb, sl.f32(kept.g), sl.f32(kept.beta), st),
          "kda_gate_fwd_rows");
     KdaChunkExtras ex = {};

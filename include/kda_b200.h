@@ -44,6 +44,9 @@ extern "C" {
  * these two calls' (of the same token), which write no weights and no memory state.  The kernel may then start beside that launch
  * and read weights and state before it has ended. */
 #define KDA_BEHIND_OWN_LAUNCH 0x400
+/* Added to the io_dtype of kda_conv_fwd_rows or kda_gate_fwd_rows: the launch before this one in the stream is one of these two calls',
+ * and neither touches what the other writes.  The kernel may then run beside it; it does not end before that one has. */
+#define KDA_BESIDE_OWN_LAUNCH 0x800
 /* kda_conv_bwd only: OR this into io_dtype when `dweight` is bfloat16; the float32 sums are rounded as they are written. */
 #define KDA_DWEIGHT_BF16 0x200
 

@@ -60,3 +60,34 @@ def test_overlapping_launches_in_a_graph(batch, heads):
             graph.replay()
             assert torch.equal(y, w)
     assert torch.equal(state.memory, eager.memory)
+
+
+@pytest.mark.parametrize("batch,tokens,heads", [(1, 77, 3), (3, 64, 8), (2, 1100, 6), (1, 20, 16)])
+def test_launches_beside_one_another_give_the_bits_of_launches_one_by_one(batch, tokens, heads):
+    """Convolutions, gate activations and the sums of partial gradients overlap inside a layer call; with events between the launches
+    (launch accounting) they do not."""
+    from experiment_swa_kda_b200 import _lib
+    m, layer = _layer(heads, 9)
+    xs = torch.randn(6, batch, tokens, heads * 128, generator=torch.Generator().manual_seed(2)).bfloat16().to(D0)
+    leaves = list(layer.parameters())
+
+    def passes():
+        out = []
+        for x in xs:
+            with torch.no_grad():
+                y, st = layer(x, output_final_state=True)
+            out += [y, st.memory, st.q_conv, st.k_conv, st.v_conv]
+            x = x.clone().requires_grad_(True)
+            y, _ = layer(x)
+            out += [y, *torch.autograd.grad(y, [x, *leaves], x.detach())]
+        torch.cuda.synchronize()
+        return out
+
+    got = passes()
+    _lib.load().kda_profile_enable(1)
+    try:
+        want = passes()
+    finally:
+        _lib.profile_report()
+        _lib.load().kda_profile_enable(0)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
