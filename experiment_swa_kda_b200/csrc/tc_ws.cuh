@@ -59,13 +59,16 @@ struct NormEpilogue {
 // chain, but 48 + 176 KB more of memory traffic for every chunk of every recurrence, and three more launches each way.  So the walk
 // falls behind where there are few recurrences and many chunks.  Forward and backward in us, split / walk, by recurrences x chunks:
 // 2 x 16: 72 / 64, 2 x 32: 79 / 94, 12 x 32: 146 / 144, 12 x 128: 415 / 481, 16 x 32: 174 / 160, 16 x 128: 515 / 540, 32 x 128: 921 / 815.
+// Eight segments halve the chain again and lengthen the fix-up's by four products; worth it where the chain is long and SMs are idle (4 / 8
+// segments: 1 x 128 123 / 111, 2 x 256 266 / 228, 6 x 256 461 / 439; 6 x 128 264 / 262, 6 x 64 158 / 163, 8 x 128 306 / 309).
 // Two segments (17 to 49 recurrences, or 16 to 31 chunks, of the measured split side) are behind the walk wherever they were chosen.
 inline int scan_segments(const KdaChunkShape& sh) {
     if (sh.n_seq <= 0) return 1;
     const bool fixed = sh.seq_len > 0 && (long long)sh.n_seq * sh.seq_len == sh.tokens;
     const long long rec = (long long)sh.n_seq * sh.heads;
     const long long chunks = fixed ? (sh.seq_len + 63) / 64 : (sh.tokens / 64) / sh.n_seq;
-    return rec < 21 && chunks * (21 - rec) > 350 ? 4 : 1;      // at most 7 x 20 scan units, one to an SM
+    if (rec >= 21 || chunks * (21 - rec) <= 350) return 1;
+    return rec <= 6 && chunks >= 96 ? 8 : 4;      // 2 nseg - 1 scan units to a recurrence: at most 140, one to an SM
 }
 
 inline TcWs carve_tc(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr) {

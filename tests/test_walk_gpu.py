@@ -38,11 +38,11 @@ def test_norm_in_the_walk_equals_the_two_operators(tokens):
         assert torch.equal(a, b)
 
 
-def test_walk_and_split_scans_agree():
-    """Two recurrences of 19 whole chunks are split; with empty sequences beside them, which make the batch look like many short ones, they walk.
+@pytest.mark.parametrize("tokens", [64 * 19 + 33, 64 * 100 + 5])      # four and eight segments
+def test_walk_and_split_scans_agree(tokens):
+    """Two recurrences of 19 or more whole chunks are split; with empty sequences beside them, which make the batch look like many short ones, they walk.
     Bounds as for split scans against single chains: bf16 operands of two groupings of the same products."""
     m = _kda_mod()
-    tokens = 64 * 19 + 33
     d = O.make_inputs(1, tokens, 2, 128, 128, seed=91, with_state=True)
     gen = torch.Generator().manual_seed(4)
     do = torch.randn(1, tokens, 2, 128, generator=gen).bfloat16().to(D0)
