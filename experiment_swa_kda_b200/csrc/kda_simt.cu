@@ -12,6 +12,7 @@
 //   H' = exp(G_end) . H - (E^T W) H + E^T U        dH = exp(G_end) . dH' - (E^T W)^T dH' + (R - A W)^T dO
 // so everything but one K x K product per step is formed for all chunks side by side, and the scans carry a quarter of
 // the work they would with Z inside: at K = V = 64 and 32 chunks 303 + 533 us became 36 + 36.
+// Each kernel but the first of a pass may start while the one before it runs and waits for its end (starts_early).
 // The equations restate reference chunk_wy_forward.cu:125-405, 761-858, 940-1275, 1498-1588
 // and, for the adjoints, chunk_wy_backward.cu:2445-2562, 2818-3331, 3337-3552, 3787-3894.
 //
@@ -364,6 +365,7 @@ constexpr size_t kIntraSmem = (kIntraFloats + 64 * 3 + 8 * kHalf + 4 * kHalf) * 
 
 __global__ void __launch_bounds__(256, 3) intra_fwd_kernel(Ws w, IntraArgs p) {
     extern __shared__ __align__(16) float sm[];
+    dependents_go();
     float* tq = sm;                      // [d][i] q~
     float* tk = tq + kHalf * kLD;        // [d][i] k~
     float* src = tk + kHalf * kLD;       // four source arrays
@@ -666,6 +668,8 @@ inline size_t scan_smem(int Kp) { return (size_t)(kScanStages * kStageFloats + 1
 template <int KT>
 __global__ void __launch_bounds__(256) scan_kernel(Ws w, ScanArgs p) {
     extern __shared__ __align__(16) float sm[];
+    dependents_go();
+    dependency_wait();
     float* ring = sm;
     float4* part = reinterpret_cast<float4*>(ring + kScanStages * kStageFloats);
     float* S = reinterpret_cast<float*>(part + 16 * kPartBlock);      // [Kp][kSLD]
@@ -773,6 +777,7 @@ __global__ void __launch_bounds__(256) scan_kernel(Ws w, ScanArgs p) {
 __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, int bf16) {
     extern __shared__ __align__(16) float sm[];
     float *Wt = sm, *Rt = sm + kTile, *Bs = sm + 2 * kTile;
+    dependency_wait();
     const int slot = blockIdx.x, h = blockIdx.y, vt = blockIdx.z;
     int len, tok0;
     w.tab.span(slot, tok0, len);
@@ -823,6 +828,7 @@ __global__ void __launch_bounds__(256) out_kernel(Ws w, void* __restrict__ o, in
 __global__ void __launch_bounds__(256) adjoint_term_kernel(Ws w, Scr s, const void* __restrict__ d_o, int bf16, int vec_v) {
     extern __shared__ __align__(16) float sm[];
     const int slot = blockIdx.x, h = blockIdx.y, VT = w.Vp / 64, kt = blockIdx.z / VT, vt = blockIdx.z % VT;
+    dependents_go();
     int len, tok0;
     w.tab.span(slot, tok0, len);
     if (len == 0) return;
@@ -854,6 +860,7 @@ template <bool ONE>
 __global__ void __launch_bounds__(256, 2) local_bwd_kernel(Ws w, Scr s, LocalArgs p) {
     extern __shared__ __align__(16) float sm[];
     float *t0 = sm, *t1 = sm + kTile, *t2 = sm + 2 * kTile, *t3 = sm + 3 * kTile, *t4 = sm + 4 * kTile, *t5 = sm + 5 * kTile;
+    dependency_wait();
     float* bet = sm + 6 * kTile;         // [64] beta, inverse norms
     float* qi_s = bet + 64;
     float* ki_s = qi_s + 64;
@@ -1372,14 +1379,19 @@ static int set_smem(Kern kern, size_t bytes) {
 // four-element accesses along a tensor's last dimension are aligned
 static int vec4(const void* p, int dim) { return dim % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
+// Whether a kernel starts beside the one before it: with at most one chunk-head to an SM.  More blocks, placed while that one still
+// holds some SMs, crowd onto the others (8 chunk-heads forward and backward 127.1 -> 123.1 us, 384 378.9 -> 389.8).
+static bool starts_early(const Ws& w) { return w.nslots > 0 && w.nslots * (long long)w.H <= 148; }
+
 static int launch_scan(const Ws& w, int n_seq, const simt::ScanArgs& a, const char* name, cudaStream_t st) {
     const size_t bytes = simt::scan_smem(w.Kp);
     // padding strips hold zeros already: E^T U and Rm^T dO of zero columns
     const dim3 grid(n_seq, w.H, ceil_div(w.V, simt::kVS));
+    cudaError_t e = cudaSuccess;
 #define KDA_SCAN(KT)                                                                                              \
     case KT:                                                                                                      \
         if (set_smem(simt::scan_kernel<KT>, bytes)) return KDA_ERR_CUDA;                                          \
-        KDA_LAUNCH(name, st, simt::scan_kernel<KT><<<grid, 256, bytes, st>>>(w, a));                               \
+        KDA_LAUNCH(name, st, e = launch_early(simt::scan_kernel<KT>, grid, 256, bytes, st, starts_early(w), 1, w, a));     \
         break
     switch (w.Kp / 64) {
         KDA_SCAN(1);
@@ -1389,7 +1401,7 @@ static int launch_scan(const Ws& w, int n_seq, const simt::ScanArgs& a, const ch
         default: return KDA_ERR_BAD_SHAPE;
     }
 #undef KDA_SCAN
-    return launch_status();
+    return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
 }
 
 static int chunk_table(const KdaChunkShape* sh, const Ws& w, const int32_t* cu, cudaStream_t st) {
@@ -1434,7 +1446,9 @@ int simt_chunk_fwd(const KdaChunkShape* sh, const void* q, const void* k, const 
     if (w.nslots > 0) {
         const size_t sm_out = (size_t)3 * simt::kTile * sizeof(float);
         if (set_smem(simt::out_kernel, sm_out)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("out_kernel", st, simt::out_kernel<<<dim3(w.nslots, w.H, VT), 256, sm_out, st>>>(w, o, bf16));
+        cudaError_t e = cudaSuccess;
+        KDA_LAUNCH("out_kernel", st, e = launch_early(simt::out_kernel, dim3(w.nslots, w.H, VT), 256, sm_out, st, starts_early(w), 1, w, o, bf16));
+        if (e != cudaSuccess) return KDA_ERR_CUDA;
     }
     return launch_status();
 }
@@ -1497,7 +1511,9 @@ int simt_chunk_bwd(const KdaChunkShape* sh, const void* q, const void* k, const 
                                 vec4(q, sh->key_dim) && vec4(k, sh->key_dim), vec_v, sh->scale};
         const auto kern = KT == 1 && w.Vp == 64 ? simt::local_bwd_kernel<true> : simt::local_bwd_kernel<false>;
         if (set_smem(kern, simt::kLocalSmem)) return KDA_ERR_CUDA;
-        KDA_LAUNCH("local_bwd_kernel", st, kern<<<dim3(w.nslots, w.H), 256, simt::kLocalSmem, st>>>(w, s, a));
+        cudaError_t e = cudaSuccess;
+        KDA_LAUNCH("local_bwd_kernel", st, e = launch_early(kern, dim3(w.nslots, w.H), 256, simt::kLocalSmem, st, starts_early(w), 1, w, s, a));
+        if (e != cudaSuccess) return KDA_ERR_CUDA;
     }
     return launch_status();
 }
