@@ -36,7 +36,7 @@ CHAIN = dict(B=2, T=4096, H=3, D=128, W=4, eps=1e-6)
 # ----------------------------------------------------------------------------------------------
 # algorithmic work (multiply-adds at triangular cost, no recompute), per 64-token chunk and head
 # ----------------------------------------------------------------------------------------------
-def kda_kernel_flops(K, V, C=64):
+def kda_kernel_flops(K, V, C=64, split_scans=True):
     tri, stri = C * (C + 1) // 2, C * (C - 1) // 2
     fwd = {
         "build_am_kernel": tri * K + stri * K + C ** 3 / 6,
@@ -49,7 +49,7 @@ def kda_kernel_flops(K, V, C=64):
     bwd["bwd_local_kernel"] = 2 * fwd_total - sum(bwd.values())
     tcl = {   # tensor-core lane kernels: the multiply-adds each one actually performs (different kernel boundaries and
         # a regrouped recurrence, so the parts do not add up to the reference-algorithm total below)
-        "tc_intra_fwd_kernel": fwd["build_am_kernel"] + fwd["uw_kernel"] + C * K * K + C * C * K,   # + the chunk transition
+        "tc_intra_fwd_kernel": fwd["build_am_kernel"] + fwd["uw_kernel"] + (C * K * K + C * C * K if split_scans else 0),   # the chunk transition
         "tc_affine_scan_fwd_kernel": K * K * V + C * K * V,
         "tc_chunk_out_kernel": 2 * C * K * V + C * C * V,
         "tc_affine_scan_bwd_kernel": K * K * V + C * K * V,

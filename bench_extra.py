@@ -97,7 +97,7 @@ def run_varlen(args, rank, world, local, dist):
         return None
     peaks, src = _peaks()
     nch = sum((n + 63) // 64 for n in lens) * Hl
-    flops = kda_kernel_flops(D, D)
+    flops = kda_kernel_flops(D, D, split_scans="tc_scan_fixup_kernel" in rep)
     tot = sum(v[1] for v in rep.values()) or 1.0
     kern = {}
     for name, (n, tms) in rep.items():
