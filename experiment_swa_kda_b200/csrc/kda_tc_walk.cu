@@ -1,7 +1,7 @@
 // Tensor-core lane (K = V = 128): a recurrence and everything it feeds, in one walk over its chunks.
 //
 // Forward, from the intra-chunk panels of a chunk and its incoming state H:
-//     Z = U - W H        O = R H + A Z        H' = e^{G_end} . H + E^T Z
+//     Z = U - W H        O = R H + A Z        H' = e^{G_end} . H + E^T U - E^T (W H)
 // Backward, with the adjoint H' of the chunk's outgoing state, last chunk first:
 //     dZ = A^T dO + E H'        adjoint of H = e^{G_end} . H' + R^T dO - W^T dZ
 // What the backward reads of the forward (H, Z) and the intra-chunk backward of this one (H', dZ) leaves on the way.  Split scans
@@ -49,6 +49,9 @@ __device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t* w) {
 }
 __device__ __forceinline__ void stsm4(uint32_t addr, const uint32_t* w) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+__device__ __forceinline__ void stsm4_t(uint32_t addr, const uint32_t* w) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
 // A barrier of four output warps: they go on together or not at all.
 __device__ __forceinline__ bool output_sync(int id, bool ok) {
@@ -121,16 +124,21 @@ constexpr int kWkFwdThreads = (kWkState + 12) * 32, kWkBwdThreads = (kWkState + 
 // specialised by warp and meet only through mbarriers:
 //   state warps (8)     own the state in registers (thread: key row, 32 columns), form Z and the next state
 //   next warp           one lane issues the TMA loads, as far ahead as the two stages allow
-//   next warp           one lane issues the products: W H (backward: E H'), R H beside it; E^T Z (W^T dZ), A Z beside it
+//   next warp           one lane issues the products: W H (backward: E H'), R H beside it; E^T (W H) (W^T dZ), A Z beside it
 //   next warp           one lane stores the panels
 //   next warp           forward with the norm: one lane loads the gate's tiles
 //   output warps (2x4)  forward: read every other chunk's output out, normalise it if asked, store it
-// Backward: the terms of the next step without the state, A^T dO and R^T dO, are issued behind this step's last product.
+// The terms of the next step without the state, E^T U (backward: A^T dO and R^T dO), are issued behind this step's last product.
+// Why not E^T Z in one product: U is in bf16 already, and Z = U - W H would be rounded a second time on its way into the sum that the state
+// is.  The final state was then 1.08 to 1.20 times as far from float64 as that of split scans, which have E^T U and H Pn apart as well; now
+// 1.00.  W H takes U's place in the stage, piece by piece where a warp has read U.  The price is a product and 8 KB more a step that shared
+// memory has to find time for, and operands that are wanted earlier: 1.17 -> 1.39 us with 32 recurrences of 128 chunks, 381 -> 406 us below.
+// (E^T Z and E^T times what rounding took from Z: 1.45; E^T U between W H and R H: 1.43.)
 // The norm needs whole rows: the two blocks of a recurrence are a cluster then and swap their sums of squares, warp by warp.
 // Many recurrences: bound by the bytes of the panels, 136 KB a chunk-head forward and 120 backward (16,544 chunk-heads in 352
-// recurrences: 373 and 327 us, 0.93 of the copy rate; scan and output kernel took 268 + 310 us, scan and dZ kernel 262 + 219, and the
-// intra-chunk forward, which formed the scans' maps, 966 instead of 798).  Few: a step of about 2,150 cycles forward and 1,840 backward,
-// of which the products' operands, the loads and the stores keep shared memory busy for 1,800 (a product reads A and B at 128 bytes a
+// recurrences: 406 and 337 us, 0.85 and 0.91 of the copy rate; scan and output kernel took 258 + 305 us, scan and dZ kernel 254 + 219, and the
+// intra-chunk forward, which formed the scans' maps, 915 instead of 801).  Few: a step of about 2,600 cycles forward and 1,840 backward,
+// of which the products' operands, the loads and the stores keep shared memory busy for 2,050 and 1,800 (a product reads A and B at 128 bytes a
 // cycle, no faster than it multiplies them); what a step waits for besides is the way from a product's end to the next one's start, twice.
 // Whatever can be there early is therefore looked for while a product runs, a lane that issues products commits three times a step, and
 // two sets of output warps have two steps each.  Sixteen state warps of 16 columns were no faster (2,010 backward); four output warps
@@ -180,7 +188,8 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
         mbar_fence_init();
         abort_flag = 0;
     }
-    if (warp == 1) tmem_alloc(&tmem_slot, 256);
+    constexpr uint32_t kTmemCols = kBwd ? 256 : 512;      // 192, 320 in use
+    if (warp == 1) tmem_alloc(&tmem_slot, kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -190,7 +199,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
     }
     const uint32_t tmem = tmem_slot;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    constexpr uint32_t c1 = 0, c2 = 64, c3 = 128;      // accumulators: W H (M = 64); next state (backward: two); forward: output (M = 64, two)
+    constexpr uint32_t c1 = 0, c2 = 64, c3 = 192;      // accumulators: W H (M = 64); next state (two); forward: output (M = 64, two)
     auto ph = [](int c) { return (uint32_t)(c >> 1) & 1u; };      // parity of step c's phase of a barrier with two buffers
     auto ph3 = [](int c) { return (uint32_t)(c / 3) & 1u; };      // ... with three
 
@@ -233,7 +242,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             for (; c < n && ok; ++c) {
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    const int g = kBwd ? i : (i == 0 ? 0 : 3 - i);      // in the order in which they are needed
+                    const int g = kBwd ? i : 2 - i;      // in the order in which they are needed
                     if (ok && c > 1 && (i == 0 || (kBwd && i == 2))) ok = mbar_wait(bar_free(g, c & 1), ph(c - 2), p.status, 100);
                     if (ok) load(c, g);
                 }
@@ -269,11 +278,18 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             const uint32_t s0 = smem_u32(sm) & 0x3ffffu;
             constexpr uint32_t id64_mn_mn = umma_idesc_bf16(64, 64, kMajorMN, kMajorMN), id64_k_mn = umma_idesc_bf16(64, 64, kMajorK, kMajorMN);
             constexpr uint32_t id128_mn_mn = umma_idesc_bf16(128, 64, kMajorMN, kMajorMN), id128n_k_mn = umma_idesc_bf16(128, 64, kMajorK, kMajorMN, 1);
+            constexpr uint32_t id128_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK), id128n_mn_k = umma_idesc_bf16(128, 64, kMajorMN, kMajorK, 1);
             // a tile [rows][64] whose rows are the contraction index; with several blocks of 64 columns these are `blk` bytes apart
             auto mn = [](uint32_t a) { return umma_smem_desc_sw128(a, 8192, 1024); };
             auto km = [](uint32_t a) { return umma_smem_desc_sw128(a, 16, 1024); };
-            auto early = [&](int c) {      // backward: the terms of step c without the state
+            auto early = [&](int c) {      // the terms of step c without the state
                 const uint32_t st = s0 + (c & 1) * kWkStage;
+                if (!kBwd) {
+#pragma unroll
+                    for (int k16 = 0; k16 < 4; ++k16)     // E^T U
+                        umma_bf16_ss(tmem + c2 + 64 * (c & 1), mn(st + kWkE) + (k16 * 2048), km(st + kWkU) + (k16 * 32), id128_mn_k, k16 > 0);
+                    return;
+                }
 #pragma unroll
                 for (int k16 = 0; k16 < 4; ++k16)     // A^T dO
                     umma_bf16_ss(tmem + c1, km(st + kWkA) + (k16 * 32), mn(st + kWkU) + (k16 * 2048), id64_k_mn, k16 > 0);
@@ -286,7 +302,8 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
                 ok = ok && mbar_wait(b, parity, p.status, code);
                 return ok;
             };
-            if (kBwd && wait(bar_full(0, 0), 0, 103)) {
+            auto early_full = [&](int c) { return kBwd ? wait(bar_full(0, c & 1), ph(c), 103) : wait(bar_full(1, c & 1), ph(c), 103) && wait(bar_full(2, c & 1), ph(c), 103); };
+            if (early_full(0)) {
                 tc_fence_after();
                 early(0);
             }
@@ -306,11 +323,11 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
 #pragma unroll
                     for (int k16 = 0; k16 < 8; ++k16)     // R H
                         umma_bf16_ss(tmem + c3 + 64 * s, km(st + kWkR) + ((k16 >> 2) * 8192 + (k16 & 3) * 32), mn(hs) + (k16 * 2048), id64_k_mn, k16 > 0);
-                    if (!wait(bar_full(1, s), ph(c), 104) || !wait(&bar_z[s], ph(c), 107)) break;
+                    if (!wait(&bar_z[s], ph(c), 107)) break;
                     tc_fence_after();
 #pragma unroll
-                    for (int k16 = 0; k16 < 4; ++k16)     // E^T Z
-                        umma_bf16_ss(tmem + c2, mn(st + kWkE) + (k16 * 2048), mn(zs) + (k16 * 2048), id128_mn_mn, k16 > 0);
+                    for (int k16 = 0; k16 < 4; ++k16)     // - E^T (W H), which lies where U did
+                        umma_bf16_ss(tmem + c2 + 64 * s, mn(st + kWkE) + (k16 * 2048), km(st + kWkU) + (k16 * 32), id128n_mn_k, 1);
                     umma_commit(&bar_m2[s]);
 #pragma unroll
                     for (int k16 = 0; k16 < 4; ++k16)     // + A Z
@@ -327,11 +344,11 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
                     for (int k16 = 0; k16 < 4; ++k16)     // - W^T dZ
                         umma_bf16_ss(tmem + c2 + 64 * s, km(st + kWkW) + (k16 * 32), mn(zs) + (k16 * 2048), id128n_k_mn, 1);
                     umma_commit(&bar_m2[s]);
-                    if (c + 1 < n) {      // dZ's accumulator has been read, the other state accumulator was read a step ago
-                        if (!wait(bar_full(0, s ^ 1), ph(c + 1), 103)) break;
-                        tc_fence_after();
-                        early(c + 1);
-                    }
+                }
+                if (c + 1 < n) {      // the other state accumulator was read a step ago (backward: and dZ's has been)
+                    if (!early_full(c + 1)) break;
+                    tc_fence_after();
+                    early(c + 1);
                 }
             }
             if (!ok) abort_flag = 1;
@@ -522,16 +539,18 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             ok = mbar_wait(bar_full(2, st), ph(c), p.status, 115);
             constexpr int kPieces = kWkCols / 8;   // 8-column pieces a warp: [2i + a] columns kWkCols hf + 8i + 2(l%4) + {0, 1}, tokens 16q + l/4 + 8a
             uint32_t zw[2 * kPieces];
+            // U^T lies value by value: this lane's address of pieces 2m, 2m + 1 of what its warp owns
+            auto u_at = [&](int m) { return s0 + st * kWkStage + kWkU + sw128_off(kWkCols * hf + 8 * (2 * m + (mi >> 1)) + mr, 2 * q + (mi & 1)); };
             if (!kBwd && ok) {
 #pragma unroll
-                for (int m = 0; m < kPieces / 2; ++m)        // U^T lies value by value
-                    ldsm4_t(s0 + st * kWkStage + kWkU + sw128_off(kWkCols * hf + 8 * (2 * m + (mi >> 1)) + mr, 2 * q + (mi & 1)), zw + 4 * m);
+                for (int m = 0; m < kPieces / 2; ++m) ldsm4_t(u_at(m), zw + 4 * m);
             }
             const f2 dec = f2_all(dec_ring[c & 3][k]);
             if (p.keep && c > 1) ok = ok && mbar_wait(&bar_zout[st], ph(c - 2), p.status, 117);
             ok = ok && mbar_wait(&bar_m1[st], ph(c), p.status, 116);
             if (!ok) break;
             tc_fence_after();
+            uint32_t wh[2 * kPieces];
             {
                 uint32_t r[4 * kPieces];
                 tmem_ld_16(tmem + lane_base + c1 + kWkCols * hf, r);
@@ -539,12 +558,15 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
 #pragma unroll
                 for (int i = 0; i < 2 * kPieces; ++i) {
                     const f2 x = f2_make(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                    if (!kBwd) wh[i] = f2_to_bf16(x);
                     zw[i] = f2_to_bf16(kBwd ? x : f2_fma(x, f2_all(-1.f), f2_from_bf16(zw[i])));
                 }
             }
 #pragma unroll
-            for (int m = 0; m < kPieces / 2; ++m)
+            for (int m = 0; m < kPieces / 2; ++m) {
                 stsm4(s0 + kWkZ + st * 8192 + sw128_off(16 * q + 8 * (mi & 1) + mr, kPieces * hf + 2 * m + (mi >> 1)), zw + 4 * m);
+                if (!kBwd) stsm4_t(u_at(m), wh + 4 * m);      // over U: its product came before W H, and this warp alone has read these pieces
+            }
             fence_async_smem();
             tc_fence_before();
             warp_arrive(&bar_z[st], lane);
@@ -554,7 +576,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             tc_fence_after();
             {
                 uint32_t r[kWkCols];
-                tmem_ld_cols(tmem + lane_base + c2 + (kBwd ? 64 * st : 0) + kWkCols * hf, r);
+                tmem_ld_cols(tmem + lane_base + c2 + 64 * st + kWkCols * hf, r);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < kWkCols / 2; ++j) s[j] = f2_fma(dec, s[j], f2_make(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])));
@@ -574,7 +596,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
     __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, 256);
+    if (warp == 1) tmem_dealloc(tmem, kTmemCols);
     if (norm) {      // the other block may still be writing its sums into this one
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

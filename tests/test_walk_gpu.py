@@ -60,3 +60,57 @@ def test_walk_and_split_scans_agree(tokens):
     assert not torch.equal(res[0][0], res[1][0])            # two kernels, not one
     for a, b in zip(*res):
         assert O.rel_l2(a.float(), b.float()) <= 6e-3
+
+
+@pytest.mark.parametrize("tokens", [64, 37])
+def test_a_small_initial_state_passes_through_a_walk(tokens):
+    """The final state is linear in the initial one.  One 2^-7 as large as the values moves the token updates Z = U - W H by about their bf16
+    rounding, so a walk that gave the state its rounded Z loses 0.35 and 0.21 of it.  What is left are bf16 W, E and H, each within
+    2^-9 of itself, and what two roundings leave of Z, 2^-17 of it against the 2^-7: under 1e-2 together."""
+    m = _kda_mod()
+    d = {n: t.bfloat16().to(D0) for n, t in O.make_inputs(2, tokens, 12, 128, 128, seed=91).items()}
+    h0 = 2.0 ** -7 * torch.randn(2, 12, 128, 128, generator=torch.Generator().manual_seed(6)).to(D0)
+    x = [d[n] for n in ("q", "k", "v", "g", "beta")]
+    states = [m.chunk_kda(*x, initial_state=h, output_final_state=True, lane="tc")[1].double() for h in (h0, torch.zeros_like(h0))]
+    y = [t.double() for t in x]
+    want = O.kda_recurrence(y[0], y[1], torch.zeros_like(y[2]), y[3], y[4], initial_state=h0.double(), compute_dtype=torch.float64)[1]
+    assert O.rel_l2(states[0] - states[1], want) <= 1e-2
+
+
+@pytest.mark.parametrize("tokens", [64 * 19 + 33, 64 * 36])
+def test_a_walk_is_as_close_to_float64_as_split_scans(tokens):
+    """Two recurrences are split, with empty sequences beside them they walk: outputs, final state and the gradients of values and initial state
+    (the ones the recurrence alone makes) are no further from a float64 recurrence, 3 % for the luck of one draw aside."""
+    m = _kda_mod()
+    d = O.make_inputs(1, tokens, 2, 128, 128, seed=92, with_state=True)
+    gen = torch.Generator().manual_seed(4)
+    do = torch.randn(1, tokens, 2, 128, generator=gen).bfloat16().to(D0)
+    ds = torch.randn(1, 2, 128, 128, generator=gen).to(D0)
+    x = {n: (t.float() if n == "h0" else t.bfloat16()).to(D0) for n, t in d.items()}
+    y = {n: t.double().requires_grad_(True) for n, t in x.items()}
+    eo, es = O.kda_recurrence(y["q"], y["k"], y["v"], y["g"], y["beta"], initial_state=y["h0"], compute_dtype=torch.float64)
+    want = [eo, es, *torch.autograd.grad((eo, es), [y["v"], y["h0"]], (do.double(), ds.double()))]
+    errs = []
+    for empty in (0, 5):
+        x["h0"] = torch.cat([x["h0"][:1].detach(), torch.ones(empty, 2, 128, 128, device=D0)])
+        z = {n: t.detach().requires_grad_(True) for n, t in x.items()}
+        cu = torch.tensor([0] + [tokens] * (empty + 1), dtype=torch.int32, device=D0)
+        o, s = m.chunk_kda(z["q"], z["k"], z["v"], z["g"], z["beta"], initial_state=z["h0"], output_final_state=True, cu_seqlens=cu, lane="tc")
+        dv, dh = torch.autograd.grad((o, s), [z["v"], z["h0"]], (do, torch.cat([ds, torch.ones(empty, 2, 128, 128, device=D0)])))
+        errs.append([O.rel_l2(a.double(), b.detach()) for a, b in zip((o, s[:1], dv, dh[:1]), want)])
+    for split, walk in zip(*errs):
+        assert walk <= 1.03 * split, errs
+
+
+def test_an_infinite_value_spoils_its_own_column():
+    m = _kda_mod()
+    d = {n: t.bfloat16().to(D0) for n, t in O.make_inputs(2, 200, 12, 128, 128, seed=93).items()}
+    states = []
+    for infinite in (False, True):
+        v = d["v"].clone()
+        if infinite:
+            v[1, 70, 3, 17] = float("inf")
+        states.append(m.chunk_kda(d["q"], d["k"], v, d["g"], d["beta"], output_final_state=True, lane="tc")[1])
+    assert not states[1][1, 3, 17].isfinite().any()
+    states[1][1, 3, 17] = states[0][1, 3, 17]
+    assert torch.equal(*states)
