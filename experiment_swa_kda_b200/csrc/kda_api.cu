@@ -119,7 +119,7 @@ extern "C" int kda_chunk_fwd_ex(const KdaChunkShape* shape, const KdaChunkExtras
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0 || workspace_bytes < kda_chunk_workspace_bytes(shape))
         return KDA_ERR_WORKSPACE;
     const int64_t hk = (int64_t)shape->heads * shape->key_dim, gate_ld = ex->gate_ld ? ex->gate_ld : hk, x_ld = ex->x_ld ? ex->x_ld : hk;
-    // the norm's epilogue writes o in 8-byte pieces
+    // the epilogues with the norm write o in 8-byte pieces where it does not start on 16
     if (off16({q, k, v, g, h0, final_state}) || reinterpret_cast<uintptr_t>(o) % (norm ? 8 : 16) != 0) return KDA_ERR_UNSUPPORTED;
     if (norm && (gate_ld < hk || gate_ld % 8 != 0 || off16({ex->gate, ex->y, ex->norm_weight}))) return KDA_ERR_UNSUPPORTED;
     if (conv && (x_ld < hk || x_ld % 8 != 0 || off16({ex->conv_weight[0], ex->conv_weight[1], ex->conv_weight[2]}))) return KDA_ERR_UNSUPPORTED;

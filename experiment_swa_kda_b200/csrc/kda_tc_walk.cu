@@ -96,6 +96,7 @@ struct WalkArgs {
     const float* s_in;        // V-first initial state (forward: h0, backward: cotangent of the final state), or null
     float* s_out;             // V-first final state of the walk (forward: final state, backward: dh0), or null
     __nv_bfloat16* o;         // forward: [tokens][H][128]; nullptr with the norm's epilogue when only y is wanted
+    int o_map;                // o starts on 16 bytes and is stored through its map; with the norm it may start on 8
     int H;
     int keep;                 // 1: the states and Z go to their panels (a backward follows, or this is one)
     int* status;
@@ -489,21 +490,26 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             fence_async_smem();
             ok = output_sync(1 + set, ok);
             if (!ok) break;
-            if (len == 64) {
-                if (lead && elect_one()) {
-                    if (p.o != nullptr) tma_store_2d(&mO, sm + kWkO + set * 8192, h * 128 + half * 64, tok0);
-                    if (norm) tma_store_2d(&mY, sm + kWkG + c % 3 * 8192, h * 128 + half * 64, tok0);
-                    tma_store_commit();
-                    tma_store_wait_read();
-                    if (norm) mbar_arrive(&bar_gf[c % 3]);
-                }
-                __syncwarp();
-            } else {      // the sequence's last chunk: the rows past a ragged tail are another sequence's
+            // The sequence's last chunk goes out row by row: those past a ragged tail are another sequence's.
+            const bool whole = len == 64, o_rows = p.o != nullptr && !(whole && p.o_map);
+            if (whole && lead && elect_one()) {
+                if (p.o != nullptr && p.o_map) tma_store_2d(&mO, sm + kWkO + set * 8192, h * 128 + half * 64, tok0);
+                if (norm) tma_store_2d(&mY, sm + kWkG + c % 3 * 8192, h * 128 + half * 64, tok0);
+                tma_store_commit();
+                tma_store_wait_read();
+                if (norm) mbar_arrive(&bar_gf[c % 3]);
+            }
+            __syncwarp();
+            if (!whole || o_rows) {
                 for (int i = (tid & 127) >> 3; i < len; i += 16) {
                     const size_t at = ((size_t)(tok0 + i) * H + h) * 128 + half * 64 + 8 * (tid & 7);
                     const uint32_t off = sw128_off(i, tid & 7);
-                    if (p.o != nullptr) *reinterpret_cast<uint4*>(p.o + at) = *reinterpret_cast<const uint4*>(sm + kWkO + set * 8192 + off);
-                    if (norm) *reinterpret_cast<uint4*>(p.norm.y + at) = *reinterpret_cast<const uint4*>(sm + kWkG + c % 3 * 8192 + off);
+                    if (o_rows) {
+                        const uint2* x = reinterpret_cast<const uint2*>(sm + kWkO + set * 8192 + off);
+                        reinterpret_cast<uint2*>(p.o + at)[0] = x[0];
+                        reinterpret_cast<uint2*>(p.o + at)[1] = x[1];
+                    }
+                    if (norm && !whole) *reinterpret_cast<uint4*>(p.norm.y + at) = *reinterpret_cast<const uint4*>(sm + kWkG + c % 3 * 8192 + off);
                 }
             }
         }
@@ -642,14 +648,15 @@ int tc_walk_forward(const simt::Ws& w, const tc::TcWs& t, int n_seq, int tokens,
         rc |= make_map_bf16(&mS, t.Hp, nch * 128, 128, 64, 128);
         rc |= make_map_bf16(&mZ, t.ZT, nch * 64, 128, 64, 64);
     }
-    if (o != nullptr) rc |= make_map_bf16(&mO, o, (uint64_t)tokens, cols, 64, 64);
+    const bool o_map = o != nullptr && reinterpret_cast<uintptr_t>(o) % 16 == 0;
+    if (o_map) rc |= make_map_bf16(&mO, o, (uint64_t)tokens, cols, 64, 64);
     if (norm.gate != nullptr) {
         rc |= make_map_bf16(&mY, norm.y, (uint64_t)tokens, cols, 64, 64);
         rc |= make_map_bf16_ld(&mG, norm.gate, (uint64_t)tokens, cols, (uint64_t)norm.gate_ld, 64, 64);
     }
     if (rc) return KDA_ERR_CUDA;
     WalkArgs a;
-    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = h0; a.s_out = final_state; a.o = static_cast<__nv_bfloat16*>(o); a.H = w.H;
+    a.tab = w.tab; a.decay_end = t.decay_end; a.s_in = h0; a.s_out = final_state; a.o = static_cast<__nv_bfloat16*>(o); a.o_map = o_map; a.H = w.H; a.next = nullptr;
     a.keep = !t.fwd_only; a.status = t.status; a.norm = norm;
     return launch_walk<false>(2u * (unsigned)n_seq * (unsigned)w.H, norm.gate != nullptr, mW, mR, mE, mA, mU, mS, mZ, mO, mY, mG, a, st);
 }

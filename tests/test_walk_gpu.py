@@ -114,3 +114,30 @@ def test_an_infinite_value_spoils_its_own_column():
     assert not states[1][1, 3, 17].isfinite().any()
     states[1][1, 3, 17] = states[0][1, 3, 17]
     assert torch.equal(*states)
+
+
+@pytest.mark.parametrize("batch,tokens,path", [(2, 200, "tc_walk_fwd_kernel"), (1, 64 * 36 + 9, "tc_chunk_out_kernel")])
+def test_output_of_the_norms_forward_at_an_8_byte_address(batch, tokens, path):
+    """kda_chunk_fwd_norm takes an o that starts on 8 bytes, by a walk as by split scans."""
+    from experiment_swa_kda_b200 import _lib, ops
+    lib, H = _lib.load(), 2
+    d = {n: t.bfloat16().to(D0) for n, t in O.make_inputs(batch, tokens, H, 128, 128, seed=94).items()}
+    gate, w = torch.randn_like(d["v"]), torch.ones(128, device=D0)
+    sh = _lib.ChunkShape(batch, tokens, batch * tokens, H, 128, 128, _lib.DTYPE_BF16, _lib.DTYPE_BF16, _lib.LANE_TC, 1, 0.1)
+    ws = torch.empty(lib.kda_chunk_workspace_bytes(sh), dtype=torch.uint8, device=D0)
+    stream = torch.cuda.current_stream().cuda_stream
+    results = []
+    for shift in (0, 4):
+        o = torch.zeros(d["v"].numel() + 8, dtype=torch.bfloat16, device=D0)
+        y, inv = torch.zeros_like(d["v"]), torch.zeros(batch * tokens * H, device=D0)
+        lib.kda_profile_enable(1)
+        try:
+            rc = lib.kda_chunk_fwd_norm(sh, *(d[n].data_ptr() for n in ("q", "k", "v", "g", "beta")), None, None, o.data_ptr() + 2 * shift, None,
+                                        ws.data_ptr(), ws.numel(), gate.data_ptr(), w.data_ptr(), 1e-6, y.data_ptr(), inv.data_ptr(), stream)
+            _lib.check(rc, "kda_chunk_fwd_norm")
+            assert path in _lib.profile_report()
+        finally:
+            lib.kda_profile_enable(0)
+        assert not o[:shift].any() and not o[shift + y.numel():].any()
+        results.append([o[shift:shift + y.numel()], y, inv])
+    assert all(torch.equal(a, b) and a.any() for a, b in zip(*results))
