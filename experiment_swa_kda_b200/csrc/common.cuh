@@ -230,7 +230,8 @@ inline int set_smem_limit(Kern kern, size_t bytes) {
 }
 
 // Host-side launch check: returns a KDA_ERR_* code instead of throwing.
-inline int launch_status() {
+// Takes the error of a failed launch away as it reports it, so whoever asks has to pass the answer on.
+[[nodiscard]] inline int launch_status() {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess && getenv("KDA_B200_VERBOSE")) fprintf(stderr, "libkda_b200: CUDA error: %s\n", cudaGetErrorString(e));
     return e == cudaSuccess ? KDA_OK : KDA_ERR_CUDA;

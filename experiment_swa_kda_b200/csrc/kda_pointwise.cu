@@ -2221,7 +2221,7 @@ namespace {
 
 // Sums of the partial rows the launch before this one left: early, so that a few small blocks stand ready when its last ones end
 // (with the gap a launch of their own cost: norm 4.1 + 2.1 us behind a 8.2 us kernel, convolutions 2.3 + 2.4).
-int column_sums(const char* name, int n, int nblk, int N, const float* part, const pw::ColumnSumItems& outs, int bf16, cudaStream_t st) {
+[[nodiscard]] int column_sums(const char* name, int n, int nblk, int N, const float* part, const pw::ColumnSumItems& outs, int bf16, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     KDA_LAUNCH(name, st, e = launch_early(pw::column_sum_kernel, dim3(ceil_div(N, 32), n), 1024, 0, st, nblk > 0, 1, nblk, N, part, outs, bf16));
     return e == cudaSuccess ? launch_status() : KDA_ERR_CUDA;
@@ -2588,7 +2588,7 @@ void rms_bwd_launch(int nb, int64_t rows, int32_t dim, int32_t io_dtype, const v
         else KDA_LAUNCH("rmsnorm_bwd_kernel", st, pw::rmsnorm_bwd_kernel<false, false, PARTS><<<nb, 256, smem, st>>>(rows, dim, x, gate, weight, inv_rms, d_y, dx, dgate, part));
     }
 }
-int rms_dw_launch(int nb, int32_t dim, const float* part, float* dweight, cudaStream_t st) {
+[[nodiscard]] int rms_dw_launch(int nb, int32_t dim, const float* part, float* dweight, cudaStream_t st) {
     pw::ColumnSumItems outs = {};
     outs.out[0] = dweight;
     return column_sums("rmsnorm_dw_reduce_kernel", 1, nb, dim, part, outs, 0, st);
@@ -2606,8 +2606,7 @@ extern "C" int kda_rmsnorm_gate_bwd(int64_t rows, int32_t dim, int32_t io_dtype,
     const int nb = rows > 0 ? rms_blocks(rows) : 0;
     float* part = static_cast<float*>(scratch);
     if (nb > 0) rms_bwd_launch<pw::kRmsAll>(nb, rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, part, st);
-    rms_dw_launch(nb, dim, part, dweight, st);
-    return launch_status();
+    return rms_dw_launch(nb, dim, part, dweight, st);
 }
 
 extern "C" int kda_rmsnorm_gate_bwd_rows(int64_t rows, int32_t io_dtype, int32_t heads, int32_t gate_ld, const void* x, const void* gate,
@@ -2650,15 +2649,13 @@ extern "C" int kda_rmsnorm_gate_bwd_static(int64_t rows, int32_t dim, int32_t io
     if (!weight || !dweight) return KDA_ERR_NULL;
     if (rows > 0 && (!x || !gate || !inv_rms || !d_y || !dx || !dgate)) return KDA_ERR_NULL;
     cudaStream_t st = (cudaStream_t)stream;
-    if (rows == 0) {
-        rms_dw_launch(0, dim, nullptr, dweight, st);
-        return launch_status();
-    }
+    if (rows == 0) return rms_dw_launch(0, dim, nullptr, dweight, st);
     const int nb = rms_blocks(rows);
     // bf16 rows may start at an odd element, floats may not: 2 bytes of slack, and more than 8 rows have room for it
     float* part = nb == 1 ? dweight : reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(dx) + 3) / 4 * 4);
     rms_bwd_launch<pw::kRmsWeight>(nb, rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, part, st);
-    if (nb > 1) rms_dw_launch(nb, dim, part, dweight, st);
+    if (nb > 1)
+        if (int rc = rms_dw_launch(nb, dim, part, dweight, st)) return rc;
     rms_bwd_launch<pw::kRmsInputs>(nb, rows, dim, io_dtype, x, gate, weight, inv_rms, d_y, dx, dgate, nullptr, st);
     return launch_status();
 }

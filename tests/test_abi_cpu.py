@@ -172,3 +172,20 @@ def test_the_layers_products_follow_the_reduced_precision_setting():
             assert _native.load().product_math() == mode
     finally:
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = flag
+
+
+def test_no_launchs_status_is_dropped():
+    """launch_status() takes a failed launch's error away: a caller that ignores the answer of a function that asks reports success."""
+    csrc = os.path.join(ROOT, "experiment_swa_kda_b200", "csrc")
+    text = {f: open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc))}
+    asking = {"launch_status"}
+    while True:      # functions that return what one of these says
+        more = {n for t in text.values() for n, body in re.findall(r"^(?:\S[^\n]* )?int (\w+)\([^;{]*\) \{\n(.*?)^\}", t, re.S | re.M)
+                if re.search(r"\b(%s)(<[^<>]*>)?\(" % "|".join(sorted(asking)), body)} - asking
+        if not more:
+            break
+        asking |= more
+    assert {"column_sums", "rms_dw_launch", "simt_chunk_bwd", "kda_chunk_fwd_ex"} <= asking
+    call = re.compile(r"^\s*(?:(?:if|else|for)\b.*?\s)?(?:tc::|pw::|tok::)?(?:%s)(?:<[^<>]*>)?\(.*\);" % "|".join(sorted(asking)))
+    dropped = [(f, line) for f, t in text.items() for line in t.split("\n") if call.match(line) and not re.search(r"return|= ", line)]
+    assert not dropped, dropped
