@@ -70,8 +70,10 @@ __device__ __forceinline__ float warp_sum(float x) {
     return x;
 }
 
-// A kernel that may start while the one before it in its stream still runs (programmatic dependent launch).  Kernels launched
-// this way wait (dependency_wait) before they touch anything a kernel of the same call writes, and none of them holds tensor memory.
+// A kernel that may start while the one before it in its stream still runs (programmatic dependent launch), and while those run that that
+// one started beside.  Kernels launched this way wait (dependency_wait) before they touch anything these write; convolutions and gate
+// activations, which share nothing with them, wait at their own end, so that whatever is launched the usual way finds all of them done.
+// None of them holds tensor memory.
 template <class... P, class... A>
 inline cudaError_t launch_early(void (*kern)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool early, int cluster, A... args) {
     cudaLaunchConfig_t cfg = {};

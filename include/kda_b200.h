@@ -40,12 +40,15 @@ extern "C" {
  * not; each weight is then rounded to the activation dtype as it is loaded (the result a cast of the weight tensor
  * would give) and no converted copy of the weights is needed. */
 #define KDA_WEIGHT_F32 0x100
-/* Added to the weight_dtype of kda_rows_linear or the fb_dtype of kda_token_mix: the launch before this one in the stream is one of
- * these two calls' (of the same token), which write no weights and no memory state.  The kernel may then start beside that launch
- * and read weights and state before it has ended. */
+/* Added to the weight_dtype of kda_rows_linear or the fb_dtype of kda_token_mix: the kernel may start beside the launches before it, back to
+ * the newest one in the stream without this flag, and reads its weights (kda_token_mix: fb_weight, A_log, dt_bias, norm_weight and state_in as
+ * well) before they have ended.  So all launches from that one on are these two calls', none of them writes what this call reads early
+ * - not, for one, two kda_token_mix calls on the same state -, and that one without the flag is a launch of the usual kind.  Everything
+ * else is read, and anything is written, once the launch before has ended. */
 #define KDA_BEHIND_OWN_LAUNCH 0x400
-/* Added to the io_dtype of kda_conv_fwd_rows or kda_gate_fwd_rows: the launch before this one in the stream is one of these two calls',
- * and neither touches what the other writes.  The kernel may then run beside it; it does not end before that one has. */
+/* Added to the io_dtype of kda_conv_fwd_rows or kda_gate_fwd_rows: the kernel may run beside the launches before it, back to the newest one in
+ * the stream without this flag.  So all launches from that one on are these two calls', and none of them touches what another of them
+ * writes.  It does not end before the one before it has, so a launch without the flag finds all of them done. */
 #define KDA_BESIDE_OWN_LAUNCH 0x800
 /* kda_conv_bwd only: OR this into io_dtype when `dweight` is bfloat16; the float32 sums are rounded as they are written. */
 #define KDA_DWEIGHT_BF16 0x200
