@@ -2171,15 +2171,20 @@ extern "C" int kda_token_mix(int32_t n_seq, int32_t heads, float scale, const vo
     cudaStream_t st = (cudaStream_t)stream;
     const int blocks = n_seq * heads;
     cudaError_t e = cudaSuccess;
-    // Blocks of 32, 16 and 8 warps go one, two and four to an SM.  Clusters are placed whole, and unevenly, so blocks that would fill the
-    // SMs just once, or by halves, are on their own (a token's three launches in us before / clusters / alone: 37 x 16 states 58.2 / 61.9 /
-    // 54.2, 28 x 16 43.7 / 39.9 / -, 48 x 12 44.0 / 46.2 / 40.1).  And blocks that start beside the projections' take the SMs these leave
-    // free, four to one and none to the next: with two to an SM in the end, where that counts, they start behind them (24 x 12 28.7 / 29.8
-    // early / 25.9, 48 x 6 28.1 / 29.7 / 26.4).
-    const int nw = blocks <= 148 ? 32 : (blocks <= 256 ? 16 : 8), cluster = nw == 16 || (blocks > 340 && blocks <= 548) || blocks > 592 ? 4 : 1;
+    // Blocks of 32, 16 and 8 warps go one, two and four to an SM (148 of them).  Clusters share the gate's rows but are placed whole, and
+    // unevenly from nine tenths of all places on: blocks are on their own there, and where they come in waves (a token's three launches in us,
+    // clusters / alone, 8 warps, 2,048 wide: 480 states 44.0 / 44.6, 528 56.8 / 55.8, 544 60.4 / 55.8, 592 66.1 / 57.4, 608 65.5 / 61.0, 768 69.1 /
+    // 67.1, 1,024 75.3 / 74.3; clusters of 16 warps / 8 warps alone: 256 33.3 / 36.9, 264 (768 wide) 26.6 / 29.2, 288 41.0 / 38.4).  And blocks that
+    // start beside the projections' take the SMs these leave free, four to one and none to the next: up to three to an SM in the end they
+    // start behind them (early in clusters / behind, alone: 288 39.5 / 38.4, 1,536 wide 31.2 / 29.2, 408 41.5 / 39.9, 432 41.0 / 39.9; 448, 2,048
+    // wide, 43.5 / 45.6, 480 44.0 / 46.1).
+    constexpr int kSms = 148;
+    const int nw = blocks <= kSms ? 32 : (10 * blocks <= 9 * 2 * kSms ? 16 : 8);
+    const bool behind = nw == 8 && blocks <= 3 * kSms;
+    const int cluster = nw == 16 || (nw == 8 && !behind && 10 * blocks <= 9 * 4 * kSms) ? 4 : 1;
     const auto kern = nw == 32 ? pw::decode_kernel<1, 4, 32, true, 1>
                                : (nw == 16 ? pw::decode_kernel<1, 4, 16, true, 4> : (cluster == 4 ? pw::decode_kernel<1, 4, 8, true, 4> : pw::decode_kernel<1, 4, 8, true, 1>));
-    KDA_LAUNCH("decode_kernel", st, e = launch_early(kern, dim3(ceil_div(blocks, cluster) * cluster), 32u * nw, 0, st, early && (blocks <= 256 || blocks > 384), cluster, heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits,
+    KDA_LAUNCH("decode_kernel", st, e = launch_early(kern, dim3(ceil_div(blocks, cluster) * cluster), 32u * nw, 0, st, early && !behind, cluster, heads, 128, 128, 1, 1, 1, scale, q, k, v, nullptr, beta_logits,
                                                      state_in, state_out, mixed, 128, raw, mix));
     if (e != cudaSuccess) return KDA_ERR_CUDA;
     return launch_status();

@@ -1,5 +1,5 @@
-"""A token's three launches overlap: weights, state and the gate's weights are read while the launch before still runs, and above 148
-states the blocks of four sequences form a cluster.  Many tokens in a row have to give the bits of the launches one by one."""
+"""A token's three launches overlap: weights, state and the gate's weights are read while the launch before still runs, and at 149 to 266 and 445
+to 532 states the blocks of four sequences form a cluster.  Many tokens in a row have to give the bits of the launches one by one."""
 
 import pytest
 import torch
@@ -8,10 +8,13 @@ pytestmark = pytest.mark.gpu
 D0 = "cuda:0"
 
 
-def _layer(heads, seed):
+def _layer(heads, seed, dtype=torch.float32):
     import experiment_swa_kda_b200 as m
     torch.manual_seed(seed)
     layer = m.KimiDeltaAttention(hidden_size=heads * 128, num_heads=heads, head_dim=128, conv_size=4, norm_eps=1e-6).to(D0).eval()
+    for name, p in layer.named_parameters():
+        if name not in ("A_log", "dt_bias", "o_norm.weight"):
+            p.data = p.data.to(dtype)
     with torch.no_grad():
         for p in layer.parameters():
             if p.dim() > 1:
@@ -19,10 +22,14 @@ def _layer(heads, seed):
     return m, layer
 
 
-# one block a state up to 148 states; clusters with 0, 1, 2 and 3 sequences over; output projections of one and of two tiles a CTA
-@pytest.mark.parametrize("batch,heads", [(1, 1), (9, 16), (10, 16), (13, 12), (50, 3), (40, 4), (7, 40)])
-def test_overlapping_launches_give_the_bits_of_separate_ones(batch, heads):
-    m, layer = _layer(heads, batch)
+# 32 warps a state up to 148 states; clusters of 16 (149 .. 266: 150, 156, 160, 264) and of 8 warps (445 .. 532: 448, 455, 465, 506, 512, 532) with 0,
+# 1, 2 and 3 sequences over, and blocks over that fill the last cluster; 8 warps on their own, behind the projections (267 .. 444) and early (above 532)
+@pytest.mark.parametrize("batch,heads,dtype", [(1, 1, torch.float32), (9, 16, torch.float32), (10, 16, torch.float32), (13, 12, torch.float32), (50, 3, torch.float32),
+                                               (40, 4, torch.bfloat16), (44, 6, torch.float32), (7, 40, torch.float32), (37, 12, torch.float32), (28, 16, torch.float32),
+                                               (35, 13, torch.float32), (31, 15, torch.bfloat16), (46, 11, torch.float32), (32, 16, torch.float32), (38, 14, torch.float32),
+                                               (41, 13, torch.float32), (43, 14, torch.float32)])
+def test_overlapping_launches_give_the_bits_of_separate_ones(batch, heads, dtype):
+    m, layer = _layer(heads, batch, dtype)
     x = torch.randn(24, batch, 1, heads * 128, generator=torch.Generator().manual_seed(heads)).bfloat16().to(D0)
     a = m.KDAState.zeros(batch, heads, 128, 4, D0)
     a.memory.normal_(generator=torch.Generator(device=D0).manual_seed(1)).mul_(0.02)
