@@ -132,13 +132,14 @@ constexpr int kWkFwdThreads = (kWkState + 12) * 32, kWkBwdThreads = (kWkState + 
 // The terms of the next step without the state, E^T U (backward: A^T dO and R^T dO), are issued behind this step's last product.
 // Why not E^T Z in one product: U is in bf16 already, and Z = U - W H would be rounded a second time on its way into the sum that the state
 // is.  The final state was then 1.08 to 1.20 times as far from float64 as that of split scans, which have E^T U and H Pn apart as well; now
-// 1.00.  W H takes U's place in the stage, piece by piece where a warp has read U.  The price is a product and 8 KB more a step that shared
-// memory has to find time for, and operands that are wanted earlier: 1.17 -> 1.39 us with 32 recurrences of 128 chunks, 381 -> 406 us below.
-// (E^T Z and E^T times what rounding took from Z: 1.45; E^T U between W H and R H: 1.43.)
+// 1.00.  W H takes U's place in the stage, piece by piece where a warp has read U.  The price is a product and 8 KB more a step: 1.17 -> 1.32 us
+// with 32 recurrences of 128 chunks, 381 -> 398 us below.  The lane that issues products is busy all step long (about 50 cycles a product, more
+// a wait), so what E^T U needs comes as one group: with E and A a group of their own 1.39, R and A as well 1.5; E^T Z and E^T times what
+// rounding took from Z 1.45; E^T U between W H and R H 1.43.
 // The norm needs whole rows: the two blocks of a recurrence are a cluster then and swap their sums of squares, warp by warp.
 // Many recurrences: bound by the bytes of the panels, 136 KB a chunk-head forward and 120 backward (16,544 chunk-heads in 352
-// recurrences: 406 and 337 us, 0.85 and 0.91 of the copy rate; scan and output kernel took 258 + 305 us, scan and dZ kernel 254 + 219, and the
-// intra-chunk forward, which formed the scans' maps, 915 instead of 801).  Few: a step of about 2,600 cycles forward and 1,840 backward,
+// recurrences: 398 and 337 us, 0.87 and 0.91 of the copy rate; scan and output kernel took 258 + 305 us, scan and dZ kernel 254 + 219, and the
+// intra-chunk forward, which formed the scans' maps, 915 instead of 801).  Few: a step of about 2,400 cycles forward and 1,840 backward,
 // of which the products' operands, the loads and the stores keep shared memory busy for 2,050 and 1,800 (a product reads A and B at 128 bytes a
 // cycle, no faster than it multiplies them); what a step waits for besides is the way from a product's end to the next one's start, twice.
 // Whatever can be there early is therefore looked for while a product runs, a lane that issues products commits three times a step, and
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
     if (warp == kWkState) {
         // ------------------------------------------------------------------ load warp
         if (elect_one()) {
-            // groups by when their products are done: forward W R | E A | U, decays; backward A dO R | E | W, decays
+            // groups by when they are wanted: forward U E, decays (2) | W R A (0); backward A dO R | E | W, decays
             auto load = [&](int c, int g) {
                 const int cs = slot_of(c), ch = cs * H + h, s = c & 1;
                 uint8_t* b = sm + s * kWkStage;
@@ -216,34 +217,38 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
                 auto ld_r = [&]() { for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + kWkR + nb * 8192, &mR, f, nb * 64, ch * 64); };
                 auto ld_e = [&]() { for (int nb = 0; nb < 2; ++nb) tma_load_2d(b + kWkE + nb * 8192, &mE, f, nb * 64, ch * 64); };
                 auto ld_a = [&]() { tma_load_2d(b + kWkA, &mA, f, 0, ch * 64); };
-                if (g == 0) {
+                if (kBwd && g == 0) {
                     mbar_expect_tx(f, 32768);
-                    if (kBwd) {
-                        int tok0, len;
-                        p.tab.span(cs, tok0, len);
-                        tma_load_2d(b + kWkU, &mU, f, h * 128 + half * 64, tok0);
-                        ld_a();
-                    } else {
-                        ld_w();
-                    }
+                    int tok0, len;
+                    p.tab.span(cs, tok0, len);
+                    tma_load_2d(b + kWkU, &mU, f, h * 128 + half * 64, tok0);
+                    ld_a();
                     ld_r();
-                } else if (g == 1) {
-                    mbar_expect_tx(f, kBwd ? 16384 : 24576);
+                } else if (kBwd && g == 1) {
+                    mbar_expect_tx(f, 16384);
                     ld_e();
-                    if (!kBwd) ld_a();
+                } else if (g == 0) {
+                    mbar_expect_tx(f, 40960);
+                    ld_w();
+                    ld_r();
+                    ld_a();
                 } else {
-                    mbar_expect_tx(f, (kBwd ? 16384 : 8192) + 512);
+                    mbar_expect_tx(f, (kBwd ? 16384 : 24576) + 512);
                     bulk_load_1d(dec_ring[c & 3], p.decay_end + (size_t)ch * 128, 512, f);
-                    if (kBwd) ld_w();
-                    else tma_load_2d(b + kWkU, &mU, f, 0, ch * 128 + half * 64);
+                    if (kBwd) {
+                        ld_w();
+                    } else {
+                        tma_load_2d(b + kWkU, &mU, f, 0, ch * 128 + half * 64);
+                        ld_e();
+                    }
                 }
             };
             bool ok = true;
             int c = 0;
             for (; c < n && ok; ++c) {
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const int g = kBwd ? i : 2 - i;      // in the order in which they are needed
+                for (int i = 0; i < (kBwd ? 3 : 2); ++i) {
+                    const int g = kBwd ? i : 2 - 2 * i;      // in the order in which they are wanted
                     if (ok && c > 1 && (i == 0 || (kBwd && i == 2))) ok = mbar_wait(bar_free(g, c & 1), ph(c - 2), p.status, 100);
                     if (ok) load(c, g);
                 }
@@ -254,7 +259,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             } else {       // unwinding: the copies in flight must land first
                 abort_flag = 1;
                 for (int cc = c > 2 ? c - 3 : 0; cc < c; ++cc)
-                    for (int g = 0; g < 3; ++g) mbar_poll(bar_full(g, cc & 1), ph(cc), kSpinLimit / 8);
+                    for (int g = 0; g < 3; g += kBwd ? 1 : 2) mbar_poll(bar_full(g, cc & 1), ph(cc), kSpinLimit / 8);
             }
         }
     } else if (warp == kWkState + 1) {
@@ -303,7 +308,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
                 ok = ok && mbar_wait(b, parity, p.status, code);
                 return ok;
             };
-            auto early_full = [&](int c) { return kBwd ? wait(bar_full(0, c & 1), ph(c), 103) : wait(bar_full(1, c & 1), ph(c), 103) && wait(bar_full(2, c & 1), ph(c), 103); };
+            auto early_full = [&](int c) { return kBwd ? wait(bar_full(0, c & 1), ph(c), 103) : wait(bar_full(2, c & 1), ph(c), 103); };
             if (early_full(0)) {
                 tc_fence_after();
                 early(0);
