@@ -52,23 +52,31 @@ struct NormEpilogue {
 };
 
 // How a batch goes through its recurrences: 1 - walks (kda_tc_walk.cu), two blocks to a (sequence, head) -, or the number of segments of
-// split scans (kda_tc_pscan.cu).  The decision uses the shape alone (a packed batch is judged by its mean sequence length: the lengths
-// themselves live on the device), so the forward and the backward of a call agree; split, every sequence of the batch is cut into the
-// same number of segments, short ones into segments of one chunk or none.
-// A walk's step takes about 1.1 us each way and has everything behind it done; split scans take a quarter of a step's 0.8 us for the
-// chain, but 48 + 176 KB more of memory traffic for every chunk of every recurrence, and three more launches each way.  So the walk
-// falls behind where there are few recurrences and many chunks.  Forward and backward in us, split / walk, by recurrences x chunks:
-// 2 x 16: 72 / 64, 2 x 32: 79 / 94, 12 x 32: 146 / 144, 12 x 128: 415 / 481, 16 x 32: 174 / 160, 16 x 128: 515 / 540, 32 x 128: 921 / 815.
+// split scans (kda_tc_pscan.cu).  The decision uses the shape alone, so the forward and the backward of a call agree; split, every sequence of
+// the batch is cut into the same number of segments, short ones into segments of one chunk or none.
+// A walk's step takes about 1.2 us forward and 1.0 back and has everything behind it done; split scans take a quarter of a step's 0.8 us for
+// the chain, but 48 + 176 KB more of memory traffic for every chunk of every recurrence, and three more launches each way.  So the walk
+// falls behind where there are few recurrences and many chunks.  Forward and backward in us, four segments / walk, by recurrences x chunks:
+// 1 x 16: 86 / 82, 2 x 24: 90 / 96, 6 x 20: 92 / 90, 8 x 24: 107 / 109, 12 x 24: 119 / 113, 12 x 32: 154 / 156 (a whole layer 356 / 352), 14 x 40: 193 /
+// 193, 16 x 40: 219 / 213, 16 x 64: 295 / 309, 18 x 64: 328 / 327, 18 x 96: 459 / 469, 20 x 96: 500 / 494, 24 x 96: 608 / 549: chunks * (24 - recurrences) > 384.
 // Eight segments halve the chain again and lengthen the fix-up's by four products; worth it where the chain is long and SMs are idle (4 / 8
-// segments: 1 x 128 123 / 111, 2 x 256 266 / 228, 6 x 256 461 / 439; 6 x 128 264 / 262, 6 x 64 158 / 163, 8 x 128 306 / 309).
-// Two segments (17 to 49 recurrences, or 16 to 31 chunks, of the measured split side) are behind the walk wherever they were chosen.
+// segments: 1 x 64 109 / 109, 1 x 128 139 / 125, 2 x 192 219 / 197, 6 x 192 361 / 346; 6 x 128 270 / 266, 6 x 64 166 / 170, 8 x 128 313 / 315).
+// A walk is as long as its longest chain.  The lengths of a packed batch live on the device, so that chain is taken for 1.5 times the mean of
+// two or three sequences and 2.25 times that of more (uniform lengths between 256 and 8,192 make 1.3 to 1.9, one long document among short ones more).
+// Up to 21 recurrences, seven units each to the SMs at once, then split from 16 chunks on (sequences x heads, us split / walk, lengths from 256 to
+// 8,192: 20 x 1 406 / 473, 4 x 4 340 / 438, 16 x 1 330 / 418, 2 x 8 307 / 350, 6 x 3 293 / 328, 7 x 3 317 / 340, 10 x 2 481 / 512; up to 3,000: 4 x 4 191 / 201, 10
+// x 2 205 / 207, 7 x 3 205 / 197, 5 x 3 158 / 150).  Up to 33 there is little in it for uniform lengths, and two segments are safer (5 x 6 528 / 539, 6 x 4
+// 358 / 369, 4 x 8 573 / 571, 31 x 1 571 / 567, 16 x 2 545 / 535, 8 x 4 727 / 678; one document of 900 chunks and 30 of 4: 1,384 / 2,021); with fewer than 32
+// chunks the walk's fewer launches count (3 x 8 236 / 223, 31 x 1 244 / 225, 16 x 2 262 / 240).  Beyond, the walk is ahead for those lengths (40 x 1 705 / 647,
+// 49 x 1 787 / 709, 3 x 16 1,081 / 912) and behind for a batch that one document makes up.
 inline int scan_segments(const KdaChunkShape& sh) {
     if (sh.n_seq <= 0) return 1;
-    const bool fixed = sh.seq_len > 0 && (long long)sh.n_seq * sh.seq_len == sh.tokens;
+    const bool packed = sh.seq_len <= 0 && sh.n_seq > 1;
     const long long rec = (long long)sh.n_seq * sh.heads;
-    const long long chunks = fixed ? (sh.seq_len + 63) / 64 : (sh.tokens / 64) / sh.n_seq;
-    if (rec >= 21 || chunks * (21 - rec) <= 350) return 1;
-    return rec <= 6 && chunks >= 96 ? 8 : 4;      // 2 nseg - 1 scan units to a recurrence: at most 140, one to an SM
+    const long long chunks = sh.seq_len > 0 ? (sh.seq_len + 63) / 64 : (sh.tokens / 64) / sh.n_seq;      // of a sequence, in the mean
+    const int quarters = !packed ? 4 : (sh.n_seq < 4 ? 6 : 9);                                           // of the mean to the longest
+    if (rec < (packed ? 22 : 21) && chunks * (6 * quarters - rec) > 384 && (!packed || chunks >= 16)) return rec <= 6 && chunks >= 96 ? 8 : 4;
+    return quarters == 9 && rec <= 33 && chunks >= 32 ? 2 : 1;      // 2 nseg - 1 scan units to a recurrence
 }
 
 inline TcWs carve_tc(const KdaChunkShape& sh, void* mem, size_t* bytes = nullptr) {

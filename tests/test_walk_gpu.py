@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import kda_oracle as O
-from test_tc_lane_gpu import D0, _kda_mod, _run_activated
+from test_tc_lane_gpu import BF16_TOL, D0, _kda_mod, _run_activated
 
 pytestmark = pytest.mark.gpu
 
@@ -48,7 +48,7 @@ def test_walk_and_split_scans_agree(tokens):
     do = torch.randn(1, tokens, 2, 128, generator=gen).bfloat16().to(D0)
     ds = torch.randn(1, 2, 128, 128, generator=gen).to(D0)
     res = []
-    for empty in (0, 5):
+    for empty in (0, 8):
         x = {n: (t.float() if n == "h0" else t.bfloat16()).to(D0) for n, t in d.items()}
         x["h0"] = torch.cat([x["h0"], torch.ones(empty, 2, 128, 128, device=D0)])
         x = {n: t.requires_grad_(True) for n, t in x.items()}
@@ -141,3 +141,42 @@ def test_output_of_the_norms_forward_at_an_8_byte_address(batch, tokens, path):
         assert not o[:shift].any() and not o[shift + y.numel():].any()
         results.append([o[shift:shift + y.numel()], y, inv])
     assert all(torch.equal(a, b) and a.any() for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("lens,H,segments", [([64 * 20 + 5, 64 * 9, 64 * 16, 64 * 18 + 1], 4, 1),                                         # 16 recurrences, mean 15
+                                             ([64 * 70 + 7, 30, 64 * 3 + 9, 0], 4, 4),                                                 # 16, mean 18
+                                             ([64 * 50, 64 * 3 + 9, 64 * 19 + 63], 7, 1),                                              # 21, mean 24, three sequences
+                                             ([64 * 60, 64 * 3 + 9, 64 * 19 + 63, 0, 5, 64 * 30, 64 * 9], 3, 4),                       # 21, mean 17, seven
+                                             ([64, 64 * 110 + 7, 64 * 4 + 3, 0], 7, 1),                                                # 28, mean 28
+                                             ([64 * 120 + 1, 64, 64 * 4 + 3, 5], 6, 1),                                                # 24, mean 31
+                                             ([64 * 125 + 1, 64, 64 * 4 + 3, 5], 6, 2),                                                # 24, mean 32
+                                             ([64 * 300 + 5, 30, 0], 1, 8), ([1, 64 * 200 + 63, 64 * 90, 0], 1, 4)])                   # 3, mean 100; 4, mean 72
+def test_packed_batches_take_the_way_their_shape_says(lens, H, segments):
+    """Which kernels run, and every output against the oracle: chains of very different lengths, segments of one chunk or none, empty sequences."""
+    from experiment_swa_kda_b200 import _lib
+    m = _kda_mod()
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    d = O.make_inputs(1, cu[-1], H, 128, 128, seed=500 + H, with_state=True, n_states=len(lens))
+    x = {n: (t.float() if n == "h0" else t.bfloat16()).to(D0).requires_grad_(True) for n, t in d.items()}
+    gen = torch.Generator().manual_seed(17)
+    do, ds = torch.randn(d["v"].shape, generator=gen).bfloat16().to(D0), torch.randn(d["h0"].shape, generator=gen).to(D0)
+    _lib.load().kda_profile_enable(1)
+    try:
+        o, s = m.chunk_kda(x["q"], x["k"], x["v"], x["g"], x["beta"], initial_state=x["h0"], output_final_state=True, lane="tc",
+                           cu_seqlens=torch.tensor(cu, dtype=torch.int32, device=D0))
+        got = [o, s, *torch.autograd.grad((o, s), list(x.values()), (do, ds))]
+        ran = set(_lib.profile_report())
+    finally:
+        _lib.load().kda_profile_enable(0)
+    walked = {"tc_walk_fwd_kernel", "tc_walk_bwd_kernel"}
+    assert ran & walked == (walked if segments == 1 else set()) and ("tc_scan_fixup_kernel" in ran) == (segments > 1)
+    # segments: 2 segments - 1 final states of 96 KB a recurrence, beside what each chunk-head has
+    sh = _lib.ChunkShape(len(lens), 0, cu[-1], H, 128, 128, _lib.DTYPE_BF16, _lib.DTYPE_BF16, _lib.LANE_TC, 1, 0.1)
+    panels = (cu[-1] // 64 + len(lens)) * H * (6 * 16384 + 3 * 8192 + 2 * 32768 + 512 + 768 + (0 if segments == 1 else 16384 + 2 * 32768))
+    assert (_lib.load().kda_chunk_workspace_bytes(sh) - panels) // (len(lens) * H * 98304) == (0 if segments == 1 else 2 * segments - 1)
+    y = {n: t.detach().float().requires_grad_(True) for n, t in x.items()}
+    eo, es = O.kda_recurrence_varlen(y["q"], y["k"], y["v"], y["g"], y["beta"], cu, initial_state=y["h0"])
+    for a, b in zip(got, (eo, es, *torch.autograd.grad((eo, es), list(y.values()), (do.float(), ds)))):
+        assert O.rel_l2(a, b) <= BF16_TOL
