@@ -435,21 +435,43 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = f2_mul(f2_mul(E[e], f2_all(ec[e >> 1])), w[e]);
         put_panel(sb + kR8, 2 * I, w);
-        if constexpr (KV) {      // a key row and a quarter of its values a thread
-            f2 acc = f2_all(0.f);
+        if constexpr (KV) {
+            // Eight adjacent values of four key rows a lane; the four lanes that share the rows add up by halving.  The two halves of a
+            // sum stay apart until the end: of the forms that were tried (a key row and a quarter of its values a thread; ldmatrix; one sum
+            // a row) only this one leaves the rest of the block its registers, and a spill here is a trip to L2 (16,544 chunk-heads 1,324 ->
+            // 1,210 us, spilled loads 44 -> 12 bytes).
+            const int cg = 4 * wq + mi;
+            f2 acc[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] = f2_all(0.f);
             if (ok) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const uint32_t off = (uint32_t)(I >> 1) * 16384 + sw128_off(tid & 127, 4 * (I & 1) + j);
+                    const uint32_t off = (uint32_t)(cg >> 3) * 16384 + sw128_off(32 * I + 8 * j + mr, cg & 7);
                     const uint4 a = *reinterpret_cast<const uint4*>(Hs + off), b = *reinterpret_cast<const uint4*>(dHs + off);
-                    acc = f2_fma(f2_from_bf16(a.x), f2_from_bf16(b.x), acc);
-                    acc = f2_fma(f2_from_bf16(a.y), f2_from_bf16(b.y), acc);
-                    acc = f2_fma(f2_from_bf16(a.z), f2_from_bf16(b.z), acc);
-                    acc = f2_fma(f2_from_bf16(a.w), f2_from_bf16(b.w), acc);
+                    acc[j] = f2_fma(f2_from_bf16(a.x), f2_from_bf16(b.x), acc[j]);
+                    acc[j] = f2_fma(f2_from_bf16(a.y), f2_from_bf16(b.y), acc[j]);
+                    acc[j] = f2_fma(f2_from_bf16(a.z), f2_from_bf16(b.z), acc[j]);
+                    acc[j] = f2_fma(f2_from_bf16(a.w), f2_from_bf16(b.w), acc[j]);
                 }
             }
-            const float2 x = f2_get(acc);
-            part[tid] = x.x + x.y;
+            float v8[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 x = f2_get(acc[e]);
+                v8[2 * e] = x.x;
+                v8[2 * e + 1] = x.y;
+            }
+#pragma unroll
+            for (int o = 4; o >= 2; o >>= 1) {
+                const bool up = (mi & (o >> 1)) != 0;
+#pragma unroll
+                for (int j = 0; j < o; ++j) {
+                    const float send = up ? v8[j] : v8[j + o], keep = up ? v8[j + o] : v8[j];
+                    v8[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * o);
+                }
+            }
+            part[wq * 128 + 32 * I + 8 * mi + mr] = v8[0] + v8[1];
         } else {
             // eight adjacent channels of four value rows a lane; the warp's eight lanes that share them add up by halving
             const int cg = 4 * wq + mi;
