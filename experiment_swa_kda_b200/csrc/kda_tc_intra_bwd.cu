@@ -5,7 +5,7 @@
 // tcgen05.ld.16x256b reads, ldmatrix.trans takes from a [token][channel] tile and stmatrix puts back, transposed or not.
 //
 // Products (all on tcgen05; "^T" = channel-major result, M = 128; token x token results use M = 64):
-//   dR^T = H dO^T          dW^T = H dZ^T          dE^T = dH' Z^T            (H, dH' V-first panels: MN-major A)
+//   dR^T = H dO^T          dW^T = H dZ^T          dE^T = dH' Z^T            (H, dH' K-major A from a walk, MN-major from split scans)
 //   dP^T = dZ^T T          dQ^T = -dW^T T                                   (T row-major: MN-major B)
 //   dA   = tril(dO Z^T)    Xraw^T = v dZ^T - (e^G k) dW^T    (X = Xraw diag(beta) is the adjoint of T)
 //   Y    = T^T X           dM = -stril(Y T^T)
@@ -119,8 +119,8 @@ struct IntraBwdArgs {
 // shared-memory map (bytes, 1024-aligned base)
 constexpr int kR1 = 0;         // 64 KB  H | dH' panels            -> later: k~_I source panels (4 x 16 KB)
 constexpr int kR2 = 65536;     // 16 KB  dO tile                   -> later: X^T tile (8 KB) | Y tile (8 KB)
-constexpr int kR3 = 81920;     // 16 KB  Z^T panel                 -> later: target stacks I = 0,1 (2 x 8 KB)
-constexpr int kR4 = 98304;     // 16 KB  dZ^T panel                -> later: target stacks I = 2,3
+constexpr int kR3 = 81920;     // 16 KB  Z panel                   -> later: target stacks I = 0,1 (2 x 8 KB)
+constexpr int kR4 = 98304;     // 16 KB  dZ panel                  -> later: target stacks I = 2,3
 constexpr int kR5 = 114688;    // 48 KB  q | k | v tiles           -> later: dq | dk | dv, on their way out
 constexpr int kR6 = 163840;    //  8 KB  T
 constexpr int kR7 = 172032;    // 16 KB  dW^T                      -> later: [dA_I ; beta dM_I] tiles (4 x 4 KB), dg on its way out
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(512, 1)
     };
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
-    constexpr uint32_t kBytesA = 65536 + 3 * 16384 + 2 * 8192;      // H, dH', Z^T, dZ^T, dO, T, M~
+    constexpr uint32_t kBytesA = 65536 + 3 * 16384 + 2 * 8192;      // H, dH', Z, dZ, dO, T, M~
     // The gates come first, then what the critical products and the work beside them need.  The loads are issued by warps 1-4,
     // a few each: one thread issuing all of them held the block back.
     if (tid == 0) {

@@ -29,16 +29,6 @@ __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[16])
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_16x32(taddr, r); }
-__device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld_16x16(taddr, r); }
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* w) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
@@ -564,7 +554,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             uint32_t wh[2 * kPieces];
             {
                 uint32_t r[4 * kPieces];
-                tmem_ld_16(tmem + lane_base + c1 + kWkCols * hf, r);
+                tmem_ld_16x32(tmem + lane_base + c1 + kWkCols * hf, r);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 2 * kPieces; ++i) {
@@ -587,7 +577,7 @@ __global__ void __launch_bounds__(kBwd ? kWkBwdThreads : kWkFwdThreads, 1)
             tc_fence_after();
             {
                 uint32_t r[kWkCols];
-                tmem_ld_cols(tmem + lane_base + c2 + 64 * st + kWkCols * hf, r);
+                tmem_ld32(tmem + lane_base + c2 + 64 * st + kWkCols * hf, r);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < kWkCols / 2; ++j) s[j] = f2_fma(dec, s[j], f2_make(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])));

@@ -36,10 +36,10 @@ struct TcWs {
     int nseg;                   // scan_segments(): 1 - no split scans -, or their segments per (sequence, head); units = 2 * nseg - 1
     float* decay_end;           // [nch][128]       exp(G_end)
     int* status;                // device status word (0 = ok); points at the workspace's word (simt::Ws::status)
-    int fwd_only;               // 1: the backward-only panels (T, M~, Z^T, dH', dZ^T, Rm^T) have no storage and are not written
+    int fwd_only;               // 1: the backward-only panels (T, M~, Z, dH', dZ, Rm^T) have no storage and are not written
 };
 
-// Optional epilogue of the chunk-output kernel: the gated RMSNorm that follows the operator in the layer
+// Optional epilogue of the kernel that forms the outputs (a walk, or the split scans' chunk-output kernel): the gated RMSNorm that follows the operator in the layer
 // (y = o * rsqrt(mean(o^2) + eps) * weight * sigmoid(gate) over the 128 values of a token and head), applied to the
 // output tile while it is still on chip.  o is written as well when the caller passes it: the norm's backward needs it.
 struct NormEpilogue {

@@ -174,13 +174,14 @@ def test_non_finite_tokens_of_the_next_packed_sequence_do_not_leak_into_a_ragged
         assert torch.equal(a[:, :100], b)
 
 
-@pytest.mark.parametrize("T", [2048 + 64 * 3 + 17, 1024 + 64 * 4 + 5])      # 36 chunks -> 4 segments, 21 chunks -> 2 segments
+@pytest.mark.parametrize("T", [2048 + 64 * 3 + 17, 1024 + 64 * 4 + 5])      # 36 and 21 chunks: 4 segments
 def test_split_scans_agree_with_the_single_chain_and_the_oracle(T):
     """A long fixed-length batch with few (sequence, head) recurrences runs every state scan as 2 nseg - 1 units side by
     side (segment 0 from the true state; every later segment once from zero and once as composite maps) plus a
     chunk-parallel fix-up that walks the short chain of segment-start states itself; the same tokens handed over as a
-    packed batch (cu_seqlens) take the single chain.  Both must agree with each other closely and with the oracle inside
-    the bar: outputs, final state (non-zero initial state, ragged tail) and every gradient."""
+    packed batch of one sequence (cu_seqlens) take the same scans by way of the chunk table.  Both must agree with each other
+    closely and with the oracle inside the bar: outputs, final state (non-zero initial state, ragged tail) and every gradient.
+    Split scans against a single chain: test_walk_gpu.py."""
     m = _kda_mod()
     d = O.make_inputs(1, T, 2, 128, 128, seed=91, with_state=True)
     gen = torch.Generator().manual_seed(4)
@@ -257,7 +258,7 @@ def test_without_the_norm_the_gradient_of_q_does_not_depend_on_q():
 
 @pytest.mark.parametrize("lens,H", [([64 * 40 + 5, 30, 64 * 70 + 1], 2),          # 6 recurrences, mean 37 chunks -> 4 segments
                                     ([64 * 60 + 3, 0, 64 * 99, 1], 3),             # 12 recurrences, mean 39 chunks -> 4 segments
-                                    ([64 * 50, 64 * 3 + 9, 0, 64 * 19 + 63], 4)])  # 16 recurrences, mean 18 chunks -> 2 segments
+                                    ([64 * 50, 64 * 3 + 9, 0, 64 * 19 + 63], 4)])  # 16 recurrences, mean 18 chunks -> 4 segments
 def test_split_scans_on_packed_batches_with_short_and_empty_sequences(lens, H):
     """Packed batches with few sequences split their scans too (the decision uses the mean length), so a batch mixes long
     sequences with ones of a single chunk or none: segments of one chunk or zero chunks, composite maps that stay the
@@ -301,7 +302,7 @@ def test_convolutions_inside_the_forward_kernel_equal_convolutions_then_forward(
 
 
 def test_output_norm_in_the_chunk_output_epilogue_equals_the_two_operators_in_sequence():
-    """chunk_kda_norm (gated RMSNorm applied to the output tile inside the chunk-output kernel) against chunk_kda followed
+    """chunk_kda_norm (gated RMSNorm applied to the output tile inside the kernel that forms it, here a walk) against chunk_kda followed
     by RMSNormGated: identical y, final state and gradients (the epilogue repeats the stand-alone kernel's arithmetic),
     one library launch less; ragged packed batch with states."""
     from experiment_swa_kda_b200 import _lib

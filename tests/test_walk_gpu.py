@@ -15,7 +15,7 @@ def test_walked_recurrences_against_the_oracle(tokens):
     _run_activated(O.make_inputs(2, tokens, 3, 128, 128, seed=600 + tokens, with_state=True))
 
 
-@pytest.mark.parametrize("tokens", [64, 127, 128, 192, 193, 256, 321, 449, 837])
+@pytest.mark.parametrize("tokens", [64, 127, 128, 192, 193, 256, 321, 449, 837, 2112, 2137])      # the last two: split scans, in the chunk-output kernel
 def test_norm_in_the_walk_equals_the_two_operators(tokens):
     """The two halves of a row meet between two blocks; same bits as the operator and the norm on their own, with and without a backward."""
     m = _kda_mod()
