@@ -29,8 +29,15 @@ def test_norm_in_the_walk_equals_the_two_operators(tokens):
     o, s = m.chunk_kda(*x, output_final_state=True)
     want = norm(o, gate)
     y, sy = m.chunk_kda_norm(*x, gate, norm.weight, eps=1e-6, output_final_state=True)
-    with torch.no_grad():
-        z, sz = m.chunk_kda_norm(*x, gate, norm.weight, eps=1e-6, output_final_state=True)
+    from experiment_swa_kda_b200 import _lib
+    _lib.load().kda_profile_enable(1)
+    try:
+        with torch.no_grad():
+            z, sz = m.chunk_kda_norm(*x, gate, norm.weight, eps=1e-6, output_final_state=True)
+        ran = _lib.profile_report()
+    finally:
+        _lib.load().kda_profile_enable(0)
+    assert ("tc_chunk_out_kernel" if tokens > 2000 else "tc_walk_fwd_kernel") in ran
     for got in ((y, sy), (z, sz)):
         assert torch.equal(got[0], want) and torch.equal(got[1], s)
     dy = torch.randn(want.shape, generator=gen).bfloat16().to(D0)
